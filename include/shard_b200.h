@@ -281,6 +281,31 @@ int shard_b200_stream_quantize(const ShardSeq* seqs, int32_t batch, int32_t nkv,
                                const float* codebook, void* stream);
 
 /*
+ * The same for `n_tok` new tokens in one launch (a forward over several tokens), rows slot ..
+ * slot + n_tok - 1: token t of KV head h starts at element h * head_stride + t * tok_stride of k / v
+ * (channels contiguous; strides multiples of 4 elements).  k_idx .. v_norm are the stream buffers
+ * [cap][nkv][128] / [cap][nkv].
+ */
+int shard_b200_stream_quantize_rows(const void* k_f16, const void* v_f16, int64_t k_head_stride,
+                                    int64_t k_tok_stride, int64_t v_head_stride, int64_t v_tok_stride,
+                                    int32_t n_tok, int32_t nkv, const float* signs, const float* codebook,
+                                    uint8_t* k_idx, uint8_t* v_idx, void* k_norm, void* v_norm, int32_t slot,
+                                    void* stream);
+
+/*
+ * A compressed layer as fp16 keys and values, [nkv][rows][128] each with rows in the order
+ * [sink | middle | window | stream | fp16 decode buffer]: CacheLayer._ensure_dequant
+ * (src/shard/cache.py:87-124) with its callees, in one launch.  Of `shape` nkv, rank, n_comp, n_sink,
+ * n_win, n_stream, n_dec, dec_cap and append are used (append: new_k / new_v are quantised into stream
+ * row n_stream-1 first); middle token t has position compress_start + t.  `status_dev` (may be NULL)
+ * is set to 1 if a bounded wait inside the kernel gave up (the output is then undefined); the head of
+ * a decode workspace serves, see shard_b200_decode_status.  `codebook` may be NULL without stream rows.
+ */
+int shard_b200_read_back(const ShardSeq* seq_host, const ShardDecodeShape* shape_host, const float* inv_freq,
+                         const float* codebook, int32_t compress_start, void* k_out_f16, void* v_out_f16,
+                         int* status_dev, void* stream);
+
+/*
  * fp16 K/V [nkv][n_stream][128] of the streamed tokens: CacheLayer._dequant_stream
  * (src/shard/cache.py:243-279) + dequantize_per_token (streaming.py:74-79).  Used by
  * the non-fused read path only.

@@ -73,6 +73,21 @@ def _seq_record(gc, dev):
     return seq
 
 
+def row_tensors(gc, nkv, hd):
+    """The fp16 tokens a non-streaming cache appended: (keys, values, rows in use, rows allocated per KV
+    head).  They are views of the rows in use of buffers (1, nkv, capacity, 128) allocated ahead, or
+    plain (1, nkv, s, 128) tensors."""
+    if "decode_k" not in gc:
+        return None, None, 0, 0
+    dk, dv = gc["decode_k"], gc["decode_v"]
+    if dk.dtype != torch.float16:
+        raise NotImplementedError("fp16 models only")
+    if dk.stride(3) != 1 or dk.stride(2) != hd or dv.stride(3) != 1 or dv.stride(2) != hd or dv.stride(1) != dk.stride(1):
+        dk, dv = gc["decode_k"], gc["decode_v"] = dk.contiguous(), dv.contiguous()
+    n_dec = dk.shape[2]
+    return dk, dv, n_dec, dk.stride(1) // hd if nkv > 1 else n_dec
+
+
 class _Launch:
     """Per-layer launch state that does not change from step to step: the sequence record, the
     shape record (only n_stream / pos_q / append / n_dec are touched per step), workspace need
@@ -166,15 +181,7 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
         seq.new_k, seq.new_v = pending[0].data_ptr(), pending[1].data_ptr()
     n_dec = dec_cap = 0
     if with_fp16_segments and "decode_k" in gc:
-        # tokens a non-streaming cache appends as they are: views of the rows in use of buffers
-        # (1, nkv, capacity, 128) allocated ahead, or plain (1, nkv, s, 128) tensors
-        dk, dv = gc["decode_k"], gc["decode_v"]
-        if dk.dtype != torch.float16:
-            raise NotImplementedError("fp16 models only")
-        if dk.stride(3) != 1 or dk.stride(2) != hd or dv.stride(3) != 1 or dv.stride(2) != hd or dv.stride(1) != dk.stride(1):
-            dk, dv = gc["decode_k"], gc["decode_v"] = dk.contiguous(), dv.contiguous()
-        n_dec = dk.shape[2]
-        dec_cap = dk.stride(1) // hd if nkv > 1 else n_dec   # rows allocated per KV head
+        dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd)
         if visible_new is not None:
             n_dec = min(n_dec, int(visible_new))
         seq.dec_k, seq.dec_v = dk.data_ptr(), dv.data_ptr()

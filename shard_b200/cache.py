@@ -22,9 +22,9 @@ import math
 import torch
 from transformers.cache_utils import Cache as HFCache, CacheLayerMixin
 
-from . import ops
+from . import _lib, ops
 from ._lib import ShardError
-from .rope import dp_bit_allocation, get_rope_inv_freq, reapply_rope
+from .rope import dp_bit_allocation, get_rope_inv_freq
 from .streaming import get_codebook, stream_signs
 
 KERNEL_HEAD_DIM = 128
@@ -64,8 +64,8 @@ def pca_fit(flat, mean, rank):
 def hadamard(x):
     """Normalised Walsh-Hadamard transform on the last dim (self-inverse).
 
-    Torch expression used only by the non-fused read path and by tests; the hot
-    paths run the butterfly inside the kernels.
+    Torch expression (the reference's src/shard/cache.py:10-19) for callers; the paths of
+    this package run the butterfly inside the kernels.
     """
     d = x.shape[-1]
     h = 1
@@ -137,45 +137,44 @@ class CacheLayer(CacheLayerMixin):
 
     def _ensure_dequant(self):
         """Full fp16 K/V as [sink | middle | window | stream | fp16 decode buffer]
-        (reference: src/shard/cache.py:87-124).  Off the hot path: used on the
-        first decode step of layer 0, by non-Llama models and by multi-token
-        continuation."""
+        (reference: src/shard/cache.py:87-124), one launch: what models without the fused
+        hook attend to at every step."""
         if not self._needs_decompress:
             return
         gc = self._gpu_compressed
         if gc is None:
             return
+        from .attention import row_tensors, _seq_record
         c = self._cache_ref
-        n_total, rank = gc["k_coeffs_shape"]
-        packed = gc["k_coeffs"]
-        lo = (packed & 0x0F).to(torch.float16) - 8.0
-        hi = ((packed >> 4) & 0x0F).to(torch.float16) - 8.0
-        coeffs = torch.stack([lo, hi], dim=1).flatten()[: n_total * rank].reshape(n_total, rank)
-        coeffs = coeffs * gc["k_coeff_scale"].half()
-        basis = gc["k_basis_q"].to(torch.float16) * gc["k_basis_scale"].half()
-        recon = coeffs @ basis.T + gc["k_mean"].half()
-        B, n_comp = gc["batch"], gc["n_compress"]
-        nkv, hd = c._n_kv_heads, c.head_dim
-        k_layer = recon.view(B, n_comp, nkv, hd).permute(0, 2, 1, 3)
-        if c._rope_inv_freq is not None:
-            pos = torch.arange(gc["compress_start"], gc["compress_start"] + n_comp, device=packed.device)
-            k_mid = reapply_rope(k_layer, pos, c._rope_inv_freq).half()
-        else:
-            k_mid = k_layer.half()
-        cb = gc["v_centroids_f16"].float()
-        v_rot = cb[gc["v_indices_u8"].long()].reshape(nkv, n_comp, hd) * gc["v_ch_f16"].float().unsqueeze(1)
-        v_mid = hadamard(v_rot).view(B, nkv, n_comp, hd).half()
-        parts_k = [gc["sink_k"], k_mid, gc["win_k"]]
-        parts_v = [gc["sink_v"], v_mid, gc["win_v"]]
-        sk, sv = self._dequant_stream(gc)
-        if sk is not None:
-            parts_k.append(sk)
-            parts_v.append(sv)
-        if "decode_k" in gc:
-            parts_k.append(gc["decode_k"])
-            parts_v.append(gc["decode_v"])
-        self._keys = torch.cat(parts_k, dim=2)
-        self._values = torch.cat(parts_v, dim=2)
+        nkv, hd, n_comp = c._n_kv_heads, c.head_dim, gc["n_compress"]
+        dev = gc["k_coeffs"].device
+        _lib.require_cuda(gc["k_coeffs"])
+        pend = gc.pop("_pending", None)
+        n_stream = gc.get("stream_n", 0)
+        if pend is not None and pend[2] != n_stream - 1:
+            gc["_pending"] = pend
+            self._flush_pending()
+            pend = None
+        seq = _seq_record(gc, dev)
+        dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd)
+        n_sink, n_win = gc["sink_k"].shape[2], gc["win_k"].shape[2]
+        shape = ops.make_shape(4 * nkv, nkv, gc["k_rank_kernel"], n_comp, 0, n_comp, n_sink, n_win, n_stream, 0,
+                               append=pend is not None, n_dec=n_dec)
+        shape.dec_cap = dec_cap
+        if n_dec:
+            seq.dec_k, seq.dec_v = dk.data_ptr(), dv.data_ptr()
+        if pend is not None:
+            seq.new_k, seq.new_v = pend[0].data_ptr(), pend[1].data_ptr()
+        rows = n_sink + n_comp + n_win + n_stream + n_dec
+        keys = torch.empty(1, nkv, rows, hd, dtype=torch.float16, device=dev)
+        values = torch.empty_like(keys)
+        ws = c._decode_ws
+        if ws is None or ws.device != dev:
+            # zero-filled: the status word at its head (see `Cache.check`) must start at zero
+            ws = c._decode_ws = torch.zeros(1 << 20, dtype=torch.uint8, device=dev)
+        ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if n_stream else None,
+                      gc["compress_start"], keys, values, ws)
+        self._keys, self._values = keys, values
         self._needs_decompress = False
 
     @property
@@ -237,10 +236,9 @@ class CacheLayer(CacheLayerMixin):
 
         self._lazy_evict()
         if gc is not None and c._streaming:
-            for t in range(seq_new):
-                # with the fused decode the last token is quantised inside the decode launch
-                self._stream_append(key_states[:, :, t:t + 1, :], value_states[:, :, t:t + 1, :],
-                                    self._seq_len + t, defer=fused and t == seq_new - 1)
+            # one token is quantised by the launch that reads it next (fused decode or read-back),
+            # several by one launch here
+            self._stream_append(key_states, value_states, self._seq_len, defer=seq_new == 1)
             self._seq_len += seq_new
             self._needs_decompress = True
             if fused:
@@ -327,47 +325,23 @@ class CacheLayer(CacheLayerMixin):
             gc[f"{key}_buf"] = new
 
     def _stream_append(self, k, v, position, defer=False):
-        """Quantise one (1, nkv, 1, hd) token into the stream buffers
-        (reference: src/shard/cache.py:193-241).  With `defer` the row is reserved and the
-        token is handed to the next `decode_layer` call, whose kernel quantises it."""
+        """Quantise (1, nkv, s, hd) new tokens into the stream buffers
+        (reference: src/shard/cache.py:193-241).  With `defer` the row is reserved and the one
+        token is handed to the next launch that reads the stream, whose kernel quantises it."""
         self._flush_pending()
         gc = self._gpu_compressed
-        c = self._cache_ref
-        if c._stream_qjl:
-            raise NotImplementedError("the QJL residual is not part of the CUDA stream path")
-        if c._stream_bits != 8:
-            raise NotImplementedError("the CUDA stream quantizer emits 8-bit codes only")
-        B, heads, _, hd = k.shape
-        if B != 1:
-            raise NotImplementedError("one sequence per Cache (use one Cache per sequence)")
-        dev = k.device
+        new = k.shape[2]
         s = gc.get("stream_n", 0)
-        if "signs" not in gc or s >= gc["k_idx_buf"].shape[0]:
-            self._grow_stream(gc, k, s + 1)
-        k2 = k.reshape(heads, hd)
-        v2 = v.reshape(heads, hd)
-        if k2.dtype != torch.float16:
+        if "signs" not in gc or s + new > gc["k_idx_buf"].shape[0]:
+            self._grow_stream(gc, k, s + new)
+        if k.dtype != torch.float16 or v.dtype != torch.float16:
             raise NotImplementedError("fp16 models only")
         if defer:
-            gc["_pending"] = (k2.contiguous(), v2.contiguous(), s)
+            gc["_pending"] = (k.contiguous(), v.contiguous(), s)
         else:
-            ops.stream_quantize(k2.contiguous(), v2.contiguous(), gc["signs"], get_codebook(hd, 8, dev),
-                                gc["k_idx_buf"], gc["v_idx_buf"], gc["k_norm_buf"], gc["v_norm_buf"], s)
-        gc["stream_n"] = s + 1
-
-    def _dequant_stream(self, gc=None, *unused):
-        """fp16 (1, nkv, s, hd) K and V of the streamed tokens (reference: cache.py:243-279)."""
-        if gc is None or gc is self._gpu_compressed:
-            self._flush_pending()
-        gc = self._gpu_compressed if gc is None else gc
-        s = gc.get("stream_n", 0)
-        if s == 0 or "k_idx_buf" not in gc:
-            return None, None
-        dev = gc["k_idx_buf"].device
-        cb = get_codebook(self._cache_ref.head_dim, 8, dev)
-        sk = ops.stream_dequant(gc["k_idx_buf"][:s], gc["k_norm_buf"][:s], gc["signs"], cb)
-        sv = ops.stream_dequant(gc["v_idx_buf"][:s], gc["v_norm_buf"][:s], gc["signs"], cb)
-        return sk.unsqueeze(0), sv.unsqueeze(0)
+            ops.stream_quantize_rows(k[0], v[0], gc["signs"], get_codebook(k.shape[3], 8, k.device),
+                                     gc["k_idx_buf"], gc["v_idx_buf"], gc["k_norm_buf"], gc["v_norm_buf"], s)
+        gc["stream_n"] = s + new
 
     # -- HF glue -----------------------------------------------------------------
     def get_seq_length(self, *args, **kwargs):

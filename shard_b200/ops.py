@@ -42,6 +42,26 @@ def stream_quantize(new_k, new_v, signs, codebook, k_idx_buf, v_idx_buf, k_norm_
           "stream_quantize")
 
 
+def stream_quantize_rows(k, v, signs, codebook, k_idx_buf, v_idx_buf, k_norm_buf, v_norm_buf, slot):
+    """Append several tokens at once: k, v (nkv, s, 128) fp16 (any strides with contiguous channels) go
+    to rows slot .. slot + s - 1."""
+    require_cuda(k, v, signs, codebook, k_idx_buf)
+    nkv, s, _ = k.shape
+    if k.dtype != torch.float16 or v.dtype != torch.float16:
+        raise _lib.ShardError("expected torch.float16 keys and values")
+    if k.stride(2) != 1 or (k.stride(0) | k.stride(1)) & 3 or k.data_ptr() & 7:
+        k = k.contiguous()
+    if v.stride(2) != 1 or (v.stride(0) | v.stride(1)) & 3 or v.data_ptr() & 7:
+        v = v.contiguous()
+    if slot + s > k_idx_buf.shape[0]:
+        raise _lib.ShardError("stream buffer full")
+    check(_lib.load().shard_b200_stream_quantize_rows(
+        ptr(k), ptr(v), k.stride(0), k.stride(1), v.stride(0), v.stride(1), s, nkv, ptr(_c(signs, torch.float32)),
+        ptr(_c(codebook, torch.float32)), ptr(_c(k_idx_buf, torch.uint8)), ptr(_c(v_idx_buf, torch.uint8)),
+        ptr(_c(k_norm_buf, torch.float16)), ptr(_c(v_norm_buf, torch.float16)), slot, cur_stream()),
+        "stream_quantize_rows")
+
+
 def stream_dequant(idx, norm, signs, codebook):
     """(s, nkv, 128) u8 codes + (s, nkv) fp16 norms -> (nkv, s, 128) fp16."""
     require_cuda(idx, norm, signs, codebook)
@@ -51,6 +71,14 @@ def stream_dequant(idx, norm, signs, codebook):
                                                 ptr(_c(signs, torch.float32)), ptr(_c(codebook, torch.float32)),
                                                 s, nkv, ptr(out), cur_stream()), "stream_dequant")
     return out
+
+
+def read_back(seq, shape, inv_freq, codebook, compress_start, k_out, v_out, status=None):
+    """Compressed layer -> fp16 keys and values (nkv, rows, 128), rows [sink | middle | window | stream |
+    decode buffer].  `seq` / `shape` as for `decode_attn`; `status`: int32 device word (or None)."""
+    check(_lib.load().shard_b200_read_back(C.addressof(seq), C.byref(shape), ptr(inv_freq), ptr(codebook), int(compress_start),
+                                           ptr(_c(k_out, torch.float16)), ptr(_c(v_out, torch.float16)), ptr(status),
+                                           cur_stream()), "read_back")
 
 
 # --------------------------------------------------------------------------- prefill compressor

@@ -77,33 +77,24 @@ def hadamard(x):
     return x / math.sqrt(d)
 
 
-def kmeans(data, k, n_iter=30, seed=42, init=None):
-    """Lloyd's algorithm as the reference runs it (src/shard/cache.py:21-39).
+def initial_rows(n, k, device, seed=42):
+    """The rows `kmeans` starts from: the first k of a seeded permutation of n (src/shard/cache.py:24-25)."""
+    g = torch.Generator(device=device).manual_seed(seed)
+    return torch.randperm(n, generator=g, device=device)[:k]
 
-    Assignment and the per-centroid sums / counts come from one CUDA pass
-    (`vq_assign_accumulate`); the division and the stopping rule stay in PyTorch.  Returns the updated centroids and the assignment made against the
-    previous ones.  `init` overrides the seeded random initial centroids.
+
+def kmeans(data, k, n_iter=30, seed=42, init=None, max_abs=0.0):
+    """Lloyd's algorithm as the reference runs it (src/shard/cache.py:21-39), all iterations and the
+    stopping rule on the GPU (`ops.kmeans_lloyd`).  Returns the updated centroids and the assignment
+    made against the previous ones.  `init` overrides the seeded random initial centroids, `max_abs`
+    is a bound on |data| if the caller knows one.
     """
-    n = data.shape[0]
-    dev = data.device
     if init is None:
-        g = torch.Generator(device=dev).manual_seed(seed)
-        centroids = data[torch.randperm(n, generator=g, device=dev)[:k]].clone()
-    else:
-        centroids = init.to(dev, data.dtype).clone()
-    idx_u8 = None
-    sums = torch.zeros_like(centroids)
-    counts = torch.zeros(k, device=dev, dtype=data.dtype)
-    for it in range(n_iter):
-        # assignment and the sums / counts of the centroid update in one pass over the points
-        idx_u8 = ops.vq_assign_accumulate(data, centroids, sums, counts)
-        filled = counts > 0
-        new = centroids.clone()
-        new[filled] = sums[filled] / counts[filled].unsqueeze(1)
-        moved = (new - centroids).abs().max().item()
-        centroids = new
-        if moved < 1e-4 and it >= 5:
-            break
+        init = data[initial_rows(data.shape[0], k, data.device, seed)]
+    centroids = init.to(data.device, data.dtype).clone()
+    if n_iter < 1:
+        return centroids, None
+    idx_u8 = ops.kmeans_lloyd(data, centroids, n_iter, max_abs)
     return centroids, idx_u8
 
 
@@ -450,12 +441,15 @@ class Cache(HFCache):
         ev0 = torch.cuda.Event(enable_timing=True)
         ev1 = torch.cuda.Event(enable_timing=True)
         ev0.record()
+        # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
+        n_sub = (end - start) * self._n_kv_heads * (self.head_dim // self._v_vq_group_size)
+        init_rows = initial_rows(n_sub, self._v_vq_codebook_size, k0.device)
         for li in range(self._num_layers):
             torch.manual_seed(42 + li)
             layer = self.layers[li]
             k_full, v_full = layer._keys, layer._values
             kpart = self._compress_k(k_full[0, :, start:end, :], start)
-            vpart = self._compress_v(v_full[0, :, start:end, :])
+            vpart = self._compress_v(v_full[0, :, start:end, :], init_rows=init_rows)
             self._build_gpu_format(layer, kpart, vpart,
                                    sink_k=k_full[:, :, :sink, :].clone(), sink_v=v_full[:, :, :sink, :].clone(),
                                    win_k=k_full[:, :, end:, :].clone(), win_v=v_full[:, :, end:, :].clone(),
@@ -505,12 +499,15 @@ class Cache(HFCache):
         return {"k_basis_q": basis_q, "k_scale": scale.half(), "k_mean": mean.half(), "k_alloc": alloc,
                 "k_coeffs": packed, "k_coeff_scale": coeff_scale, "k_n_total": n}
 
-    def _compress_v(self, v_mid, init_centroids=None):
+    def _compress_v(self, v_mid, init_centroids=None, init_rows=None):
         """Hadamard-rotate, normalise per channel and vector-quantise 4-channel groups
         (reference: src/shard/cache.py:398-404, 41-52).  v_mid: (nkv, n, hd) fp16 view."""
         x, ch_max = ops.v_hadamard_normalise(v_mid)
         flat = x.view(-1, self._v_vq_group_size)
-        centroids, idx_u8 = kmeans(flat, self._v_vq_codebook_size, n_iter=30, init=init_centroids)
+        if init_centroids is None and init_rows is not None:
+            init_centroids = flat[init_rows]
+        # the data is normalised by the channels' largest magnitudes
+        centroids, idx_u8 = kmeans(flat, self._v_vq_codebook_size, n_iter=30, init=init_centroids, max_abs=1.0)
         nkv, n, hd = v_mid.shape
         return {"centroids": centroids.half(), "packed": idx_u8, "ch_maxabs": ch_max.half(),
                 "shape": (nkv, n, hd), "group_size": self._v_vq_group_size, "bits": 8,

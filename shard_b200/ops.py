@@ -179,6 +179,23 @@ def vq_assign_accumulate(x, centroids, sums, counts):
     return u8
 
 
+def kmeans_lloyd(x, centroids, n_iter, max_abs=0.0):
+    """`n_iter` Lloyd iterations over the rows of x (N, 4); `centroids` (256, 4) fp32 is updated in place.
+    Returns the u8 assignment of the last iteration (made against the centroids before it).
+    `max_abs`: a bound on |x|, 0 if not known."""
+    require_cuda(x, centroids)
+    n = x.shape[0]
+    if x.shape[1] != 4 or tuple(centroids.shape) != (256, 4):
+        raise _lib.ShardError("kmeans supports 4-dim sub-vectors and a 256-entry codebook")
+    lib = _lib.load()
+    wsb = lib.shard_b200_kmeans_workspace_bytes(n)
+    ws = torch.empty(wsb, dtype=torch.uint8, device=x.device)
+    u8 = torch.empty(n, dtype=torch.uint8, device=x.device)
+    check(lib.shard_b200_kmeans(ptr(_c(x, torch.float32)), n, float(max_abs), n_iter, ptr(_c(centroids, torch.float32)),
+                                ptr(u8), ptr(ws), wsb, cur_stream()), "kmeans")
+    return u8
+
+
 # --------------------------------------------------------------------------- decode
 def phase_table_numel(n):
     """fp16 elements of the phase table of `n` tokens (tokens are padded to blocks of 32)."""

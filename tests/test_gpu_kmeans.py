@@ -1,0 +1,55 @@
+"""The pruned k-means against the direct nearest-centroid kernel (bit-exact assignments) and a
+float64 mean of the assigned points, at tile edges, with ties, and for data of any scale."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(n, kind):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 4)).astype(np.float32) * 0.25
+    if kind == "ties":                                 # a coarse grid: many points exactly between centroids
+        x = np.round(x * 8) / 8
+    if kind == "large":
+        x *= 3000.0
+    if kind == "equal":
+        x[:] = x[0]
+    if kind == "narrow":                               # everything within a hundredth of the bound
+        x *= 0.01
+        x[0] = 1.0
+    return torch.from_numpy(x.astype(np.float32)).cuda()
+
+
+@pytest.mark.parametrize("n,kind", [(256, "plain"), (257, "ties"), (383, "plain"), (20000, "ties"), (300001, "plain"),
+                                    (300001, "large"), (1100001, "equal"), (64, "plain"), (1, "plain"), (100003, "narrow"), (6000000, "plain")])
+def test_kmeans_iterations(n, kind):
+    from shard_b200 import ops
+    x = _data(n, kind)
+    cent = x[torch.arange(256, device="cuda") * n // 256].clone()
+    if kind == "ties":
+        cent[100:110] = cent[5:15]                     # duplicates: the first of equals wins
+    for its in (1, 3):
+        before = cent.clone()
+        if its > 1:
+            ops.kmeans_lloyd(x, before, its - 1)
+        c = cent.clone()
+        idx = ops.kmeans_lloyd(x, c, its)
+        want, _ = ops.vq_assign(x, before, want_i64=False)
+        assert torch.equal(idx, want)
+        xi, ii = x.double().cpu().numpy(), idx.long().cpu().numpy()
+        counts = np.bincount(ii, minlength=256)
+        mean = np.stack([np.bincount(ii, xi[:, k], 256) for k in range(4)], 1) / np.maximum(counts, 1)[:, None]
+        mean[counts == 0] = before.double().cpu().numpy()[counts == 0]
+        assert np.abs(c.double().cpu().numpy() - mean).max() <= 2e-7 * float(x.abs().max())
+        c2 = cent.clone()
+        assert torch.equal(ops.kmeans_lloyd(x, c2, its), idx) and torch.equal(c2, c)
+
+
+def test_kmeans_stops_when_settled():
+    from shard_b200 import ops
+    x = _data(256, "plain").repeat(8, 1)
+    c = x[:256].clone()
+    idx = ops.kmeans_lloyd(x, c, 30)
+    assert (c - x[:256]).abs().max() < 2e-9 and torch.equal(idx, ops.vq_assign(x, c, want_i64=False)[0])

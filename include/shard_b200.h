@@ -399,6 +399,20 @@ size_t shard_b200_kmeans_workspace_bytes(int64_t n);
 int shard_b200_kmeans(const float* x, int64_t n, float max_abs, int32_t n_iter, float* centroids,
                       uint8_t* idx_u8, void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * The `rank` largest eigenpairs of `count` symmetric matrices a [count][p][p] (fp32, p a multiple of 128,
+ * 128..1024), side by side: the factorisation behind the PCA fit of Cache._compress_k
+ * (src/shard/cache.py:376, a randomised SVD there).  basis_out [count][p][rank]: unit eigenvectors in the
+ * columns, largest eigenvalue first; eigvals_out [count][rank].  flag_out [count]: 0, or 1 where the
+ * vectors are not orthogonal (eigenvalues equal to working precision, or a matrix that is not finite) or a
+ * bounded wait gave up: use another eigensolver for that matrix.  a and workspace 16-byte aligned;
+ * workspace: shard_b200_eigh_workspace_bytes bytes (0: sizes not supported).
+ */
+size_t shard_b200_eigh_workspace_bytes(int32_t count, int32_t p, int32_t rank);
+int shard_b200_eigh(const float* a, int32_t count, int32_t p, int32_t rank, float* basis_out,
+                    float* eigvals_out, int32_t* flag_out, void* workspace, size_t workspace_bytes,
+                    void* stream);
+
 #ifdef __cplusplus
 }
 #endif

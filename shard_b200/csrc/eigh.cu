@@ -1,0 +1,643 @@
+// Leading eigenpairs of small symmetric matrices (the p x p Gram matrices of the PCA fit, p = 128 ..
+// 1024), several matrices side by side.
+//
+//   1. tridiag_kernel      Householder reduction to tridiagonal form, one cluster of 16 CTAs per matrix.
+//                          The whole matrix stays on chip: row r lives in CTA r % 16, in TENSOR MEMORY
+//                          (64 rows x 1024 columns of fp32 are exactly its 256 KB), which its 16 warps
+//                          read and write as a register file: thread = 8 matrix columns, for which the
+//                          three vectors of a step stay in registers.  One exchange per step: every CTA
+//                          sends its rows of A v and of the next column to all others with st.async
+//                          (distributed shared memory, completion counted on the receivers' mbarriers);
+//                          everything else of a step is recomputed by every CTA from the same numbers.
+//   2. tridiag_values_kernel   eigenvalues by 33-section on Sturm counts, a warp per eigenvalue, fp64;
+//                          division-free recurrence (one multiply-add of latency per row).
+//   3. tridiag_vectors_kernel  eigenvectors of the tridiagonal matrix by twisted factorisation, fp64,
+//                          thread = vector, one warp from either end.
+//   4. eig_back_kernel     the reflectors applied to the vectors, a warp per vector, two reflectors per
+//                          pass over its registers.
+//   5. eig_check_kernel    neighbouring vectors must be orthogonal; a matrix with eigenvalues too close
+//                          for step 3 is reported to the caller.
+//
+// Bound: the latency chain of step 1 (p steps of exchange, two reductions and one pass over the matrix).
+#include <atomic>
+
+#include "tcgen05.cuh"
+
+namespace shard {
+
+constexpr int EG_CL = 16;                  // CTAs of a cluster
+constexpr int EG_THREADS = 512;
+constexpr int EG_MAX_P = 1024;
+
+struct EighParams {
+  const float* a;         // [L][p][p]
+  int p, rank;
+  float* refl;            // [L][p][p] reflector k in row k (zeros up to k, one at k + 1)
+  float* tau;             // [L][p]
+  float* d;               // [L][p]
+  float* e;               // [L][p]
+  double* lam;            // [L][rank] eigenvalues, descending
+  double* dplus;          // [L][blocks of 32 vectors][p][32]
+  double* dminus;
+  float* z;               // [L][blocks][p][32] vectors of the tridiagonal matrix
+  float* basis;           // [L][p][rank]
+  float* eigvals;         // [L][rank]
+  int* flag;              // [L] 1: vectors not orthogonal, or a wait gave up
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t cta) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void st_async_f2(uint32_t addr, float a, float b, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
+               ::"r"(addr), "f"(a), "f"(b), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void st_async_f1(uint32_t addr, float a, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
+               ::"r"(addr), "f"(a), "r"(bar) : "memory");
+}
+
+// A row's CB columns of this thread, tensor memory <-> registers.
+template <int CB>
+__device__ __forceinline__ void eg_ld(uint32_t t, uint32_t (&u)[CB]) {
+  if constexpr (CB == 8) tmem_ld_x8(t, u);
+  else if constexpr (CB == 4) tmem_ld_x4(t, u);
+  else
+#pragma unroll
+    for (int j = 0; j < CB; ++j) asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(u[j]) : "r"(t + j));
+}
+template <int CB>
+__device__ __forceinline__ void eg_st(uint32_t t, const uint32_t (&u)[CB]) {
+  if constexpr (CB == 8) tmem_st_x8(t, u);
+  else if constexpr (CB == 4) tmem_st_x4(t, u);
+  else
+#pragma unroll
+    for (int j = 0; j < CB; ++j) asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t + j), "r"(u[j]) : "memory");
+}
+// barrier of one 128-thread group, ORing a flag over it
+__device__ __forceinline__ bool eg_bar_or(int id, bool flag) {
+  uint32_t out;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %2, 0;\n\tbar.red.or.pred p, %1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(out) : "r"(id), "r"((uint32_t)flag) : "memory");
+  return out != 0;
+}
+
+// CB = p / 128 columns per thread; a CTA has RL = p / 16 rows, 4 row groups of RS = p / 64 rows each
+// (RP: RS rounded up to a power of two).
+template <int CB>
+__global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_constant__ EighParams p) {
+  constexpr int N = CB * 128, RS = CB * 2, RP = RS > 8 ? 16 : RS > 4 ? 8 : RS > 2 ? 4 : 2, LOG = RP == 16 ? 4 : RP == 8 ? 3 : RP == 4 ? 2 : 1;
+  __shared__ float2 mail[2][N];              // (A v)[r] and next column [r], from every CTA
+  __shared__ float mail_g[2][64];            // parts of v . A v
+  __shared__ float part[4][4][RP];           // row group, quarter of the columns
+  __shared__ float acol[4][RS];              // next column, own rows
+  __shared__ float vrow[2][4][RS];           // v of the own rows (this step's and the last one's)
+  __shared__ float red[4][8];
+  __shared__ float2 out[4][RS];
+  __shared__ uint64_t bars[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_w;
+  volatile int* abort_s = &abort_w;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, rg = warp >> 2;
+  const int m = blockIdx.x / EG_CL;
+  const uint32_t rank = cluster_rank();
+  const float* A = p.a + (size_t)m * N * N;
+
+  if (warp == 0) {
+    tmem_alloc(smem_u32(&tmem_slot), 512);
+    tmem_relinquish();
+    if (lane == 0) {
+      mbar_init(smem_u32(&bars[0]), 1);
+      mbar_init(smem_u32(&bars[1]), 1);
+      *abort_s = 0;
+      fence_mbar_init();
+    }
+  }
+  constexpr uint32_t TX = N * 8 + 64 * 4;    // bytes a CTA receives per step
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (tid == 0) { mbar_expect_tx(smem_u32(&bars[0]), TX); mbar_expect_tx(smem_u32(&bars[1]), TX); }
+  const uint32_t T = tmem_slot + ((uint32_t)(q * 32) << 16);
+  const int c0 = 32 * q + lane;              // own columns c0 + 128 j
+  // local row i = 4 s + rg (s < RS) is matrix row 16 i + rank, at tensor-memory columns CB * i
+#pragma unroll 4
+  for (int s = 0; s < RS; ++s) {
+    const int i = 4 * s + rg;
+    const float* row = A + (size_t)(16 * i + rank) * N + c0;
+    uint32_t v[CB];
+#pragma unroll
+    for (int j = 0; j < CB; ++j) v[j] = __float_as_uint(row[128 * j]);
+    eg_st<CB>(T + CB * i, v);
+    if (c0 == 0) acol[rg][s] = __uint_as_float(v[0]);           // column 0
+  }
+  tmem_wait_st();
+  if (tid < 4 * RS) vrow[0][tid / RS][tid % RS] = vrow[1][tid / RS][tid % RS] = 0.f;
+  __syncthreads();
+  cluster_sync();                            // every CTA's barriers are armed
+  auto send = [&](int b, float g_part) {
+    // the row group's (A v, next column) pairs to all 16 CTAs; 128 threads: CTA t / 8, rows t % 8, ...
+    const int t = tid & 127, dst = t >> 3;
+    const uint32_t rbar = map_to_cta(smem_u32(&bars[b]), dst);
+    const uint32_t base = map_to_cta(smem_u32(&mail[b][0]), dst);
+#pragma unroll
+    for (int s = t & 7; s < RS; s += 8) {
+      const float2 o = out[rg][s];
+      st_async_f2(base + 8u * (uint32_t)(16 * (4 * s + rg) + rank), o.x, o.y, rbar);
+    }
+    if ((t & 7) == 0) st_async_f1(map_to_cta(smem_u32(&mail_g[b][0]), dst) + 4u * (uint32_t)(4 * rank + rg), g_part, rbar);
+  };
+  if ((tid & 127) < RS) out[rg][tid & 127] = make_float2(0.f, acol[rg][tid & 127]);
+  named_bar_sync_128(1 + rg);
+  send(0, 0.f);
+
+  float v[CB], w[CB], vn[CB];
+#pragma unroll
+  for (int j = 0; j < CB; ++j) v[j] = 0.f;
+  for (int k = 0; k < N; ++k) {              // column k: its reflector, then the matrix updated with the last one
+    const int b = k & 1;
+    mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
+    if (tid == 0) mbar_expect_tx(smem_u32(&bars[b]), TX);
+    // gamma = tau / 2 v . p with p = tau A v: the same sum, in the same order, everywhere
+    float gam = mail_g[b][lane] + mail_g[b][lane + 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gam += __shfl_xor_sync(0xffffffffu, gam, o);
+    const float2 mk = mail[b][k];
+    const float w1 = mk.x - gam;                                // w[k]; v[k] = 1 (no v yet at k = 0: all zero)
+    float x[CB], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < CB; ++j) {
+      const int c = c0 + 128 * j;
+      const float2 pa = mail[b][c];
+      w[j] = fmaf(-gam, v[j], pa.x);
+      x[j] = pa.y - fmaf(v[j], w1, w[j]);
+      if (c <= k) x[j] = 0.f;
+      if (c == k + 1) red[rg][4] = x[j];
+      else ss = fmaf(x[j], x[j], ss);
+      if (c < k) w[j] = 0.f;
+    }
+    // row scalars of the update
+    float vr = 0.f, wr = 0.f;
+    if (lane < RS) {
+      vr = vrow[b ^ 1][rg][lane];
+      wr = fmaf(-gam, vr, mail[b][16 * (4 * lane + rg) + rank].x);
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) red[rg][q] = ss;
+    named_bar_sync_128(1 + rg);
+    const float x0 = k + 1 < N ? red[rg][4] : 0.f;
+    ss = (red[rg][0] + red[rg][1]) + (red[rg][2] + red[rg][3]);
+    float beta = x0, tau = 0.f, scale = 0.f;
+    if (ss > 0.f) {
+      beta = -copysignf(sqrtf(fmaf(x0, x0, ss)), x0);
+      tau = (beta - x0) / beta;
+      scale = 1.f / (x0 - beta);
+    }
+#pragma unroll
+    for (int j = 0; j < CB; ++j) {
+      const int c = c0 + 128 * j;
+      vn[j] = c == k + 1 ? 1.f : x[j] * scale;                  // (x is zero up to row k)
+      // own rows: the thread whose column is one of them leaves v there
+      if ((c & 15) == (int)rank && ((c >> 4) & 3) == rg) vrow[b][rg][c >> 6] = vn[j];
+    }
+    if ((k & 15) == (int)rank && rg == 0) {
+      float* o = p.refl + ((size_t)m * N + k) * N + c0;
+#pragma unroll
+      for (int j = 0; j < CB; ++j) o[128 * j] = vn[j];
+      if (tid == 0) {
+        p.d[m * N + k] = mk.y - 2.f * w1;
+        p.e[m * N + k] = beta;
+        p.tau[m * N + k] = tau;
+      }
+    }
+    if (k == N - 1) break;
+    // ---- own rows: A -= v w' + w v', then A vn and the next column -------------------------------
+    float dot[RP];
+    const bool has_col = q == (((k + 1) >> 5) & 3);
+    const int jc = (k + 1) >> 7;
+#pragma unroll
+    for (int s = 0; s < RP; ++s) dot[s] = 0.f;
+#pragma unroll
+    for (int s0 = 0; s0 < RS; s0 += 4) {
+      constexpr int B = RS < 4 ? RS : 4;
+      const int top = s0 + 3 < RS ? s0 + 3 : RS - 1;
+      if (16 * (4 * top + rg) + (int)rank > k) {                 // (uniform over the warp) a row of the four is still active
+        uint32_t u[B][CB];
+#pragma unroll
+        for (int s = 0; s < B; ++s)
+          if (s0 + s < RS) eg_ld<CB>(T + CB * (4 * (s0 + s) + rg), u[s]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int s = 0; s < B; ++s) {
+          if (s0 + s < RS) {
+            const float vs = __shfl_sync(0xffffffffu, vr, s0 + s), ws = __shfl_sync(0xffffffffu, wr, s0 + s);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < CB; ++j) {
+              const float a = fmaf(-ws, v[j], fmaf(-vs, w[j], __uint_as_float(u[s][j])));
+              sum = fmaf(a, vn[j], sum);
+              u[s][j] = __float_as_uint(a);
+            }
+            eg_st<CB>(T + CB * (4 * (s0 + s) + rg), u[s]);
+            dot[s0 + s] = sum;
+            if (has_col) {
+              uint32_t sel = u[s][0];
+              switch (jc) {
+                case 1: if (CB > 1) sel = u[s][1 < CB ? 1 : 0]; break;
+                case 2: if (CB > 2) sel = u[s][2 < CB ? 2 : 0]; break;
+                case 3: if (CB > 3) sel = u[s][3 < CB ? 3 : 0]; break;
+                case 4: if (CB > 4) sel = u[s][4 < CB ? 4 : 0]; break;
+                case 5: if (CB > 5) sel = u[s][5 < CB ? 5 : 0]; break;
+                case 6: if (CB > 6) sel = u[s][6 < CB ? 6 : 0]; break;
+                case 7: if (CB > 7) sel = u[s][7 < CB ? 7 : 0]; break;
+              }
+              if (lane == ((k + 1) & 31)) acol[rg][s0 + s] = __uint_as_float(sel);
+            }
+          }
+        }
+      }
+    }
+    tmem_wait_st();
+    // sums over the lanes, all rows at once: halve the rows a lane carries, fold the lanes
+    {
+      int off = 16;
+#pragma unroll
+      for (int h = RP / 2; h >= 1; h >>= 1) {
+        const bool up = (lane & off) != 0;
+#pragma unroll
+        for (int s = 0; s < h; ++s) {
+          const float keep = up ? dot[s + h] : dot[s], give = up ? dot[s] : dot[s + h];
+          dot[s] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+        off >>= 1;
+      }
+      for (; off >= 1; off >>= 1) dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], off);
+      // lane bits from the top select the row: bit 4 -> row bit log2(RS) - 1, ...
+      if ((lane & ((32 >> LOG) - 1)) == 0) part[rg][q][lane >> (5 - LOG)] = dot[0];
+    }
+    named_bar_sync_128(1 + rg);
+    float g = 0.f;
+    {
+      // every warp of the row group finishes all RS rows (and keeps the same g); its first warp stores
+      float pr = 0.f, ac = 0.f, vnr = 0.f;
+      if (lane < RS) {
+        if (16 * (4 * lane + rg) + (int)rank > k)
+          pr = tau * ((part[rg][0][lane] + part[rg][1][lane]) + (part[rg][2][lane] + part[rg][3][lane]));
+        ac = acol[rg][lane];
+        vnr = vrow[b][rg][lane];
+        if (q == 0) out[rg][lane] = make_float2(pr, ac);
+      }
+      g = 0.5f * tau * warp_sum(vnr * pr);
+    }
+    if (eg_bar_or(1 + rg, *abort_s != 0)) break;                 // (uniform over the row group)
+    send(b ^ 1, g);
+#pragma unroll
+    for (int j = 0; j < CB; ++j) v[j] = vn[j];
+  }
+  if (tid == 0 && *abort_s) atomicExch(p.flag + m, 1);
+  tc_fence_before();
+  cluster_sync();                            // nobody is still sending to a CTA that leaves
+  if (warp == 0) tmem_dealloc(tmem_slot, 512);
+}
+
+// ---------------------------------------------------------------------------
+// eigenvalues of the tridiagonal matrix
+// ---------------------------------------------------------------------------
+// The matrix in fp64, scaled to eigenvalues within [-1, 1] (Gershgorin): td[i] = (d_i, e_i^2).
+// Returns the scale.
+__device__ __forceinline__ double eg_load(const EighParams& p, int m, double2* td, int tid, int threads) {
+  __shared__ float mx[32];
+  const int n = p.p;
+  const float *d = p.d + (size_t)m * n, *e = p.e + (size_t)m * n;
+  float g = 0.f;
+  for (int i = tid; i < n; i += threads)
+    g = fmaxf(g, fabsf(d[i]) + (i ? fabsf(e[i - 1]) : 0.f) + (i + 1 < n ? fabsf(e[i]) : 0.f));
+  g = warp_max(g);
+  if ((tid & 31) == 0) mx[tid >> 5] = g;
+  __syncthreads();
+  for (int i = 0; i < threads / 32; ++i) g = fmaxf(g, mx[i]);
+  const double s = g > 0.f ? 1.0 / (1.0001 * (double)g) : 1.0;
+  for (int i = tid; i < n; i += threads) {
+    const double ei = i + 1 < n ? (double)e[i] * s : 0.0;
+    td[i] = make_double2((double)d[i] * s, ei * ei > 1e-40 ? ei * ei : 1e-40);   // (never zero: the recurrence goes on)
+  }
+  __syncthreads();
+  return 1.0 / s;
+}
+// keeps (a, b), consecutive terms of the recurrence, away from overflow and underflow
+__device__ __forceinline__ void eg_rescale(double& a, double& b) {
+  const int ex = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
+  const double f = __hiloint2double(0x7fe00000 - max(ex, 0x00100000), 0);
+  a *= f;
+  b *= f;
+}
+
+// warp = eigenvalue number w (descending); 32 trial points split its interval into 33 per round
+__global__ void __launch_bounds__(256) tridiag_values_kernel(const __grid_constant__ EighParams p) {
+  __shared__ double2 td[EG_MAX_P];
+  const int m = blockIdx.y, n = p.p, lane = threadIdx.x & 31;
+  const double unscale = eg_load(p, m, td, threadIdx.x, 256);
+  const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (w >= p.rank) return;
+  double lo = -1.0, width = 2.0;
+  for (int round = 0; round < 11; ++round) {            // 33^-11: below fp64's resolution of the interval
+    const double step = width / 33.0, x = lo + step * (lane + 1);
+    double b = 1.0, a = td[0].x - x;                    // p_{i-1}, p_i
+    int neg = __double2hiint(a) < 0;
+    int i = 1;
+    for (; i + 8 <= n; i += 8) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const double c = fma(td[i + j].x - x, a, -td[i + j - 1].y * b);
+        neg += (unsigned)(__double2hiint(c) ^ __double2hiint(a)) >> 31;
+        b = a;
+        a = c;
+      }
+      eg_rescale(a, b);
+    }
+    for (; i < n; ++i) {
+      const double c = fma(td[i].x - x, a, -td[i - 1].y * b);
+      neg += (unsigned)(__double2hiint(c) ^ __double2hiint(a)) >> 31;
+      b = a;
+      a = c;
+    }
+    // neg eigenvalues lie below x; the one sought has n - 1 - w below it
+    const unsigned int left = __ballot_sync(0xffffffffu, neg <= n - 1 - w);
+    const int k = __popc(left);                         // it lies right of the first k points
+    lo += step * k;
+    width = step;
+  }
+  if (lane == 0) {
+    const double l = lo + 0.5 * width;
+    p.lam[(size_t)m * p.rank + w] = l;                  // of the scaled matrix
+    p.eigvals[(size_t)m * p.rank + w] = (float)(l * unscale);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// eigenvectors of the tridiagonal matrix: T - lambda = L D+ L' = U D- U'; the vector is built from the
+// row where the two factorisations meet best, z_r = 1, z_i = -(e_i / D+_i) z_{i+1} above it and
+// z_i = -(e_{i-1} / D-_i) z_{i-1} below
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_constant__ EighParams p) {
+  __shared__ double2 td[EG_MAX_P];
+  __shared__ double gmin[2][32];
+  __shared__ int gat[2][32];
+  const int m = blockIdx.y, n = p.p, lane = threadIdx.x & 31, side = threadIdx.x >> 5;
+  eg_load(p, m, td, threadIdx.x, 64);
+  const int w = blockIdx.x * 32 + lane;
+  const double lam = p.lam[(size_t)m * p.rank + min(w, p.rank - 1)];
+  const size_t base = ((size_t)m * gridDim.x + blockIdx.x) * n * 32 + lane;
+  double* dp = p.dplus + base;
+  double* dm = p.dminus + base;
+  {
+    // D_i = p_i / p_{i-1}: the recurrence carries the numerators, the divisions hang off it
+    double* out = side ? dm : dp;
+    double b = 1.0, a = 0.0;
+    int i = 0;
+    auto step = [&](int r) {                            // r: row, from this side
+      const int row = side ? n - 1 - r : r;
+      const double off = r ? (side ? td[row].y : td[row - 1].y) : 0.0;
+      const double c = r ? fma(td[row].x - lam, a, -off * b) : td[row].x - lam;
+      if (r) b = a;
+      a = c;
+      double q = a / b;
+      if (q == 0.0) q = 1e-30;
+      out[(size_t)row * 32] = q;
+    };
+    for (; i + 8 <= n; i += 8) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) step(i + j);
+      eg_rescale(a, b);
+    }
+    for (; i < n; ++i) step(i);
+  }
+  __syncthreads();
+  {
+    double best = 1e300;
+    int at = 0;
+    const int lo = side ? n / 2 : 0, hi = side ? n : n / 2;
+#pragma unroll 4
+    for (int i = lo; i < hi; ++i) {
+      const double g = fabs(dp[(size_t)i * 32] + dm[(size_t)i * 32] - (td[i].x - lam));
+      if (g < best) { best = g; at = i; }
+    }
+    gmin[side][lane] = best;
+    gat[side][lane] = at;
+  }
+  __syncthreads();
+  const int r = gmin[1][lane] < gmin[0][lane] ? gat[1][lane] : gat[0][lane];
+  float* z = p.z + base;
+  // signs of e are needed here, and its scale cancels: sqrt(e_i^2) carries the sign of e_i
+  const float* e = p.e + (size_t)m * n;
+  double v = 1.0;
+  if (side == 0) {
+    z[(size_t)r * 32] = 1.f;
+#pragma unroll 4
+    for (int i = n - 2; i >= 0; --i) {
+      const double f = -copysign(sqrt(td[i].y), (double)e[i]) / dp[(size_t)i * 32];
+      if (i < r) { v *= f; z[(size_t)i * 32] = (float)v; }
+    }
+  } else {
+#pragma unroll 4
+    for (int i = 1; i < n; ++i) {
+      const double f = -copysign(sqrt(td[i - 1].y), (double)e[i - 1]) / dm[(size_t)i * 32];
+      if (i > r) { v *= f; z[(size_t)i * 32] = (float)v; }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// back to the matrix's own coordinates: x = H_0 H_1 ... H_{n-3} z, a warp per vector
+// ---------------------------------------------------------------------------
+// CB chunks of 128 rows; lane owns rows 128 j + 4 lane .. + 3.  Two reflectors per pass: with
+// x' = x - t1 v1 (v1.x), v2.x' = v2.x - t1 (v1.x)(v2.v1), so the three sums go through one set of shuffles.
+template <int CB>
+__global__ void __launch_bounds__(128) eig_back_kernel(const __grid_constant__ EighParams p) {
+  constexpr int N = CB * 128;
+  const int m = blockIdx.y, lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (w >= p.rank) return;
+  const int n_blocks = (p.rank + 31) / 32;
+  const float* z = p.z + ((size_t)m * n_blocks + (w >> 5)) * N * 32 + (w & 31);
+  float x[CB][4];
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < CB; ++j)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      x[j][t] = z[(size_t)(128 * j + 4 * lane + t) * 32];
+      ss = fmaf(x[j][t], x[j][t], ss);
+    }
+  const float inv = rsqrtf(warp_sum(ss));
+#pragma unroll
+  for (int j = 0; j < CB; ++j)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) x[j][t] *= inv;
+  const float* refl = p.refl + (size_t)m * N * N + 4 * lane;
+  const float* tau = p.tau + (size_t)m * N;
+  float4 a[CB], b[CB];
+  auto load = [&](int k, float4 (&r)[CB]) {
+#pragma unroll
+    for (int j = 0; j < CB; ++j)
+      r[j] = (k >= 0 && 128 * (j + 1) > k + 1) ? *reinterpret_cast<const float4*>(refl + (size_t)k * N + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  // the first pair is (n - 2, n - 3): reflector n - 2 is trivial (tau = 0)
+  load(N - 2, a);
+  load(N - 3, b);
+#pragma unroll 1
+  for (int k = N - 2; k >= 0; k -= 2) {
+    const float t1 = __ldg(tau + k), t2 = k >= 1 ? __ldg(tau + k - 1) : 0.f;
+    float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+    for (int j = 0; j < CB; ++j) {
+      s1 = fmaf(a[j].x, x[j][0], fmaf(a[j].y, x[j][1], fmaf(a[j].z, x[j][2], fmaf(a[j].w, x[j][3], s1))));
+      s2 = fmaf(b[j].x, x[j][0], fmaf(b[j].y, x[j][1], fmaf(b[j].z, x[j][2], fmaf(b[j].w, x[j][3], s2))));
+      s3 = fmaf(b[j].x, a[j].x, fmaf(b[j].y, a[j].y, fmaf(b[j].z, a[j].z, fmaf(b[j].w, a[j].w, s3))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+    }
+    s1 *= t1;
+    s2 = t2 * fmaf(-s1, s3, s2);
+#pragma unroll
+    for (int j = 0; j < CB; ++j) {
+      x[j][0] = fmaf(-s2, b[j].x, fmaf(-s1, a[j].x, x[j][0]));
+      x[j][1] = fmaf(-s2, b[j].y, fmaf(-s1, a[j].y, x[j][1]));
+      x[j][2] = fmaf(-s2, b[j].z, fmaf(-s1, a[j].z, x[j][2]));
+      x[j][3] = fmaf(-s2, b[j].w, fmaf(-s1, a[j].w, x[j][3]));
+    }
+    load(k - 2, a);
+    load(k - 3, b);
+  }
+  float* out = p.basis + (size_t)m * N * p.rank + w;
+#pragma unroll
+  for (int j = 0; j < CB; ++j)
+#pragma unroll
+    for (int t = 0; t < 4; ++t) out[(size_t)(128 * j + 4 * lane + t) * p.rank] = x[j][t];
+}
+
+// Vectors of close eigenvalues that step 3 could not tell apart: the next two neighbours of every vector
+// must be orthogonal to it, and its length one.
+__global__ void __launch_bounds__(256) eig_check_kernel(const __grid_constant__ EighParams p) {
+  const int m = blockIdx.y, w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (w >= p.rank) return;
+  const float* v = p.basis + (size_t)m * p.p * p.rank;
+  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+  for (int i = lane; i < p.p; i += 32) {
+    const float* row = v + (size_t)i * p.rank;
+    const float a = row[w];
+    s0 = fmaf(a, a, s0);
+    s1 = fmaf(a, w + 1 < p.rank ? row[w + 1] : 0.f, s1);
+    s2 = fmaf(a, w + 2 < p.rank ? row[w + 2] : 0.f, s2);
+  }
+  s0 = warp_sum(s0);
+  s1 = warp_sum(s1);
+  s2 = warp_sum(s2);
+  if (lane == 0 && !(fabsf(s0 - 1.f) < 1e-3f && fabsf(s1) < 1e-3f && fabsf(s2) < 1e-3f)) p.flag[m] = 1;   // (NaN: flagged)
+}
+
+template <int CB>
+static int launch_eigh(const EighParams& p, int count, cudaStream_t st) {
+  static std::atomic<bool> configured[MAX_DEVICES];
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev < 0 || dev >= MAX_DEVICES) return SHARD_E_ARG;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(tridiag_kernel<CB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(EG_CL * count);
+  cfg.blockDim = dim3(EG_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = EG_CL;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, tridiag_kernel<CB>, p);
+  if (e != cudaSuccess) return (int)e;
+  tridiag_values_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);
+  tridiag_vectors_kernel<<<dim3((p.rank + 31) / 32, count), 64, 0, st>>>(p);
+  eig_back_kernel<CB><<<dim3((p.rank + 3) / 4, count), 128, 0, st>>>(p);
+  eig_check_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : (int)e;
+}
+
+struct EighLayout { size_t refl, tau, d, e, lam, dplus, dminus, z, bytes; };
+static EighLayout eg_layout(size_t L, size_t p, size_t rank) {
+  EighLayout l;
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t nb = (rank + 31) / 32 * 32;
+  l.refl = 0;
+  l.tau = l.refl + up(L * p * p * 4);
+  l.d = l.tau + up(L * p * 4);
+  l.e = l.d + up(L * p * 4);
+  l.lam = l.e + up(L * p * 4);
+  l.dplus = l.lam + up(L * rank * 8);
+  l.dminus = l.dplus + up(L * nb * p * 8);
+  l.z = l.dminus + up(L * nb * p * 8);
+  l.bytes = l.z + up(L * nb * p * 4);
+  return l;
+}
+
+}  // namespace shard
+
+using namespace shard;
+
+extern "C" size_t shard_b200_eigh_workspace_bytes(int32_t count, int32_t p, int32_t rank) {
+  if (count < 1 || p < 128 || p > EG_MAX_P || (p % 128) || rank < 1 || rank > p) return 0;
+  return eg_layout(count, p, rank).bytes;
+}
+
+extern "C" int shard_b200_eigh(const float* a, int32_t count, int32_t p, int32_t rank, float* basis_out, float* eigvals_out,
+                               int32_t* flag_out, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!a || !basis_out || !eigvals_out || !flag_out || !workspace) return SHARD_E_ARG;
+  const size_t need = shard_b200_eigh_workspace_bytes(count, p, rank);
+  if (need == 0) return SHARD_E_ARG;
+  if (workspace_bytes < need) return SHARD_E_WORKSPACE;
+  if (((uintptr_t)a | (uintptr_t)workspace) & 15) return SHARD_E_ALIGN;
+  const EighLayout l = eg_layout(count, p, rank);
+  unsigned char* ws = (unsigned char*)workspace;
+  EighParams q{};
+  q.a = a;
+  q.p = p;
+  q.rank = rank;
+  q.refl = (float*)(ws + l.refl);
+  q.tau = (float*)(ws + l.tau);
+  q.d = (float*)(ws + l.d);
+  q.e = (float*)(ws + l.e);
+  q.lam = (double*)(ws + l.lam);
+  q.dplus = (double*)(ws + l.dplus);
+  q.dminus = (double*)(ws + l.dminus);
+  q.z = (float*)(ws + l.z);
+  q.basis = basis_out;
+  q.eigvals = eigvals_out;
+  q.flag = flag_out;
+  cudaStream_t st = (cudaStream_t)stream;
+  cudaError_t e = cudaMemsetAsync(flag_out, 0, (size_t)count * 4, st);
+  if (e != cudaSuccess) return (int)e;
+  switch (p / 128) {
+    case 1: return launch_eigh<1>(q, count, st);
+    case 2: return launch_eigh<2>(q, count, st);
+    case 3: return launch_eigh<3>(q, count, st);
+    case 4: return launch_eigh<4>(q, count, st);
+    case 5: return launch_eigh<5>(q, count, st);
+    case 6: return launch_eigh<6>(q, count, st);
+    case 7: return launch_eigh<7>(q, count, st);
+    default: return launch_eigh<8>(q, count, st);
+  }
+}

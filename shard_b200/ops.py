@@ -179,6 +179,25 @@ def vq_assign_accumulate(x, centroids, sums, counts):
     return u8
 
 
+def eigh_top(a, rank):
+    """The `rank` largest eigenpairs of the symmetric matrices a (count, p, p) fp32: (basis (count, p,
+    rank) with the eigenvectors in its columns, largest first, eigenvalues (count, rank), flag (count,)
+    int32: 1 where the result must not be used)."""
+    require_cuda(a)
+    count, p, _ = a.shape
+    lib = _lib.load()
+    wsb = lib.shard_b200_eigh_workspace_bytes(count, p, rank)
+    if wsb == 0:
+        raise _lib.ShardError(f"eigh_top supports p % 128 == 0, 128 <= p <= 1024, rank <= p (got {p}, {rank})")
+    ws = torch.empty(wsb, dtype=torch.uint8, device=a.device)
+    basis = torch.empty(count, p, rank, dtype=torch.float32, device=a.device)
+    eigvals = torch.empty(count, rank, dtype=torch.float32, device=a.device)
+    flag = torch.empty(count, dtype=torch.int32, device=a.device)
+    check(lib.shard_b200_eigh(ptr(_c(a, torch.float32)), count, p, rank, ptr(basis), ptr(eigvals), ptr(flag), ptr(ws), wsb,
+                              cur_stream()), "eigh")
+    return basis, eigvals, flag
+
+
 def kmeans_lloyd(x, centroids, n_iter, max_abs=0.0):
     """`n_iter` Lloyd iterations over the rows of x (N, 4); `centroids` (256, 4) fp32 is updated in place.
     Returns the u8 assignment of the last iteration (made against the centroids before it).

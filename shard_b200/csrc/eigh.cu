@@ -3,7 +3,7 @@
 //
 //   1. tridiag_kernel      Householder reduction to tridiagonal form, one cluster of 16 CTAs per matrix.
 //                          The whole matrix stays on chip: row r lives in CTA r % 16, in TENSOR MEMORY
-//                          (64 rows x 1024 columns of fp32 are exactly its 256 KB), which its 16 warps
+//                          (64 rows x 1024 columns of fp32 are exactly its 256 KB), which four warps
 //                          read and write as a register file: thread = 8 matrix columns, for which the
 //                          three vectors of a step stay in registers.  One exchange per step: every CTA
 //                          sends its rows of A v and of the next column to all others with st.async
@@ -20,13 +20,14 @@
 //
 // Bound: the latency chain of step 1 (p steps of exchange, two reductions and one pass over the matrix).
 #include <atomic>
+#include <type_traits>
 
 #include "tcgen05.cuh"
 
 namespace shard {
 
 constexpr int EG_CL = 16;                  // CTAs of a cluster
-constexpr int EG_THREADS = 512;
+constexpr int EG_THREADS = 128;
 constexpr int EG_MAX_P = 1024;
 
 struct EighParams {
@@ -54,31 +55,43 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t cta) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(cta));
   return r;
 }
-__device__ __forceinline__ void st_async_f2(uint32_t addr, float a, float b, uint32_t bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
-               ::"r"(addr), "f"(a), "f"(b), "r"(bar) : "memory");
+__device__ __forceinline__ void st_async_f4(uint32_t addr, float a, float b, float c, float d, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+               ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void st_async_f1(uint32_t addr, float a, uint32_t bar) {
   asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];"
                ::"r"(addr), "f"(a), "r"(bar) : "memory");
 }
 
-// A row's CB columns of this thread, tensor memory <-> registers.
-template <int CB>
-__device__ __forceinline__ void eg_ld(uint32_t t, uint32_t (&u)[CB]) {
-  if constexpr (CB == 8) tmem_ld_x8(t, u);
-  else if constexpr (CB == 4) tmem_ld_x4(t, u);
-  else
-#pragma unroll
-    for (int j = 0; j < CB; ++j) asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(u[j]) : "r"(t + j));
+// A row's columns of this thread, tensor memory <-> registers.
+template <int W, int O = 0, int M>
+__device__ __forceinline__ void eg_ld(uint32_t t, uint32_t (&u)[M]) {
+  if constexpr (W - O >= 8)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(u[O]), "=r"(u[O + 1]), "=r"(u[O + 2]), "=r"(u[O + 3]), "=r"(u[O + 4]), "=r"(u[O + 5]), "=r"(u[O + 6]), "=r"(u[O + 7]) : "r"(t + O));
+  else if constexpr (W - O >= 4) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(u[O]), "=r"(u[O + 1]), "=r"(u[O + 2]), "=r"(u[O + 3]) : "r"(t + O));
+    eg_ld<W, O + 4>(t, u);
+  } else if constexpr (W - O >= 2) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(u[O]), "=r"(u[O + 1]) : "r"(t + O));
+    eg_ld<W, O + 2>(t, u);
+  } else if constexpr (W - O == 1)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(u[O]) : "r"(t + O));
 }
-template <int CB>
-__device__ __forceinline__ void eg_st(uint32_t t, const uint32_t (&u)[CB]) {
-  if constexpr (CB == 8) tmem_st_x8(t, u);
-  else if constexpr (CB == 4) tmem_st_x4(t, u);
-  else
-#pragma unroll
-    for (int j = 0; j < CB; ++j) asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t + j), "r"(u[j]) : "memory");
+template <int W, int O = 0, int M>
+__device__ __forceinline__ void eg_st(uint32_t t, const uint32_t (&u)[M]) {
+  if constexpr (W - O >= 8)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(t + O), "r"(u[O]), "r"(u[O + 1]),
+                 "r"(u[O + 2]), "r"(u[O + 3]), "r"(u[O + 4]), "r"(u[O + 5]), "r"(u[O + 6]), "r"(u[O + 7]) : "memory");
+  else if constexpr (W - O >= 4) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(t + O), "r"(u[O]), "r"(u[O + 1]), "r"(u[O + 2]), "r"(u[O + 3]) : "memory");
+    eg_st<W, O + 4>(t, u);
+  } else if constexpr (W - O >= 2) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1,%2};" ::"r"(t + O), "r"(u[O]), "r"(u[O + 1]) : "memory");
+    eg_st<W, O + 2>(t, u);
+  } else if constexpr (W - O == 1)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t + O), "r"(u[O]) : "memory");
 }
 // barrier of one 128-thread group, ORing a flag over it
 __device__ __forceinline__ bool eg_bar_or(int id, bool flag) {
@@ -88,28 +101,47 @@ __device__ __forceinline__ bool eg_bar_or(int id, bool flag) {
   return out != 0;
 }
 
-// CB = p / 128 columns per thread; a CTA has RL = p / 16 rows, 4 row groups of RS = p / 64 rows each
-// (RP: RS rounded up to a power of two).
+// Packed pairs of fp32: one instruction does both multiply-adds.
+__device__ __forceinline__ unsigned long long f2_pack(float a, float b) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// CB = p / 128 columns per thread; a CTA has RL = p / 16 rows, worked on in chunks of RC rows of 4-row
+// loads (p = 128: one chunk of 8).  Four warps: a step's scalar work is a chain that more warps would only repeat.
+constexpr int EG_MAIL = 66;                 // float2 per sender in the mailbox: 64 rows + padding against bank conflicts
+
 template <int CB>
 __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_constant__ EighParams p) {
-  constexpr int N = CB * 128, RS = CB * 2, RP = RS > 8 ? 16 : RS > 4 ? 8 : RS > 2 ? 4 : 2, LOG = RP == 16 ? 4 : RP == 8 ? 3 : RP == 4 ? 2 : 1;
-  __shared__ float2 mail[2][N];              // (A v)[r] and next column [r], from every CTA
-  __shared__ float mail_g[2][64];            // parts of v . A v
-  __shared__ float part[4][4][RP];           // row group, quarter of the columns
-  __shared__ float acol[4][RS];              // next column, own rows
-  __shared__ float vrow[2][4][RS];           // v of the own rows (this step's and the last one's)
-  __shared__ float red[4][8];
-  __shared__ float2 out[4][RS];
+  constexpr int N = CB * 128, RL = CB * 8, RC = RL % 16 ? 8 : 16, LOG = RC == 16 ? 4 : 3;
+  __shared__ __align__(16) float2 mail[2][EG_CL * EG_MAIL];   // (A v, next column) of every row, by sender
+  __shared__ __align__(16) float mail_g[2][EG_CL];         // parts of tau / 2 v . p
+  __shared__ __align__(16) float part[4][RL];   // A v of the own rows, quarter of the columns
+  __shared__ __align__(16) float acol[RL];   // next column, own rows
+  __shared__ __align__(16) float vrow[2][RL];   // v of the own rows (this step's and the last one's)
+  __shared__ __align__(16) float4 vw[RL];    // (-v, -v, -w, -w) of the own rows
+  __shared__ float red[12];
   __shared__ uint64_t bars[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_w;
   volatile int* abort_s = &abort_w;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = warp & 3, rg = warp >> 2;
+  const int tid = threadIdx.x, q = tid >> 5, lane = tid & 31;
   const int m = blockIdx.x / EG_CL;
-  const uint32_t rank = cluster_rank();
+  const int rank = (int)cluster_rank();
   const float* A = p.a + (size_t)m * N * N;
 
-  if (warp == 0) {
+  if (q == 0) {
     tmem_alloc(smem_u32(&tmem_slot), 512);
     tmem_relinquish();
     if (lane == 0) {
@@ -119,191 +151,238 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
       fence_mbar_init();
     }
   }
-  constexpr uint32_t TX = N * 8 + 64 * 4;    // bytes a CTA receives per step
+  constexpr uint32_t TX = N * 8 + EG_CL * 4; // bytes a CTA receives per step
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (tid == 0) { mbar_expect_tx(smem_u32(&bars[0]), TX); mbar_expect_tx(smem_u32(&bars[1]), TX); }
   const uint32_t T = tmem_slot + ((uint32_t)(q * 32) << 16);
-  const int c0 = 32 * q + lane;              // own columns c0 + 128 j
-  // local row i = 4 s + rg (s < RS) is matrix row 16 i + rank, at tensor-memory columns CB * i
+  const int c0 = tid;                        // own columns c0 + 128 j
+  // local row i is matrix row 16 i + rank, at tensor-memory columns CB * i
 #pragma unroll 4
-  for (int s = 0; s < RS; ++s) {
-    const int i = 4 * s + rg;
+  for (int i = 0; i < RL; ++i) {
     const float* row = A + (size_t)(16 * i + rank) * N + c0;
     uint32_t v[CB];
 #pragma unroll
     for (int j = 0; j < CB; ++j) v[j] = __float_as_uint(row[128 * j]);
     eg_st<CB>(T + CB * i, v);
-    if (c0 == 0) acol[rg][s] = __uint_as_float(v[0]);           // column 0
+    if (c0 == 0) acol[i] = __uint_as_float(v[0]);               // column 0
   }
   tmem_wait_st();
-  if (tid < 4 * RS) vrow[0][tid / RS][tid % RS] = vrow[1][tid / RS][tid % RS] = 0.f;
+  if (tid < RL) {
+    vrow[0][tid] = vrow[1][tid] = 0.f;
+    part[0][tid] = part[1][tid] = part[2][tid] = part[3][tid] = 0.f;
+  }
   __syncthreads();
   cluster_sync();                            // every CTA's barriers are armed
-  auto send = [&](int b, float g_part) {
-    // the row group's (A v, next column) pairs to all 16 CTAs; 128 threads: CTA t / 8, rows t % 8, ...
-    const int t = tid & 127, dst = t >> 3;
-    const uint32_t rbar = map_to_cta(smem_u32(&bars[b]), dst);
-    const uint32_t base = map_to_cta(smem_u32(&mail[b][0]), dst);
+  // Warp q delivers to CTAs 4 q .. 4 q + 3: lane = row pair, both (A v, next column) pairs in one 16-byte store.
+  uint32_t far[4];
 #pragma unroll
-    for (int s = t & 7; s < RS; s += 8) {
-      const float2 o = out[rg][s];
-      st_async_f2(base + 8u * (uint32_t)(16 * (4 * s + rg) + rank), o.x, o.y, rbar);
+  for (int d = 0; d < 4; ++d) far[d] = map_to_cta(smem_u32(&mail[0][0]), 4 * q + d);
+  const uint32_t bar_off = smem_u32(&bars[0]) - smem_u32(&mail[0][0]), g_off = smem_u32(&mail_g[0][0]) - smem_u32(&mail[0][0]);
+  auto send_rows = [&](int b, float p0, float a0, float p1, float a1) {
+    if (2 * lane < RL) {
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+        st_async_f4(far[d] + (uint32_t)((b * EG_CL + rank) * EG_MAIL + 2 * lane) * 8u, p0, a0, p1, a1, far[d] + bar_off + 8u * (uint32_t)b);
     }
-    if ((t & 7) == 0) st_async_f1(map_to_cta(smem_u32(&mail_g[b][0]), dst) + 4u * (uint32_t)(4 * rank + rg), g_part, rbar);
   };
-  if ((tid & 127) < RS) out[rg][tid & 127] = make_float2(0.f, acol[rg][tid & 127]);
-  named_bar_sync_128(1 + rg);
-  send(0, 0.f);
+  auto send_gamma = [&](int b, float g) {
+    if (lane == 0) {
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+        st_async_f1(far[d] + g_off + 4u * (uint32_t)(b * EG_CL + rank), g, far[d] + bar_off + 8u * (uint32_t)b);
+    }
+  };
+  const int pair = min(2 * lane, RL - 2);    // own rows of this lane in the delivery
+  send_rows(0, 0.f, acol[pair], 0.f, acol[pair + 1]);
+  send_gamma(0, 0.f);
 
-  float v[CB], w[CB], vn[CB];
+  float v[CB];                               // the last reflector (columns from block J0 on)
 #pragma unroll
   for (int j = 0; j < CB; ++j) v[j] = 0.f;
-  for (int k = 0; k < N; ++k) {              // column k: its reflector, then the matrix updated with the last one
-    const int b = k & 1;
-    mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
-    if (tid == 0) mbar_expect_tx(smem_u32(&bars[b]), TX);
-    // gamma = tau / 2 v . p with p = tau A v: the same sum, in the same order, everywhere
-    float gam = mail_g[b][lane] + mail_g[b][lane + 32];
+  // gamma = tau / 2 v . p with p = tau A v: the same sum, in the same order, everywhere
+  auto gamma = [&](int b) {
+    const float4* g4 = reinterpret_cast<const float4*>(mail_g[b]);
+    float4 s4 = g4[0];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) gam += __shfl_xor_sync(0xffffffffu, gam, o);
-    const float2 mk = mail[b][k];
-    const float w1 = mk.x - gam;                                // w[k]; v[k] = 1 (no v yet at k = 0: all zero)
-    float x[CB], ss = 0.f;
+    for (int i = 1; i < EG_CL / 4; ++i) { const float4 t = g4[i]; s4.x += t.x; s4.y += t.y; s4.z += t.z; s4.w += t.w; }
+    return (s4.x + s4.y) + (s4.z + s4.w);
+  };
+  // Columns k with (k + 1) / 128 == J0: the blocks of 128 columns before J0 have retired, and the next
+  // column lies in block J0.  Column k: its reflector; then one pass over the own rows still active:
+  // A -= v w' + w v' with the last reflector, A times the new one, the next column.
+  auto phase = [&](auto j0c) -> bool {
+    constexpr int J0 = decltype(j0c)::value, W = CB - J0, P = W / 2;
+#pragma unroll 1
+    for (int k = J0 ? 128 * J0 - 1 : 0; k < 128 * J0 + 127; ++k) {
+      const int b = k & 1;
+      mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
+      if (tid == 0) mbar_expect_tx(smem_u32(&bars[b]), TX);
+      const float gam = gamma(b);
+      const float2 mk = mail[b][(k & 15) * EG_MAIL + (k >> 4)];
+      const float w1 = mk.x - gam;                              // w[k]; v[k] = 1 (no v yet at k = 0: all zero)
+      float x[W], w[W], ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const int c = c0 + 128 * j;
-      const float2 pa = mail[b][c];
-      w[j] = fmaf(-gam, v[j], pa.x);
-      x[j] = pa.y - fmaf(v[j], w1, w[j]);
-      if (c <= k) x[j] = 0.f;
-      if (c == k + 1) red[rg][4] = x[j];
-      else ss = fmaf(x[j], x[j], ss);
-      if (c < k) w[j] = 0.f;
-    }
-    // row scalars of the update
-    float vr = 0.f, wr = 0.f;
-    if (lane < RS) {
-      vr = vrow[b ^ 1][rg][lane];
-      wr = fmaf(-gam, vr, mail[b][16 * (4 * lane + rg) + rank].x);
-    }
-    ss = warp_sum(ss);
-    if (lane == 0) red[rg][q] = ss;
-    named_bar_sync_128(1 + rg);
-    const float x0 = k + 1 < N ? red[rg][4] : 0.f;
-    ss = (red[rg][0] + red[rg][1]) + (red[rg][2] + red[rg][3]);
-    float beta = x0, tau = 0.f, scale = 0.f;
-    if (ss > 0.f) {
-      beta = -copysignf(sqrtf(fmaf(x0, x0, ss)), x0);
-      tau = (beta - x0) / beta;
-      scale = 1.f / (x0 - beta);
-    }
-#pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      const int c = c0 + 128 * j;
-      vn[j] = c == k + 1 ? 1.f : x[j] * scale;                  // (x is zero up to row k)
-      // own rows: the thread whose column is one of them leaves v there
-      if ((c & 15) == (int)rank && ((c >> 4) & 3) == rg) vrow[b][rg][c >> 6] = vn[j];
-    }
-    if ((k & 15) == (int)rank && rg == 0) {
-      float* o = p.refl + ((size_t)m * N + k) * N + c0;
-#pragma unroll
-      for (int j = 0; j < CB; ++j) o[128 * j] = vn[j];
-      if (tid == 0) {
-        p.d[m * N + k] = mk.y - 2.f * w1;
-        p.e[m * N + k] = beta;
-        p.tau[m * N + k] = tau;
+      for (int j = 0; j < W; ++j) {
+        const float2 pa = mail[b][(c0 & 15) * EG_MAIL + (c0 >> 4) + 8 * (J0 + j)];
+        w[j] = fmaf(-gam, v[J0 + j], pa.x);
+        x[j] = pa.y - fmaf(v[J0 + j], w1, w[j]);
       }
-    }
-    if (k == N - 1) break;
-    // ---- own rows: A -= v w' + w v', then A vn and the next column -------------------------------
-    float dot[RP];
-    const bool has_col = q == (((k + 1) >> 5) & 3);
-    const int jc = (k + 1) >> 7;
+      const int cj = c0 + 128 * J0;                             // only block J0 has columns up to k + 1
+      if (cj <= k) x[0] = 0.f;
+      if (cj == k + 1) red[4] = x[0];
+      else ss = x[0] * x[0];
 #pragma unroll
-    for (int s = 0; s < RP; ++s) dot[s] = 0.f;
+      for (int j = 1; j < W; ++j) ss = fmaf(x[j], x[j], ss);
+      if (tid < RL) {                                           // row scalars of the update
+        const float vr = vrow[b ^ 1][tid];
+        const float wr = fmaf(-gam, vr, mail[b][rank * EG_MAIL + tid].x);
+        vw[tid] = make_float4(-vr, -vr, -wr, -wr);
+      }
+      ss = warp_sum(ss);
+      if (lane == 0) red[q] = ss;
+      __syncthreads();
+      const float x0 = red[4];
+      ss = (red[0] + red[1]) + (red[2] + red[3]);
+      float beta = x0, tau = 0.f, scale = 0.f;
+      if (ss > 0.f) {
+        beta = -copysignf(sqrtf(fmaf(x0, x0, ss)), x0);
+        tau = (beta - x0) / beta;
+        scale = 1.f / (x0 - beta);
+      }
+      float vn[W];
 #pragma unroll
-    for (int s0 = 0; s0 < RS; s0 += 4) {
-      constexpr int B = RS < 4 ? RS : 4;
-      const int top = s0 + 3 < RS ? s0 + 3 : RS - 1;
-      if (16 * (4 * top + rg) + (int)rank > k) {                 // (uniform over the warp) a row of the four is still active
-        uint32_t u[B][CB];
+      for (int j = 0; j < W; ++j) vn[j] = x[j] * scale;         // (x is zero up to row k)
+      if (cj == k + 1) vn[0] = 1.f;
+      if ((tid & 15) == rank) {
 #pragma unroll
-        for (int s = 0; s < B; ++s)
-          if (s0 + s < RS) eg_ld<CB>(T + CB * (4 * (s0 + s) + rg), u[s]);
-        tmem_wait_ld();
+        for (int j = 0; j < W; ++j) vrow[b][(c0 >> 4) + 8 * (J0 + j)] = vn[j];   // own columns that are own rows too
+      }
+      unsigned long long v2[P + 1], w2[P + 1], n2[P + 1];
 #pragma unroll
-        for (int s = 0; s < B; ++s) {
-          if (s0 + s < RS) {
-            const float vs = __shfl_sync(0xffffffffu, vr, s0 + s), ws = __shfl_sync(0xffffffffu, wr, s0 + s);
-            float sum = 0.f;
+      for (int j = 0; j < P; ++j) {
+        v2[j] = f2_pack(v[J0 + 2 * j], v[J0 + 2 * j + 1]);
+        w2[j] = f2_pack(w[2 * j], w[2 * j + 1]);
+        n2[j] = f2_pack(vn[2 * j], vn[2 * j + 1]);
+      }
+      const bool has_col = cj == k + 1;                         // this thread holds the next column
+#pragma unroll 1
+      for (int ch = 0; ch < RL / RC; ++ch) {
+        if (16 * (RC * ch + RC - 1) + rank <= k) continue;      // (uniform) all of the chunk's rows have retired
+        float dot[RC];
+        uint32_t u[2][4][W];
+        const uint32_t Tc = T + CB * RC * ch + J0;
 #pragma unroll
-            for (int j = 0; j < CB; ++j) {
-              const float a = fmaf(-ws, v[j], fmaf(-vs, w[j], __uint_as_float(u[s][j])));
-              sum = fmaf(a, vn[j], sum);
-              u[s][j] = __float_as_uint(a);
-            }
-            eg_st<CB>(T + CB * (4 * (s0 + s) + rg), u[s]);
-            dot[s0 + s] = sum;
-            if (has_col) {
-              uint32_t sel = u[s][0];
-              switch (jc) {
-                case 1: if (CB > 1) sel = u[s][1 < CB ? 1 : 0]; break;
-                case 2: if (CB > 2) sel = u[s][2 < CB ? 2 : 0]; break;
-                case 3: if (CB > 3) sel = u[s][3 < CB ? 3 : 0]; break;
-                case 4: if (CB > 4) sel = u[s][4 < CB ? 4 : 0]; break;
-                case 5: if (CB > 5) sel = u[s][5 < CB ? 5 : 0]; break;
-                case 6: if (CB > 6) sel = u[s][6 < CB ? 6 : 0]; break;
-                case 7: if (CB > 7) sel = u[s][7 < CB ? 7 : 0]; break;
-              }
-              if (lane == ((k + 1) & 31)) acol[rg][s0 + s] = __uint_as_float(sel);
+        for (int r = 0; r < 4; ++r) eg_ld<W>(Tc + CB * r, u[0][r]);
+#pragma unroll
+        for (int b4 = 0; b4 < RC / 4; ++b4) {
+          ulonglong2 rw[4];                                     // (fetched and stored four rows at a time: the rows' chains overlap)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) rw[r] = *reinterpret_cast<const ulonglong2*>(&vw[RC * ch + 4 * b4 + r]);
+          tmem_wait_ld();
+          if (b4 + 1 < RC / 4) {                                // the next four rows come in while these are worked on
+#pragma unroll
+            for (int r = 0; r < 4; ++r) eg_ld<W>(Tc + CB * (4 * (b4 + 1) + r), u[(b4 + 1) & 1][r]);
+          }
+          unsigned long long acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+          for (int j = 0; j < P; ++j) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              uint32_t(&y)[W] = u[b4 & 1][r];
+              unsigned long long a = f2_pack(__uint_as_float(y[2 * j]), __uint_as_float(y[2 * j + 1]));
+              a = f2_fma(rw[r].y, v2[j], f2_fma(rw[r].x, w2[j], a));
+              acc[r] = f2_fma(a, n2[j], acc[r]);
+              const float2 f = f2_unpack(a);
+              y[2 * j] = __float_as_uint(f.x);
+              y[2 * j + 1] = __float_as_uint(f.y);
             }
           }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            uint32_t(&y)[W] = u[b4 & 1][r];
+            const float2 f = f2_unpack(acc[r]);
+            float sum = f.x + f.y;
+            if (W & 1) {
+              const float2 rv = f2_unpack(rw[r].x), rz = f2_unpack(rw[r].y);
+              const float a = fmaf(rz.x, v[CB - 1], fmaf(rv.x, w[W - 1], __uint_as_float(y[W - 1])));
+              sum = fmaf(a, vn[W - 1], sum);
+              y[W - 1] = __float_as_uint(a);
+            }
+            dot[4 * b4 + r] = sum;
+          }
+#pragma unroll
+          for (int r = 0; r < 4; ++r) eg_st<W>(Tc + CB * (4 * b4 + r), u[b4 & 1][r]);
+          if (has_col) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acol[RC * ch + 4 * b4 + r] = __uint_as_float(u[b4 & 1][r][0]);
+          }
+        }
+        // sums over the lanes, all rows of the chunk at once: halve the rows a lane carries, fold the lanes
+        int off = 16;
+#pragma unroll
+        for (int h = RC / 2; h >= 1; h >>= 1) {
+          const bool up = (lane & off) != 0;
+#pragma unroll
+          for (int r = 0; r < h; ++r) {
+            const float keep = up ? dot[r + h] : dot[r], give = up ? dot[r] : dot[r + h];
+            dot[r] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+          }
+          off >>= 1;
+        }
+        for (; off >= 1; off >>= 1) dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], off);
+        // lane bits from the top select the row
+        if ((lane & ((32 >> LOG) - 1)) == 0) part[q][RC * ch + (lane >> (5 - LOG))] = dot[0];
+      }
+      tmem_wait_st();
+      if (eg_bar_or(1, *abort_s != 0)) return false;            // (uniform over the CTA)
+      {
+        float2 s0 = *reinterpret_cast<const float2*>(&part[0][pair]), s1 = *reinterpret_cast<const float2*>(&part[1][pair]);
+        const float2 s2 = *reinterpret_cast<const float2*>(&part[2][pair]), s3 = *reinterpret_cast<const float2*>(&part[3][pair]);
+        const float2 ac = *reinterpret_cast<const float2*>(&acol[pair]), vr = *reinterpret_cast<const float2*>(&vrow[b][pair]);
+        const float p0 = 16 * pair + rank > k ? tau * ((s0.x + s1.x) + (s2.x + s3.x)) : 0.f;
+        const float p1 = 16 * (pair + 1) + rank > k ? tau * ((s0.y + s1.y) + (s2.y + s3.y)) : 0.f;
+        send_rows(b ^ 1, p0, ac.x, p1, ac.y);
+        const float g = 2 * lane < RL ? fmaf(vr.x, p0, vr.y * p1) : 0.f;
+        send_gamma(b ^ 1, 0.5f * tau * warp_sum(g));
+      }
+      if ((k & 15) == rank) {                                   // the record of the step, off the critical path
+        float* o = p.refl + ((size_t)m * N + k) * N + c0 + 128 * J0;   // (retired columns are never read)
+#pragma unroll
+        for (int j = 0; j < W; ++j) o[128 * j] = vn[j];
+        if (tid == 0) {
+          p.d[m * N + k] = mk.y - 2.f * w1;
+          p.e[m * N + k] = beta;
+          p.tau[m * N + k] = tau;
         }
       }
-    }
-    tmem_wait_st();
-    // sums over the lanes, all rows at once: halve the rows a lane carries, fold the lanes
-    {
-      int off = 16;
 #pragma unroll
-      for (int h = RP / 2; h >= 1; h >>= 1) {
-        const bool up = (lane & off) != 0;
-#pragma unroll
-        for (int s = 0; s < h; ++s) {
-          const float keep = up ? dot[s + h] : dot[s], give = up ? dot[s] : dot[s + h];
-          dot[s] = keep + __shfl_xor_sync(0xffffffffu, give, off);
-        }
-        off >>= 1;
-      }
-      for (; off >= 1; off >>= 1) dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], off);
-      // lane bits from the top select the row: bit 4 -> row bit log2(RS) - 1, ...
-      if ((lane & ((32 >> LOG) - 1)) == 0) part[rg][q][lane >> (5 - LOG)] = dot[0];
+      for (int j = 0; j < W; ++j) v[J0 + j] = vn[j];
     }
-    named_bar_sync_128(1 + rg);
-    float g = 0.f;
-    {
-      // every warp of the row group finishes all RS rows (and keeps the same g); its first warp stores
-      float pr = 0.f, ac = 0.f, vnr = 0.f;
-      if (lane < RS) {
-        if (16 * (4 * lane + rg) + (int)rank > k)
-          pr = tau * ((part[rg][0][lane] + part[rg][1][lane]) + (part[rg][2][lane] + part[rg][3][lane]));
-        ac = acol[rg][lane];
-        vnr = vrow[b][rg][lane];
-        if (q == 0) out[rg][lane] = make_float2(pr, ac);
-      }
-      g = 0.5f * tau * warp_sum(vnr * pr);
+    return true;
+  };
+  bool ok = phase(std::integral_constant<int, 0>());
+  if constexpr (CB > 1) ok = ok && phase(std::integral_constant<int, (CB > 1 ? 1 : 0)>());
+  if constexpr (CB > 2) ok = ok && phase(std::integral_constant<int, (CB > 2 ? 2 : 0)>());
+  if constexpr (CB > 3) ok = ok && phase(std::integral_constant<int, (CB > 3 ? 3 : 0)>());
+  if constexpr (CB > 4) ok = ok && phase(std::integral_constant<int, (CB > 4 ? 4 : 0)>());
+  if constexpr (CB > 5) ok = ok && phase(std::integral_constant<int, (CB > 5 ? 5 : 0)>());
+  if constexpr (CB > 6) ok = ok && phase(std::integral_constant<int, (CB > 6 ? 6 : 0)>());
+  if constexpr (CB > 7) ok = ok && phase(std::integral_constant<int, (CB > 7 ? 7 : 0)>());
+  if (ok) {                                  // the last column: only its diagonal entry
+    constexpr int k = N - 1, b = k & 1;
+    mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
+    const float2 mk = mail[b][(k & 15) * EG_MAIL + (k >> 4)];
+    if ((k & 15) == rank && tid == 0) {
+      p.d[m * N + k] = mk.y - 2.f * (mk.x - gamma(b));
+      p.e[m * N + k] = p.tau[m * N + k] = 0.f;
     }
-    if (eg_bar_or(1 + rg, *abort_s != 0)) break;                 // (uniform over the row group)
-    send(b ^ 1, g);
-#pragma unroll
-    for (int j = 0; j < CB; ++j) v[j] = vn[j];
   }
   if (tid == 0 && *abort_s) atomicExch(p.flag + m, 1);
   tc_fence_before();
   cluster_sync();                            // nobody is still sending to a CTA that leaves
-  if (warp == 0) tmem_dealloc(tmem_slot, 512);
+  if (q == 0) tmem_dealloc(tmem_slot, 512);
 }
 
 // ---------------------------------------------------------------------------

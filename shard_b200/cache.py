@@ -5,14 +5,11 @@ reference's src/shard/cache.py (prefill keeps raw K/V; the first decode step
 compresses every layer; later steps append to an 8-bit stream or an fp16
 buffer), but every array-sized computation runs in libshard_b200.so:
 
-* K: RoPE removal -> (PyTorch) low-rank SVD -> host bit allocation -> int8 basis
+* K: RoPE removal -> covariance -> eigensolver kernels -> host bit allocation -> int8 basis
   -> projection kernel -> two-stage int4 quantiser + nibble packing;
-* V: Hadamard + per-channel normalisation kernel -> k-means whose assignment step
-  is the `vq_assign` kernel;
+* V: Hadamard + per-channel normalisation kernel -> k-means kernels;
 * decode append: the Lloyd-Max stream quantizer kernel.
 
-What stays in PyTorch is what the reference also leaves to PyTorch: the
-randomised SVD, the centroid update (`index_add_`) and small host-side logic.
 There is no CPU path: tensors must live on a CUDA device.
 """
 from __future__ import annotations
@@ -32,6 +29,45 @@ KERNEL_RANK_STEP = 32
 KERNEL_MAX_RANK = 192
 
 
+# matrices whose eigensolver launches run side by side: each takes a cluster of 16 SMs, and seven such
+# clusters fit a B200 (its GPCs are a little short of 148 SMs' worth of them)
+EIGH_GROUP = 7
+
+
+def gram_matrix(flat, mean):
+    """(flat - mean)^T (flat - mean) of the rows of `flat` (n, p), fp32."""
+    xc = flat - mean
+    # full-precision fp32 products whatever the global TF32 switch says: the trailing
+    # eigenvalues are 1e-4 of the leading ones and decide the bit allocation
+    prev = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    try:
+        return xc.T @ xc
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = prev
+
+
+class LeadingEigenpairs:
+    """The `rank` largest eigenpairs of each (p, p) matrix of `gram` (count, p, p): launched on the current
+    stream when made, waited for by `result` (on the same stream)."""
+
+    def __init__(self, gram, rank):
+        self.gram, self.rank = gram, rank
+        self.basis, self.eigvals, self.flag = ops.eigh_top(gram, rank)
+
+    def result(self):
+        """basis (count, p, rank), eigenvectors in the columns, largest first; eigenvalues (count, rank)
+        on the host.  Matrices the package's solver reports as too close to degenerate go to
+        torch.linalg.eigh."""
+        rank = self.rank
+        host = torch.cat([self.eigvals, self.flag.unsqueeze(1).float()], dim=1).cpu()
+        for i in torch.nonzero(host[:, rank]).flatten().tolist():
+            w, v = torch.linalg.eigh(self.gram[i])
+            self.basis[i] = v.flip(-1)[:, :rank]
+            host[i, :rank] = w.flip(-1)[:rank].cpu()
+        return self.basis, host[:, :rank]
+
+
 def pca_fit(flat, mean, rank):
     """Top-`rank` principal directions of the rows of `flat` (n, p) around `mean`: the
     eigenvectors of the p x p covariance, largest eigenvalue first, and those eigenvalues.
@@ -39,26 +75,13 @@ def pca_fit(flat, mean, rank):
     Replaces the reference's randomised `torch.svd_lowrank(flat - mean, q=rank, niter=24)`
     (src/shard/cache.py:376: 48 passes over the n x p matrix) by one pass -- the Gram matrix
     (flat - mean)^T (flat - mean), a p x p x n contraction in fp32 -- and a symmetric
-    eigensolver on the small p x p matrix.  The subspace is the exact optimum the randomised
-    method approximates, so it captures at least as much variance; individual vectors differ
+    eigensolver on the small p x p matrix (`ops.eigh_top`).  The subspace is the exact optimum the
+    randomised method approximates, so it captures at least as much variance; individual vectors differ
     in sign and, within near-equal eigenvalues, by rotations, which the rest of the path is
     indifferent to (the basis is an input of everything downstream).
     """
-    n, p = flat.shape
-    xc = flat - mean
-    # full-precision fp32 products whatever the global TF32 switch says: the trailing
-    # eigenvalues are 1e-4 of the leading ones and decide the bit allocation
-    prev = torch.backends.cuda.matmul.allow_tf32
-    torch.backends.cuda.matmul.allow_tf32 = False
-    try:
-        gram = xc.T @ xc
-    finally:
-        torch.backends.cuda.matmul.allow_tf32 = prev
-    evals, evecs = torch.linalg.eigh(gram)
-    order = torch.arange(p - 1, p - 1 - rank, -1, device=flat.device)
-    basis = evecs[:, order].contiguous()
-    eigvals = (evals[order].clamp(min=0) / n).float()
-    return basis, eigvals
+    basis, eigvals = LeadingEigenpairs(gram_matrix(flat, mean).unsqueeze(0), rank).result()
+    return basis[0], (eigvals[0].clamp(min=0) / flat.shape[0]).to(flat.device)
 
 
 def hadamard(x):
@@ -444,20 +467,71 @@ class Cache(HFCache):
         # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
         n_sub = (end - start) * self._n_kv_heads * (self.head_dim // self._v_vq_group_size)
         init_rows = initial_rows(n_sub, self._v_vq_codebook_size, k0.device)
-        for li in range(self._num_layers):
-            torch.manual_seed(42 + li)
-            layer = self.layers[li]
-            k_full, v_full = layer._keys, layer._values
-            kpart = self._compress_k(k_full[0, :, start:end, :], start)
-            vpart = self._compress_v(v_full[0, :, start:end, :], init_rows=init_rows)
-            self._build_gpu_format(layer, kpart, vpart,
-                                   sink_k=k_full[:, :, :sink, :].clone(), sink_v=v_full[:, :, :sink, :].clone(),
-                                   win_k=k_full[:, :, end:, :].clone(), win_v=v_full[:, :, end:, :].clone(),
-                                   n_comp=end - start, batch=B, start=start)
+        if self._k_pca == "svd_lowrank":
+            for li in range(self._num_layers):
+                torch.manual_seed(42 + li)
+                k_full, v_full = self.layers[li]._keys, self.layers[li]._values
+                kpart = self._compress_k(k_full[0, :, start:end, :], start)
+                vpart = self._compress_v(v_full[0, :, start:end, :], init_rows=init_rows)
+                self._finish_layer(li, kpart, vpart, start, end)
+        else:
+            self._compress_side_by_side(start, end, init_rows)
         ev1.record()
         ev1.synchronize()
         self.compress_seconds = ev0.elapsed_time(ev1) / 1e3
         self._compressed = True
+
+    def _compress_side_by_side(self, start, end, init_rows):
+        """Layers in groups.  The eigensolver of a group's key covariances is a long chain of small steps
+        on a few SMs: it runs on a second stream beside the group's value path (k-means) and the next
+        group's covariances; the host waits only for the eigenvalues, which decide the bit widths."""
+        n_layers = self._num_layers
+        main = torch.cuda.current_stream()
+        side = torch.cuda.Stream(main.device)
+        n_groups = -(-n_layers // EIGH_GROUP)
+        bounds = [n_layers * g // n_groups for g in range(n_groups + 1)]
+
+        def covariances(g):
+            layers, grams = [], []
+            for li in range(bounds[g], bounds[g + 1]):
+                k_mid = self.layers[li]._keys[0, :, start:end, :]
+                flat = ops.undo_rope(k_mid, start, self._inv_freq(k_mid.device))
+                mean = flat.mean(dim=0)
+                layers.append((flat, mean))
+                grams.append(gram_matrix(flat, mean))
+            return layers, torch.stack(grams), main.record_event()
+
+        n, p = end - start, self._per_layer_dim
+        rank = min(self._max_rank_k, p, n - 1)
+        ready = covariances(0)
+        for g in range(n_groups):
+            layers, gram, done = ready
+            side.wait_event(done)
+            with torch.cuda.stream(side):
+                solved = LeadingEigenpairs(gram, rank)
+            vparts = [self._compress_v(self.layers[li]._values[0, :, start:end, :], init_rows=init_rows)
+                      for li in range(bounds[g], bounds[g + 1])]
+            if g + 1 < n_groups:
+                ready = covariances(g + 1)
+            with torch.cuda.stream(side):
+                basis, eig_host = solved.result()
+                fin = side.record_event()
+            main.wait_event(fin)
+            for i, li in enumerate(range(bounds[g], bounds[g + 1])):
+                flat, mean = layers[i]
+                kpart = self._quantise_k(flat, mean, basis[i], eig_host[i].clamp(min=0) / n)
+                self._finish_layer(li, kpart, vparts[i], start, end)
+        # the second stream's tensors go back to the allocator behind everything enqueued here
+        side.wait_stream(main)
+
+    def _finish_layer(self, li, kpart, vpart, start, end):
+        layer = self.layers[li]
+        k_full, v_full = layer._keys, layer._values
+        sink = self._sink_tokens
+        self._build_gpu_format(layer, kpart, vpart,
+                               sink_k=k_full[:, :, :sink, :].clone(), sink_v=v_full[:, :, :sink, :].clone(),
+                               win_k=k_full[:, :, end:, :].clone(), win_v=v_full[:, :, end:, :].clone(),
+                               n_comp=end - start, batch=k_full.shape[0], start=start)
 
     def _compress_k(self, k_mid, pos_start, basis=None):
         """Un-rotate, fit a joint PCA over all KV heads, quantise basis to int8 and
@@ -482,6 +556,11 @@ class Cache(HFCache):
         else:
             basis = basis.to(dev, torch.float32)[:, :rank]
             eigvals = ((flat - mean) @ basis).pow(2).sum(dim=0) / n
+        return self._quantise_k(flat, mean, basis, eigvals)
+
+    def _quantise_k(self, flat, mean, basis, eigvals):
+        """Bit allocation, int8 basis, projection and int4 codes of un-rotated keys `flat` (n, dim)."""
+        n = flat.shape[0]
         budget = max(64, int(self._per_layer_dim * 16 / self._k_target_cr))
         alloc = dp_bit_allocation(eigvals, budget)
         keep = sum(1 for b in alloc if b > 0)

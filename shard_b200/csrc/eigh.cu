@@ -3,7 +3,7 @@
 //
 //   1. tridiag_kernel      Householder reduction to tridiagonal form, one cluster of 16 CTAs per matrix.
 //                          The whole matrix stays on chip: row r lives in CTA r % 16, in TENSOR MEMORY
-//                          (64 rows x 1024 columns of fp32 are exactly its 256 KB), which four warps
+//                          (64 rows x 1024 columns of fp32 are exactly its 256 KB), which its warps
 //                          read and write as a register file: thread = 8 matrix columns, for which the
 //                          three vectors of a step stay in registers.  One exchange per step: every CTA
 //                          sends its rows of A v and of the next column to all others with st.async
@@ -27,7 +27,7 @@
 namespace shard {
 
 constexpr int EG_CL = 16;                  // CTAs of a cluster
-constexpr int EG_THREADS = 128;
+constexpr int EG_THREADS = 256;
 constexpr int EG_MAX_P = 1024;
 
 struct EighParams {
@@ -93,10 +93,10 @@ __device__ __forceinline__ void eg_st(uint32_t t, const uint32_t (&u)[M]) {
   } else if constexpr (W - O == 1)
     asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(t + O), "r"(u[O]) : "memory");
 }
-// barrier of one 128-thread group, ORing a flag over it
+// barrier of the CTA, ORing a flag over it
 __device__ __forceinline__ bool eg_bar_or(int id, bool flag) {
   uint32_t out;
-  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %2, 0;\n\tbar.red.or.pred p, %1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %2, 0;\n\tbar.red.or.pred p, %1, 256, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                : "=r"(out) : "r"(id), "r"((uint32_t)flag) : "memory");
   return out != 0;
 }
@@ -119,7 +119,7 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
 }
 
 // CB = p / 128 columns per thread; a CTA has RL = p / 16 rows, worked on in chunks of RC rows of 4-row
-// loads (p = 128: one chunk of 8).  Four warps: a step's scalar work is a chain that more warps would only repeat.
+// loads (p = 128: one chunk of 8).  Eight warps: a step's scalar work is a chain that more warps would only repeat.
 constexpr int EG_MAIL = 66;                 // float2 per sender in the mailbox: 64 rows + padding against bank conflicts
 
 template <int CB>
@@ -136,12 +136,13 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_w;
   volatile int* abort_s = &abort_w;
-  const int tid = threadIdx.x, q = tid >> 5, lane = tid & 31;
+  // warps q and q + 4 hold the same columns (and repeat each other's scalar work); the rows' chunks are split
+  const int tid = threadIdx.x & 127, rg = threadIdx.x >> 7, q = tid >> 5, lane = tid & 31;
   const int m = blockIdx.x / EG_CL;
   const int rank = (int)cluster_rank();
   const float* A = p.a + (size_t)m * N * N;
 
-  if (q == 0) {
+  if (threadIdx.x < 32) {
     tmem_alloc(smem_u32(&tmem_slot), 512);
     tmem_relinquish();
     if (lane == 0) {
@@ -155,12 +156,12 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (tid == 0) { mbar_expect_tx(smem_u32(&bars[0]), TX); mbar_expect_tx(smem_u32(&bars[1]), TX); }
+  if (threadIdx.x == 0) { mbar_expect_tx(smem_u32(&bars[0]), TX); mbar_expect_tx(smem_u32(&bars[1]), TX); }
   const uint32_t T = tmem_slot + ((uint32_t)(q * 32) << 16);
   const int c0 = tid;                        // own columns c0 + 128 j
   // local row i is matrix row 16 i + rank, at tensor-memory columns CB * i
 #pragma unroll 4
-  for (int i = 0; i < RL; ++i) {
+  for (int i = rg; i < RL; i += 2) {
     const float* row = A + (size_t)(16 * i + rank) * N + c0;
     uint32_t v[CB];
 #pragma unroll
@@ -175,22 +176,22 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
   }
   __syncthreads();
   cluster_sync();                            // every CTA's barriers are armed
-  // Warp q delivers to CTAs 4 q .. 4 q + 3: lane = row pair, both (A v, next column) pairs in one 16-byte store.
-  uint32_t far[4];
+  // Warp w delivers to CTAs 2 w and 2 w + 1: lane = row pair, both (A v, next column) pairs in one 16-byte store.
+  uint32_t far[2];
 #pragma unroll
-  for (int d = 0; d < 4; ++d) far[d] = map_to_cta(smem_u32(&mail[0][0]), 4 * q + d);
+  for (int d = 0; d < 2; ++d) far[d] = map_to_cta(smem_u32(&mail[0][0]), 2 * (q + 4 * rg) + d);
   const uint32_t bar_off = smem_u32(&bars[0]) - smem_u32(&mail[0][0]), g_off = smem_u32(&mail_g[0][0]) - smem_u32(&mail[0][0]);
   auto send_rows = [&](int b, float p0, float a0, float p1, float a1) {
     if (2 * lane < RL) {
 #pragma unroll
-      for (int d = 0; d < 4; ++d)
+      for (int d = 0; d < 2; ++d)
         st_async_f4(far[d] + (uint32_t)((b * EG_CL + rank) * EG_MAIL + 2 * lane) * 8u, p0, a0, p1, a1, far[d] + bar_off + 8u * (uint32_t)b);
     }
   };
   auto send_gamma = [&](int b, float g) {
     if (lane == 0) {
 #pragma unroll
-      for (int d = 0; d < 4; ++d)
+      for (int d = 0; d < 2; ++d)
         st_async_f1(far[d] + g_off + 4u * (uint32_t)(b * EG_CL + rank), g, far[d] + bar_off + 8u * (uint32_t)b);
     }
   };
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
     for (int k = J0 ? 128 * J0 - 1 : 0; k < 128 * J0 + 127; ++k) {
       const int b = k & 1;
       mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
-      if (tid == 0) mbar_expect_tx(smem_u32(&bars[b]), TX);
+      if (threadIdx.x == 0) mbar_expect_tx(smem_u32(&bars[b]), TX);
       const float gam = gamma(b);
       const float2 mk = mail[b][(k & 15) * EG_MAIL + (k >> 4)];
       const float w1 = mk.x - gam;                              // w[k]; v[k] = 1 (no v yet at k = 0: all zero)
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
       }
       const int cj = c0 + 128 * J0;                             // only block J0 has columns up to k + 1
       if (cj <= k) x[0] = 0.f;
-      if (cj == k + 1) red[4] = x[0];
+      if (cj == k + 1) red[4] = x[0];                           // (both of its threads, the same value)
       else ss = x[0] * x[0];
 #pragma unroll
       for (int j = 1; j < W; ++j) ss = fmaf(x[j], x[j], ss);
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
       }
       const bool has_col = cj == k + 1;                         // this thread holds the next column
 #pragma unroll 1
-      for (int ch = 0; ch < RL / RC; ++ch) {
+      for (int ch = rg; ch < RL / RC; ch += 2) {
         if (16 * (RC * ch + RC - 1) + rank <= k) continue;      // (uniform) all of the chunk's rows have retired
         float dot[RC];
         uint32_t u[2][4][W];
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
         const float g = 2 * lane < RL ? fmaf(vr.x, p0, vr.y * p1) : 0.f;
         send_gamma(b ^ 1, 0.5f * tau * warp_sum(g));
       }
-      if ((k & 15) == rank) {                                   // the record of the step, off the critical path
+      if ((k & 15) == rank && rg == 0) {                        // the record of the step, off the critical path
         float* o = p.refl + ((size_t)m * N + k) * N + c0 + 128 * J0;   // (retired columns are never read)
 #pragma unroll
         for (int j = 0; j < W; ++j) o[128 * j] = vn[j];
@@ -374,15 +375,15 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
     constexpr int k = N - 1, b = k & 1;
     mbar_wait(smem_u32(&bars[b]), (uint32_t)((k >> 1) & 1), abort_s);
     const float2 mk = mail[b][(k & 15) * EG_MAIL + (k >> 4)];
-    if ((k & 15) == rank && tid == 0) {
+    if ((k & 15) == rank && threadIdx.x == 0) {
       p.d[m * N + k] = mk.y - 2.f * (mk.x - gamma(b));
       p.e[m * N + k] = p.tau[m * N + k] = 0.f;
     }
   }
-  if (tid == 0 && *abort_s) atomicExch(p.flag + m, 1);
+  if (threadIdx.x == 0 && *abort_s) atomicExch(p.flag + m, 1);
   tc_fence_before();
   cluster_sync();                            // nobody is still sending to a CTA that leaves
-  if (q == 0) tmem_dealloc(tmem_slot, 512);
+  if (threadIdx.x < 32) tmem_dealloc(tmem_slot, 512);
 }
 
 // ---------------------------------------------------------------------------

@@ -385,18 +385,18 @@ int shard_b200_vq_assign_accumulate(const float* x, const float* centroids, int6
                                     float* sums, float* counts, void* stream);
 
 /*
- * k-means of [n][4] points with 256 centroids: kmeans (src/shard/cache.py:21-39) without its random
- * initialisation: the points are sorted once, then n_iter iterations run in as many launches.  `centroids` holds the initial centroids and
- * receives the final ones; idx_u8 [n] receives the assignment of the last iteration that ran (made
+ * k-means of `count` independent sets of [n][4] points with 256 centroids each: kmeans (src/shard/cache.py:21-39) without its random
+ * initialisation: the points are sorted once, then n_iter iterations run in as many launches.  `centroids` [count][256][4] holds the initial centroids and
+ * receives the final ones; idx_u8 [count][n] receives the assignment of the last iteration that ran (made
  * against the centroids before it).  Iterations stop having an effect once the largest move of a
  * centroid coordinate is below 1e-4, from the sixth on.  Assignments are exactly those of
  * shard_b200_vq_assign; the sums behind the means are fixed-point (2^-30 of the data's range), so the
- * result does not depend on any order.  max_abs: a bound on |x|, or 0 to have it computed.
- * workspace: shard_b200_kmeans_workspace_bytes(n) bytes (about 22 per point; 0 if n is out of range,
+ * result does not depend on any order.  max_abs: a bound on |x| of all sets, or 0 to have it computed.
+ * workspace: shard_b200_kmeans_workspace_bytes(count, n) bytes (about 22 per point; 0 if n is out of range,
  * 1 .. 2^31 - 1), 16-byte aligned.  x and centroids 16-byte aligned.
  */
-size_t shard_b200_kmeans_workspace_bytes(int64_t n);
-int shard_b200_kmeans(const float* x, int64_t n, float max_abs, int32_t n_iter, float* centroids,
+size_t shard_b200_kmeans_workspace_bytes(int32_t count, int64_t n);
+int shard_b200_kmeans(const float* x, int32_t count, int64_t n, float max_abs, int32_t n_iter, float* centroids,
                       uint8_t* idx_u8, void* workspace, size_t workspace_bytes, void* stream);
 
 /*

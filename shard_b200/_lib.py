@@ -81,8 +81,8 @@ _SIGNATURES = {
     "shard_b200_int4_pack": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
     "shard_b200_v_hadamard_normalise": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_int32,
                                                   C.c_void_p, C.c_void_p, C.c_void_p]),
-    "shard_b200_kmeans_workspace_bytes": (C.c_size_t, [C.c_int64]),
-    "shard_b200_kmeans": (C.c_int, [C.c_void_p, C.c_int64, C.c_float, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,
+    "shard_b200_kmeans_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int64]),
+    "shard_b200_kmeans": (C.c_int, [C.c_void_p, C.c_int32, C.c_int64, C.c_float, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,
                                     C.c_size_t, C.c_void_p]),
     "shard_b200_eigh_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32, C.c_int32]),
     "shard_b200_eigh": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p,

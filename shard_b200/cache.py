@@ -34,6 +34,11 @@ KERNEL_MAX_RANK = 192
 EIGH_GROUP = 7
 
 
+# sub-vectors whose k-means run side by side: layers of up to 8K tokens share launches, which a single
+# short layer leaves mostly empty
+KMEANS_POINTS = 16 << 20
+
+
 def gram_matrix(flat, mean):
     """(flat - mean)^T (flat - mean) of the rows of `flat` (n, p), fp32."""
     xc = flat - mean
@@ -509,8 +514,8 @@ class Cache(HFCache):
             side.wait_event(done)
             with torch.cuda.stream(side):
                 solved = LeadingEigenpairs(gram, rank)
-            vparts = [self._compress_v(self.layers[li]._values[0, :, start:end, :], init_rows=init_rows)
-                      for li in range(bounds[g], bounds[g + 1])]
+            vparts = self._compress_v_layers([self.layers[li]._values[0, :, start:end, :]
+                                              for li in range(bounds[g], bounds[g + 1])], init_rows=init_rows)
             if g + 1 < n_groups:
                 ready = covariances(g + 1)
             with torch.cuda.stream(side):
@@ -580,17 +585,32 @@ class Cache(HFCache):
 
     def _compress_v(self, v_mid, init_centroids=None, init_rows=None):
         """Hadamard-rotate, normalise per channel and vector-quantise 4-channel groups
-        (reference: src/shard/cache.py:398-404, 41-52).  v_mid: (nkv, n, hd) fp16 view."""
-        x, ch_max = ops.v_hadamard_normalise(v_mid)
-        flat = x.view(-1, self._v_vq_group_size)
-        if init_centroids is None and init_rows is not None:
-            init_centroids = flat[init_rows]
-        # the data is normalised by the channels' largest magnitudes
-        centroids, idx_u8 = kmeans(flat, self._v_vq_codebook_size, n_iter=30, init=init_centroids, max_abs=1.0)
-        nkv, n, hd = v_mid.shape
-        return {"centroids": centroids.half(), "packed": idx_u8, "ch_maxabs": ch_max.half(),
-                "shape": (nkv, n, hd), "group_size": self._v_vq_group_size, "bits": 8,
-                "n_orig": idx_u8.numel()}
+        (reference: src/shard/cache.py:398-404, 41-52).  v_mid: (nkv, n, hd) fp16 view; `init_rows` are the
+        sub-vectors to start from if the caller has drawn them (`initial_rows`)."""
+        return self._compress_v_layers([v_mid], init_centroids, init_rows)[0]
+
+    def _compress_v_layers(self, v_mids, init_centroids=None, init_rows=None):
+        """`_compress_v` of several layers; short prompts' layers go through k-means side by side."""
+        nkv, n, hd = v_mids[0].shape
+        gs = self._v_vq_group_size
+        n_sub = nkv * n * (hd // gs)
+        side_by_side = max(1, min(len(v_mids), KMEANS_POINTS // n_sub))
+        parts = []
+        for i in range(0, len(v_mids), side_by_side):
+            vs = v_mids[i:i + side_by_side]
+            x = torch.empty(len(vs), n_sub, gs, dtype=torch.float32, device=vs[0].device)
+            ch_max = [ops.v_hadamard_normalise(v, out=x[j])[1].half() for j, v in enumerate(vs)]
+            if init_centroids is not None:
+                centroids = init_centroids.to(x.device, torch.float32).clone().unsqueeze(0)
+            else:
+                if init_rows is None:
+                    init_rows = initial_rows(n_sub, self._v_vq_codebook_size, x.device)
+                centroids = x[:, init_rows].contiguous()
+            # the data is normalised by the channels' largest magnitudes
+            idx = ops.kmeans_lloyd(x, centroids, 30, 1.0)
+            parts += [{"centroids": centroids[j].half(), "packed": idx[j], "ch_maxabs": ch_max[j], "shape": (nkv, n, hd),
+                       "group_size": gs, "bits": 8, "n_orig": n_sub} for j in range(len(vs))]
+        return parts
 
     def _build_gpu_format(self, layer, k, v, sink_k, sink_v, win_k, win_v, n_comp, batch, start):
         """Assemble the per-layer tensor dictionary (reference: src/shard/cache.py:406-460)

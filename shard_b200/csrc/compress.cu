@@ -144,25 +144,68 @@ __global__ void int4_pack_kernel(const int8_t* __restrict__ q, int64_t n_values,
 // ---------------------------------------------------------------------------
 // V: Hadamard + per-channel max-abs normalisation
 // ---------------------------------------------------------------------------
-// pass 1: x = H128(v) / sqrt(128); ch_max = max_t |x|   (uint atomicMax on non-negative floats)
-__global__ void __launch_bounds__(256) v_rotate_kernel(const __half* __restrict__ v, int64_t head_stride,
-                                                       int64_t tok_stride, int nkv, int n,
-                                                       float* __restrict__ x, uint32_t* __restrict__ ch_max) {
-  const int lane = threadIdx.x & 31;
-  const int kv = blockIdx.y;
-  float am[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < n; t += gridDim.x * (blockDim.x >> 5)) {
-    const uint2 raw = *reinterpret_cast<const uint2*>(v + kv * head_stride + (int64_t)t * tok_stride + 4 * lane);
-    const __half2 h01 = *reinterpret_cast<const __half2*>(&raw.x);
-    const __half2 h23 = *reinterpret_cast<const __half2*>(&raw.y);
-    float y[4] = {__low2float(h01), __high2float(h01), __low2float(h23), __high2float(h23)};
-    fwht128_lane4(y, lane);
+// Bound: memory traffic.  The rotated values are computed twice -- pass 1 reads the fp16 values and keeps
+// only the channels' maxima, pass 2 reads them again and writes the normalised fp32 result -- because
+// writing them out and reading them back costs more than the butterfly.  A row is held by 8 lanes, 16
+// channels each: stages 1..8 of the butterfly inside a lane, 16..64 by shuffle (12 shuffles a row; with
+// 4 channels a lane it was 20, and the pass was bound by them).
+// 32K tokens x 8 heads: 295 us with the rotated values written by pass 1 and 4-channel lanes, see the
+// launch function for the figure of this form.
+//
+// H128(v) / sqrt(128) of the lane's 16 channels of one row (bit-identical to the stage-by-stage form)
+__device__ __forceinline__ void v_rotate16(const __half* __restrict__ row, int sub, float (&y)[16]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { y[i] = __fdiv_rn(y[i], SQRT_HD); am[i] = fmaxf(am[i], fabsf(y[i])); }
-    *reinterpret_cast<float4*>(x + ((size_t)kv * n + t) * HD + 4 * lane) = make_float4(y[0], y[1], y[2], y[3]);
+  for (int i = 0; i < 4; ++i) {
+    const uint2 raw = reinterpret_cast<const uint2*>(row + 16 * sub)[i];
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+    y[4 * i] = a.x; y[4 * i + 1] = a.y; y[4 * i + 2] = b.x; y[4 * i + 3] = b.y;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) atomicMax(ch_max + kv * HD + 4 * lane + i, __float_as_uint(am[i]));
+  for (int h = 1; h < 16; h <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (!(i & h)) { const float a = y[i], b = y[i + h]; y[i] = __fadd_rn(a, b); y[i + h] = __fsub_rn(a, b); }
+    }
+  }
+#pragma unroll
+  for (int bit = 1; bit < 8; bit <<= 1) {
+    const bool upper = (sub & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, y[i], bit);
+      y[i] = upper ? __fsub_rn(other, y[i]) : __fadd_rn(y[i], other);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) y[i] = __fdiv_rn(y[i], SQRT_HD);
+}
+
+// pass 1: ch_max = max_t |x|   (uint atomicMax on non-negative floats, one per block and channel)
+__global__ void __launch_bounds__(256) v_channel_max_kernel(const __half* __restrict__ v, int64_t head_stride,
+                                                            int64_t tok_stride, int n, uint32_t* __restrict__ ch_max) {
+  __shared__ uint32_t m_s[HD];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, kv = blockIdx.y;
+  if (threadIdx.x < HD) m_s[threadIdx.x] = 0u;
+  __syncthreads();
+  float am[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) am[i] = 0.f;
+  // (every lane takes part in the shuffles: rows behind the last one repeat it)
+  for (int t0 = (blockIdx.x * 8 + warp) * 4; t0 < n; t0 += gridDim.x * 32) {
+    const int t = min(t0 + (lane >> 3), n - 1);
+    float y[16];
+    v_rotate16(v + kv * head_stride + (int64_t)t * tok_stride, sub, y);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) am[i] = fmaxf(am[i], fabsf(y[i]));
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    am[i] = fmaxf(am[i], __shfl_xor_sync(0xffffffffu, am[i], 8));
+    am[i] = fmaxf(am[i], __shfl_xor_sync(0xffffffffu, am[i], 16));
+    if (lane < 8) atomicMax(&m_s[16 * sub + i], __float_as_uint(am[i]));
+  }
+  __syncthreads();
+  if (threadIdx.x < HD) atomicMax(ch_max + kv * HD + threadIdx.x, m_s[threadIdx.x]);
 }
 
 __global__ void v_clamp_kernel(float* ch_max, int count) {
@@ -170,18 +213,25 @@ __global__ void v_clamp_kernel(float* ch_max, int count) {
   if (i < count) ch_max[i] = fmaxf(ch_max[i], 1e-8f);
 }
 
-// pass 2: x /= ch_max
-__global__ void __launch_bounds__(256) v_normalise_kernel(float* __restrict__ x, const float* __restrict__ ch_max,
-                                                          int nkv, int n) {
-  const size_t total4 = (size_t)nkv * n * (HD / 4);
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total4;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int d4 = (int)(i & 31);
-    const int kv = (int)(i / ((size_t)n * 32));
-    float4 y = reinterpret_cast<float4*>(x)[i];
-    const float4 c = *reinterpret_cast<const float4*>(ch_max + kv * HD + 4 * d4);
-    y.x = __fdiv_rn(y.x, c.x); y.y = __fdiv_rn(y.y, c.y); y.z = __fdiv_rn(y.z, c.z); y.w = __fdiv_rn(y.w, c.w);
-    reinterpret_cast<float4*>(x)[i] = y;
+// pass 2: x = H128(v) / sqrt(128) / ch_max
+__global__ void __launch_bounds__(256) v_normalise_kernel(const __half* __restrict__ v, int64_t head_stride,
+                                                          int64_t tok_stride, int n, const float* __restrict__ ch_max,
+                                                          float* __restrict__ x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, kv = blockIdx.y;
+  float c[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) c[i] = ch_max[kv * HD + 16 * sub + i];
+  for (int t0 = (blockIdx.x * 8 + warp) * 4; t0 < n; t0 += gridDim.x * 32) {
+    const int t = min(t0 + (lane >> 3), n - 1);
+    float y[16];
+    v_rotate16(v + kv * head_stride + (int64_t)t * tok_stride, sub, y);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) y[i] = __fdiv_rn(y[i], c[i]);
+    if (t0 + (lane >> 3) < n) {
+      float4* o = reinterpret_cast<float4*>(x + ((size_t)kv * n + t) * HD + 16 * sub);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
+    }
   }
 }
 
@@ -298,13 +348,11 @@ extern "C" int shard_b200_v_hadamard_normalise(const void* v_f16, int64_t head_s
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(ch_max_out, 0, (size_t)nkv * HD * sizeof(float), st);
   if (e != cudaSuccess) return (int)e;
-  const int bx = capped_blocks((n + 7) / 8, 2);
-  v_rotate_kernel<<<dim3(bx, nkv), 256, 0, st>>>((const __half*)v_f16, head_stride, tok_stride, nkv, n, x_out,
-                                                 (uint32_t*)ch_max_out);
+  const int per_head = capped_blocks((long long)nkv * ((n + 31) / 32), 8) / nkv;   // blocks of 32 rows, eight per SM at most
+  const dim3 grid(per_head > 0 ? per_head : 1, nkv);
+  v_channel_max_kernel<<<grid, 256, 0, st>>>((const __half*)v_f16, head_stride, tok_stride, n, (uint32_t*)ch_max_out);
   v_clamp_kernel<<<(nkv * HD + 255) / 256, 256, 0, st>>>(ch_max_out, nkv * HD);
-  const size_t total4 = (size_t)nkv * n * 32;
-  const int blocks = capped_blocks((long long)((total4 + 255) / 256), 16);
-  v_normalise_kernel<<<blocks, 256, 0, st>>>(x_out, ch_max_out, nkv, n);
+  v_normalise_kernel<<<grid, 256, 0, st>>>((const __half*)v_f16, head_stride, tok_stride, n, ch_max_out, x_out);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }

@@ -31,13 +31,13 @@ namespace shard {
 constexpr int KM_THREADS = 512, KM_WARPS = KM_THREADS / 32;
 constexpr int KM_TILE = 64;                   // points per box: two per lane
 constexpr int KM_MAX_RUN = 8;                 // tiles per run
-constexpr int KM_FLUSH_POINTS = 60000;        // points a CTA books between two flushes: partial sums stay within int32
+constexpr int KM_CTA_POINTS = 60000;          // points a CTA books at most: its partial sums stay within int32
 
 struct KmeansHeader {      // head of the workspace; zero when the first iteration starts
   int done;                // converged: the launches behind it do nothing
   int ticket;              // CTAs that have finished the current iteration
   unsigned int max_bits;   // max |x| (as float bits) if the caller did not name a bound
-  int pad;
+  unsigned int next_run;   // runs handed out in the current iteration
   long long sums[256 * 4]; // fixed point
   int counts[256];
 };
@@ -78,8 +78,26 @@ struct KmeansParams {
   float max_abs;           // bound on |x|, or 0: take h->max_bits
   int bits;
   int run;                 // tiles per run
+  int warp_runs;           // runs a warp takes at most
   int it;
+  size_t ws_stride;        // bytes from one problem's workspace to the next one's (problem = blockIdx.y)
 };
+// the parameters of problem number b of a batch
+__device__ __forceinline__ KmeansParams km_problem(KmeansParams p, int b) {
+  const size_t o = (size_t)b * p.ws_stride;
+  auto at = [&](auto* ptr) { return reinterpret_cast<decltype(ptr)>(reinterpret_cast<unsigned char*>(ptr) + o); };
+  p.x += (size_t)b * p.n;
+  p.centroids += (size_t)b * 256;
+  p.idx += (size_t)b * p.n;
+  p.h = at(p.h);
+  p.cells = at(p.cells);
+  p.totals = at(p.totals);
+  p.xs = at(p.xs);
+  p.perm = at(p.perm);
+  p.boxes = at(p.boxes);
+  p.idx_s = at(p.idx_s);
+  return p;
+}
 
 // distance exactly as the nearest-centroid rule defines it
 __device__ __forceinline__ float km_sq4(float d0, float d1, float d2, float d3) {
@@ -146,20 +164,22 @@ __device__ __forceinline__ unsigned int km_cell(float4 v, float scale, int bits)
   return key;
 }
 
-__global__ void __launch_bounds__(256) kmeans_max_abs_kernel(const float4* __restrict__ x, long long n, unsigned int* out) {
+__global__ void __launch_bounds__(256) kmeans_max_abs_kernel(const __grid_constant__ KmeansParams pp) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
   float m = 0.f;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float4 v = x[i];
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (long long)gridDim.x * blockDim.x) {
+    const float4 v = p.x[i];
     m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
   }
   m = warp_max(m);
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(&p.h->max_bits, __float_as_uint(m));
 }
 
 // Points per cell, then (SCATTER) the points to their places.  Lanes whose points all fall into one
 // cell count together: constant data would otherwise queue up at one counter.
 template <bool SCATTER>
-__global__ void __launch_bounds__(256) kmeans_sort_kernel(const __grid_constant__ KmeansParams p) {
+__global__ void __launch_bounds__(256) kmeans_sort_kernel(const __grid_constant__ KmeansParams pp) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
   const float scale = km_scale(p);
   const int lane = threadIdx.x & 31;
   const long long n_up = (p.n + 31) & ~31ll;
@@ -183,7 +203,10 @@ __global__ void __launch_bounds__(256) kmeans_sort_kernel(const __grid_constant_
   }
 }
 // counters -> places within a block of 1024 cells; the blocks' totals
-__global__ void __launch_bounds__(1024) kmeans_scan_kernel(unsigned int* __restrict__ cells, unsigned int* __restrict__ totals) {
+__global__ void __launch_bounds__(1024) kmeans_scan_kernel(const __grid_constant__ KmeansParams pp, bool of_totals) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
+  unsigned int* cells = of_totals ? p.totals : p.cells;
+  unsigned int* totals = of_totals ? nullptr : p.totals;
   __shared__ unsigned int ws[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned int* c = cells + (size_t)blockIdx.x * 1024 + tid;
@@ -206,7 +229,8 @@ __global__ void __launch_bounds__(1024) kmeans_scan_kernel(unsigned int* __restr
 }
 
 // boxes of the sorted points; the last tile is filled up with its last point
-__global__ void __launch_bounds__(256) kmeans_boxes_kernel(const __grid_constant__ KmeansParams p) {
+__global__ void __launch_bounds__(256) kmeans_boxes_kernel(const __grid_constant__ KmeansParams pp) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
   const int lane = threadIdx.x & 31;
   const long long n_tiles = (p.n + KM_TILE - 1) / KM_TILE;
   for (long long t = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); t < n_tiles; t += (long long)gridDim.x * 8) {
@@ -227,12 +251,14 @@ __global__ void __launch_bounds__(256) kmeans_boxes_kernel(const __grid_constant
   }
 }
 
-__global__ void __launch_bounds__(256) kmeans_unsort_kernel(const __grid_constant__ KmeansParams p) {
+__global__ void __launch_bounds__(256) kmeans_unsort_kernel(const __grid_constant__ KmeansParams pp) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (long long)gridDim.x * blockDim.x)
     p.idx[p.perm[i]] = p.idx_s[i];
 }
 
-__global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const __grid_constant__ KmeansParams p) {
+__global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const __grid_constant__ KmeansParams pp) {
+  const KmeansParams p = km_problem(pp, blockIdx.y);
   __shared__ float4 c_s[256];
   __shared__ int acc_s[256 * 9];                               // high and low halves of the sums' changes, count's change
   __shared__ uint8_t run_s[KM_WARPS][256];                     // survivors of the run test, ascending
@@ -240,29 +266,13 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
   __shared__ int last_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < 256 * 9; i += KM_THREADS) acc_s[i] = 0;
-  const float qscale = km_scale(p) * 1073741824.f;             // fixed point: 2^30 per unit of scaled data
   griddep_launch();
   griddep_wait();                                              // the centroids of the iteration before
   if (__ldcg(&p.h->done)) return;                              // (uniform over the grid: set by an earlier launch)
+  const float qscale = km_scale(p) * 1073741824.f;             // fixed point: 2^30 per unit of scaled data
   if (tid < 256) c_s[tid] = __ldcg(p.centroids + tid);
   __syncthreads();
 
-  auto flush = [&]() {
-    __syncthreads();
-    for (int i = tid; i < 256 * 4; i += KM_THREADS) {
-      int* a = acc_s + (i >> 2) * 9 + (i & 3);
-      const long long v = (long long)a[0] * 32768 + a[4];
-      if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&p.h->sums[i]), (unsigned long long)v);
-      a[0] = 0;
-      a[4] = 0;
-    }
-    if (tid < 256) {
-      const int c = acc_s[tid * 9 + 8];
-      if (c) atomicAdd(&p.h->counts[tid], c);
-      acc_s[tid * 9 + 8] = 0;
-    }
-    __syncthreads();
-  };
   // Books the lanes' points with `go`: added to centroid k (sign 1) or taken off it (-1).  A few lanes
   // add one by one; more are first summed per centroid (sorted points: a warp knows two or three).
   auto book = [&](float4 pt, int k, bool go, int sign) {
@@ -302,15 +312,22 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
 
   const long long n_tiles = (p.n + KM_TILE - 1) / KM_TILE;
   const long long n_runs = (n_tiles + p.run - 1) / p.run;
-  const long long n_warps = (long long)gridDim.x * KM_WARPS;
-  const long long rounds = (n_runs + n_warps - 1) / n_warps;   // the same for every warp of the grid
-  const int flush_rounds = max(1, KM_FLUSH_POINTS / (KM_WARPS * p.run * KM_TILE));
   const float inf = __int_as_float(0x7f800000);
-  for (long long r = 0; r < rounds; ++r) {
-    const long long run = r * n_warps + (long long)blockIdx.x * KM_WARPS + warp;
+  // Runs are handed out one at a time (their work differs, and some SMs may be busy with another
+  // stream's kernels); the next one is asked for while the current one is worked on.
+  auto ask = [&]() {
+    unsigned int v = 0;
+    if (lane == 0) v = atomicAdd(&p.h->next_run, 1u);
+    return v;
+  };
+  unsigned int asked = ask();
+  for (int quota = p.warp_runs; quota > 0; --quota) {
+    const long long run = __shfl_sync(0xffffffffu, asked, 0);
+    if (run >= n_runs) break;
+    if (quota > 1) asked = ask();
     const long long t_lo = run * p.run;
     const int nt = (int)min((long long)p.run, n_tiles - t_lo);
-    if (nt > 0) {
+    {
       // ---- the run's box against all centroids ---------------------------------------------------
       const float4* bx = p.boxes + 2 * t_lo;
       const float4 my_lo = bx[2 * min(lane, nt - 1)], my_hi = bx[2 * min(lane, nt - 1) + 1];   // lane j < nt: box of tile j
@@ -403,23 +420,33 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
         const bool ch0 = live0 && (p.it == 0 || arg0 != old0), ch1 = live1 && (p.it == 0 || arg1 != old1);
         if (ch0) p.idx_s[i0] = (uint8_t)arg0;
         if (ch1) p.idx_s[i1] = (uint8_t)arg1;
-        book(p0, arg0, ch0, 1);
-        book(p1, arg1, ch1, 1);
-        if (p.it > 0) {
-          book(p0, old0, ch0, -1);
-          book(p1, old1, ch1, -1);
+        if (__any_sync(0xffffffffu, ch0 || ch1)) {
+          book(p0, arg0, ch0, 1);
+          book(p1, arg1, ch1, 1);
+          if (p.it > 0) {
+            book(p0, old0, ch0, -1);
+            book(p1, old1, ch1, -1);
+          }
         }
         __syncwarp();
       }
     }
-    if ((r + 1) % flush_rounds == 0 && r + 1 < rounds) flush();
   }
-  flush();
+  __syncthreads();
+  for (int i = tid; i < 256 * 4; i += KM_THREADS) {
+    const int* a = acc_s + (i >> 2) * 9 + (i & 3);
+    const long long v = (long long)a[0] * 32768 + a[4];
+    if (v) atomicAdd(reinterpret_cast<unsigned long long*>(&p.h->sums[i]), (unsigned long long)v);
+  }
+  if (tid < 256) {
+    const int c = acc_s[tid * 9 + 8];
+    if (c) atomicAdd(&p.h->counts[tid], c);
+  }
   __threadfence();
   __syncthreads();
   if (tid == 0) {
     const int last = atomicAdd(&p.h->ticket, 1) == (int)gridDim.x - 1;
-    if (last) atomicExch(&p.h->ticket, 0);
+    if (last) { atomicExch(&p.h->ticket, 0); atomicExch(&p.h->next_run, 0u); }
     last_s = last;
   }
   __syncthreads();
@@ -447,17 +474,19 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
 
 using namespace shard;
 
-extern "C" size_t shard_b200_kmeans_workspace_bytes(int64_t n) {
-  if (n < 1 || n >= (1ll << 31)) return 0;
-  return km_layout(n).bytes;
+extern "C" size_t shard_b200_kmeans_workspace_bytes(int32_t count, int64_t n) {
+  if (count < 1 || count > 65535 || n < 1 || n >= (1ll << 31)) return 0;
+  return km_layout(n).bytes * (size_t)count;
 }
 
-extern "C" int shard_b200_kmeans(const float* x, int64_t n, float max_abs, int32_t n_iter, float* centroids, uint8_t* idx_u8,
-                                 void* workspace, size_t workspace_bytes, void* stream) {
-  if (!x || !centroids || !idx_u8 || !workspace || n < 1 || n >= (1ll << 31) || n_iter < 1 || !(max_abs >= 0.f)) return SHARD_E_ARG;
-  const KmeansLayout l = km_layout(n);
-  if (workspace_bytes < l.bytes) return SHARD_E_WORKSPACE;
+extern "C" int shard_b200_kmeans(const float* x, int32_t count, int64_t n, float max_abs, int32_t n_iter, float* centroids,
+                                 uint8_t* idx_u8, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!x || !centroids || !idx_u8 || !workspace || n_iter < 1 || !(max_abs >= 0.f)) return SHARD_E_ARG;
+  const size_t need = shard_b200_kmeans_workspace_bytes(count, n);
+  if (need == 0) return SHARD_E_ARG;
+  if (workspace_bytes < need) return SHARD_E_WORKSPACE;
   if (((uintptr_t)x | (uintptr_t)centroids | (uintptr_t)workspace) & 15) return SHARD_E_ALIGN;
+  const KmeansLayout l = km_layout(n);
   cudaStream_t st = (cudaStream_t)stream;
   unsigned char* ws = (unsigned char*)workspace;
   KmeansParams p{};
@@ -474,28 +503,35 @@ extern "C" int shard_b200_kmeans(const float* x, int64_t n, float max_abs, int32
   p.idx_s = ws + l.idx;
   p.max_abs = max_abs;
   p.bits = l.bits;
-  cudaError_t e = cudaMemsetAsync(ws, 0, l.xs, st);            // header, counters, totals
+  p.ws_stride = l.bytes;
+  // header, counters, totals
+  cudaError_t e = cudaMemset2DAsync(ws, l.bytes, 0, l.xs, count, st);
   if (e != cudaSuccess) return (int)e;
-  const int wide = capped_blocks((n + 255) / 256, 8);
-  if (max_abs == 0.f) kmeans_max_abs_kernel<<<wide, 256, 0, st>>>(p.x, n, &p.h->max_bits);
-  const int n_blocks = 1 << (4 * l.bits - 10);
-  kmeans_sort_kernel<false><<<wide, 256, 0, st>>>(p);
-  kmeans_scan_kernel<<<n_blocks, 1024, 0, st>>>(p.cells, p.totals);
-  kmeans_scan_kernel<<<1, 1024, 0, st>>>(p.totals, nullptr);
-  kmeans_sort_kernel<true><<<wide, 256, 0, st>>>(p);
+  const int wide = capped_blocks((n + 255) / 256, count > 4 ? 2 : 8);
+  const dim3 g_wide(wide, count);
+  if (max_abs == 0.f) kmeans_max_abs_kernel<<<g_wide, 256, 0, st>>>(p);
+  kmeans_sort_kernel<false><<<g_wide, 256, 0, st>>>(p);
+  kmeans_scan_kernel<<<dim3(1 << (4 * l.bits - 10), count), 1024, 0, st>>>(p, false);
+  kmeans_scan_kernel<<<dim3(1, count), 1024, 0, st>>>(p, true);
+  kmeans_sort_kernel<true><<<g_wide, 256, 0, st>>>(p);
   const long long tiles = (n + KM_TILE - 1) / KM_TILE;
-  kmeans_boxes_kernel<<<capped_blocks((tiles + 7) / 8, 8), 256, 0, st>>>(p);
+  kmeans_boxes_kernel<<<dim3(capped_blocks((tiles + 7) / 8, 8), count), 256, 0, st>>>(p);
   // Longer runs share the test against all centroids (a third of a tile's work at run = 1), shorter
-  // ones give every warp of the machine work: the longest that still does.
+  // ones give every warp of the machine work: the longest that still leaves each two runs.
   const int sms = sm_count() > 0 ? sm_count() : 1;
   p.run = 1;
-  while (p.run < KM_MAX_RUN && tiles / (2 * p.run) >= (long long)sms * 2 * KM_WARPS) p.run *= 2;
+  while (p.run < KM_MAX_RUN && tiles * count / (2 * p.run) >= (long long)sms * 2 * KM_WARPS * 2) p.run *= 2;
   const long long runs = (tiles + p.run - 1) / p.run;
-  const int blocks = capped_blocks((runs + KM_WARPS - 1) / KM_WARPS, 2);
+  p.warp_runs = KM_CTA_POINTS / (KM_WARPS * p.run * KM_TILE);
+  // two CTAs per SM over all problems, but never fewer than the runs need at warp_runs each
+  long long blocks = (2ll * sms + count - 1) / count;
+  const long long most = (runs + KM_WARPS - 1) / KM_WARPS, least = (runs + KM_WARPS * p.warp_runs - 1) / ((long long)KM_WARPS * p.warp_runs);
+  if (blocks > most) blocks = most;
+  if (blocks < least) blocks = least;
   for (int it = 0; it < n_iter; ++it) {
     p.it = it;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
+    cfg.gridDim = dim3((unsigned int)blocks, count);
     cfg.blockDim = dim3(KM_THREADS);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -506,7 +542,7 @@ extern "C" int shard_b200_kmeans(const float* x, int64_t n, float max_abs, int32
     e = cudaLaunchKernelEx(&cfg, kmeans_iteration_kernel, p);
     if (e != cudaSuccess) return (int)e;
   }
-  kmeans_unsort_kernel<<<wide, 256, 0, st>>>(p);
+  kmeans_unsort_kernel<<<g_wide, 256, 0, st>>>(p);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }

@@ -136,13 +136,16 @@ def int4_pack(x):
     return out
 
 
-def v_hadamard_normalise(v):
-    """v: (nkv, n, 128) fp16 view -> (x (nkv, n, 128) fp32 = H(v)/ch_max, ch_max (nkv, 128) fp32)."""
+def v_hadamard_normalise(v, out=None):
+    """v: (nkv, n, 128) fp16 view -> (x (nkv, n, 128) fp32 = H(v)/ch_max, ch_max (nkv, 128) fp32).
+    `out`: a contiguous tensor to write x into."""
     require_cuda(v)
     if v.dtype != torch.float16 or v.stride(-1) != 1:
         raise _lib.ShardError("v_hadamard_normalise expects fp16 values with a contiguous head dimension")
     nkv, n, _ = v.shape
-    x = torch.empty(nkv, n, HD, dtype=torch.float32, device=v.device)
+    x = torch.empty(nkv, n, HD, dtype=torch.float32, device=v.device) if out is None else _c(out, torch.float32)
+    if x.numel() != nkv * n * HD:
+        raise _lib.ShardError("out must hold nkv * n * 128 values")
     ch = torch.empty(nkv, HD, dtype=torch.float32, device=v.device)
     check(_lib.load().shard_b200_v_hadamard_normalise(ptr(v), v.stride(0), v.stride(1), nkv, n, ptr(x),
                                                       ptr(ch), cur_stream()), "v_hadamard_normalise")
@@ -200,17 +203,21 @@ def eigh_top(a, rank):
 
 def kmeans_lloyd(x, centroids, n_iter, max_abs=0.0):
     """`n_iter` Lloyd iterations over the rows of x (N, 4); `centroids` (256, 4) fp32 is updated in place.
-    Returns the u8 assignment of the last iteration (made against the centroids before it).
+    Returns the u8 assignment of the last iteration (made against the centroids before it).  A leading
+    dimension, x (count, N, 4) and centroids (count, 256, 4), runs independent sets side by side.
     `max_abs`: a bound on |x|, 0 if not known."""
     require_cuda(x, centroids)
-    n = x.shape[0]
-    if x.shape[1] != 4 or tuple(centroids.shape) != (256, 4):
+    n = x.shape[-2]
+    count = x.shape[0] if x.dim() == 3 else 1
+    if x.shape[-1] != 4 or tuple(centroids.shape) != (*x.shape[:-2], 256, 4):
         raise _lib.ShardError("kmeans supports 4-dim sub-vectors and a 256-entry codebook")
     lib = _lib.load()
-    wsb = lib.shard_b200_kmeans_workspace_bytes(n)
+    wsb = lib.shard_b200_kmeans_workspace_bytes(count, n)
+    if wsb == 0:
+        raise _lib.ShardError(f"kmeans supports 1 <= n < 2**31 points (got {n})")
     ws = torch.empty(wsb, dtype=torch.uint8, device=x.device)
-    u8 = torch.empty(n, dtype=torch.uint8, device=x.device)
-    check(lib.shard_b200_kmeans(ptr(_c(x, torch.float32)), n, float(max_abs), n_iter, ptr(_c(centroids, torch.float32)),
+    u8 = torch.empty(x.shape[:-1], dtype=torch.uint8, device=x.device)
+    check(lib.shard_b200_kmeans(ptr(_c(x, torch.float32)), count, n, float(max_abs), n_iter, ptr(_c(centroids, torch.float32)),
                                 ptr(u8), ptr(ws), wsb, cur_stream()), "kmeans")
     return u8
 

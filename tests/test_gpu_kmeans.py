@@ -53,3 +53,14 @@ def test_kmeans_stops_when_settled():
     c = x[:256].clone()
     idx = ops.kmeans_lloyd(x, c, 30)
     assert (c - x[:256]).abs().max() < 2e-9 and torch.equal(idx, ops.vq_assign(x, c, want_i64=False)[0])
+
+
+def test_kmeans_sets_side_by_side():
+    from shard_b200 import ops
+    x = torch.stack([_data(70001, k) for k in ("plain", "narrow", "ties")]) * torch.tensor([1.0, 0.5, 0.25], device="cuda").view(3, 1, 1)
+    cent = x[:, 1000:1256].contiguous()
+    together = cent.clone()
+    idx = ops.kmeans_lloyd(x, together, 8, 4.0)
+    for i in range(3):
+        alone = cent[i].clone()
+        assert torch.equal(idx[i], ops.kmeans_lloyd(x[i], alone, 8, 4.0)) and torch.equal(alone, together[i])

@@ -339,6 +339,22 @@ int shard_b200_k_project(const float* flat, const float* mean, const float* w, i
                          int32_t keep, float* proj_out, void* workspace, size_t workspace_bytes,
                          void* stream);
 
+/*
+ * int8 quantisation of the PCA basis (src/shard/cache.py:386-391): basis [dim][keep] fp32 with
+ * `row_stride` elements between rows -> basis_q int8 [dim][keep], scale fp16 [keep] (= max|column| / 127,
+ * at least 1e-6 / 127), w fp32 [dim][keep] = basis_q * scale and basis_f16 = fp16(basis_q) * fp16(scale).
+ */
+int shard_b200_k_basis_quantise(const float* basis, int64_t row_stride, int32_t dim, int32_t keep,
+                                int8_t* basis_q_out, void* scale_f16_out, float* w_out,
+                                void* basis_f16_out, void* stream);
+
+/*
+ * The dynamic programme of dp_bit_allocation (src/shard/rope.py:49-84) on the host: bits per group of PCA
+ * components from the groups' variances and sizes.  Host pointers only, no CUDA call.
+ */
+int shard_b200_dp_bit_allocation(const double* group_var_host, const int32_t* group_size_host,
+                                 int32_t n_groups, int32_t total_budget, int32_t* group_bits_host);
+
 /* Scratch bytes for shard_b200_k_quantize_pack. */
 size_t shard_b200_k_quantize_workspace_bytes(int32_t n, int32_t keep);
 

@@ -469,30 +469,27 @@ class Cache(HFCache):
         ev0 = torch.cuda.Event(enable_timing=True)
         ev1 = torch.cuda.Event(enable_timing=True)
         ev0.record()
-        # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
-        n_sub = (end - start) * self._n_kv_heads * (self.head_dim // self._v_vq_group_size)
-        init_rows = initial_rows(n_sub, self._v_vq_codebook_size, k0.device)
         if self._k_pca == "svd_lowrank":
             for li in range(self._num_layers):
                 torch.manual_seed(42 + li)
                 k_full, v_full = self.layers[li]._keys, self.layers[li]._values
                 kpart = self._compress_k(k_full[0, :, start:end, :], start)
-                vpart = self._compress_v(v_full[0, :, start:end, :], init_rows=init_rows)
+                vpart = self._compress_v(v_full[0, :, start:end, :])
                 self._finish_layer(li, kpart, vpart, start, end)
         else:
-            self._compress_side_by_side(start, end, init_rows)
+            self._compress_side_by_side(start, end)
         ev1.record()
         ev1.synchronize()
         self.compress_seconds = ev0.elapsed_time(ev1) / 1e3
         self._compressed = True
 
-    def _compress_side_by_side(self, start, end, init_rows):
+    def _compress_side_by_side(self, start, end):
         """Layers in groups.  The eigensolver of a group's key covariances is a long chain of small steps
         on a few SMs: it runs on a second stream beside the group's value path (k-means) and the next
         group's covariances; the host waits only for the eigenvalues, which decide the bit widths."""
         n_layers = self._num_layers
         main = torch.cuda.current_stream()
-        side = torch.cuda.Stream(main.device)
+        side = torch.cuda.Stream(main.device, priority=-1)     # its few CTAs are placed before k-means' many
         n_groups = -(-n_layers // EIGH_GROUP)
         bounds = [n_layers * g // n_groups for g in range(n_groups + 1)]
 
@@ -508,7 +505,13 @@ class Cache(HFCache):
 
         n, p = end - start, self._per_layer_dim
         rank = min(self._max_rank_k, p, n - 1)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
+            init_rows = initial_rows(n * p // self._v_vq_group_size, self._v_vq_codebook_size, main.device)
+            drawn = side.record_event()
         ready = covariances(0)
+        main.wait_event(drawn)
         for g in range(n_groups):
             layers, gram, done = ready
             side.wait_event(done)
@@ -572,15 +575,12 @@ class Cache(HFCache):
         keep -= keep & 1
         if keep <= 0:
             raise ShardError("bit allocation kept no PCA component")
-        basis = basis[:, :keep].contiguous()
         alloc = alloc[:keep]
-        col_max = basis.abs().max(dim=0).values.clamp(min=1e-6)
-        scale = col_max / 127.0
-        basis_q = (basis / scale).round().clamp(-127, 127).to(torch.int8)
-        w = (basis_q.float() * scale.float()).contiguous()
-        proj = ops.k_project(flat, mean.float().contiguous(), w)
+        basis = basis[:, :keep]
+        basis_q, scale, w, basis_f16 = ops.k_basis_quantise(basis if basis.stride(1) == 1 else basis.contiguous())
+        proj = ops.k_project(flat, mean, w)
         packed, coeff_scale = ops.k_quantize_pack(proj, alloc)
-        return {"k_basis_q": basis_q, "k_scale": scale.half(), "k_mean": mean.half(), "k_alloc": alloc,
+        return {"k_basis_q": basis_q, "k_scale": scale, "k_basis_f16": basis_f16, "k_mean": mean.half(), "k_alloc": alloc,
                 "k_coeffs": packed, "k_coeff_scale": coeff_scale, "k_n_total": n}
 
     def _compress_v(self, v_mid, init_centroids=None, init_rows=None):
@@ -618,7 +618,7 @@ class Cache(HFCache):
         nkv, hd = self._n_kv_heads, self.head_dim
         keep = len(k["k_alloc"])
         ng = hd // v["group_size"]
-        basis_f16 = (k["k_basis_q"].to(torch.float16) * k["k_scale"].to(torch.float16)).contiguous()
+        basis_f16 = k["k_basis_f16"]
         coeff_scale_f16 = k["k_coeff_scale"].half()
         gc = {
             "k_coeffs": k["k_coeffs"],
@@ -628,7 +628,7 @@ class Cache(HFCache):
             "k_basis_scale": k["k_scale"],
             "k_basis_f16": basis_f16,
             "k_mean": k["k_mean"],
-            "k_mean_f16": k["k_mean"].to(torch.float16).contiguous(),
+            "k_mean_f16": k["k_mean"],
             "k_alloc": k["k_alloc"],
             "v_qdata": v,
             "v_packed": v["packed"],

@@ -7,6 +7,8 @@
 // PyTorch code performs them, so that the codes are bit-identical for identical
 // fp32 inputs.  Reductions that decide codes (min, max, max-abs) are
 // order-independent.
+#include <vector>
+
 #include "common.cuh"
 
 namespace shard {
@@ -128,6 +130,36 @@ __global__ void __launch_bounds__(256) kq_pack_kernel(const float* __restrict__ 
       q[e] = (int)v;
     }
     packed[i] = (uint8_t)(((q[0] + 8) & 15) | (((q[1] + 8) & 15) << 4));
+  }
+}
+
+// int8 basis: per column scale = max(max|b|, 1e-6) / 127, code = clamp(rint(b / scale), +-127); and what
+// the projection and the decode kernels take: w = code * scale (fp32) and fp16(code) * fp16(scale).
+// A block takes 32 columns, 8 rows at a time.
+__global__ void __launch_bounds__(256) k_basis_quantise_kernel(const float* __restrict__ basis, int64_t stride, int dim, int keep,
+                                                               int8_t* __restrict__ basis_q, __half* __restrict__ scale_f16,
+                                                               float* __restrict__ w, __half* __restrict__ basis_f16) {
+  __shared__ float mx[8][32];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), r0 = threadIdx.x >> 5;
+  const bool live = c < keep;
+  float m = 0.f;
+  if (live)
+    for (int r = r0; r < dim; r += 8) m = fmaxf(m, fabsf(basis[(size_t)r * stride + c]));
+  mx[r0][threadIdx.x & 31] = m;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) m = fmaxf(m, mx[i][threadIdx.x & 31]);
+  if (!live) return;
+  const float scale = __fdiv_rn(fmaxf(m, 1e-6f), 127.0f);
+  const __half s16 = __float2half_rn(scale);
+  if (r0 == 0) scale_f16[c] = s16;
+  for (int r = r0; r < dim; r += 8) {
+    float q = rintf(__fdiv_rn(basis[(size_t)r * stride + c], scale));
+    q = fminf(fmaxf(q, -127.f), 127.f);
+    const size_t o = (size_t)r * keep + c;
+    basis_q[o] = (int8_t)(int)q;
+    w[o] = __fmul_rn(q, scale);
+    basis_f16[o] = __hmul(__float2half_rn(q), s16);
   }
 }
 
@@ -326,6 +358,52 @@ extern "C" int shard_b200_k_quantize_pack(const float* proj, const int32_t* allo
   const int blocks = capped_blocks((long long)((total + 255) / 256), 16);
   kq_pack_kernel<<<blocks, 256, 0, st>>>(proj, alloc_bits, n, keep, ws, coeff_scale_out, packed_out);
   SHARD_CHECK_LAUNCH();
+  return SHARD_OK;
+}
+
+extern "C" int shard_b200_k_basis_quantise(const float* basis, int64_t row_stride, int32_t dim, int32_t keep, int8_t* basis_q_out,
+                                           void* scale_f16_out, float* w_out, void* basis_f16_out, void* stream) {
+  if (!basis || !basis_q_out || !scale_f16_out || !w_out || !basis_f16_out || dim < 1 || keep < 1 || row_stride < keep) return SHARD_E_ARG;
+  k_basis_quantise_kernel<<<(keep + 31) / 32, 256, 0, (cudaStream_t)stream>>>(basis, row_stride, dim, keep, basis_q_out,
+                                                                              (__half*)scale_f16_out, w_out, (__half*)basis_f16_out);
+  SHARD_CHECK_LAUNCH();
+  return SHARD_OK;
+}
+
+// Host: the dynamic programme of dp_bit_allocation in double precision, first minimum wins.
+extern "C" int shard_b200_dp_bit_allocation(const double* group_var_host, const int32_t* group_size_host, int32_t n_groups,
+                                            int32_t total_budget, int32_t* group_bits_host) {
+  constexpr int MAX_GROUPS = 64, UNIT = 16;
+  static const int choices[5] = {0, 2, 4, 6, 8};
+  if (!group_var_host || !group_size_host || !group_bits_host || n_groups < 1 || n_groups > MAX_GROUPS || total_budget < 0) return SHARD_E_ARG;
+  const int cap = total_budget / UNIT + 1;
+  const double inf = 1.0 / 0.0;
+  std::vector<double> best((size_t)(n_groups + 1) * (cap + 1), inf);
+  std::vector<int> pick((size_t)(n_groups + 1) * (cap + 1), 0);
+  for (int b = 0; b <= cap; ++b) best[b] = 0.0;
+  auto cost_of = [&](int g, int bits) { return bits == 0 ? 0 : (group_size_host[g] * bits + UNIT - 1) / UNIT; };
+  for (int g = 0; g < n_groups; ++g) {
+    const double* from = best.data() + (size_t)g * (cap + 1);
+    double* to = best.data() + (size_t)(g + 1) * (cap + 1);
+    int* pk = pick.data() + (size_t)(g + 1) * (cap + 1);
+    for (int c = 0; c < 5; ++c) {                       // (choices outside: the order in which a minimum is first met is the same)
+      const int bits = choices[c], cost = cost_of(g, bits);
+      const double err = bits == 0 ? group_var_host[g] * 4.0 : group_var_host[g] / (3.0 * (double)(1 << (2 * bits)));
+      for (int b = cost; b <= cap; ++b) {
+        const double total = from[b - cost] + err;
+        if (total < to[b]) { to[b] = total; pk[b] = bits; }
+      }
+    }
+  }
+  int b = 0;
+  const double* last = best.data() + (size_t)n_groups * (cap + 1);
+  for (int i = 1; i <= cap; ++i)
+    if (last[i] < last[b]) b = i;
+  for (int g = n_groups - 1; g >= 0; --g) {
+    const int bits = pick[(size_t)(g + 1) * (cap + 1) + b];
+    group_bits_host[g] = bits;
+    b -= cost_of(g, bits);
+  }
   return SHARD_OK;
 }
 

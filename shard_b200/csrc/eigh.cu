@@ -9,7 +9,7 @@
 //                          sends its rows of A v and of the next column to all others with st.async
 //                          (distributed shared memory, completion counted on the receivers' mbarriers);
 //                          everything else of a step is recomputed by every CTA from the same numbers.
-//   2. tridiag_values_kernel   eigenvalues by 33-section on Sturm counts, a warp per eigenvalue, fp64;
+//   2. tridiag_values_kernel   eigenvalues by 129-section on Sturm counts, a CTA per eigenvalue, fp64;
 //                          division-free recurrence (one multiply-add of latency per row).
 //   3. tridiag_vectors_kernel  eigenvectors of the tridiagonal matrix by twisted factorisation, fp64,
 //                          thread = vector, one warp from either end.
@@ -418,42 +418,45 @@ __device__ __forceinline__ void eg_rescale(double& a, double& b) {
   b *= f;
 }
 
-// warp = eigenvalue number w (descending); 32 trial points split its interval into 33 per round
-__global__ void __launch_bounds__(256) tridiag_values_kernel(const __grid_constant__ EighParams p) {
+// CTA = eigenvalue number w (descending); 128 trial points, one per thread, split its interval into 129
+// per round.  A step of the recurrence is the latency of one multiply-add; more points per round would
+// save rounds but the fp64 pipes are full at 7 matrices already.
+constexpr int EG_PTS = 128;
+__global__ void __launch_bounds__(EG_PTS) tridiag_values_kernel(const __grid_constant__ EighParams p) {
   __shared__ double2 td[EG_MAX_P];
-  const int m = blockIdx.y, n = p.p, lane = threadIdx.x & 31;
-  const double unscale = eg_load(p, m, td, threadIdx.x, 256);
-  const int w = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (w >= p.rank) return;
+  __shared__ int left[2][EG_PTS / 32];
+  const int m = blockIdx.y, n = p.p, w = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double unscale = eg_load(p, m, td, threadIdx.x, EG_PTS);
   double lo = -1.0, width = 2.0;
-  for (int round = 0; round < 11; ++round) {            // 33^-11: below fp64's resolution of the interval
-    const double step = width / 33.0, x = lo + step * (lane + 1);
+  for (int round = 0; round < 8; ++round) {             // 129^-8: below fp64's resolution of the interval
+    const double step = width / 129.0, x = lo + step * (double)(threadIdx.x + 1);
     double b = 1.0, a = td[0].x - x;                    // p_{i-1}, p_i
     int neg = __double2hiint(a) < 0;
-    int i = 1;
-    for (; i + 8 <= n; i += 8) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const double c = fma(td[i + j].x - x, a, -td[i + j - 1].y * b);
-        neg += (unsigned)(__double2hiint(c) ^ __double2hiint(a)) >> 31;
-        b = a;
-        a = c;
-      }
-      eg_rescale(a, b);
-    }
-    for (; i < n; ++i) {
+    auto row = [&](int i) {
       const double c = fma(td[i].x - x, a, -td[i - 1].y * b);
       neg += (unsigned)(__double2hiint(c) ^ __double2hiint(a)) >> 31;
       b = a;
       a = c;
+    };
+    int i = 1;
+    for (; i + 8 <= n; i += 8) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) row(i + j);
+      eg_rescale(a, b);
     }
-    // neg eigenvalues lie below x; the one sought has n - 1 - w below it
-    const unsigned int left = __ballot_sync(0xffffffffu, neg <= n - 1 - w);
-    const int k = __popc(left);                         // it lies right of the first k points
+    for (; i < n; ++i) row(i);
+    // neg eigenvalues lie below a point; the one sought has n - 1 - w below it, so it lies right of the
+    // first k points
+    const unsigned int bal = __ballot_sync(0xffffffffu, neg <= n - 1 - w);
+    if (lane == 0) left[round & 1][warp] = __popc(bal);
+    __syncthreads();
+    int k = 0;
+#pragma unroll
+    for (int t = 0; t < EG_PTS / 32; ++t) k += left[round & 1][t];
     lo += step * k;
     width = step;
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     const double l = lo + 0.5 * width;
     p.lam[(size_t)m * p.rank + w] = l;                  // of the scaled matrix
     p.eigvals[(size_t)m * p.rank + w] = (float)(l * unscale);
@@ -465,12 +468,22 @@ __global__ void __launch_bounds__(256) tridiag_values_kernel(const __grid_consta
 // row where the two factorisations meet best, z_r = 1, z_i = -(e_i / D+_i) z_{i+1} above it and
 // z_i = -(e_{i-1} / D-_i) z_{i-1} below
 // ---------------------------------------------------------------------------
+// 1 / b to fp64 accuracy: two Newton steps on the hardware's 20-bit estimate
+__device__ __forceinline__ double eg_recip(double b) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(b));
+  r = fma(r, fma(-b, r, 1.0), r);
+  return fma(r, fma(-b, r, 1.0), r);
+}
+
 __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_constant__ EighParams p) {
   __shared__ double2 td[EG_MAX_P];
+  __shared__ double off_s[EG_MAX_P];                    // e_i, scaled like td
   __shared__ double gmin[2][32];
   __shared__ int gat[2][32];
   const int m = blockIdx.y, n = p.p, lane = threadIdx.x & 31, side = threadIdx.x >> 5;
   eg_load(p, m, td, threadIdx.x, 64);
+  for (int i = threadIdx.x; i < n; i += 64) off_s[i] = copysign(sqrt(td[i].y), (double)p.e[(size_t)m * n + i]);
   const int w = blockIdx.x * 32 + lane;
   const double lam = p.lam[(size_t)m * p.rank + min(w, p.rank - 1)];
   const size_t base = ((size_t)m * gridDim.x + blockIdx.x) * n * 32 + lane;
@@ -487,8 +500,8 @@ __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_consta
       const double c = r ? fma(td[row].x - lam, a, -off * b) : td[row].x - lam;
       if (r) b = a;
       a = c;
-      double q = a / b;
-      if (q == 0.0) q = 1e-30;
+      double q = a * eg_recip(b);
+      if (fabs(q) < 1e-30) q = 1e-30;
       out[(size_t)row * 32] = q;
     };
     for (; i + 8 <= n; i += 8) {
@@ -503,7 +516,7 @@ __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_consta
     double best = 1e300;
     int at = 0;
     const int lo = side ? n / 2 : 0, hi = side ? n : n / 2;
-#pragma unroll 4
+#pragma unroll 8
     for (int i = lo; i < hi; ++i) {
       const double g = fabs(dp[(size_t)i * 32] + dm[(size_t)i * 32] - (td[i].x - lam));
       if (g < best) { best = g; at = i; }
@@ -514,20 +527,18 @@ __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_consta
   __syncthreads();
   const int r = gmin[1][lane] < gmin[0][lane] ? gat[1][lane] : gat[0][lane];
   float* z = p.z + base;
-  // signs of e are needed here, and its scale cancels: sqrt(e_i^2) carries the sign of e_i
-  const float* e = p.e + (size_t)m * n;
   double v = 1.0;
   if (side == 0) {
     z[(size_t)r * 32] = 1.f;
-#pragma unroll 4
+#pragma unroll 8
     for (int i = n - 2; i >= 0; --i) {
-      const double f = -copysign(sqrt(td[i].y), (double)e[i]) / dp[(size_t)i * 32];
+      const double f = -off_s[i] * eg_recip(dp[(size_t)i * 32]);
       if (i < r) { v *= f; z[(size_t)i * 32] = (float)v; }
     }
   } else {
-#pragma unroll 4
+#pragma unroll 8
     for (int i = 1; i < n; ++i) {
-      const double f = -copysign(sqrt(td[i - 1].y), (double)e[i - 1]) / dm[(size_t)i * 32];
+      const double f = -off_s[i - 1] * eg_recip(dm[(size_t)i * 32]);
       if (i > r) { v *= f; z[(size_t)i * 32] = (float)v; }
     }
   }
@@ -567,12 +578,8 @@ __global__ void __launch_bounds__(128) eig_back_kernel(const __grid_constant__ E
     for (int j = 0; j < CB; ++j)
       r[j] = (k >= 0 && 128 * (j + 1) > k + 1) ? *reinterpret_cast<const float4*>(refl + (size_t)k * N + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  // the first pair is (n - 2, n - 3): reflector n - 2 is trivial (tau = 0)
-  load(N - 2, a);
-  load(N - 3, b);
-#pragma unroll 1
-  for (int k = N - 2; k >= 0; k -= 2) {
-    const float t1 = __ldg(tau + k), t2 = k >= 1 ? __ldg(tau + k - 1) : 0.f;
+  auto apply = [&](int k, const float4 (&a)[CB], const float4 (&b)[CB]) {
+    const float t1 = k >= 0 ? __ldg(tau + k) : 0.f, t2 = k >= 1 ? __ldg(tau + k - 1) : 0.f;
     float s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
     for (int j = 0; j < CB; ++j) {
@@ -595,8 +602,19 @@ __global__ void __launch_bounds__(128) eig_back_kernel(const __grid_constant__ E
       x[j][2] = fmaf(-s2, b[j].z, fmaf(-s1, a[j].z, x[j][2]));
       x[j][3] = fmaf(-s2, b[j].w, fmaf(-s1, a[j].w, x[j][3]));
     }
-    load(k - 2, a);
-    load(k - 3, b);
+  };
+  // pairs (n - 2, n - 3), ... (reflector n - 2 is trivial: tau = 0); the next pair is on its way while one is applied
+  float4 a2[CB], b2[CB];
+  load(N - 2, a);
+  load(N - 3, b);
+#pragma unroll 1
+  for (int k = N - 2; k >= 0; k -= 4) {
+    load(k - 2, a2);
+    load(k - 3, b2);
+    apply(k, a, b);
+    load(k - 4, a);
+    load(k - 5, b);
+    apply(k - 2, a2, b2);
   }
   float* out = p.basis + (size_t)m * N * p.rank + w;
 #pragma unroll
@@ -649,7 +667,7 @@ static int launch_eigh(const EighParams& p, int count, cudaStream_t st) {
   cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, tridiag_kernel<CB>, p);
   if (e != cudaSuccess) return (int)e;
-  tridiag_values_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);
+  tridiag_values_kernel<<<dim3(p.rank, count), EG_PTS, 0, st>>>(p);
   tridiag_vectors_kernel<<<dim3((p.rank + 31) / 32, count), 64, 0, st>>>(p);
   eig_back_kernel<CB><<<dim3((p.rank + 3) / 4, count), 128, 0, st>>>(p);
   eig_check_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);

@@ -112,6 +112,23 @@ def k_project(flat, mean, w):
     return proj
 
 
+def k_basis_quantise(basis):
+    """int8 codes of a (dim, keep) fp32 basis (any row stride): (basis_q int8, scale fp16 (keep,),
+    w fp32 = basis_q * scale, basis_f16)."""
+    require_cuda(basis)
+    if basis.dtype != torch.float32 or basis.stride(1) != 1:
+        raise _lib.ShardError("k_basis_quantise expects fp32 rows with contiguous columns")
+    dim, keep = basis.shape
+    dev = basis.device
+    q = torch.empty(dim, keep, dtype=torch.int8, device=dev)
+    scale = torch.empty(keep, dtype=torch.float16, device=dev)
+    w = torch.empty(dim, keep, dtype=torch.float32, device=dev)
+    b16 = torch.empty(dim, keep, dtype=torch.float16, device=dev)
+    check(_lib.load().shard_b200_k_basis_quantise(ptr(basis), basis.stride(0), dim, keep, ptr(q), ptr(scale), ptr(w), ptr(b16),
+                                                  cur_stream()), "k_basis_quantise")
+    return q, scale, w, b16
+
+
 def k_quantize_pack(proj, alloc):
     """Two-stage quantisation of projected keys to packed int4; returns (packed u8, coeff_scale fp32)."""
     require_cuda(proj)

@@ -7,7 +7,11 @@ torch expressions of the non-fused read path.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
+
+from . import _lib
 
 
 def rotate_half(x):
@@ -56,15 +60,12 @@ def get_rope_inv_freq(model):
 
 
 _GROUP = 64                 # components share a bit width in groups of 64
-_BIT_CHOICES = (0, 2, 4, 6, 8)
-_DROP_PENALTY = 4.0         # a dropped group is charged 4x its variance
-_COST_UNIT = 16             # budget is counted in units of 16 bits
 
 
 def dp_bit_allocation(variances, total_budget):
     """Bits per PCA component by dynamic programming (reference: rope.py:49-84).
 
-    Minimises sum_g err(g, bits_g) subject to sum_g ceil(size_g * bits_g / 16)
+    The programme itself runs in the library (host code).  Minimises sum_g err(g, bits_g) subject to sum_g ceil(size_g * bits_g / 16)
     <= total_budget // 16 + 1, with err = 4 * var for 0 bits and
     var / (3 * 4**bits) otherwise.  Ties keep the first (smallest) option.
     """
@@ -73,30 +74,10 @@ def dp_bit_allocation(variances, total_budget):
     n_groups = (d + _GROUP - 1) // _GROUP
     sizes = [min(_GROUP, d - g * _GROUP) for g in range(n_groups)]
     gvar = [v[g * _GROUP: g * _GROUP + sizes[g]].sum().item() for g in range(n_groups)]
-    cap = total_budget // _COST_UNIT + 1
-    inf = float("inf")
-    best = [[inf] * (cap + 1) for _ in range(n_groups + 1)]
-    pick = [[0] * (cap + 1) for _ in range(n_groups + 1)]
-    best[0] = [0.0] * (cap + 1)
-
-    def cost_of(g, bits):
-        return 0 if bits == 0 else (sizes[g] * bits + _COST_UNIT - 1) // _COST_UNIT
-
+    bits = (C.c_int32 * n_groups)()
+    _lib.check(_lib.load().shard_b200_dp_bit_allocation((C.c_double * n_groups)(*gvar), (C.c_int32 * n_groups)(*sizes), n_groups,
+                                                        total_budget, bits), "dp_bit_allocation")
+    alloc = []
     for g in range(n_groups):
-        for b in range(cap + 1):
-            for bits in _BIT_CHOICES:
-                c = cost_of(g, bits)
-                if c > b:
-                    continue
-                err = gvar[g] * _DROP_PENALTY if bits == 0 else gvar[g] / (3.0 * (1 << (2 * bits)))
-                total = best[g][b - c] + err
-                if total < best[g + 1][b]:
-                    best[g + 1][b] = total
-                    pick[g + 1][b] = bits
-    b = min(range(cap + 1), key=lambda i: best[n_groups][i])
-    alloc = [0] * d
-    for g in range(n_groups - 1, -1, -1):
-        bits = pick[g + 1][b]
-        alloc[g * _GROUP: g * _GROUP + sizes[g]] = [bits] * sizes[g]
-        b -= cost_of(g, bits)
+        alloc += [bits[g]] * sizes[g]
     return alloc

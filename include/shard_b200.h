@@ -306,6 +306,22 @@ int shard_b200_read_back(const ShardSeq* seq_host, const ShardDecodeShape* shape
                          int* status_dev, void* stream);
 
 /*
+ * Causal attention of `n_tok` new query tokens over a compressed layer whose newest rows are those tokens
+ * (already appended: the last n_tok of the streamed rows, or of the fp16 decode buffer): the read-back of
+ * the layer plus stock attention in the reference (src/shard/attention.py:357-362, src/shard/cache.py:87-124).
+ * Query token j of head h starts at element h * q_head_stride + j * q_tok_stride of q (channels
+ * contiguous, strides multiples of 4) and sees every row but the new tokens behind it.
+ * out: fp16 [n_tok][n_q][128].  `shape` as for shard_b200_read_back (plus n_q; append is ignored).
+ * workspace: shard_b200_multiquery_workspace_bytes bytes, 128-byte aligned: the layer as fp16 tile
+ * images (64 KB per 128 rows and KV head) and partial results.
+ */
+size_t shard_b200_multiquery_workspace_bytes(const ShardDecodeShape* shape_host, int32_t n_tok);
+int shard_b200_multiquery_attn(const ShardSeq* seq_host, const ShardDecodeShape* shape_host, const void* q_f16,
+                               int64_t q_head_stride, int64_t q_tok_stride, int32_t n_tok, const float* inv_freq,
+                               const float* codebook, int32_t compress_start, void* out_f16, void* workspace,
+                               size_t workspace_bytes, int* status_dev, void* stream);
+
+/*
  * fp16 K/V [nkv][n_stream][128] of the streamed tokens: CacheLayer._dequant_stream
  * (src/shard/cache.py:243-279) + dequantize_per_token (streaming.py:74-79).  Used by
  * the non-fused read path only.
@@ -324,6 +340,41 @@ int shard_b200_stream_dequant(const uint8_t* idx, const void* norm_f16, const fl
 int shard_b200_undo_rope(const void* k_f16, int64_t head_stride, int64_t tok_stride, int32_t nkv,
                          int32_t n, int32_t pos_start, const float* inv_freq, float* flat_out,
                          void* stream);
+
+/*
+ * shard_b200_undo_rope plus what the PCA fit needs of its result: the column means (fp32 and, if not
+ * NULL, fp16) and the Gram matrix (flat - mean)^T (flat - mean), fp32 [dim][dim] with dim = nkv*128, at
+ * fp32 accuracy on the tensor cores.  flat_out and workspace 16-byte aligned; workspace:
+ * shard_b200_k_covariance_workspace_bytes bytes (0: sizes not supported, nkv <= 32); its second 32-bit word is
+ * set to 1 if a bounded wait gave up.
+ */
+size_t shard_b200_k_covariance_workspace_bytes(int32_t nkv, int32_t n);
+int shard_b200_k_covariance(const void* k_f16, int64_t head_stride, int64_t tok_stride, int32_t nkv, int32_t n,
+                            int32_t pos_start, const float* inv_freq, float* flat_out, float* mean_out,
+                            void* mean_f16_out, float* gram_out, void* workspace, size_t workspace_bytes,
+                            void* stream);
+
+/*
+ * Everything behind the PCA fit of one layer's keys in one call: shard_b200_k_basis_quantise of basis
+ * [nkv*128][keep], shard_b200_k_project, shard_b200_k_quantize_pack with alloc_bits_host [keep] (a HOST
+ * array), the coefficient scales as fp16, and -- if wprep_out is not NULL, keep a multiple of 32 --
+ * shard_b200_decode_prepare.  workspace: shard_b200_k_encode_workspace_bytes bytes, 16-byte aligned.
+ */
+size_t shard_b200_k_encode_workspace_bytes(int32_t nkv, int32_t n, int32_t keep);
+int shard_b200_k_encode(const float* flat, const float* mean, const void* mean_f16, const float* basis,
+                        int64_t basis_row_stride, const int32_t* alloc_bits_host, int32_t n, int32_t nkv,
+                        int32_t keep, int8_t* basis_q_out, void* scale_f16_out, void* basis_f16_out,
+                        uint8_t* packed_out, void* coeff_scale_f16_out, void* wprep_out, void* workspace,
+                        size_t workspace_bytes, void* stream);
+
+/*
+ * The fp16 tokens a compressed layer keeps at both ends of the prompt (src/shard/cache.py:352-356):
+ * out = [sink K | sink V | window K | window V], fp16 [nkv][rows][128] each; sink rows are tokens
+ * 0 .. n_sink-1, window rows win_start .. win_start + n_win - 1.  Strides in elements.
+ */
+int shard_b200_kv_ends(const void* k_f16, const void* v_f16, int64_t k_head_stride, int64_t k_tok_stride,
+                       int64_t v_head_stride, int64_t v_tok_stride, int32_t nkv, int32_t n_sink, int32_t n_win,
+                       int32_t win_start, void* out_f16, void* stream);
 
 /*
  * proj[n][keep] = (flat - mean) @ w: the PCA projection of Cache._compress_k

@@ -16,8 +16,10 @@ from ._lib import ShardSeq, ptr
 from .streaming import get_codebook
 
 GQA = 4
-# a forward over more new tokens than this after compression takes the dequantised path (one launch
-# per query token would no longer pay)
+# from this many new tokens on, one read-back of the layer serves all of them; below, a decode launch per
+# query token is cheaper
+MIN_MULTIQUERY_TOKENS = 3
+# a forward over more new tokens than this after compression takes the dequantised path
 MAX_FUSED_QUERY_TOKENS = 256
 
 
@@ -86,6 +88,28 @@ def row_tensors(gc, nkv, hd):
         dk, dv = gc["decode_k"], gc["decode_v"] = dk.contiguous(), dv.contiguous()
     n_dec = dk.shape[2]
     return dk, dv, n_dec, dk.stride(1) // hd if nkv > 1 else n_dec
+
+
+def layer_record(gc, nkv, hd, dev):
+    """ShardSeq, ShardDecodeShape and number of rows of a whole layer: what reads all of it takes."""
+    seq = _seq_record(gc, dev)
+    dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd)
+    n_comp, n_stream = gc["n_compress"], gc.get("stream_n", 0)
+    n_sink, n_win = gc["sink_k"].shape[2], gc["win_k"].shape[2]
+    shape = ops.make_shape(GQA * nkv, nkv, gc["k_rank_kernel"], n_comp, 0, n_comp, n_sink, n_win, n_stream, 0, n_dec=n_dec)
+    shape.dec_cap = dec_cap
+    if n_dec:
+        seq.dec_k, seq.dec_v = dk.data_ptr(), dv.data_ptr()
+    return seq, shape, n_sink + n_comp + n_win + n_stream + n_dec
+
+
+def status_word(cache, dev):
+    """The cache's decode workspace, whose head is the status word `Cache.check` reads."""
+    ws = cache._decode_ws
+    if ws is None or ws.device != dev:
+        # zero-filled: the header's status word and arrival counters must start at zero
+        ws = cache._decode_ws = torch.zeros(1 << 20, dtype=torch.uint8, device=dev)
+    return ws
 
 
 class _Launch:
@@ -225,8 +249,9 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
     several new tokens after compression, which the reference serves by dequantising the whole
     cache (src/shard/attention.py:357-362, src/shard/cache.py:87-124) -- `pos_q` is the position
     of the LAST query; query j attends to everything before the s new tokens plus the first j + 1
-    of them (causal), one launch per query token, nothing dequantised.  The new tokens must
-    already have been appended (`update`).
+    of them (causal).  The new tokens must already have been appended (`update`).  Two query tokens
+    are two decode launches; more share one read-back of the layer into tensor-core tiles, over which
+    they attend as the rows of dense products.
 
     `attn_mask` is accepted for signature compatibility: for one sequence without padding the
     causal mask is what the above implements (the reference's own fused variant skips it for the
@@ -247,6 +272,21 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
     if n_new_total < s_q:
         raise _lib.ShardError("append the new tokens (update) before attending with them")
     res = torch.empty(s_q, n_q, hd, dtype=torch.float16, device=q_rope.device)
+    nkv = cache._n_kv_heads
+    if (s_q >= MIN_MULTIQUERY_TOKENS and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
+            and not (gc.get("stream_n", 0) and "decode_k" in gc)):
+        # all query tokens over one read-back of the layer
+        dev = q_rope.device
+        _lib.require_cuda(q_rope, gc["k_wprep"])
+        seq, shape, _ = layer_record(gc, nkv, hd, dev)
+        ops.multiquery_attn(q_rope[0], seq, shape, cache._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
+                            gc["compress_start"], res, status_word(cache, dev))
+        gc.pop("_fresh", None)                         # (these launches read the layer's tensors the plain way)
+        res = res.permute(1, 0, 2).unsqueeze(0)        # (1, n_q, s, hd)
+        if out is not None:
+            out.copy_(res)
+            return out
+        return res
     prev_keep = getattr(cache, "_phase_keep", 1)
     cache._phase_keep = max(prev_keep, min(s_q, 8))    # the layers of this forward share the tables
     try:

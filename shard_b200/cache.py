@@ -126,6 +126,18 @@ def kmeans(data, k, n_iter=30, seed=42, init=None, max_abs=0.0):
     return centroids, idx_u8
 
 
+_second_streams = {}
+
+
+def _second_stream(device):
+    """The stream compression uses beside the current one, one per device: what is allocated on it comes
+    from the allocator's pool of that stream call after call.  High priority: the eigensolver's few CTAs
+    are placed before k-means' many."""
+    if device not in _second_streams:
+        _second_streams[device] = torch.cuda.Stream(device, priority=-1)
+    return _second_streams[device]
+
+
 class CacheLayer(CacheLayerMixin):
     """One layer's K/V: raw after prefill, compressed (`_gpu_compressed`) afterwards."""
 
@@ -163,36 +175,24 @@ class CacheLayer(CacheLayerMixin):
         gc = self._gpu_compressed
         if gc is None:
             return
-        from .attention import row_tensors, _seq_record
+        from .attention import layer_record, status_word
         c = self._cache_ref
-        nkv, hd, n_comp = c._n_kv_heads, c.head_dim, gc["n_compress"]
+        nkv, hd = c._n_kv_heads, c.head_dim
         dev = gc["k_coeffs"].device
         _lib.require_cuda(gc["k_coeffs"])
         pend = gc.pop("_pending", None)
-        n_stream = gc.get("stream_n", 0)
-        if pend is not None and pend[2] != n_stream - 1:
+        if pend is not None and pend[2] != gc.get("stream_n", 0) - 1:
             gc["_pending"] = pend
             self._flush_pending()
             pend = None
-        seq = _seq_record(gc, dev)
-        dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd)
-        n_sink, n_win = gc["sink_k"].shape[2], gc["win_k"].shape[2]
-        shape = ops.make_shape(4 * nkv, nkv, gc["k_rank_kernel"], n_comp, 0, n_comp, n_sink, n_win, n_stream, 0,
-                               append=pend is not None, n_dec=n_dec)
-        shape.dec_cap = dec_cap
-        if n_dec:
-            seq.dec_k, seq.dec_v = dk.data_ptr(), dv.data_ptr()
+        seq, shape, rows = layer_record(gc, nkv, hd, dev)
         if pend is not None:
             seq.new_k, seq.new_v = pend[0].data_ptr(), pend[1].data_ptr()
-        rows = n_sink + n_comp + n_win + n_stream + n_dec
+            shape.append = 1
         keys = torch.empty(1, nkv, rows, hd, dtype=torch.float16, device=dev)
         values = torch.empty_like(keys)
-        ws = c._decode_ws
-        if ws is None or ws.device != dev:
-            # zero-filled: the status word at its head (see `Cache.check`) must start at zero
-            ws = c._decode_ws = torch.zeros(1 << 20, dtype=torch.uint8, device=dev)
-        ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if n_stream else None,
-                      gc["compress_start"], keys, values, ws)
+        ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
+                      gc["compress_start"], keys, values, status_word(c, dev))
         self._keys, self._values = keys, values
         self._needs_decompress = False
 
@@ -333,15 +333,16 @@ class CacheLayer(CacheLayerMixin):
         if need <= cap:
             return
         new_cap = max(need, c._decode_capacity if cap == 0 else cap * 2)
-        for key, shape, dtype in (("k_idx", (B, heads, hd), torch.uint8),
-                                  ("v_idx", (B, heads, hd), torch.uint8),
-                                  ("k_norm", (B, heads), torch.float16),
-                                  ("v_norm", (B, heads), torch.float16)):
-            new = torch.zeros((new_cap, *shape), device=dev, dtype=dtype)
-            old = gc.get(f"{key}_buf")
-            if old is not None:
-                new[: old.shape[0]].copy_(old)
-            gc[f"{key}_buf"] = new
+        # one allocation: codes of K and V, then their norms
+        n_idx, n_norm = new_cap * heads * hd, new_cap * heads
+        raw = torch.zeros(2 * n_idx + 4 * n_norm, device=dev, dtype=torch.uint8)
+        k_idx, v_idx, norms = raw.split([n_idx, n_idx, 4 * n_norm])
+        k_norm, v_norm = norms.view(torch.float16).view(2, new_cap, B, heads).unbind(0)
+        for key, new in (("k_idx_buf", k_idx.view(new_cap, B, heads, hd)), ("v_idx_buf", v_idx.view(new_cap, B, heads, hd)),
+                         ("k_norm_buf", k_norm), ("v_norm_buf", v_norm)):
+            if key in gc:
+                new[: cap].copy_(gc[key])
+            gc[key] = new
 
     def _stream_append(self, k, v, position, defer=False):
         """Quantise (1, nkv, s, hd) new tokens into the stream buffers
@@ -475,7 +476,7 @@ class Cache(HFCache):
                 k_full, v_full = self.layers[li]._keys, self.layers[li]._values
                 kpart = self._compress_k(k_full[0, :, start:end, :], start)
                 vpart = self._compress_v(v_full[0, :, start:end, :])
-                self._finish_layer(li, kpart, vpart, start, end)
+                self._finish_layer(li, kpart, vpart, self._ends(li, end), start, end)
         else:
             self._compress_side_by_side(start, end)
         ev1.record()
@@ -489,19 +490,9 @@ class Cache(HFCache):
         group's covariances; the host waits only for the eigenvalues, which decide the bit widths."""
         n_layers = self._num_layers
         main = torch.cuda.current_stream()
-        side = torch.cuda.Stream(main.device, priority=-1)     # its few CTAs are placed before k-means' many
+        side = _second_stream(main.device)
         n_groups = -(-n_layers // EIGH_GROUP)
         bounds = [n_layers * g // n_groups for g in range(n_groups + 1)]
-
-        def covariances(g):
-            layers, grams = [], []
-            for li in range(bounds[g], bounds[g + 1]):
-                k_mid = self.layers[li]._keys[0, :, start:end, :]
-                flat = ops.undo_rope(k_mid, start, self._inv_freq(k_mid.device))
-                mean = flat.mean(dim=0)
-                layers.append((flat, mean))
-                grams.append(gram_matrix(flat, mean))
-            return layers, torch.stack(grams), main.record_event()
 
         n, p = end - start, self._per_layer_dim
         rank = min(self._max_rank_k, p, n - 1)
@@ -510,15 +501,32 @@ class Cache(HFCache):
             # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
             init_rows = initial_rows(n * p // self._v_vq_group_size, self._v_vq_codebook_size, main.device)
             drawn = side.record_event()
+        dev = main.device
+        inv_freq = self._inv_freq(dev)
+        cov_ws = enc_ws = None
+
+        def covariances(g):
+            nonlocal cov_ws
+            count = bounds[g + 1] - bounds[g]
+            flat = torch.empty(count, n, p, dtype=torch.float32, device=dev)
+            mean = torch.empty(count, p, dtype=torch.float32, device=dev)
+            mean_f16 = torch.empty(count, p, dtype=torch.float16, device=dev)
+            gram = torch.empty(count, p, p, dtype=torch.float32, device=dev)
+            rows = list(zip(flat.unbind(0), mean.unbind(0), mean_f16.unbind(0)))
+            for li, (f, m, m16), gr in zip(range(bounds[g], bounds[g + 1]), rows, gram.unbind(0)):
+                cov_ws = ops.k_covariance(self.layers[li]._keys[0, :, start:end, :], start, inv_freq, f, m, m16, gr, cov_ws)
+            return rows, gram, main.record_event()
+
         ready = covariances(0)
         main.wait_event(drawn)
         for g in range(n_groups):
-            layers, gram, done = ready
+            rows, gram, done = ready
             side.wait_event(done)
             with torch.cuda.stream(side):
                 solved = LeadingEigenpairs(gram, rank)
             vparts = self._compress_v_layers([self.layers[li]._values[0, :, start:end, :]
                                               for li in range(bounds[g], bounds[g + 1])], init_rows=init_rows)
+            ends = [self._ends(li, end) for li in range(bounds[g], bounds[g + 1])]
             if g + 1 < n_groups:
                 ready = covariances(g + 1)
             with torch.cuda.stream(side):
@@ -526,20 +534,19 @@ class Cache(HFCache):
                 fin = side.record_event()
             main.wait_event(fin)
             for i, li in enumerate(range(bounds[g], bounds[g + 1])):
-                flat, mean = layers[i]
-                kpart = self._quantise_k(flat, mean, basis[i], eig_host[i].clamp(min=0) / n)
-                self._finish_layer(li, kpart, vparts[i], start, end)
+                kpart, enc_ws = self._quantise_k(*rows[i], basis[i], eig_host[i].clamp(min=0) / n, enc_ws)
+                self._finish_layer(li, kpart, vparts[i], ends[i], start, end)
         # the second stream's tensors go back to the allocator behind everything enqueued here
         side.wait_stream(main)
 
-    def _finish_layer(self, li, kpart, vpart, start, end):
+    def _ends(self, li, end):
         layer = self.layers[li]
-        k_full, v_full = layer._keys, layer._values
-        sink = self._sink_tokens
-        self._build_gpu_format(layer, kpart, vpart,
-                               sink_k=k_full[:, :, :sink, :].clone(), sink_v=v_full[:, :, :sink, :].clone(),
-                               win_k=k_full[:, :, end:, :].clone(), win_v=v_full[:, :, end:, :].clone(),
-                               n_comp=end - start, batch=k_full.shape[0], start=start)
+        return ops.kv_ends(layer._keys[0], layer._values[0], self._sink_tokens, self._residual_window, end)
+
+    def _finish_layer(self, li, kpart, vpart, ends, start, end):
+        sink_k, sink_v, win_k, win_v = ends
+        self._build_gpu_format(self.layers[li], kpart, vpart, sink_k=sink_k, sink_v=sink_v, win_k=win_k, win_v=win_v,
+                               n_comp=end - start, batch=1, start=start)
 
     def _compress_k(self, k_mid, pos_start, basis=None):
         """Un-rotate, fit a joint PCA over all KV heads, quantise basis to int8 and
@@ -564,9 +571,9 @@ class Cache(HFCache):
         else:
             basis = basis.to(dev, torch.float32)[:, :rank]
             eigvals = ((flat - mean) @ basis).pow(2).sum(dim=0) / n
-        return self._quantise_k(flat, mean, basis, eigvals)
+        return self._quantise_k(flat, mean, mean.half(), basis, eigvals)[0]
 
-    def _quantise_k(self, flat, mean, basis, eigvals):
+    def _quantise_k(self, flat, mean, mean_f16, basis, eigvals, workspace=None):
         """Bit allocation, int8 basis, projection and int4 codes of un-rotated keys `flat` (n, dim)."""
         n = flat.shape[0]
         budget = max(64, int(self._per_layer_dim * 16 / self._k_target_cr))
@@ -577,11 +584,10 @@ class Cache(HFCache):
             raise ShardError("bit allocation kept no PCA component")
         alloc = alloc[:keep]
         basis = basis[:, :keep]
-        basis_q, scale, w, basis_f16 = ops.k_basis_quantise(basis if basis.stride(1) == 1 else basis.contiguous())
-        proj = ops.k_project(flat, mean, w)
-        packed, coeff_scale = ops.k_quantize_pack(proj, alloc)
-        return {"k_basis_q": basis_q, "k_scale": scale, "k_basis_f16": basis_f16, "k_mean": mean.half(), "k_alloc": alloc,
-                "k_coeffs": packed, "k_coeff_scale": coeff_scale, "k_n_total": n}
+        basis_q, scale, basis_f16, packed, coeff_scale, wprep, workspace = ops.k_encode(
+            flat, mean, mean_f16, basis if basis.stride(1) == 1 else basis.contiguous(), alloc, workspace)
+        return {"k_basis_q": basis_q, "k_scale": scale, "k_basis_f16": basis_f16, "k_mean": mean_f16, "k_alloc": alloc,
+                "k_coeffs": packed, "k_coeff_scale": coeff_scale, "k_wprep": wprep, "k_n_total": n}, workspace
 
     def _compress_v(self, v_mid, init_centroids=None, init_rows=None):
         """Hadamard-rotate, normalise per channel and vector-quantise 4-channel groups
@@ -619,7 +625,7 @@ class Cache(HFCache):
         keep = len(k["k_alloc"])
         ng = hd // v["group_size"]
         basis_f16 = k["k_basis_f16"]
-        coeff_scale_f16 = k["k_coeff_scale"].half()
+        coeff_scale_f16 = k["k_coeff_scale"]
         gc = {
             "k_coeffs": k["k_coeffs"],
             "k_coeff_scale": coeff_scale_f16,
@@ -638,7 +644,7 @@ class Cache(HFCache):
             "sink_k": sink_k, "sink_v": sink_v, "win_k": win_k, "win_v": win_v,
             "n_compress": n_comp, "batch": batch, "compress_start": start,
         }
-        attach_kernel_format(gc, nkv)
+        attach_kernel_format(gc, nkv, k["k_wprep"])
         layer._gpu_compressed = gc
         layer._keys = None
         layer._values = None
@@ -729,10 +735,11 @@ class Cache(HFCache):
         return self.compress_ratio()
 
 
-def attach_kernel_format(gc, nkv):
+def attach_kernel_format(gc, nkv, wprep=None):
     """Add what the decode kernel needs beyond the reference's dictionary: the
     fragment-ordered weights, and (only when the kept rank is not a multiple of 32) a
-    copy of the coefficients padded with zero nibbles to the next multiple."""
+    copy of the coefficients padded with zero nibbles to the next multiple.  `wprep`: those weights
+    if the caller has them already."""
     n_total, keep = gc["k_coeffs_shape"]
     basis = gc["k_basis_f16"]
     cscale = gc["k_coeff_scale"].to(torch.float16).contiguous()
@@ -749,6 +756,6 @@ def attach_kernel_format(gc, nkv):
         gc["k_coeffs_padded"] = coeffs
     gc["k_rank_kernel"] = rank_k
     gc["k_coeffs_kernel"] = coeffs
-    gc["k_wprep"] = ops.decode_prepare(basis, cscale, gc["k_mean_f16"], nkv, rank_k)
+    gc["k_wprep"] = wprep if wprep is not None else ops.decode_prepare(basis, cscale, gc["k_mean_f16"], nkv, rank_k)
     gc["_fresh"] = True      # the next decode launch follows the kernels that wrote these tensors
     return gc

@@ -1,4 +1,4 @@
-// Prefill compressor kernels: RoPE removal, the two-stage int4
+// Prefill compressor kernels: the two-stage int4
 // quantiser with nibble packing, Hadamard + per-channel normalisation of V and
 // nearest-centroid VQ assignment.
 //
@@ -12,30 +12,6 @@
 #include "common.cuh"
 
 namespace shard {
-
-// ---------------------------------------------------------------------------
-// undo RoPE: flat[t][kv*128+d] = k*cos - rotate_half(k)*sin, fp32
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) undo_rope_kernel(const __half* __restrict__ k, int64_t head_stride,
-                                                        int64_t tok_stride, int nkv, int n, int pos_start,
-                                                        const float* __restrict__ inv_freq,
-                                                        float* __restrict__ flat) {
-  // one block per token; thread (kv_sub, i) covers pair i of several heads
-  const int t = blockIdx.x;
-  const int i = threadIdx.x & 63;
-  const float phase = __fmul_rn((float)(pos_start + t), inv_freq[i]);
-  float sn, cs;
-  sincosf(phase, &sn, &cs);
-  for (int kv = threadIdx.x >> 6; kv < nkv; kv += 2) {
-    const __half* row = k + kv * head_stride + (int64_t)t * tok_stride;
-    const float lo = __half2float(row[i]);
-    const float hi = __half2float(row[i + 64]);
-    float* o = flat + (size_t)t * nkv * HD + kv * HD;
-    // d < 64: k[d]*cos - (-k[d+64])*sin ; d >= 64: k[d]*cos - k[d-64]*sin
-    o[i] = __fadd_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn));
-    o[i + 64] = __fsub_rn(__fmul_rn(hi, cs), __fmul_rn(lo, sn));
-  }
-}
 
 // ---------------------------------------------------------------------------
 // K quantiser
@@ -55,7 +31,14 @@ __global__ void kq_init_kernel(uint32_t* ws, int keep) {
   if (j < keep) { ws[j] = 0xffffffffu; ws[keep + j] = 0u; ws[2 * keep + j] = 0u; }
 }
 
-constexpr int KQ_ROWS = 64;  // rows per block
+// the same, and the bit widths handed over as a kernel argument
+struct KqBits { uint8_t b[256]; };
+__global__ void kq_init_bits_kernel(uint32_t* ws, int keep, const __grid_constant__ KqBits bits, int32_t* __restrict__ alloc) {
+  const int j = threadIdx.x;
+  if (j < keep) { ws[j] = 0xffffffffu; ws[keep + j] = 0u; ws[2 * keep + j] = 0u; alloc[j] = bits.b[j]; }
+}
+
+constexpr int KQ_ROWS = 32;  // rows per block (short prompts need the blocks), eight loads in flight per thread
 
 __global__ void __launch_bounds__(256) kq_minmax_kernel(const float* __restrict__ proj, int n, int keep,
                                                         uint32_t* __restrict__ ws) {
@@ -63,6 +46,7 @@ __global__ void __launch_bounds__(256) kq_minmax_kernel(const float* __restrict_
   for (int j = threadIdx.x; j < keep; j += blockDim.x) {
     float lo = __int_as_float(0x7f800000), hi = neg_inf();
     const int r1 = min(r0 + KQ_ROWS, n);
+#pragma unroll 8
     for (int r = r0; r < r1; ++r) {
       const float v = proj[(size_t)r * keep + j];
       lo = fminf(lo, v); hi = fmaxf(hi, v);
@@ -92,14 +76,19 @@ __global__ void __launch_bounds__(256) kq_absmax_kernel(const float* __restrict_
     const float levels = (float)((1 << bits) - 1);
     float am = 0.f;
     const int r1 = min(r0 + KQ_ROWS, n);
+#pragma unroll 8
     for (int r = r0; r < r1; ++r) am = fmaxf(am, fabsf(kq_xhat(proj[(size_t)r * keep + j], lo, rng, levels)));
     atomicMax(ws + 2 * keep + j, __float_as_uint(am));  // non-negative floats order as integers
   }
 }
 
-__global__ void kq_scale_kernel(const uint32_t* __restrict__ ws, int keep, float* __restrict__ coeff_scale) {
+__global__ void kq_scale_kernel(const uint32_t* __restrict__ ws, int keep, float* __restrict__ coeff_scale,
+                                __half* __restrict__ scale_f16) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < keep) coeff_scale[j] = __fdiv_rn(fmaxf(__uint_as_float(ws[2 * keep + j]), 1e-6f), 7.0f);
+  if (j >= keep) return;
+  const float s = __fdiv_rn(fmaxf(__uint_as_float(ws[2 * keep + j]), 1e-6f), 7.0f);
+  coeff_scale[j] = s;
+  if (scale_f16) scale_f16[j] = __float2half_rn(s);
 }
 
 __global__ void __launch_bounds__(256) kq_pack_kernel(const float* __restrict__ proj,
@@ -135,32 +124,46 @@ __global__ void __launch_bounds__(256) kq_pack_kernel(const float* __restrict__ 
 
 // int8 basis: per column scale = max(max|b|, 1e-6) / 127, code = clamp(rint(b / scale), +-127); and what
 // the projection and the decode kernels take: w = code * scale (fp32) and fp16(code) * fp16(scale).
-// A block takes 32 columns, 8 rows at a time.
-__global__ void __launch_bounds__(256) k_basis_quantise_kernel(const float* __restrict__ basis, int64_t stride, int dim, int keep,
-                                                               int8_t* __restrict__ basis_q, __half* __restrict__ scale_f16,
-                                                               float* __restrict__ w, __half* __restrict__ basis_f16) {
-  __shared__ float mx[8][32];
-  const int c = blockIdx.x * 32 + (threadIdx.x & 31), r0 = threadIdx.x >> 5;
+// A block takes 16 columns, 64 rows at a time.
+__global__ void __launch_bounds__(1024) k_basis_quantise_kernel(const float* __restrict__ basis, int64_t stride, int dim, int keep,
+                                                                int8_t* __restrict__ basis_q, __half* __restrict__ scale_f16,
+                                                                float* __restrict__ w, __half* __restrict__ basis_f16) {
+  constexpr int KEPT = 16;                     // rows a thread keeps in registers between the passes (dim <= 1024)
+  __shared__ float mx[64][17];
+  const int cl = threadIdx.x & 15, c = blockIdx.x * 16 + cl, r0 = threadIdx.x >> 4;
   const bool live = c < keep;
-  float m = 0.f;
-  if (live)
-    for (int r = r0; r < dim; r += 8) m = fmaxf(m, fabsf(basis[(size_t)r * stride + c]));
-  mx[r0][threadIdx.x & 31] = m;
-  __syncthreads();
+  float v[KEPT], m = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) m = fmaxf(m, mx[i][threadIdx.x & 31]);
+  for (int i = 0; i < KEPT; ++i) {
+    const int r = r0 + 64 * i;
+    v[i] = live && r < dim ? basis[(size_t)r * stride + c] : 0.f;
+    m = fmaxf(m, fabsf(v[i]));
+  }
+  if (live)
+    for (int r = r0 + 64 * KEPT; r < dim; r += 64) m = fmaxf(m, fabsf(basis[(size_t)r * stride + c]));
+  mx[r0][cl] = m;
+  __syncthreads();
+  for (int h = 32; h > 0; h >>= 1) {
+    if (r0 < h) mx[r0][cl] = fmaxf(mx[r0][cl], mx[r0 + h][cl]);
+    __syncthreads();
+  }
+  m = mx[0][cl];
   if (!live) return;
   const float scale = __fdiv_rn(fmaxf(m, 1e-6f), 127.0f);
   const __half s16 = __float2half_rn(scale);
   if (r0 == 0) scale_f16[c] = s16;
-  for (int r = r0; r < dim; r += 8) {
-    float q = rintf(__fdiv_rn(basis[(size_t)r * stride + c], scale));
+  auto put = [&](int r, float x) {
+    float q = rintf(__fdiv_rn(x, scale));
     q = fminf(fmaxf(q, -127.f), 127.f);
     const size_t o = (size_t)r * keep + c;
     basis_q[o] = (int8_t)(int)q;
     w[o] = __fmul_rn(q, scale);
     basis_f16[o] = __hmul(__float2half_rn(q), s16);
-  }
+  };
+#pragma unroll
+  for (int i = 0; i < KEPT; ++i)
+    if (r0 + 64 * i < dim) put(r0 + 64 * i, v[i]);
+  for (int r = r0 + 64 * KEPT; r < dim; r += 64) put(r, basis[(size_t)r * stride + c]);
 }
 
 __global__ void int4_pack_kernel(const int8_t* __restrict__ q, int64_t n_values, uint8_t* __restrict__ packed) {
@@ -324,20 +327,20 @@ __global__ void __launch_bounds__(256) vq_assign_kernel(const float4* __restrict
 
 using namespace shard;
 
-extern "C" int shard_b200_undo_rope(const void* k_f16, int64_t head_stride, int64_t tok_stride, int32_t nkv,
-                                    int32_t n, int32_t pos_start, const float* inv_freq, float* flat_out,
-                                    void* stream) {
-  if (!k_f16 || !inv_freq || !flat_out || nkv < 1 || n < 0) return SHARD_E_ARG;
-  if (n == 0) return SHARD_OK;
-  undo_rope_kernel<<<n, 128, 0, (cudaStream_t)stream>>>((const __half*)k_f16, head_stride, tok_stride, nkv, n,
-                                                         pos_start, inv_freq, flat_out);
-  SHARD_CHECK_LAUNCH();
-  return SHARD_OK;
-}
-
 extern "C" size_t shard_b200_k_quantize_workspace_bytes(int32_t n, int32_t keep) {
   (void)n;
   return (size_t)3 * (keep > 0 ? keep : 0) * sizeof(uint32_t);
+}
+
+// (the counters and bit widths are in place)
+static void launch_kq(const float* proj, const int32_t* alloc, int n, int keep, uint32_t* ws, float* coeff_scale, __half* scale_f16,
+                      uint8_t* packed, cudaStream_t st) {
+  const int row_blocks = (n + KQ_ROWS - 1) / KQ_ROWS;
+  kq_minmax_kernel<<<row_blocks, 256, 0, st>>>(proj, n, keep, ws);
+  kq_absmax_kernel<<<row_blocks, 256, 0, st>>>(proj, alloc, n, keep, ws);
+  kq_scale_kernel<<<(keep + 255) / 256, 256, 0, st>>>(ws, keep, coeff_scale, scale_f16);
+  const size_t total = (size_t)n * (keep / 2);
+  kq_pack_kernel<<<capped_blocks((long long)((total + 255) / 256), 16), 256, 0, st>>>(proj, alloc, n, keep, ws, coeff_scale, packed);
 }
 
 extern "C" int shard_b200_k_quantize_pack(const float* proj, const int32_t* alloc_bits, int32_t n, int32_t keep,
@@ -349,14 +352,59 @@ extern "C" int shard_b200_k_quantize_pack(const float* proj, const int32_t* allo
   if ((uintptr_t)proj & 7) return SHARD_E_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   uint32_t* ws = (uint32_t*)workspace;
-  const int row_blocks = (n + KQ_ROWS - 1) / KQ_ROWS;
   kq_init_kernel<<<(keep + 255) / 256, 256, 0, st>>>(ws, keep);
-  kq_minmax_kernel<<<row_blocks, 256, 0, st>>>(proj, n, keep, ws);
-  kq_absmax_kernel<<<row_blocks, 256, 0, st>>>(proj, alloc_bits, n, keep, ws);
-  kq_scale_kernel<<<(keep + 255) / 256, 256, 0, st>>>(ws, keep, coeff_scale_out);
-  const size_t total = (size_t)n * (keep / 2);
-  const int blocks = capped_blocks((long long)((total + 255) / 256), 16);
-  kq_pack_kernel<<<blocks, 256, 0, st>>>(proj, alloc_bits, n, keep, ws, coeff_scale_out, packed_out);
+  launch_kq(proj, alloc_bits, n, keep, ws, coeff_scale_out, nullptr, packed_out, st);
+  SHARD_CHECK_LAUNCH();
+  return SHARD_OK;
+}
+
+// workspace of shard_b200_k_encode: w | projection | bit widths, counters, scales | projection's own
+struct KEncodeLayout { size_t proj, small, project, bytes; };
+static KEncodeLayout k_encode_layout(int nkv, int n, int keep) {
+  KEncodeLayout l;
+  auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  l.proj = up((size_t)nkv * HD * keep * 4);
+  l.small = l.proj + up((size_t)n * keep * 4);
+  l.project = l.small + up((size_t)5 * keep * 4);
+  l.bytes = l.project + shard_b200_k_project_workspace_bytes(nkv * HD, keep);
+  return l;
+}
+
+extern "C" size_t shard_b200_k_encode_workspace_bytes(int32_t nkv, int32_t n, int32_t keep) {
+  if (nkv < 1 || n < 1 || shard_b200_k_project_workspace_bytes(nkv * HD, keep) == 0) return 0;
+  return k_encode_layout(nkv, n, keep).bytes;
+}
+
+extern "C" int shard_b200_k_encode(const float* flat, const float* mean, const void* mean_f16, const float* basis,
+                                   int64_t basis_row_stride, const int32_t* alloc_bits_host, int32_t n, int32_t nkv, int32_t keep,
+                                   int8_t* basis_q_out, void* scale_f16_out, void* basis_f16_out, uint8_t* packed_out,
+                                   void* coeff_scale_f16_out, void* wprep_out, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!flat || !mean || !mean_f16 || !basis || !alloc_bits_host || !basis_q_out || !scale_f16_out || !basis_f16_out || !packed_out ||
+      !coeff_scale_f16_out || !workspace)
+    return SHARD_E_ARG;
+  const size_t need = shard_b200_k_encode_workspace_bytes(nkv, n, keep);
+  if (need == 0) return SHARD_E_ARG;
+  if (workspace_bytes < need) return SHARD_E_WORKSPACE;
+  KqBits bits{};
+  for (int j = 0; j < keep; ++j) {
+    if (alloc_bits_host[j] < 0 || alloc_bits_host[j] > 8) return SHARD_E_ARG;
+    bits.b[j] = (uint8_t)alloc_bits_host[j];
+  }
+  const KEncodeLayout l = k_encode_layout(nkv, n, keep);
+  cudaStream_t st = (cudaStream_t)stream;
+  unsigned char* ws = (unsigned char*)workspace;
+  float* w = (float*)ws;
+  float* proj = (float*)(ws + l.proj);
+  int32_t* alloc = (int32_t*)(ws + l.small);
+  uint32_t* counters = (uint32_t*)alloc + keep;
+  float* coeff_scale = (float*)(counters + 3 * keep);
+  int rc = shard_b200_k_basis_quantise(basis, basis_row_stride, nkv * HD, keep, basis_q_out, scale_f16_out, w, basis_f16_out, stream);
+  if (rc) return rc;
+  rc = shard_b200_k_project(flat, mean, w, n, nkv * HD, keep, proj, ws + l.project, l.bytes - l.project, stream);
+  if (rc) return rc;
+  kq_init_bits_kernel<<<1, 256, 0, st>>>(counters, keep, bits, alloc);
+  launch_kq(proj, alloc, n, keep, counters, coeff_scale, (__half*)coeff_scale_f16_out, packed_out, st);
+  if (wprep_out) return shard_b200_decode_prepare(basis_f16_out, coeff_scale_f16_out, mean_f16, nkv, keep, wprep_out, stream);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }
@@ -364,7 +412,7 @@ extern "C" int shard_b200_k_quantize_pack(const float* proj, const int32_t* allo
 extern "C" int shard_b200_k_basis_quantise(const float* basis, int64_t row_stride, int32_t dim, int32_t keep, int8_t* basis_q_out,
                                            void* scale_f16_out, float* w_out, void* basis_f16_out, void* stream) {
   if (!basis || !basis_q_out || !scale_f16_out || !w_out || !basis_f16_out || dim < 1 || keep < 1 || row_stride < keep) return SHARD_E_ARG;
-  k_basis_quantise_kernel<<<(keep + 31) / 32, 256, 0, (cudaStream_t)stream>>>(basis, row_stride, dim, keep, basis_q_out,
+  k_basis_quantise_kernel<<<(keep + 15) / 16, 1024, 0, (cudaStream_t)stream>>>(basis, row_stride, dim, keep, basis_q_out,
                                                                               (__half*)scale_f16_out, w_out, (__half*)basis_f16_out);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
@@ -404,6 +452,36 @@ extern "C" int shard_b200_dp_bit_allocation(const double* group_var_host, const 
     group_bits_host[g] = bits;
     b -= cost_of(g, bits);
   }
+  return SHARD_OK;
+}
+
+// Sink and window rows of a layer's prompt, four contiguous tensors: out = [sink K | sink V | window K | window V],
+// each [nkv][rows][128].  A warp per row.
+__global__ void __launch_bounds__(256) kv_ends_kernel(const __half* __restrict__ k, const __half* __restrict__ v, int64_t k_head,
+                                                      int64_t k_tok, int64_t v_head, int64_t v_tok, int nkv, int n_sink, int n_win,
+                                                      int win_start, __half* __restrict__ out) {
+  const int lane = threadIdx.x & 31, rows = n_sink + n_win;
+  const int u = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (u >= 2 * rows * nkv) return;
+  const int r = u % rows, kv = (u / rows) % nkv, is_v = u / (rows * nkv);
+  const int t = r < n_sink ? r : win_start + r - n_sink;
+  const __half* src = (is_v ? v + kv * v_head + (int64_t)t * v_tok : k + kv * k_head + (int64_t)t * k_tok) + 4 * lane;
+  __half* dst = r < n_sink ? out + (((size_t)is_v * nkv + kv) * n_sink + r) * HD
+                           : out + (size_t)2 * nkv * n_sink * HD + (((size_t)is_v * nkv + kv) * n_win + r - n_sink) * HD;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) dst[4 * lane + i] = src[i];
+}
+
+extern "C" int shard_b200_kv_ends(const void* k_f16, const void* v_f16, int64_t k_head_stride, int64_t k_tok_stride,
+                                  int64_t v_head_stride, int64_t v_tok_stride, int32_t nkv, int32_t n_sink, int32_t n_win,
+                                  int32_t win_start, void* out_f16, void* stream) {
+  if (!k_f16 || !v_f16 || !out_f16 || nkv < 1 || n_sink < 0 || n_win < 0) return SHARD_E_ARG;
+  const long long warps = 2ll * (n_sink + n_win) * nkv;
+  if (warps == 0) return SHARD_OK;
+  kv_ends_kernel<<<(unsigned int)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>(
+      (const __half*)k_f16, (const __half*)v_f16, k_head_stride, k_tok_stride, v_head_stride, v_tok_stride, nkv, n_sink, n_win, win_start,
+      (__half*)out_f16);
+  SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }
 

@@ -418,41 +418,45 @@ __device__ __forceinline__ void eg_rescale(double& a, double& b) {
   b *= f;
 }
 
-// CTA = eigenvalue number w (descending); 128 trial points, one per thread, split its interval into 129
-// per round.  A step of the recurrence is the latency of one multiply-add; more points per round would
-// save rounds but the fp64 pipes are full at 7 matrices already.
+// CTA = eigenvalue number w (descending); 128 trial points, two per thread (they share the reads of the
+// matrix), split its interval into 129 per round.  A step of the recurrence is the latency of one
+// multiply-add; more points per round would save rounds, but four matrices fill the fp64 pipes already.
 constexpr int EG_PTS = 128;
-__global__ void __launch_bounds__(EG_PTS) tridiag_values_kernel(const __grid_constant__ EighParams p) {
+__global__ void __launch_bounds__(EG_PTS / 2) tridiag_values_kernel(const __grid_constant__ EighParams p) {
   __shared__ double2 td[EG_MAX_P];
-  __shared__ int left[2][EG_PTS / 32];
+  __shared__ int left[2][EG_PTS / 64];
   const int m = blockIdx.y, n = p.p, w = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const double unscale = eg_load(p, m, td, threadIdx.x, EG_PTS);
+  const double unscale = eg_load(p, m, td, threadIdx.x, EG_PTS / 2);
   double lo = -1.0, width = 2.0;
-  for (int round = 0; round < 8; ++round) {             // 129^-8: below fp64's resolution of the interval
-    const double step = width / 129.0, x = lo + step * (double)(threadIdx.x + 1);
-    double b = 1.0, a = td[0].x - x;                    // p_{i-1}, p_i
-    int neg = __double2hiint(a) < 0;
+  for (int round = 0; round < 7; ++round) {             // 129^-7 = 2^-49 of the interval
+    const double step = width / 129.0, x0 = lo + step * (double)(threadIdx.x + 1), x1 = lo + step * (double)(threadIdx.x + 1 + EG_PTS / 2);
+    double b0 = 1.0, a0 = td[0].x - x0, b1 = 1.0, a1 = td[0].x - x1;   // p_{i-1}, p_i at both points
+    int neg0 = __double2hiint(a0) < 0, neg1 = __double2hiint(a1) < 0;
+    double e2 = td[0].y;
     auto row = [&](int i) {
-      const double c = fma(td[i].x - x, a, -td[i - 1].y * b);
-      neg += (unsigned)(__double2hiint(c) ^ __double2hiint(a)) >> 31;
-      b = a;
-      a = c;
+      const double2 t = td[i];
+      const double c0 = fma(t.x - x0, a0, -e2 * b0), c1 = fma(t.x - x1, a1, -e2 * b1);
+      neg0 += (unsigned)(__double2hiint(c0) ^ __double2hiint(a0)) >> 31;
+      neg1 += (unsigned)(__double2hiint(c1) ^ __double2hiint(a1)) >> 31;
+      b0 = a0; a0 = c0; b1 = a1; a1 = c1;
+      e2 = t.y;
     };
     int i = 1;
     for (; i + 8 <= n; i += 8) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) row(i + j);
-      eg_rescale(a, b);
+      eg_rescale(a0, b0);
+      eg_rescale(a1, b1);
     }
     for (; i < n; ++i) row(i);
     // neg eigenvalues lie below a point; the one sought has n - 1 - w below it, so it lies right of the
     // first k points
-    const unsigned int bal = __ballot_sync(0xffffffffu, neg <= n - 1 - w);
-    if (lane == 0) left[round & 1][warp] = __popc(bal);
+    const int both = __popc(__ballot_sync(0xffffffffu, neg0 <= n - 1 - w)) + __popc(__ballot_sync(0xffffffffu, neg1 <= n - 1 - w));
+    if (lane == 0) left[round & 1][warp] = both;
     __syncthreads();
     int k = 0;
 #pragma unroll
-    for (int t = 0; t < EG_PTS / 32; ++t) k += left[round & 1][t];
+    for (int t = 0; t < EG_PTS / 64; ++t) k += left[round & 1][t];
     lo += step * k;
     width = step;
   }
@@ -547,7 +551,8 @@ __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_consta
 // ---------------------------------------------------------------------------
 // back to the matrix's own coordinates: x = H_0 H_1 ... H_{n-3} z, a warp per vector
 // ---------------------------------------------------------------------------
-// CB chunks of 128 rows; lane owns rows 128 j + 4 lane .. + 3.  Two reflectors per pass: with
+// CB chunks of 128 rows; lane owns rows 128 j + 4 lane .. + 3.  (Two vectors per warp halve the reads of
+// the reflectors but leave too few warps to hide them: 430 against 260 us for four matrices.)  Two reflectors per pass: with
 // x' = x - t1 v1 (v1.x), v2.x' = v2.x - t1 (v1.x)(v2.v1), so the three sums go through one set of shuffles.
 template <int CB>
 __global__ void __launch_bounds__(128) eig_back_kernel(const __grid_constant__ EighParams p) {
@@ -667,7 +672,7 @@ static int launch_eigh(const EighParams& p, int count, cudaStream_t st) {
   cfg.numAttrs = 1;
   e = cudaLaunchKernelEx(&cfg, tridiag_kernel<CB>, p);
   if (e != cudaSuccess) return (int)e;
-  tridiag_values_kernel<<<dim3(p.rank, count), EG_PTS, 0, st>>>(p);
+  tridiag_values_kernel<<<dim3(p.rank, count), EG_PTS / 2, 0, st>>>(p);
   tridiag_vectors_kernel<<<dim3((p.rank + 31) / 32, count), 64, 0, st>>>(p);
   eig_back_kernel<CB><<<dim3((p.rank + 3) / 4, count), 128, 0, st>>>(p);
   eig_check_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);

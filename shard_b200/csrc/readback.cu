@@ -430,10 +430,9 @@ int launch_read_back_any(const ShardSeq& seq, const ShardDecodeShape& sh, const 
 
 using namespace shard;
 
-extern "C" int shard_b200_read_back(const ShardSeq* seq_host, const ShardDecodeShape* shape_host, const float* inv_freq,
-                                    const float* codebook, int32_t compress_start, void* k_out_f16, void* v_out_f16,
-                                    int* status_dev, void* stream) {
-  if (!seq_host || !shape_host || !inv_freq || !k_out_f16 || !v_out_f16) return SHARD_E_ARG;
+// Pointers and sizes of a read-back (also of the multi-query attention, which starts with one).
+int shard_b200_check_read_back(const ShardSeq* seq_host, const ShardDecodeShape* shape_host, const float* codebook) {
+  if (!seq_host || !shape_host) return SHARD_E_ARG;
   const ShardSeq& s = *seq_host;
   const ShardDecodeShape& sh = *shape_host;
   if (sh.nkv < 1 || sh.rank < 32 || sh.rank > 192 || (sh.rank % 32) || sh.n_comp < 0 || sh.n_sink < 0 || sh.n_win < 0 ||
@@ -448,8 +447,19 @@ extern "C" int shard_b200_read_back(const ShardSeq* seq_host, const ShardDecodeS
   if (((uintptr_t)s.k_coeffs & 15) || ((uintptr_t)s.k_wprep & 15) || ((uintptr_t)s.v_indices & 15) || ((uintptr_t)s.v_centroids & 7) ||
       ((uintptr_t)s.v_ch & 7) || ((uintptr_t)s.sink_k & 7) || ((uintptr_t)s.sink_v & 7) || ((uintptr_t)s.win_k & 7) ||
       ((uintptr_t)s.win_v & 7) || ((uintptr_t)s.dec_k & 7) || ((uintptr_t)s.dec_v & 7) || ((uintptr_t)s.st_k_idx & 3) ||
-      ((uintptr_t)s.st_v_idx & 3) || ((uintptr_t)s.signs & 15) || ((uintptr_t)s.new_k & 7) || ((uintptr_t)s.new_v & 7) ||
-      (((uintptr_t)k_out_f16 | (uintptr_t)v_out_f16) & 15))
+      ((uintptr_t)s.st_v_idx & 3) || ((uintptr_t)s.signs & 15) || ((uintptr_t)s.new_k & 7) || ((uintptr_t)s.new_v & 7))
     return SHARD_E_ALIGN;
+  return SHARD_OK;
+}
+
+extern "C" int shard_b200_read_back(const ShardSeq* seq_host, const ShardDecodeShape* shape_host, const float* inv_freq,
+                                    const float* codebook, int32_t compress_start, void* k_out_f16, void* v_out_f16,
+                                    int* status_dev, void* stream) {
+  if (!inv_freq || !k_out_f16 || !v_out_f16) return SHARD_E_ARG;
+  const int rc = shard_b200_check_read_back(seq_host, shape_host, codebook);
+  if (rc != SHARD_OK) return rc;
+  const ShardSeq& s = *seq_host;
+  const ShardDecodeShape& sh = *shape_host;
+  if (((uintptr_t)k_out_f16 | (uintptr_t)v_out_f16) & 15) return SHARD_E_ALIGN;
   return launch_read_back_any(s, sh, inv_freq, codebook, compress_start, k_out_f16, v_out_f16, false, status_dev, (cudaStream_t)stream);
 }

@@ -81,6 +81,24 @@ def read_back(seq, shape, inv_freq, codebook, compress_start, k_out, v_out, stat
                                            cur_stream()), "read_back")
 
 
+def multiquery_attn(q, seq, shape, inv_freq, codebook, compress_start, out, status=None):
+    """Causal attention of the layer's newest tokens: q (n_q, s, 128) fp16 (contiguous channels), out
+    (s, n_q, 128).  `seq` / `shape` as for `read_back`; the s tokens are the last of the stream or of the
+    decode buffer."""
+    require_cuda(q, out, inv_freq)
+    if q.stride(2) != 1 or (q.stride(0) | q.stride(1)) & 3 or q.data_ptr() & 7:
+        q = q.contiguous()
+    s = q.shape[1]
+    lib = _lib.load()
+    wsb = lib.shard_b200_multiquery_workspace_bytes(C.byref(shape), s)
+    if wsb == 0:
+        raise _lib.ShardError("multi-query shape rejected by the library")
+    ws = torch.empty(wsb, dtype=torch.uint8, device=q.device)
+    check(lib.shard_b200_multiquery_attn(C.addressof(seq), C.byref(shape), ptr(q), q.stride(0), q.stride(1), s, ptr(inv_freq),
+                                         ptr(codebook), int(compress_start), ptr(_c(out, torch.float16)), ptr(ws), wsb, ptr(status),
+                                         cur_stream()), "multiquery_attn")
+
+
 # --------------------------------------------------------------------------- prefill compressor
 def undo_rope(k, pos_start, inv_freq):
     """k: (nkv, n, 128) fp16 view (last dim contiguous) -> (n, nkv*128) fp32 without RoPE."""
@@ -93,6 +111,68 @@ def undo_rope(k, pos_start, inv_freq):
                                            ptr(_c(inv_freq, torch.float32)), ptr(flat), cur_stream()),
           "undo_rope")
     return flat
+
+
+def k_covariance(k, pos_start, inv_freq, flat, mean, mean_f16, gram, workspace=None):
+    """`undo_rope` of k (nkv, n, 128) fp16 into flat (n, nkv*128), the column means into mean (fp32) and
+    mean_f16, and (flat - mean)^T (flat - mean) into gram.  Returns the scratch for the next call."""
+    require_cuda(k, inv_freq, flat, gram)
+    if k.dtype != torch.float16 or k.stride(-1) != 1:
+        raise _lib.ShardError("k_covariance expects fp16 keys with a contiguous head dimension")
+    nkv, n, _ = k.shape
+    lib = _lib.load()
+    wsb = lib.shard_b200_k_covariance_workspace_bytes(nkv, n)
+    if wsb == 0:
+        raise _lib.ShardError(f"k_covariance supports up to 32 KV heads (got {nkv})")
+    if workspace is None or workspace.numel() < wsb:
+        workspace = torch.empty(wsb, dtype=torch.uint8, device=k.device)
+    check(lib.shard_b200_k_covariance(ptr(k), k.stride(0), k.stride(1), nkv, n, int(pos_start), ptr(_c(inv_freq, torch.float32)),
+                                      ptr(_c(flat, torch.float32)), ptr(_c(mean, torch.float32)), ptr(_c(mean_f16, torch.float16)),
+                                      ptr(_c(gram, torch.float32)), ptr(workspace), wsb, cur_stream()), "k_covariance")
+    return workspace
+
+
+def k_encode(flat, mean, mean_f16, basis, alloc, workspace=None):
+    """Codes of one layer's un-rotated keys: int8 basis, projection, int4 coefficients, and -- when the
+    number of kept components is a multiple of 32 -- the decode kernel's weights.  basis (dim, keep) fp32
+    rows, alloc: bits per component (host).  Returns (basis_q, scale fp16, basis_f16, packed,
+    coeff_scale fp16, wprep or None, workspace)."""
+    require_cuda(flat, mean, mean_f16, basis)
+    n, dim = flat.shape
+    keep = basis.shape[1]
+    nkv = dim // HD
+    dev = flat.device
+    lib = _lib.load()
+    wsb = lib.shard_b200_k_encode_workspace_bytes(nkv, n, keep)
+    if wsb == 0:
+        raise _lib.ShardError(f"k_encode supports dim % 128 == 0, dim <= 1024, even keep <= 192 (got {dim}, {keep})")
+    if basis.dtype != torch.float32 or basis.stride(1) != 1:
+        raise _lib.ShardError("k_encode expects fp32 basis rows with contiguous columns")
+    if workspace is None or workspace.numel() < wsb:
+        workspace = torch.empty(wsb, dtype=torch.uint8, device=dev)
+    basis_q = torch.empty(dim, keep, dtype=torch.int8, device=dev)
+    basis_f16 = torch.empty(dim, keep, dtype=torch.float16, device=dev)
+    scales = torch.empty(2, keep, dtype=torch.float16, device=dev)
+    packed = torch.empty(n * keep // 2, dtype=torch.uint8, device=dev)
+    wprep = torch.empty(lib.shard_b200_wprep_bytes(nkv, keep), dtype=torch.uint8, device=dev) if keep % 32 == 0 else None
+    check(lib.shard_b200_k_encode(ptr(_c(flat, torch.float32)), ptr(_c(mean, torch.float32)), ptr(_c(mean_f16, torch.float16)),
+                                  ptr(basis), basis.stride(0), (C.c_int32 * keep)(*alloc), n, nkv, keep, ptr(basis_q), ptr(scales),
+                                  ptr(basis_f16), ptr(packed), scales.data_ptr() + 2 * keep, ptr(wprep), ptr(workspace), wsb,
+                                  cur_stream()), "k_encode")
+    scale, coeff_scale = scales.unbind(0)
+    return basis_q, scale, basis_f16, packed, coeff_scale, wprep, workspace
+
+
+def kv_ends(k, v, n_sink, n_win, win_start):
+    """Contiguous copies of the first `n_sink` tokens and of `n_win` tokens from `win_start` on, of k and v
+    (nkv, n, 128) fp16: (sink_k, sink_v, win_k, win_v), each (1, nkv, rows, 128)."""
+    require_cuda(k, v)
+    nkv = k.shape[0]
+    out = torch.empty(2 * nkv * (n_sink + n_win) * HD, dtype=torch.float16, device=k.device)
+    check(_lib.load().shard_b200_kv_ends(ptr(k), ptr(v), k.stride(0), k.stride(1), v.stride(0), v.stride(1), nkv, n_sink, n_win,
+                                         win_start, ptr(out), cur_stream()), "kv_ends")
+    sink, win = out.split([2 * nkv * n_sink * HD, 2 * nkv * n_win * HD])
+    return (*sink.view(2, 1, nkv, n_sink, HD).unbind(0), *win.view(2, 1, nkv, n_win, HD).unbind(0))
 
 
 def k_project(flat, mean, w):
@@ -110,23 +190,6 @@ def k_project(flat, mean, w):
                                    ptr(_c(w, torch.float32)), n, dim, keep, ptr(proj), ptr(ws), wsb, cur_stream()),
           "k_project")
     return proj
-
-
-def k_basis_quantise(basis):
-    """int8 codes of a (dim, keep) fp32 basis (any row stride): (basis_q int8, scale fp16 (keep,),
-    w fp32 = basis_q * scale, basis_f16)."""
-    require_cuda(basis)
-    if basis.dtype != torch.float32 or basis.stride(1) != 1:
-        raise _lib.ShardError("k_basis_quantise expects fp32 rows with contiguous columns")
-    dim, keep = basis.shape
-    dev = basis.device
-    q = torch.empty(dim, keep, dtype=torch.int8, device=dev)
-    scale = torch.empty(keep, dtype=torch.float16, device=dev)
-    w = torch.empty(dim, keep, dtype=torch.float32, device=dev)
-    b16 = torch.empty(dim, keep, dtype=torch.float16, device=dev)
-    check(_lib.load().shard_b200_k_basis_quantise(ptr(basis), basis.stride(0), dim, keep, ptr(q), ptr(scale), ptr(w), ptr(b16),
-                                                  cur_stream()), "k_basis_quantise")
-    return q, scale, w, b16
 
 
 def k_quantize_pack(proj, alloc):

@@ -9,6 +9,7 @@ part of this path (it is off by default there) and is rejected.
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
@@ -85,8 +86,9 @@ def get_codebook(d, bits, device):
     return _cache[key]
 
 
+@functools.lru_cache(maxsize=256)
 def stream_signs(layer_idx, hd, device):
     """Per-layer +-1 vector from torch's CPU generator seeded 42 + 7919 * layer
-    (reference: src/shard/cache.py:201-204)."""
+    (reference: src/shard/cache.py:201-204).  A constant like the codebook; do not write to it."""
     g = torch.Generator(device="cpu").manual_seed(42 + layer_idx * 7919)
     return (torch.randint(0, 2, (hd,), generator=g) * 2 - 1).to(device, torch.float32)

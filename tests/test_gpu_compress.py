@@ -1,0 +1,84 @@
+"""The compressor's fused entry points against their parts and float64, at tile edges and with strided views."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _keys(nkv, n, seed, scale=1.0, offset=0.0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    k = torch.randn(n + 3, nkv, 128, generator=g, device="cuda") * scale + offset
+    return k.half().transpose(0, 1)[:, 2:n + 2, :]         # token-major storage, a view of it
+
+
+def _inv_freq():
+    return 1.0 / (500000.0 ** (torch.arange(0, 128, 2, dtype=torch.float32, device="cuda") / 128))
+
+
+@pytest.mark.parametrize("nkv,n,scale,offset", [(1, 1, 1.0, 0.0), (1, 65, 1.0, 3.0), (2, 63, 1e-3, 0.0), (8, 200, 100.0, 0.0),
+                                                (4, 1985, 1.0, 0.5), (8, 9000, 1.0, 0.0), (16, 700, 1.0, 0.0)])
+def test_k_covariance(nkv, n, scale, offset):
+    from shard_b200 import ops
+    k, p = _keys(nkv, n, n, scale, offset), nkv * 128
+    flat = torch.empty(n, p, device="cuda")
+    mean, mean16, gram = torch.empty(p, device="cuda"), torch.empty(p, dtype=torch.float16, device="cuda"), torch.empty(p, p, device="cuda")
+    ws = ops.k_covariance(k, 7, _inv_freq(), flat, mean, mean16, gram)
+    assert int(ws[4:8].view(torch.int32)) == 0
+    assert torch.equal(flat, ops.undo_rope(k, 7, _inv_freq()))
+    want = flat.double().mean(0)
+    assert (mean.double() - want).abs().max() <= 1e-6 * flat.abs().max() and torch.equal(mean16, mean.half())
+    xc = flat.double() - mean.double()
+    g64 = xc.T @ xc
+    # relative to the columns' lengths: two fp16 parts per value, promoted sums
+    norm = xc.norm(dim=0).clamp(min=1e-30)
+    assert ((gram.double() - g64).abs() / (norm[:, None] * norm[None, :])).max() < (1e-6 if n > 1 else float("inf"))
+    assert torch.equal(gram, gram.T.contiguous())
+
+
+@pytest.mark.parametrize("nkv,n,keep", [(2, 129, 64), (8, 1000, 192), (4, 333, 150), (8, 77, 2)])
+def test_k_encode_equals_its_parts(nkv, n, keep):
+    from shard_b200 import ops
+    p = nkv * 128
+    g = torch.Generator(device="cuda").manual_seed(n)
+    flat = torch.randn(n, p, generator=g, device="cuda")
+    mean = flat.mean(0)
+    basis = torch.linalg.qr(torch.randn(p, 192, generator=g, device="cuda"))[0].contiguous()
+    alloc = [(8, 6, 4, 2)[j * 4 // keep] for j in range(keep)]
+    q, scale, b16, packed, cs, wprep, _ = ops.k_encode(flat, mean, mean.half(), basis[:, :keep], alloc)
+    b = basis[:, :keep].contiguous()
+    s = b.abs().max(dim=0).values.clamp(min=1e-6) / 127.0
+    bq = (b / s).round().clamp(-127, 127).to(torch.int8)
+    assert torch.equal(q, bq) and torch.equal(scale, s.half()) and torch.equal(b16, bq.half() * s.half())
+    proj = ops.k_project(flat, mean, (bq.float() * s).contiguous())
+    pk, c32 = ops.k_quantize_pack(proj, alloc)
+    assert torch.equal(packed, pk) and torch.equal(cs, c32.half())
+    if keep % 32:
+        assert wprep is None
+    else:
+        assert torch.equal(wprep, ops.decode_prepare(b16, cs, mean.half(), nkv, keep))
+
+
+@pytest.mark.parametrize("n_sink,n_win,n", [(4, 64, 200), (0, 3, 9), (5, 0, 5)])
+def test_kv_ends(n_sink, n_win, n):
+    from shard_b200 import ops
+    k, v = _keys(8, n, 1), _keys(8, n, 2).contiguous()
+    sk, sv, wk, wv = ops.kv_ends(k, v, n_sink, n_win, n - n_win)
+    assert torch.equal(sk[0], k[:, :n_sink]) and torch.equal(sv[0], v[:, :n_sink])
+    assert torch.equal(wk[0], k[:, n - n_win:]) and torch.equal(wv[0], v[:, n - n_win:])
+
+
+@pytest.mark.parametrize("nkv,n", [(1, 1), (3, 31), (8, 33), (8, 5001)])
+def test_v_hadamard_normalise_views(nkv, n):
+    from shard_b200 import ops
+    v = _keys(nkv, n, n)
+    x, ch = ops.v_hadamard_normalise(v)
+    y = v.double()
+    h = 1
+    while h < 128:
+        y = y.reshape(nkv, n, -1, 2, h)
+        y = torch.cat([y[..., :1, :] + y[..., 1:, :], y[..., :1, :] - y[..., 1:, :]], -2).reshape(nkv, n, 128)
+        h *= 2
+    y = y / 128 ** 0.5
+    m = y.abs().amax(dim=1)
+    assert ((ch.double() - m).abs() <= 1e-6 * m).all()
+    assert (x.double() - y / m[:, None, :]).abs().max() < 1e-5

@@ -1,0 +1,40 @@
+"""Attention of several new tokens over a compressed layer (one launch for all of them) against float64
+attention over the layer's read-back, at the edges of query and key tiles, in both append modes."""
+import pytest
+import torch
+
+from gpu_helpers import random_gc
+from test_gpu_readback import _cache
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_comp,rank,nkv,before,s,streaming", [
+    (1, 32, 1, 0, 3, True), (128, 192, 8, 2, 4, False), (129, 150, 2, 70, 31, True), (700, 192, 8, 5, 32, True),
+    (2000, 192, 4, 60, 33, False), (5000, 192, 8, 0, 200, True), (300, 64, 8, 1, 256, False), (9001, 192, 8, 9, 7, True)])
+def test_multiquery(n_comp, rank, nkv, before, s, streaming):
+    from shard_b200 import fused_attention_compressed
+    gc_np = random_gc(n_comp, rank=rank, nkv=nkv, seed=s)
+    cache, layer = _cache(gc_np, nkv, streaming, capacity=before + s)
+    g = torch.Generator(device="cuda").manual_seed(s)
+    k, v = (torch.randn(1, before + s, nkv, 128, generator=g, device="cuda").half().transpose(1, 2) for _ in range(2))
+    q = torch.randn(1, s, 4 * nkv, 128, generator=g, device="cuda").half().transpose(1, 2)
+    cache._fused_decode_update = True
+    if before:
+        layer.update(k[:, :, :before], v[:, :, :before])
+    layer.update(k[:, :, before:], v[:, :, before:])
+    cache._fused_decode_update = False
+    out = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)
+    cache.check()
+    assert out.shape == (1, 4 * nkv, s, 128)
+    layer._needs_decompress = True
+    keys, values = layer.keys[0].double(), layer.values[0].double()
+    n = keys.shape[1]
+    sc = torch.einsum("hqd,hnd->hqn", q[0].double(), keys.repeat_interleave(4, 0)) / 128 ** 0.5
+    # rows: sink, middle, window, then the tokens in order: the last s are the queries' own
+    hidden = torch.arange(n, device="cuda")[None, :] > n - s + torch.arange(s, device="cuda")[:, None]
+    want = torch.softmax(sc.masked_fill(hidden, float("-inf")), -1) @ values.repeat_interleave(4, 0)
+    err = (out[0].double() - want).abs()
+    assert (err <= 1.5e-3 + 5e-3 * want.abs()).all(), err.max()
+    again = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq, out=torch.empty_like(out).contiguous())
+    assert torch.equal(again, out)

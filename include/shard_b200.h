@@ -87,7 +87,8 @@ typedef struct ShardDecodeShape {
   int32_t n_stream;       /* streamed tokens to attend to                                */
   int32_t pos_q;          /* position of the query token                                 */
   int32_t partial_out;    /* 0: out = fp16 attention; 1: out = fp32 (m, l, acc) partial  */
-  int32_t append;         /* 1: first quantise new_k/new_v into stream row n_stream-1 (fused append) */
+  int32_t append;         /* 1: first quantise new_k/new_v into stream row n_stream-1 (fused append);
+                             2: first copy them into row n_dec-1 of dec_k / dec_v (no streamed rows) */
   int32_t n_dec;          /* rows of the fp16 decode buffer (dec_k / dec_v)              */
   int32_t no_overlap;     /* 1: plain launch, no early start behind the preceding kernel (see decode_attn) */
   int32_t dec_cap;        /* rows allocated per KV head in dec_k / dec_v (0: exactly n_dec)    */
@@ -296,8 +297,8 @@ int shard_b200_stream_quantize_rows(const void* k_f16, const void* v_f16, int64_
  * A compressed layer as fp16 keys and values, [nkv][rows][128] each with rows in the order
  * [sink | middle | window | stream | fp16 decode buffer]: CacheLayer._ensure_dequant
  * (src/shard/cache.py:87-124) with its callees, in one launch.  Of `shape` nkv, rank, n_comp, n_sink,
- * n_win, n_stream, n_dec, dec_cap and append are used (append: new_k / new_v are quantised into stream
- * row n_stream-1 first); middle token t has position compress_start + t.  `status_dev` (may be NULL)
+ * n_win, n_stream, n_dec, dec_cap and append are used (append: new_k / new_v become the newest row
+ * first, as in shard_b200_decode_attn); middle token t has position compress_start + t.  `status_dev` (may be NULL)
  * is set to 1 if a bounded wait inside the kernel gave up (the output is then undefined); the head of
  * a decode workspace serves, see shard_b200_decode_status.  `codebook` may be NULL without stream rows.
  */

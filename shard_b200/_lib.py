@@ -131,6 +131,24 @@ def load():
     return lib
 
 
+_host = None
+
+
+def host():
+    """The native host half of a decode step (`_host.so`, see csrc/host.cpp), bound to the library."""
+    global _host
+    if _host is None:
+        try:
+            import torch  # noqa: F401  (its libraries are what the extension links against)
+            from . import _host as mod
+        except ImportError as e:
+            raise ShardError(f"shard_b200/_host.so is missing or does not load ({e}): build it with "
+                             "`python -m shard_b200.build`") from e
+        mod.bind(C.cast(load().shard_b200_decode_attn, C.c_void_p).value)
+        _host = mod
+    return _host
+
+
 def symbols():
     return list(_SIGNATURES)
 

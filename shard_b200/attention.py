@@ -9,6 +9,8 @@ Hadamard -- is one kernel launch of libshard_b200.so.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 
 from . import _lib, ops
@@ -116,7 +118,7 @@ class _Launch:
     """Per-layer launch state that does not change from step to step: the sequence record, the
     shape record (only n_stream / pos_q / append / n_dec are touched per step), workspace need
     and the constant device pointers."""
-    __slots__ = ("key", "seq", "shape", "need", "inv_ptr", "cb", "cb_ptr", "dev", "dev_index", "kbuf")
+    __slots__ = ("key", "seq", "shape", "need", "inv_ptr", "cb", "cb_ptr", "dev", "dev_index", "kbuf", "inv_freq")
 
 
 def _launch_state(gc, cache, dev, nkv, n_q, t0, t1, with_fp16_segments, partial_out):
@@ -143,15 +145,21 @@ def _launch_state(gc, cache, dev, nkv, n_q, t0, t1, with_fp16_segments, partial_
             probe = ops.make_shape(n_q, nkv, gc["k_rank_kernel"], gc["n_compress"], t0, t1, n_sink, n_win, 1, 0,
                                    partial_out)
             ls.need = ops.decode_workspace_bytes(probe, 1)
-        ls.inv_ptr = ptr(cache._inv_freq(dev))
+        ls.inv_freq = cache._inv_freq(dev)
+        ls.inv_ptr = ptr(ls.inv_freq)
         ls.cb = get_codebook(128, 8, dev)
         ls.cb_ptr = ptr(ls.cb)
         gc["_launch"] = ls
+        # whole-layer decode steps go the native way from the next one on
+        gc.pop("_native", None)
+        if (t0, t1) == (0, gc["n_compress"]) and t1 > 0 and with_fp16_segments and not partial_out:
+            step = _lib.host().make_step(C.addressof(ls.seq), C.addressof(ls.shape), ls.inv_ptr, ls.cb_ptr, ls.need, dev.index)
+            gc["_native"] = (step, (gc["compress_start"], t0, t1), ls)
     return ls
 
 
 def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_fp16_segments=True, out=None,
-                 push=None, visible_new=None):
+                 push=None, visible_new=None, plain_step=False):
     """Run the fused decode for one layer.
 
     q_rope: (1, n_q, 1, 128) fp16 CUDA.  `tok_range` limits the middle segment to
@@ -160,13 +168,28 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
     `push` (a `parallel.PeerExchange`, with `partial_out`) makes the launch deliver that
     record into every rank's exchange buffer itself.  `visible_new` limits the decoded tokens
     (streamed rows, or rows of the fp16 decode buffer) the query attends to, to the first
-    `visible_new` of them: the causal mask of a forward over several new tokens.
+    `visible_new` of them: the causal mask of a forward over several new tokens.  `plain_step` says that
+    none of these options is used, and asks for the result as (1, n_q, 1, 128): the native path.
 
     A bounded wait that gives up inside the kernel leaves a status word in the cache's
     workspace; `Cache.check()` reads it (once per step or request, it synchronises).
     """
     gc = layer._gpu_compressed
     cache = layer._cache_ref
+    if plain_step:
+        native = gc.get("_native")
+        if native is not None:
+            # all of the step in native code; None: something is out of the ordinary
+            step, (start, t0, t1), _ = native
+            pos_q = int(pos_q)
+            if cache._phase_key != (pos_q, start, t0, t1):
+                _phase_for(cache, gc, pos_q, t0, t1, cache._decode_ws.device)
+            res = _lib.host().attend(step, gc, cache._decode_ws, cache._phase.data_ptr(), q_rope, pos_q, out)
+            if res is not None:
+                if type(res) is int:
+                    _lib.check(res, "decode_attn")
+                return res
+        return decode_layer(q_rope, layer, pos_q, out=out).view(1, -1, 1, 128)
     if not q_rope.is_cuda:
         raise _lib.ShardError("shard_b200 kernels need CUDA tensors; there is no CPU fallback")
     B, n_q, s_q, hd = q_rope.shape
@@ -193,6 +216,13 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
         gc["_pending"] = pending
         layer._flush_pending()
         pending = None
+    append = int(pending is not None)
+    if "_pending_dec" in gc:
+        # the newest row of the fp16 decode buffer is still to be written: by this launch if it is its last row
+        if with_fp16_segments and n_stream == 0 and (visible_new is None or int(visible_new) >= gc["decode_k"].shape[2]):
+            pending, append = gc.pop("_pending_dec"), 2
+        else:
+            layer._flush_pending()
     seq, shape = ls.seq, ls.shape
     if n_stream > 0:
         kbuf = gc["k_idx_buf"]
@@ -222,7 +252,7 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
     # with `push` and no `out` the record only goes to the exchange buffers
     seq.q, seq.out = q2.data_ptr(), (None if out is None else out.data_ptr())
     seq.phase = _phase_for(cache, gc, pos_q, t0, t1, dev).data_ptr() if t1 > t0 else None
-    shape.n_stream, shape.pos_q, shape.append = n_stream, int(pos_q), int(pending is not None)
+    shape.n_stream, shape.pos_q, shape.append = n_stream, int(pos_q), append
     shape.n_dec, shape.dec_cap = n_dec, dec_cap
     # the first launch on a freshly built dictionary follows the kernels that wrote its codes and
     # weights: it must not start early behind them
@@ -262,10 +292,9 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
     gc = getattr(layer, "_gpu_compressed", None)
     if gc is None:
         return None
+    if q_rope.shape[2] == 1:
+        return decode_layer(q_rope, layer, pos_q, out=out, plain_step=True)
     _, n_q, s_q, hd = q_rope.shape
-    if s_q == 1:
-        res = decode_layer(q_rope, layer, pos_q, out=None if out is None else out.view(n_q, hd))
-        return res.view(1, n_q, 1, hd)
     cache = layer._cache_ref
     layer._flush_pending()                             # every new token is in its row before the first query looks
     n_new_total = gc.get("stream_n", 0) if "k_idx_buf" in gc else (gc["decode_k"].shape[2] if "decode_k" in gc else 0)

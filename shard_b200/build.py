@@ -32,6 +32,7 @@ def _newest_source_mtime():
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu under csrc/ and link the shared library; returns its path."""
+    build_host(force)
     if not force and os.path.exists(LIB) and os.path.getmtime(LIB) >= _newest_source_mtime():
         return LIB
     nvcc = _nvcc()
@@ -56,6 +57,30 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
     return LIB
+
+
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_LIB = os.path.join(HERE, "_host.so")
+
+
+def build_host(force: bool = False) -> str:
+    """Compile the native host half of a decode step (a CPython extension against torch's headers)."""
+    newest = max(os.path.getmtime(HOST_SRC), os.path.getmtime(os.path.join(os.path.dirname(HERE), "include", "shard_b200.h")))
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= newest:
+        return HOST_LIB
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    includes = [sysconfig.get_paths()["include"], os.path.join(root, "include"),
+                os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{p}" for p in includes], HOST_SRC, "-o", HOST_LIB,
+           f"-L{os.path.join(root, 'lib')}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host.cpp:\n{r.stdout}\n{r.stderr}")
+    return HOST_LIB
 
 
 if __name__ == "__main__":

@@ -185,10 +185,12 @@ class CacheLayer(CacheLayerMixin):
             gc["_pending"] = pend
             self._flush_pending()
             pend = None
+        pend_dec = gc.pop("_pending_dec", None)
         seq, shape, rows = layer_record(gc, nkv, hd, dev)
-        if pend is not None:
-            seq.new_k, seq.new_v = pend[0].data_ptr(), pend[1].data_ptr()
-            shape.append = 1
+        if pend is not None or pend_dec is not None:
+            new = pend if pend is not None else pend_dec
+            seq.new_k, seq.new_v = new[0].data_ptr(), new[1].data_ptr()
+            shape.append = 1 if pend is not None else 2
         keys = torch.empty(1, nkv, rows, hd, dtype=torch.float16, device=dev)
         values = torch.empty_like(keys)
         ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
@@ -230,67 +232,31 @@ class CacheLayer(CacheLayerMixin):
             self._values = value_states
             return key_states, value_states
 
-        if self.layer_idx == 0 and c is not None and not c._compressed:
+        if self._gpu_compressed is None and self.layer_idx == 0 and c is not None and not c._compressed:
             c.compress()
 
         gc = self._gpu_compressed
-        fused = bool(getattr(c, "_fused_decode_update", False))
-        if fused and gc is not None and seq_new == 1 and c._streaming:
-            # the decode hot path: the token is handed to the next decode launch, which quantises it
-            # into its stream row; nothing is launched here
-            if "_pending" in gc:
-                self._flush_pending()
-            s = gc.get("stream_n", 0)
-            if "signs" not in gc or s >= gc["k_idx_buf"].shape[0]:
-                self._grow_stream(gc, key_states, s + 1)
-            k2, v2 = key_states, value_states
-            if k2.stride(3) != 1 or k2.stride(1) != k2.shape[3] or v2.stride(3) != 1 or v2.stride(1) != v2.shape[3]:
-                k2, v2 = k2.contiguous(), v2.contiguous()
-            gc["_pending"] = (k2, v2, s)
-            gc["stream_n"] = s + 1
-            self._seq_len += 1
+        if gc is not None:
+            fused = getattr(c, "_fused_decode_update", False)
+            if not fused:
+                self._lazy_evict()
+            streaming = bool(c._streaming)
+            # one token is handed to the launch that reads it next (fused decode or read-back), which
+            # puts it into its row: nothing is launched here
+            if not (seq_new == 1 and _lib.host().defer(gc, key_states, value_states, streaming)):
+                if streaming:
+                    self._stream_append(key_states, value_states, self._seq_len, defer=seq_new == 1)
+                else:
+                    self._fp16_append(key_states, value_states, defer=seq_new == 1)
+            self._seq_len += seq_new
             self._needs_decompress = True
-            c._last_accessed_layer = self.layer_idx
-            return key_states, value_states
+            if fused:
+                c._last_accessed_layer = self.layer_idx
+                return key_states, value_states
+            self._ensure_dequant()
+            return self._keys, self._values
 
         self._lazy_evict()
-        if gc is not None and c._streaming:
-            # one token is quantised by the launch that reads it next (fused decode or read-back),
-            # several by one launch here
-            self._stream_append(key_states, value_states, self._seq_len, defer=seq_new == 1)
-            self._seq_len += seq_new
-            self._needs_decompress = True
-            if fused:
-                return key_states, value_states
-            self._ensure_dequant()
-            return self._keys, self._values
-
-        if gc is not None:
-            # tokens a non-streaming cache keeps as they are: appended in place to a buffer allocated
-            # ahead (doubling when full); gc["decode_k"] / ["decode_v"] are views of the rows in use
-            n = gc["decode_k"].shape[2] if "decode_k" in gc else 0
-            buf_k = gc.get("_dec_buf_k")
-            if buf_k is None or n + seq_new > buf_k.shape[2] or buf_k.dtype != key_states.dtype:
-                cap = max(c._decode_capacity, 2 * (n + seq_new))
-                B, nkv, _, hd = key_states.shape
-                new_k = torch.empty(B, nkv, cap, hd, dtype=key_states.dtype, device=key_states.device)
-                new_v = torch.empty(B, nkv, cap, hd, dtype=value_states.dtype, device=value_states.device)
-                if n:
-                    new_k[:, :, :n].copy_(gc["decode_k"])
-                    new_v[:, :, :n].copy_(gc["decode_v"])
-                buf_k, gc["_dec_buf_k"], gc["_dec_buf_v"] = new_k, new_k, new_v
-            buf_v = gc["_dec_buf_v"]
-            buf_k[:, :, n:n + seq_new].copy_(key_states)
-            buf_v[:, :, n:n + seq_new].copy_(value_states)
-            gc["decode_k"] = buf_k[:, :, :n + seq_new]
-            gc["decode_v"] = buf_v[:, :, :n + seq_new]
-            self._seq_len += seq_new
-            self._needs_decompress = True
-            if fused:
-                return key_states, value_states
-            self._ensure_dequant()
-            return self._keys, self._values
-
         self._ensure_dequant()
         self._seq_len += seq_new
         if self._keys is not None:
@@ -301,10 +267,42 @@ class CacheLayer(CacheLayerMixin):
             self._values = value_states
         return self._keys, self._values
 
+    # -- fp16 decode buffer ------------------------------------------------------
+    def _fp16_append(self, k, v, defer=False):
+        """Append (1, nkv, s, hd) new tokens as they are, in place, to a buffer allocated ahead (doubling
+        when full); gc["decode_k"] / ["decode_v"] are views of the rows in use.  With `defer` the one
+        token is left to the next launch that reads the rows, whose kernel writes it."""
+        self._flush_pending()
+        gc, c = self._gpu_compressed, self._cache_ref
+        new = k.shape[2]
+        n = gc["decode_k"].shape[2] if "decode_k" in gc else 0
+        buf_k = gc.get("_dec_buf_k")
+        if buf_k is None or n + new > buf_k.shape[2] or buf_k.dtype != k.dtype:
+            cap = max(c._decode_capacity, 2 * (n + new))
+            B, nkv, _, hd = k.shape
+            new_k = torch.empty(B, nkv, cap, hd, dtype=k.dtype, device=k.device)
+            new_v = torch.empty(B, nkv, cap, hd, dtype=v.dtype, device=v.device)
+            if n:
+                new_k[:, :, :n].copy_(gc["decode_k"])
+                new_v[:, :, :n].copy_(gc["decode_v"])
+            buf_k, gc["_dec_buf_k"], gc["_dec_buf_v"] = new_k, new_k, new_v
+        buf_v = gc["_dec_buf_v"]
+        if defer and k.dtype == torch.float16 and v.dtype == torch.float16 and gc.get("stream_n", 0) == 0:
+            gc["_pending_dec"] = (k.contiguous(), v.contiguous())
+        else:
+            buf_k[:, :, n:n + new].copy_(k)
+            buf_v[:, :, n:n + new].copy_(v)
+        gc["decode_k"] = buf_k[:, :, :n + new]
+        gc["decode_v"] = buf_v[:, :, :n + new]
+
     # -- 8-bit stream -----------------------------------------------------------
     def _flush_pending(self):
-        """Quantise a token whose append was left to the next decode launch and never got one."""
+        """Write the row of a token whose append was left to the next launch and never got one."""
         gc = self._gpu_compressed
+        pend = gc.pop("_pending_dec", None) if gc is not None else None
+        if pend is not None:
+            gc["decode_k"][:, :, -1:].copy_(pend[0])
+            gc["decode_v"][:, :, -1:].copy_(pend[1])
         pend = gc.pop("_pending", None) if gc is not None else None
         if pend is not None:
             k2, v2, slot = pend

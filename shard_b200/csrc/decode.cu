@@ -218,7 +218,9 @@ static int decode_attn_impl(const ShardSeq* seqs, int32_t batch, const ShardDeco
   if (rc != SHARD_OK) return rc;
   const ShardDecodeShape& sh = *shape_host;
   if (sh.n_stream > 0 && !codebook) return SHARD_E_ARG;
-  if (sh.append && (sh.n_stream < 1 || (batch == 1 && (!seqs->new_k || !seqs->new_v)))) return SHARD_E_ARG;
+  if (sh.append < 0 || sh.append > 2) return SHARD_E_ARG;
+  if (sh.append == 2 && (sh.n_dec < 1 || sh.n_stream > 0)) return SHARD_E_ARG;   // the appended row is the last one
+  if (sh.append && ((sh.append == 1 && sh.n_stream < 1) || (batch == 1 && (!seqs->new_k || !seqs->new_v)))) return SHARD_E_ARG;
   if ((uintptr_t)workspace & 15) return SHARD_E_ALIGN;
   if (workspace_bytes < ws_bytes(sh, batch)) return SHARD_E_WORKSPACE;
   const DecodePlan pl = make_plan(sh, batch);
@@ -243,7 +245,7 @@ static int decode_attn_impl(const ShardSeq* seqs, int32_t batch, const ShardDeco
         ((uintptr_t)s.sink_v & 7) || ((uintptr_t)s.win_k & 7) || ((uintptr_t)s.win_v & 7) ||
         ((uintptr_t)s.dec_k & 7) || ((uintptr_t)s.dec_v & 7) ||
         ((uintptr_t)s.st_k_idx & 3) || ((uintptr_t)s.st_v_idx & 3) || ((uintptr_t)s.signs & 15) ||
-        ((uintptr_t)s.v_ch & 7))
+        ((uintptr_t)s.v_ch & 7) || (sh.append && (((uintptr_t)s.new_k & 7) || ((uintptr_t)s.new_v & 7))))
       return SHARD_E_ALIGN;
   } else {
     if (push) return SHARD_E_ARG;

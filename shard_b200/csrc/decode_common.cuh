@@ -93,13 +93,20 @@ __device__ __forceinline__ void stage_query(const ShardSeq& sq, int kv, int pos_
   }
 }
 
-// Fused append: the CTA that owns streamed row n_stream-1 first quantises the step's new
-// K/V vector of its KV head into that row (one warp each for K and V).  The caller synchronises
-// the CTA afterwards; the rows are then read back with L2-coherent loads.
+// Fused append: the CTA that owns the newest row first puts the step's new K/V vector of its KV head
+// into it (one warp each for K and V): quantised into streamed row n_stream-1 (append = 1), or copied
+// into row n_dec-1 of the fp16 decode buffer (append = 2).  The caller synchronises the CTA afterwards;
+// the rows are then read back with L2-coherent loads.
 __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const ShardDecodeShape& sh, int kv,
                                                  const float* __restrict__ cbs, bool is_v, int lane) {
-  const size_t row = (size_t)(sh.n_stream - 1) * sh.nkv + kv;
   const __half* src = reinterpret_cast<const __half*>(is_v ? sq.new_v : sq.new_k) + kv * HD;
+  if (sh.append == 2) {
+    __half* dst = reinterpret_cast<__half*>(const_cast<void*>(is_v ? sq.dec_v : sq.dec_k)) +
+                  ((size_t)kv * (sh.dec_cap > 0 ? sh.dec_cap : sh.n_dec) + sh.n_dec - 1) * HD;
+    reinterpret_cast<uint2*>(dst)[lane] = reinterpret_cast<const uint2*>(src)[lane];
+    return;
+  }
+  const size_t row = (size_t)(sh.n_stream - 1) * sh.nkv + kv;
   uint8_t* idx_out = (is_v ? sq.st_v_idx : sq.st_k_idx) + row * HD;
   __half* norm_out = reinterpret_cast<__half*>(is_v ? sq.st_v_norm : sq.st_k_norm) + row;
   quantize_vec_warp(src, sq.signs, cbs, idx_out, norm_out, lane);
@@ -144,8 +151,8 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
     const __half* kb = reinterpret_cast<const __half*>(in_sink ? sq.sink_k : (in_dec ? sq.dec_k : sq.win_k));
     const __half* vb = reinterpret_cast<const __half*>(in_sink ? sq.sink_v : (in_dec ? sq.dec_v : sq.win_v));
     const size_t off = ((size_t)kv * rows + r) * HD + 4 * lane;
-    const uint2 kr = *reinterpret_cast<const uint2*>(kb + off);
-    const uint2 vr = *reinterpret_cast<const uint2*>(vb + off);
+    const uint2 kr = __ldcg(reinterpret_cast<const uint2*>(kb + off));   // (the newest row was written a moment ago)
+    const uint2 vr = __ldcg(reinterpret_cast<const uint2*>(vb + off));
     const float2 k01 = __half22float2(*reinterpret_cast<const __half2*>(&kr.x));
     const float2 k23 = __half22float2(*reinterpret_cast<const __half2*>(&kr.y));
     const float2 v01 = __half22float2(*reinterpret_cast<const __half2*>(&vr.x));

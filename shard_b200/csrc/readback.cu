@@ -90,10 +90,17 @@ __device__ __forceinline__ void rb_rows(const ReadBackParams& p, int cta, int n_
         const __half* kb = reinterpret_cast<const __half*>(in_sink ? sq.sink_k : (in_dec ? sq.dec_k : sq.win_k));
         const __half* vb = reinterpret_cast<const __half*>(in_sink ? sq.sink_v : (in_dec ? sq.dec_v : sq.win_v));
         const size_t off = ((size_t)kv * rows + r) * HD + 4 * lane;
-        k = *reinterpret_cast<const uint2*>(kb + off);
-        v = *reinterpret_cast<const uint2*>(vb + off);
+        if (sh.append == 2 && u == n_rows - 1) {                 // the newest fp16 row is still to be written
+          k = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.new_k) + kv * HD + 4 * lane);
+          v = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.new_v) + kv * HD + 4 * lane);
+          *reinterpret_cast<uint2*>(const_cast<__half*>(kb) + off) = k;
+          *reinterpret_cast<uint2*>(const_cast<__half*>(vb) + off) = v;
+        } else {
+          k = *reinterpret_cast<const uint2*>(kb + off);
+          v = *reinterpret_cast<const uint2*>(vb + off);
+        }
       } else {
-        if (sh.append && u == n_fp + sh.n_stream - 1) {
+        if (sh.append == 1 && u == n_fp + sh.n_stream - 1) {
           append_new_token(sq, sh, kv, cbs, false, lane);
           append_new_token(sq, sh, kv, cbs, true, lane);
           __syncwarp();
@@ -443,7 +450,9 @@ int shard_b200_check_read_back(const ShardSeq* seq_host, const ShardDecodeShape*
   if (sh.n_win > 0 && (!s.win_k || !s.win_v)) return SHARD_E_ARG;
   if (sh.n_dec > 0 && (!s.dec_k || !s.dec_v)) return SHARD_E_ARG;
   if (sh.n_stream > 0 && (!codebook || !s.st_k_idx || !s.st_v_idx || !s.st_k_norm || !s.st_v_norm || !s.signs)) return SHARD_E_ARG;
-  if (sh.append && (sh.n_stream < 1 || !s.new_k || !s.new_v)) return SHARD_E_ARG;
+  if (sh.append < 0 || sh.append > 2 || (sh.append && (!s.new_k || !s.new_v)) || (sh.append == 1 && sh.n_stream < 1) ||
+      (sh.append == 2 && sh.n_dec < 1))
+    return SHARD_E_ARG;
   if (((uintptr_t)s.k_coeffs & 15) || ((uintptr_t)s.k_wprep & 15) || ((uintptr_t)s.v_indices & 15) || ((uintptr_t)s.v_centroids & 7) ||
       ((uintptr_t)s.v_ch & 7) || ((uintptr_t)s.sink_k & 7) || ((uintptr_t)s.sink_v & 7) || ((uintptr_t)s.win_k & 7) ||
       ((uintptr_t)s.win_v & 7) || ((uintptr_t)s.dec_k & 7) || ((uintptr_t)s.dec_v & 7) || ((uintptr_t)s.st_k_idx & 3) ||

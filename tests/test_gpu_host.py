@@ -1,0 +1,70 @@
+"""The native host half of a decode step: same rows and same outputs as the Python path, in both append
+modes, over buffer growth and a restarted reply."""
+import pytest
+import torch
+
+from gpu_helpers import random_gc
+from test_gpu_readback import _cache
+
+pytestmark = pytest.mark.gpu
+
+
+class _Counting:
+    """The native module, counting the steps it took."""
+
+    def __init__(self, real):
+        self.real, self.taken = real, 0
+
+    def __getattr__(self, name):
+        return getattr(self.real, name)
+
+    def attend(self, *a):
+        r = self.real.attend(*a)
+        self.taken += r is not None
+        return r
+
+
+@pytest.mark.parametrize("streaming,nkv,n_comp", [(True, 8, 700), (False, 8, 700), (False, 1, 130), (True, 2, 1)])
+def test_native_steps(streaming, nkv, n_comp, monkeypatch):
+    from shard_b200 import _lib, fused_attention_compressed
+    from shard_b200.attention import decode_layer
+    counting = _Counting(_lib.host())
+    monkeypatch.setattr(_lib, "_host", counting)
+    cache, layer = _cache(random_gc(n_comp, nkv=nkv, seed=1), nkv, streaming, capacity=16)
+    other, ref = _cache(random_gc(n_comp, nkv=nkv, seed=1), nkv, streaming, capacity=16)
+    cache._fused_decode_update = other._fused_decode_update = True
+    g = torch.Generator(device="cuda").manual_seed(2)
+    gc, rgc = layer._gpu_compressed, ref._gpu_compressed
+
+    def token():
+        return [torch.randn(1, nkv, 1, 128, generator=g, device="cuda").half() for _ in range(2)]
+
+    def append_ref(k, v):                                   # the same rows, written the general way
+        if streaming:
+            ref._stream_append(k, v, 0)
+        else:
+            ref._fp16_append(k, v)
+
+    for step in range(20):                                  # the buffers (16 rows) grow on the way
+        k, v = token()
+        q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+        layer.update(k, v)
+        out = fused_attention_compressed(q, layer, 5000 + step, cache._rope_inv_freq)
+        append_ref(k, v)
+        assert torch.equal(out.view(-1, 128), decode_layer(q, ref, 5000 + step))
+        if step == 10:                                      # the reply starts over: rows are dropped
+            if streaming:
+                gc["stream_n"] = rgc["stream_n"] = 3
+            else:
+                for d in (gc, rgc):
+                    d["decode_k"], d["decode_v"] = d["decode_k"][:, :, :3], d["decode_v"][:, :, :3]
+    assert counting.taken >= 17
+    n = gc["stream_n"] if streaming else None
+    for name in ("k_idx_buf", "v_idx_buf", "k_norm_buf", "v_norm_buf") if streaming else ("decode_k", "decode_v"):
+        assert torch.equal(gc[name][:n], rgc[name][:n])
+    # a token whose append never met a launch is written by the next one that reads the rows
+    k, v = token()
+    for _ in range(2):
+        layer.update(k, v)
+        append_ref(k, v)
+    assert torch.equal(layer.keys, ref.keys) and torch.equal(layer.values, ref.values)

@@ -15,6 +15,8 @@ There is no CPU path: tensors must live on a CUDA device.
 from __future__ import annotations
 
 import math
+import threading
+from concurrent.futures import ThreadPoolExecutor
 
 import torch
 from transformers.cache_utils import Cache as HFCache, CacheLayerMixin
@@ -52,6 +54,56 @@ def gram_matrix(flat, mean):
         torch.backends.cuda.matmul.allow_tf32 = prev
 
 
+# Matrices of up to this many rows go to torch.linalg.eigh, which has a Jacobi solver for them.  Its
+# vectors are a few 1e-6 of the largest eigenvalue off, and at the 2 bits per coefficient that so few
+# heads get, that decides about one code in a hundred: with a more exact solver the reconstructed keys
+# move by 4 percent.  Caches of such models have to come out as they always did, so solver, covariance
+# and mean stay PyTorch's there; what can be done is to solve the layers side by side (8 matrices of 512
+# rows: 170 ms one after the other, 26 ms in eight threads).
+TORCH_EIGH_MAX = 512
+
+
+class TorchEigenpairs:
+    """`LeadingEigenpairs` by torch.linalg.eigh, one thread and stream per matrix."""
+    _threads, _lock = None, threading.Lock()
+
+    def __init__(self, gram, rank):
+        count, p, _ = gram.shape
+        self.rank = rank
+        self.basis = torch.empty(count, p, rank, dtype=torch.float32, device=gram.device)
+        self.host = torch.empty(count, rank, dtype=torch.float32)
+        done = torch.cuda.current_stream().record_event()
+        with TorchEigenpairs._lock:
+            if TorchEigenpairs._threads is None:
+                torch.linalg.eigh(torch.eye(2, device=gram.device))    # PyTorch loads its solver in one thread
+                TorchEigenpairs._threads = ThreadPoolExecutor(EIGH_GROUP, thread_name_prefix="shard_b200_eigh")
+        self.jobs = [TorchEigenpairs._threads.submit(self._solve, gram[i], i, done) for i in range(count)]
+
+    def _solve(self, gram, i, done):
+        stream = _stream_of_thread(gram.device)
+        with torch.no_grad(), torch.cuda.device(gram.device), torch.cuda.stream(stream):
+            stream.wait_event(done)
+            w, v = torch.linalg.eigh(gram)
+            self.basis[i].copy_(v.flip(-1)[:, :self.rank])
+            self.host[i] = w.flip(-1)[:self.rank].cpu()
+            stream.synchronize()
+
+    def result(self):
+        for job in self.jobs:
+            job.result()
+        return self.basis, self.host
+
+
+_thread_local = threading.local()
+
+
+def _stream_of_thread(device):
+    streams = _thread_local.__dict__.setdefault("streams", {})
+    if device not in streams:
+        streams[device] = torch.cuda.Stream(device)
+    return streams[device]
+
+
 class LeadingEigenpairs:
     """The `rank` largest eigenpairs of each (p, p) matrix of `gram` (count, p, p): launched on the current
     stream when made, waited for by `result` (on the same stream)."""
@@ -73,6 +125,10 @@ class LeadingEigenpairs:
         return self.basis, host[:, :rank]
 
 
+def leading_eigenpairs(gram, rank):
+    return TorchEigenpairs(gram, rank) if gram.shape[1] <= TORCH_EIGH_MAX else LeadingEigenpairs(gram, rank)
+
+
 def pca_fit(flat, mean, rank):
     """Top-`rank` principal directions of the rows of `flat` (n, p) around `mean`: the
     eigenvectors of the p x p covariance, largest eigenvalue first, and those eigenvalues.
@@ -80,12 +136,12 @@ def pca_fit(flat, mean, rank):
     Replaces the reference's randomised `torch.svd_lowrank(flat - mean, q=rank, niter=24)`
     (src/shard/cache.py:376: 48 passes over the n x p matrix) by one pass -- the Gram matrix
     (flat - mean)^T (flat - mean), a p x p x n contraction in fp32 -- and a symmetric
-    eigensolver on the small p x p matrix (`ops.eigh_top`).  The subspace is the exact optimum the
+    eigensolver on the small p x p matrix (`leading_eigenpairs`).  The subspace is the exact optimum the
     randomised method approximates, so it captures at least as much variance; individual vectors differ
     in sign and, within near-equal eigenvalues, by rotations, which the rest of the path is
     indifferent to (the basis is an input of everything downstream).
     """
-    basis, eigvals = LeadingEigenpairs(gram_matrix(flat, mean).unsqueeze(0), rank).result()
+    basis, eigvals = leading_eigenpairs(gram_matrix(flat, mean).unsqueeze(0), rank).result()
     return basis[0], (eigvals[0].clamp(min=0) / flat.shape[0]).to(flat.device)
 
 
@@ -487,6 +543,8 @@ class Cache(HFCache):
         on a few SMs: it runs on a second stream beside the group's value path (k-means) and the next
         group's covariances; the host waits only for the eigenvalues, which decide the bit widths."""
         n_layers = self._num_layers
+        # (the state the global generator is left in: the reference seeds it for every layer's randomised SVD)
+        torch.manual_seed(42 + n_layers - 1)
         main = torch.cuda.current_stream()
         side = _second_stream(main.device)
         n_groups = -(-n_layers // EIGH_GROUP)
@@ -505,6 +563,14 @@ class Cache(HFCache):
 
         def covariances(g):
             nonlocal cov_ws
+            if p <= TORCH_EIGH_MAX:
+                rows, grams = [], []
+                for li in range(bounds[g], bounds[g + 1]):
+                    flat = ops.undo_rope(self.layers[li]._keys[0, :, start:end, :], start, inv_freq)
+                    mean = flat.mean(dim=0)
+                    rows.append((flat, mean, mean.half()))
+                    grams.append(gram_matrix(flat, mean))
+                return rows, torch.stack(grams), main.record_event()
             count = bounds[g + 1] - bounds[g]
             flat = torch.empty(count, n, p, dtype=torch.float32, device=dev)
             mean = torch.empty(count, p, dtype=torch.float32, device=dev)
@@ -521,7 +587,7 @@ class Cache(HFCache):
             rows, gram, done = ready
             side.wait_event(done)
             with torch.cuda.stream(side):
-                solved = LeadingEigenpairs(gram, rank)
+                solved = leading_eigenpairs(gram, rank)
             vparts = self._compress_v_layers([self.layers[li]._values[0, :, start:end, :]
                                               for li in range(bounds[g], bounds[g + 1])], init_rows=init_rows)
             ends = [self._ends(li, end) for li in range(bounds[g], bounds[g + 1])]

@@ -50,10 +50,24 @@ static DecodePlan make_plan(const ShardDecodeShape& sh, int batch) {
   const int n_tiles = (n_tok + TILE_TOK - 1) / TILE_TOK;
   const int groups = sh.nkv * batch;
   if (n_tiles > 0) {
-    // one CTA per SM: spread the tiles of every (sequence, KV head) evenly over its CTAs
-    int chunks = (groups >= CTA_SLOTS) ? (n_tiles + 15) / 16 : CTA_SLOTS / groups;
-    if (chunks > n_tiles) chunks = n_tiles;
-    if (chunks < 1) chunks = 1;
+    // One CTA per SM.  Fewer (sequence, KV head) pairs than SMs: one wave, the tiles of every pair spread
+    // evenly over its CTAs.  More: CTAs come in waves, and a CTA costs its tiles (3 K cycles each) plus
+    // what it does outside the tile loop (about 16 K cycles: set-up, first tile's latency, epilogue),
+    // CTA_TILES tiles' worth; the number of chunks whose waves cost least.
+    int chunks = CTA_SLOTS / groups;
+    if (chunks < 1) {
+      constexpr int CTA_TILES = 5;
+      long long best = 0;
+      for (int c = 1; c <= n_tiles && c <= 16; ++c) {
+        const long long waves = ((long long)groups * c + CTA_SLOTS - 1) / CTA_SLOTS;
+        const long long cost = waves * ((n_tiles + c - 1) / c + CTA_TILES);
+        if (chunks < 1 || cost < best) { best = cost; chunks = c; }
+      }
+    }
+    // no chunk without a tile, unless the rows want more CTAs than there are tiles (64 rows each)
+    const int n_rows = sh.n_sink + sh.n_win + sh.n_dec + sh.n_stream, row_ctas = (n_rows + 63) / 64;
+    const int most = groups < CTA_SLOTS && row_ctas > n_tiles ? row_ctas : n_tiles;
+    if (chunks > most) chunks = most;
     pl.n_chunks = chunks;
     pl.tiles_per_chunk = n_tiles / chunks;
     pl.tiles_rem = n_tiles % chunks;
@@ -200,9 +214,12 @@ static int check_shape(const ShardDecodeShape* sh) {
 
 // scratch layout: header (status word, arrival counters; zero between calls), then
 // [batch][n_parts][n_q][132] fp32 partial records
+// (with a middle segment the size does not depend on the number of rows: room for every chunk they may ask for)
 static size_t ws_bytes(const ShardDecodeShape& sh, int batch) {
-  const DecodePlan pl = make_plan(sh, batch);
-  return ws_header_bytes(batch, sh.nkv) + (size_t)batch * pl.n_parts * sh.n_q * PART * sizeof(float);
+  int parts = make_plan(sh, batch).n_parts;
+  const int groups = sh.nkv * batch, slots = cta_slots();
+  if (sh.tok_end > sh.tok_begin && groups < slots && parts < slots / groups) parts = slots / groups;
+  return ws_header_bytes(batch, sh.nkv) + (size_t)batch * parts * sh.n_q * PART * sizeof(float);
 }
 
 extern "C" size_t shard_b200_decode_workspace_bytes(const ShardDecodeShape* shape_host, int32_t batch) {

@@ -57,21 +57,6 @@ __device__ __forceinline__ void softmax_init(SoftmaxState& st) {
   }
 }
 
-// online-softmax update with one token whose 4 scores are warp-uniform
-__device__ __forceinline__ void row_update(SoftmaxState& st, const float (&s)[GQA], const float (&v)[4]) {
-#pragma unroll
-  for (int h = 0; h < GQA; ++h) {
-    const float mn = fmaxf(st.m[h], s[h]);
-    const float alpha = (st.m[h] == neg_inf()) ? 0.f : exp2f((st.m[h] - mn) * LOG2E);
-    const float pr = exp2f((s[h] - mn) * LOG2E);
-    st.m[h] = mn;
-    st.l[h] = st.l[h] * alpha + pr;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) st.acc[h][c] = st.acc[h][c] * alpha + pr * v[c];
-  }
-}
-
-
 // Un-rotated query (fp16 arithmetic, as the reference does it) and the query as given,
 // for the 4 heads of KV group `kv`; thread d < 128 handles channel d.
 __device__ __forceinline__ void stage_query(const ShardSeq& sq, int kv, int pos_q, const float* __restrict__ inv_freq,
@@ -112,93 +97,206 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
   quantize_vec_warp(src, sq.signs, cbs, idx_out, norm_out, lane);
 }
 
-// Rows outside the compressed middle, in one index space: u < n_sink + n_win + n_dec is an fp16
-// row (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  A warp takes rows u_first, u_first + u_step, ...;
-// lane owns channels 4*lane..+3.  `qr` is the query as given (fp32 copy in shared memory), `cbs`
-// the stream codebook in shared memory (needed for streamed rows only).
+// Rows outside the compressed middle, in one index space: u < n_sink + n_win + n_dec is an fp16 row
+// (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  A warp takes
+// rows u_first, u_first + u_step, ..., four at a time: lane owns channels 4*lane..+3 of every row, the
+// sixteen dot products (row, head) are summed over the lanes by halving (16 shuffles, which leave product
+// lane / 2 in the lane), so a lane weighs one (row, head) alone, and the weights go round by shuffle.
+//
+// A streamed row is never rotated back: its key is norm / sqrt(128) . signs o H(codebook[code]), so the
+// QUERY is taken to the code space (H(signs o q) / sqrt(128)) and the score is
+// norm . (query . codebook[code]); streamed values are summed in code space (weight . norm .
+// codebook[code]) and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of
+// accumulators serves both kinds.
+//
+// Bound: a warp's chain of dependent instructions (the unpack warps run this nearly alone on their
+// schedulers).  A streamed row with two butterflies and four full reductions of its own took 3 K cycles.
+// `qr` is the query as given (fp32 copy in shared memory), `cbs` the stream codebook in shared memory
+// (needed for streamed rows only).
+__device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u, const __half*& k, const __half*& v) {
+  const int n_sw = sh.n_sink + sh.n_win;
+  const bool in_sink = u < sh.n_sink, in_dec = u >= n_sw;
+  const int r = in_sink ? u : (in_dec ? u - n_sw : u - sh.n_sink);
+  const int rows = in_sink ? sh.n_sink : (in_dec ? (sh.dec_cap > 0 ? sh.dec_cap : sh.n_dec) : sh.n_win);
+  const size_t off = ((size_t)kv * rows + r) * HD;
+  k = reinterpret_cast<const __half*>(in_sink ? sq.sink_k : (in_dec ? sq.dec_k : sq.win_k)) + off;
+  v = reinterpret_cast<const __half*>(in_sink ? sq.sink_v : (in_dec ? sq.dec_v : sq.win_v)) + off;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
+// Asks for a warp's rows to be brought to the L2 cache (a step over many layers finds none of them there).
+// Only a hint, and the L2 is where all SMs and kernels meet, so it may be given before the launch in
+// front has finished.
+__device__ __forceinline__ void prefetch_rows(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u_first, int u_step, int lane) {
+  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, n_rows = n_fp + sh.n_stream;
+  for (int u = u_first + lane * u_step; u < n_rows; u += 32 * u_step) {
+    if (u < n_fp) {
+      const __half *k, *v;
+      fp16_row(sq, sh, kv, u, k, v);
+      prefetch_l2(k);
+      prefetch_l2(k + 64);
+      prefetch_l2(v);
+      prefetch_l2(v + 64);
+    } else {
+      const size_t row = (size_t)(u - n_fp) * sh.nkv + kv;
+      prefetch_l2(sq.st_k_idx + row * HD);
+      prefetch_l2(sq.st_v_idx + row * HD);
+      prefetch_l2(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
+      prefetch_l2(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
+    }
+  }
+  if (sh.n_stream > 0 && lane < 4) prefetch_l2(sq.signs + 32 * lane);
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& sq, const ShardDecodeShape& sh,
                                              int kv, int u_first, int u_step,
                                              const float* __restrict__ qr, const float* __restrict__ cbs, int lane) {
-  const int n_sw = sh.n_sink + sh.n_win, n_fp = n_sw + sh.n_dec, n_rows = n_fp + sh.n_stream;
+  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, n_rows = n_fp + sh.n_stream;
   if (u_first >= n_rows) return;
-  float4 qv[GQA];
+  // this warp's first streamed row
+  const int u_stream = u_first >= n_fp ? u_first : u_first + (n_fp - u_first + u_step - 1) / u_step * u_step;
+  const int row_own = lane >> 3;                         // the (row of a batch, head) this lane weighs
+  float m_own = neg_inf(), l_own = 0.f;                  // of that head; log2 domain
+  float4 q[GQA];
 #pragma unroll
-  for (int h = 0; h < GQA; ++h) qv[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
-  auto attend = [&](const float (&kx)[4], const float (&vx)[4]) {
-    float s[GQA];
+  for (int h = 0; h < GQA; ++h) q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
+  float4 sg = make_float4(0.f, 0.f, 0.f, 0.f);
+  bool stream = u_stream < n_rows;
+  if (stream) {
+    sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
 #pragma unroll
     for (int h = 0; h < GQA; ++h) {
-      float d = qv[h].x * kx[0];
-      d = fmaf(qv[h].y, kx[1], d);
-      d = fmaf(qv[h].z, kx[2], d);
-      s[h] = fmaf(qv[h].w, kx[3], d);
+      float x[4] = {q[h].x * sg.x, q[h].y * sg.y, q[h].z * sg.z, q[h].w * sg.w};
+      fwht128_lane4(x, lane);
+      q[h] = make_float4(x[0] * INV_SQRT_HD, x[1] * INV_SQRT_HD, x[2] * INV_SQRT_HD, x[3] * INV_SQRT_HD);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) s[h] += __shfl_xor_sync(0xffffffffu, s[h], o);   // four reductions side by side
-    }
-#pragma unroll
-    for (int h = 0; h < GQA; ++h) s[h] *= INV_SQRT_HD;
-    row_update(st, s, vx);
-  };
-  // ---- fp16 rows: sink, window, fp16 decode buffer ---------------------------------------------
-  int u = u_first;
-  for (; u < n_fp; u += u_step) {
-    const bool in_sink = u < sh.n_sink, in_dec = u >= n_sw;
-    const int r = in_sink ? u : (in_dec ? u - n_sw : u - sh.n_sink);
-    const int rows = in_sink ? sh.n_sink : (in_dec ? (sh.dec_cap > 0 ? sh.dec_cap : sh.n_dec) : sh.n_win);
-    const __half* kb = reinterpret_cast<const __half*>(in_sink ? sq.sink_k : (in_dec ? sq.dec_k : sq.win_k));
-    const __half* vb = reinterpret_cast<const __half*>(in_sink ? sq.sink_v : (in_dec ? sq.dec_v : sq.win_v));
-    const size_t off = ((size_t)kv * rows + r) * HD + 4 * lane;
-    const uint2 kr = __ldcg(reinterpret_cast<const uint2*>(kb + off));   // (the newest row was written a moment ago)
-    const uint2 vr = __ldcg(reinterpret_cast<const uint2*>(vb + off));
-    const float2 k01 = __half22float2(*reinterpret_cast<const __half2*>(&kr.x));
-    const float2 k23 = __half22float2(*reinterpret_cast<const __half2*>(&kr.y));
-    const float2 v01 = __half22float2(*reinterpret_cast<const __half2*>(&vr.x));
-    const float2 v23 = __half22float2(*reinterpret_cast<const __half2*>(&vr.y));
-    const float kx[4] = {k01.x, k01.y, k23.x, k23.y}, vx[4] = {v01.x, v01.y, v23.x, v23.y};
-    attend(kx, vx);
   }
-  // ---- streamed rows (u is this warp's first row behind the fp16 rows) ---------------------------
-  if (u >= n_rows) return;
-  const float4 sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
-  const float sgn[4] = {sg.x, sg.y, sg.z, sg.w};
-  // L2-coherent loads: a row may have been written by this CTA a moment ago (fused append).  The
-  // next row's codes and norms are fetched while the current row is worked on.
-  auto fetch = [&](int ur, uint32_t& kc, uint32_t& vc, unsigned short& kn16, unsigned short& vn16) {
-    const size_t row = (size_t)(ur - n_fp) * sh.nkv + kv;
-    kn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
-    vn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
-    kc = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + row * HD + 4 * lane));
-    vc = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + row * HD + 4 * lane));
+  uint2 kr[4], vr[4];                                    // the batch's rows: four codes (x), or four fp16 values
+  float kn, vn;                                          // norms of row `row_own`
+  // (L2-coherent loads: the newest row may have been written by this CTA a moment ago)
+  auto load = [&](int u0, int end) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int u = u0 + r * u_step;
+      kr[r] = vr[r] = make_uint2(0u, 0u);
+      if (u < end) {
+        if (stream) {
+          const size_t at = ((size_t)(u - n_fp) * sh.nkv + kv) * HD + 4 * lane;
+          kr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + at));
+          vr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + at));
+        } else {
+          const __half *k, *v;
+          fp16_row(sq, sh, kv, u, k, v);
+          kr[r] = __ldcg(reinterpret_cast<const uint2*>(k) + lane);
+          vr[r] = __ldcg(reinterpret_cast<const uint2*>(v) + lane);
+        }
+      }
+    }
+    kn = vn = 1.f;
+    const int u = u0 + row_own * u_step;
+    if (stream && u < end) {
+      const size_t row = (size_t)(u - n_fp) * sh.nkv + kv;
+      kn = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row)));
+      vn = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row)));
+    }
   };
-  uint32_t kc_next = 0u, vc_next = 0u;
-  unsigned short kn_next = 0, vn_next = 0;
-  fetch(u, kc_next, vc_next, kn_next, vn_next);
-  for (; u < n_rows; u += u_step) {
-    const uint32_t kc = kc_next, vc = vc_next;
-    const float kn = __half2float(__ushort_as_half(kn_next)), vn = __half2float(__ushort_as_half(vn_next));
-    if (u + u_step < n_rows) fetch(u + u_step, kc_next, vc_next, kn_next, vn_next);
-    // fp16 value of channels 4*lane..+3 exactly as the reference's dequantize_per_token + norm
-    // scaling produce it
-    float xk[4], xv[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      xk[i] = cbs[(kc >> (8 * i)) & 0xff];
-      xv[i] = cbs[(vc >> (8 * i)) & 0xff];
+  auto values = [&](uint2 raw, float (&x)[4]) {
+    if (stream) {
+      x[0] = cbs[raw.x & 0xff]; x[1] = cbs[(raw.x >> 8) & 0xff]; x[2] = cbs[(raw.x >> 16) & 0xff]; x[3] = cbs[raw.x >> 24];
+    } else {
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+      x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
     }
-    fwht128_lane4(xk, lane);
-    fwht128_lane4(xv, lane);
-    float kx[4], vx[4];
+  };
+  int u = stream ? u_stream : u_first, end = stream ? n_rows : n_fp;
+  load(u, end);
+#pragma unroll 1
+  while (true) {
+    // ---- scores --------------------------------------------------------------------------------------
+    float s[16];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const __half ku = __float2half_rn(__fmul_rn(__fdiv_rn(xk[i], SQRT_HD), sgn[i]));
-      const __half vu = __float2half_rn(__fmul_rn(__fdiv_rn(xv[i], SQRT_HD), sgn[i]));
-      kx[i] = __half2float(__float2half_rn(__fmul_rn(__half2float(ku), kn)));
-      vx[i] = __half2float(__float2half_rn(__fmul_rn(__half2float(vu), vn)));
+    for (int r = 0; r < 4; ++r) {
+      float x[4] = {0.f, 0.f, 0.f, 0.f};
+      if (u + r * u_step < end) values(kr[r], x);        // (uniform)
+#pragma unroll
+      for (int h = 0; h < GQA; ++h)
+        s[4 * r + h] = fmaf(q[h].x, x[0], fmaf(q[h].y, x[1], fmaf(q[h].z, x[2], q[h].w * x[3])));
     }
-    attend(kx, vx);
+#pragma unroll
+    for (int half = 8, off = 16; half >= 1; half >>= 1, off >>= 1) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int i = 0; i < half; ++i) {
+        const float keep = up ? s[i + half] : s[i], give = up ? s[i] : s[i + half];
+        s[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+    }
+    const float sum = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);      // product lane / 2 = (row_own, head)
+    const bool live = u + row_own * u_step < end;
+    const float sc = live ? sum * kn * (INV_SQRT_HD * LOG2E) : neg_inf();
+    float mx = fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 8));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));                // over the batch's rows (at least one is live)
+    const float mn = fmaxf(m_own, mx), al = ex2(m_own - mn), pr = ex2(sc - mn), pv = pr * vn;
+    m_own = mn;
+    l_own = fmaf(l_own, al, pr);
+    if (__any_sync(0xffffffffu, al != 1.f)) {
+#pragma unroll
+      for (int h = 0; h < GQA; ++h) {
+        const float a = __shfl_sync(0xffffffffu, al, 2 * h);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) st.acc[h][c] *= a;
+      }
+    }
+    // ---- values ---------------------------------------------------------------------------------------
+    uint2 vc[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) vc[r] = vr[r];
+    const int u_now = u, end_now = end;
+    const bool more = u + 4 * u_step < end;
+    u += 4 * u_step;
+    if (more) load(u, end);                              // the next batch on its way
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      if (u_now + r * u_step < end_now) {                // (uniform)
+        float x[4];
+        values(vc[r], x);
+#pragma unroll
+        for (int h = 0; h < GQA; ++h) {
+          const float p = __shfl_sync(0xffffffffu, pv, 8 * r + 2 * h);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) st.acc[h][c] = fmaf(p, x[c], st.acc[h][c]);
+        }
+      }
+    }
+    if (more) continue;
+    if (!stream) break;
+    // ---- the streamed sums back from the code space, the fp16 rows next ---------------------------------
+#pragma unroll
+    for (int h = 0; h < GQA; ++h) {
+      fwht128_lane4(st.acc[h], lane);
+      st.acc[h][0] *= sg.x * INV_SQRT_HD; st.acc[h][1] *= sg.y * INV_SQRT_HD;
+      st.acc[h][2] *= sg.z * INV_SQRT_HD; st.acc[h][3] *= sg.w * INV_SQRT_HD;
+      q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
+    }
+    stream = false;
+    u = u_first;
+    end = n_fp;
+    if (u >= end) break;
+    load(u, end);
+  }
+  // state per head (m, l the same in every lane): lanes 2 h + 8 r hold head h's sums of row r, twice
+  l_own += __shfl_xor_sync(0xffffffffu, l_own, 8);
+  l_own += __shfl_xor_sync(0xffffffffu, l_own, 16);
+#pragma unroll
+  for (int h = 0; h < GQA; ++h) {
+    st.m[h] = __shfl_sync(0xffffffffu, m_own, 2 * h) * LN2;
+    st.l[h] = __shfl_sync(0xffffffffu, l_own, 2 * h);
   }
 }
 

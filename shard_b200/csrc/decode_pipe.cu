@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     c_cnt[0] = n_my > 0 ? 1 : 0; c_cnt[1] = n_my > 1 ? 1 : 0;
     fence_mbar_init();
     if (n_my > 0) issue_coef(0);
-    for (int a = 0; a < W_ATOMS; ++a) {
+    for (int a = 0; a < W_ATOMS && n_my > 0; ++a) {      // (a CTA for rows alone needs no weights)
       mbar_expect_tx(W_FULL(a), 16384u);
       bulk_g2s(smem_u32(w_s + a * 16384), reinterpret_cast<const unsigned char*>(sq.k_wprep) + (size_t)kv * W_BYTES + a * 16384,
                16384u, W_FULL(a));
@@ -587,6 +587,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       tmem_st_x8(lane_A + R / 2, ones);
     }
     bool bad = false;
+    if (p.n_row_parts > 0) prefetch_rows(sq, sh, kv, part + p.n_row_parts * quad, p.n_row_parts * 4, lane);
     for (int it = 0; it < n_my && !bad; ++it) {
       bad = !mbar_wait(C_FULL(it & 1), (uint32_t)((it >> 1) & 1), abort_s);
       const uint4* row = reinterpret_cast<const uint4*>(c_s + (it & 1) * pp_c_bytes(NW) + m * (R / 2));
@@ -712,7 +713,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   }
   if (tid == 0 && *abort_s) {
     // gave up somewhere: do not leave while a bulk copy may still be landing in this CTA's memory
-    for (int a = 0; a < W_ATOMS; ++a) mbar_wait(W_FULL(a), 0u, abort_s);
+    for (int a = 0; a < W_ATOMS && n_my > 0; ++a) mbar_wait(W_FULL(a), 0u, abort_s);
     for (int b = 0; b < 2; ++b)
       if (c_cnt[b] > 0) mbar_wait(C_FULL(b), (uint32_t)((c_cnt[b] - 1) & 1), abort_s);
     if (p.status) atomicExch(p.status, 1);

@@ -98,8 +98,9 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
 }
 
 // Rows outside the compressed middle, in one index space: u < n_sink + n_win + n_dec is an fp16 row
-// (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  A warp takes
-// rows u_first, u_first + u_step, ..., four at a time: lane owns channels 4*lane..+3 of every row, the
+// (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  They are dealt
+// out in blocks of four of a kind, the fp16 rows' blocks first: a warp takes blocks b_first, b_first + b_step,
+// ....  Lane owns channels 4*lane..+3 of every row of a block, the
 // sixteen dot products (row, head) are summed over the lanes by halving (16 shuffles, which leave product
 // lane / 2 in the lane), so a lane weighs one (row, head) alone, and the weights go round by shuffle.
 //
@@ -109,8 +110,10 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
 // codebook[code]) and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of
 // accumulators serves both kinds.
 //
-// Bound: a warp's chain of dependent instructions (the unpack warps run this nearly alone on their
-// schedulers).  A streamed row with two butterflies and four full reductions of its own took 3 K cycles.
+// Bound: a warp's chain of dependent instructions and loads (the unpack warps run this nearly alone on
+// their schedulers): a block costs about the same with one row as with four, so with few rows no warp should
+// have two, and the next block's rows are on their way while one is worked on.  A streamed row with two
+// butterflies and four full reductions of its own took 3 K cycles.
 // `qr` is the query as given (fp32 copy in shared memory), `cbs` the stream codebook in shared memory
 // (needed for streamed rows only).
 __device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u, const __half*& k, const __half*& v) {
@@ -124,21 +127,30 @@ __device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeSh
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+constexpr int ROW_BLOCK = 4;
+// blocks of fp16 rows, blocks of streamed rows, and the block the newest row is in
+__host__ __device__ inline int row_blocks_fp16(const ShardDecodeShape& sh) { return (sh.n_sink + sh.n_win + sh.n_dec + ROW_BLOCK - 1) / ROW_BLOCK; }
+__host__ __device__ inline int row_blocks(const ShardDecodeShape& sh) { return row_blocks_fp16(sh) + (sh.n_stream + ROW_BLOCK - 1) / ROW_BLOCK; }
+
 // Asks for a warp's rows to be brought to the L2 cache (a step over many layers finds none of them there).
 // Only a hint, and the L2 is where all SMs and kernels meet, so it may be given before the launch in
 // front has finished.
-__device__ __forceinline__ void prefetch_rows(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u_first, int u_step, int lane) {
-  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, n_rows = n_fp + sh.n_stream;
-  for (int u = u_first + lane * u_step; u < n_rows; u += 32 * u_step) {
-    if (u < n_fp) {
+__device__ __forceinline__ void prefetch_rows(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int b_first, int b_step, int lane) {
+  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, fp_blocks = row_blocks_fp16(sh), blocks = row_blocks(sh);
+  for (int b = b_first + (lane >> 2) * b_step; b < blocks; b += 8 * b_step) {
+    const int r = lane & 3;
+    if (b < fp_blocks) {
+      if (4 * b + r >= n_fp) continue;
       const __half *k, *v;
-      fp16_row(sq, sh, kv, u, k, v);
+      fp16_row(sq, sh, kv, 4 * b + r, k, v);
       prefetch_l2(k);
       prefetch_l2(k + 64);
       prefetch_l2(v);
       prefetch_l2(v + 64);
     } else {
-      const size_t row = (size_t)(u - n_fp) * sh.nkv + kv;
+      const int u = 4 * (b - fp_blocks) + r;
+      if (u >= sh.n_stream) continue;
+      const size_t row = (size_t)u * sh.nkv + kv;
       prefetch_l2(sq.st_k_idx + row * HD);
       prefetch_l2(sq.st_v_idx + row * HD);
       prefetch_l2(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
@@ -155,19 +167,47 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& sq, const ShardDecodeShape& sh,
-                                             int kv, int u_first, int u_step,
+                                             int kv, int b_first, int b_step,
                                              const float* __restrict__ qr, const float* __restrict__ cbs, int lane) {
-  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, n_rows = n_fp + sh.n_stream;
-  if (u_first >= n_rows) return;
-  // this warp's first streamed row
-  const int u_stream = u_first >= n_fp ? u_first : u_first + (n_fp - u_first + u_step - 1) / u_step * u_step;
-  const int row_own = lane >> 3;                         // the (row of a batch, head) this lane weighs
+  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, fp_blocks = row_blocks_fp16(sh), blocks = row_blocks(sh);
+  if (b_first >= blocks) return;
+  int b_stream = b_first;                                // this warp's first block of streamed rows
+  if (b_stream < fp_blocks) b_stream += (fp_blocks - b_first + b_step - 1) / b_step * b_step;
+  const int row_own = lane >> 3;                         // the (row of a block, head) this lane weighs
   float m_own = neg_inf(), l_own = 0.f;                  // of that head; log2 domain
+  uint2 kr[4], vr[4];                                    // a block's rows: four codes (x), or four fp16 values
+  unsigned short kn16 = 0, vn16 = 0;                     // norms of row `row_own`
+  // (L2-coherent loads: the newest row may have been written by this CTA a moment ago)
+  auto load = [&](int b) {
+    if (b >= fp_blocks) {
+      const int u0 = 4 * (b - fp_blocks);
+      const size_t rs = (size_t)sh.nkv * HD, at = ((size_t)u0 * sh.nkv + kv) * HD + 4 * lane;
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {                      // (rows behind the last repeat it; they get no weight)
+        const size_t o = at + (size_t)min(r, sh.n_stream - 1 - u0) * rs;
+        kr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + o));
+        vr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + o));
+      }
+      const size_t row = (size_t)(u0 + min(row_own, sh.n_stream - 1 - u0)) * sh.nkv + kv;
+      kn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
+      vn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const __half *k, *v;
+        fp16_row(sq, sh, kv, min(4 * b + r, n_fp - 1), k, v);
+        kr[r] = __ldcg(reinterpret_cast<const uint2*>(k) + lane);
+        vr[r] = __ldcg(reinterpret_cast<const uint2*>(v) + lane);
+      }
+    }
+  };
+  bool stream = b_stream < blocks;
+  int b = stream ? b_stream : b_first;
+  load(b);
   float4 q[GQA];
 #pragma unroll
   for (int h = 0; h < GQA; ++h) q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
   float4 sg = make_float4(0.f, 0.f, 0.f, 0.f);
-  bool stream = u_stream < n_rows;
   if (stream) {
     sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
 #pragma unroll
@@ -177,57 +217,37 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
       q[h] = make_float4(x[0] * INV_SQRT_HD, x[1] * INV_SQRT_HD, x[2] * INV_SQRT_HD, x[3] * INV_SQRT_HD);
     }
   }
-  uint2 kr[4], vr[4];                                    // the batch's rows: four codes (x), or four fp16 values
-  float kn, vn;                                          // norms of row `row_own`
-  // (L2-coherent loads: the newest row may have been written by this CTA a moment ago)
-  auto load = [&](int u0, int end) {
+  auto values = [&](const uint2 (&raw)[4], float (&x)[4][4]) {
+    if (stream) {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int u = u0 + r * u_step;
-      kr[r] = vr[r] = make_uint2(0u, 0u);
-      if (u < end) {
-        if (stream) {
-          const size_t at = ((size_t)(u - n_fp) * sh.nkv + kv) * HD + 4 * lane;
-          kr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + at));
-          vr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + at));
-        } else {
-          const __half *k, *v;
-          fp16_row(sq, sh, kv, u, k, v);
-          kr[r] = __ldcg(reinterpret_cast<const uint2*>(k) + lane);
-          vr[r] = __ldcg(reinterpret_cast<const uint2*>(v) + lane);
-        }
+      for (int r = 0; r < 4; ++r) {
+        x[r][0] = cbs[raw[r].x & 0xff]; x[r][1] = cbs[(raw[r].x >> 8) & 0xff];
+        x[r][2] = cbs[(raw[r].x >> 16) & 0xff]; x[r][3] = cbs[raw[r].x >> 24];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].x)), c = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].y));
+        x[r][0] = a.x; x[r][1] = a.y; x[r][2] = c.x; x[r][3] = c.y;
       }
     }
-    kn = vn = 1.f;
-    const int u = u0 + row_own * u_step;
-    if (stream && u < end) {
-      const size_t row = (size_t)(u - n_fp) * sh.nkv + kv;
-      kn = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row)));
-      vn = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row)));
-    }
   };
-  auto values = [&](uint2 raw, float (&x)[4]) {
-    if (stream) {
-      x[0] = cbs[raw.x & 0xff]; x[1] = cbs[(raw.x >> 8) & 0xff]; x[2] = cbs[(raw.x >> 16) & 0xff]; x[3] = cbs[raw.x >> 24];
-    } else {
-      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-      x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-    }
-  };
-  int u = stream ? u_stream : u_first, end = stream ? n_rows : n_fp;
-  load(u, end);
 #pragma unroll 1
   while (true) {
     // ---- scores --------------------------------------------------------------------------------------
-    float s[16];
+    float s[16], x[4][4];
+    values(kr, x);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      float x[4] = {0.f, 0.f, 0.f, 0.f};
-      if (u + r * u_step < end) values(kr[r], x);        // (uniform)
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int h = 0; h < GQA; ++h)
-        s[4 * r + h] = fmaf(q[h].x, x[0], fmaf(q[h].y, x[1], fmaf(q[h].z, x[2], q[h].w * x[3])));
-    }
+        s[4 * r + h] = fmaf(q[h].x, x[r][0], fmaf(q[h].y, x[r][1], fmaf(q[h].z, x[r][2], q[h].w * x[r][3])));
+    values(vr, x);                                       // (the value rows' look-ups overlap the reduction)
+    const float kn = stream ? __half2float(__ushort_as_half(kn16)) : 1.f, vn = stream ? __half2float(__ushort_as_half(vn16)) : 1.f;
+    const bool live = (stream ? 4 * (b - fp_blocks) + row_own < sh.n_stream : 4 * b + row_own < n_fp);
+    const int next = b + b_step;
+    const bool more = next < (stream ? blocks : fp_blocks), turn = !more && stream && b_first < fp_blocks;
+    if (more || turn) load(more ? next : b_first);       // the next block on its way
 #pragma unroll
     for (int half = 8, off = 16; half >= 1; half >>= 1, off >>= 1) {
       const bool up = (lane & off) != 0;
@@ -238,10 +258,9 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
       }
     }
     const float sum = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);      // product lane / 2 = (row_own, head)
-    const bool live = u + row_own * u_step < end;
     const float sc = live ? sum * kn * (INV_SQRT_HD * LOG2E) : neg_inf();
     float mx = fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 8));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));                // over the batch's rows (at least one is live)
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));                // over the block's rows (at least one is live)
     const float mn = fmaxf(m_own, mx), al = ex2(m_own - mn), pr = ex2(sc - mn), pv = pr * vn;
     m_own = mn;
     l_own = fmaf(l_own, al, pr);
@@ -254,26 +273,15 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
       }
     }
     // ---- values ---------------------------------------------------------------------------------------
-    uint2 vc[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) vc[r] = vr[r];
-    const int u_now = u, end_now = end;
-    const bool more = u + 4 * u_step < end;
-    u += 4 * u_step;
-    if (more) load(u, end);                              // the next batch on its way
+    for (int r = 0; r < 4; ++r)
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      if (u_now + r * u_step < end_now) {                // (uniform)
-        float x[4];
-        values(vc[r], x);
+      for (int h = 0; h < GQA; ++h) {
+        const float p = __shfl_sync(0xffffffffu, pv, 8 * r + 2 * h);
 #pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const float p = __shfl_sync(0xffffffffu, pv, 8 * r + 2 * h);
-#pragma unroll
-          for (int c = 0; c < 4; ++c) st.acc[h][c] = fmaf(p, x[c], st.acc[h][c]);
-        }
+        for (int c = 0; c < 4; ++c) st.acc[h][c] = fmaf(p, x[r][c], st.acc[h][c]);
       }
-    }
+    b = next;
     if (more) continue;
     if (!stream) break;
     // ---- the streamed sums back from the code space, the fp16 rows next ---------------------------------
@@ -282,13 +290,12 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
       fwht128_lane4(st.acc[h], lane);
       st.acc[h][0] *= sg.x * INV_SQRT_HD; st.acc[h][1] *= sg.y * INV_SQRT_HD;
       st.acc[h][2] *= sg.z * INV_SQRT_HD; st.acc[h][3] *= sg.w * INV_SQRT_HD;
-      q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
     }
+    if (!turn) break;
+#pragma unroll
+    for (int h = 0; h < GQA; ++h) q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
     stream = false;
-    u = u_first;
-    end = n_fp;
-    if (u >= end) break;
-    load(u, end);
+    b = b_first;
   }
   // state per head (m, l the same in every lane): lanes 2 h + 8 r hold head h's sums of row r, twice
   l_own += __shfl_xor_sync(0xffffffffu, l_own, 8);

@@ -106,7 +106,7 @@ __device__ __forceinline__ bool named_bar_or(int id, int count, bool flag) {
 
 
 // A launch without a middle segment (a cache that holds fp16 and streamed rows only): every CTA
-// attends to its share of the rows (row u belongs to CTA u % gridDim.x, one warp per row), the CTA
+// attends to its share of the rows (block b of four belongs to CTA b % gridDim.x), the CTA
 // that owns the newest streamed row quantises it first, the last CTA of a KV head combines.
 constexpr int ROWS_THREADS = 512;
 constexpr int ROWS_SMEM_BYTES = (2 * GQA * HD + 256 + (ROWS_THREADS / 32) * GQA * 130) * 4;
@@ -116,8 +116,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) decode_rows_only_kernel(const
   const ShardDecodeShape& sh = p.sh;
   const int kv = blockIdx.y, part = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_rows = sh.n_sink + sh.n_win + sh.n_dec + sh.n_stream;
-  const bool append_here = sh.append && p.n_row_parts > 0 && (n_rows - 1) % p.n_row_parts == part;
+  const bool append_here = sh.append && p.n_row_parts > 0 && (row_blocks(sh) - 1) % p.n_row_parts == part;
   float* rec_rows = p.ws + (((size_t)blockIdx.z * p.n_parts + part) * sh.n_q + (size_t)kv * GQA) * PART;
   griddep_launch();
   griddep_wait();
@@ -178,9 +177,8 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* rec_base = p.ws + (((size_t)blockIdx.z * p.n_parts + part) * sh.n_q + (size_t)kv * GQA) * PART;
 
-  const int n_rows = sh.n_sink + sh.n_win + sh.n_dec + sh.n_stream;
   // the CTA that owns the newest streamed row quantises it before anybody reads the stream
-  const bool append_here = sh.append && p.n_row_parts > 0 && (n_rows - 1) % p.n_row_parts == part;
+  const bool append_here = sh.append && p.n_row_parts > 0 && (row_blocks(sh) - 1) % p.n_row_parts == part;
 
   griddep_launch();
 
@@ -620,8 +618,8 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       }
     }
     // The unpack warps run about three tiles ahead of the consumers.  In that slack they take this
-    // CTA's share of the fp16 / streamed rows (row u belongs to CTA u % n_row_parts), one warp per
-    // row.  The rows get a record of their own: standard V space, while the middle's record is in rotated space.
+    // CTA's share of the fp16 / streamed rows (block b of four rows belongs to CTA b % n_row_parts).
+    // The rows get a record of their own: standard V space, while the middle's record is in rotated space.
     // The coefficient staging buffers are free by now and serve as merge scratch.
     bad = named_bar_or(4, 128, bad || *abort_s);
     griddep_wait();

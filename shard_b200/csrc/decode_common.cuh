@@ -99,10 +99,10 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
 
 // Rows outside the compressed middle, in one index space: u < n_sink + n_win + n_dec is an fp16 row
 // (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  They are dealt
-// out in blocks of four of a kind, the fp16 rows' blocks first: a warp takes blocks b_first, b_first + b_step,
-// ....  Lane owns channels 4*lane..+3 of every row of a block, the
-// sixteen dot products (row, head) are summed over the lanes by halving (16 shuffles, which leave product
-// lane / 2 in the lane), so a lane weighs one (row, head) alone, and the weights go round by shuffle.
+// out in pairs of a kind, the fp16 rows' pairs first: a warp takes pairs b_first, b_first + b_step, ....
+// Lane owns channels 4*lane..+3 of both rows; the eight dot products (row, head) are summed over the lanes by
+// halving (9 shuffles, which leave product lane / 4 in the lane), so a lane weighs one (row, head) alone,
+// and the weights go round by shuffle.
 //
 // A streamed row is never rotated back: its key is norm / sqrt(128) . signs o H(codebook[code]), so the
 // QUERY is taken to the code space (H(signs o q) / sqrt(128)) and the score is
@@ -111,9 +111,9 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
 // accumulators serves both kinds.
 //
 // Bound: a warp's chain of dependent instructions and loads (the unpack warps run this nearly alone on
-// their schedulers): a block costs about the same with one row as with four, so with few rows no warp should
-// have two, and the next block's rows are on their way while one is worked on.  A streamed row with two
-// butterflies and four full reductions of its own took 3 K cycles.
+// their schedulers), so the code is kept short, and small in registers -- more of them, or a function of
+// its own, and the compiler spills in the tile loop.  A streamed row with two butterflies and four full
+// reductions of its own took 3 K cycles, a pair here about 1 K.
 // `qr` is the query as given (fp32 copy in shared memory), `cbs` the stream codebook in shared memory
 // (needed for streamed rows only).
 __device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u, const __half*& k, const __half*& v) {
@@ -125,40 +125,9 @@ __device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeSh
   k = reinterpret_cast<const __half*>(in_sink ? sq.sink_k : (in_dec ? sq.dec_k : sq.win_k)) + off;
   v = reinterpret_cast<const __half*>(in_sink ? sq.sink_v : (in_dec ? sq.dec_v : sq.win_v)) + off;
 }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
-constexpr int ROW_BLOCK = 4;
-// blocks of fp16 rows, blocks of streamed rows, and the block the newest row is in
-__host__ __device__ inline int row_blocks_fp16(const ShardDecodeShape& sh) { return (sh.n_sink + sh.n_win + sh.n_dec + ROW_BLOCK - 1) / ROW_BLOCK; }
-__host__ __device__ inline int row_blocks(const ShardDecodeShape& sh) { return row_blocks_fp16(sh) + (sh.n_stream + ROW_BLOCK - 1) / ROW_BLOCK; }
-
-// Asks for a warp's rows to be brought to the L2 cache (a step over many layers finds none of them there).
-// Only a hint, and the L2 is where all SMs and kernels meet, so it may be given before the launch in
-// front has finished.
-__device__ __forceinline__ void prefetch_rows(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int b_first, int b_step, int lane) {
-  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, fp_blocks = row_blocks_fp16(sh), blocks = row_blocks(sh);
-  for (int b = b_first + (lane >> 2) * b_step; b < blocks; b += 8 * b_step) {
-    const int r = lane & 3;
-    if (b < fp_blocks) {
-      if (4 * b + r >= n_fp) continue;
-      const __half *k, *v;
-      fp16_row(sq, sh, kv, 4 * b + r, k, v);
-      prefetch_l2(k);
-      prefetch_l2(k + 64);
-      prefetch_l2(v);
-      prefetch_l2(v + 64);
-    } else {
-      const int u = 4 * (b - fp_blocks) + r;
-      if (u >= sh.n_stream) continue;
-      const size_t row = (size_t)u * sh.nkv + kv;
-      prefetch_l2(sq.st_k_idx + row * HD);
-      prefetch_l2(sq.st_v_idx + row * HD);
-      prefetch_l2(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
-      prefetch_l2(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
-    }
-  }
-  if (sh.n_stream > 0 && lane < 4) prefetch_l2(sq.signs + 32 * lane);
-}
+// pairs of fp16 rows, and of all rows (the newest row is in the last)
+__host__ __device__ inline int row_pairs_fp16(const ShardDecodeShape& sh) { return (sh.n_sink + sh.n_win + sh.n_dec + 1) >> 1; }
+__host__ __device__ inline int row_pairs(const ShardDecodeShape& sh) { return row_pairs_fp16(sh) + ((sh.n_stream + 1) >> 1); }
 
 __device__ __forceinline__ float ex2(float x) {
   float r;
@@ -166,50 +135,48 @@ __device__ __forceinline__ float ex2(float x) {
   return r;
 }
 
+// st.m in the log2 domain
 __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& sq, const ShardDecodeShape& sh,
                                              int kv, int b_first, int b_step,
                                              const float* __restrict__ qr, const float* __restrict__ cbs, int lane) {
-  const int n_fp = sh.n_sink + sh.n_win + sh.n_dec, fp_blocks = row_blocks_fp16(sh), blocks = row_blocks(sh);
-  if (b_first >= blocks) return;
-  int b_stream = b_first;                                // this warp's first block of streamed rows
-  if (b_stream < fp_blocks) b_stream += (fp_blocks - b_first + b_step - 1) / b_step * b_step;
-  const int row_own = lane >> 3;                         // the (row of a block, head) this lane weighs
+  const int fp_pairs = row_pairs_fp16(sh), pairs = row_pairs(sh);
+  if (b_first >= pairs) return;
+  const int own = lane >> 4;                             // the (row of a pair, head lane / 4 % 4) this lane weighs
   float m_own = neg_inf(), l_own = 0.f;                  // of that head; log2 domain
-  uint2 kr[4], vr[4];                                    // a block's rows: four codes (x), or four fp16 values
-  unsigned short kn16 = 0, vn16 = 0;                     // norms of row `row_own`
-  // (L2-coherent loads: the newest row may have been written by this CTA a moment ago)
+  uint2 kr[2], vr[2];                                    // the next pair: four codes (x), or four fp16 values
+  unsigned short kn16 = 0, vn16 = 0;                     // norms of row `own`
+  // (L2-coherent loads: the newest row may have been written by this CTA a moment ago; a row behind the
+  // last repeats it and gets no weight)
   auto load = [&](int b) {
-    if (b >= fp_blocks) {
-      const int u0 = 4 * (b - fp_blocks);
-      const size_t rs = (size_t)sh.nkv * HD, at = ((size_t)u0 * sh.nkv + kv) * HD + 4 * lane;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {                      // (rows behind the last repeat it; they get no weight)
-        const size_t o = at + (size_t)min(r, sh.n_stream - 1 - u0) * rs;
-        kr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + o));
-        vr[r].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + o));
-      }
-      const size_t row = (size_t)(u0 + min(row_own, sh.n_stream - 1 - u0)) * sh.nkv + kv;
-      kn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
-      vn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
+    if (b >= fp_pairs) {
+      const int u = 2 * (b - fp_pairs), more = u + 1 < sh.n_stream ? 1 : 0;
+      const size_t row = (size_t)u * sh.nkv + kv, at = row * HD + 4 * lane, next = (size_t)(more * sh.nkv) * HD;
+      kr[0].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + at));
+      kr[1].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + at + next));
+      vr[0].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + at));
+      vr[1].x = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + at + next));
+      kn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row + own * more * sh.nkv);
+      vn16 = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row + own * more * sh.nkv);
     } else {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) {
+      for (int r = 0; r < 2; ++r) {
         const __half *k, *v;
-        fp16_row(sq, sh, kv, min(4 * b + r, n_fp - 1), k, v);
+        fp16_row(sq, sh, kv, min(2 * b + r, sh.n_sink + sh.n_win + sh.n_dec - 1), k, v);
         kr[r] = __ldcg(reinterpret_cast<const uint2*>(k) + lane);
         vr[r] = __ldcg(reinterpret_cast<const uint2*>(v) + lane);
       }
     }
   };
-  bool stream = b_stream < blocks;
-  int b = stream ? b_stream : b_first;
+  int b = b_first;
+  if (b < fp_pairs) b += (fp_pairs - b_first + b_step - 1) / b_step * b_step;
+  bool stream = b < pairs;
+  if (!stream) b = b_first;
   load(b);
   float4 q[GQA];
 #pragma unroll
   for (int h = 0; h < GQA; ++h) q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
-  float4 sg = make_float4(0.f, 0.f, 0.f, 0.f);
   if (stream) {
-    sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
+    const float4 sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
 #pragma unroll
     for (int h = 0; h < GQA; ++h) {
       float x[4] = {q[h].x * sg.x, q[h].y * sg.y, q[h].z * sg.z, q[h].w * sg.w};
@@ -217,39 +184,35 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
       q[h] = make_float4(x[0] * INV_SQRT_HD, x[1] * INV_SQRT_HD, x[2] * INV_SQRT_HD, x[3] * INV_SQRT_HD);
     }
   }
-  auto values = [&](const uint2 (&raw)[4], float (&x)[4][4]) {
+  auto values = [&](uint2 raw, float (&x)[4]) {
     if (stream) {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        x[r][0] = cbs[raw[r].x & 0xff]; x[r][1] = cbs[(raw[r].x >> 8) & 0xff];
-        x[r][2] = cbs[(raw[r].x >> 16) & 0xff]; x[r][3] = cbs[raw[r].x >> 24];
-      }
+      x[0] = cbs[raw.x & 0xff]; x[1] = cbs[(raw.x >> 8) & 0xff]; x[2] = cbs[(raw.x >> 16) & 0xff]; x[3] = cbs[raw.x >> 24];
     } else {
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].x)), c = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].y));
-        x[r][0] = a.x; x[r][1] = a.y; x[r][2] = c.x; x[r][3] = c.y;
-      }
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x)), c = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+      x[0] = a.x; x[1] = a.y; x[2] = c.x; x[3] = c.y;
     }
   };
 #pragma unroll 1
   while (true) {
     // ---- scores --------------------------------------------------------------------------------------
-    float s[16], x[4][4];
-    values(kr, x);
+    float s[8], x0[4], x1[4];
+    values(kr[0], x0);
+    values(kr[1], x1);
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int h = 0; h < GQA; ++h)
-        s[4 * r + h] = fmaf(q[h].x, x[r][0], fmaf(q[h].y, x[r][1], fmaf(q[h].z, x[r][2], q[h].w * x[r][3])));
-    values(vr, x);                                       // (the value rows' look-ups overlap the reduction)
+    for (int h = 0; h < GQA; ++h) {
+      s[h] = fmaf(q[h].x, x0[0], fmaf(q[h].y, x0[1], fmaf(q[h].z, x0[2], q[h].w * x0[3])));
+      s[4 + h] = fmaf(q[h].x, x1[0], fmaf(q[h].y, x1[1], fmaf(q[h].z, x1[2], q[h].w * x1[3])));
+    }
+    values(vr[0], x0);                                   // (the value rows' look-ups overlap the reduction)
+    values(vr[1], x1);
     const float kn = stream ? __half2float(__ushort_as_half(kn16)) : 1.f, vn = stream ? __half2float(__ushort_as_half(vn16)) : 1.f;
-    const bool live = (stream ? 4 * (b - fp_blocks) + row_own < sh.n_stream : 4 * b + row_own < n_fp);
-    const int next = b + b_step;
-    const bool more = next < (stream ? blocks : fp_blocks), turn = !more && stream && b_first < fp_blocks;
-    if (more || turn) load(more ? next : b_first);       // the next block on its way
+    const bool live = stream ? 2 * (b - fp_pairs) + own < sh.n_stream : 2 * b + own < sh.n_sink + sh.n_win + sh.n_dec;
+    b += b_step;
+    const bool more = b < (stream ? pairs : fp_pairs), turn = !more && stream && b_first < fp_pairs;
+    if (turn) b = b_first;
+    if (more || turn) load(b);                           // the next pair on its way
 #pragma unroll
-    for (int half = 8, off = 16; half >= 1; half >>= 1, off >>= 1) {
+    for (int half = 4, off = 16; half >= 1; half >>= 1, off >>= 1) {
       const bool up = (lane & off) != 0;
 #pragma unroll
       for (int i = 0; i < half; ++i) {
@@ -257,34 +220,24 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
         s[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
       }
     }
-    const float sum = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);      // product lane / 2 = (row_own, head)
-    const float sc = live ? sum * kn * (INV_SQRT_HD * LOG2E) : neg_inf();
-    float mx = fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 8));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));                // over the block's rows (at least one is live)
-    const float mn = fmaxf(m_own, mx), al = ex2(m_own - mn), pr = ex2(sc - mn), pv = pr * vn;
+    float sc = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 2);
+    sc += __shfl_xor_sync(0xffffffffu, sc, 1);           // product lane / 4 = (own, head)
+    sc = live ? sc * kn * (INV_SQRT_HD * LOG2E) : neg_inf();
+    const float mn = fmaxf(m_own, fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 16)));   // (at least one row is live)
+    const float al = ex2(m_own - mn), pr = ex2(sc - mn), pv = pr * vn;
     m_own = mn;
     l_own = fmaf(l_own, al, pr);
-    if (__any_sync(0xffffffffu, al != 1.f)) {
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) {
-        const float a = __shfl_sync(0xffffffffu, al, 2 * h);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) st.acc[h][c] *= a;
-      }
-    }
     // ---- values ---------------------------------------------------------------------------------------
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int h = 0; h < GQA; ++h) {
+      const float a = __shfl_sync(0xffffffffu, al, 4 * h), p0 = __shfl_sync(0xffffffffu, pv, 4 * h), p1 = __shfl_sync(0xffffffffu, pv, 16 + 4 * h);
 #pragma unroll
-      for (int h = 0; h < GQA; ++h) {
-        const float p = __shfl_sync(0xffffffffu, pv, 8 * r + 2 * h);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) st.acc[h][c] = fmaf(p, x[r][c], st.acc[h][c]);
-      }
-    b = next;
+      for (int c = 0; c < 4; ++c) st.acc[h][c] = fmaf(p1, x1[c], fmaf(p0, x0[c], st.acc[h][c] * a));
+    }
     if (more) continue;
     if (!stream) break;
     // ---- the streamed sums back from the code space, the fp16 rows next ---------------------------------
+    const float4 sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
 #pragma unroll
     for (int h = 0; h < GQA; ++h) {
       fwht128_lane4(st.acc[h], lane);
@@ -295,22 +248,20 @@ __device__ __forceinline__ void process_rows(SoftmaxState& st, const ShardSeq& s
 #pragma unroll
     for (int h = 0; h < GQA; ++h) q[h] = *reinterpret_cast<const float4*>(qr + h * HD + 4 * lane);
     stream = false;
-    b = b_first;
   }
-  // state per head (m, l the same in every lane): lanes 2 h + 8 r hold head h's sums of row r, twice
-  l_own += __shfl_xor_sync(0xffffffffu, l_own, 8);
+  // state per head, the same in every lane: lanes 4 h + 16 r hold head h's sums of row r
   l_own += __shfl_xor_sync(0xffffffffu, l_own, 16);
 #pragma unroll
   for (int h = 0; h < GQA; ++h) {
-    st.m[h] = __shfl_sync(0xffffffffu, m_own, 2 * h) * LN2;
-    st.l[h] = __shfl_sync(0xffffffffu, l_own, 2 * h);
+    st.m[h] = __shfl_sync(0xffffffffu, m_own, 4 * h);
+    st.l[h] = __shfl_sync(0xffffffffu, l_own, 4 * h);
   }
 }
 
-// Merge of per-warp softmax states (lane owns channels 4*lane..+3, m/l are warp-uniform) into one
+// Merge of per-warp softmax states (lane owns channels 4*lane..+3, m/l are warp-uniform, m in the log2
+// domain) into one
 // record per head, in two steps with a barrier of the caller's choice in between:
-// partial_store by every one of the NWARPS warps (index `w`), then partial_merge by 128 threads
-// (d = 0..127).  `scratch` needs NWARPS*4*130 floats.
+// partial_store by every one of the NWARPS warps (index `w`), then partial_merge by four warps.  `scratch` needs NWARPS*4*130 floats.
 template <int NWARPS>
 __device__ __forceinline__ void partial_store(const SoftmaxState& st, float* __restrict__ scratch, int w, int lane) {
   float* mw = scratch;
@@ -326,28 +277,33 @@ __device__ __forceinline__ void partial_store(const SoftmaxState& st, float* __r
         make_float4(st.acc[h][0], st.acc[h][1], st.acc[h][2], st.acc[h][3]);
 }
 
-template <int NWARPS>
-__device__ __forceinline__ void partial_merge(const float* scratch, float* __restrict__ rec_base, int d) {
+// Warp `h` < 4 merges query head h; ROTATED: into the rotated space of the middle's accumulator
+// (normalised Hadamard over the channels; the combine's inverse takes it back).
+template <int NWARPS, bool ROTATED>
+__device__ __forceinline__ void partial_merge(const float* scratch, float* __restrict__ rec_base, int h, int lane) {
   const float* mw = scratch;
   const float* lw = mw + NWARPS * GQA;
   const float* aw = lw + NWARPS * GQA;
+  float M = neg_inf();
 #pragma unroll
-  for (int h = 0; h < GQA; ++h) {
-    float M = neg_inf();
+  for (int w = 0; w < NWARPS; ++w) M = fmaxf(M, mw[w * GQA + h]);
+  float L = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int w = 0; w < NWARPS; ++w) M = fmaxf(M, mw[w * GQA + h]);
-    float L = 0.f, a = 0.f;
-#pragma unroll
-    for (int w = 0; w < NWARPS; ++w) {
-      const float mwv = mw[w * GQA + h];
-      const float wt = (mwv == neg_inf()) ? 0.f : exp2f((mwv - M) * LOG2E);
-      L = fmaf(wt, lw[w * GQA + h], L);
-      a = fmaf(wt, aw[(w * GQA + h) * HD + d], a);
-    }
-    float* rec = rec_base + h * PART;
-    if (d == 0) { rec[0] = M; rec[1] = L; rec[2] = 0.f; rec[3] = 0.f; }
-    rec[4 + d] = a;
+  for (int w = 0; w < NWARPS; ++w) {
+    const float mwv = mw[w * GQA + h];
+    const float wt = (mwv == neg_inf()) ? 0.f : ex2(mwv - M);
+    const float4 v = *reinterpret_cast<const float4*>(aw + (w * GQA + h) * HD + 4 * lane);
+    L = fmaf(wt, lw[w * GQA + h], L);
+    a[0] = fmaf(wt, v.x, a[0]); a[1] = fmaf(wt, v.y, a[1]); a[2] = fmaf(wt, v.z, a[2]); a[3] = fmaf(wt, v.w, a[3]);
   }
+  if (ROTATED) {
+    fwht128_lane4(a, lane);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[c] *= INV_SQRT_HD;
+  }
+  float* rec = rec_base + h * PART;
+  if (lane == 0) *reinterpret_cast<float4*>(rec) = make_float4(M * LN2, L, 0.f, 0.f);    // (the record carries the natural-log maximum)
+  *reinterpret_cast<float4*>(rec + 4 + 4 * lane) = make_float4(a[0], a[1], a[2], a[3]);
 }
 
 // Fused combine.  Every CTA of one (sequence, KV head) calls this after its record is written

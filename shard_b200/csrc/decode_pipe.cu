@@ -106,7 +106,7 @@ __device__ __forceinline__ bool named_bar_or(int id, int count, bool flag) {
 
 
 // A launch without a middle segment (a cache that holds fp16 and streamed rows only): every CTA
-// attends to its share of the rows (block b of four belongs to CTA b % gridDim.x), the CTA
+// attends to its share of the rows (pair b belongs to CTA b % gridDim.x), the CTA
 // that owns the newest streamed row quantises it first, the last CTA of a KV head combines.
 constexpr int ROWS_THREADS = 512;
 constexpr int ROWS_SMEM_BYTES = (2 * GQA * HD + 256 + (ROWS_THREADS / 32) * GQA * 130) * 4;
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) decode_rows_only_kernel(const
   const ShardDecodeShape& sh = p.sh;
   const int kv = blockIdx.y, part = blockIdx.x;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool append_here = sh.append && p.n_row_parts > 0 && (row_blocks(sh) - 1) % p.n_row_parts == part;
+  const bool append_here = sh.append && p.n_row_parts > 0 && (row_pairs(sh) - 1) % p.n_row_parts == part;
   float* rec_rows = p.ws + (((size_t)blockIdx.z * p.n_parts + part) * sh.n_q + (size_t)kv * GQA) * PART;
   griddep_launch();
   griddep_wait();
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) decode_rows_only_kernel(const
   process_rows(st, sq, sh, kv, part + p.n_row_parts * warp, p.n_row_parts * (ROWS_THREADS / 32), qr, cbs, lane);
   partial_store<ROWS_THREADS / 32>(st, scratch, warp, lane);
   __syncthreads();
-  if (tid < HD) partial_merge<ROWS_THREADS / 32>(scratch, rec_rows, tid);
+  if (warp < GQA) partial_merge<ROWS_THREADS / 32, false>(scratch, rec_rows, warp, lane);
   ticket_combine<ROWS_THREADS>(p, sq, kv, blockIdx.z, scratch, tid);
 }
 
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   float* rec_base = p.ws + (((size_t)blockIdx.z * p.n_parts + part) * sh.n_q + (size_t)kv * GQA) * PART;
 
   // the CTA that owns the newest streamed row quantises it before anybody reads the stream
-  const bool append_here = sh.append && p.n_row_parts > 0 && (row_blocks(sh) - 1) % p.n_row_parts == part;
+  const bool append_here = sh.append && p.n_row_parts > 0 && (row_pairs(sh) - 1) % p.n_row_parts == part;
 
   griddep_launch();
 
@@ -585,7 +585,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       tmem_st_x8(lane_A + R / 2, ones);
     }
     bool bad = false;
-    if (p.n_row_parts > 0) prefetch_rows(sq, sh, kv, part + p.n_row_parts * quad, p.n_row_parts * 4, lane);
     for (int it = 0; it < n_my && !bad; ++it) {
       bad = !mbar_wait(C_FULL(it & 1), (uint32_t)((it >> 1) & 1), abort_s);
       const uint4* row = reinterpret_cast<const uint4*>(c_s + (it & 1) * pp_c_bytes(NW) + m * (R / 2));
@@ -618,8 +617,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       }
     }
     // The unpack warps run about three tiles ahead of the consumers.  In that slack they take this
-    // CTA's share of the fp16 / streamed rows (block b of four rows belongs to CTA b % n_row_parts).
-    // The rows get a record of their own: standard V space, while the middle's record is in rotated space.
+    // CTA's share of the fp16 / streamed rows (pair b belongs to CTA b % n_row_parts) and leave its state,
+    // in the rotated space of the middle's accumulator, for the epilogue.  (Some rows behind every tile
+    // instead of all behind the last: the unpack is on the tile loop's critical path, 12 to 30 % slower.)
     // The coefficient staging buffers are free by now and serve as merge scratch.
     bad = named_bar_or(4, 128, bad || *abort_s);
     griddep_wait();
@@ -632,34 +632,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       float* scratch = reinterpret_cast<float*>(c_s);
       partial_store<4>(st, scratch, quad, lane);
       named_bar_sync(4, 128);
-      partial_merge<4>(scratch, rows_rec_s, m);
-      // Into the rotated space of the middle's accumulator (normalised Hadamard over the channels of
-      // each head; the combine's inverse transform takes it back): the CTA then has one record.
-      float v[GQA];
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) v[h] = rows_rec_s[h * PART + 4 + m];
-#pragma unroll
-      for (int hh = 1; hh < 32; hh <<= 1) {
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const float other = __shfl_xor_sync(0xffffffffu, v[h], hh);
-          v[h] = (m & hh) ? other - v[h] : v[h] + other;
-        }
-      }
-      for (int hh = 32; hh < HD; hh <<= 1) {
-        named_bar_sync(4, 128);
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) rows_rec_s[h * PART + 4 + m] = v[h];
-        named_bar_sync(4, 128);
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const float other = rows_rec_s[h * PART + 4 + (m ^ hh)];
-          v[h] = (m & hh) ? other - v[h] : v[h] + other;
-        }
-      }
-      named_bar_sync(4, 128);
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) rows_rec_s[h * PART + 4 + m] = v[h] / SQRT_HD;
+      partial_merge<4, true>(scratch, rows_rec_s, quad, lane);
     } else {
       // no rows for this launch (or gave up): an empty state
 #pragma unroll

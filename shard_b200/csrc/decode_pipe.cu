@@ -56,6 +56,7 @@ constexpr int PP_TMEM_COLS = 512;
 // constant columns 1, 0, ...), and per consumer group 16 columns of scores + 16 of P.V accumulator
 constexpr int PP_COL_A = 256;
 constexpr int PP_COL_SO = 360;
+constexpr int ROW_STATE = GQA * HD + 2 * GQA;   // a consumer warp's row sums: acc[4][128], max[4], sum-exp[4]
 constexpr float PP_LAZY_LOG2 = 8.f;   // a softmax reference point moves only when exceeded by more than 2^8
 constexpr int PP_V_BYTES = 32768, PP_P_BYTES = 4096, PP_Q_BYTES = 4096;
 constexpr int PP_CB_COPIES = 4;       // interleaved copies of the V codebook: lane l reads copy l % 4, entry e of copy c at 4e + c
@@ -180,6 +181,10 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   // the CTA that owns the newest streamed row quantises it before anybody reads the stream
   const bool append_here = sh.append && p.n_row_parts > 0 && (row_pairs(sh) - 1) % p.n_row_parts == part;
 
+  // The rows are the unpack warps' (they run about three tiles ahead of the consumers); with more than
+  // eight pairs for each of them all sixteen warps take a share.
+  const bool wide_rows = p.n_row_parts > 0 && row_pairs(sh) > 32 * p.n_row_parts;
+
   griddep_launch();
 
   // barrier addresses
@@ -255,6 +260,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  bool rows_ok = false;
   float acc[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) acc[j] = 0.f;
@@ -575,6 +581,17 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     // giving up: do not leave while a copy this thread asked for may still be landing
     if ((bad || *abort_s) && issuer && vc_issued > 0)
       mbar_wait(V_FULL(g), (uint32_t)((vc_issued - 1) & 1), abort_s);
+    // every consumer group parks its state in its own V tile (its last MMA3 has completed), so one CTA
+    // barrier separates the tile loops from the merge
+    float* acc_g = reinterpret_cast<float*>(v_g);      // [16][128], then the row sums (wide rows)
+#pragma unroll
+    for (int h = 0; h < GQA; ++h) {
+      const float l = warp_sum(run_l[h]);
+      if (lane == 0) { m_s[16 * g + 4 * quad + h] = run_m[h]; l_s[16 * g + 4 * quad + h] = l; }
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc_g[j * HD + m] = acc[j];
+    rows_ok = !bad;
   } else {
     // =============================== unpack warps =========================================
     const int quad = warp - PP_UNPACK_WARP0, m = quad * 32 + lane;
@@ -616,48 +633,45 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
         if (lane == 0) mbar_arrive(A_FULL(j));          // this warp's rows of the third are in place
       }
     }
-    // The unpack warps run about three tiles ahead of the consumers.  In that slack they take this
-    // CTA's share of the fp16 / streamed rows (pair b belongs to CTA b % n_row_parts) and leave its state,
-    // in the rotated space of the middle's accumulator, for the epilogue.  (Some rows behind every tile
-    // instead of all behind the last: the unpack is on the tile loop's critical path, 12 to 30 % slower.)
-    // The coefficient staging buffers are free by now and serve as merge scratch.
+    // the coefficient staging buffers are free by now and serve as the rows' merge scratch
     bad = named_bar_or(4, 128, bad || *abort_s);
     griddep_wait();
-    if (!bad && p.n_row_parts > 0) {
-      bad = !mbar_wait(Q_READY, 0u, abort_s);
-      if (append_here) bad |= !mbar_wait(APPEND_DONE, 0u, abort_s);
-      SoftmaxState st;
-      softmax_init(st);
-      if (!bad) process_rows(st, sq, sh, kv, part + p.n_row_parts * quad, p.n_row_parts * 4, qr_s, cbs_s, lane);
+    rows_ok = !bad;
+  }
+
+  // ---- rows: this warp's share of the fp16 and streamed rows (pair b belongs to CTA b % n_row_parts); the
+  // unpack warps merge theirs into one state, in the rotated space of the middle's accumulator.  (Some rows
+  // behind every tile instead of all behind the last: the unpack is on the tile loop's critical path, 12 to
+  // 30 % slower.) -------------------------------------------------------------------------------------------
+  if (warp >= PP_CONS_WARPS || wide_rows) {
+    const int row_w = (warp + 4) & 15;                    // unpack warps first
+    SoftmaxState st;
+    softmax_init(st);
+    if (rows_ok && p.n_row_parts > 0) {
+      rows_ok = mbar_wait(Q_READY, 0u, abort_s);
+      if (append_here) rows_ok = rows_ok && mbar_wait(APPEND_DONE, 0u, abort_s);
+      if (rows_ok)
+        process_rows(st, sq, sh, kv, part + p.n_row_parts * row_w, p.n_row_parts * (wide_rows ? 16 : 4), qr_s, cbs_s, lane);
+    }
+    if (row_w < 4) {
       float* scratch = reinterpret_cast<float*>(c_s);
-      partial_store<4>(st, scratch, quad, lane);
+      partial_store<4>(st, scratch, row_w, lane);
       named_bar_sync(4, 128);
-      partial_merge<4, true>(scratch, rows_rec_s, quad, lane);
+      partial_merge<4, true>(scratch, rows_rec_s, row_w, lane);
     } else {
-      // no rows for this launch (or gave up): an empty state
+      float* sums = reinterpret_cast<float*>(v_s + ((row_w - 4) >> 2) * PP_V_BYTES + 8192) + (row_w & 3) * ROW_STATE;
 #pragma unroll
       for (int h = 0; h < GQA; ++h) {
-        if (m == 0) { rows_rec_s[h * PART] = neg_inf(); rows_rec_s[h * PART + 1] = 0.f; }
-        rows_rec_s[h * PART + 4 + m] = 0.f;
+        fwht128_lane4(st.acc[h], lane);
+        *reinterpret_cast<float4*>(sums + h * HD + 4 * lane) = make_float4(st.acc[h][0] * INV_SQRT_HD, st.acc[h][1] * INV_SQRT_HD,
+                                                                           st.acc[h][2] * INV_SQRT_HD, st.acc[h][3] * INV_SQRT_HD);
+        if (lane == 0) { sums[GQA * HD + h] = st.m[h]; sums[GQA * HD + GQA + h] = st.l[h]; }
       }
     }
   }
 
   // ---- epilogue: merge the 12 token-warps' states per head and emit the record -------------------
-  // every consumer group parks its state in its own V tile (its last MMA3 has completed), so one
-  // CTA barrier separates the tile loops from the merge
   const float ch_scale = __half2float(reinterpret_cast<const __half*>(sq.v_ch)[kv * HD + (tid & 127)]);
-  if (warp < PP_CONS_WARPS) {
-    const int g = warp >> 2, quad = warp & 3, m = quad * 32 + lane;
-    float* acc_g = reinterpret_cast<float*>(v_s + g * PP_V_BYTES);   // [16][128]
-#pragma unroll
-    for (int h = 0; h < GQA; ++h) {
-      const float l = warp_sum(run_l[h]);
-      if (lane == 0) { m_s[16 * g + 4 * quad + h] = run_m[h]; l_s[16 * g + 4 * quad + h] = l; }
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc_g[j * HD + m] = acc[j];
-  }
   __syncthreads();
   {
     // run_m is kept in the log2 domain (score * log2 e); the record carries the natural-log maximum
@@ -665,6 +679,11 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     // the rows' state (natural-log reference, already in rotated space and final units)
     const float rows_m = rows_rec_s[h * PART] * LOG2E, rows_l = rows_rec_s[h * PART + 1], rows_a = rows_rec_s[h * PART + 4 + m];
     float M = rows_m;
+    auto row_state = [&](int e) { return reinterpret_cast<const float*>(v_s + (e >> 2) * PP_V_BYTES + 8192) + (e & 3) * ROW_STATE; };
+    if (wide_rows) {
+#pragma unroll 1
+      for (int e = 0; e < 12; ++e) M = fmaxf(M, row_state(e)[GQA * HD + h]);
+    }
 #pragma unroll
     for (int e = 0; e < 12; ++e) M = fmaxf(M, m_s[16 * (e >> 2) + 4 * (e & 3) + h]);
     float L = 0.f, a = 0.f;
@@ -678,9 +697,19 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     }
     const float wr = (rows_m == neg_inf()) ? 0.f : exp2f(rows_m - M);
     L = fmaf(wr, rows_l, L);
+    float ra = wr * rows_a;
+    if (wide_rows) {
+#pragma unroll 1
+      for (int e = 0; e < 12; ++e) {
+        const float* rs = row_state(e);
+        const float mv = rs[GQA * HD + h], wt = (mv == neg_inf()) ? 0.f : exp2f(mv - M);
+        L = fmaf(wt, rs[GQA * HD + GQA + h], L);
+        ra = fmaf(wt, rs[h * HD + m], ra);
+      }
+    }
     float* rec = rec_base + h * PART;
     if (m == 0) { rec[0] = M * LN2; rec[1] = L; rec[2] = 0.f; rec[3] = 0.f; }
-    rec[4 + m] = fmaf(wr, rows_a, a * ch_scale);
+    rec[4 + m] = fmaf(a, ch_scale, ra);
   }
   if (tid == 0 && *abort_s) {
     // gave up somewhere: do not leave while a bulk copy may still be landing in this CTA's memory

@@ -1,0 +1,34 @@
+"""Decode attention with few and with many rows outside the compressed middle (fp16 or streamed): pairs and
+odd rows, all warps on the rows, more row CTAs than tiles, against float64 attention over the read-back."""
+import pytest
+import torch
+
+from gpu_helpers import random_gc
+from test_gpu_readback import _cache
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_comp,nkv,rows,streaming", [
+    (700, 8, 1, True), (700, 8, 2, False), (130, 8, 75, True), (130, 8, 76, False), (1, 2, 700, False), (1, 8, 901, True),
+    (2560, 8, 1153, True), (2560, 8, 1100, False), (5000, 8, 3001, True), (300, 1, 4001, True)])
+def test_decode_rows(n_comp, nkv, rows, streaming):
+    from shard_b200 import fused_attention_compressed
+    cache, layer = _cache(random_gc(n_comp, nkv=nkv, seed=rows), nkv, streaming, capacity=rows + 4)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda").half() for _ in range(2))
+    cache._fused_decode_update = True
+    if rows > 1:
+        layer.update(k[:, :, :-1], v[:, :, :-1])
+    for step in range(2):
+        if step == 0:
+            layer.update(k[:, :, -1:], v[:, :, -1:])       # the newest row is written by the decode launch
+        q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+        out = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)
+        cache.check()
+        layer._needs_decompress = True
+        keys, values = layer.keys[0].double(), layer.values[0].double()
+        sc = torch.einsum("hqd,hnd->hqn", q[0].double(), keys.repeat_interleave(4, 0)) / 128 ** 0.5
+        want = torch.softmax(sc, -1) @ values.repeat_interleave(4, 0)
+        err = (out[0].double() - want).abs()
+        assert (err <= 1.5e-3 + 5e-3 * want.abs()).all(), err.max()

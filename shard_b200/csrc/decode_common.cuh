@@ -307,11 +307,12 @@ __device__ __forceinline__ void partial_merge(const float* scratch, float* __res
 }
 
 // Fused combine.  Every CTA of one (sequence, KV head) calls this after its record is written
-// (`released`: the caller has already issued __threadfence + __syncthreads after those writes).
-// Each takes a ticket; the CTA that draws the last one sees all records of that KV head
-// (release/acquire through the fences around the ticket), merges them for the head's four
+// (`synced`: the caller has already synchronised the CTA after those writes).
+// Each takes a ticket; the CTA that draws the last one sees all records of that KV head (the ticket's
+// thread releases the CTA's writes, which the barrier has ordered before it, and acquires the others';
+// fences by every thread cost 2 K cycles more), merges them for the head's four
 // query heads, and puts the counter back to zero for the next call.  The result does not depend
-// on which CTA is last: the parts are always summed in the same order.  `sm` needs 3072 floats
+// on which CTA is last: the parts are always summed in the same order.  `sm` needs 1536 floats
 // (or GQA*HD + 2*GQA*n_parts + 8 for more than 64 parts) that are free; NTHREADS >= 512.
 //
 // The merging CTA is the critical path of the whole launch and runs this code once, out of a
@@ -323,24 +324,26 @@ __device__ __forceinline__ void partial_merge(const float* scratch, float* __res
 // 128 channels (two butterflies inside the thread, five by shuffle) and writes the output.
 template <int NTHREADS>
 __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const ShardSeq& sq, int kv, int b,
-                                               float* sm_raw, int tid, bool released = false) {
+                                               float* sm_raw, int tid, bool synced = false) {
   volatile float* sm = sm_raw;   // exchanged between threads: every access must reach shared memory
   static_assert(NTHREADS >= GQA * HD, "16 merging warps");
   __shared__ int last_s;
-  if (!released) {               // the caller has not yet fenced its record writes and synchronised the CTA
-    __threadfence();
-    __syncthreads();
-  }
+  if (!synced) __syncthreads();
   if (tid == 0) {
     int* ctr = p.tickets + b * p.sh.nkv + kv;
+    __threadfence();
     const int last = atomicAdd(ctr, 1) == p.n_ctas - 1;
-    if (last) atomicExch(ctr, 0);
+    if (last) {
+      __threadfence();
+      *reinterpret_cast<volatile int*>(ctr) = 0;         // (nobody looks at it before the next launch)
+    }
     last_s = last;
   }
   __syncthreads();
   if (!last_s) return;
-  __threadfence();
-  const int n_q = p.sh.n_q, n_parts = p.n_parts, n_rot = p.n_chunks;
+  // (the records of a launch are all of a kind: in rotated space, or, without a middle segment, standard)
+  const int n_q = p.sh.n_q, n_parts = p.n_parts;
+  const bool rotated = p.n_chunks > 0;
   const int w = tid >> 5, lane = tid & 31;
   const float* base0 = p.ws + ((size_t)b * n_parts * n_q + (size_t)kv * GQA) * PART;
   const size_t pstride = (size_t)n_q * PART;
@@ -348,7 +351,6 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
   float M = neg_inf(), L = 0.f;                       // of head w % 4 (the same in every lane)
   float o4[4] = {0.f, 0.f, 0.f, 0.f};                 // channels 4*lane .. 4*lane+3 of head w (fin threads)
   if (n_parts <= 64) {
-    float rot4[4] = {0.f, 0.f, 0.f, 0.f}, std4[4] = {0.f, 0.f, 0.f, 0.f};
     if (w < 16) {
       const int hl = w & 3, sub = w >> 2;
       const float* rec0 = base0 + hl * PART;
@@ -381,47 +383,28 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
 #pragma unroll
         for (int k = 0; k < KB; ++k) {
           const int pi = sub + 4 * (k0 + k);          // the same in every lane of the warp
-          const float wt = __shfl_sync(0xffffffffu, (pi & 32) ? wj[1] : wj[0], pi & 31);
-          if (pi < n_parts) {
-            float* dst = pi < n_rot ? rot4 : std4;
-            dst[0] = fmaf(wt, a[k].x, dst[0]); dst[1] = fmaf(wt, a[k].y, dst[1]);
-            dst[2] = fmaf(wt, a[k].z, dst[2]); dst[3] = fmaf(wt, a[k].w, dst[3]);
-          }
+          const float wt = __shfl_sync(0xffffffffu, (pi & 32) ? wj[1] : wj[0], pi & 31);   // (behind the last part: 0)
+          o4[0] = fmaf(wt, a[k].x, o4[0]); o4[1] = fmaf(wt, a[k].y, o4[1]);
+          o4[2] = fmaf(wt, a[k].z, o4[2]); o4[3] = fmaf(wt, a[k].w, o4[3]);
         }
       }
       if (sub > 0) {
-        float4* part4 = reinterpret_cast<float4*>(sm_raw) + ((sub - 1) * GQA + hl) * 64 + lane;
-        part4[0] = make_float4(rot4[0], rot4[1], rot4[2], rot4[3]);
-        part4[32] = make_float4(std4[0], std4[1], std4[2], std4[3]);
+        reinterpret_cast<float4*>(sm_raw)[((sub - 1) * GQA + hl) * 32 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
       }
     }
     __syncthreads();
     if (fin) {
 #pragma unroll
       for (int sub = 1; sub < 4; ++sub) {
-        const float4* part4 = reinterpret_cast<const float4*>(sm_raw) + ((sub - 1) * GQA + w) * 64 + lane;
-        const float4 r = part4[0], t = part4[32];
-        rot4[0] += r.x; rot4[1] += r.y; rot4[2] += r.z; rot4[3] += r.w;
-        std4[0] += t.x; std4[1] += t.y; std4[2] += t.z; std4[3] += t.w;
+        const float4 r = reinterpret_cast<const float4*>(sm_raw)[((sub - 1) * GQA + w) * 32 + lane];
+        o4[0] += r.x; o4[1] += r.y; o4[2] += r.z; o4[3] += r.w;
       }
-      if (n_rot > 0) {
-        // inverse (= forward) normalised Hadamard over the 128 channels of the head; channel
-        // d = 4*lane + c: the butterflies of distance 1 and 2 inside the thread, the others by shuffle
-        { const float x0 = rot4[0] + rot4[1], x1 = rot4[0] - rot4[1], x2 = rot4[2] + rot4[3], x3 = rot4[2] - rot4[3];
-          rot4[0] = x0 + x2; rot4[1] = x1 + x3; rot4[2] = x0 - x2; rot4[3] = x1 - x3; }
+      if (rotated) {
+        // inverse (= forward) normalised Hadamard over the 128 channels of the head
+        fwht128_lane4(o4, lane);
 #pragma unroll
-        for (int hh = 1; hh < 32; hh <<= 1) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float other = __shfl_xor_sync(0xffffffffu, rot4[c], hh);
-            rot4[c] = (lane & hh) ? other - rot4[c] : rot4[c] + other;
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) rot4[c] = rot4[c] / SQRT_HD;
+        for (int c = 0; c < 4; ++c) o4[c] = o4[c] * INV_SQRT_HD;
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) o4[c] = rot4[c] + std4[c];
     }
   } else {
     // many parts: thread = (head tid / 128, channel tid % 128), (max, sum-exp) of every part of the
@@ -437,7 +420,7 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
       ls[idx] = __ldcg(rec + 1);
     }
     __syncthreads();
-    float Mh = neg_inf(), Lh = 0.f, rot = 0.f, stdv = 0.f;
+    float Mh = neg_inf(), Lh = 0.f, v = 0.f;
     if (active) {
       for (int pi = 0; pi < n_parts; ++pi) Mh = fmaxf(Mh, ms[hl * n_parts + pi]);
       const float* accp = base0 + hl * PART + 4 + d;
@@ -447,11 +430,10 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
         const float m = ms[hl * n_parts + pi];
         const float wt = (m == neg_inf()) ? 0.f : exp2f((m - Mh) * LOG2E);
         Lh = fmaf(wt, ls[hl * n_parts + pi], Lh);
-        if (pi < n_rot) rot = fmaf(wt, a, rot); else stdv = fmaf(wt, a, stdv);
+        v = fmaf(wt, a, v);
       }
     }
-    float v = rot;
-    if (n_rot > 0) {
+    if (rotated) {
       for (int hh = 1; hh < HD; hh <<= 1) {
         if (active) sm[tid] = v;
         __syncthreads();
@@ -464,7 +446,7 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
       v = v / SQRT_HD;
     }
     if (active) {
-      sm[tid] = v + stdv;
+      sm[tid] = v;
       if (d == 0) { sm[GQA * HD + hl] = Mh; sm[GQA * HD + GQA + hl] = Lh; }
     }
     __syncthreads();

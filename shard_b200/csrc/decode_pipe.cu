@@ -719,7 +719,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     if (p.status) atomicExch(p.status, 1);
   }
   // one barrier serves the hand-back of tensor memory and the release of this CTA's records
-  __threadfence();
   tc_fence_before();
   __syncthreads();
   if (warp == PP_UNPACK_WARP0) tmem_dealloc(tmem_base, PP_TMEM_COLS);

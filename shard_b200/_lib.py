@@ -144,7 +144,8 @@ def host():
         except ImportError as e:
             raise ShardError(f"shard_b200/_host.so is missing or does not load ({e}): build it with "
                              "`python -m shard_b200.build`") from e
-        mod.bind(C.cast(load().shard_b200_decode_attn, C.c_void_p).value)
+        lib = load()
+        mod.bind(*(C.cast(f, C.c_void_p).value for f in (lib.shard_b200_decode_attn, lib.shard_b200_phase_table)))
         _host = mod
     return _host
 

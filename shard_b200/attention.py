@@ -181,10 +181,22 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
         if native is not None:
             # all of the step in native code; None: something is out of the ordinary
             step, (start, t0, t1), _ = native
+            host = _lib.host()
             pos_q = int(pos_q)
-            if cache._phase_key != (pos_q, start, t0, t1):
-                _phase_for(cache, gc, pos_q, t0, t1, cache._decode_ws.device)
-            res = _lib.host().attend(step, gc, cache._decode_ws, cache._phase.data_ptr(), q_rope, pos_q, out)
+            key = (pos_q, start, t0, t1)
+            if cache._phase_key != key:
+                old = cache._phase_key
+                rc = None
+                if old is not None and old[1:] == key[1:] and len(cache._phase_tabs) == 1:
+                    # the next step: the same tokens seen from another position, in the table's own memory
+                    rc = host.phase_table(step, start + t0, pos_q, t1 - t0, cache._phase)
+                if rc is not None:
+                    _lib.check(rc, "phase_table")
+                    cache._phase_tabs = {key: cache._phase}
+                    cache._phase_key = key
+                else:
+                    _phase_for(cache, gc, pos_q, t0, t1, cache._decode_ws.device)
+            res = host.attend(step, gc, cache._decode_ws, cache._phase.data_ptr(), q_rope, pos_q, out)
             if res is not None:
                 if type(res) is int:
                     _lib.check(res, "decode_attn")

@@ -19,7 +19,9 @@
 namespace {
 
 using DecodeFn = int (*)(const ShardSeq*, int32_t, const ShardDecodeShape*, const float*, const float*, void*, size_t, void*);
+using PhaseFn = int (*)(int32_t, int32_t, int32_t, const float*, void*, void*);
 DecodeFn g_decode = nullptr;
+PhaseFn g_phase = nullptr;
 
 PyObject *s_pending, *s_pending_dec, *s_stream_n, *s_k_idx, *s_v_idx, *s_k_norm, *s_v_norm, *s_signs, *s_decode_k, *s_decode_v,
     *s_buf_k, *s_buf_v, *s_fresh;
@@ -54,11 +56,26 @@ bool one_token(const at::Tensor& t, int64_t heads, int64_t hd) {
          (heads == 1 || t.stride(1) == hd) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 7) == 0;
 }
 
-// bind(address of shard_b200_decode_attn)
-PyObject* py_bind(PyObject*, PyObject* arg) {
-  g_decode = reinterpret_cast<DecodeFn>(PyLong_AsVoidPtr(arg));
+// bind(address of shard_b200_decode_attn, address of shard_b200_phase_table)
+PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) return PyErr_Format(PyExc_TypeError, "bind takes 2 arguments");
+  g_decode = reinterpret_cast<DecodeFn>(PyLong_AsVoidPtr(a[0]));
+  g_phase = reinterpret_cast<PhaseFn>(PyLong_AsVoidPtr(a[1]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
+}
+
+// phase_table(step, start, pos, n, table): the table of a step's layers, for another query position; returns
+// the library's status, or None: not done
+PyObject* py_phase_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 5) return PyErr_Format(PyExc_TypeError, "phase_table takes 5 arguments");
+  Step* st = static_cast<Step*>(PyCapsule_GetPointer(a[0], "shard_b200.step"));
+  if (!st) return nullptr;
+  if (!THPVariable_Check(a[4]) || c10::cuda::current_device() != st->device) Py_RETURN_NONE;
+  const int32_t start = (int32_t)PyLong_AsLong(a[1]), pos = (int32_t)PyLong_AsLong(a[2]), tokens = (int32_t)PyLong_AsLong(a[3]);
+  if (PyErr_Occurred()) return nullptr;
+  return PyLong_FromLong(g_phase(start, pos, tokens, st->inv_freq, THPVariable_Unpack(a[4]).data_ptr(),
+                                 c10::cuda::getCurrentCUDAStream(st->device).stream()));
 }
 
 // make_step(seq address, shape address, inv_freq pointer, codebook pointer, workspace bytes, device index)
@@ -203,7 +220,8 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 PyMethodDef methods[] = {
-    {"bind", py_bind, METH_O, nullptr},
+    {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
+    {"phase_table", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_phase_table)), METH_FASTCALL, nullptr},
     {"make_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_make_step)), METH_FASTCALL, nullptr},
     {"defer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_defer)), METH_FASTCALL, nullptr},
     {"attend", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attend)), METH_FASTCALL, nullptr},

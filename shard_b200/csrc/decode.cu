@@ -68,6 +68,7 @@ static DecodePlan make_plan(const ShardDecodeShape& sh, int batch) {
     const int n_rows = sh.n_sink + sh.n_win + sh.n_dec + sh.n_stream, row_ctas = (n_rows + 63) / 64;
     const int most = groups < CTA_SLOTS && row_ctas > n_tiles ? row_ctas : n_tiles;
     if (chunks > most) chunks = most;
+    if (chunks > MAX_PARTS) chunks = MAX_PARTS;              // (more only with more SMs than this GPU has)
     pl.n_chunks = chunks;
     pl.tiles_per_chunk = n_tiles / chunks;
     pl.tiles_rem = n_tiles % chunks;
@@ -218,7 +219,8 @@ static int check_shape(const ShardDecodeShape* sh) {
 static size_t ws_bytes(const ShardDecodeShape& sh, int batch) {
   int parts = make_plan(sh, batch).n_parts;
   const int groups = sh.nkv * batch, slots = cta_slots();
-  if (sh.tok_end > sh.tok_begin && groups < slots && parts < slots / groups) parts = slots / groups;
+  const int most = slots / groups < MAX_PARTS ? slots / groups : MAX_PARTS;
+  if (sh.tok_end > sh.tok_begin && parts < most) parts = most;
   return ws_header_bytes(batch, sh.nkv) + (size_t)batch * parts * sh.n_q * PART * sizeof(float);
 }
 

@@ -10,6 +10,7 @@ namespace shard {
 
 constexpr int ROWS_PER_CTA = 32;        // rows per CTA when a launch has no middle segment
 constexpr int MAX_ROW_CTAS = 18;
+constexpr int MAX_PARTS = 160;          // records of a (sequence, KV head) that the fused combine merges
 
 // Sequence-split decode: where the launch's result goes when it is delivered straight into the
 // exchange buffers of all ranks (layout in peer_layout.cuh).  world == 0: no delivery.
@@ -312,20 +313,21 @@ __device__ __forceinline__ void partial_merge(const float* scratch, float* __res
 // thread releases the CTA's writes, which the barrier has ordered before it, and acquires the others';
 // fences by every thread cost 2 K cycles more), merges them for the head's four
 // query heads, and puts the counter back to zero for the next call.  The result does not depend
-// on which CTA is last: the parts are always summed in the same order.  `sm` needs 1536 floats
-// (or GQA*HD + 2*GQA*n_parts + 8 for more than 64 parts) that are free; NTHREADS >= 512.
+// on which CTA is last: the parts are always summed in the same order.  `sm_raw` needs 1536 floats that are free,
+// 16-byte aligned; NTHREADS >= 512; at most MAX_PARTS parts (the host's plan sees to it).
 //
 // The merging CTA is the critical path of the whole launch and runs this code once, out of a
 // cold instruction cache: it is kept short.  Warp w < 16 takes query head w % 4 and the parts
-// p = w / 4 (mod 4), lane = channels 4*lane .. 4*lane+3: one 16-byte load per part and lane, all of
-// a warp's loads in flight together; lane j also fetches (max, sum-exp) of parts j and j + 32, from
-// which the warp derives the weights and hands them round by shuffle.  The four partial sums of a
+// p = w / 4 (mod 4), lane = channels 4*lane .. 4*lane+3: one 16-byte load per part and lane, the
+// loads of 32 parts in flight together; lane j also fetches (max, sum-exp) of parts j, j + 32, ..., from
+// which the warp derives the weights and hands them round by shuffle.  One path for any number of parts
+// (18 with 8 KV heads, up to 148 with one; against a second path of one thread per channel for more than
+// 64 parts, 30K context, 2 KV heads, 4 layers: 110 -> 83 us; 8 KV heads, 12 layers of 8K: 202 -> 198 us).  The four partial sums of a
 // head meet in shared memory; warp h < 4 adds them in order, runs the inverse Hadamard over the
 // 128 channels (two butterflies inside the thread, five by shuffle) and writes the output.
 template <int NTHREADS>
 __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const ShardSeq& sq, int kv, int b,
                                                float* sm_raw, int tid, bool synced = false) {
-  volatile float* sm = sm_raw;   // exchanged between threads: every access must reach shared memory
   static_assert(NTHREADS >= GQA * HD, "16 merging warps");
   __shared__ int last_s;
   if (!synced) __syncthreads();
@@ -349,112 +351,68 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
   const size_t pstride = (size_t)n_q * PART;
   const bool fin = tid < GQA * 32;                    // warp hl < 4 finishes query head hl
   float M = neg_inf(), L = 0.f;                       // of head w % 4 (the same in every lane)
-  float o4[4] = {0.f, 0.f, 0.f, 0.f};                 // channels 4*lane .. 4*lane+3 of head w (fin threads)
-  if (n_parts <= 64) {
-    if (w < 16) {
-      const int hl = w & 3, sub = w >> 2;
-      const float* rec0 = base0 + hl * PART;
-      constexpr int KB = 5;                            // loads of a batch (18 parts: one batch)
-      float4 a[KB];
+  float o4[4] = {0.f, 0.f, 0.f, 0.f};                 // channels 4*lane .. 4*lane+3 of that head
+  if (w < 16) {
+    const int hl = w & 3, sub = w >> 2;
+    const float* rec0 = base0 + hl * PART;
+    constexpr int KB = 8;                              // this warp's parts of a block of 32: all their loads in flight
+    float4 a[KB];
+    auto load = [&](int p0) {
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
-        const int pi = sub + 4 * k;
+        const int pi = p0 + sub + 4 * k;
         a[k] = pi < n_parts ? __ldcg(reinterpret_cast<const float4*>(rec0 + pi * pstride + 4) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      float mj[2], lj[2], wj[2];
+    };
+    load(0);
+    float mj[MAX_PARTS / 32], lj[MAX_PARTS / 32];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int pj = lane + 32 * k;
-        mj[k] = pj < n_parts ? __ldcg(rec0 + pj * pstride) : neg_inf();
-        lj[k] = pj < n_parts ? __ldcg(rec0 + pj * pstride + 1) : 0.f;
+    for (int k = 0; k < MAX_PARTS / 32; ++k) {
+      const int pj = lane + 32 * k;
+      mj[k] = neg_inf();
+      lj[k] = 0.f;
+      if (pj < n_parts) {
+        const float2 ml = __ldcg(reinterpret_cast<const float2*>(rec0 + pj * pstride));
+        mj[k] = ml.x;
+        lj[k] = ml.y;
       }
-      M = warp_max(fmaxf(mj[0], mj[1]));
+      M = fmaxf(M, mj[k]);
+    }
+    M = warp_max(M);
+    const float Ms = M == neg_inf() ? 0.f : M;         // (nothing attended to: all weights 0)
 #pragma unroll
-      for (int k = 0; k < 2; ++k) wj[k] = (mj[k] == neg_inf()) ? 0.f : exp2f((mj[k] - M) * LOG2E);
-      L = warp_sum(fmaf(wj[0], lj[0], wj[1] * lj[1]));
-      for (int k0 = 0; sub + 4 * k0 < n_parts; k0 += KB) {
-        if (k0 > 0) {
+    for (int k = 0; k < MAX_PARTS / 32; ++k) {
+      mj[k] = ex2((mj[k] - Ms) * LOG2E);               // now the weights; 0 behind the last part
+      L = fmaf(mj[k], lj[k], L);
+    }
+    L = warp_sum(L);
+#pragma unroll 1
+    for (int p0 = 0; p0 < n_parts; p0 += 32) {
+      if (p0 > 0) load(p0);
+      float wj = mj[0];
 #pragma unroll
-          for (int k = 0; k < KB; ++k) {
-            const int pi = sub + 4 * (k0 + k);
-            a[k] = pi < n_parts ? __ldcg(reinterpret_cast<const float4*>(rec0 + pi * pstride + 4) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        }
+      for (int k = 1; k < MAX_PARTS / 32; ++k) wj = p0 == 32 * k ? mj[k] : wj;
 #pragma unroll
-        for (int k = 0; k < KB; ++k) {
-          const int pi = sub + 4 * (k0 + k);          // the same in every lane of the warp
-          const float wt = __shfl_sync(0xffffffffu, (pi & 32) ? wj[1] : wj[0], pi & 31);   // (behind the last part: 0)
-          o4[0] = fmaf(wt, a[k].x, o4[0]); o4[1] = fmaf(wt, a[k].y, o4[1]);
-          o4[2] = fmaf(wt, a[k].z, o4[2]); o4[3] = fmaf(wt, a[k].w, o4[3]);
-        }
-      }
-      if (sub > 0) {
-        reinterpret_cast<float4*>(sm_raw)[((sub - 1) * GQA + hl) * 32 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
+      for (int k = 0; k < KB; ++k) {
+        const float wt = __shfl_sync(0xffffffffu, wj, sub + 4 * k);
+        o4[0] = fmaf(wt, a[k].x, o4[0]); o4[1] = fmaf(wt, a[k].y, o4[1]);
+        o4[2] = fmaf(wt, a[k].z, o4[2]); o4[3] = fmaf(wt, a[k].w, o4[3]);
       }
     }
-    __syncthreads();
-    if (fin) {
+    if (sub > 0) reinterpret_cast<float4*>(sm_raw)[((sub - 1) * GQA + hl) * 32 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
+  }
+  __syncthreads();
+  if (fin) {
 #pragma unroll
-      for (int sub = 1; sub < 4; ++sub) {
-        const float4 r = reinterpret_cast<const float4*>(sm_raw)[((sub - 1) * GQA + w) * 32 + lane];
-        o4[0] += r.x; o4[1] += r.y; o4[2] += r.z; o4[3] += r.w;
-      }
-      if (rotated) {
-        // inverse (= forward) normalised Hadamard over the 128 channels of the head
-        fwht128_lane4(o4, lane);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) o4[c] = o4[c] * INV_SQRT_HD;
-      }
-    }
-  } else {
-    // many parts: thread = (head tid / 128, channel tid % 128), (max, sum-exp) of every part of the
-    // four heads staged in shared memory, the result handed to the finishing threads through it
-    const bool active = tid < GQA * HD;
-    const int hl = (tid >> 7) & (GQA - 1), d = tid & (HD - 1);
-    volatile float* ms = sm + GQA * HD + 8;             // [GQA][n_parts]
-    volatile float* ls = ms + GQA * n_parts;            // [GQA][n_parts]
-    for (int idx = tid; idx < GQA * n_parts; idx += NTHREADS) {
-      const int hh = idx / n_parts, pi = idx - hh * n_parts;
-      const float* rec = base0 + pi * pstride + hh * PART;
-      ms[idx] = __ldcg(rec);
-      ls[idx] = __ldcg(rec + 1);
-    }
-    __syncthreads();
-    float Mh = neg_inf(), Lh = 0.f, v = 0.f;
-    if (active) {
-      for (int pi = 0; pi < n_parts; ++pi) Mh = fmaxf(Mh, ms[hl * n_parts + pi]);
-      const float* accp = base0 + hl * PART + 4 + d;
-#pragma unroll 4
-      for (int pi = 0; pi < n_parts; ++pi) {
-        const float a = __ldcg(accp + pi * pstride);
-        const float m = ms[hl * n_parts + pi];
-        const float wt = (m == neg_inf()) ? 0.f : exp2f((m - Mh) * LOG2E);
-        Lh = fmaf(wt, ls[hl * n_parts + pi], Lh);
-        v = fmaf(wt, a, v);
-      }
+    for (int sub = 1; sub < 4; ++sub) {
+      const float4 r = reinterpret_cast<const float4*>(sm_raw)[((sub - 1) * GQA + w) * 32 + lane];
+      o4[0] += r.x; o4[1] += r.y; o4[2] += r.z; o4[3] += r.w;
     }
     if (rotated) {
-      for (int hh = 1; hh < HD; hh <<= 1) {
-        if (active) sm[tid] = v;
-        __syncthreads();
-        if (active) {
-          const float other = sm[tid ^ hh];
-          v = (d & hh) ? other - v : v + other;
-        }
-        __syncthreads();
-      }
-      v = v / SQRT_HD;
-    }
-    if (active) {
-      sm[tid] = v;
-      if (d == 0) { sm[GQA * HD + hl] = Mh; sm[GQA * HD + GQA + hl] = Lh; }
-    }
-    __syncthreads();
-    if (fin) {
+      // inverse (= forward) normalised Hadamard over the 128 channels of the head
+      fwht128_lane4(o4, lane);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) o4[c] = sm[w * HD + 4 * lane + c];
-      M = sm[GQA * HD + w];
-      L = sm[GQA * HD + GQA + w];
+      for (int c = 0; c < 4; ++c) o4[c] = o4[c] * INV_SQRT_HD;
     }
   }
   const int h = kv * GQA + w;                          // query head of a finishing thread

@@ -1,5 +1,5 @@
 """Decode attention with few and with many rows outside the compressed middle (fp16 or streamed): pairs and
-odd rows, all warps on the rows, more row CTAs than tiles, against float64 attention over the read-back."""
+odd rows, all warps on the rows, more row CTAs than tiles, many partial results to merge, against float64 attention over the read-back."""
 import pytest
 import torch
 
@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n_comp,nkv,rows,streaming", [
     (700, 8, 1, True), (700, 8, 2, False), (130, 8, 75, True), (130, 8, 76, False), (1, 2, 700, False), (1, 8, 901, True),
-    (2560, 8, 1153, True), (2560, 8, 1100, False), (5000, 8, 3001, True), (300, 1, 4001, True)])
+    (2560, 8, 1153, True), (2560, 8, 1100, False), (5000, 8, 3001, True), (300, 1, 4001, True),
+    (4096, 1, 2, True), (4097, 1, 3, False), (18900, 1, 2, True), (8300, 2, 5, False)])   # 32, 33, 148 and 65 partial results to merge
 def test_decode_rows(n_comp, nkv, rows, streaming):
     from shard_b200 import fused_attention_compressed
     cache, layer = _cache(random_gc(n_comp, nkv=nkv, seed=rows), nkv, streaming, capacity=rows + 4)

@@ -23,7 +23,13 @@
 //
 // Bound: instruction issue (about 250 instructions per 32 points and iteration; the direct search needs
 // 3 500, a tensor-core search with exact re-check of the close calls measured 370 us per iteration at
-// 8.4 M points); the points' 134 MB at 8.4 M are 21 us at the measured copy rate.
+// 8.4 M points) and 20 us per launch at either end; the points' 134 MB at 8.4 M are 21 us at the measured
+// copy rate.  8.4 M points, 30 iterations: 40 ms for the direct search with host round trips, 4.1 ms with
+// every move booked where it is found, 3.7 ms with moves collected until they fill a warp (600 -> 500
+// instructions per 64 points) and every warp's first run dealt out without asking.  Distances in packed
+// fp32 pairs (2 instructions fewer in 3) measured 3 % more: the pairs cost registers.  Keeping each tile's
+// distance to its nearest boundary to skip tiles the centroids' moves cannot have touched would skip one
+// tile in ten by the last iteration.
 #include "tcgen05.cuh"
 
 namespace shard {
@@ -31,6 +37,7 @@ namespace shard {
 constexpr int KM_THREADS = 512, KM_WARPS = KM_THREADS / 32;
 constexpr int KM_TILE = 64;                   // points per box: two per lane
 constexpr int KM_MAX_RUN = 8;                 // tiles per run
+constexpr int KM_QUEUE = 64;                  // points a warp may have waiting to be booked (see `flush`)
 constexpr int KM_CTA_POINTS = 60000;          // points a CTA books at most: its partial sums stay within int32
 
 struct KmeansHeader {      // head of the workspace; zero when the first iteration starts
@@ -99,15 +106,6 @@ __device__ __forceinline__ KmeansParams km_problem(KmeansParams p, int b) {
   return p;
 }
 
-// distance exactly as the nearest-centroid rule defines it
-__device__ __forceinline__ float km_sq4(float d0, float d1, float d2, float d3) {
-  float dist = __fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-  dist = __fadd_rn(dist, __fmul_rn(d2, d2));
-  return __fadd_rn(dist, __fmul_rn(d3, d3));
-}
-__device__ __forceinline__ float km_dist(float4 p, float4 c) {
-  return km_sq4(__fsub_rn(p.x, c.x), __fsub_rn(p.y, c.y), __fsub_rn(p.z, c.z), __fsub_rn(p.w, c.w));
-}
 // Middle and half-widths of a box (the half-widths rounded up), and their squared length.
 struct KmBox { float4 mid, h; float hh; };
 __device__ __forceinline__ KmBox km_box(float4 lo, float4 hi) {
@@ -131,6 +129,13 @@ __device__ __forceinline__ bool km_may_win(const KmBox& b, float4 c, float d, fl
   const float reach = fmaf(fabsf(c.x - near.x), b.h.x, fmaf(fabsf(c.y - near.y), b.h.y,
                       fmaf(fabsf(c.z - near.z), b.h.z, fabsf(c.w - near.w) * b.h.w)));
   return !(d - d_near - 2.f * reach > KM_SLACK * (d + b.hh));   // (true for NaN)
+}
+// distance exactly as the nearest-centroid rule defines it
+__device__ __forceinline__ float km_dist(float4 p, float4 c) {
+  const float d0 = __fsub_rn(p.x, c.x), d1 = __fsub_rn(p.y, c.y), d2 = __fsub_rn(p.z, c.z), d3 = __fsub_rn(p.w, c.w);
+  float dist = __fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
+  dist = __fadd_rn(dist, __fmul_rn(d2, d2));
+  return __fadd_rn(dist, __fmul_rn(d3, d3));
 }
 // minimum over the warp of a non-negative float (or +inf)
 __device__ __forceinline__ float warp_min_nonneg(float v) {
@@ -261,8 +266,10 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
   const KmeansParams p = km_problem(pp, blockIdx.y);
   __shared__ float4 c_s[256];
   __shared__ int acc_s[256 * 9];                               // high and low halves of the sums' changes, count's change
+  __shared__ float4 wait_s[KM_WARPS][KM_QUEUE];                // points that changed sides, not booked yet
+  __shared__ uint16_t sides_s[KM_WARPS][KM_QUEUE];             // ... their centroids: new, old << 8
   __shared__ uint8_t run_s[KM_WARPS][256];                     // survivors of the run test, ascending
-  __shared__ uint8_t few_s[KM_WARPS][256];                     // survivors of the tile test
+  __shared__ __align__(2) uint8_t few_s[KM_WARPS][258];        // survivors of the tile test
   __shared__ int last_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < 256 * 9; i += KM_THREADS) acc_s[i] = 0;
@@ -273,32 +280,22 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
   if (tid < 256) c_s[tid] = __ldcg(p.centroids + tid);
   __syncthreads();
 
-  // Books the lanes' points with `go`: added to centroid k (sign 1) or taken off it (-1).  A few lanes
-  // add one by one; more are first summed per centroid (sorted points: a warp knows two or three).
-  auto book = [&](float4 pt, int k, bool go, int sign) {
+  auto fixed = [&](float v, int& hi, int& lo) {
+    const int fx = __float2int_rn(v * qscale);                 // |.| <= 2^30
+    hi = fx >> 15;
+    lo = fx & 32767;
+  };
+  // Books the lanes' points with `go` under centroid k, summed per centroid first (sorted points: a warp
+  // knows two or three).
+  auto book = [&](float4 pt, int k, bool go) {
     unsigned int todo = __ballot_sync(0xffffffffu, go);
-    if (!todo) return;
-    const float pv[4] = {pt.x, pt.y, pt.z, pt.w};
     int hi[4], lo[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int fx = __float2int_rn(pv[c] * qscale);           // |.| <= 2^30
-      hi[c] = sign * (fx >> 15);
-      lo[c] = sign * (fx & 32767);
-    }
-    if (__popc(todo) <= 4) {
-      if (go) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) { atomicAdd(&acc_s[k * 9 + c], hi[c]); atomicAdd(&acc_s[k * 9 + 4 + c], lo[c]); }
-        atomicAdd(&acc_s[k * 9 + 8], sign);
-      }
-      return;
-    }
+    fixed(pt.x, hi[0], lo[0]); fixed(pt.y, hi[1], lo[1]); fixed(pt.z, hi[2], lo[2]); fixed(pt.w, hi[3], lo[3]);
     while (todo) {
       const int kk = __shfl_sync(0xffffffffu, k, __ffs(todo) - 1);
       const bool mine = go && k == kk;
       const unsigned int who = __ballot_sync(0xffffffffu, mine);
-      int s = sign * __popc(who);                              // lane c < 8 ends up with sum c, the others with the count
+      int s = __popc(who);                                     // lane c < 8 ends up with sum c, the others with the count
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const int a = __reduce_add_sync(0xffffffffu, mine ? hi[c] : 0), b = __reduce_add_sync(0xffffffffu, mine ? lo[c] : 0);
@@ -309,6 +306,32 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
       todo &= ~who;
     }
   };
+  // Later iterations move one point in a hundred.  Booking those where they are found would run mostly
+  // empty warps through it (a third of the kernel's instructions); they wait in shared memory until
+  // there is one for every lane.
+  int waiting = 0;
+  auto flush = [&](int first) {
+    __syncwarp();
+    if (first + lane < waiting) {
+      const float4 pt = wait_s[warp][first + lane];
+      const int sides = sides_s[warp][first + lane];
+      int *on = acc_s + (sides & 255) * 9, *off = acc_s + (sides >> 8) * 9;
+      const float pv[4] = {pt.x, pt.y, pt.z, pt.w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        int hi, lo;
+        fixed(pv[c], hi, lo);
+        atomicAdd(on + c, hi);
+        atomicAdd(on + 4 + c, lo);
+        atomicAdd(off + c, -hi);
+        atomicAdd(off + 4 + c, -lo);
+      }
+      atomicAdd(on + 8, 1);
+      atomicAdd(off + 8, -1);
+    }
+    waiting = first;
+    __syncwarp();
+  };
 
   const long long n_tiles = (p.n + KM_TILE - 1) / KM_TILE;
   const long long n_runs = (n_tiles + p.run - 1) / p.run;
@@ -317,10 +340,10 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
   // stream's kernels); the next one is asked for while the current one is worked on.
   auto ask = [&]() {
     unsigned int v = 0;
-    if (lane == 0) v = atomicAdd(&p.h->next_run, 1u);
+    if (lane == 0) v = gridDim.x * KM_WARPS + atomicAdd(&p.h->next_run, 1u);
     return v;
   };
-  unsigned int asked = ask();
+  unsigned int asked = blockIdx.x * KM_WARPS + warp;           // (the first without asking: they would queue up at the counter)
   for (int quota = p.warp_runs; quota > 0; --quota) {
     const long long run = __shfl_sync(0xffffffffu, asked, 0);
     if (run >= n_runs) break;
@@ -331,6 +354,7 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
       // ---- the run's box against all centroids ---------------------------------------------------
       const float4* bx = p.boxes + 2 * t_lo;
       const float4 my_lo = bx[2 * min(lane, nt - 1)], my_hi = bx[2 * min(lane, nt - 1) + 1];   // lane j < nt: box of tile j
+      const KmBox mine = km_box(my_lo, my_hi);
       float4 lo = my_lo, hi = my_hi;
       for (int o = 1; o < p.run; o <<= 1) {                    // (lanes 0..run-1 hold every box: run is a power of two)
         lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, o)); hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, o));
@@ -366,26 +390,38 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
       // ---- tile by tile -----------------------------------------------------------------------------
       float4 n0 = make_float4(0.f, 0.f, 0.f, 0.f), n1 = n0;
       int o0 = 0, o1 = 0;
+      const unsigned int at = (unsigned int)t_lo * KM_TILE + lane, end = (unsigned int)p.n;
       auto fetch = [&](int q) {
-        const long long i0 = (t_lo + q) * KM_TILE + lane;
-        n0 = p.xs[min(i0, p.n - 1)];
-        n1 = p.xs[min(i0 + 32, p.n - 1)];
-        if (p.it > 0) { o0 = __ldcg(p.idx_s + min(i0, p.n - 1)); o1 = __ldcg(p.idx_s + min(i0 + 32, p.n - 1)); }
+        const unsigned int i0 = min(at + q * KM_TILE, end - 1), i1 = min(at + q * KM_TILE + 32, end - 1);
+        n0 = p.xs[i0];
+        n1 = p.xs[i1];
+        if (p.it > 0) { o0 = __ldcg(p.idx_s + i0); o1 = __ldcg(p.idx_s + i1); }
       };
       fetch(0);
       for (int q = 0; q < nt; ++q) {
         const float4 p0 = n0, p1 = n1;
         const int old0 = o0, old1 = o1;
         if (q + 1 < nt) fetch(q + 1);
-        float best0 = inf, best1 = inf;
-        int arg0 = 0, arg1 = 0;
-        {
-          float4 tl, th;
-          tl.x = __shfl_sync(0xffffffffu, my_lo.x, q); tl.y = __shfl_sync(0xffffffffu, my_lo.y, q);
-          tl.z = __shfl_sync(0xffffffffu, my_lo.z, q); tl.w = __shfl_sync(0xffffffffu, my_lo.w, q);
-          th.x = __shfl_sync(0xffffffffu, my_hi.x, q); th.y = __shfl_sync(0xffffffffu, my_hi.y, q);
-          th.z = __shfl_sync(0xffffffffu, my_hi.z, q); th.w = __shfl_sync(0xffffffffu, my_hi.w, q);
-          const KmBox tb = km_box(tl, th);
+        KmBox tb;
+        tb.mid.x = __shfl_sync(0xffffffffu, mine.mid.x, q); tb.mid.y = __shfl_sync(0xffffffffu, mine.mid.y, q);
+        tb.mid.z = __shfl_sync(0xffffffffu, mine.mid.z, q); tb.mid.w = __shfl_sync(0xffffffffu, mine.mid.w, q);
+        tb.h.x = __shfl_sync(0xffffffffu, mine.h.x, q); tb.h.y = __shfl_sync(0xffffffffu, mine.h.y, q);
+        tb.h.z = __shfl_sync(0xffffffffu, mine.h.z, q); tb.h.w = __shfl_sync(0xffffffffu, mine.h.w, q);
+        tb.hh = __shfl_sync(0xffffffffu, mine.hh, q);
+        int cnt = 0;
+        auto keep = [&](bool in, int k) {
+          const unsigned int bal = __ballot_sync(0xffffffffu, in);
+          if (in) few_s[warp][cnt + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)k;
+          cnt += __popc(bal);
+        };
+        if (len <= 32) {                                       // (nearly always)
+          const int k = run_s[warp][min(lane, len - 1)];
+          const float4 c = c_s[k];
+          const float dk = km_mid_dist(tb, c);
+          dmin = warp_min_nonneg(dk);
+          near = c_s[__shfl_sync(0xffffffffu, k, (__ffs(__ballot_sync(0xffffffffu, dk == dmin)) - 1) & 31)];
+          keep(lane < len && km_may_win(tb, c, dk, near, dmin), k);
+        } else {
           dn = inf;
           kn = 0;
           for (int j = lane; j < len; j += 32) {
@@ -394,44 +430,56 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
             if (dk < dn) { dn = dk; kn = k; }
           }
           dmin = warp_min_nonneg(dn);
-          kn = __shfl_sync(0xffffffffu, kn, (__ffs(__ballot_sync(0xffffffffu, dn == dmin)) - 1) & 31);
-          near = c_s[kn];
-          int cnt = 0;
+          near = c_s[__shfl_sync(0xffffffffu, kn, (__ffs(__ballot_sync(0xffffffffu, dn == dmin)) - 1) & 31)];
           for (int j0 = 0; j0 < len; j0 += 32) {
             const int k = run_s[warp][min(j0 + lane, len - 1)];
             const float4 c = c_s[k];
-            const bool in = j0 + lane < len && km_may_win(tb, c, km_mid_dist(tb, c), near, dmin);
-            const unsigned int bal = __ballot_sync(0xffffffffu, in);
-            if (in) few_s[warp][cnt + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)k;
-            cnt += __popc(bal);
-          }
-          __syncwarp();
-#pragma unroll 4
-          for (int j = 0; j < cnt; ++j) {
-            const int k = few_s[warp][j];
-            const float4 c = c_s[k];
-            const float d0 = km_dist(p0, c), d1 = km_dist(p1, c);
-            if (d0 < best0) { best0 = d0; arg0 = k; }
-            if (d1 < best1) { best1 = d1; arg1 = k; }
+            keep(j0 + lane < len && km_may_win(tb, c, km_mid_dist(tb, c), near, dmin), k);
           }
         }
-        const long long i0 = (t_lo + q) * KM_TILE + lane, i1 = i0 + 32;
-        const bool live0 = i0 < p.n, live1 = i1 < p.n;
+        __syncwarp();
+        // the few left, two at a time; an odd last one twice (a tie changes nothing)
+        float best0 = inf, best1 = inf;
+        int arg0 = 0, arg1 = 0;
+        for (int j = 0; j < cnt; j += 2) {
+          const unsigned int ks = *reinterpret_cast<const uint16_t*>(&few_s[warp][j]);
+          const int ka = ks & 255, kb = j + 1 < cnt ? ks >> 8 : ka;
+          float a0, a1, b0, b1;
+          const float4 ca = c_s[ka], cb = c_s[kb];
+          a0 = km_dist(p0, ca); a1 = km_dist(p1, ca);
+          b0 = km_dist(p0, cb); b1 = km_dist(p1, cb);
+          if (a0 < best0) { best0 = a0; arg0 = ka; }
+          if (a1 < best1) { best1 = a1; arg1 = ka; }
+          if (b0 < best0) { best0 = b0; arg0 = kb; }
+          if (b1 < best1) { best1 = b1; arg1 = kb; }
+        }
+        const unsigned int i0 = at + q * KM_TILE, i1 = i0 + 32;
+        const bool live0 = i0 < end, live1 = i1 < end;
         const bool ch0 = live0 && (p.it == 0 || arg0 != old0), ch1 = live1 && (p.it == 0 || arg1 != old1);
         if (ch0) p.idx_s[i0] = (uint8_t)arg0;
         if (ch1) p.idx_s[i1] = (uint8_t)arg1;
-        if (__any_sync(0xffffffffu, ch0 || ch1)) {
-          book(p0, arg0, ch0, 1);
-          book(p1, arg1, ch1, 1);
-          if (p.it > 0) {
-            book(p0, old0, ch0, -1);
-            book(p1, old1, ch1, -1);
-          }
+        if (p.it == 0) {
+          book(p0, arg0, ch0);
+          book(p1, arg1, ch1);
+        } else {
+          const unsigned int todo0 = __ballot_sync(0xffffffffu, ch0), todo1 = __ballot_sync(0xffffffffu, ch1);
+          auto queue = [&](float4 pt, int k, int old, bool go, unsigned int todo) {
+            if (go) {
+              const int slot = waiting + __popc(todo & ((1u << lane) - 1u));
+              wait_s[warp][slot] = pt;
+              sides_s[warp][slot] = (uint16_t)(k | old << 8);
+            }
+            waiting += __popc(todo);
+            if (waiting >= 32) flush(waiting - 32);            // (at most 31 waited before: never more than 63)
+          };
+          if (todo0) queue(p0, arg0, old0, ch0, todo0);
+          if (todo1) queue(p1, arg1, old1, ch1, todo1);
         }
         __syncwarp();
       }
     }
   }
+  if (waiting) flush(0);
   __syncthreads();
   for (int i = tid; i < 256 * 4; i += KM_THREADS) {
     const int* a = acc_s + (i >> 2) * 9 + (i & 3);

@@ -17,7 +17,8 @@
 //
 // Bound: the exponentials (16 per SM and cycle: 1 K cycles a tile) and the tensor work (1 K cycles a
 // tile) are about equal and overlap only partly, one softmax group per CTA; the images' 64 KB per tile
-// and KV head come from L2.
+// and KV head come from L2.  48 new tokens over 8K, 8 KV heads: 26 us a layer, and 26 us for the read-back
+// in front of it (one decode launch per query token: 1 600 us a layer).
 #include <atomic>
 
 #include "decode_common.cuh"

@@ -15,7 +15,8 @@
 // all heads.  Warps 0-3 turn accumulators into keys; warps 4-7 do the values meanwhile, one thread per
 // (token, head) vector with the whole 128-point butterfly in registers (no shuffles).  Both write
 // through a swizzled shared-memory tile so that global stores are full lines.
-// Measured (one layer, 8 KV heads): see the table at the launch function.
+// Measured (8 KV heads, 192 components): 22 us for a layer of 8K tokens (34 MB written: 1.5 TB/s), 70 us for
+// one of 32K (1.9 TB/s); three 8K layers with their host work 71 us, 5 477 us as PyTorch operations.
 #include <atomic>
 
 #include "decode_common.cuh"

@@ -872,7 +872,7 @@ def run_compress_profile(args):
     mean = flat.mean(dim=0).contiguous()
     basis, eig = pca_fit(flat, mean, RANK)
     row("pca_fit (torch: Gram matrix GEMM + eigh)", timed(lambda: pca_fit(flat, mean, RANK), reps=3, warm=1),
-        flops=2 * n * 1024 * 1024, note="library GEMM + cuSOLVER eigensolver on 1024 x 1024")
+        flops=2 * n * 1024 * 1024, note="Gram matrix on the tensor cores + eigh.cu on one 1024 x 1024 matrix")
     scale = basis.abs().amax(0).clamp(min=1e-6) / 127.0
     w = ((basis / scale).round().clamp(-127, 127) * scale).contiguous()
     proj = ops.k_project(flat, mean, w)
@@ -884,7 +884,7 @@ def run_compress_profile(args):
     row("kq_* (min/max, max-abs, scale, pack)", timed(lambda: ops.k_quantize_pack(proj, alloc)),
         nbytes=3 * n * RANK * 4 + n * RANK // 2, note="three passes over the fp32 projection, writes packed int4")
     x, ch = ops.v_hadamard_normalise(v_mid)
-    row("v_rotate / v_clamp / v_normalise", timed(lambda: ops.v_hadamard_normalise(v_mid)),
+    row("v_channel_max / v_clamp / v_normalise", timed(lambda: ops.v_hadamard_normalise(v_mid)),
         nbytes=n * 1024 * (2 + 4 + 4 + 4), note="reads fp16 values, writes fp32, normalises in place")
     flat_v = x.view(-1, 4)
     g = torch.Generator(device=dev).manual_seed(42)

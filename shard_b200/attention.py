@@ -118,7 +118,7 @@ class _Launch:
     """Per-layer launch state that does not change from step to step: the sequence record, the
     shape record (only n_stream / pos_q / append / n_dec are touched per step), workspace need
     and the constant device pointers."""
-    __slots__ = ("key", "seq", "shape", "need", "inv_ptr", "cb", "cb_ptr", "dev", "dev_index", "kbuf", "inv_freq")
+    __slots__ = ("key", "seq", "shape", "need", "inv_ptr", "cb", "cb_ptr", "dev", "dev_index", "inv_freq")
 
 
 def _launch_state(gc, cache, dev, nkv, n_q, t0, t1, with_fp16_segments, partial_out):
@@ -134,7 +134,6 @@ def _launch_state(gc, cache, dev, nkv, n_q, t0, t1, with_fp16_segments, partial_
         ls.key = key
         ls.dev, ls.dev_index = dev, dev.index
         ls.seq = _seq_record(gc, dev)
-        ls.kbuf = None
         ls.shape = ops.make_shape(n_q, nkv, gc["k_rank_kernel"], gc["n_compress"], t0, t1, n_sink, n_win, 0, 0,
                                   partial_out)
         # With a middle segment the scratch size does not depend on the number of rows (they ride
@@ -236,13 +235,10 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
         else:
             layer._flush_pending()
     seq, shape = ls.seq, ls.shape
-    if n_stream > 0:
-        kbuf = gc["k_idx_buf"]
-        if ls.kbuf is not kbuf:                        # the stream buffers were (re)allocated
-            ls.kbuf = kbuf
-            seq.st_k_idx, seq.st_v_idx = kbuf.data_ptr(), gc["v_idx_buf"].data_ptr()
-            seq.st_k_norm, seq.st_v_norm = gc["k_norm_buf"].data_ptr(), gc["v_norm_buf"].data_ptr()
-            seq.signs = gc["signs"].data_ptr()
+    if n_stream > 0:                                   # (asked for at every step: the buffers move when they grow)
+        seq.st_k_idx, seq.st_v_idx = gc["k_idx_buf"].data_ptr(), gc["v_idx_buf"].data_ptr()
+        seq.st_k_norm, seq.st_v_norm = gc["k_norm_buf"].data_ptr(), gc["v_norm_buf"].data_ptr()
+        seq.signs = gc["signs"].data_ptr()
     if pending is not None:
         seq.new_k, seq.new_v = pending[0].data_ptr(), pending[1].data_ptr()
     n_dec = dec_cap = 0

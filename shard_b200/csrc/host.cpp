@@ -6,8 +6,7 @@
 // call.  Here they are direct accesses to the tensors and the same ShardSeq / ShardDecodeShape records,
 // and the library's entry point is called through its address.  Anything out of the ordinary (another
 // dtype, layout or device, buffers to grow, a pending token that does not fit) returns None and the Python
-// path does it, with its checks and messages.
-#include <Python.h>
+// path does it, with its checks and messages.  #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -35,7 +34,6 @@ struct Step {
   const float* codebook;
   size_t need;              // workspace bytes
   int device;
-  PyObject* kbuf;           // stream buffer whose pointers the record holds (identity only)
 };
 void step_free(PyObject* cap) { delete static_cast<Step*>(PyCapsule_GetPointer(cap, "shard_b200.step")); }
 
@@ -83,7 +81,7 @@ PyObject* py_make_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 6) return PyErr_Format(PyExc_TypeError, "make_step takes 6 arguments");
   Step* s = new Step{static_cast<ShardSeq*>(PyLong_AsVoidPtr(a[0])), static_cast<ShardDecodeShape*>(PyLong_AsVoidPtr(a[1])),
                      static_cast<const float*>(PyLong_AsVoidPtr(a[2])), static_cast<const float*>(PyLong_AsVoidPtr(a[3])),
-                     PyLong_AsSize_t(a[4]), (int)PyLong_AsLong(a[5]), nullptr};
+                     PyLong_AsSize_t(a[4]), (int)PyLong_AsLong(a[5])};
   if (PyErr_Occurred()) { delete s; return nullptr; }
   return PyCapsule_New(s, "shard_b200.step", step_free);
 }
@@ -181,17 +179,12 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
     seq.new_k = new_k->data_ptr();
     seq.new_v = new_v->data_ptr();
   }
-  if (n_stream > 0) {
-    PyObject* kbuf = PyDict_GetItemWithError(gc, s_k_idx);
-    if (!kbuf) Py_RETURN_NONE;
-    if (kbuf != st->kbuf) {                                      // the stream buffers were (re)allocated
-      seq.st_k_idx = static_cast<uint8_t*>(data_at(gc, s_k_idx));
-      seq.st_v_idx = static_cast<uint8_t*>(data_at(gc, s_v_idx));
-      seq.st_k_norm = data_at(gc, s_k_norm);
-      seq.st_v_norm = data_at(gc, s_v_norm);
-      seq.signs = static_cast<const float*>(data_at(gc, s_signs));
-      st->kbuf = kbuf;
-    }
+  if (n_stream > 0) {                                            // (asked for at every step: the buffers move when they grow)
+    seq.st_k_idx = static_cast<uint8_t*>(data_at(gc, s_k_idx));
+    seq.st_v_idx = static_cast<uint8_t*>(data_at(gc, s_v_idx));
+    seq.st_k_norm = data_at(gc, s_k_norm);
+    seq.st_v_norm = data_at(gc, s_v_norm);
+    seq.signs = static_cast<const float*>(data_at(gc, s_signs));
   }
   seq.q = q.data_ptr();
   seq.phase = PyLong_AsVoidPtr(a[3]);

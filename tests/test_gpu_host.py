@@ -68,3 +68,33 @@ def test_native_steps(streaming, nkv, n_comp, monkeypatch):
         layer.update(k, v)
         append_ref(k, v)
     assert torch.equal(layer.keys, ref.keys) and torch.equal(layer.values, ref.values)
+
+
+def test_stream_buffers_that_moved_behind_the_same_object():
+    """A step takes the stream buffers' memory from the tensors as they are, also where a tensor object of the
+    same identity holds other memory (as when a freed object's address is used again)."""
+    from shard_b200 import fused_attention_compressed
+    from shard_b200.attention import decode_layer
+    cache, layer = _cache(random_gc(300, nkv=2, seed=1), 2, True, capacity=16)
+    other, ref = _cache(random_gc(300, nkv=2, seed=1), 2, True, capacity=16)
+    cache._fused_decode_update = True
+    g = torch.Generator(device="cuda").manual_seed(3)
+    gc, names = layer._gpu_compressed, ("k_idx_buf", "v_idx_buf", "k_norm_buf", "v_norm_buf")
+    before = None
+    for t in range(8):
+        k, v = (torch.randn(1, 2, 1, 128, generator=g, device="cuda").half() for _ in range(2))
+        q = torch.randn(1, 8, 1, 128, generator=g, device="cuda").half()
+        if t in (4, 6):
+            before = [gc[n].data for n in names]            # (stays allocated)
+            for n in names:
+                gc[n].data = gc[n].data.clone()
+            copies = [b.clone() for b in before]
+        layer.update(k, v)
+        out = (fused_attention_compressed(q, layer, 400 + t, cache._rope_inv_freq) if t != 6
+               else decode_layer(q, layer, 400 + t))        # (the general path as well)
+        ref._stream_append(k, v, 0)
+        assert torch.equal(out.view(-1, 128), decode_layer(q, ref, 400 + t))
+        if before is not None:
+            assert all(torch.equal(b, c) for b, c in zip(before, copies))
+    for n in names:
+        assert torch.equal(gc[n][:8], ref._gpu_compressed[n][:8])

@@ -6,11 +6,14 @@
 // call.  Here they are direct accesses to the tensors and the same ShardSeq / ShardDecodeShape records,
 // and the library's entry point is called through its address.  Anything out of the ordinary (another
 // dtype, layout or device, buffers to grow, a pending token that does not fit) returns None and the Python
-// path does it, with its checks and messages.  #include <Python.h>
+// path does it, with its checks and messages.  What torch throws (an allocation that fails) becomes the Python
+// exception it would be there.
+#include <Python.h>
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/shard_b200.h"
@@ -66,6 +69,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // phase_table(step, start, pos, n, table): the table of a step's layers, for another query position; returns
 // the library's status, or None: not done
 PyObject* py_phase_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 5) return PyErr_Format(PyExc_TypeError, "phase_table takes 5 arguments");
   Step* st = static_cast<Step*>(PyCapsule_GetPointer(a[0], "shard_b200.step"));
   if (!st) return nullptr;
@@ -74,6 +78,7 @@ PyObject* py_phase_table(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (PyErr_Occurred()) return nullptr;
   return PyLong_FromLong(g_phase(start, pos, tokens, st->inv_freq, THPVariable_Unpack(a[4]).data_ptr(),
                                  c10::cuda::getCurrentCUDAStream(st->device).stream()));
+  END_HANDLE_TH_ERRORS
 }
 
 // make_step(seq address, shape address, inv_freq pointer, codebook pointer, workspace bytes, device index)
@@ -88,6 +93,7 @@ PyObject* py_make_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 // defer(gc, k, v, streaming) -> True: the token has its row and is left to the launch that reads it; None: not done
 PyObject* py_defer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 4) return PyErr_Format(PyExc_TypeError, "defer takes 4 arguments");
   PyObject* gc = a[0];
   if (!PyDict_Check(gc) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2])) Py_RETURN_NONE;
@@ -129,11 +135,13 @@ PyObject* py_defer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_XDECREF(pend);
   if (!ok) return nullptr;
   Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
 }
 
 // attend(step, gc, workspace, phase pointer, q, pos, out or None) -> (1, n_q, 1, hd) fp16; None: not done;
 // an int: the library's status
 PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
   if (n != 7) return PyErr_Format(PyExc_TypeError, "attend takes 7 arguments");
   Step* st = static_cast<Step*>(PyCapsule_GetPointer(a[0], "shard_b200.step"));
   PyObject* gc = a[1];
@@ -210,6 +218,7 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (rc != 0) return PyLong_FromLong(rc);
   if (append == 1 ? PyDict_DelItem(gc, s_pending) : append == 2 ? PyDict_DelItem(gc, s_pending_dec) : 0) return nullptr;
   return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef methods[] = {

@@ -98,3 +98,37 @@ def test_stream_buffers_that_moved_behind_the_same_object():
             assert all(torch.equal(b, c) for b, c in zip(before, copies))
     for n in names:
         assert torch.equal(gc[n][:8], ref._gpu_compressed[n][:8])
+
+
+def test_a_failed_allocation_is_a_python_exception():
+    """The native step's output does not fit: the error torch raises, not the end of the process."""
+    from shard_b200 import fused_attention_compressed
+    cache, layer = _cache(random_gc(300, nkv=8, seed=1), 8, True, capacity=16)
+    cache._fused_decode_update = True
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def step(t):
+        k, v = (torch.randn(1, 8, 1, 128, generator=g, device="cuda").half() for _ in range(2))
+        layer.update(k, v)
+        return k, v, torch.randn(1, 32, 1, 128, generator=g, device="cuda").half()
+
+    for t in range(3):
+        _, _, q = step(t)
+        want = fused_attention_compressed(q, layer, 400 + t, cache._rope_inv_freq)
+    _, _, q = step(3)
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)
+    held = []
+    try:
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            while len(held) < 100000:
+                held.append(torch.empty(32 * 128, dtype=torch.float16, device="cuda"))
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            fused_attention_compressed(q, layer, 403, cache._rope_inv_freq)
+    finally:
+        held.clear()
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    out = fused_attention_compressed(q, layer, 403, cache._rope_inv_freq)      # the token is still to be appended
+    cache.check()
+    assert out.shape == want.shape and "_pending" not in layer._gpu_compressed

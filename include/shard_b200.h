@@ -294,6 +294,15 @@ int shard_b200_stream_quantize_rows(const void* k_f16, const void* v_f16, int64_
                                     void* stream);
 
 /*
+ * New tokens as they are: token t of k_f16 / v_f16 (element strides per KV head and token, multiples of 4;
+ * channels contiguous) goes to row `row` + t of the fp16 decode buffers [nkv][dec_cap][128]: the fp16
+ * append of CacheLayer.update (src/shard/cache.py:138-191).  One launch for keys and values.
+ */
+int shard_b200_append_rows(const void* k_f16, const void* v_f16, int64_t k_head_stride, int64_t k_tok_stride,
+                           int64_t v_head_stride, int64_t v_tok_stride, int32_t n_tok, int32_t nkv, void* dec_k_f16,
+                           void* dec_v_f16, int64_t dec_cap, int64_t row, void* stream);
+
+/*
  * A compressed layer as fp16 keys and values, [nkv][rows][128] each with rows in the order
  * [sink | middle | window | stream | fp16 decode buffer]: CacheLayer._ensure_dequant
  * (src/shard/cache.py:87-124) with its callees, in one launch.  Of `shape` nkv, rank, n_comp, n_sink,

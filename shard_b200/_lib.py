@@ -66,6 +66,8 @@ _SIGNATURES = {
     "shard_b200_stream_quantize_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                                   C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                                   C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]),
+    "shard_b200_append_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int32, C.c_int32,
+                                         C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),
     "shard_b200_read_back": (C.c_int, [C.c_void_p, C.POINTER(ShardDecodeShape), C.c_void_p, C.c_void_p, C.c_int32,
                                        C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "shard_b200_multiquery_workspace_bytes": (C.c_size_t, [C.POINTER(ShardDecodeShape), C.c_int32]),
@@ -145,7 +147,8 @@ def host():
             raise ShardError(f"shard_b200/_host.so is missing or does not load ({e}): build it with "
                              "`python -m shard_b200.build`") from e
         lib = load()
-        mod.bind(*(C.cast(f, C.c_void_p).value for f in (lib.shard_b200_decode_attn, lib.shard_b200_phase_table)))
+        mod.bind(*(C.cast(f, C.c_void_p).value for f in (lib.shard_b200_decode_attn, lib.shard_b200_phase_table,
+                                                            lib.shard_b200_append_rows)))
         _host = mod
     return _host
 

@@ -227,13 +227,6 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
         gc["_pending"] = pending
         layer._flush_pending()
         pending = None
-    append = int(pending is not None)
-    if "_pending_dec" in gc:
-        # the newest row of the fp16 decode buffer is still to be written: by this launch if it is its last row
-        if with_fp16_segments and n_stream == 0 and (visible_new is None or int(visible_new) >= gc["decode_k"].shape[2]):
-            pending, append = gc.pop("_pending_dec"), 2
-        else:
-            layer._flush_pending()
     seq, shape = ls.seq, ls.shape
     if n_stream > 0:                                   # (asked for at every step: the buffers move when they grow)
         seq.st_k_idx, seq.st_v_idx = gc["k_idx_buf"].data_ptr(), gc["v_idx_buf"].data_ptr()
@@ -260,7 +253,7 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
     # with `push` and no `out` the record only goes to the exchange buffers
     seq.q, seq.out = q2.data_ptr(), (None if out is None else out.data_ptr())
     seq.phase = _phase_for(cache, gc, pos_q, t0, t1, dev).data_ptr() if t1 > t0 else None
-    shape.n_stream, shape.pos_q, shape.append = n_stream, int(pos_q), append
+    shape.n_stream, shape.pos_q, shape.append = n_stream, int(pos_q), int(pending is not None)
     shape.n_dec, shape.dec_cap = n_dec, dec_cap
     # the first launch on a freshly built dictionary follows the kernels that wrote its codes and
     # weights: it must not start early behind them

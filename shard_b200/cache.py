@@ -222,10 +222,11 @@ class CacheLayer(CacheLayerMixin):
                 prev._needs_decompress = True
         c._last_accessed_layer = self.layer_idx
 
-    def _ensure_dequant(self):
+    def _ensure_dequant(self, new=None):
         """Full fp16 K/V as [sink | middle | window | stream | fp16 decode buffer]
         (reference: src/shard/cache.py:87-124), one launch: what models without the fused
-        hook attend to at every step."""
+        hook attend to at every step.  `new`: keys and values of the newest fp16 row, which is still to be
+        written."""
         if not self._needs_decompress:
             return
         gc = self._gpu_compressed
@@ -241,12 +242,11 @@ class CacheLayer(CacheLayerMixin):
             gc["_pending"] = pend
             self._flush_pending()
             pend = None
-        pend_dec = gc.pop("_pending_dec", None)
         seq, shape, rows = layer_record(gc, nkv, hd, dev)
-        if pend is not None or pend_dec is not None:
-            new = pend if pend is not None else pend_dec
-            seq.new_k, seq.new_v = new[0].data_ptr(), new[1].data_ptr()
+        if pend is not None or new is not None:
             shape.append = 1 if pend is not None else 2
+            new = pend if pend is not None else new
+            seq.new_k, seq.new_v = new[0].data_ptr(), new[1].data_ptr()
         keys = torch.empty(1, nkv, rows, hd, dtype=torch.float16, device=dev)
         values = torch.empty_like(keys)
         ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
@@ -293,23 +293,34 @@ class CacheLayer(CacheLayerMixin):
 
         gc = self._gpu_compressed
         if gc is not None:
-            fused = getattr(c, "_fused_decode_update", False)
+            fused = bool(getattr(c, "_fused_decode_update", False))
             if not fused:
                 self._lazy_evict()
             streaming = bool(c._streaming)
-            # one token is handed to the launch that reads it next (fused decode or read-back), which
-            # puts it into its row: nothing is launched here
-            if not (seq_new == 1 and _lib.host().defer(gc, key_states, value_states, streaming)):
+            # One token of the stream is handed to the launch that reads it next (fused decode or read-back),
+            # which quantises it into its row: nothing is launched here, and until then the tensors are the
+            # caller's own.  A fp16 row is written before `update` returns: the buffer is public, and the
+            # caller may use its tensors for other things before it attends.
+            new = None
+            if not (seq_new == 1 and _lib.host().append(gc, key_states, value_states, streaming, fused)):
                 if streaming:
                     self._stream_append(key_states, value_states, self._seq_len, defer=seq_new == 1)
                 else:
-                    self._fp16_append(key_states, value_states, defer=seq_new == 1)
+                    self._fp16_append(key_states, value_states)
+            elif not (streaming or fused):
+                new = key_states, value_states             # (the read-back below writes it)
             self._seq_len += seq_new
             self._needs_decompress = True
             if fused:
                 c._last_accessed_layer = self.layer_idx
                 return key_states, value_states
-            self._ensure_dequant()
+            try:
+                self._ensure_dequant(new)
+            except BaseException:
+                if new is not None:                        # its row has been given out
+                    gc["decode_k"][:, :, -1:].copy_(new[0])
+                    gc["decode_v"][:, :, -1:].copy_(new[1])
+                raise
             return self._keys, self._values
 
         self._lazy_evict()
@@ -324,10 +335,9 @@ class CacheLayer(CacheLayerMixin):
         return self._keys, self._values
 
     # -- fp16 decode buffer ------------------------------------------------------
-    def _fp16_append(self, k, v, defer=False):
+    def _fp16_append(self, k, v):
         """Append (1, nkv, s, hd) new tokens as they are, in place, to a buffer allocated ahead (doubling
-        when full); gc["decode_k"] / ["decode_v"] are views of the rows in use.  With `defer` the one
-        token is left to the next launch that reads the rows, whose kernel writes it."""
+        when full); gc["decode_k"] / ["decode_v"] are views of the rows in use."""
         self._flush_pending()
         gc, c = self._gpu_compressed, self._cache_ref
         new = k.shape[2]
@@ -343,11 +353,8 @@ class CacheLayer(CacheLayerMixin):
                 new_v[:, :, :n].copy_(gc["decode_v"])
             buf_k, gc["_dec_buf_k"], gc["_dec_buf_v"] = new_k, new_k, new_v
         buf_v = gc["_dec_buf_v"]
-        if defer and k.dtype == torch.float16 and v.dtype == torch.float16 and gc.get("stream_n", 0) == 0:
-            gc["_pending_dec"] = (k.contiguous(), v.contiguous())
-        else:
-            buf_k[:, :, n:n + new].copy_(k)
-            buf_v[:, :, n:n + new].copy_(v)
+        buf_k[:, :, n:n + new].copy_(k)
+        buf_v[:, :, n:n + new].copy_(v)
         gc["decode_k"] = buf_k[:, :, :n + new]
         gc["decode_v"] = buf_v[:, :, :n + new]
 
@@ -355,10 +362,6 @@ class CacheLayer(CacheLayerMixin):
     def _flush_pending(self):
         """Write the row of a token whose append was left to the next launch and never got one."""
         gc = self._gpu_compressed
-        pend = gc.pop("_pending_dec", None) if gc is not None else None
-        if pend is not None:
-            gc["decode_k"][:, :, -1:].copy_(pend[0])
-            gc["decode_v"][:, :, -1:].copy_(pend[1])
         pend = gc.pop("_pending", None) if gc is not None else None
         if pend is not None:
             k2, v2, slot = pend

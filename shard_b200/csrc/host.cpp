@@ -24,8 +24,10 @@ using DecodeFn = int (*)(const ShardSeq*, int32_t, const ShardDecodeShape*, cons
 using PhaseFn = int (*)(int32_t, int32_t, int32_t, const float*, void*, void*);
 DecodeFn g_decode = nullptr;
 PhaseFn g_phase = nullptr;
+using AppendFn = int (*)(const void*, const void*, int64_t, int64_t, int64_t, int64_t, int32_t, int32_t, void*, void*, int64_t, int64_t, void*);
+AppendFn g_append = nullptr;
 
-PyObject *s_pending, *s_pending_dec, *s_stream_n, *s_k_idx, *s_v_idx, *s_k_norm, *s_v_norm, *s_signs, *s_decode_k, *s_decode_v,
+PyObject *s_pending, *s_stream_n, *s_k_idx, *s_v_idx, *s_k_norm, *s_v_norm, *s_signs, *s_decode_k, *s_decode_v,
     *s_buf_k, *s_buf_v, *s_fresh;
 
 // What does not change from step to step of one layer (the records belong to the Python launch state,
@@ -57,11 +59,12 @@ bool one_token(const at::Tensor& t, int64_t heads, int64_t hd) {
          (heads == 1 || t.stride(1) == hd) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 7) == 0;
 }
 
-// bind(address of shard_b200_decode_attn, address of shard_b200_phase_table)
+// bind(addresses of shard_b200_decode_attn, shard_b200_phase_table, shard_b200_append_rows)
 PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  if (n != 2) return PyErr_Format(PyExc_TypeError, "bind takes 2 arguments");
+  if (n != 3) return PyErr_Format(PyExc_TypeError, "bind takes 3 arguments");
   g_decode = reinterpret_cast<DecodeFn>(PyLong_AsVoidPtr(a[0]));
   g_phase = reinterpret_cast<PhaseFn>(PyLong_AsVoidPtr(a[1]));
+  g_append = reinterpret_cast<AppendFn>(PyLong_AsVoidPtr(a[2]));
   if (PyErr_Occurred()) return nullptr;
   Py_RETURN_NONE;
 }
@@ -91,17 +94,19 @@ PyObject* py_make_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return PyCapsule_New(s, "shard_b200.step", step_free);
 }
 
-// defer(gc, k, v, streaming) -> True: the token has its row and is left to the launch that reads it; None: not done
-PyObject* py_defer(PyObject*, PyObject* const* a, Py_ssize_t n) {
+// append(gc, k, v, streaming, now) -> True: the token has its row; None: not done.  A token of the stream is left to
+// the launch that reads it next.  An fp16 row is written now, on the current stream; without `now` the caller's
+// next call is the read-back that writes it.
+PyObject* py_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 4) return PyErr_Format(PyExc_TypeError, "defer takes 4 arguments");
+  if (n != 5) return PyErr_Format(PyExc_TypeError, "append takes 5 arguments");
   PyObject* gc = a[0];
   if (!PyDict_Check(gc) || !THPVariable_Check(a[1]) || !THPVariable_Check(a[2])) Py_RETURN_NONE;
   const at::Tensor &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
   if (k.dim() != 4 || k.scalar_type() != at::kHalf || v.scalar_type() != at::kHalf || !k.is_cuda() || v.device() != k.device()) Py_RETURN_NONE;
   const int64_t heads = k.size(1);
   if (!one_token(k, heads, SHARD_HEAD_DIM) || !one_token(v, heads, SHARD_HEAD_DIM)) Py_RETURN_NONE;
-  if (PyDict_GetItemWithError(gc, s_pending) || PyDict_GetItemWithError(gc, s_pending_dec)) Py_RETURN_NONE;
+  if (PyDict_GetItemWithError(gc, s_pending)) Py_RETURN_NONE;
   if (a[3] == Py_True) {
     const at::Tensor* buf = tensor_at(gc, s_k_idx);
     if (!buf || !PyDict_GetItemWithError(gc, s_signs)) Py_RETURN_NONE;
@@ -123,16 +128,20 @@ PyObject* py_defer(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!bk || !bv || !dk || bk->scalar_type() != at::kHalf) Py_RETURN_NONE;
   PyObject* so = PyDict_GetItemWithError(gc, s_stream_n);
   if (so && PyLong_AsLong(so) != 0) { PyErr_Clear(); Py_RETURN_NONE; }
-  const int64_t rows = dk->size(2);
-  if (rows >= bk->size(2) || bk->size(1) != heads || dk->data_ptr() != bk->data_ptr()) Py_RETURN_NONE;
+  const int64_t rows = dk->size(2), cap = bk->size(2);
+  if (rows >= cap || bk->size(1) != heads || dk->data_ptr() != bk->data_ptr()) Py_RETURN_NONE;
+  if (a[4] == Py_True) {
+    const int device = k.get_device();
+    if (c10::cuda::current_device() != device || bk->get_device() != device) Py_RETURN_NONE;
+    const int rc = g_append(k.data_ptr(), v.data_ptr(), SHARD_HEAD_DIM, 0, SHARD_HEAD_DIM, 0, 1, (int32_t)heads, bk->data_ptr(),
+                            bv->data_ptr(), cap, rows, c10::cuda::getCurrentCUDAStream(device).stream());
+    if (rc != 0) Py_RETURN_NONE;                                 // (the general path says why)
+  }
   PyObject* nk = THPVariable_Wrap(bk->narrow(2, 0, rows + 1));
   PyObject* nv = THPVariable_Wrap(bv->narrow(2, 0, rows + 1));
-  PyObject* pend = PyTuple_Pack(2, a[1], a[2]);
-  const bool ok = nk && nv && pend && !PyDict_SetItem(gc, s_decode_k, nk) && !PyDict_SetItem(gc, s_decode_v, nv) &&
-                  !PyDict_SetItem(gc, s_pending_dec, pend);
+  const bool ok = nk && nv && !PyDict_SetItem(gc, s_decode_k, nk) && !PyDict_SetItem(gc, s_decode_v, nv);
   Py_XDECREF(nk);
   Py_XDECREF(nv);
-  Py_XDECREF(pend);
   if (!ok) return nullptr;
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
@@ -156,11 +165,10 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyObject* so = PyDict_GetItemWithError(gc, s_stream_n);
   const int n_stream = so ? (int)PyLong_AsLong(so) : 0;
   PyObject* pend = PyDict_GetItemWithError(gc, s_pending);
-  PyObject* pend_dec = PyDict_GetItemWithError(gc, s_pending_dec);
   const at::Tensor *new_k = nullptr, *new_v = nullptr;
   int append = 0;
   if (pend) {
-    if (pend_dec || PyLong_AsLong(PyTuple_GET_ITEM(pend, 2)) != n_stream - 1) Py_RETURN_NONE;
+    if (PyLong_AsLong(PyTuple_GET_ITEM(pend, 2)) != n_stream - 1) Py_RETURN_NONE;
     new_k = &THPVariable_Unpack(PyTuple_GET_ITEM(pend, 0));
     new_v = &THPVariable_Unpack(PyTuple_GET_ITEM(pend, 1));
     append = 1;
@@ -175,12 +183,6 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
     dec_cap = sh.nkv > 1 ? (int)(dk->stride(1) / SHARD_HEAD_DIM) : n_dec;
     seq.dec_k = dk->data_ptr();
     seq.dec_v = dv->data_ptr();
-    if (pend_dec) {
-      if (n_stream > 0) Py_RETURN_NONE;
-      new_k = &THPVariable_Unpack(PyTuple_GET_ITEM(pend_dec, 0));
-      new_v = &THPVariable_Unpack(PyTuple_GET_ITEM(pend_dec, 1));
-      append = 2;
-    }
   }
   if (append) {
     if (!fp16_cuda(*new_k, st->device) || !fp16_cuda(*new_v, st->device)) Py_RETURN_NONE;
@@ -216,7 +218,7 @@ PyObject* py_attend(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const int rc = g_decode(&seq, 1, &sh, st->inv_freq, n_stream > 0 ? st->codebook : nullptr, ws.data_ptr(), (size_t)ws.numel(),
                           c10::cuda::getCurrentCUDAStream(st->device).stream());
   if (rc != 0) return PyLong_FromLong(rc);
-  if (append == 1 ? PyDict_DelItem(gc, s_pending) : append == 2 ? PyDict_DelItem(gc, s_pending_dec) : 0) return nullptr;
+  if (append && PyDict_DelItem(gc, s_pending)) return nullptr;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -225,7 +227,7 @@ PyMethodDef methods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
     {"phase_table", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_phase_table)), METH_FASTCALL, nullptr},
     {"make_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_make_step)), METH_FASTCALL, nullptr},
-    {"defer", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_defer)), METH_FASTCALL, nullptr},
+    {"append", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_append)), METH_FASTCALL, nullptr},
     {"attend", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_attend)), METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host half of a decode step.", -1, methods, nullptr, nullptr, nullptr, nullptr};
@@ -234,7 +236,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host half of a dec
 
 PyMODINIT_FUNC PyInit__host() {
   const struct { PyObject** s; const char* name; } names[] = {
-      {&s_pending, "_pending"}, {&s_pending_dec, "_pending_dec"}, {&s_stream_n, "stream_n"}, {&s_k_idx, "k_idx_buf"},
+      {&s_pending, "_pending"}, {&s_stream_n, "stream_n"}, {&s_k_idx, "k_idx_buf"},
       {&s_v_idx, "v_idx_buf"}, {&s_k_norm, "k_norm_buf"}, {&s_v_norm, "v_norm_buf"}, {&s_signs, "signs"},
       {&s_decode_k, "decode_k"}, {&s_decode_v, "decode_v"}, {&s_buf_k, "_dec_buf_k"}, {&s_buf_v, "_dec_buf_v"}, {&s_fresh, "_fresh"}};
   for (const auto& x : names)

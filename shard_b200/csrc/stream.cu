@@ -1,4 +1,5 @@
-// 8-bit Lloyd-Max quantiser for tokens appended during decode, and its inverse.
+// 8-bit Lloyd-Max quantiser for tokens appended during decode, and its inverse; the append of tokens kept as
+// they are.
 //
 // One warp handles one (tensor, KV head) vector of 128 channels; lane l owns
 // channels 4l..4l+3.  Every arithmetic step that decides a code is a single
@@ -8,7 +9,7 @@
 //   u   = x / n                                   (IEEE division)
 //   rot = H128(u * signs) / fp32(sqrt(128))       (butterfly order h = 1..64)
 //   idx = nearest codebook entry, ties to the right neighbour
-#include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace shard {
 
@@ -59,6 +60,34 @@ __global__ void __launch_bounds__(128) stream_quantize_rows_kernel(const __grid_
   const __half* src = is_v ? p.v + kv * p.v_head + t * p.v_tok : p.k + kv * p.k_head + t * p.k_tok;
   const size_t row = (size_t)(p.slot + t) * p.nkv + kv;
   quantize_vec_warp(src, p.signs, cb, (is_v ? p.v_idx : p.k_idx) + row * HD, (is_v ? p.v_norm : p.k_norm) + row, lane);
+}
+
+// New tokens of a cache that keeps them as they are: keys and values to rows row .. row + n_tok - 1 of the
+// fp16 decode buffers [nkv][cap][128], a warp per vector.  One launch instead of two strided copies, and it
+// lets the decode launch behind it place its CTAs meanwhile.  Bound: one launch's latency, 1.7 us a layer (12K tokens
+// of context, 4 KV heads, 8 layers: 142 us a step; 129 us with the row written by the decode launch, which is
+// sound only as long as the caller leaves its tensors alone until then).
+struct AppendRowsParams {
+  const __half *k, *v;
+  int64_t k_head, k_tok, v_head, v_tok;
+  __half *dst_k, *dst_v;
+  int64_t cap, row;
+  int nkv, n_tok;
+};
+
+__global__ void __launch_bounds__(256) append_rows_kernel(const __grid_constant__ AppendRowsParams p) {
+  griddep_launch();
+  griddep_wait();                                        // the tokens may come from the kernel in front
+  const int lane = threadIdx.x & 31;
+  const long long half_units = (long long)p.nkv * p.n_tok;
+  for (long long u = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); u < 2 * half_units; u += (long long)gridDim.x * 8) {
+    const bool is_v = u >= half_units;
+    const long long w = is_v ? u - half_units : u;
+    const long long kv = w / p.n_tok, t = w - kv * p.n_tok;
+    const __half* src = is_v ? p.v + kv * p.v_head + t * p.v_tok : p.k + kv * p.k_head + t * p.k_tok;
+    __half* dst = (is_v ? p.dst_v : p.dst_k) + (kv * p.cap + p.row + t) * HD;
+    reinterpret_cast<uint2*>(dst)[lane] = reinterpret_cast<const uint2*>(src)[lane];
+  }
 }
 
 // out[kv][t][:] = fp16( fp32(fp16(H128(cb[idx]) / sqrt(128) * signs)) * fp32(norm) )
@@ -135,6 +164,29 @@ extern "C" int shard_b200_stream_quantize_rows(const void* k_f16, const void* v_
   shard::stream_quantize_rows_kernel<<<dim3((2 * nkv + 3) / 4, n_tok), 128, 0, (cudaStream_t)stream>>>(p);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
+}
+
+extern "C" int shard_b200_append_rows(const void* k_f16, const void* v_f16, int64_t k_head_stride, int64_t k_tok_stride,
+                                      int64_t v_head_stride, int64_t v_tok_stride, int32_t n_tok, int32_t nkv, void* dec_k_f16,
+                                      void* dec_v_f16, int64_t dec_cap, int64_t row, void* stream) {
+  if (!k_f16 || !v_f16 || !dec_k_f16 || !dec_v_f16 || n_tok < 0 || nkv < 1 || row < 0 || row + n_tok > dec_cap) return SHARD_E_ARG;
+  if ((((uintptr_t)k_f16 | (uintptr_t)v_f16 | (uintptr_t)dec_k_f16 | (uintptr_t)dec_v_f16) & 7) ||
+      ((k_head_stride | k_tok_stride | v_head_stride | v_tok_stride) & 3))
+    return SHARD_E_ALIGN;
+  if (n_tok == 0) return SHARD_OK;
+  shard::AppendRowsParams p{(const __half*)k_f16, (const __half*)v_f16, k_head_stride, k_tok_stride, v_head_stride, v_tok_stride,
+                            (__half*)dec_k_f16, (__half*)dec_v_f16, dec_cap, row, nkv, n_tok};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(shard::capped_blocks((2ll * nkv * n_tok + 7) / 8, 8));
+  cfg.blockDim = dim3(256);
+  cfg.stream = (cudaStream_t)stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, shard::append_rows_kernel, p);
+  return e == cudaSuccess ? SHARD_OK : (int)e;
 }
 
 extern "C" int shard_b200_stream_dequant(const uint8_t* idx, const void* norm_f16, const float* signs,

@@ -61,10 +61,6 @@ def shard_layer_tokens(gc: dict, rank: int, world: int) -> dict:
     Pure tensor slicing: works on any device.
     """
     begin, end = split_ranges(gc["n_compress"], world)[rank]
-    if "_pending_dec" in gc:                           # the newest fp16 row is still to be written
-        k, v = gc.pop("_pending_dec")
-        gc["decode_k"][:, :, -1:].copy_(k)
-        gc["decode_v"][:, :, -1:].copy_(v)
     n_total, keep = gc["k_coeffs_shape"]
     rows = gc["k_coeffs"].view(n_total, keep // 2)[begin:end]
     out = {k: v for k, v in gc.items() if not k.startswith("_") and k not in (

@@ -132,3 +132,40 @@ def test_a_failed_allocation_is_a_python_exception():
     out = fused_attention_compressed(q, layer, 403, cache._rope_inv_freq)      # the token is still to be appended
     cache.check()
     assert out.shape == want.shape and "_pending" not in layer._gpu_compressed
+
+
+@pytest.mark.parametrize("nkv,n_comp", [(8, 300), (1, 1)])
+def test_fp16_rows_are_the_caches_own(nkv, n_comp):
+    """A cache that keeps tokens as they are has copied them when `update` returns: the caller's tensors may
+    change before it attends, and the rows are there for whoever reads `decode_k` / `decode_v`."""
+    from shard_b200 import fused_attention_compressed
+    from shard_b200.attention import decode_layer
+    cache, layer = _cache(random_gc(n_comp, nkv=nkv, seed=1), nkv, False, capacity=16)
+    other, ref = _cache(random_gc(n_comp, nkv=nkv, seed=1), nkv, False, capacity=16)
+    cache._fused_decode_update = True
+    g = torch.Generator(device="cuda").manual_seed(3)
+    k, v = (torch.empty(1, nkv, 1, 128, dtype=torch.float16, device="cuda") for _ in range(2))
+    gc, rows = layer._gpu_compressed, []
+    for t in range(24):                                    # the same two tensors for every token, over a growth of the buffers
+        k.normal_(generator=g)
+        v.normal_(generator=g)
+        rows.append((k.clone(), v.clone()))
+        ref._fp16_append(*rows[-1])
+        q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+        layer.update(k, v)
+        k.zero_()
+        v.fill_(float("nan"))
+        for name, i in (("decode_k", 0), ("decode_v", 1)):
+            assert torch.equal(gc[name], torch.cat([r[i] for r in rows], 2))
+        out = fused_attention_compressed(q, layer, 400 + t, cache._rope_inv_freq)
+        assert torch.equal(out.view(-1, 128), decode_layer(q, ref, 400 + t))
+    cache._fused_decode_update = False
+    k.normal_(generator=g)
+    v.normal_(generator=g)
+    rows.append((k.clone(), v.clone()))
+    keys, values = layer.update(k, v)                      # written by the read-back
+    k.zero_()
+    v.zero_()
+    for got, name, i in ((keys, "decode_k", 0), (values, "decode_v", 1)):
+        want = torch.cat([r[i] for r in rows], 2)
+        assert torch.equal(gc[name], want) and torch.equal(got[:, :, -len(rows):], want)

@@ -33,3 +33,25 @@ def test_decode_rows(n_comp, nkv, rows, streaming):
         want = torch.softmax(sc, -1) @ values.repeat_interleave(4, 0)
         err = (out[0].double() - want).abs()
         assert (err <= 1.5e-3 + 5e-3 * want.abs()).all(), err.max()
+
+
+@pytest.mark.parametrize("n_comp,nkv", [(700, 8), (0, 2)])
+def test_decode_launch_writes_the_newest_fp16_row(n_comp, nkv):
+    """`append = 2` of the C entry point: the launch copies new_k / new_v into the last row, then attends."""
+    from shard_b200 import ops
+    from shard_b200.attention import decode_layer
+    cache, layer = _cache(random_gc(max(n_comp, 1), nkv=nkv, seed=5), nkv, False, capacity=16)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    k, v = (torch.randn(1, nkv, 9, 128, generator=g, device="cuda").half() for _ in range(2))
+    layer._fp16_append(k, v)
+    q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+    tok = (0, n_comp)
+    want = decode_layer(q, layer, 800, tok_range=tok).clone()
+    gc, out = layer._gpu_compressed, torch.empty(4 * nkv, 128, dtype=torch.float16, device="cuda")
+    for name in ("decode_k", "decode_v"):
+        gc[name][:, :, -1:].zero_()
+    last = [x[0, :, -1].contiguous() for x in (k, v)]
+    ls = gc["_launch"]
+    ls.seq.new_k, ls.seq.new_v, ls.seq.out, ls.shape.append = last[0].data_ptr(), last[1].data_ptr(), out.data_ptr(), 2
+    ops.decode_attn(ls.seq, 1, ls.shape, ls.inv_ptr, None, cache._decode_ws)
+    assert torch.equal(out, want) and torch.equal(gc["decode_k"], k) and torch.equal(gc["decode_v"], v)

@@ -295,7 +295,9 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
         return None
     if q_rope.shape[2] == 1:
         return decode_layer(q_rope, layer, pos_q, out=out, plain_step=True)
-    _, n_q, s_q, hd = q_rope.shape
+    B, n_q, s_q, hd = q_rope.shape
+    if B != 1:
+        raise NotImplementedError("query tokens of one sequence only")
     cache = layer._cache_ref
     layer._flush_pending()                             # every new token is in its row before the first query looks
     n_new_total = gc.get("stream_n", 0) if "k_idx_buf" in gc else (gc["decode_k"].shape[2] if "decode_k" in gc else 0)

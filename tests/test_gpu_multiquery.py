@@ -38,3 +38,15 @@ def test_multiquery(n_comp, rank, nkv, before, s, streaming):
     assert (err <= 1.5e-3 + 5e-3 * want.abs()).all(), err.max()
     again = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq, out=torch.empty_like(out).contiguous())
     assert torch.equal(again, out)
+
+
+@pytest.mark.parametrize("s", [1, 2, 3, 40])
+def test_queries_of_two_sequences_are_refused(s):
+    from shard_b200 import fused_attention_compressed
+    cache, layer = _cache(random_gc(200, nkv=2, seed=s), 2, True)
+    cache._fused_decode_update = True
+    new = torch.randn(1, 2, s, 128, device="cuda").half()
+    layer.update(new, new)
+    q = torch.randn(2, 8, s, 128, device="cuda").half()
+    with pytest.raises(NotImplementedError):
+        fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)

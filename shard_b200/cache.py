@@ -302,7 +302,8 @@ class CacheLayer(CacheLayerMixin):
             # caller's own.  A fp16 row is written before `update` returns: the buffer is public, and the
             # caller may use its tensors for other things before it attends.
             new = None
-            if not (seq_new == 1 and _lib.host().append(gc, key_states, value_states, streaming, fused)):
+            native = seq_new == 1 and not (streaming and (c._stream_qjl or c._stream_bits != 8))
+            if not (native and _lib.host().append(gc, key_states, value_states, streaming, fused)):
                 if streaming:
                     self._stream_append(key_states, value_states, self._seq_len, defer=seq_new == 1)
                 else:
@@ -334,10 +335,19 @@ class CacheLayer(CacheLayerMixin):
             self._values = value_states
         return self._keys, self._values
 
+    def _check_tokens(self, k, v):
+        """New tokens of the one sequence, with the cache's heads (the kernels take as many as the cache has)."""
+        c = self._cache_ref
+        if k.shape[0] != 1:
+            raise NotImplementedError("one sequence per Cache (use one Cache per sequence)")
+        if k.shape != v.shape or k.shape[1] != c._n_kv_heads or k.shape[3] != c.head_dim:
+            raise ShardError(f"expected keys and values (1, {c._n_kv_heads}, s, {c.head_dim}), got {tuple(k.shape)} and {tuple(v.shape)}")
+
     # -- fp16 decode buffer ------------------------------------------------------
     def _fp16_append(self, k, v):
         """Append (1, nkv, s, hd) new tokens as they are, in place, to a buffer allocated ahead (doubling
         when full); gc["decode_k"] / ["decode_v"] are views of the rows in use."""
+        self._check_tokens(k, v)
         self._flush_pending()
         gc, c = self._gpu_compressed, self._cache_ref
         new = k.shape[2]
@@ -374,15 +384,7 @@ class CacheLayer(CacheLayerMixin):
         """(Re)allocate the stream buffers for at least `need` rows: the cache's decode capacity at
         first, doubling afterwards (reference: src/shard/cache.py:220-230, which starts at 16 rows)."""
         c = self._cache_ref
-        if c._stream_qjl:
-            raise NotImplementedError("the QJL residual is not part of the CUDA stream path")
-        if c._stream_bits != 8:
-            raise NotImplementedError("the CUDA stream quantizer emits 8-bit codes only")
         B, heads, _, hd = k.shape
-        if B != 1:
-            raise NotImplementedError("one sequence per Cache (use one Cache per sequence)")
-        if k.dtype != torch.float16:
-            raise NotImplementedError("fp16 models only")
         dev = k.device
         if "signs" not in gc:
             gc["signs"] = stream_signs(self.layer_idx, hd, dev)
@@ -405,14 +407,20 @@ class CacheLayer(CacheLayerMixin):
         """Quantise (1, nkv, s, hd) new tokens into the stream buffers
         (reference: src/shard/cache.py:193-241).  With `defer` the row is reserved and the one
         token is handed to the next launch that reads the stream, whose kernel quantises it."""
+        c = self._cache_ref
+        if c._stream_qjl:
+            raise NotImplementedError("the QJL residual is not part of the CUDA stream path")
+        if c._stream_bits != 8:
+            raise NotImplementedError("the CUDA stream quantizer emits 8-bit codes only")
+        self._check_tokens(k, v)
+        if k.dtype != torch.float16 or v.dtype != torch.float16:
+            raise NotImplementedError("fp16 models only")
         self._flush_pending()
         gc = self._gpu_compressed
         new = k.shape[2]
         s = gc.get("stream_n", 0)
         if "signs" not in gc or s + new > gc["k_idx_buf"].shape[0]:
             self._grow_stream(gc, k, s + new)
-        if k.dtype != torch.float16 or v.dtype != torch.float16:
-            raise NotImplementedError("fp16 models only")
         if defer:
             gc["_pending"] = (k.contiguous(), v.contiguous(), s)
         else:

@@ -113,6 +113,7 @@ PyObject* py_append(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyObject* so = PyDict_GetItemWithError(gc, s_stream_n);
     const long s = so ? PyLong_AsLong(so) : 0;
     if (s < 0 || s >= buf->size(0)) { PyErr_Clear(); Py_RETURN_NONE; }
+    if (buf->dim() != 4 || buf->size(2) != heads) Py_RETURN_NONE;
     PyObject* row = PyLong_FromLong(s);
     PyObject* next = PyLong_FromLong(s + 1);
     PyObject* pend = PyTuple_Pack(3, a[1], a[2], row);

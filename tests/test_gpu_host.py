@@ -169,3 +169,36 @@ def test_fp16_rows_are_the_caches_own(nkv, n_comp):
     for got, name, i in ((keys, "decode_k", 0), (values, "decode_v", 1)):
         want = torch.cat([r[i] for r in rows], 2)
         assert torch.equal(gc[name], want) and torch.equal(got[:, :, -len(rows):], want)
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("s", [1, 3])
+def test_tokens_that_do_not_fit_the_cache_are_refused(streaming, s):
+    """Tokens of two sequences, of other heads, or (stream) with options the kernels do not have: refused
+    also when the buffers have room, and the cache is as it was."""
+    from shard_b200._lib import ShardError
+    cache, layer = _cache(random_gc(200, nkv=2, seed=1), 2, streaming, capacity=64)
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def new(*shape):
+        return torch.randn(*shape, 128, generator=g, device="cuda").half()
+
+    keys, _ = layer.update(new(1, 2, 2), new(1, 2, 2))
+    n, want = layer.get_seq_length(), keys.clone()
+    for fused in (True, False):
+        cache._fused_decode_update = fused
+        for shape, err in (((2, 2, s), NotImplementedError), ((1, 1, s), ShardError), ((1, 4, s), ShardError)):
+            with pytest.raises(err):
+                layer.update(new(*shape), new(*shape))
+        with pytest.raises(ShardError):
+            layer.update(new(1, 2, s), new(1, 2, s + 1))
+        if streaming:
+            for flag, value in (("_stream_qjl", True), ("_stream_bits", 4)):
+                was = getattr(cache, flag)
+                setattr(cache, flag, value)
+                with pytest.raises(NotImplementedError):
+                    layer.update(new(1, 2, s), new(1, 2, s))
+                setattr(cache, flag, was)
+    assert layer.get_seq_length() == n
+    layer._needs_decompress = True
+    assert torch.equal(layer.keys, want)

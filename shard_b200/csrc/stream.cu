@@ -37,15 +37,15 @@ __global__ void __launch_bounds__(128) stream_quantize_kernel(const __grid_const
   quantize_vec_warp(src, s.signs, cb, idx_out, norm_out, lane);
 }
 
-// Several new tokens at once (a forward over more than one token): token blockIdx.y of `k` / `v`
-// (element strides per KV head and token, channels contiguous) goes to row slot + blockIdx.y.
+// Several new tokens at once (a forward over more than one token): token t of `k` / `v` (element strides per
+// KV head and token, channels contiguous) goes to row slot + t; a warp per vector.
 struct StreamRowsParams {
   const __half *k, *v;
   int64_t k_head, k_tok, v_head, v_tok;
   const float *signs, *codebook;
   uint8_t *k_idx, *v_idx;
   __half *k_norm, *v_norm;
-  int nkv, slot;
+  int nkv, slot, n_tok;
 };
 
 __global__ void __launch_bounds__(128) stream_quantize_rows_kernel(const __grid_constant__ StreamRowsParams p) {
@@ -53,13 +53,16 @@ __global__ void __launch_bounds__(128) stream_quantize_rows_kernel(const __grid_
   for (int i = threadIdx.x; i < 256; i += blockDim.x) cb[i] = p.codebook[i];
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  const int vec = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (vec >= 2 * p.nkv) return;
-  const bool is_v = vec >= p.nkv;
-  const int kv = is_v ? vec - p.nkv : vec, t = blockIdx.y;
-  const __half* src = is_v ? p.v + kv * p.v_head + t * p.v_tok : p.k + kv * p.k_head + t * p.k_tok;
-  const size_t row = (size_t)(p.slot + t) * p.nkv + kv;
-  quantize_vec_warp(src, p.signs, cb, (is_v ? p.v_idx : p.k_idx) + row * HD, (is_v ? p.v_norm : p.k_norm) + row, lane);
+  const long long n_vec = 2ll * p.nkv * p.n_tok;
+  for (long long u = (long long)blockIdx.x * 4 + (threadIdx.x >> 5); u < n_vec; u += (long long)gridDim.x * 4) {
+    const long long t = u / (2 * p.nkv);
+    const int vec = (int)(u - t * (2 * p.nkv));
+    const bool is_v = vec >= p.nkv;
+    const int kv = is_v ? vec - p.nkv : vec;
+    const __half* src = is_v ? p.v + kv * p.v_head + t * p.v_tok : p.k + kv * p.k_head + t * p.k_tok;
+    const size_t row = (size_t)(p.slot + t) * p.nkv + kv;
+    quantize_vec_warp(src, p.signs, cb, (is_v ? p.v_idx : p.k_idx) + row * HD, (is_v ? p.v_norm : p.k_norm) + row, lane);
+  }
 }
 
 // New tokens of a cache that keeps them as they are: keys and values to rows row .. row + n_tok - 1 of the
@@ -152,16 +155,16 @@ extern "C" int shard_b200_stream_quantize_rows(const void* k_f16, const void* v_
                                                int32_t n_tok, int32_t nkv, const float* signs, const float* codebook,
                                                uint8_t* k_idx, uint8_t* v_idx, void* k_norm, void* v_norm, int32_t slot,
                                                void* stream) {
-  if (!k_f16 || !v_f16 || !signs || !codebook || !k_idx || !v_idx || !k_norm || !v_norm || n_tok < 0 || n_tok > 65535 ||
-      nkv < 1 || slot < 0)
+  if (!k_f16 || !v_f16 || !signs || !codebook || !k_idx || !v_idx || !k_norm || !v_norm || n_tok < 0 || nkv < 1 || slot < 0 ||
+      n_tok > INT32_MAX - slot)
     return SHARD_E_ARG;
   if (((uintptr_t)k_f16 & 7) || ((uintptr_t)v_f16 & 7) || (k_head_stride & 3) || (k_tok_stride & 3) || (v_head_stride & 3) ||
       (v_tok_stride & 3) || ((uintptr_t)k_idx & 3) || ((uintptr_t)v_idx & 3) || ((uintptr_t)signs & 15))
     return SHARD_E_ALIGN;
   if (n_tok == 0) return SHARD_OK;
   shard::StreamRowsParams p{(const __half*)k_f16, (const __half*)v_f16, k_head_stride, k_tok_stride, v_head_stride, v_tok_stride,
-                            signs, codebook, k_idx, v_idx, (__half*)k_norm, (__half*)v_norm, nkv, slot};
-  shard::stream_quantize_rows_kernel<<<dim3((2 * nkv + 3) / 4, n_tok), 128, 0, (cudaStream_t)stream>>>(p);
+                            signs, codebook, k_idx, v_idx, (__half*)k_norm, (__half*)v_norm, nkv, slot, n_tok};
+  shard::stream_quantize_rows_kernel<<<shard::capped_blocks((2ll * nkv * n_tok + 3) / 4, 16), 128, 0, (cudaStream_t)stream>>>(p);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }

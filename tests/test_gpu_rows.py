@@ -55,3 +55,19 @@ def test_decode_launch_writes_the_newest_fp16_row(n_comp, nkv):
     ls.seq.new_k, ls.seq.new_v, ls.seq.out, ls.shape.append = last[0].data_ptr(), last[1].data_ptr(), out.data_ptr(), 2
     ops.decode_attn(ls.seq, 1, ls.shape, ls.inv_ptr, None, cache._decode_ws)
     assert torch.equal(out, want) and torch.equal(gc["decode_k"], k) and torch.equal(gc["decode_v"], v)
+
+
+@pytest.mark.parametrize("n", [65535, 65536, 70001])
+def test_many_tokens_in_one_append(n):
+    """A turn of more tokens than a grid has rows: the codes are those of the same tokens appended in parts."""
+    cache, layer = _cache(random_gc(1, nkv=2, seed=5), 2, True, capacity=16)
+    other, ref = _cache(random_gc(1, nkv=2, seed=5), 2, True, capacity=n)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    k, v = (torch.randn(1, 2, n, 128, generator=g, device="cuda").half() for _ in range(2))
+    cache._fused_decode_update = other._fused_decode_update = True
+    layer.update(k, v)
+    for i in range(0, n, 9000):
+        ref.update(k[:, :, i:i + 9000], v[:, :, i:i + 9000])
+    assert layer.get_seq_length() == ref.get_seq_length()
+    for name in ("k_idx_buf", "v_idx_buf", "k_norm_buf", "v_norm_buf"):
+        assert torch.equal(layer._gpu_compressed[name][:n], ref._gpu_compressed[name][:n])

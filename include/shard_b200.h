@@ -356,7 +356,8 @@ int shard_b200_undo_rope(const void* k_f16, int64_t head_stride, int64_t tok_str
  * NULL, fp16) and the Gram matrix (flat - mean)^T (flat - mean), fp32 [dim][dim] with dim = nkv*128, at
  * fp32 accuracy on the tensor cores.  flat_out and workspace 16-byte aligned; workspace:
  * shard_b200_k_covariance_workspace_bytes bytes (0: sizes not supported, nkv <= 32); its second 32-bit word is
- * set to 1 if a bounded wait gave up.
+ * set to 1 if a bounded wait gave up (the matrix is then undefined) and never cleared: the caller zeroes it
+ * once, and reads it when it next waits for the device.
  */
 size_t shard_b200_k_covariance_workspace_bytes(int32_t nkv, int32_t n);
 int shard_b200_k_covariance(const void* k_f16, int64_t head_stride, int64_t tok_stride, int32_t nkv, int32_t n,
@@ -368,7 +369,9 @@ int shard_b200_k_covariance(const void* k_f16, int64_t head_stride, int64_t tok_
  * Everything behind the PCA fit of one layer's keys in one call: shard_b200_k_basis_quantise of basis
  * [nkv*128][keep], shard_b200_k_project, shard_b200_k_quantize_pack with alloc_bits_host [keep] (a HOST
  * array), the coefficient scales as fp16, and -- if wprep_out is not NULL, keep a multiple of 32 --
- * shard_b200_decode_prepare.  workspace: shard_b200_k_encode_workspace_bytes bytes, 16-byte aligned.
+ * shard_b200_decode_prepare.  workspace: shard_b200_k_encode_workspace_bytes bytes, 16-byte aligned;
+ * its first 32-bit word is set to 1 if a bounded wait of the projection gave up (the codes are then undefined) and
+ * never cleared: the caller zeroes it once, and reads it when it next waits for the device.
  */
 size_t shard_b200_k_encode_workspace_bytes(int32_t nkv, int32_t n, int32_t keep);
 int shard_b200_k_encode(const float* flat, const float* mean, const void* mean_f16, const float* basis,

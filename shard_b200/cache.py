@@ -106,10 +106,11 @@ def _stream_of_thread(device):
 
 class LeadingEigenpairs:
     """The `rank` largest eigenpairs of each (p, p) matrix of `gram` (count, p, p): launched on the current
-    stream when made, waited for by `result` (on the same stream)."""
+    stream when made, waited for by `result` (on the same stream).  `status`: the status word of the kernels
+    that made `gram`, looked at then."""
 
-    def __init__(self, gram, rank):
-        self.gram, self.rank = gram, rank
+    def __init__(self, gram, rank, status=None):
+        self.gram, self.rank, self.status = gram, rank, status
         self.basis, self.eigvals, self.flag = ops.eigh_top(gram, rank)
 
     def result(self):
@@ -117,7 +118,10 @@ class LeadingEigenpairs:
         on the host.  Matrices the package's solver reports as too close to degenerate go to
         torch.linalg.eigh."""
         rank = self.rank
-        host = torch.cat([self.eigvals, self.flag.unsqueeze(1).float()], dim=1).cpu()
+        made = torch.zeros_like(self.flag) if self.status is None else self.status.expand_as(self.flag)
+        host = torch.cat([self.eigvals, torch.stack([self.flag, made], 1).float()], dim=1).cpu()
+        if host[:, rank + 1].any():
+            raise ShardError("the covariance of the keys is undefined: a wait inside its kernel gave up")
         for i in torch.nonzero(host[:, rank]).flatten().tolist():
             w, v = torch.linalg.eigh(self.gram[i])
             self.basis[i] = v.flip(-1)[:, :rank]
@@ -125,8 +129,14 @@ class LeadingEigenpairs:
         return self.basis, host[:, :rank]
 
 
-def leading_eigenpairs(gram, rank):
-    return TorchEigenpairs(gram, rank) if gram.shape[1] <= TORCH_EIGH_MAX else LeadingEigenpairs(gram, rank)
+def leading_eigenpairs(gram, rank, status=None):
+    return TorchEigenpairs(gram, rank) if gram.shape[1] <= TORCH_EIGH_MAX else LeadingEigenpairs(gram, rank, status)
+
+
+def check_encoded(workspace):
+    """Raise if a wait inside a `k_encode` call with this scratch gave up (waits for the device)."""
+    if int(ops.encode_status(workspace).item()):
+        raise ShardError("the key codes are undefined: a wait inside the projection gave up")
 
 
 def pca_fit(flat, mean, rank):
@@ -598,7 +608,7 @@ class Cache(HFCache):
             rows, gram, done = ready
             side.wait_event(done)
             with torch.cuda.stream(side):
-                solved = leading_eigenpairs(gram, rank)
+                solved = leading_eigenpairs(gram, rank, None if cov_ws is None else ops.covariance_status(cov_ws))
             vparts = self._compress_v_layers([self.layers[li]._values[0, :, start:end, :]
                                               for li in range(bounds[g], bounds[g + 1])], init_rows=init_rows)
             ends = [self._ends(li, end) for li in range(bounds[g], bounds[g + 1])]
@@ -613,6 +623,7 @@ class Cache(HFCache):
                 self._finish_layer(li, kpart, vparts[i], ends[i], start, end)
         # the second stream's tensors go back to the allocator behind everything enqueued here
         side.wait_stream(main)
+        check_encoded(enc_ws)
 
     def _ends(self, li, end):
         layer = self.layers[li]
@@ -646,7 +657,9 @@ class Cache(HFCache):
         else:
             basis = basis.to(dev, torch.float32)[:, :rank]
             eigvals = ((flat - mean) @ basis).pow(2).sum(dim=0) / n
-        return self._quantise_k(flat, mean, mean.half(), basis, eigvals)[0]
+        kpart, workspace = self._quantise_k(flat, mean, mean.half(), basis, eigvals)
+        check_encoded(workspace)
+        return kpart
 
     def _quantise_k(self, flat, mean, mean_f16, basis, eigvals, workspace=None):
         """Bit allocation, int8 basis, projection and int4 codes of un-rotated keys `flat` (n, dim)."""

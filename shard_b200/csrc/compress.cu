@@ -31,10 +31,12 @@ __global__ void kq_init_kernel(uint32_t* ws, int keep) {
   if (j < keep) { ws[j] = 0xffffffffu; ws[keep + j] = 0u; ws[2 * keep + j] = 0u; }
 }
 
-// the same, and the bit widths handed over as a kernel argument
+// the same, and the bit widths handed over as a kernel argument; passes the projection's status word on
 struct KqBits { uint8_t b[256]; };
-__global__ void kq_init_bits_kernel(uint32_t* ws, int keep, const __grid_constant__ KqBits bits, int32_t* __restrict__ alloc) {
+__global__ void kq_init_bits_kernel(uint32_t* ws, int keep, const __grid_constant__ KqBits bits, int32_t* __restrict__ alloc,
+                                    const int* __restrict__ gave_up, int* __restrict__ status) {
   const int j = threadIdx.x;
+  if (j == 0 && *gave_up) *status = 1;
   if (j < keep) { ws[j] = 0xffffffffu; ws[keep + j] = 0u; ws[2 * keep + j] = 0u; alloc[j] = bits.b[j]; }
 }
 
@@ -358,12 +360,13 @@ extern "C" int shard_b200_k_quantize_pack(const float* proj, const int32_t* allo
   return SHARD_OK;
 }
 
-// workspace of shard_b200_k_encode: w | projection | bit widths, counters, scales | projection's own
-struct KEncodeLayout { size_t proj, small, project, bytes; };
+// workspace of shard_b200_k_encode: status word | w | projection | bit widths, counters, scales | projection's own
+struct KEncodeLayout { size_t w, proj, small, project, bytes; };
 static KEncodeLayout k_encode_layout(int nkv, int n, int keep) {
   KEncodeLayout l;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  l.proj = up((size_t)nkv * HD * keep * 4);
+  l.w = 256;
+  l.proj = l.w + up((size_t)nkv * HD * keep * 4);
   l.small = l.proj + up((size_t)n * keep * 4);
   l.project = l.small + up((size_t)5 * keep * 4);
   l.bytes = l.project + shard_b200_k_project_workspace_bytes(nkv * HD, keep);
@@ -393,7 +396,7 @@ extern "C" int shard_b200_k_encode(const float* flat, const float* mean, const v
   const KEncodeLayout l = k_encode_layout(nkv, n, keep);
   cudaStream_t st = (cudaStream_t)stream;
   unsigned char* ws = (unsigned char*)workspace;
-  float* w = (float*)ws;
+  float* w = (float*)(ws + l.w);
   float* proj = (float*)(ws + l.proj);
   int32_t* alloc = (int32_t*)(ws + l.small);
   uint32_t* counters = (uint32_t*)alloc + keep;
@@ -402,7 +405,7 @@ extern "C" int shard_b200_k_encode(const float* flat, const float* mean, const v
   if (rc) return rc;
   rc = shard_b200_k_project(flat, mean, w, n, nkv * HD, keep, proj, ws + l.project, l.bytes - l.project, stream);
   if (rc) return rc;
-  kq_init_bits_kernel<<<1, 256, 0, st>>>(counters, keep, bits, alloc);
+  kq_init_bits_kernel<<<1, 256, 0, st>>>(counters, keep, bits, alloc, (const int*)(ws + l.project), (int*)ws);
   launch_kq(proj, alloc, n, keep, counters, coeff_scale, (__half*)coeff_scale_f16_out, packed_out, st);
   if (wprep_out) return shard_b200_decode_prepare(basis_f16_out, coeff_scale_f16_out, mean_f16, nkv, keep, wprep_out, stream);
   SHARD_CHECK_LAUNCH();

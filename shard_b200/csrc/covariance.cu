@@ -393,7 +393,7 @@ extern "C" int shard_b200_k_covariance(const void* k_f16, int64_t head_stride, i
   int* status = (int*)(ws + 4);
   float* sums = (float*)(ws + l.sums);
   float* part = (float*)(ws + l.part);
-  e = cudaMemsetAsync(ws, 0, 16, st);
+  e = cudaMemsetAsync(max_bits, 0, sizeof(*max_bits), st);      // (the status word stays as it is: the caller's to zero)
   if (e != cudaSuccess) return (int)e;
   undo_rope_kernel<true><<<l.rope_blocks, 256, 0, st>>>((const __half*)k_f16, head_stride, tok_stride, nkv, n, l.per_block, pos_start,
                                                         inv_freq, flat_out, sums, max_bits);

@@ -115,7 +115,8 @@ def undo_rope(k, pos_start, inv_freq):
 
 def k_covariance(k, pos_start, inv_freq, flat, mean, mean_f16, gram, workspace=None):
     """`undo_rope` of k (nkv, n, 128) fp16 into flat (n, nkv*128), the column means into mean (fp32) and
-    mean_f16, and (flat - mean)^T (flat - mean) into gram.  Returns the scratch for the next call."""
+    mean_f16, and (flat - mean)^T (flat - mean) into gram.  Returns the scratch for the next call; its
+    `covariance_status` is non-zero once a wait inside a call gave up."""
     require_cuda(k, inv_freq, flat, gram)
     if k.dtype != torch.float16 or k.stride(-1) != 1:
         raise _lib.ShardError("k_covariance expects fp16 keys with a contiguous head dimension")
@@ -126,17 +127,29 @@ def k_covariance(k, pos_start, inv_freq, flat, mean, mean_f16, gram, workspace=N
         raise _lib.ShardError(f"k_covariance supports up to 32 KV heads (got {nkv})")
     if workspace is None or workspace.numel() < wsb:
         workspace = torch.empty(wsb, dtype=torch.uint8, device=k.device)
+        covariance_status(workspace).zero_()
     check(lib.shard_b200_k_covariance(ptr(k), k.stride(0), k.stride(1), nkv, n, int(pos_start), ptr(_c(inv_freq, torch.float32)),
                                       ptr(_c(flat, torch.float32)), ptr(_c(mean, torch.float32)), ptr(_c(mean_f16, torch.float16)),
                                       ptr(_c(gram, torch.float32)), ptr(workspace), wsb, cur_stream()), "k_covariance")
     return workspace
 
 
+def covariance_status(workspace):
+    """The status word (int32 tensor of one element) in the scratch of `k_covariance`."""
+    return workspace[4:8].view(torch.int32)
+
+
+def encode_status(workspace):
+    """The status word (int32 tensor of one element) in the scratch of `k_encode`."""
+    return workspace[:4].view(torch.int32)
+
+
 def k_encode(flat, mean, mean_f16, basis, alloc, workspace=None):
     """Codes of one layer's un-rotated keys: int8 basis, projection, int4 coefficients, and -- when the
     number of kept components is a multiple of 32 -- the decode kernel's weights.  basis (dim, keep) fp32
     rows, alloc: bits per component (host).  Returns (basis_q, scale fp16, basis_f16, packed,
-    coeff_scale fp16, wprep or None, workspace)."""
+    coeff_scale fp16, wprep or None, workspace); the workspace's `encode_status` is non-zero once a wait
+    inside a call gave up."""
     require_cuda(flat, mean, mean_f16, basis)
     n, dim = flat.shape
     keep = basis.shape[1]
@@ -150,6 +163,7 @@ def k_encode(flat, mean, mean_f16, basis, alloc, workspace=None):
         raise _lib.ShardError("k_encode expects fp32 basis rows with contiguous columns")
     if workspace is None or workspace.numel() < wsb:
         workspace = torch.empty(wsb, dtype=torch.uint8, device=dev)
+        encode_status(workspace).zero_()
     basis_q = torch.empty(dim, keep, dtype=torch.int8, device=dev)
     basis_f16 = torch.empty(dim, keep, dtype=torch.float16, device=dev)
     scales = torch.empty(2, keep, dtype=torch.float16, device=dev)

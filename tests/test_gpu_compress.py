@@ -82,3 +82,46 @@ def test_v_hadamard_normalise_views(nkv, n):
     m = y.abs().amax(dim=1)
     assert ((ch.double() - m).abs() <= 1e-6 * m).all()
     assert (x.double() - y / m[:, None, :]).abs().max() < 1e-5
+
+
+@pytest.mark.parametrize("where,nkv", [("k_covariance", 8), ("k_encode", 8), ("k_encode", 2)])
+def test_a_wait_that_gave_up_is_reported(where, nkv, monkeypatch):
+    """The status words of the compressor's kernels end as an error of `compress`, whichever layer raised them."""
+    from shard_b200 import Cache, ops
+    from shard_b200._lib import ShardError
+    real, calls = getattr(ops, where), []
+    word = ops.covariance_status if where == "k_covariance" else ops.encode_status
+
+    def once(*a):
+        r = real(*a)
+        calls.append(1)
+        if len(calls) == 2:                                # the second layer of nine, in the first of two groups
+            word(r if where == "k_covariance" else r[-1]).fill_(1)
+        return r
+
+    monkeypatch.setattr(ops, where, once)
+    cache = Cache(num_layers=9, n_kv_heads=nkv, rope_inv_freq=_inv_freq().cpu())
+    for li in range(9):
+        cache.update(_keys(nkv, 400, li).unsqueeze(0), _keys(nkv, 400, 50 + li).unsqueeze(0), li)
+    with pytest.raises(ShardError, match="gave up"):
+        cache.compress()
+    assert not cache._compressed
+    if where == "k_covariance":                            # nothing was built on that matrix
+        assert all(layer._gpu_compressed is None and layer._keys is not None for layer in cache.layers)
+
+
+def test_status_words_stay_set():
+    """A later call does not clear what an earlier one reported."""
+    from shard_b200 import ops
+    k, p = _keys(8, 300, 1), 1024
+    flat, mean, gram = torch.empty(300, p, device="cuda"), torch.empty(p, device="cuda"), torch.empty(p, p, device="cuda")
+    mean16 = torch.empty(p, dtype=torch.float16, device="cuda")
+    basis = torch.linalg.qr(torch.randn(p, 64, device="cuda"))[0].contiguous()
+    cov = ops.k_covariance(k, 7, _inv_freq(), flat, mean, mean16, gram)
+    enc = ops.k_encode(flat, mean, mean16, basis, [4] * 64)[-1]
+    assert int(ops.covariance_status(cov)) == 0 and int(ops.encode_status(enc)) == 0
+    ops.covariance_status(cov).fill_(1)
+    ops.encode_status(enc).fill_(1)
+    ops.k_covariance(k, 7, _inv_freq(), flat, mean, mean16, gram, cov)
+    ops.k_encode(flat, mean, mean16, basis, [4] * 64, enc)
+    assert int(ops.covariance_status(cov)) == 1 and int(ops.encode_status(enc)) == 1

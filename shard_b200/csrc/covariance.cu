@@ -4,8 +4,9 @@
 //   flat[t][kv*128+d] = undo RoPE(k)      mean = column means      G = (flat - mean)^T (flat - mean)
 //
 // G is the largest dense contraction of the compressor (2 n p^2: 69 GFLOP for a 32K layer; a library
-// fp32 GEMM takes 1.25 ms).  It runs on the tensor cores at fp32 accuracy: the centred, scaled values
-// are split into two fp16 parts (22 bits), three products -- head.head, head.tail, tail.head -- go into
+// fp32 GEMM takes 1.25 ms).  It runs on the tensor cores at fp32 accuracy: the centred values, scaled to
+// the top of fp16's range, are split into two fp16 parts (22 bits for every value within 2^17 of the largest; a
+// scale to [0, 1] would leave the parts of a value 2^10 below it 12 bits), three products -- head.head, head.tail, tail.head -- go into
 // one fp32 accumulator, and because the tensor core adds with truncation the accumulator is added to
 // fp32 registers (round to nearest) every 64 tokens.  Rows are tokens, so both operands are
 // MN-major: a token's 64 dimensions are one 128-byte row of the swizzled operand, no transposition.
@@ -121,13 +122,14 @@ struct GramParams {
   int* status;
 };
 
-// scale that brings |x - mean| (at most twice the largest |x|) into [0, 1]
+// scale that brings |x - mean| (at most twice the largest |x|) below 2^15: a tail then has its full precision
+// unless its value is 2^17 times smaller (fp16's smallest step is 2^-24), and squares stay far from fp32's limit
 __device__ __forceinline__ float gram_scale(const unsigned int* max_bits) {
   const float m = 2.f * __uint_as_float(__ldcg(max_bits));
   if (!(m > 0.f) || isinf(m)) return 1.f;
   int e;
   frexpf(m, &e);
-  return ldexpf(1.f, -e);
+  return ldexpf(1.f, 15 - e);
 }
 // tile number -> blocks (i, j), i <= j, of the upper triangle
 __device__ __forceinline__ void gram_tile(int t, int blocks, int& i, int& j) {

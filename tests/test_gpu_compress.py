@@ -125,3 +125,31 @@ def test_status_words_stay_set():
     ops.k_covariance(k, 7, _inv_freq(), flat, mean, mean16, gram, cov)
     ops.k_encode(flat, mean, mean16, basis, [4] * 64, enc)
     assert int(ops.covariance_status(cov)) == 1 and int(ops.encode_status(enc)) == 1
+
+
+@pytest.mark.parametrize("kind,ratio", [("element", 256.0), ("element", 4096.0), ("channel", 1024.0), ("token", 1024.0), ("small", 1e-4)])
+def test_k_covariance_of_uneven_keys(kind, ratio):
+    """One large element, channel or token beside ordinary ones, or channels far below the others: the matrix
+    stays within a fp32 product's error of float64, relative to each pair of columns."""
+    from shard_b200 import ops
+    n, p = 8192, 1024
+    g = torch.Generator(device="cuda").manual_seed(int(ratio) + len(kind))
+    k = torch.randn(8, n, 128, generator=g, device="cuda")
+    if kind == "element":
+        k[3, 77, 5] = 4 * ratio
+    elif kind == "channel":
+        k[3, :, 5] *= ratio
+    elif kind == "token":
+        k[:, 77] *= ratio
+    else:
+        k[4:, :, ::3] *= ratio
+    k = k.half()
+    flat, mean, gram = torch.empty(n, p, device="cuda"), torch.empty(p, device="cuda"), torch.empty(p, p, device="cuda")
+    # no rotation: the channels stay as uneven as they are
+    ops.k_covariance(k, 0, torch.zeros(64, device="cuda"), flat, mean, torch.empty(p, dtype=torch.float16, device="cuda"), gram)
+    xc = flat.double() - mean.double()
+    norm = xc.norm(dim=0)
+    err = (gram.double() - xc.T @ xc).abs() / (norm[:, None] * norm[None, :])
+    # the tensor core truncates: 12 additions (4 k-steps of 3 products) to one accumulator at 2^-23 of it, all at
+    # the size of the result where one token dominates; the split drops 2^-22 of either factor
+    assert err.max() < 12 * 2.0 ** -23 + 2 * 2.0 ** -22

@@ -41,6 +41,13 @@ EIGH_GROUP = 7
 KMEANS_POINTS = 16 << 20
 
 
+# Bytes of un-rotated fp32 keys (twice the size of a layer's prompt keys) that compression holds from the
+# covariance to the projection, over the two groups of layers in flight.  Where they would be more (7.5 GB for a
+# prompt of 131K tokens) they exist for one layer at a time and are made a second time for its projection: 83 us for
+# a layer of 32K tokens, 1.5 % of its compression.
+ROWS_BYTES = 512 << 20
+
+
 def gram_matrix(flat, mean):
     """(flat - mean)^T (flat - mean) of the rows of `flat` (n, p), fp32."""
     xc = flat - mean
@@ -581,25 +588,28 @@ class Cache(HFCache):
         dev = main.device
         inv_freq = self._inv_freq(dev)
         cov_ws = enc_ws = None
+        in_flight = max(hi - lo for lo, hi in zip(bounds[:-2] or bounds, bounds[2:] or bounds[1:]))
+        keep_rows = 4 * n * p * in_flight <= ROWS_BYTES
+
+        def keys(li):
+            return self.layers[li]._keys[0, :, start:end, :]
 
         def covariances(g):
             nonlocal cov_ws
-            if p <= TORCH_EIGH_MAX:
-                rows, grams = [], []
-                for li in range(bounds[g], bounds[g + 1]):
-                    flat = ops.undo_rope(self.layers[li]._keys[0, :, start:end, :], start, inv_freq)
-                    mean = flat.mean(dim=0)
-                    rows.append((flat, mean, mean.half()))
-                    grams.append(gram_matrix(flat, mean))
-                return rows, torch.stack(grams), main.record_event()
             count = bounds[g + 1] - bounds[g]
-            flat = torch.empty(count, n, p, dtype=torch.float32, device=dev)
+            flat = torch.empty(count if keep_rows else 1, n, p, dtype=torch.float32, device=dev)
             mean = torch.empty(count, p, dtype=torch.float32, device=dev)
             mean_f16 = torch.empty(count, p, dtype=torch.float16, device=dev)
             gram = torch.empty(count, p, p, dtype=torch.float32, device=dev)
-            rows = list(zip(flat.unbind(0), mean.unbind(0), mean_f16.unbind(0)))
+            rows = list(zip(flat.expand(count, n, p).unbind(0), mean.unbind(0), mean_f16.unbind(0)))
             for li, (f, m, m16), gr in zip(range(bounds[g], bounds[g + 1]), rows, gram.unbind(0)):
-                cov_ws = ops.k_covariance(self.layers[li]._keys[0, :, start:end, :], start, inv_freq, f, m, m16, gr, cov_ws)
+                if p <= TORCH_EIGH_MAX:
+                    ops.undo_rope(keys(li), start, inv_freq, out=f)
+                    torch.mean(f, dim=0, out=m)
+                    m16.copy_(m)
+                    gr.copy_(gram_matrix(f, m))
+                else:
+                    cov_ws = ops.k_covariance(keys(li), start, inv_freq, f, m, m16, gr, cov_ws)
             return rows, gram, main.record_event()
 
         ready = covariances(0)
@@ -619,6 +629,8 @@ class Cache(HFCache):
                 fin = side.record_event()
             main.wait_event(fin)
             for i, li in enumerate(range(bounds[g], bounds[g + 1])):
+                if not keep_rows:
+                    ops.undo_rope(keys(li), start, inv_freq, out=rows[i][0])
                 kpart, enc_ws = self._quantise_k(*rows[i], basis[i], eig_host[i].clamp(min=0) / n, enc_ws)
                 self._finish_layer(li, kpart, vparts[i], ends[i], start, end)
         # the second stream's tensors go back to the allocator behind everything enqueued here

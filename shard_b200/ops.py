@@ -100,13 +100,15 @@ def multiquery_attn(q, seq, shape, inv_freq, codebook, compress_start, out, stat
 
 
 # --------------------------------------------------------------------------- prefill compressor
-def undo_rope(k, pos_start, inv_freq):
-    """k: (nkv, n, 128) fp16 view (last dim contiguous) -> (n, nkv*128) fp32 without RoPE."""
+def undo_rope(k, pos_start, inv_freq, out=None):
+    """k: (nkv, n, 128) fp16 view (last dim contiguous) -> (n, nkv*128) fp32 without RoPE, in `out` if given."""
     require_cuda(k, inv_freq)
     if k.dtype != torch.float16 or k.stride(-1) != 1:
         raise _lib.ShardError("undo_rope expects fp16 keys with a contiguous head dimension")
     nkv, n, _ = k.shape
-    flat = torch.empty(n, nkv * HD, dtype=torch.float32, device=k.device)
+    flat = torch.empty(n, nkv * HD, dtype=torch.float32, device=k.device) if out is None else _c(out, torch.float32)
+    if flat.numel() != n * nkv * HD:
+        raise _lib.ShardError("out must hold n * nkv * 128 values")
     check(_lib.load().shard_b200_undo_rope(ptr(k), k.stride(0), k.stride(1), nkv, n, int(pos_start),
                                            ptr(_c(inv_freq, torch.float32)), ptr(flat), cur_stream()),
           "undo_rope")

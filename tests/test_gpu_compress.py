@@ -153,3 +153,41 @@ def test_k_covariance_of_uneven_keys(kind, ratio):
     # the tensor core truncates: 12 additions (4 k-steps of 3 products) to one accumulator at 2^-23 of it, all at
     # the size of the result where one token dominates; the split drops 2^-22 of either factor
     assert err.max() < 12 * 2.0 ** -23 + 2 * 2.0 ** -22
+
+
+@pytest.mark.parametrize("nkv", [8, 4])
+def test_memory_of_compressing_many_layers(nkv):
+    """Peak memory: k-means over as many points as run side by side (fp32 points, their sorted copy, numbers and
+    codes: 40 bytes each), the fp32 rows that may be kept, a few copies of ONE layer's, and the result."""
+    from shard_b200 import Cache
+    from shard_b200.cache import KMEANS_POINTS, ROWS_BYTES
+    layers, n, p = 14, 320000 // nkv, nkv * 128
+    cache = Cache(num_layers=layers, n_kv_heads=nkv, rope_inv_freq=_inv_freq().cpu())
+    for li in range(layers):
+        cache.update(_keys(nkv, n, li).unsqueeze(0), _keys(nkv, n, 50 + li).unsqueeze(0), li)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    cache.compress()
+    extra = torch.cuda.max_memory_allocated() - before
+    result = layers * n * (p // 4 + 192 // 2) + layers * 4 * p * p          # codes; weights and the like
+    assert extra < max(KMEANS_POINTS, n * p // 4) * 40 + ROWS_BYTES + 4 * n * p * 4 + result + (64 << 20)
+
+
+@pytest.mark.parametrize("nkv,layers", [(8, 1), (8, 8), (4, 3), (8, 17)])
+def test_rows_made_twice_give_the_same_cache(nkv, layers, monkeypatch):
+    """The keys' codes do not depend on whether the un-rotated rows were kept or made again."""
+    from shard_b200 import Cache
+    from shard_b200 import cache as mod
+    made = []
+    for budget in (1 << 40, 0):
+        monkeypatch.setattr(mod, "ROWS_BYTES", budget)
+        cache = Cache(num_layers=layers, n_kv_heads=nkv, rope_inv_freq=_inv_freq().cpu())
+        for li in range(layers):
+            cache.update(_keys(nkv, 300, li).unsqueeze(0), _keys(nkv, 300, 50 + li).unsqueeze(0), li)
+        cache.compress()
+        made.append([layer._gpu_compressed for layer in cache.layers])
+    for a, b in zip(*made):
+        for name in ("k_coeffs", "k_coeff_scale", "k_basis_q", "k_basis_scale", "k_mean", "k_wprep"):
+            assert torch.equal(a[name], b[name]), name

@@ -122,6 +122,13 @@ __device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsig
 
 // CB = p / 128 columns per thread; a CTA has RL = p / 16 rows, worked on in chunks of RC rows of 4-row
 // loads (p = 128: one chunk of 8).  Eight warps: a step's scalar work is a chain that more warps would only repeat.
+//
+// One CTA per SM, whatever the registers would allow: a CTA takes all of the SM's tensor memory and then waits for
+// its cluster, so two clusters that shared two SMs, each holding the tensor memory of one, would wait for each other
+// for good.  The launch asks for more shared memory than half an SM has, which keeps every two of these CTAs apart,
+// also those of launches on different streams; CTAs of other kernels wait for tensor memory but nobody waits for them.
+constexpr int EG_RESERVED_SMEM = 116 << 10;
+static_assert(2 * EG_RESERVED_SMEM > (228 << 10), "two CTAs do not fit one SM");
 constexpr int EG_MAIL = 66;                 // float2 per sender in the mailbox: 64 rows + padding against bank conflicts
 
 template <int CB>
@@ -660,11 +667,14 @@ static int launch_eigh(const EighParams& p, int count, cudaStream_t st) {
   if (!configured[dev].load(std::memory_order_acquire)) {
     e = cudaFuncSetAttribute(tridiag_kernel<CB>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return (int)e;
+    e = cudaFuncSetAttribute(tridiag_kernel<CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, EG_RESERVED_SMEM);
+    if (e != cudaSuccess) return (int)e;
     configured[dev].store(true, std::memory_order_release);
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(EG_CL * count);
   cfg.blockDim = dim3(EG_THREADS);
+  cfg.dynamicSmemBytes = EG_RESERVED_SMEM;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -43,3 +43,22 @@ def test_eigh_top_reports_what_it_cannot_do():
     a[0, 3, 3] = float("nan")
     _, _, flag = ops.eigh_top(a, 64)
     assert flag.tolist() == [1, 0]
+
+
+@pytest.mark.parametrize("sizes", [((128, 9), (256, 9)), ((384, 8), (640, 8)), ((1024, 7), (128, 12))])
+def test_launches_on_two_streams(sizes):
+    """More clusters than fit the GPU, of two sizes at once (smaller matrices need fewer registers: without the
+    reserved shared memory their CTAs could share SMs): every result is the one of a launch alone."""
+    from shard_b200 import ops
+    a = [torch.stack([_matrix(p, "decay", s) for s in range(count)]) for p, count in sizes]
+    want = [ops.eigh_top(m, 64) for m in a]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in a]
+    for _ in range(3):
+        got = []
+        for m, st in zip(a, streams):
+            with torch.cuda.stream(st):
+                got.append(ops.eigh_top(m, 64))
+        torch.cuda.synchronize()
+        for w, g in zip(want, got):
+            assert int(g[2].sum()) == 0 and all(torch.equal(x, y) for x, y in zip(w, g))

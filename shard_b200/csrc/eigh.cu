@@ -392,6 +392,11 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
   if (threadIdx.x == 0 && *abort_s) atomicExch(p.flag + m, 1);
   tc_fence_before();
   cluster_sync();                            // nobody is still sending to a CTA that leaves
+  if (*abort_s) {
+    // gave up: what the others had sent by then was not waited for and may still be on its way into this CTA's
+    // shared memory (a microsecond)
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
   if (threadIdx.x < 32) tmem_dealloc(tmem_slot, 512);
 }
 

@@ -178,12 +178,14 @@ __global__ void __launch_bounds__(PJ_THREADS, 1) k_project_tc_kernel(const float
         bulk_g2s(smem_u32(smem + s * stage_bytes + 2 * PJ_A_BYTES), wimg + (size_t)c * b_bytes, b_bytes, FULL(s));
       };
       issue_b(0);
+      int asked = 1;
       for (int c = 0; c < n_chunks && ok; ++c) {
         const int s = c & 1, grp = c / PJ_GROUP, b = grp & 1;
         if (c + 1 < n_chunks) {
           if (c + 1 >= PJ_STAGES) ok = mbar_wait(EMPTY((c + 1) & 1), (uint32_t)((((c + 1) >> 1) - 1) & 1), abort_s);
           if (!ok) break;
           issue_b(c + 1);
+          asked = c + 2;
         }
         const bool first = (c % PJ_GROUP) == 0;
         if (first && grp >= 2) ok = mbar_wait(ACC_FREE(b), (uint32_t)(((grp >> 1) - 1) & 1), abort_s);
@@ -205,7 +207,11 @@ __global__ void __launch_bounds__(PJ_THREADS, 1) k_project_tc_kernel(const float
         umma_commit(EMPTY(s));
         if ((c % PJ_GROUP) == PJ_GROUP - 1 || c == n_chunks - 1) umma_commit(ACC_FULL(b));
       }
-      if (!ok) *abort_s = 1;
+      if (!ok) {
+        // gave up: do not leave while a copy may still be landing in this CTA's shared memory
+        *abort_s = 1;
+        for (int c = max(0, asked - 2); c < asked; ++c) mbar_wait(FULL(c & 1), (uint32_t)((c >> 1) & 1), abort_s);
+      }
     }
     __syncwarp();
   } else {

@@ -1,5 +1,7 @@
 """The native host half of a decode step: same rows and same outputs as the Python path, in both append
 modes, over buffer growth and a restarted reply."""
+import gc
+
 import pytest
 import torch
 
@@ -116,14 +118,18 @@ def test_a_failed_allocation_is_a_python_exception():
         _, _, q = step(t)
         want = fused_attention_compressed(q, layer, 400 + t, cache._rope_inv_freq)
     _, _, q = step(3)
+    gc.collect()
     torch.cuda.empty_cache()
     total = torch.cuda.get_device_properties(0).total_memory
     torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (8 << 20)) / total)
     held = []
     try:
-        with pytest.raises(torch.cuda.OutOfMemoryError):
-            while len(held) < 100000:
-                held.append(torch.empty(32 * 128, dtype=torch.float16, device="cuda"))
+        for size in (1 << 20, 32 * 128, 32 * 128):         # (until nothing is left, whatever earlier work had cached)
+            while len(held) < 200000:
+                try:
+                    held.append(torch.empty(size, dtype=torch.float16, device="cuda"))
+                except torch.cuda.OutOfMemoryError:
+                    break
         with pytest.raises(torch.cuda.OutOfMemoryError):
             fused_attention_compressed(q, layer, 403, cache._rope_inv_freq)
     finally:

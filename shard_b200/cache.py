@@ -614,6 +614,7 @@ class Cache(HFCache):
 
         ready = covariances(0)
         main.wait_event(drawn)
+        init_rows.record_stream(main)
         for g in range(n_groups):
             rows, gram, done = ready
             side.wait_event(done)
@@ -628,6 +629,9 @@ class Cache(HFCache):
                 basis, eig_host = solved.result()
                 fin = side.record_event()
             main.wait_event(fin)
+            # made on the second stream, read on this one: another thread that compresses on the same device shares
+            # the second stream, and its allocations there must not reuse this memory too early
+            basis.record_stream(main)
             for i, li in enumerate(range(bounds[g], bounds[g + 1])):
                 if not keep_rows:
                     ops.undo_rope(keys(li), start, inv_freq, out=rows[i][0])

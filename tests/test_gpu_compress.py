@@ -191,3 +191,44 @@ def test_rows_made_twice_give_the_same_cache(nkv, layers, monkeypatch):
     for a, b in zip(*made):
         for name in ("k_coeffs", "k_coeff_scale", "k_basis_q", "k_basis_scale", "k_mean", "k_wprep"):
             assert torch.equal(a[name], b[name]), name
+
+
+@pytest.mark.parametrize("nkv", [8, 4])
+def test_threads_compress_side_by_side(nkv):
+    """Caches compressed at the same time by threads with streams of their own come out as one after the other."""
+    import threading
+    from shard_b200 import Cache
+    names = ("k_coeffs", "k_coeff_scale", "k_basis_q", "k_basis_scale", "k_mean", "k_wprep", "v_indices_u8", "v_centroids_f16", "sink_k", "win_v")
+    prompts = [[(_keys(nkv, 600 + 128 * c, 10 * c + li).unsqueeze(0), _keys(nkv, 600 + 128 * c, 50 + 10 * c + li).unsqueeze(0))
+                for li in range(9)] for c in range(4)]
+    torch.cuda.synchronize()
+
+    def compressed(c):
+        cache = Cache(num_layers=9, n_kv_heads=nkv, rope_inv_freq=_inv_freq().cpu())
+        for li, (k, v) in enumerate(prompts[c]):
+            cache.update(k, v, li)
+        cache.compress()
+        return [{n: layer._gpu_compressed[n].clone() for n in names} for layer in cache.layers]
+
+    want = [compressed(c) for c in range(4)]
+    got, errors = [None] * 4, []
+
+    def work(c):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(4):
+                    got[c] = compressed(c)
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:                             # (raised in the test's own thread below)
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for a, b in zip(want, got):
+        for x, y in zip(a, b):
+            for n in names:
+                assert torch.equal(x[n], y[n]), n

@@ -439,7 +439,7 @@ class CacheLayer(CacheLayerMixin):
         if "signs" not in gc or s + new > gc["k_idx_buf"].shape[0]:
             self._grow_stream(gc, k, s + new)
         if defer:
-            gc["_pending"] = (k.contiguous(), v.contiguous(), s)
+            gc["_pending"] = (ops.packed_token(k), ops.packed_token(v), s)
         else:
             ops.stream_quantize_rows(k[0], v[0], gc["signs"], get_codebook(k.shape[3], 8, k.device),
                                      gc["k_idx_buf"], gc["v_idx_buf"], gc["k_norm_buf"], gc["v_norm_buf"], s)

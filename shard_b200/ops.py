@@ -25,6 +25,18 @@ def _c(t, dtype=None):
     return t
 
 
+def _readable_rows(t):
+    """(heads, s, 128) fp16 whose rows the kernels can read 8 bytes at a time: `t`, or a copy."""
+    if t.stride(2) != 1 or (t.stride(0) | t.stride(1)) & 3 or t.data_ptr() & 7:
+        return t.clone(memory_format=torch.contiguous_format)      # (contiguous() would keep a misaligned start)
+    return t
+
+
+def packed_token(t):
+    """(1, heads, 1, 128) as [heads][128] on an 8-byte boundary: `t`, or a copy."""
+    return t.clone(memory_format=torch.contiguous_format) if not t.is_contiguous() or t.data_ptr() & 7 else t
+
+
 # --------------------------------------------------------------------------- stream quantizer
 def stream_quantize(new_k, new_v, signs, codebook, k_idx_buf, v_idx_buf, k_norm_buf, v_norm_buf, slot):
     """Append one token (nkv, 128) fp16 K/V as 8-bit codes + fp16 norms at row `slot`."""
@@ -49,10 +61,7 @@ def stream_quantize_rows(k, v, signs, codebook, k_idx_buf, v_idx_buf, k_norm_buf
     nkv, s, _ = k.shape
     if k.dtype != torch.float16 or v.dtype != torch.float16:
         raise _lib.ShardError("expected torch.float16 keys and values")
-    if k.stride(2) != 1 or (k.stride(0) | k.stride(1)) & 3 or k.data_ptr() & 7:
-        k = k.contiguous()
-    if v.stride(2) != 1 or (v.stride(0) | v.stride(1)) & 3 or v.data_ptr() & 7:
-        v = v.contiguous()
+    k, v = _readable_rows(k), _readable_rows(v)
     if slot + s > k_idx_buf.shape[0]:
         raise _lib.ShardError("stream buffer full")
     check(_lib.load().shard_b200_stream_quantize_rows(
@@ -86,8 +95,7 @@ def multiquery_attn(q, seq, shape, inv_freq, codebook, compress_start, out, stat
     (s, n_q, 128).  `seq` / `shape` as for `read_back`; the s tokens are the last of the stream or of the
     decode buffer."""
     require_cuda(q, out, inv_freq)
-    if q.stride(2) != 1 or (q.stride(0) | q.stride(1)) & 3 or q.data_ptr() & 7:
-        q = q.contiguous()
+    q = _readable_rows(q)
     s = q.shape[1]
     lib = _lib.load()
     wsb = lib.shard_b200_multiquery_workspace_bytes(C.byref(shape), s)

@@ -208,3 +208,30 @@ def test_tokens_that_do_not_fit_the_cache_are_refused(streaming, s):
     assert layer.get_seq_length() == n
     layer._needs_decompress = True
     assert torch.equal(layer.keys, want)
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("s", [1, 2, 5])
+def test_tensors_that_start_between_8_byte_boundaries(streaming, s):
+    """Views that start one element into a buffer: same rows, same attention."""
+    from shard_b200 import fused_attention_compressed
+    caches = [_cache(random_gc(300, nkv=2, seed=1), 2, streaming, capacity=16) for _ in range(2)]
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def shifted(t):
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+        buf[1:].copy_(t.reshape(-1))
+        return buf[1:].view(t.shape)
+
+    for step in range(3):
+        k, v = (torch.randn(1, 2, s, 128, generator=g, device="cuda").half() for _ in range(2))
+        q = torch.randn(1, 8, s, 128, generator=g, device="cuda").half()
+        outs = []
+        for (cache, layer), f in zip(caches, (lambda t: t, shifted)):
+            cache._fused_decode_update = True
+            layer.update(f(k), f(v))
+            outs.append(fused_attention_compressed(f(q), layer, layer.get_seq_length() - 1, cache._rope_inv_freq))
+            cache._fused_decode_update = False
+            if step == 2:
+                outs.append(layer.update(f(k), f(v))[0])
+        assert all(torch.equal(a, b) for a, b in zip(outs[:len(outs) // 2], outs[len(outs) // 2:]))

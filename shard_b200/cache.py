@@ -254,9 +254,8 @@ class CacheLayer(CacheLayerMixin):
         nkv, hd = c._n_kv_heads, c.head_dim
         dev = gc["k_coeffs"].device
         _lib.require_cuda(gc["k_coeffs"])
-        pend = gc.pop("_pending", None)
+        pend = gc.get("_pending")
         if pend is not None and pend[2] != gc.get("stream_n", 0) - 1:
-            gc["_pending"] = pend
             self._flush_pending()
             pend = None
         seq, shape, rows = layer_record(gc, nkv, hd, dev)
@@ -268,6 +267,7 @@ class CacheLayer(CacheLayerMixin):
         values = torch.empty_like(keys)
         ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
                       gc["compress_start"], keys, values, status_word(c, dev))
+        gc.pop("_pending", None)                           # (only now: the launch has it)
         self._keys, self._values = keys, values
         self._needs_decompress = False
 

@@ -85,3 +85,27 @@ def test_read_back(n_comp, rank, nkv, n_new, streaming):
     # fp16 output, weights rounded to fp16 once
     assert np.abs(gk - k64).max() <= 2e-3 * np.abs(k64).max() and np.linalg.norm(gk - k64) <= 6e-4 * np.linalg.norm(k64)
     assert (np.abs(gv - v64) <= 1e-5 + 6e-4 * np.abs(v64)).all()
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+def test_a_token_survives_a_read_back_that_failed(streaming, monkeypatch):
+    """The newest token is not lost when the launch that would have written it cannot be made."""
+    from shard_b200 import ops
+    from shard_b200._lib import ShardError
+    caches = [_cache(random_gc(300, nkv=2, seed=1), 2, streaming) for _ in range(2)]
+    k, v = (torch.randn(1, 2, 3, 128, device="cuda").half() for _ in range(2))
+
+    def fail(*a):
+        raise ShardError("no")
+
+    for i, (cache, layer) in enumerate(caches):
+        layer.update(k[:, :, :1], v[:, :, :1])
+        if i == 0:
+            with monkeypatch.context() as m:
+                m.setattr(ops, "read_back", fail)
+                with pytest.raises(ShardError):
+                    layer.update(k[:, :, 1:2], v[:, :, 1:2])
+        else:
+            layer.update(k[:, :, 1:2], v[:, :, 1:2])
+    (_, a), (_, b) = caches
+    assert torch.equal(a.keys, b.keys) and torch.equal(a.values, b.values)

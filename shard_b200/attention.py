@@ -92,10 +92,11 @@ def row_tensors(gc, nkv, hd):
     return dk, dv, n_dec, dk.stride(1) // hd if nkv > 1 else n_dec
 
 
-def layer_record(gc, nkv, hd, dev):
-    """ShardSeq, ShardDecodeShape and number of rows of a whole layer: what reads all of it takes."""
+def layer_record(gc, nkv, hd, dev, with_rows=True):
+    """ShardSeq, ShardDecodeShape and number of rows of a whole layer (without the decoded fp16 tokens if
+    not `with_rows`): what reads all of it takes."""
     seq = _seq_record(gc, dev)
-    dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd)
+    dk, dv, n_dec, dec_cap = row_tensors(gc, nkv, hd) if with_rows else (None, None, 0, 0)
     n_comp, n_stream = gc["n_compress"], gc.get("stream_n", 0)
     n_sink, n_win = gc["sink_k"].shape[2], gc["win_k"].shape[2]
     shape = ops.make_shape(GQA * nkv, nkv, gc["k_rank_kernel"], n_comp, 0, n_comp, n_sink, n_win, n_stream, 0, n_dec=n_dec)

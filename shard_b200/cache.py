@@ -253,21 +253,32 @@ class CacheLayer(CacheLayerMixin):
         c = self._cache_ref
         nkv, hd = c._n_kv_heads, c.head_dim
         dev = gc["k_coeffs"].device
+        if dev.type == "cuda" and dev.index != torch.cuda.current_device():
+            with torch.cuda.device(dev):
+                return self._ensure_dequant(new)
         _lib.require_cuda(gc["k_coeffs"])
+        if "k_wprep" not in gc:                            # a dictionary in the reference's form
+            attach_kernel_format(gc, nkv)
         pend = gc.get("_pending")
         if pend is not None and pend[2] != gc.get("stream_n", 0) - 1:
             self._flush_pending()
             pend = None
-        seq, shape, rows = layer_record(gc, nkv, hd, dev)
+        # decoded tokens of another dtype are not the kernel's: they are appended to what it returns
+        other = "decode_k" in gc and not (gc["decode_k"].dtype == gc["decode_v"].dtype == torch.float16)
+        seq, shape, rows = layer_record(gc, nkv, hd, dev, with_rows=not other)
         if pend is not None or new is not None:
             shape.append = 1 if pend is not None else 2
             new = pend if pend is not None else new
             seq.new_k, seq.new_v = new[0].data_ptr(), new[1].data_ptr()
         keys = torch.empty(1, nkv, rows, hd, dtype=torch.float16, device=dev)
         values = torch.empty_like(keys)
-        ops.read_back(seq, shape, c._inv_freq(dev), get_codebook(hd, 8, dev) if shape.n_stream else None,
+        # (no RoPE is a rotation by nothing)
+        inv_freq = c._inv_freq(dev) if c._rope_inv_freq is not None else torch.zeros(hd // 2, device=dev)
+        ops.read_back(seq, shape, inv_freq, get_codebook(hd, 8, dev) if shape.n_stream else None,
                       gc["compress_start"], keys, values, status_word(c, dev))
         gc.pop("_pending", None)                           # (only now: the launch has it)
+        if other:
+            keys, values = torch.cat([keys, gc["decode_k"]], dim=2), torch.cat([values, gc["decode_v"]], dim=2)
         self._keys, self._values = keys, values
         self._needs_decompress = False
 

@@ -87,6 +87,29 @@ def test_read_back(n_comp, rank, nkv, n_new, streaming):
     assert (np.abs(gv - v64) <= 1e-5 + 6e-4 * np.abs(v64)).all()
 
 
+def test_read_back_of_tokens_in_another_dtype():
+    """A reply whose tokens are not fp16 (the model's type changed after compression): they are kept and read
+    back as they are, behind the layer's own."""
+    cache, layer = _cache(random_gc(300, nkv=2, seed=1), 2, False)
+    want = layer.keys.clone(), layer.values.clone()
+    k, v = (torch.randn(1, 2, 3, 128, device="cuda") for _ in range(2))
+    layer.update(k[:, :, :2], v[:, :, :2])
+    keys, values = layer.update(k[:, :, 2:], v[:, :, 2:])
+    for got, old, new in ((keys, want[0], k), (values, want[1], v)):
+        assert got.dtype == torch.float32 and torch.equal(got, torch.cat([old, new], 2))
+
+
+def test_read_back_of_a_dictionary_without_kernel_tensors():
+    """The reference's tensors are enough to read a layer back."""
+    cache, layer = _cache(random_gc(300, rank=150, nkv=2, seed=1), 2, True)
+    gc = layer._gpu_compressed
+    want = layer.keys.clone(), layer.values.clone()
+    for name in ("k_wprep", "k_coeffs_kernel", "k_coeffs_padded", "k_rank_kernel", "_fresh", "_seq"):
+        gc.pop(name, None)
+    layer._needs_decompress = True
+    assert torch.equal(layer.keys, want[0]) and torch.equal(layer.values, want[1])
+
+
 @pytest.mark.parametrize("streaming", [True, False])
 def test_a_token_survives_a_read_back_that_failed(streaming, monkeypatch):
     """The newest token is not lost when the launch that would have written it cannot be made."""

@@ -518,6 +518,10 @@ class Cache(HFCache):
         self._phase_key = None
         self._inv_freq_dev = None
         self.compress_seconds = None
+        try:
+            _lib.host()                                    # loaded here and not inside the first decode step (1.2 ms)
+        except ShardError:
+            pass                                           # (the first call that needs it says what is missing)
         super().__init__(layers=[CacheLayer(i) for i in range(num_layers)])
         for layer in self.layers:
             layer._cache_ref = self

@@ -341,6 +341,8 @@ class CacheLayer(CacheLayerMixin):
             self._seq_len += seq_new
             self._needs_decompress = True
             if fused:
+                if self._keys is not None:                 # an earlier read-back, out of date by now: a layer's fp16
+                    self._keys = self._values = None       # keys and values need not be held through the reply
                 c._last_accessed_layer = self.layer_idx
                 return key_states, value_states
             try:

@@ -132,3 +132,23 @@ def test_a_token_survives_a_read_back_that_failed(streaming, monkeypatch):
             layer.update(k[:, :, 1:2], v[:, :, 1:2])
     (_, a), (_, b) = caches
     assert torch.equal(a.keys, b.keys) and torch.equal(a.values, b.values)
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+def test_fused_steps_do_not_hold_read_back_layers(streaming):
+    """A reply that goes on with the fused kernel keeps no fp16 copy of a layer from an earlier read-back."""
+    from gpu_helpers import gc_to_device
+    from shard_b200 import Cache
+    cache = Cache(num_layers=3, n_kv_heads=2, rope_inv_freq=torch.ones(64))
+    cache._streaming, cache._compressed = streaming, True
+    k, v = (torch.randn(1, 2, 1, 128, device="cuda").half() for _ in range(2))
+    for layer in cache.layers:
+        layer._gpu_compressed = gc_to_device(random_gc(300, nkv=2, seed=1), nkv=2)
+        layer._prefilled = layer._needs_decompress = True
+        layer._seq_len = 368
+    for fused in (False, True):
+        cache._fused_decode_update = fused
+        for layer in cache.layers:
+            layer.update(k, v)
+    assert all(layer._keys is None and layer._values is None for layer in cache.layers)
+    assert cache.layers[2].keys.shape[2] == 370

@@ -18,9 +18,14 @@ from ._lib import ShardSeq, ptr
 from .streaming import get_codebook
 
 GQA = 4
-# from this many new tokens on, one read-back of the layer serves all of them; below, a decode launch per
-# query token is cheaper
+# From this many new tokens on, one read-back of the layer serves all of them; below, a decode launch per
+# query token is taken.  Three tokens, us a layer (read-back and attention / three decode launches, several layers
+# sharing their phase tables): 8 KV heads 32 / 84 at 2K tokens of context, 42 / 84 at 8K, 112 / 120 at 32K,
+# 198 / 194 at 64K, 337 / 332 at 128K; 4 heads 72 / 89, 127 / 127, 211 / 201 from 32K on; 2 heads 57 / 83, 91 / 100,
+# 151 / 139.  Four tokens: the read-back at every context (8 heads 335 / 440 at 128K).
 MIN_MULTIQUERY_TOKENS = 3
+# Three tokens take their own launches where the layer's middle is longer than this.
+THREE_TOKENS_MAX_MIDDLE = 49152
 # a forward over more new tokens than this after compression takes the dequantised path
 MAX_FUSED_QUERY_TOKENS = 256
 
@@ -282,7 +287,7 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
     cache (src/shard/attention.py:357-362, src/shard/cache.py:87-124) -- `pos_q` is the position
     of the LAST query; query j attends to everything before the s new tokens plus the first j + 1
     of them (causal).  The new tokens must already have been appended (`update`).  Two query tokens
-    are two decode launches; more share one read-back of the layer into tensor-core tiles, over which
+    are two decode launches, three over a very long context three; more share one read-back of the layer into tensor-core tiles, over which
     they attend as the rows of dense products.
 
     `attn_mask` is accepted for signature compatibility: for one sequence without padding the
@@ -306,7 +311,7 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
         raise _lib.ShardError("append the new tokens (update) before attending with them")
     res = torch.empty(s_q, n_q, hd, dtype=torch.float16, device=q_rope.device)
     nkv = cache._n_kv_heads
-    if (s_q >= MIN_MULTIQUERY_TOKENS and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
+    if (s_q >= MIN_MULTIQUERY_TOKENS and (s_q > 3 or gc["n_compress"] <= THREE_TOKENS_MAX_MIDDLE) and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
             and not (gc.get("stream_n", 0) and "decode_k" in gc)):
         # all query tokens over one read-back of the layer
         dev = q_rope.device

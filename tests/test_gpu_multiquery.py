@@ -50,3 +50,8 @@ def test_queries_of_two_sequences_are_refused(s):
     q = torch.randn(2, 8, s, 128, device="cuda").half()
     with pytest.raises(NotImplementedError):
         fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)
+
+
+@pytest.mark.parametrize("n_comp", [49152, 49153])
+def test_three_tokens_either_side_of_the_rule(n_comp):
+    test_multiquery(n_comp, 192, 1, 3, 3, True)

@@ -6,19 +6,23 @@
 // the M dimension of dense products, instead of one reconstruction of all keys per query token.
 //
 //   CTA = (share of the tiles, 128 query rows, KV head), 5 warps:
-//     warps 0-3   thread = query row: scores (tensor memory) -> online softmax -> fp16 weights, written
-//                 over the scores; the accumulator is rescaled only when a row's reference point moves
-//                 by more than 2^8
+//     warps 0-3   thread = query row: scores (tensor memory) -> online softmax -> weights, written over the
+//                 scores as two fp16 parts (22 bits); the accumulator is rescaled only when a row's
+//                 reference point moves by more than 2^8
 //     warp 4      bulk copies of the tile images (two stages each) and all MMAs: S = Q K^T for the next
-//                 tile while the softmax works on this one, then O += P V with P from tensor memory
+//                 tile while the softmax works on this one, then O += P V with P's parts from tensor memory
+//
+// Weights of 11 bits would leave the output further from float64 than the decode launch's, which attends to
+// the rows outside the middle in fp32 and has exact fp16 values in the middle: up to 25 % where decoded tokens carry
+// the attention (2-norm 2.9e-4 against 2.3e-4; 2.2e-4 with both parts), 5 % with two KV heads.
 //
 // Shares are merged by multiquery_merge_kernel (their partial rows are fp32; a single share writes the
 // result itself).
 //
 // Bound: the exponentials (16 per SM and cycle: 1 K cycles a tile) and the tensor work (1 K cycles a
 // tile) are about equal and overlap only partly, one softmax group per CTA; the images' 64 KB per tile
-// and KV head come from L2.  48 new tokens over 8K, 8 KV heads: 26 us a layer, and 26 us for the read-back
-// in front of it (one decode launch per query token: 1 600 us a layer).
+// and KV head come from L2.  48 new tokens over 8K, 8 KV heads: 30 us a layer (26 with weights of 11 bits), and
+// 26 us for the read-back in front of it (one decode launch per query token: 1 600 us a layer).
 #include <atomic>
 
 #include "decode_common.cuh"
@@ -152,6 +156,9 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) multiquery_kernel(const __grid_
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
           umma_ts(tmem_base + MQ_COL_O, tmem_base + 128 * b + 8 * ks, vd + (uint64_t)((ks * 2048) >> 4), IDESC_O, (t > 0 || ks > 0) ? 1u : 0u, 1u);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)                          // the weights' tails
+          umma_ts(tmem_base + MQ_COL_O, tmem_base + 128 * b + 64 + 8 * ks, vd + (uint64_t)((ks * 2048) >> 4), IDESC_O, 1u, 1u);
         umma_commit(O_DONE(b), 1u);
       }
       if (!ok) {
@@ -198,12 +205,22 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) multiquery_kernel(const __grid_
       }
       const float ref = m == neg_inf() ? 0.f : m;                // (nothing visible yet: weights are exp2(-inf) = 0)
       float sum[2] = {0.f, 0.f};
+      // (in registers since tmem_wait_ld: the stage's columns may be overwritten, heads 0..63, tails 64..127)
 #pragma unroll
-      for (int c = 0; c < 128; c += 2) {
-        const float a = exp2f(fmaf(__uint_as_float(sc[c]), K, -ref)), d = exp2f(fmaf(__uint_as_float(sc[c + 1]), K, -ref));
-        sum[0] += a;
-        sum[1] += d;
-        sc[c >> 1] = pack_half2(a, d);
+      for (int q = 0; q < 4; ++q) {
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          const float a = exp2f(fmaf(__uint_as_float(sc[32 * q + 2 * e]), K, -ref)), d = exp2f(fmaf(__uint_as_float(sc[32 * q + 2 * e + 1]), K, -ref));
+          sum[0] += a;
+          sum[1] += d;
+          const __half2 h = __floats2half2_rn(a, d);
+          const float2 f = __half22float2(h);
+          hi[e] = as_u32(h);
+          lo[e] = pack_half2(a - f.x, d - f.y);
+        }
+        tmem_st_x16(S + 16 * q, hi);
+        tmem_st_x16(S + 64 + 16 * q, lo);
       }
       l = l * alpha + (sum[0] + sum[1]);
       if (t > 0) {
@@ -224,8 +241,6 @@ __global__ void __launch_bounds__(MQ_THREADS, 1) multiquery_kernel(const __grid_
           }
         }
       }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_st_x16(S + 16 * c, *reinterpret_cast<uint32_t(*)[16]>(&sc[16 * c]));
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();

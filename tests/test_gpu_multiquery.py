@@ -55,3 +55,25 @@ def test_queries_of_two_sequences_are_refused(s):
 @pytest.mark.parametrize("n_comp", [49152, 49153])
 def test_three_tokens_either_side_of_the_rule(n_comp):
     test_multiquery(n_comp, 192, 1, 3, 3, True)
+
+
+@pytest.mark.parametrize("nkv,rows,s", [(4, 1400, 20), (8, 300, 3), (1, 77, 33)])
+def test_rows_outside_the_middle_are_weighed_in_full(nkv, rows, s):
+    """Where the decoded tokens carry the attention the output is float64's, rounded to fp16: their weights
+    have 22 bits, so nothing but the rounding of the output (and a tenth of it) is left."""
+    from shard_b200 import fused_attention_compressed
+    gc_np = random_gc(1, nkv=nkv, seed=s)
+    cache, layer = _cache(gc_np, nkv, False, capacity=rows + s)
+    g = torch.Generator(device="cuda").manual_seed(s)
+    k, v = (torch.randn(1, nkv, rows + s, 128, generator=g, device="cuda").half() for _ in range(2))
+    q = torch.randn(1, 4 * nkv, s, 128, generator=g, device="cuda").half()
+    cache._fused_decode_update = True
+    layer.update(k, v)
+    out = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)[0].double()
+    layer._needs_decompress = True
+    keys, values = layer.keys[0].double(), layer.values[0].double()
+    n = keys.shape[1]
+    sc = torch.einsum("hqd,hnd->hqn", q[0].double(), keys.repeat_interleave(4, 0)) / 128 ** 0.5
+    hidden = torch.arange(n, device="cuda")[None, :] > n - s + torch.arange(s, device="cuda")[:, None]
+    want = torch.softmax(sc.masked_fill(hidden, float("-inf")), -1) @ values.repeat_interleave(4, 0)
+    assert (out - want).norm() <= 1.1 * (want.half().double() - want).norm()

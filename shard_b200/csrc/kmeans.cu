@@ -13,6 +13,9 @@
 //   30 at 2 M) go through the same test with each tile's own box, and the few left (5, 10) are evaluated
 //   for the points.
 //
+// A point that is not finite is at no distance below infinity from anything, so it belongs to centroid 0 like a
+// first minimum: its infinities and NaN go into that centroid beside the fixed-point sums (`odd`).
+//
 // A centroid is dropped only if it is farther by more than the rounding of both sides can hide
 // (KM_SLACK), so the assignment is the exact one.
 //
@@ -45,6 +48,7 @@ struct KmeansHeader {      // head of the workspace; zero when the first iterati
   int ticket;              // CTAs that have finished the current iteration
   unsigned int max_bits;   // max |x| (as float bits) if the caller did not name a bound
   unsigned int next_run;   // runs handed out in the current iteration
+  unsigned int odd;        // three bits per channel: some point has +inf, -inf, NaN there
   long long sums[256 * 4]; // fixed point
   int counts[256];
 };
@@ -174,7 +178,10 @@ __global__ void __launch_bounds__(256) kmeans_max_abs_kernel(const __grid_consta
   float m = 0.f;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (long long)gridDim.x * blockDim.x) {
     const float4 v = p.x[i];
-    m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (isfinite(f[j])) m = fmaxf(m, fabsf(f[j]));
   }
   m = warp_max(m);
   if ((threadIdx.x & 31) == 0) atomicMax(&p.h->max_bits, __float_as_uint(m));
@@ -192,6 +199,13 @@ __global__ void __launch_bounds__(256) kmeans_sort_kernel(const __grid_constant_
     const bool live = i < p.n;
     const float4 v = live ? p.x[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     const unsigned int key = live ? km_cell(v, scale, p.bits) : 0xffffffffu;
+    if (!SCATTER && live && !isfinite((v.x - v.x) + (v.y - v.y) + (v.z - v.z) + (v.w - v.w))) {
+      const float f[4] = {v.x, v.y, v.z, v.w};
+      unsigned int bits = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) bits |= (isnan(f[j]) ? 4u : isinf(f[j]) ? (f[j] > 0.f ? 1u : 2u) : 0u) << (3 * j);
+      atomicOr(&p.h->odd, bits);
+    }
     const bool one = __all_sync(0xffffffffu, key == __shfl_sync(0xffffffffu, key, 0));
     unsigned int pos = 0;
     if (one) {
@@ -501,7 +515,7 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
   if (!last_s) return;
   // ---- the last CTA: centroids = means of their points (empty clusters stay), largest move ----------
   __threadfence();
-  float moved = 0.f;
+  bool settled = true;
   if (tid < 256) {
     const int cnt = __ldcg(&p.h->counts[tid]);
     if (cnt > 0) {
@@ -510,11 +524,19 @@ __global__ void __launch_bounds__(KM_THREADS, 2) kmeans_iteration_kernel(const _
       const double unit = (double)cnt * (double)qscale;
 #pragma unroll
       for (int j = 0; j < 4; ++j) nv[j] = (float)((double)__ldcg(&p.h->sums[4 * tid + j]) / unit);
+      if (tid == 0) {
+        const unsigned int odd = __ldcg(&p.h->odd);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const unsigned int o = (odd >> (3 * j)) & 7u;
+          if (o) nv[j] = o == 1u ? __int_as_float(0x7f800000) : o == 2u ? neg_inf() : __int_as_float(0x7fffffff);
+        }
+      }
       p.centroids[tid] = make_float4(nv[0], nv[1], nv[2], nv[3]);
-      moved = fmaxf(fmaxf(fabsf(nv[0] - c.x), fabsf(nv[1] - c.y)), fmaxf(fabsf(nv[2] - c.z), fabsf(nv[3] - c.w)));
+      settled = fabsf(nv[0] - c.x) < 1e-4f && fabsf(nv[1] - c.y) < 1e-4f && fabsf(nv[2] - c.z) < 1e-4f && fabsf(nv[3] - c.w) < 1e-4f;
     }
   }
-  const int still = __syncthreads_or(tid < 256 && !(moved < 1e-4f));
+  const int still = __syncthreads_or(!settled);
   if (tid == 0 && !still && p.it >= 5) p.h->done = 1;
 }
 

@@ -64,3 +64,27 @@ def test_kmeans_sets_side_by_side():
     for i in range(3):
         alone = cent[i].clone()
         assert torch.equal(idx[i], ops.kmeans_lloyd(x[i], alone, 8, 4.0)) and torch.equal(alone, together[i])
+
+
+@pytest.mark.parametrize("max_abs", [0.0, 4.0])
+@pytest.mark.parametrize("odd", [{7: float("inf")}, {7: float("nan"), 9000: float("-inf")}, {0: float("inf"), 63: float("-inf"), 64: float("nan")}])
+def test_kmeans_of_points_that_are_not_finite(odd, max_abs):
+    """They go to centroid 0 and take it with them, channel by channel; the others are clustered as ever."""
+    from shard_b200 import ops
+    x = _data(20000, "plain")
+    for j, (i, v) in enumerate(odd.items()):
+        x[i, (j + 1) % 4] = v
+        x[i, (j + 3) % 4] *= 0.5
+    cent = x[torch.arange(256, device="cuda") * 78 + 1].clone()
+    cent[0] = 0.01
+    c = cent.clone()
+    idx = ops.kmeans_lloyd(x, c, 9, max_abs)
+    want, u8 = cent.clone(), None
+    for it in range(9):
+        u8, _ = ops.vq_assign(x, want, want_i64=False)
+        counts = torch.bincount(u8.long(), minlength=256)
+        sums = torch.zeros(256, 4, dtype=torch.float64, device="cuda").index_add_(0, u8.long(), x.double())
+        want = torch.where(counts[:, None] > 0, sums / counts[:, None], want.double()).float()
+    assert torch.equal(idx, u8) and all(int(idx[i]) == 0 for i in odd)
+    assert torch.equal(torch.isfinite(c), torch.isfinite(want)) and not torch.isfinite(c[0]).all()
+    assert torch.allclose(c, want, rtol=0, atol=2e-6, equal_nan=True)

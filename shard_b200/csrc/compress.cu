@@ -7,6 +7,7 @@
 // PyTorch code performs them, so that the codes are bit-identical for identical
 // fp32 inputs.  Reductions that decide codes (min, max, max-abs) are
 // order-independent.
+#include <new>
 #include <vector>
 
 #include "common.cuh"
@@ -424,13 +425,23 @@ extern "C" int shard_b200_k_basis_quantise(const float* basis, int64_t row_strid
 // Host: the dynamic programme of dp_bit_allocation in double precision, first minimum wins.
 extern "C" int shard_b200_dp_bit_allocation(const double* group_var_host, const int32_t* group_size_host, int32_t n_groups,
                                             int32_t total_budget, int32_t* group_bits_host) {
-  constexpr int MAX_GROUPS = 64, UNIT = 16;
+  constexpr int UNIT = 16;
   static const int choices[5] = {0, 2, 4, 6, 8};
-  if (!group_var_host || !group_size_host || !group_bits_host || n_groups < 1 || n_groups > MAX_GROUPS || total_budget < 0) return SHARD_E_ARG;
-  const int cap = total_budget / UNIT + 1;
+  if (!group_var_host || !group_size_host || !group_bits_host || n_groups < 1 || total_budget < -UNIT) return SHARD_E_ARG;
+  // (a budget beyond what eight bits for everything cost changes nothing, but would be a table of that length)
+  long long most = 0;
+  for (int g = 0; g < n_groups; ++g) most += ((long long)group_size_host[g] * 8 + UNIT - 1) / UNIT;
+  const long long asked = (total_budget < 0 ? -1 : total_budget / UNIT) + 1;
+  const int cap = (int)(asked < most ? asked : most);
   const double inf = 1.0 / 0.0;
-  std::vector<double> best((size_t)(n_groups + 1) * (cap + 1), inf);
-  std::vector<int> pick((size_t)(n_groups + 1) * (cap + 1), 0);
+  std::vector<double> best;
+  std::vector<int> pick;
+  try {
+    best.assign((size_t)(n_groups + 1) * (cap + 1), inf);
+    pick.assign((size_t)(n_groups + 1) * (cap + 1), 0);
+  } catch (const std::bad_alloc&) {
+    return SHARD_E_TOO_LARGE;
+  }
   for (int b = 0; b <= cap; ++b) best[b] = 0.0;
   auto cost_of = [&](int g, int bits) { return bits == 0 ? 0 : (group_size_host[g] * bits + UNIT - 1) / UNIT; };
   for (int g = 0; g < n_groups; ++g) {

@@ -8,6 +8,7 @@ torch expressions of the non-fused read path.
 from __future__ import annotations
 
 import ctypes as C
+from operator import index
 
 import torch
 
@@ -65,18 +66,20 @@ _GROUP = 64                 # components share a bit width in groups of 64
 def dp_bit_allocation(variances, total_budget):
     """Bits per PCA component by dynamic programming (reference: rope.py:49-84).
 
-    The programme itself runs in the library (host code).  Minimises sum_g err(g, bits_g) subject to sum_g ceil(size_g * bits_g / 16)
-    <= total_budget // 16 + 1, with err = 4 * var for 0 bits and
+    The programme itself runs in the library (host code).  Minimises sum_g err(g, bits_g) subject to
+    sum_g ceil(size_g * bits_g / 16) <= total_budget // 16 + 1, with err = 4 * var for 0 bits and
     var / (3 * 4**bits) otherwise.  Ties keep the first (smallest) option.
     """
     v = variances.float().cpu()
     d = int(v.shape[0])
     n_groups = (d + _GROUP - 1) // _GROUP
     sizes = [min(_GROUP, d - g * _GROUP) for g in range(n_groups)]
+    if n_groups == 0:
+        return []
     gvar = [v[g * _GROUP: g * _GROUP + sizes[g]].sum().item() for g in range(n_groups)]
     bits = (C.c_int32 * n_groups)()
     _lib.check(_lib.load().shard_b200_dp_bit_allocation((C.c_double * n_groups)(*gvar), (C.c_int32 * n_groups)(*sizes), n_groups,
-                                                        total_budget, bits), "dp_bit_allocation")
+                                                        min(index(total_budget), 16 * d), bits), "dp_bit_allocation")
     alloc = []
     for g in range(n_groups):
         alloc += [bits[g]] * sizes[g]

@@ -2,6 +2,9 @@
 import subprocess
 import sys
 
+import pytest
+import torch
+
 from conftest import REPO
 
 
@@ -19,3 +22,51 @@ def test_a_cache_can_be_made_without_the_native_module(monkeypatch):
 
     monkeypatch.setattr(_lib, "host", missing)
     assert Cache(num_layers=2).get_seq_length() == 0
+
+
+def _allocation(variances, budget):
+    """The dynamic programme of the reference, table by table."""
+    v = variances.float()
+    sizes = [min(64, len(v) - i) for i in range(0, len(v), 64)]
+    var = [v[64 * g:64 * g + s].sum().item() for g, s in enumerate(sizes)]
+    cap = budget // 16 + 1
+    best = [[0.0] * (cap + 1)] + [[float("inf")] * (cap + 1) for _ in sizes]
+    pick = [[0] * (cap + 1) for _ in range(len(sizes) + 1)]
+    cost = [{b: (s * b + 15) // 16 for b in (0, 2, 4, 6, 8)} for s in sizes]
+    for g in range(len(sizes)):
+        for b in range(cap + 1):
+            for bits, c in cost[g].items():
+                if c <= b:
+                    total = best[g][b - c] + (var[g] * 4 if bits == 0 else var[g] / (3.0 * 4 ** bits))
+                    if total < best[g + 1][b]:
+                        best[g + 1][b], pick[g + 1][b] = total, bits
+    b = min(range(cap + 1), key=lambda i: best[-1][i])
+    out = [0] * len(sizes)
+    for g in reversed(range(len(sizes))):
+        out[g] = pick[g + 1][b]
+        b -= cost[g][out[g]]
+    return [bits for bits, s in zip(out, sizes) for _ in range(s)]
+
+
+@pytest.mark.parametrize("d,budget", [(192, 819), (1, 64), (64, 0), (65, -1), (200, -16), (5000, 3000), (4097, 40000), (100, 5000)])
+def test_bit_allocation(d, budget):
+    """Any number of components and any budget the programme can be asked for."""
+    from shard_b200.rope import dp_bit_allocation
+    v = torch.exp(-0.01 * torch.arange(d)) * (1 + 0.3 * torch.rand(d, generator=torch.Generator().manual_seed(d)))
+    assert dp_bit_allocation(v, budget) == _allocation(v, budget)
+    for odd in (float("nan"), float("inf")):
+        w = v.clone()
+        w[d // 2] = odd
+        assert dp_bit_allocation(w, budget) == _allocation(w, budget)
+
+
+def test_bit_allocation_ends():
+    from shard_b200._lib import ShardError
+    from shard_b200.rope import dp_bit_allocation
+    assert dp_bit_allocation(torch.zeros(0), 100) == []
+    v = torch.rand(300, generator=torch.Generator().manual_seed(1))
+    assert dp_bit_allocation(v, 1 << 40) == dp_bit_allocation(v, 1 << 20) == _allocation(v, 10000) == [8] * 300
+    with pytest.raises(ShardError):
+        dp_bit_allocation(v, -17)
+    with pytest.raises(TypeError):
+        dp_bit_allocation(v, 100.5)

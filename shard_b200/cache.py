@@ -225,6 +225,20 @@ class CacheLayer(CacheLayerMixin):
         self._gpu_compressed = None
         self.is_initialized = False
 
+    def __getstate__(self):
+        """For copies of a cache (`copy.deepcopy`, pickle): everything but the launch records, which hold
+        addresses; they are made again at the copy's first launch."""
+        state = self.__dict__.copy()
+        gc = state["_gpu_compressed"]
+        if gc is not None:
+            state["_gpu_compressed"] = {k: v for k, v in gc.items() if k not in ("_seq", "_launch", "_native")}
+        return state
+
+    def __copy__(self):
+        new = type(self).__new__(type(self))               # (a shallow copy shares the dictionary itself)
+        new.__dict__.update(self.__dict__)
+        return new
+
     # -- lazy materialisation (non-fused reads) -------------------------------
     def _lazy_evict(self):
         c = self._cache_ref

@@ -235,3 +235,36 @@ def test_tensors_that_start_between_8_byte_boundaries(streaming, s):
             if step == 2:
                 outs.append(layer.update(f(k), f(v))[0])
         assert all(torch.equal(a, b) for a, b in zip(outs[:len(outs) // 2], outs[len(outs) // 2:]))
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("fused", [True, False])
+def test_a_cache_can_be_copied_between_steps(streaming, fused):
+    """copy.deepcopy in the middle of a reply (a prompt's cache drawn from twice): both go on by themselves."""
+    import copy
+
+    from shard_b200 import fused_attention_compressed
+    cache, layer = _cache(random_gc(300, nkv=2, seed=1), 2, streaming, capacity=16)
+    g = torch.Generator(device="cuda").manual_seed(3)
+
+    def token():
+        return [torch.randn(1, n, 1, 128, generator=g, device="cuda").half() for n in (2, 2, 8)]
+
+    def step(cache, k, v, q):
+        layer = cache.layers[0]
+        cache._fused_decode_update = fused
+        r = layer.update(k, v)
+        if not fused:
+            return [x.clone() for x in r]
+        return [fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq).clone()]
+
+    for _ in range(4):
+        step(cache, *token())
+    other = copy.deepcopy(cache)
+    first, second = token(), token()
+    a = step(cache, *first)                                # the original goes one way ...
+    b = step(other, *second)                               # ... the copy another ...
+    again = copy.deepcopy(other)
+    assert all(not torch.equal(x, y) for x, y in zip(a, b))
+    third = token()
+    assert all(torch.equal(x, y) for x, y in zip(step(other, *third), step(again, *third)))

@@ -24,7 +24,7 @@ from transformers.cache_utils import Cache as HFCache, CacheLayerMixin
 from . import _lib, ops
 from ._lib import ShardError
 from .rope import dp_bit_allocation, get_rope_inv_freq
-from .streaming import get_codebook, stream_signs
+from .streaming import get_codebook, layer_signs
 
 KERNEL_HEAD_DIM = 128
 KERNEL_RANK_STEP = 32
@@ -431,7 +431,7 @@ class CacheLayer(CacheLayerMixin):
         B, heads, _, hd = k.shape
         dev = k.device
         if "signs" not in gc:
-            gc["signs"] = stream_signs(self.layer_idx, hd, dev)
+            gc["signs"] = layer_signs(self.layer_idx, hd, dev)
         cap = gc["k_idx_buf"].shape[0] if "k_idx_buf" in gc else 0
         if need <= cap:
             return

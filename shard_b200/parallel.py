@@ -266,7 +266,7 @@ class BatchedDecoder:
     """
 
     def __init__(self, caches, stream_capacity=512):
-        from .streaming import get_codebook, stream_signs
+        from .streaming import get_codebook, layer_signs
         if not caches:
             raise ValueError("no caches")
         self.caches = caches
@@ -305,7 +305,7 @@ class BatchedDecoder:
                     "v_idx": torch.zeros(stream_capacity, self.nkv, self.hd, dtype=torch.uint8, device=dev),
                     "k_norm": torch.zeros(stream_capacity, self.nkv, dtype=torch.float16, device=dev),
                     "v_norm": torch.zeros(stream_capacity, self.nkv, dtype=torch.float16, device=dev),
-                    "signs": stream_signs(li, self.hd, dev),
+                    "signs": layer_signs(li, self.hd, dev),
                 }
                 self._keep.append(bufs)
                 gc["batched_stream"] = bufs

@@ -86,9 +86,15 @@ def get_codebook(d, bits, device):
     return _cache[key]
 
 
-@functools.lru_cache(maxsize=256)
 def stream_signs(layer_idx, hd, device):
     """Per-layer +-1 vector from torch's CPU generator seeded 42 + 7919 * layer
-    (reference: src/shard/cache.py:201-204).  A constant like the codebook; do not write to it."""
+    (reference: src/shard/cache.py:201-204)."""
     g = torch.Generator(device="cpu").manual_seed(42 + layer_idx * 7919)
     return (torch.randint(0, 2, (hd,), generator=g) * 2 - 1).to(device, torch.float32)
+
+
+@functools.lru_cache(maxsize=256)
+def layer_signs(layer_idx, hd, device):
+    """`stream_signs` as the package's own caches share them (`device`: of a tensor, with its index): a
+    constant like the codebook, not to be written to."""
+    return stream_signs(layer_idx, hd, device)

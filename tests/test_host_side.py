@@ -70,3 +70,11 @@ def test_bit_allocation_ends():
         dp_bit_allocation(v, -17)
     with pytest.raises(TypeError):
         dp_bit_allocation(v, 100.5)
+
+
+def test_stream_signs_are_the_callers():
+    """Every call gives a tensor of its own."""
+    from shard_b200.streaming import stream_signs
+    a, b = stream_signs(3, 128, "cpu"), stream_signs(3, 128, "cpu")
+    a.zero_()
+    assert bool((b.abs() == 1).all()) and torch.equal(b, stream_signs(3, 128, "cpu"))

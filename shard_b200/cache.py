@@ -79,6 +79,7 @@ class TorchEigenpairs:
         self.rank = rank
         self.basis = torch.empty(count, p, rank, dtype=torch.float32, device=gram.device)
         self.host = torch.empty(count, rank, dtype=torch.float32)
+        self.inference = torch.is_inference_mode_enabled()     # (the mode is a thread's own, and the result is of this one)
         done = torch.cuda.current_stream().record_event()
         with TorchEigenpairs._lock:
             if TorchEigenpairs._threads is None:
@@ -88,7 +89,7 @@ class TorchEigenpairs:
 
     def _solve(self, gram, i, done):
         stream = _stream_of_thread(gram.device)
-        with torch.no_grad(), torch.cuda.device(gram.device), torch.cuda.stream(stream):
+        with torch.inference_mode(self.inference), torch.no_grad(), torch.cuda.device(gram.device), torch.cuda.stream(stream):
             stream.wait_event(done)
             w, v = torch.linalg.eigh(gram)
             self.basis[i].copy_(v.flip(-1)[:, :self.rank])

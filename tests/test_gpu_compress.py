@@ -232,3 +232,30 @@ def test_threads_compress_side_by_side(nkv):
         for x, y in zip(a, b):
             for n in names:
                 assert torch.equal(x[n], y[n]), n
+
+
+@pytest.mark.parametrize("nkv", [8, 4])
+@pytest.mark.parametrize("streaming", [True, False])
+def test_prompt_and_reply_under_inference_mode(nkv, streaming):
+    """torch.inference_mode around everything: the same cache and the same attention as under no_grad."""
+    from shard_b200 import Cache, fused_attention_compressed
+    res = []
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            cache = Cache(num_layers=2, n_kv_heads=nkv, rope_inv_freq=_inv_freq().cpu())
+            cache._streaming = streaming
+            for li in range(2):
+                cache.update(_keys(nkv, 400, li).unsqueeze(0), _keys(nkv, 400, 50 + li).unsqueeze(0), li)
+            cache.compress()
+            out = []
+            for t in range(3):
+                for fused in (True, False):
+                    cache._fused_decode_update = fused
+                    for li, layer in enumerate(cache.layers):
+                        k, v = (_keys(nkv, 1, 100 + 10 * t + li + s).unsqueeze(0) for s in (0, 500))
+                        r = layer.update(k, v)
+                        q = _keys(4 * nkv, 1, 900 + t).unsqueeze(0)
+                        out += [fused_attention_compressed(q, layer, layer.get_seq_length() - 1).clone()] if fused else list(r)
+            out += [layer._gpu_compressed[n] for layer in cache.layers for n in ("k_coeffs", "k_basis_q", "v_indices_u8")]
+            res.append([o.clone() for o in out])
+    assert all(torch.equal(a, b) for a, b in zip(*res))

@@ -132,7 +132,7 @@ def _launch_state(gc, cache, dev, nkv, n_q, t0, t1, with_fp16_segments, partial_
     n_win = gc["win_k"].shape[2] if with_fp16_segments else 0
     key = (t0, t1, n_sink, n_win, bool(partial_out), gc["n_compress"], gc["k_rank_kernel"], dev)
     ls = gc.get("_launch")
-    if ls is None or ls.key != key:
+    if ls is None or ls.key != key or ls.inv_freq is not cache._inv_freq(dev):
         _lib.require_cuda(gc["k_wprep"], gc["v_indices_u8"])       # same device as the query, and the current one
         if gc["k_wprep"].device != dev:
             raise _lib.ShardError(f"query on {dev} but the cache lives on {gc['k_wprep'].device}")
@@ -183,7 +183,8 @@ def decode_layer(q_rope, layer, pos_q, tok_range=None, partial_out=False, with_f
     cache = layer._cache_ref
     if plain_step:
         native = gc.get("_native")
-        if native is not None:
+        # (a dictionary may have come from another cache, with a workspace and frequencies of its own)
+        if native is not None and cache._decode_ws is not None and native[2].inv_freq is cache._inv_freq_dev:
             # all of the step in native code; None: something is out of the ordinary
             step, (start, t0, t1), _ = native
             host = _lib.host()

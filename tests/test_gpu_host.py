@@ -268,3 +268,23 @@ def test_a_cache_can_be_copied_between_steps(streaming, fused):
     assert all(not torch.equal(x, y) for x, y in zip(a, b))
     third = token()
     assert all(torch.equal(x, y) for x, y in zip(step(other, *third), step(again, *third)))
+
+
+def test_a_layer_moved_to_another_cache():
+    """The dictionary of a layer that has taken native steps serves a cache with other RoPE frequencies."""
+    from shard_b200 import fused_attention_compressed
+    from shard_b200.attention import decode_layer
+    cache, layer = _cache(random_gc(300, nkv=2, seed=1), 2, True, capacity=16)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(1, 8, 1, 128, generator=g, device="cuda").half()
+    for t in range(3):
+        fused_attention_compressed(q, layer, 400 + t, cache._rope_inv_freq)
+    others = [_cache(random_gc(300, nkv=2, seed=1), 2, True, capacity=16) for _ in range(2)]
+    for c, _ in others:
+        c._rope_inv_freq = c._rope_inv_freq * 0.5
+    (_, moved), (_, ref) = others
+    moved._gpu_compressed = layer._gpu_compressed
+    for t in range(3):
+        out = fused_attention_compressed(q, moved, 400 + t)
+        assert torch.equal(out.view(-1, 128), decode_layer(q, ref, 400 + t))
+    assert not torch.equal(out, fused_attention_compressed(q, layer, 402))

@@ -118,7 +118,8 @@ class LeadingEigenpairs:
     that made `gram`, looked at then."""
 
     def __init__(self, gram, rank, status=None):
-        self.gram, self.rank, self.status = gram, rank, status
+        self.gram, self.rank = gram, rank
+        self.status = None if status is None else word_on_host(status)
         self.basis, self.eigvals, self.flag = ops.eigh_top(gram, rank)
 
     def result(self):
@@ -126,9 +127,8 @@ class LeadingEigenpairs:
         on the host.  Matrices the package's solver reports as too close to degenerate go to
         torch.linalg.eigh."""
         rank = self.rank
-        made = torch.zeros_like(self.flag) if self.status is None else self.status.expand_as(self.flag)
-        host = torch.cat([self.eigvals, torch.stack([self.flag, made], 1).float()], dim=1).cpu()
-        if host[:, rank + 1].any():
+        host = torch.cat([self.eigvals, self.flag.unsqueeze(1).float()], dim=1).cpu()
+        if self.status is not None and int(self.status):
             raise ShardError("the covariance of the keys is undefined: a wait inside its kernel gave up")
         for i in torch.nonzero(host[:, rank]).flatten().tolist():
             w, v = torch.linalg.eigh(self.gram[i])
@@ -141,9 +141,14 @@ def leading_eigenpairs(gram, rank, status=None):
     return TorchEigenpairs(gram, rank) if gram.shape[1] <= TORCH_EIGH_MAX else LeadingEigenpairs(gram, rank, status)
 
 
-def check_encoded(workspace):
-    """Raise if a wait inside a `k_encode` call with this scratch gave up (waits for the device)."""
-    if int(ops.encode_status(workspace).item()):
+def word_on_host(word):
+    """Pinned copy of a device word, valid once the current stream has reached this point."""
+    return torch.empty(1, dtype=word.dtype, pin_memory=True).copy_(word, non_blocking=True)
+
+
+def check_encoded(word):
+    """Raise if a wait inside a `k_encode` call gave up (`word`: its scratch's `encode_status`, on the host)."""
+    if int(word):
         raise ShardError("the key codes are undefined: a wait inside the projection gave up")
 
 
@@ -591,10 +596,17 @@ class Cache(HFCache):
                 kpart = self._compress_k(k_full[0, :, start:end, :], start)
                 vpart = self._compress_v(v_full[0, :, start:end, :])
                 self._finish_layer(li, kpart, vpart, self._ends(li, end), start, end)
+            encoded = None
         else:
-            self._compress_side_by_side(start, end)
+            try:
+                encoded = self._compress_side_by_side(start, end)
+            except BaseException:
+                _second_stream(k0.device).wait_stream(torch.cuda.current_stream())   # (as at its end)
+                raise
         ev1.record()
         ev1.synchronize()
+        if encoded is not None:
+            check_encoded(encoded)
         self.compress_seconds = ev0.elapsed_time(ev1) / 1e3
         self._compressed = True
 
@@ -620,6 +632,7 @@ class Cache(HFCache):
         dev = main.device
         inv_freq = self._inv_freq(dev)
         cov_ws = enc_ws = None
+        bases = []
         in_flight = max(hi - lo for lo, hi in zip(bounds[:-2] or bounds, bounds[2:] or bounds[1:]))
         keep_rows = 4 * n * p * in_flight <= ROWS_BYTES
 
@@ -646,7 +659,6 @@ class Cache(HFCache):
 
         ready = covariances(0)
         main.wait_event(drawn)
-        init_rows.record_stream(main)
         for g in range(n_groups):
             rows, gram, done = ready
             side.wait_event(done)
@@ -661,17 +673,17 @@ class Cache(HFCache):
                 basis, eig_host = solved.result()
                 fin = side.record_event()
             main.wait_event(fin)
-            # made on the second stream, read on this one: another thread that compresses on the same device shares
-            # the second stream, and its allocations there must not reuse this memory too early
-            basis.record_stream(main)
+            bases.append(basis)
             for i, li in enumerate(range(bounds[g], bounds[g + 1])):
                 if not keep_rows:
                     ops.undo_rope(keys(li), start, inv_freq, out=rows[i][0])
                 kpart, enc_ws = self._quantise_k(*rows[i], basis[i], eig_host[i].clamp(min=0) / n, enc_ws)
                 self._finish_layer(li, kpart, vparts[i], ends[i], start, end)
-        # the second stream's tensors go back to the allocator behind everything enqueued here
+        # What was made on the second stream and read on this one (the bases, the rows drawn) goes back to the
+        # allocator behind everything enqueued here: other threads of the device share the second stream, and
+        # their allocations there come after this wait.
         side.wait_stream(main)
-        check_encoded(enc_ws)
+        return word_on_host(ops.encode_status(enc_ws))
 
     def _ends(self, li, end):
         layer = self.layers[li]
@@ -706,7 +718,7 @@ class Cache(HFCache):
             basis = basis.to(dev, torch.float32)[:, :rank]
             eigvals = ((flat - mean) @ basis).pow(2).sum(dim=0) / n
         kpart, workspace = self._quantise_k(flat, mean, mean.half(), basis, eigvals)
-        check_encoded(workspace)
+        check_encoded(ops.encode_status(workspace).cpu())
         return kpart
 
     def _quantise_k(self, flat, mean, mean_f16, basis, eigvals, workspace=None):

@@ -28,14 +28,34 @@
 namespace shard {
 
 // ---------------------------------------------------------------------------
-// undo RoPE: flat[t][kv*128+d] = k*cos - rotate_half(k)*sin, fp32; optionally the columns' sums and the
-// largest magnitude
+// undo RoPE: flat[t][kv*128+d] = k*cos - rotate_half(k)*sin, fp32
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void undo_rope_pair(const __half* __restrict__ row, float* __restrict__ o, int i, float cs, float sn,
+                                               float& a, float& b) {
+  const float lo = __half2float(row[i]), hi = __half2float(row[i + 64]);
+  // d < 64: k[d]*cos - (-k[d+64])*sin ; d >= 64: k[d]*cos - k[d-64]*sin
+  a = __fadd_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn));
+  b = __fsub_rn(__fmul_rn(hi, cs), __fmul_rn(lo, sn));
+  o[i] = a;
+  o[i + 64] = b;
+}
+
+// A block per token: as many of them in flight as the loads and stores need (32K tokens x 8 heads, 201 MB: 51 us;
+// with the loop over tokens of the kernel below 95 us).
+__global__ void __launch_bounds__(128) undo_rope_kernel(const __half* __restrict__ k, int64_t head_stride, int64_t tok_stride, int nkv,
+                                                        int pos_start, const float* __restrict__ inv_freq, float* __restrict__ flat) {
+  const int t = blockIdx.x, i = threadIdx.x & 63;
+  float sn, cs, a, b;
+  sincosf(__fmul_rn((float)(pos_start + t), inv_freq[i]), &sn, &cs);
+  for (int kv = threadIdx.x >> 6; kv < nkv; kv += 2)
+    undo_rope_pair(k + kv * head_stride + (int64_t)t * tok_stride, flat + (size_t)t * nkv * HD + kv * HD, i, cs, sn, a, b);
+}
+
+// The same with the columns' sums and the largest magnitude.
 constexpr int UR_MAX_HEADS_PER_THREAD = 8;   // column sums are kept for up to 32 KV heads
 
 // Block: tokens blockIdx.x * per_block ...; thread: pair i = tid & 63 of heads tid / 64, + 4, ...
-template <bool STATS>
-__global__ void __launch_bounds__(256) undo_rope_kernel(const __half* __restrict__ k, int64_t head_stride, int64_t tok_stride,
+__global__ void __launch_bounds__(256) undo_rope_stats_kernel(const __half* __restrict__ k, int64_t head_stride, int64_t tok_stride,
                                                         int nkv, int n, int per_block, int pos_start,
                                                         const float* __restrict__ inv_freq, float* __restrict__ flat,
                                                         float* __restrict__ part_sums, unsigned int* __restrict__ max_bits) {
@@ -49,37 +69,24 @@ __global__ void __launch_bounds__(256) undo_rope_kernel(const __half* __restrict
     const float phase = __fmul_rn((float)(pos_start + t), freq);
     float sn, cs;
     sincosf(phase, &sn, &cs);
-    auto head = [&](int kv, float& sl, float& sh) {
-      const __half* row = k + kv * head_stride + (int64_t)t * tok_stride;
-      const float lo = __half2float(row[i]), hi = __half2float(row[i + 64]);
-      float* o = flat + (size_t)t * nkv * HD + kv * HD;
-      // d < 64: k[d]*cos - (-k[d+64])*sin ; d >= 64: k[d]*cos - k[d-64]*sin
-      const float a = __fadd_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn));
-      const float b = __fsub_rn(__fmul_rn(hi, cs), __fmul_rn(lo, sn));
-      o[i] = a;
-      o[i + 64] = b;
-      if (STATS) {
-        sl += a;
-        sh += b;
+#pragma unroll
+    for (int j = 0; j < UR_MAX_HEADS_PER_THREAD; ++j) {
+      const int kv = h0 + 4 * j;
+      if (kv < nkv) {
+        float a, b;
+        undo_rope_pair(k + kv * head_stride + (int64_t)t * tok_stride, flat + (size_t)t * nkv * HD + kv * HD, i, cs, sn, a, b);
+        s_lo[j] += a;
+        s_hi[j] += b;
         mx = fmaxf(mx, fmaxf(fabsf(a), fabsf(b)));
       }
-    };
-    if (STATS) {
-#pragma unroll
-      for (int j = 0; j < UR_MAX_HEADS_PER_THREAD; ++j)
-        if (h0 + 4 * j < nkv) head(h0 + 4 * j, s_lo[j], s_hi[j]);
-    } else {
-      for (int kv = h0; kv < nkv; kv += 4) head(kv, s_lo[0], s_hi[0]);
     }
   }
-  if (STATS) {
-    float* o = part_sums + (size_t)blockIdx.x * nkv * HD;
+  float* o = part_sums + (size_t)blockIdx.x * nkv * HD;
 #pragma unroll
-    for (int j = 0; j < UR_MAX_HEADS_PER_THREAD; ++j)
-      if (h0 + 4 * j < nkv) { o[(h0 + 4 * j) * HD + i] = s_lo[j]; o[(h0 + 4 * j) * HD + 64 + i] = s_hi[j]; }
-    mx = warp_max(mx);
-    if ((threadIdx.x & 31) == 0) atomicMax(max_bits, __float_as_uint(mx));
-  }
+  for (int j = 0; j < UR_MAX_HEADS_PER_THREAD; ++j)
+    if (h0 + 4 * j < nkv) { o[(h0 + 4 * j) * HD + i] = s_lo[j]; o[(h0 + 4 * j) * HD + 64 + i] = s_hi[j]; }
+  mx = warp_max(mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(max_bits, __float_as_uint(mx));
 }
 
 // mean of 32 columns per block: 8 rows of partial sums at a time
@@ -357,9 +364,7 @@ extern "C" int shard_b200_undo_rope(const void* k_f16, int64_t head_stride, int6
                                     void* stream) {
   if (!k_f16 || !inv_freq || !flat_out || nkv < 1 || n < 0) return SHARD_E_ARG;
   if (n == 0) return SHARD_OK;
-  const int per_block = (n + 4 * sm_count() - 1) / (4 * (sm_count() > 0 ? sm_count() : 1));
-  undo_rope_kernel<false><<<(n + per_block - 1) / per_block, 256, 0, (cudaStream_t)stream>>>(
-      (const __half*)k_f16, head_stride, tok_stride, nkv, n, per_block, pos_start, inv_freq, flat_out, nullptr, nullptr);
+  undo_rope_kernel<<<n, 128, 0, (cudaStream_t)stream>>>((const __half*)k_f16, head_stride, tok_stride, nkv, pos_start, inv_freq, flat_out);
   SHARD_CHECK_LAUNCH();
   return SHARD_OK;
 }
@@ -397,7 +402,7 @@ extern "C" int shard_b200_k_covariance(const void* k_f16, int64_t head_stride, i
   float* part = (float*)(ws + l.part);
   e = cudaMemsetAsync(max_bits, 0, sizeof(*max_bits), st);      // (the status word stays as it is: the caller's to zero)
   if (e != cudaSuccess) return (int)e;
-  undo_rope_kernel<true><<<l.rope_blocks, 256, 0, st>>>((const __half*)k_f16, head_stride, tok_stride, nkv, n, l.per_block, pos_start,
+  undo_rope_stats_kernel<<<l.rope_blocks, 256, 0, st>>>((const __half*)k_f16, head_stride, tok_stride, nkv, n, l.per_block, pos_start,
                                                         inv_freq, flat_out, sums, max_bits);
   column_mean_kernel<<<p / 32, 256, 0, st>>>(sums, l.rope_blocks, p, n, mean_out, (__half*)mean_f16_out);
   GramParams g{flat_out, mean_out, n, p, l.chunks_per_share, part, max_bits, status};

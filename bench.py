@@ -831,7 +831,7 @@ def run_compress_profile(args):
     import torch
     import synth
     from shard_b200 import Cache, ops
-    from shard_b200.cache import kmeans, pca_fit
+    from shard_b200.cache import kmeans
     from shard_b200.streaming import get_codebook, stream_signs
 
     torch.cuda.set_device(0)
@@ -870,9 +870,17 @@ def run_compress_profile(args):
     row("undo_rope_kernel", timed(lambda: ops.undo_rope(k_mid, SINK, inv)), nbytes=n * 1024 * (2 + 4),
         note="reads fp16 keys, writes fp32")
     mean = flat.mean(dim=0).contiguous()
-    basis, eig = pca_fit(flat, mean, RANK)
-    row("pca_fit (torch: Gram matrix GEMM + eigh)", timed(lambda: pca_fit(flat, mean, RANK), reps=3, warm=1),
-        flops=2 * n * 1024 * 1024, note="Gram matrix on the tensor cores + eigh.cu on one 1024 x 1024 matrix")
+    cov = [torch.empty_like(flat), torch.empty_like(mean), torch.empty_like(mean, dtype=torch.float16),
+           torch.empty(1024, 1024, device=dev)]
+    ws = ops.k_covariance(k_mid, SINK, inv, *cov)
+    row("k_covariance (undo RoPE, mean, gram_kernel, gram_sum)", timed(lambda: ops.k_covariance(k_mid, SINK, inv, *cov, ws)),
+        nbytes=n * 1024 * (2 + 4), flops=n * 1024 * 1024,
+        note="half of the symmetric Gram matrix; three fp16 products of it on the tensor cores")
+    gram = cov[3].unsqueeze(0)
+    basis, eig, _ = ops.eigh_top(gram, RANK)
+    basis = basis[0]
+    row("eigh_top (five kernels)", timed(lambda: ops.eigh_top(gram, RANK)),
+        note="the 192 leading eigenpairs of one 1024 x 1024 matrix: a latency chain on 16 SMs")
     scale = basis.abs().amax(0).clamp(min=1e-6) / 127.0
     w = ((basis / scale).round().clamp(-127, 127) * scale).contiguous()
     proj = ops.k_project(flat, mean, w)
@@ -885,7 +893,7 @@ def run_compress_profile(args):
         nbytes=3 * n * RANK * 4 + n * RANK // 2, note="three passes over the fp32 projection, writes packed int4")
     x, ch = ops.v_hadamard_normalise(v_mid)
     row("v_channel_max / v_clamp / v_normalise", timed(lambda: ops.v_hadamard_normalise(v_mid)),
-        nbytes=n * 1024 * (2 + 4 + 4 + 4), note="reads fp16 values, writes fp32, normalises in place")
+        nbytes=n * 1024 * (2 + 2 + 4), note="reads fp16 values twice (maxima, then normalisation), writes fp32")
     flat_v = x.view(-1, 4)
     g = torch.Generator(device=dev).manual_seed(42)
     cent = flat_v[torch.randperm(flat_v.shape[0], generator=g, device=dev)[:256]].clone()

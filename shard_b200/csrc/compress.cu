@@ -41,14 +41,16 @@ __global__ void kq_init_bits_kernel(uint32_t* ws, int keep, const __grid_constan
   if (j < keep) { ws[j] = 0xffffffffu; ws[keep + j] = 0u; ws[2 * keep + j] = 0u; alloc[j] = bits.b[j]; }
 }
 
-constexpr int KQ_ROWS = 32;  // rows per block (short prompts need the blocks), eight loads in flight per thread
+// Rows per block: a short prompt needs the blocks (1K tokens: 62 us with 32 rows, 63 with 64 and without the eight
+// loads in flight per thread), a long one more rows per atomic (32K: 80 us with 64, 84 with 32; 131K: 231, 238).
+static inline int kq_rows(int n) { return n >= 16384 ? 64 : 32; }
 
-__global__ void __launch_bounds__(256) kq_minmax_kernel(const float* __restrict__ proj, int n, int keep,
+__global__ void __launch_bounds__(256) kq_minmax_kernel(const float* __restrict__ proj, int n, int keep, int rows,
                                                         uint32_t* __restrict__ ws) {
-  const int r0 = blockIdx.x * KQ_ROWS;
+  const int r0 = blockIdx.x * rows;
   for (int j = threadIdx.x; j < keep; j += blockDim.x) {
     float lo = __int_as_float(0x7f800000), hi = neg_inf();
-    const int r1 = min(r0 + KQ_ROWS, n);
+    const int r1 = min(r0 + rows, n);
 #pragma unroll 8
     for (int r = r0; r < r1; ++r) {
       const float v = proj[(size_t)r * keep + j];
@@ -68,9 +70,9 @@ __device__ __forceinline__ float kq_xhat(float x, float lo, float rng, float lev
 }
 
 __global__ void __launch_bounds__(256) kq_absmax_kernel(const float* __restrict__ proj,
-                                                        const int32_t* __restrict__ alloc, int n, int keep,
+                                                        const int32_t* __restrict__ alloc, int n, int keep, int rows,
                                                         uint32_t* __restrict__ ws) {
-  const int r0 = blockIdx.x * KQ_ROWS;
+  const int r0 = blockIdx.x * rows;
   for (int j = threadIdx.x; j < keep; j += blockDim.x) {
     const int bits = alloc[j];
     if (bits == 0) continue;
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(256) kq_absmax_kernel(const float* __restrict_
     const float rng = fmaxf(__fsub_rn(ord2f(ws[keep + j]), lo), 1e-6f);
     const float levels = (float)((1 << bits) - 1);
     float am = 0.f;
-    const int r1 = min(r0 + KQ_ROWS, n);
+    const int r1 = min(r0 + rows, n);
 #pragma unroll 8
     for (int r = r0; r < r1; ++r) am = fmaxf(am, fabsf(kq_xhat(proj[(size_t)r * keep + j], lo, rng, levels)));
     atomicMax(ws + 2 * keep + j, __float_as_uint(am));  // non-negative floats order as integers
@@ -338,9 +340,9 @@ extern "C" size_t shard_b200_k_quantize_workspace_bytes(int32_t n, int32_t keep)
 // (the counters and bit widths are in place)
 static void launch_kq(const float* proj, const int32_t* alloc, int n, int keep, uint32_t* ws, float* coeff_scale, __half* scale_f16,
                       uint8_t* packed, cudaStream_t st) {
-  const int row_blocks = (n + KQ_ROWS - 1) / KQ_ROWS;
-  kq_minmax_kernel<<<row_blocks, 256, 0, st>>>(proj, n, keep, ws);
-  kq_absmax_kernel<<<row_blocks, 256, 0, st>>>(proj, alloc, n, keep, ws);
+  const int rows = kq_rows(n), row_blocks = (n + rows - 1) / rows;
+  kq_minmax_kernel<<<row_blocks, 256, 0, st>>>(proj, n, keep, rows, ws);
+  kq_absmax_kernel<<<row_blocks, 256, 0, st>>>(proj, alloc, n, keep, rows, ws);
   kq_scale_kernel<<<(keep + 255) / 256, 256, 0, st>>>(ws, keep, coeff_scale, scale_f16);
   const size_t total = (size_t)n * (keep / 2);
   kq_pack_kernel<<<capped_blocks((long long)((total + 255) / 256), 16), 256, 0, st>>>(proj, alloc, n, keep, ws, coeff_scale, packed);

@@ -259,3 +259,18 @@ def test_prompt_and_reply_under_inference_mode(nkv, streaming):
             out += [layer._gpu_compressed[n] for layer in cache.layers for n in ("k_coeffs", "k_basis_q", "v_indices_u8")]
             res.append([o.clone() for o in out])
     assert all(torch.equal(a, b) for a, b in zip(*res))
+
+
+@pytest.mark.parametrize("n", [31, 33, 16383, 16384, 16449])
+def test_k_quantize_pack_either_side_of_the_row_rule(n):
+    """Codes and scales are the oracle's with 32 and with 64 rows per block, also where the last block is short."""
+    import numpy as np
+    from oracle import shard_oracle as O
+    from shard_b200 import ops
+    rng = np.random.default_rng(n)
+    proj = (rng.standard_normal((n, 6)) * [10, 3, 1, 0.3, 0.1, 1e-4]).astype(np.float32)
+    proj[-1] *= 4                                          # the extremes lie in the last block
+    alloc = [8, 6, 4, 2, 2, 0]
+    packed, scale = ops.k_quantize_pack(torch.from_numpy(proj).cuda(), alloc)
+    q, want, _ = O.k_int4_codes(proj, alloc)
+    assert np.array_equal(scale.cpu().numpy(), want) and np.array_equal(packed.cpu().numpy(), O.int4_pack(q))

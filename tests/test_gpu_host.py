@@ -288,3 +288,20 @@ def test_a_layer_moved_to_another_cache():
         out = fused_attention_compressed(q, moved, 400 + t)
         assert torch.equal(out.view(-1, 128), decode_layer(q, ref, 400 + t))
     assert not torch.equal(out, fused_attention_compressed(q, layer, 402))
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("fused", [True, False])
+def test_an_update_without_tokens(streaming, fused):
+    """Nothing is appended, with and without rows already there."""
+    cache, layer = _cache(random_gc(300, nkv=2, seed=1), 2, streaming, capacity=16)
+    none = torch.empty(1, 2, 0, 128, dtype=torch.float16, device="cuda")
+    k = torch.randn(1, 2, 3, 128, device="cuda").half()
+    want = layer.keys.clone()
+    cache._fused_decode_update = fused
+    layer.update(none, none)
+    assert layer.get_seq_length() == 368 and torch.equal(layer.keys, want)
+    layer.update(k, k)
+    want = layer.keys.clone()
+    layer.update(none, none)
+    assert layer.get_seq_length() == 371 and torch.equal(layer.keys, want) and want.shape[2] == 371

@@ -93,29 +93,28 @@ static DecodePlan make_plan(const ShardDecodeShape& sh, int batch) {
 // ---------------------------------------------------------------------------
 // phase table
 // ---------------------------------------------------------------------------
-// Layout: tokens in blocks of 32; within a block 16 planes of 32 x 16 bytes: plane c < 8 holds
-// the cosines of pairs 8c..8c+7 of the block's 32 tokens (one 16-byte group per token), plane
-// 8 + c the sines.  A warp whose lanes own 32 consecutive tokens reads a plane as 512
-// contiguous bytes.  One thread computes one token's 8 pairs of one plane pair.
+// Layout: tokens in blocks of 32, 8 KB each; entry (m, kp, lane) of a block, 16 bytes at 16 (32 (4 m + kp) + lane), is what
+// lane `lane` of the warp that attends to the block needs for row 8 m + lane / 4 in its k-steps 2 kp and 2 kp + 1 of the
+// scores product: cos and sin of pairs 8 k + 2 (lane % 4) and + 1, for k = 2 kp and then for k = 2 kp + 1.  So the warp
+// reads 512 contiguous bytes per load and the values are matrix fragments as they come.  The last block is
+// written whole (its tokens behind the end are read, and masked).  One thread computes one entry.
 __global__ void __launch_bounds__(256) phase_table_kernel(int delta0, int n, const float* __restrict__ inv_freq,
                                                           uint4* __restrict__ out) {
-  const int n_blocks = (n + 31) >> 5;
-  const int total = n_blocks * 8 * 32;
+  const int total = ((n + 31) >> 5) * 512;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int r = idx & 31, c = (idx >> 5) & 7, blk = idx >> 8;
-    const int t = blk * 32 + r;
-    if (t >= n) continue;
-    uint32_t cw[4], sw[4];
+    const int lane = idx & 31, kp = (idx >> 5) & 3, m = (idx >> 7) & 3, blk = idx >> 9;
+    const float delta = (float)(delta0 + 32 * blk + 8 * m + (lane >> 2));
+    uint32_t w[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int k = 0; k < 2; ++k) {
+      const int pair = 8 * (2 * kp + k) + 2 * (lane & 3);
       float sn0, cs0, sn1, cs1;
-      sincosf(__fmul_rn((float)(delta0 + t), inv_freq[8 * c + 2 * j]), &sn0, &cs0);
-      sincosf(__fmul_rn((float)(delta0 + t), inv_freq[8 * c + 2 * j + 1]), &sn1, &cs1);
-      cw[j] = (uint32_t)__half_as_ushort(__float2half_rn(cs0)) | ((uint32_t)__half_as_ushort(__float2half_rn(cs1)) << 16);
-      sw[j] = (uint32_t)__half_as_ushort(__float2half_rn(sn0)) | ((uint32_t)__half_as_ushort(__float2half_rn(sn1)) << 16);
+      sincosf(__fmul_rn(delta, inv_freq[pair]), &sn0, &cs0);
+      sincosf(__fmul_rn(delta, inv_freq[pair + 1]), &sn1, &cs1);
+      w[2 * k] = (uint32_t)__half_as_ushort(__float2half_rn(cs0)) | ((uint32_t)__half_as_ushort(__float2half_rn(cs1)) << 16);
+      w[2 * k + 1] = (uint32_t)__half_as_ushort(__float2half_rn(sn0)) | ((uint32_t)__half_as_ushort(__float2half_rn(sn1)) << 16);
     }
-    out[((size_t)blk * 16 + c) * 32 + r] = make_uint4(cw[0], cw[1], cw[2], cw[3]);
-    out[((size_t)blk * 16 + 8 + c) * 32 + r] = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+    out[idx] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -178,7 +177,7 @@ extern "C" int shard_b200_phase_table(int32_t compress_start, int32_t pos_q, int
   if (!inv_freq || !out || n_tok < 0) return SHARD_E_ARG;
   if ((uintptr_t)out & 15) return SHARD_E_ALIGN;
   if (n_tok == 0) return SHARD_OK;
-  const int total = ((n_tok + 31) / 32) * 256;
+  const int total = ((n_tok + 31) / 32) * 512;
   const int blocks = capped_blocks((total + 255) / 256, 8);
   phase_table_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(compress_start - pos_q, n_tok, inv_freq, (uint4*)out);
   SHARD_CHECK_LAUNCH();

@@ -10,6 +10,7 @@ namespace shard {
 
 constexpr int ROWS_PER_CTA = 32;        // rows per CTA when a launch has no middle segment
 constexpr int MAX_ROW_CTAS = 18;
+constexpr int HEAD_PARTS = 8;           // records of a query head that one warp loads at a time
 constexpr int MAX_PARTS = 160;          // records of a (sequence, KV head) that the fused combine merges
 
 // Sequence-split decode: where the launch's result goes when it is delivered straight into the
@@ -41,6 +42,9 @@ struct DecodeParams {
   int n_ctas;           // CTAs per (sequence, KV head) = gridDim.x
   PeerPush push;        // sequence-split: deliver the combined record to every rank's exchange buffer
 };
+
+// release and acquire at device scope (lighter than the sequentially consistent __threadfence)
+__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 struct SoftmaxState {
   float m[GQA];
@@ -98,7 +102,7 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
   quantize_vec_warp(src, sq.signs, cbs, idx_out, norm_out, lane);
 }
 
-// Rows outside the compressed middle, in one index space: u < n_sink + n_win + n_dec is an fp16 row
+// Rows of a launch without a middle segment (with one: decode_pipe.cu's blocks of sixteen), in one index space: u < n_sink + n_win + n_dec is an fp16 row
 // (sink rows first, then window, then the fp16 decode buffer), the rest are streamed rows.  They are dealt
 // out in pairs of a kind, the fp16 rows' pairs first: a warp takes pairs b_first, b_first + b_step, ....
 // Lane owns channels 4*lane..+3 of both rows; the eight dot products (row, head) are summed over the lanes by
@@ -111,10 +115,8 @@ __device__ __forceinline__ void append_new_token(const ShardSeq& sq, const Shard
 // codebook[code]) and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of
 // accumulators serves both kinds.
 //
-// Bound: a warp's chain of dependent instructions and loads (the unpack warps run this nearly alone on
-// their schedulers), so the code is kept short, and small in registers -- more of them, or a function of
-// its own, and the compiler spills in the tile loop.  A streamed row with two butterflies and four full
-// reductions of its own took 3 K cycles, a pair here about 1 K.
+// Bound: a warp's chain of dependent instructions and loads, so the code is kept short, and small in registers.  A
+// streamed row with two butterflies and four full reductions of its own took 3 K cycles, a pair here about 1 K.
 // `qr` is the query as given (fp32 copy in shared memory), `cbs` the stream codebook in shared memory
 // (needed for streamed rows only).
 __device__ __forceinline__ void fp16_row(const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u, const __half*& k, const __half*& v) {
@@ -278,9 +280,8 @@ __device__ __forceinline__ void partial_store(const SoftmaxState& st, float* __r
         make_float4(st.acc[h][0], st.acc[h][1], st.acc[h][2], st.acc[h][3]);
 }
 
-// Warp `h` < 4 merges query head h; ROTATED: into the rotated space of the middle's accumulator
-// (normalised Hadamard over the channels; the combine's inverse takes it back).
-template <int NWARPS, bool ROTATED>
+// Warp `h` < 4 merges query head h.
+template <int NWARPS>
 __device__ __forceinline__ void partial_merge(const float* scratch, float* __restrict__ rec_base, int h, int lane) {
   const float* mw = scratch;
   const float* lw = mw + NWARPS * GQA;
@@ -297,40 +298,153 @@ __device__ __forceinline__ void partial_merge(const float* scratch, float* __res
     L = fmaf(wt, lw[w * GQA + h], L);
     a[0] = fmaf(wt, v.x, a[0]); a[1] = fmaf(wt, v.y, a[1]); a[2] = fmaf(wt, v.z, a[2]); a[3] = fmaf(wt, v.w, a[3]);
   }
-  if (ROTATED) {
-    fwht128_lane4(a, lane);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) a[c] *= INV_SQRT_HD;
-  }
   float* rec = rec_base + h * PART;
   if (lane == 0) *reinterpret_cast<float4*>(rec) = make_float4(M * LN2, L, 0.f, 0.f);    // (the record carries the natural-log maximum)
   *reinterpret_cast<float4*>(rec + 4 + 4 * lane) = make_float4(a[0], a[1], a[2], a[3]);
 }
 
-// Fused combine.  Every CTA of one (sequence, KV head) calls this after its record is written
-// (`synced`: the caller has already synchronised the CTA after those writes).
-// Each takes a ticket; the CTA that draws the last one sees all records of that KV head (the ticket's
-// thread releases the CTA's writes, which the barrier has ordered before it, and acquires the others';
-// fences by every thread cost 2 K cycles more), merges them for the head's four
-// query heads, and puts the counter back to zero for the next call.  The result does not depend
-// on which CTA is last: the parts are always summed in the same order.  `sm_raw` needs 1536 floats that are free,
-// 16-byte aligned; NTHREADS >= 512; at most MAX_PARTS parts (the host's plan sees to it).
-//
-// The merging CTA is the critical path of the whole launch and runs this code once, out of a
-// cold instruction cache: it is kept short.  Warp w < 16 takes query head w % 4 and the parts
-// p = w / 4 (mod 4), lane = channels 4*lane .. 4*lane+3: one 16-byte load per part and lane, the
-// loads of 32 parts in flight together; lane j also fetches (max, sum-exp) of parts j, j + 32, ..., from
-// which the warp derives the weights and hands them round by shuffle.  One path for any number of parts
-// (18 with 8 KV heads, up to 148 with one; against a second path of one thread per channel for more than
-// 64 parts, 30K context, 2 KV heads, 4 layers: 110 -> 83 us; 8 KV heads, 12 layers of 8K: 202 -> 198 us).  The four partial sums of a
-// head meet in shared memory; warp h < 4 adds them in order, runs the inverse Hadamard over the
-// 128 channels (two butterflies inside the thread, five by shuffle) and writes the output.
-template <int NTHREADS>
-__device__ __forceinline__ void ticket_combine(const DecodeParams& p, const ShardSeq& sq, int kv, int b,
-                                               float* sm_raw, int tid, bool synced = false) {
-  static_assert(NTHREADS >= GQA * HD, "16 merging warps");
+// Merge of all records of a query head, by the NSUB warps (w = 0 .. NSUB - 1) that a CTA gives it.  Few records: warp 0 merges
+// them; more: each warp takes every NSUB-th and the sums meet in `sm_head` (NSUB * 128 floats, the head's own, 16-byte aligned).
+// True in the warp that has the result: maximum, sum-exp (the same in every lane) and channels 4 lane .. + 3, back from the rotated
+// space.  The order of the sums depends on the number of parts alone, not on which CTA merges.  The merging CTA is the
+// critical path of its launch and runs this code once, out of a cold instruction cache: it is kept short, and all loads of KB
+// parts are in flight together.  Lane j also fetches (max, sum-exp) of parts j, j + 32, ..., from which the warp derives the weights and
+// hands them round by shuffle.
+template <int NSUB>
+__device__ __forceinline__ bool head_merge(const DecodeParams& p, int b, int h, int hq, int w, int lane, float* sm_head, float& M, float& L, float (&o4)[4]) {
+  constexpr int KB = HEAD_PARTS;
+  const int n_parts = p.n_parts, n_q = p.sh.n_q;
+  const bool split = n_parts > KB;
+  if (w > 0 && !split) return false;
+  const float* rec0 = p.ws + ((size_t)b * n_parts * n_q + h) * PART;
+  const size_t pstride = (size_t)n_q * PART;
+  const int step = split ? NSUB : 1;
+  float4 a[KB];
+  auto load = [&](int p0) {
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+      const int pi = p0 + w + step * k;
+      a[k] = pi < n_parts ? __ldcg(reinterpret_cast<const float4*>(rec0 + pi * pstride + 4) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  load(0);
+  float mj[MAX_PARTS / 32], lj[MAX_PARTS / 32];
+  M = neg_inf(); L = 0.f;
+#pragma unroll
+  for (int k = 0; k < MAX_PARTS / 32; ++k) {
+    const int pj = lane + 32 * k;
+    mj[k] = neg_inf();
+    lj[k] = 0.f;
+    if (pj < n_parts) {
+      const float2 ml = __ldcg(reinterpret_cast<const float2*>(rec0 + pj * pstride));
+      mj[k] = ml.x;
+      lj[k] = ml.y;
+    }
+    M = fmaxf(M, mj[k]);
+  }
+  M = warp_max(M);
+  const float Ms = M == neg_inf() ? 0.f : M;             // (nothing attended to: all weights 0)
+#pragma unroll
+  for (int k = 0; k < MAX_PARTS / 32; ++k) {
+    mj[k] = ex2((mj[k] - Ms) * LOG2E);                   // now the weights; 0 behind the last part
+    L = fmaf(mj[k], lj[k], L);
+  }
+  L = warp_sum(L);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) o4[c] = 0.f;
+#pragma unroll 1
+  for (int p0 = 0; p0 < n_parts; p0 += KB * step) {
+    if (p0 > 0) load(p0);
+#pragma unroll
+    for (int k = 0; k < KB; ++k) {
+      const int pi = p0 + w + step * k;
+      float wj = mj[0];
+      if (split) {
+#pragma unroll
+        for (int j = 1; j < MAX_PARTS / 32; ++j) wj = (pi >> 5) == j ? mj[j] : wj;
+      }
+      const float wt = __shfl_sync(0xffffffffu, wj, pi & 31);
+      o4[0] = fmaf(wt, a[k].x, o4[0]); o4[1] = fmaf(wt, a[k].y, o4[1]);
+      o4[2] = fmaf(wt, a[k].z, o4[2]); o4[3] = fmaf(wt, a[k].w, o4[3]);
+    }
+  }
+  if (split) {
+    float4* sums = reinterpret_cast<float4*>(sm_head) + lane;
+    if (w > 0) sums[w * 32] = make_float4(o4[0], o4[1], o4[2], o4[3]);
+    asm volatile("bar.sync %0, %1;" ::"r"(8 + hq), "r"(NSUB * 32) : "memory");
+    if (w > 0) return false;
+#pragma unroll
+    for (int j = 1; j < NSUB; ++j) {
+      const float4 r = sums[j * 32];
+      o4[0] += r.x; o4[1] += r.y; o4[2] += r.z; o4[3] += r.w;
+    }
+  }
+  // (the records of a launch are all of a kind: in rotated space, or, without a middle segment, standard)
+  if (p.n_chunks > 0) {
+    // inverse (= forward) normalised Hadamard over the 128 channels
+    fwht128_lane4(o4, lane);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) o4[c] = o4[c] * INV_SQRT_HD;
+  }
+  return true;
+}
+
+// the launch's output for one query head, by the warp that has its merged record
+__device__ __forceinline__ void head_output(const DecodeParams& p, const ShardSeq& sq, int h, int lane, float M, float L, const float (&o4)[4]) {
+  if (p.sh.partial_out) {
+    float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(sq.out) + (size_t)h * PART);
+    if (lane == 0) rec[0] = make_float4(M, L, 0.f, 0.f);
+    rec[1 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
+  } else {
+    const float inv = 1.f / L;
+    const __half2 lo = __floats2half2_rn(o4[0] * inv, o4[1] * inv), hi = __floats2half2_rn(o4[2] * inv, o4[3] * inv);
+    uint2 pk;
+    pk.x = *reinterpret_cast<const uint32_t*>(&lo);
+    pk.y = *reinterpret_cast<const uint32_t*>(&hi);
+    reinterpret_cast<uint2*>(reinterpret_cast<__half*>(sq.out) + (size_t)h * HD)[lane] = pk;
+  }
+}
+
+// Fused combine, head by head.  The warp that has written a query head's record (w = 0 of the head's NSUB) takes a ticket for it; the
+// warp that draws the last one sees all records of that head and merges them.  No CTA barrier: heads finish on their own.
+// The four heads' counts share the KV head's word, a byte each (at most MAX_PARTS = 160 arrivals); each is back at zero for the
+// next call.
+template <int NSUB>
+__device__ __forceinline__ void head_combine(const DecodeParams& p, const ShardSeq& sq, int kv, int b, int hq, int w, int lane, float* sm_head) {
+  __shared__ int last_of[GQA];
+  int last = 0;
+  if (w == 0) {
+    __syncwarp();
+    if (lane == 0) {
+      unsigned int* ctr = reinterpret_cast<unsigned int*>(p.tickets) + b * p.sh.nkv + kv;
+      fence_acq_rel_gpu();
+      last = ((atomicAdd(ctr, 1u << (8 * hq)) >> (8 * hq)) & 255u) == (unsigned int)(p.n_ctas - 1);
+      if (last) {
+        fence_acq_rel_gpu();
+        atomicSub(ctr, (unsigned int)p.n_ctas << (8 * hq));   // (nobody looks at it before the next launch)
+      }
+      last_of[hq] = last;
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+  }
+  if (p.n_parts > HEAD_PARTS) {                          // (the head's other warps are needed)
+    asm volatile("bar.sync %0, %1;" ::"r"(8 + hq), "r"(NSUB * 32) : "memory");
+    last = last_of[hq];
+  }
+  if (!last) return;
+  float M, L, o4[4];
+  if (head_merge<NSUB>(p, b, kv * GQA + hq, hq, w, lane, sm_head, M, L, o4)) head_output(p, sq, kv * GQA + hq, lane, M, L, o4);
+}
+
+// Fused combine, all four heads by the CTA that draws the KV head's last ticket: for launches that deliver to the exchange buffers, where
+// one flag stands for the KV head, and for launches without a middle segment.  Every CTA of one (sequence, KV head) calls this after
+// its record is written.  (The ticket's thread releases the CTA's writes, which the barrier has ordered before it, and
+// acquires the others'.)  Warp h + 4 w is the w-th of query head h's NSUB.
+template <int NTHREADS, int NSUB>
+__device__ __forceinline__ void ticket_combine(const DecodeParams& p, const ShardSeq& sq, int kv, int b, float* sm_raw, int tid) {
+  static_assert(NTHREADS >= NSUB * GQA * 32, "the merging warps");
   __shared__ int last_s;
-  if (!synced) __syncthreads();
+  __syncthreads();
   if (tid == 0) {
     int* ctr = p.tickets + b * p.sh.nkv + kv;
     __threadfence();
@@ -343,80 +457,10 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
   }
   __syncthreads();
   if (!last_s) return;
-  // (the records of a launch are all of a kind: in rotated space, or, without a middle segment, standard)
-  const int n_q = p.sh.n_q, n_parts = p.n_parts;
-  const bool rotated = p.n_chunks > 0;
-  const int w = tid >> 5, lane = tid & 31;
-  const float* base0 = p.ws + ((size_t)b * n_parts * n_q + (size_t)kv * GQA) * PART;
-  const size_t pstride = (size_t)n_q * PART;
-  const bool fin = tid < GQA * 32;                    // warp hl < 4 finishes query head hl
-  float M = neg_inf(), L = 0.f;                       // of head w % 4 (the same in every lane)
-  float o4[4] = {0.f, 0.f, 0.f, 0.f};                 // channels 4*lane .. 4*lane+3 of that head
-  if (w < 16) {
-    const int hl = w & 3, sub = w >> 2;
-    const float* rec0 = base0 + hl * PART;
-    constexpr int KB = 8;                              // this warp's parts of a block of 32: all their loads in flight
-    float4 a[KB];
-    auto load = [&](int p0) {
-#pragma unroll
-      for (int k = 0; k < KB; ++k) {
-        const int pi = p0 + sub + 4 * k;
-        a[k] = pi < n_parts ? __ldcg(reinterpret_cast<const float4*>(rec0 + pi * pstride + 4) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    };
-    load(0);
-    float mj[MAX_PARTS / 32], lj[MAX_PARTS / 32];
-#pragma unroll
-    for (int k = 0; k < MAX_PARTS / 32; ++k) {
-      const int pj = lane + 32 * k;
-      mj[k] = neg_inf();
-      lj[k] = 0.f;
-      if (pj < n_parts) {
-        const float2 ml = __ldcg(reinterpret_cast<const float2*>(rec0 + pj * pstride));
-        mj[k] = ml.x;
-        lj[k] = ml.y;
-      }
-      M = fmaxf(M, mj[k]);
-    }
-    M = warp_max(M);
-    const float Ms = M == neg_inf() ? 0.f : M;         // (nothing attended to: all weights 0)
-#pragma unroll
-    for (int k = 0; k < MAX_PARTS / 32; ++k) {
-      mj[k] = ex2((mj[k] - Ms) * LOG2E);               // now the weights; 0 behind the last part
-      L = fmaf(mj[k], lj[k], L);
-    }
-    L = warp_sum(L);
-#pragma unroll 1
-    for (int p0 = 0; p0 < n_parts; p0 += 32) {
-      if (p0 > 0) load(p0);
-      float wj = mj[0];
-#pragma unroll
-      for (int k = 1; k < MAX_PARTS / 32; ++k) wj = p0 == 32 * k ? mj[k] : wj;
-#pragma unroll
-      for (int k = 0; k < KB; ++k) {
-        const float wt = __shfl_sync(0xffffffffu, wj, sub + 4 * k);
-        o4[0] = fmaf(wt, a[k].x, o4[0]); o4[1] = fmaf(wt, a[k].y, o4[1]);
-        o4[2] = fmaf(wt, a[k].z, o4[2]); o4[3] = fmaf(wt, a[k].w, o4[3]);
-      }
-    }
-    if (sub > 0) reinterpret_cast<float4*>(sm_raw)[((sub - 1) * GQA + hl) * 32 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
-  }
-  __syncthreads();
-  if (fin) {
-#pragma unroll
-    for (int sub = 1; sub < 4; ++sub) {
-      const float4 r = reinterpret_cast<const float4*>(sm_raw)[((sub - 1) * GQA + w) * 32 + lane];
-      o4[0] += r.x; o4[1] += r.y; o4[2] += r.z; o4[3] += r.w;
-    }
-    if (rotated) {
-      // inverse (= forward) normalised Hadamard over the 128 channels of the head
-      fwht128_lane4(o4, lane);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) o4[c] = o4[c] * INV_SQRT_HD;
-    }
-  }
-  const int h = kv * GQA + w;                          // query head of a finishing thread
-  const float4 o = make_float4(o4[0], o4[1], o4[2], o4[3]), ml = make_float4(M, L, 0.f, 0.f);
+  const int n_q = p.sh.n_q, lane = tid & 31, w = tid >> 5;
+  const int h = kv * GQA + (w & 3);                      // query head of the warp
+  float M, L, o4[4];
+  const bool fin = w < NSUB * GQA && head_merge<NSUB>(p, b, h, w & 3, w >> 2, lane, sm_raw + (w & 3) * (NSUB * HD), M, L, o4);
   if (p.push.world > 0) {
     // Sequence-split decode: this CTA holds the rank's final record of four query heads.  It goes
     // straight into slot epoch % 2 of EVERY rank's exchange buffer (plain peer stores over
@@ -430,8 +474,8 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
       for (int r = 0; r < p.push.world; ++r) {
         float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.push.bufs[r] + flag_bytes) + slot * slot_floats +
                                                 ((size_t)p.push.rank * n_q + h) * PART);
-        if (lane == 0) rec[0] = ml;
-        rec[1 + lane] = o;
+        if (lane == 0) rec[0] = make_float4(M, L, 0.f, 0.f);
+        rec[1 + lane] = make_float4(o4[0], o4[1], o4[2], o4[3]);
       }
     }
     __threadfence_system();
@@ -456,26 +500,17 @@ __device__ __forceinline__ void ticket_combine(const DecodeParams& p, const Shar
       __syncthreads();
       if (last_s) {
         if (tid == 0 && p.push.status) atomicExch(p.push.status, 1);
-      } else if (tid < GQA * HD) {
-        const int hq = kv * GQA + (tid >> 7), d = tid & (HD - 1);
-        reinterpret_cast<__half*>(p.push.merged_out)[(size_t)hq * HD + d] =
-            merge_rank_records(p.push.bufs[p.push.rank], p.push.world, p.sh.nkv, slot, hq, d);
+      } else {
+        for (int i = tid; i < GQA * HD; i += NTHREADS) {
+          const int hq = kv * GQA + (i >> 7), d = i & (HD - 1);
+          reinterpret_cast<__half*>(p.push.merged_out)[(size_t)hq * HD + d] =
+              merge_rank_records(p.push.bufs[p.push.rank], p.push.world, p.sh.nkv, slot, hq, d);
+        }
       }
     }
     if (!sq.out) return;
   }
-  if (!fin) return;
-  if (p.sh.partial_out) {
-    float4* rec = reinterpret_cast<float4*>(reinterpret_cast<float*>(sq.out) + (size_t)h * PART);
-    if (lane == 0) rec[0] = ml;
-    rec[1 + lane] = o;
-  } else {
-    const __half2 lo = __floats2half2_rn(o4[0] / L, o4[1] / L), hi = __floats2half2_rn(o4[2] / L, o4[3] / L);
-    uint2 pk;
-    pk.x = *reinterpret_cast<const uint32_t*>(&lo);
-    pk.y = *reinterpret_cast<const uint32_t*>(&hi);
-    reinterpret_cast<uint2*>(reinterpret_cast<__half*>(sq.out) + (size_t)h * HD)[lane] = pk;
-  }
+  if (fin) head_output(p, sq, h, lane, M, L, o4);
 }
 
 }  // namespace shard

@@ -1,42 +1,42 @@
 // One decode step of one layer in one launch: split-KV pass over the compressed middle
-// (tcgen05 + tensor memory + bulk copy engine, warp-specialised, three tiles in flight per SM),
-// the fp16 / streamed rows, the stream append and the combine.
+// (tcgen05 + tensor memory + bulk copy engine for the reconstruction of the keys, mma.sync fragments for the
+// narrow products), the fp16 / streamed rows, the stream append and the combine.
 //
-// One CTA per SM (16 warps) owns one KV head and a run of 128-token tiles of the middle segment.
+// One CTA per SM (16 warps) owns one KV head and a run of 128-token tiles of the middle segment.  Two pipelines take the
+// tiles in turn; each has an A slot and a key stage in tensor memory, an issuing thread and a group of four consumer warps.
 //
-//   copy engine         the weights W once; per tile the packed int4 coefficient rows (two buffers,
-//                       two tiles ahead) and the V codes (one buffer per consumer group) land in
-//                       shared memory and are announced on mbarriers -- no load instruction touches
-//                       the cache data
-//   unpack warps (4)    coefficient rows -> fp16 A operand in tensor memory (one A slot, handed back
-//                       by MMA1 in thirds so that the next tile's unpack overlaps its later k-steps);
-//                       in their slack at the end: this CTA's share of the fp16 sink / window rows
-//                       and the streamed rows (dequantised on the fly), transformed into the rotated
-//                       space of the middle's accumulator and handed to the epilogue
-//   consumer groups (3 x 4 warps; group g owns V / P slot g and tiles g, g+3, ...), thread = token
-//                       row; one thread per group issues all tensor-core work of the group:
-//                       MMA1  K_n[128 tok x 128] = A . W^T           (A from TMEM, W in smem; the last
-//                             k-step adds the mean), for the tile two ahead
-//                       K_n -> half2 -> rotate by the relative phase -> K~ written in place
-//                       MMA2  S[128 tok x 16]    = K~ . Q^T          (A = K~ from TMEM)
-//                       meanwhile the token's 32 VQ codes are expanded into the group's V tile
-//                       per-warp online softmax with a lazily moving reference point -> P
-//                       MMA3  O[128 ch x 16]    += V^T . P^T         (V, P in smem; accumulates in
-//                             tensor memory, rescaled only when a reference point moved)
-//   append              in the CTA that owns the newest streamed row two warps of the last consumer
-//                       group quantise the new token while its other two stage the query
-//   epilogue            the 12 token-warps' states and the rows' state merge into ONE record per CTA
-//   combine             the last CTA of a (sequence, KV head) to finish merges all records
+//   copying threads (2) bulk copies: the weights W once, the packed int4 coefficient rows of a tile, its V codes.  No load
+//                       instruction touches the cache data.  In the CTA that owns the newest streamed row their
+//                       two warps first quantise the new token into it
+//   unpack warps (4)    coefficient rows -> fp16 A operand in tensor memory; then this CTA's share of the fp16 sink / window /
+//                       decode rows and the streamed rows, sixteen at a time
+//   issuing threads (2) MMA1  K_n[128 tok x 128] = A . W^T   (A from tensor memory, W in shared memory; the last k-step adds the
+//                       mean).  Two threads, because a hand-over takes a few hundred cycles, during which the tensor core
+//                       would stand still: 368 us for four layers of 131K tokens, 393 with one
+//   consumer warps (8)  K_n -> half2 -> rotated by the relative phase, in the registers' layout of an mma.sync fragment, so that
+//                       S[token][query] = K~ . Q^T needs no trip back through memory; per-warp online softmax with a lazily moving
+//                       reference point; the weights transposed in registers (movmatrix) and
+//                       O[pair of channels][(query, parity)] += V[pair][(token, parity')] . P -- contracted over (token, parity), a
+//                       codebook entry of four channels IS the A fragment: the codes are looked up straight into it and no V tile is ever
+//                       written.  All sums of a warp stay in 16 registers
+//   epilogue            the 12 warps' states merge into ONE record per CTA and query head
+//   combine             per query head: the last warp to write a record merges all of them
 //
-// Launched with programmatic stream serialization: the set-up, the first tiles' unpack,
-// reconstruction products, rotation and V expansion use only tensors that no decode call writes
-// (and the phase table, complete before a launch can start) and run before griddepcontrol.wait.
+// A 16-column product on tcgen05 costs as much as one of 128 columns (59 cycles against 67 for a k-step), so scores and P.V took
+// 0.94 of a tile's 1.8 K cycles on the tensor core; as mma.sync they take 32 instructions of 8 cycles a warp.  What they cost
+// instead: a stream of tcgen05.mma keeps mma.sync waiting, so the consumers' products run between the reconstruction
+// products of two tiles.  That, with the latency of a consumer's chain (tensor memory, rotation, scores, softmax, look-ups, P.V: about
+// 3 K cycles), bounds a tile: 2.7 K cycles.  Against the kernel with all products on tcgen05, shared-memory V tiles and three groups
+// (us a pass): 8K x 12 layers 197 -> 161, 32K x 12 383 -> 345, 131K x 4 408 -> 360, 64 sequences of 8K x 2 923 -> 742.
+// Measured and not kept: eight warps to a tile (80 registers: 8K 197, 131K 377), one paced issuing thread, the stage
+// handed back before the scores product, polling instead of suspended waits (131K 396).
 //
-// Tensor memory: two key stages of 128 columns (tile t uses stage t % 2: un-rotated keys in fp32,
-// overwritten in place by K~ as fp16x2 in columns 0-63 of the stage), the A operand at [256, 360),
-// and per consumer group 16 columns of scores and 16 of P.V accumulator from column 360 on.
+// Launched with programmatic stream serialization: the set-up, the first tiles' unpack and reconstruction products use only
+// tensors that no decode call writes and run before griddepcontrol.wait.
+//
+// Tensor memory: two key stages of 128 columns, two A slots of R/2 + 8 columns from column 256 on.
 // Every hand-over is an mbarrier whose waiters see each of its phases; every wait is bounded and
-// raises the CTA's abort flag when it gives up, after which all roles drain, bulk copies in flight
+// raises the CTA's abort flag when it gives up, after which all roles drain, bulk copies and tensor-core work in flight
 // are waited for, tensor memory is freed and the status word is set.
 #include <atomic>
 #include <cstdlib>
@@ -46,42 +46,47 @@
 
 namespace shard {
 
-constexpr int PP_STAGES = 3;
-constexpr int PP_CONS_WARPS = 12;
-constexpr int PP_UNPACK_WARP0 = 12;
-constexpr int PP_WARPS = 16;
-constexpr int PP_THREADS = PP_WARPS * 32;
+constexpr int PP_ST = 2;                            // pipelines: each an A slot, a key stage, an issuing thread and a consumer group; tile t is pipeline t % 2's
+constexpr int PP_CONS_WARPS = 4 * PP_ST;
+constexpr int PP_UNPACK_WARP0 = PP_CONS_WARPS;
+constexpr int PP_MMA_WARP = PP_CONS_WARPS + 4;
+constexpr int PP_ROW_WARPS = PP_CONS_WARPS + 4;     // warps that can attend to rows
+constexpr int PP_MEET = HD + 4;                     // floats of a warp's sum in the epilogue
+constexpr int PP_SUB = PP_ROW_WARPS / GQA;          // warps per query head in the epilogue and the combine
+constexpr int PP_COEF_WARP = PP_MMA_WARP + PP_ST, PP_VCODE_WARP = PP_COEF_WARP + 1;   // one copying thread each
+constexpr int PP_THREADS = (PP_VCODE_WARP + 1) * 32;
 constexpr int PP_TMEM_COLS = 512;
-// tensor memory: two key stages of 128 columns, the A operand slot (R/2 coefficient columns + 8
-// constant columns 1, 0, ...), and per consumer group 16 columns of scores + 16 of P.V accumulator
-constexpr int PP_COL_A = 256;
-constexpr int PP_COL_SO = 360;
-constexpr int ROW_STATE = GQA * HD + 2 * GQA;   // a consumer warp's row sums: acc[4][128], max[4], sum-exp[4]
-constexpr float PP_LAZY_LOG2 = 8.f;   // a softmax reference point moves only when exceeded by more than 2^8
-constexpr int PP_V_BYTES = 32768, PP_P_BYTES = 4096, PP_Q_BYTES = 4096;
-constexpr int PP_CB_COPIES = 4;       // interleaved copies of the V codebook: lane l reads copy l % 4, entry e of copy c at 4e + c
-constexpr int PP_CB_BYTES = 2048 * PP_CB_COPIES;
-constexpr int PP_ROWQ_BYTES = (GQA * HD + 256) * 4;   // queries as given + stream codebook, for the row path
-constexpr int PP_MISC_BYTES = 1024 + 1024;   // state + barriers, and slack for 1 KB alignment
+constexpr int PP_COL_A = 128 * PP_ST;               // the A operand slots: R/2 coefficient columns + 8 constant columns 1, 0, ... each
+__host__ __device__ constexpr int pp_a_cols(int nw) { return 16 * nw + 8; }
+constexpr int PP_STATE = GQA * HD + 2 * GQA;        // a warp's state, floats: acc[4][128], max[4], sum-exp[4]
+constexpr float PP_LAZY_LOG2 = 8.f;                 // a softmax reference point moves only when exceeded by more than 2^8
+constexpr int PP_C_BUFS = 4;                        // coefficient tiles in shared memory
+constexpr int PP_V_BUFS = 6;                        // V code tiles (4 KB) in shared memory
+constexpr int PP_SPLIT_COPIES = 16;                 // copies of the stream codebook as two fp16 parts, entry e of copy c at 16 e + c: at most two look-ups of a warp meet in a bank
+constexpr int PP_SPLIT_BYTES = 256 * 4 * PP_SPLIT_COPIES;
+constexpr int PP_CB_COPIES = 16;                    // copies of the V codebook, entry e of copy c at 16 e + c: a half-warp's look-ups never meet in a bank
 
 // W holds R + 16 contraction positions (the last 16 carry the mean), in 64-position atoms of 16 KB
 __host__ __device__ constexpr int pp_w_bytes(int nw) { return ((32 * nw + 16 + 63) / 64) * 16384; }
-// staging filled by the bulk copy engine: two tiles of packed coefficients (128 rows x R/2 bytes)
-// and one tile of V codes (128 rows x 32 bytes) per consumer group
-// (at least 5312 bytes each, so that the pair can double as the 8.3 KB row-merge scratch plus the
-// 2.1 KB record of the rows)
-__host__ __device__ constexpr int pp_c_bytes(int nw) { return 128 * 16 * nw < 5312 ? 5312 : 128 * 16 * nw; }
-constexpr int PP_VC_BYTES = 128 * VQ_GROUPS;
-__host__ __device__ constexpr int pp_smem_bytes(int nw) {
-  return pp_w_bytes(nw) + PP_STAGES * (PP_V_BYTES + PP_P_BYTES) + PP_Q_BYTES + PP_CB_BYTES + PP_ROWQ_BYTES +
-         2 * pp_c_bytes(nw) + PP_STAGES * PP_VC_BYTES + PP_MISC_BYTES;
+__host__ __device__ constexpr int pp_c_bytes(int nw) { return nw < 2 ? 2560 : 128 * 16 * nw; }    // (all of them hold the epilogue's sums)
+// Shared memory, by address within the CTA's window.  The codebook sits on a multiple of 32 KB, so that a
+// look-up's address is (code's bits | this lane's base): one shift and one three-input logic operation.
+constexpr int PP_OFF_MISC = 0;                                        // barriers, flags
+constexpr int PP_OFF_QG = 1024;                                       // queries as given, fp16 [4][128]
+constexpr int PP_OFF_QS = PP_OFF_QG + GQA * HD * 2;                   // queries in the stream's code space, two fp16 parts [4][2][128]
+constexpr int PP_OFF_QF = PP_OFF_QS + GQA * HD * 4;                   // un-rotated queries as matrix fragments [8 k-steps][4 q x 4][2 x half2]
+constexpr int PP_OFF_CBS = PP_OFF_QF + 1024;                          // stream codebook, fp32 [256]
+constexpr int PP_OFF_V = PP_OFF_CBS + 1024;                           // V codes [buffer][128 tokens][32]
+constexpr int PP_HEAD_BYTES = PP_OFF_V + PP_V_BUFS * 4096;
+constexpr int PP_CB_ALIGN = 256 * 8 * PP_CB_COPIES;
+static_assert(PP_CB_ALIGN % PP_SPLIT_BYTES == 0, "both tables are looked up by (bits of the code | base of the lane)");
+static_assert(PP_C_BUFS * 2560 >= GQA * PP_SUB * PP_MEET * 4, "the epilogue's sums fit the coefficients' place");
+static_assert(PP_HEAD_BYTES <= PP_CB_ALIGN - 2048, "the head of the layout ends before the first multiple of 32 KB");
+__host__ __device__ constexpr int pp_smem_bytes(int nw) {             // from the end of the 1 KB the system keeps
+  return 2 * PP_CB_ALIGN + PP_SPLIT_BYTES - 1024 + pp_w_bytes(nw) + PP_C_BUFS * pp_c_bytes(nw) + PP_ROW_WARPS * PP_STATE * 4;
 }
 
 // single-thread forms (the caller is one elected thread)
-__device__ __forceinline__ void umma_ss_1t(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
-}
 __device__ __forceinline__ void umma_ts_1t(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc) : "memory");
@@ -89,22 +94,279 @@ __device__ __forceinline__ void umma_ts_1t(uint32_t d_tmem, uint32_t a_tmem, uin
 __device__ __forceinline__ void umma_commit_1t(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// Plain barrier among a subset of the CTA's warps (id 1..15, `count` threads).
-__device__ __forceinline__ void named_bar_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+// Legacy tensor path for the narrow products: D[16 x 8] += A[16 x 16] . B[16 x 8], fp16 with fp32 accumulation.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// The same barrier, also ORing a flag over the participants.  The roles use it to agree on giving
-// up: a warp whose bounded wait failed never leaves its siblings alone at a barrier -- everybody
-// reaches the barrier, learns the combined flag and leaves the tile loop together.
-__device__ __forceinline__ bool named_bar_or(int id, int count, bool flag) {
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %3, 0;\n\t"
-      "bar.red.or.pred p, %1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(out) : "r"(id), "r"(count), "r"((uint32_t)flag) : "memory");
-  return out != 0;
+// 16 lanes (rows) x 16 columns of tensor memory, in the register layout of an mma.sync accumulator: r[4 i + 0, 1] are columns
+// 8 i + 2 (lane % 4) + 0, 1 of row lane / 4, r[4 i + 2, 3] those of row lane / 4 + 8
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr));
 }
-
+// wait for the loads above, naming their registers so that no use moves in front of the wait
+__device__ __forceinline__ void tmem_wait_frags(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]) :: "memory");
+}
+// transpose of an 8 x 8 matrix of 16-bit values spread over the warp, two per lane
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t r;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+  return r;
+}
+__device__ __forceinline__ uint2 lds_u2(uint32_t addr) {
+  uint2 r;
+  asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(r.x), "=r"(r.y) : "r"(addr));
+  return r;
+}
+__device__ __forceinline__ uint32_t lds_u1(uint32_t addr) {
+  uint32_t r;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r) : "r"(addr));
+  return r;
+}
+// ---- rows outside the middle, sixteen at a time on the tensor core -----------------------------------------------------------
+// A block of rows has the form of the middle's products: keys are A fragments (a row's 128 channels in any order, as long as the
+// query's are in the same), the scores come out with row lane / 4 (+ 8) and query head lane % 4 in a lane, and the values
+// are contracted over (row, parity of the channel).  Everything that was 32-bit arithmetic when a warp took two rows at a time
+// keeps 22 bits: the weights, the codebook and the queries in code space are two fp16 parts each, both products of
+// every pair; queries and keys of fp16 rows are exact, and all sums are fp32.  The weights of the values, p times the norm of a streamed row, have a
+// running reference of their own, so that they are at most 1 whatever the norms are.
+// Bound: latency of one block (loads, a chain of products, a softmax over 16 rows) -- about 130 instructions for 16 fp16 rows and
+// 600 for streamed ones, whose codes are looked up one by one; two rows at a time, with a reduction over the lanes for each, took
+// 1 K cycles a pair.
+//
+// A streamed row is never rotated back: its key is norm / sqrt(128) . signs o H(codebook[code]), so the QUERY is taken to the
+// code space (H(signs o q) / sqrt(128)) and the score is norm . (query . codebook[code]); streamed values are summed in code space
+// and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of accumulators serves both kinds.
+struct RowState {
+  float m, l, u;      // of query head lane % 4, log2 domain: reference and sum of the weights, reference of the value weights
+  float o[4][4];      // channels 16 (lane / 4) + 4 i + j of that head
+};
+__device__ __forceinline__ void row_state_init(RowState& st) {
+  st.m = neg_inf(); st.l = 0.f; st.u = neg_inf();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] = 0.f;
+}
+// x as the sum of two fp16 values, the larger in the lower half
+__device__ __forceinline__ uint32_t split_half2(float x) {
+  const __half hi = __float2half_rn(x), lo = __float2half_rn(x - __half2float(hi));
+  return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
+}
+// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255]; one warp
+__device__ __forceinline__ void stream_query(const float* __restrict__ signs, const __half* q, __half* out, int lane) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(q + 4 * lane);
+  const float2 a = __half22float2(as_half2(raw.x)), c = __half22float2(as_half2(raw.y));
+  const float4 sg = *reinterpret_cast<const float4*>(signs + 4 * lane);
+  float x[4] = {a.x * sg.x, a.y * sg.y, c.x * sg.z, c.y * sg.w};
+  fwht128_lane4(x, lane);
+  uint32_t sp[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sp[j] = split_half2(x[j] * INV_SQRT_HD);
+  *reinterpret_cast<uint2*>(out + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x5410), __byte_perm(sp[2], sp[3], 0x5410));
+  *reinterpret_cast<uint2*>(out + HD + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x7632), __byte_perm(sp[2], sp[3], 0x7632));
+}
+// weights of a block's rows: this lane has the scores sc[r] of rows lane / 4 + 8 r (log2 domain, -inf: no such row) and the
+// logarithms lv[r] of their values' norms; gives the value weights as B fragments, w[part][m][slot] for rows 8 m + 2 (lane % 4) + slot
+__device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2], const float (&lv)[2], uint32_t (&w)[2][2][2], int lane) {
+  const float u0 = sc[0] + lv[0], u1 = sc[1] + lv[1];
+  float tm = fmaxf(sc[0], sc[1]), tu = fmaxf(u0, u1);
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {
+    tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, off));
+    tu = fmaxf(tu, __shfl_xor_sync(0xffffffffu, tu, off));
+  }
+  const float m = fmaxf(st.m, tm), u = fmaxf(st.u, tu);
+  const float m0 = m == neg_inf() ? 0.f : m, uu = u == neg_inf() ? 0.f : u;
+  st.l = fmaf(st.l, ex2(st.m - m0), ex2(sc[0] - m0) + ex2(sc[1] - m0));
+  const float al = ex2(st.u - uu);
+  st.m = m; st.u = u;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] *= al;
+  const uint32_t odd = (lane >> 2) & 1, sel0 = odd ? 0x1044u : 0x4410u, sel1 = odd ? 0x3244u : 0x4432u;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const uint32_t sp = split_half2(ex2((r ? u1 : u0) - uu));
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      const uint32_t x = transpose_8x8(__byte_perm(sp, 0u, part ? 0x3232 : 0x1010));
+      w[part][r][0] = __byte_perm(x, 0u, sel0);
+      w[part][r][1] = __byte_perm(x, 0u, sel1);
+    }
+  }
+}
+// fp16 rows u0 .. u0 + 15 (sink rows first, then window, then the fp16 decode buffer)
+__device__ __forceinline__ void fp16_block(RowState& st, const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u0, const __half* qg_s, int lane) {
+  const int g8 = lane >> 2, t4 = lane & 3, last = sh.n_sink + sh.n_win + sh.n_dec - 1;
+  // keys: channels 32 j + 8 t4 .. + 7 of rows g8 and g8 + 8; values: channels 16 g8 .. + 15 of rows 2 t4, 2 t4 + 1, and 8 further
+  // (8-byte loads: the rows may start between 16-byte boundaries; L2-coherent: the newest row may be this CTA's.  A row behind the
+  // last repeats it and gets no weight.)
+  uint2 k[2][8], v[4][4];
+  const __half *kp, *vp;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    fp16_row(sq, sh, kv, min(u0 + g8 + 8 * r, last), kp, vp);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[r][j] = __ldcg(reinterpret_cast<const uint2*>(kp + 32 * (j >> 1) + 8 * t4 + 4 * (j & 1)));
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    fp16_row(sq, sh, kv, min(u0 + 8 * (r >> 1) + 2 * t4 + (r & 1), last), kp, vp);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[r][i] = __ldcg(reinterpret_cast<const uint2*>(vp + 16 * g8 + 4 * i));
+  }
+  float s[2][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint4 q = *reinterpret_cast<const uint4*>(qg_s + (g8 >> 1) * HD + 32 * j + 8 * t4);
+    mma_16816(s[0], k[0][2 * j].x, k[1][2 * j].x, k[0][2 * j].y, k[1][2 * j].y, q.x, q.y);
+    mma_16816(s[1], k[0][2 * j + 1].x, k[1][2 * j + 1].x, k[0][2 * j + 1].y, k[1][2 * j + 1].y, q.z, q.w);
+  }
+  float sc[2];
+  const float lv[2] = {0.f, 0.f};
+#pragma unroll
+  for (int r = 0; r < 2; ++r) sc[r] = u0 + g8 + 8 * r <= last ? (s[0][2 * r] + s[1][2 * r]) * (INV_SQRT_HD * LOG2E) : neg_inf();
+  uint32_t w[2][2][2];
+  block_weights(st, sc, lv, w, lane);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int part = 0; part < 2; ++part)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        mma_16816(st.o[i], v[2 * m][i].x, v[2 * m][i].y, v[2 * m + 1][i].x, v[2 * m + 1][i].y, w[part][m][0], w[part][m][1]);
+}
+// four codes -> the two fp16 parts of their codebook entries, part p of entries (0, 1) in x[p][0] and of (2, 3) in x[p][1]
+__device__ __forceinline__ void split_values(uint32_t codes, uint32_t split, uint32_t (&x)[2][2]) {
+  uint32_t e[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) e[j] = lds_u1(((j == 0 ? codes << 6 : codes >> (8 * j - 6)) & 0x3FC0u) | split);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    x[0][j] = __byte_perm(e[2 * j], e[2 * j + 1], 0x5410);
+    x[1][j] = __byte_perm(e[2 * j], e[2 * j + 1], 0x7632);
+  }
+}
+// streamed rows u0 .. u0 + 15; `split`: address of this lane's copy of the split codebook
+__device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u0, const __half* qs_s,
+                                             uint32_t split, int lane) {
+  const int g8 = lane >> 2, t4 = lane & 3, last = sh.n_stream - 1;
+  uint32_t k[2][8], v[4][4];
+  float kn[2], lv[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const size_t row = (size_t)min(u0 + g8 + 8 * r, last) * sh.nkv + kv;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) k[r][j] = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + row * HD + 32 * (j >> 1) + 8 * t4 + 4 * (j & 1)));
+    kn[r] = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row)));
+    lv[r] = __log2f(__half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row))));
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const size_t row = (size_t)min(u0 + 8 * (r >> 1) + 2 * t4 + (r & 1), last) * sh.nkv + kv;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[r][i] = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + row * HD + 16 * g8 + 4 * i));
+  }
+  // columns 2 h and 2 h + 1 are the two parts of query head h: their sum is the score
+  float s[2][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint4 q = *reinterpret_cast<const uint4*>(qs_s + g8 * HD + 32 * j + 8 * t4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t x0[2][2], x1[2][2];
+      split_values(k[0][2 * j + h], split, x0);
+      split_values(k[1][2 * j + h], split, x1);
+#pragma unroll
+      for (int part = 0; part < 2; ++part) mma_16816(s[part], x0[part][0], x1[part][0], x0[part][1], x1[part][1], h ? q.z : q.x, h ? q.w : q.y);
+    }
+  }
+  float sc[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * kn[r] * (INV_SQRT_HD * LOG2E) : neg_inf();
+  uint32_t w[2][2][2];
+  block_weights(st, sc, lv, w, lane);
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t x0[2][2], x1[2][2];
+      split_values(v[2 * m][i], split, x0);
+      split_values(v[2 * m + 1][i], split, x1);
+#pragma unroll
+      for (int part = 0; part < 4; ++part)
+        mma_16816(st.o[i], x0[part >> 1][0], x0[part >> 1][1], x1[part >> 1][0], x1[part >> 1][1], w[part & 1][m][0], w[part & 1][m][1]);
+    }
+}
+// normalised 128-point Hadamard transform of every query head's sums (channel 16 (lane / 4) + 4 i + j in o[i][j])
+__device__ __forceinline__ void row_sums_fwht(RowState& st, int lane) {
+#pragma unroll
+  for (int h = 1; h < 16; h <<= 1)
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (!(i & h)) {
+        const float a = st.o[i >> 2][i & 3], b = st.o[(i | h) >> 2][(i | h) & 3];
+        st.o[i >> 2][i & 3] = a + b;
+        st.o[(i | h) >> 2][(i | h) & 3] = a - b;
+      }
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) {
+    const float sgn = (lane & off) ? -1.f : 1.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      float& x = st.o[i >> 2][i & 3];
+      x = fmaf(sgn, x, __shfl_xor_sync(0xffffffffu, x, off));
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] *= INV_SQRT_HD;
+}
+// the streamed sums out of the code space
+__device__ __forceinline__ void stream_sums_back(RowState& st, const float* __restrict__ signs, int lane) {
+  row_sums_fwht(st, lane);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 sg = *reinterpret_cast<const float4*>(signs + 16 * (lane >> 2) + 4 * i);
+    st.o[i][0] *= sg.x; st.o[i][1] *= sg.y; st.o[i][2] *= sg.z; st.o[i][3] *= sg.w;
+  }
+}
+// into the rotated space, and out to the epilogue as a warp's state (acc[4][128], max[4], sum-exp[4]); `merge`: joined with the state
+// that the warp has there from its tiles
+__device__ __forceinline__ void row_state_store(RowState& st, float* out, bool merge, int lane) {
+  const int g8 = lane >> 2, t4 = lane & 3;
+  row_sums_fwht(st, lane);
+  float l = st.l;
+#pragma unroll
+  for (int off = 4; off < 32; off <<= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+  float m = st.m, f0 = 0.f;
+  if (merge) {
+    const float m_mid = out[GQA * HD + t4], l_mid = out[GQA * HD + GQA + t4];
+    m = fmaxf(m, m_mid);
+    const float ref = m == neg_inf() ? 0.f : m;
+    f0 = ex2(m_mid - ref);
+    l = fmaf(l, ex2(st.m - ref), l_mid * f0);
+  }
+  const float f = st.u == neg_inf() ? 0.f : ex2(st.u - m);
+  __syncwarp();
+  if (g8 == 0) { out[GQA * HD + t4] = m; out[GQA * HD + GQA + t4] = l; }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float4* at = reinterpret_cast<float4*>(out + t4 * HD + 16 * g8 + 4 * i);
+    float4 x = make_float4(st.o[i][0] * f, st.o[i][1] * f, st.o[i][2] * f, st.o[i][3] * f);
+    if (merge) {
+      const float4 mid = *at;
+      x.x = fmaf(mid.x, f0, x.x); x.y = fmaf(mid.y, f0, x.y); x.z = fmaf(mid.z, f0, x.z); x.w = fmaf(mid.w, f0, x.w);
+    }
+    *at = x;
+  }
+}
 
 // A launch without a middle segment (a cache that holds fp16 and streamed rows only): every CTA
 // attends to its share of the rows (pair b belongs to CTA b % gridDim.x), the CTA
@@ -137,8 +399,8 @@ __global__ void __launch_bounds__(ROWS_THREADS, 1) decode_rows_only_kernel(const
   process_rows(st, sq, sh, kv, part + p.n_row_parts * warp, p.n_row_parts * (ROWS_THREADS / 32), qr, cbs, lane);
   partial_store<ROWS_THREADS / 32>(st, scratch, warp, lane);
   __syncthreads();
-  if (warp < GQA) partial_merge<ROWS_THREADS / 32, false>(scratch, rec_rows, warp, lane);
-  ticket_combine<ROWS_THREADS>(p, sq, kv, blockIdx.z, scratch, tid);
+  if (warp < GQA) partial_merge<ROWS_THREADS / 32>(scratch, rec_rows, warp, lane);
+  ticket_combine<ROWS_THREADS, 4>(p, sq, kv, blockIdx.z, scratch, tid);
 }
 
 template <int NW>  // rank / 32
@@ -147,29 +409,26 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   constexpr int KSTEPS = R / 16 + 1;   // + one step whose A columns are (1, 0, ...) and whose W slice is the mean
   constexpr int W_BYTES = pp_w_bytes(NW);
   constexpr int W_ATOMS = W_BYTES / 16384;
-  constexpr int NSUB = (NW + 1) / 2;   // thirds of the A slot: 4 k-steps (64 ranks) each
+  constexpr int A_COLS = pp_a_cols(NW);
 
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  unsigned char* w_s = smem;
-  unsigned char* v_s = w_s + W_BYTES;                              // [3] V tiles, MN-major, 128B swizzle
-  unsigned char* p_s = v_s + PP_STAGES * PP_V_BYTES;               // [3] P operands [16 x 128 tok]
-  unsigned char* q_s = p_s + PP_STAGES * PP_P_BYTES;               // Q operand [16 x 128]
-  uint2* cbv = reinterpret_cast<uint2*>(q_s + PP_Q_BYTES);         // V codebook
-  float* qr_s = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(cbv) + PP_CB_BYTES);   // queries as given [4][128]
-  float* cbs_s = qr_s + GQA * HD;                                  // stream codebook [256]
-  unsigned char* c_s = reinterpret_cast<unsigned char*>(cbs_s + 256);         // [2] coefficient tiles
-  float* rows_rec_s = reinterpret_cast<float*>(c_s) + 4 * GQA * 130;   // record of this CTA's rows (valid once the coefficient buffers are free)
-  unsigned char* vc_s = c_s + 2 * pp_c_bytes(NW);                  // [3] V code tiles
-  float* misc = reinterpret_cast<float*>(vc_s + PP_STAGES * PP_VC_BYTES);
-  float* alpha_s = misc;                                           // [3][16]
-  float* m_s = misc + 48;                                          // [3][16]
-  float* l_s = misc + 96;                                          // [3][16]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 144);
-  volatile int* abort_s = reinterpret_cast<volatile int*>(misc + 145);
-  volatile int* c_cnt = reinterpret_cast<volatile int*>(misc + 146);   // [2] coefficient tiles requested per buffer
-  volatile int* mma1_next = reinterpret_cast<volatile int*>(misc + 208);   // next tile whose MMA1 is to be issued
-  uint64_t* bars = reinterpret_cast<uint64_t*>(misc + 148);        // 29 mbarriers
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  const uint32_t raw_u = smem_u32(smem_raw);
+  const uint32_t cb_u = (raw_u + PP_HEAD_BYTES + PP_CB_ALIGN - 1) & ~(uint32_t)(PP_CB_ALIGN - 1);
+  if (cb_u != PP_CB_ALIGN) {                                       // (the layout is sized for a window that starts this low)
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
+    return;
+  }
+  unsigned char* cbv = smem_raw + (cb_u - raw_u);                  // V codebook, 16 copies
+  uint4* split_s = reinterpret_cast<uint4*>(cbv + PP_CB_ALIGN);    // split stream codebook
+  unsigned char* w_s = cbv + PP_CB_ALIGN + PP_SPLIT_BYTES;                      // weights (1 KB aligned)
+  unsigned char* c_s = w_s + W_BYTES;                              // coefficient tiles
+  float* state_s = reinterpret_cast<float*>(c_s + PP_C_BUFS * pp_c_bytes(NW));   // states: consumer warps, unpack warps
+  __half* qg_s = reinterpret_cast<__half*>(smem_raw + PP_OFF_QG);
+  __half* qs_s = reinterpret_cast<__half*>(smem_raw + PP_OFF_QS);
+  float* cbs_s = reinterpret_cast<float*>(smem_raw + PP_OFF_CBS);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + PP_OFF_MISC);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + PP_OFF_MISC + 960);
+  volatile int* abort_s = reinterpret_cast<volatile int*>(smem_raw + PP_OFF_MISC + 964);
 
   const ShardSeq& sq = p.table ? p.table[blockIdx.z] : p.one;
   const ShardDecodeShape& sh = p.sh;
@@ -178,551 +437,471 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float* rec_base = p.ws + (((size_t)blockIdx.z * p.n_parts + part) * sh.n_q + (size_t)kv * GQA) * PART;
 
-  // the CTA that owns the newest streamed row quantises it before anybody reads the stream
-  const bool append_here = sh.append && p.n_row_parts > 0 && (row_pairs(sh) - 1) % p.n_row_parts == part;
-
-  // The rows are the unpack warps' (they run about three tiles ahead of the consumers); with more than
-  // eight pairs for each of them all sixteen warps take a share.
-  const bool wide_rows = p.n_row_parts > 0 && row_pairs(sh) > 32 * p.n_row_parts;
+  // The rows outside the middle go in blocks of 16 of a kind, the streamed ones' first; block b is CTA b % n_row_parts's.  They
+  // are the unpack warps' while those have about a block to every two tiles; beyond that all warps but the issuing and copying ones
+  // take a share when their tiles are done.
+  const int blocks_s = (sh.n_stream + 15) >> 4, n_fp16 = sh.n_sink + sh.n_win + sh.n_dec, blocks = blocks_s + ((n_fp16 + 15) >> 4);
+  // the CTA that owns the newest row writes it before anybody reads it
+  const bool append_here = sh.append && p.n_row_parts > 0 && ((sh.append == 1 ? blocks_s : blocks) - 1) % p.n_row_parts == part;
+  const bool wide_rows = p.n_row_parts > 0 && blocks > 4 * p.n_row_parts * max(1, (p.tiles_per_chunk + 1) >> 1);
+  const int n_row_warps = wide_rows ? PP_ROW_WARPS : 4;
 
   griddep_launch();
 
-  // barrier addresses
   const uint32_t bar0 = smem_u32(bars);
-  auto KN_FULL = [&](int g) { return bar0 + 8u * (uint32_t)g; };          // MMA1 of group g's next tile done
-  auto S_FULL = [&](int g) { return bar0 + 8u * (uint32_t)(3 + g); };     // MMA2 done
-  auto O_DONE = [&](int g) { return bar0 + 8u * (uint32_t)(6 + g); };     // MMA3 done (V tile, P and O of the group are free / final)
-  auto A_EMPTY = [&](int j) { return bar0 + 8u * (uint32_t)(12 + j); };   // MMA1 has read third j of the A slot
-  auto A_FULL = [&](int j) { return bar0 + 8u * (uint32_t)(25 + j); };    // third j of the next tile's A operand is in place
-  auto W_FULL = [&](int a) { return bar0 + 8u * (uint32_t)(15 + a); };    // atom a (64 contraction positions) of the weights has landed
-  auto C_FULL = [&](int b) { return bar0 + 8u * (uint32_t)(19 + b); };    // coefficient tile has landed
-  auto V_FULL = [&](int g) { return bar0 + 8u * (uint32_t)(21 + g); };    // V code tile has landed
-  const uint32_t APPEND_DONE = bar0 + 8u * 24u;                           // the newest streamed row has been written
-  const uint32_t Q_READY = bar0 + 8u * 28u;                               // the query operand and the fp32 queries are staged
+  auto KN_FULL = [&](int s) { return bar0 + 8u * (uint32_t)s; };           // MMA1 of pipeline s done: keys in its stage, its A slot free
+  auto KN_EMPTY = [&](int s) { return bar0 + 8u * (uint32_t)(2 + s); };    // the group's four warps have read the stage
+  auto A_FULL = [&](int s) { return bar0 + 8u * (uint32_t)(4 + s); };      // the A operand is in its slot
+  auto MMA_DONE = [&](int s) { return bar0 + 8u * (uint32_t)(6 + s); };    // an issuing thread's work has completed (after giving up)
+  auto W_FULL = [&](int a) { return bar0 + 8u * (uint32_t)(8 + a); };      // atom a (64 contraction positions) of the weights has landed
+  auto C_FULL = [&](int b) { return bar0 + 8u * (uint32_t)(12 + b); };     // coefficient tile has landed
+  auto C_EMPTY = [&](int b) { return bar0 + 8u * (uint32_t)(16 + b); };    // the unpack warps have read it
+  auto V_FULL = [&](int b) { return bar0 + 8u * (uint32_t)(20 + b); };     // V code tile has landed
+  auto V_EMPTY = [&](int b) { return bar0 + 8u * (uint32_t)(28 + b); };    // its group has read it
+  const uint32_t CB_READY = bar0 + 8u * 36u;                               // the codebooks are in shared memory
+  const uint32_t Q_READY = bar0 + 8u * 37u;                                // the query fragments and the queries as given are staged
+  const uint32_t QS_READY = bar0 + 8u * 39u;                               // the queries in code space are there
+  const uint32_t APPEND_DONE = bar0 + 8u * 38u;                            // the newest streamed row has been written
 
   // tiles of this chunk: evenly spread, the first `tiles_rem` chunks get one more
   const int tile_lo = part * p.tiles_per_chunk + min(part, p.tiles_rem);
   const int n_my = p.tiles_per_chunk + (part < p.tiles_rem ? 1 : 0);
-  // bulk copies of tile `it` of this chunk: its packed coefficient rows into buffer it % 2, its
-  // V codes into the buffer of consumer group it % 3.  The last tile of the segment may be
-  // short; the rows behind it keep whatever the buffer held (any byte pattern decodes to finite
-  // values, and those rows get zero weight).
+  const int tok_lo = sh.tok_begin + tile_lo * 128;
+  // Bulk copy of the packed coefficient rows of tile `it` into its buffer.  The last tile of the segment may be
+  // short; the rows behind it keep whatever the buffer held (any byte pattern decodes to finite values, and
+  // those rows get zero weight).
   auto issue_coef = [&](int it) {
-    const int t0 = sh.tok_begin + (tile_lo + it) * 128;
+    const int t0 = tok_lo + it * 128, b = it % PP_C_BUFS;
     const uint32_t bytes = (uint32_t)min(128, sh.tok_end - t0) * (uint32_t)(R / 2);
-    mbar_expect_tx(C_FULL(it & 1), bytes);
-    bulk_g2s(smem_u32(c_s + (it & 1) * pp_c_bytes(NW)), sq.k_coeffs + (size_t)t0 * (R / 2), bytes, C_FULL(it & 1));
-  };
-  auto issue_vcodes = [&](int it) {
-    const int t0 = sh.tok_begin + (tile_lo + it) * 128, g = it % PP_STAGES;
-    const uint32_t bytes = (uint32_t)min(128, sh.tok_end - t0) * (uint32_t)VQ_GROUPS;
-    mbar_expect_tx(V_FULL(g), bytes);
-    bulk_g2s(smem_u32(vc_s + g * PP_VC_BYTES), sq.v_indices + ((size_t)kv * sh.n_comp + t0) * VQ_GROUPS, bytes,
-             V_FULL(g));
+    mbar_expect_tx(C_FULL(b), bytes);
+    bulk_g2s(smem_u32(c_s + b * pp_c_bytes(NW)), sq.k_coeffs + (size_t)t0 * (R / 2), bytes, C_FULL(b));
   };
 
-  // ---- one-time set-up, first part: tensor memory, mbarriers, the first bulk copies ---------------
+  auto issue_vcodes = [&](int it) {
+    const int t0 = tok_lo + it * 128, b = it % PP_V_BUFS;
+    const uint32_t bytes = (uint32_t)min(128, sh.tok_end - t0) * (uint32_t)VQ_GROUPS;
+    mbar_expect_tx(V_FULL(b), bytes);
+    bulk_g2s(smem_u32(smem_raw + PP_OFF_V) + (uint32_t)b * 4096u, sq.v_indices + ((size_t)kv * sh.n_comp + t0) * VQ_GROUPS, bytes, V_FULL(b));
+  };
+
+  // ---- one-time set-up ----------------------------------------------------------------------------
   if (warp == PP_UNPACK_WARP0) {
     tmem_alloc(smem_u32(tmem_slot), PP_TMEM_COLS);
     tmem_relinquish();
   }
-  if (tid == 0) {
-    // first the barriers of the bulk copies, so that the copy engine starts as early as possible:
-    // the first coefficient tile, the weights atom by atom (the first k-steps only need the first
-    // atom), the second coefficient tile and the first V code tile of every consumer group
-    mbar_init(C_FULL(0), 1); mbar_init(C_FULL(1), 1);
+  if (tid == PP_COEF_WARP * 32) {
+    // first the barriers of the bulk copies, so that the copy engine starts as early as possible
+    for (int b = 0; b < PP_C_BUFS; ++b) { mbar_init(C_FULL(b), 1); mbar_init(C_EMPTY(b), 4); }
     for (int a = 0; a < W_ATOMS; ++a) mbar_init(W_FULL(a), 1);
-    for (int g = 0; g < PP_STAGES; ++g) mbar_init(V_FULL(g), 1);
-    c_cnt[0] = n_my > 0 ? 1 : 0; c_cnt[1] = n_my > 1 ? 1 : 0;
     fence_mbar_init();
     if (n_my > 0) issue_coef(0);
-    for (int a = 0; a < W_ATOMS && n_my > 0; ++a) {      // (a CTA for rows alone needs no weights)
+    for (int a = 0; a < W_ATOMS && n_my > 0; ++a) {        // (a CTA for rows alone needs no weights)
       mbar_expect_tx(W_FULL(a), 16384u);
       bulk_g2s(smem_u32(w_s + a * 16384), reinterpret_cast<const unsigned char*>(sq.k_wprep) + (size_t)kv * W_BYTES + a * 16384,
                16384u, W_FULL(a));
     }
-    if (n_my > 1) issue_coef(1);
-    for (int j = 0; j < min(PP_STAGES, n_my); ++j) issue_vcodes(j);
-  } else if (tid == 32) {
-    for (int s = 0; s < PP_STAGES; ++s) {
-      mbar_init(KN_FULL(s), 1); mbar_init(S_FULL(s), 1); mbar_init(O_DONE(s), 1); mbar_init(A_EMPTY(s), 1);
-    }
-    *mma1_next = 0;
-    for (int j = 0; j < 3; ++j) mbar_init(A_FULL(j), 4);
+    for (int it = 1; it < min(PP_C_BUFS, n_my); ++it) issue_coef(it);
+  } else if (tid == PP_VCODE_WARP * 32) {
+    for (int b = 0; b < PP_V_BUFS; ++b) { mbar_init(V_FULL(b), 1); mbar_init(V_EMPTY(b), 4); }
+    fence_mbar_init();
+    for (int it = 0; it < min(PP_V_BUFS, n_my); ++it) issue_vcodes(it);
+  } else if (tid == PP_MMA_WARP * 32) {
+    for (int s = 0; s < PP_ST; ++s) { mbar_init(KN_FULL(s), 1); mbar_init(KN_EMPTY(s), 4); mbar_init(A_FULL(s), 4); mbar_init(MMA_DONE(s), 1); }
+    mbar_init(CB_READY, PP_CONS_WARPS);
+    mbar_init(Q_READY, PP_CONS_WARPS);
     mbar_init(APPEND_DONE, 2);
-    mbar_init(Q_READY, 2);
+    mbar_init(QS_READY, 4);
     *abort_s = 0;
     fence_mbar_init();
   }
+  const int quad = warp & 3, grp = warp >> 2;
+  const int n_use = warp < PP_CONS_WARPS && n_my > grp ? (n_my - grp + PP_ST - 1) / PP_ST : 0;   // tiles of this warp's group
   // (one CTA barrier for what everybody needs: tensor memory, the mbarriers, the copies in flight)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-
-  bool rows_ok = false;
-  float acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; ++j) acc[j] = 0.f;
-  float run_m[GQA], run_l[GQA];
-#pragma unroll
-  for (int h = 0; h < GQA; ++h) { run_m[h] = neg_inf(); run_l[h] = 0.f; }
+  bool ok = true;
+  int asked = min(warp == PP_COEF_WARP ? PP_C_BUFS : PP_V_BUFS, n_my);   // tiles a copying thread has asked for
 
   if (warp < PP_CONS_WARPS) {
     // =============================== consumer groups ======================================
-    const int g = warp >> 2, quad = warp & 3, m = quad * 32 + lane;
-    // Second part of the set-up, by the consumer warps alone -- the unpack warps are already at
-    // work on the first tile: the codebooks into shared memory, zeros where they have to stay.
-    if (tid < 256) {
-      const uint2 e = reinterpret_cast<const uint2*>(sq.v_centroids)[tid];
-#pragma unroll
-      for (int c = 0; c < PP_CB_COPIES; ++c) cbv[PP_CB_COPIES * tid + c] = e;
-    } else if (sh.n_stream > 0) {
-      for (int i = tid - 256; i < 256; i += 128) cbs_s[i] = p.codebook[i];
-    }
+    const int g8 = lane >> 2, t4 = lane & 3;          // the lane's row and column pair in a matrix fragment
+    // the codebooks into shared memory, by the consumer warps alone: the others are already at work
     {
-      // P rows that a token's warp does not own stay zero for the whole kernel, and so do rows 4..15
-      // of the Q operand (it follows the P operands in memory)
-      uint4* z = reinterpret_cast<uint4*>(p_s);
-      for (int i = tid; i < (PP_STAGES * PP_P_BYTES + PP_Q_BYTES) / 16; i += PP_CONS_WARPS * 32) z[i] = make_uint4(0u, 0u, 0u, 0u);
+      const uint2 e = reinterpret_cast<const uint2*>(sq.v_centroids)[tid & 255];
+      if (tid < 256) {
+#pragma unroll
+        for (int c = 0; c < PP_CB_COPIES / 2; ++c)
+          *reinterpret_cast<uint4*>(cbv + tid * (8 * PP_CB_COPIES) + (((c + lane) & (PP_CB_COPIES / 2 - 1)) << 4)) = make_uint4(e.x, e.y, e.x, e.y);
+      }
+      if (sh.n_stream > 0 && tid < 256) {
+        const float c = p.codebook[tid];
+        cbs_s[tid] = c;
+        const uint32_t sp = split_half2(c);
+#pragma unroll
+        for (int j = 0; j < PP_SPLIT_COPIES / 4; ++j) split_s[PP_SPLIT_COPIES / 4 * tid + ((j + (lane >> 1)) & (PP_SPLIT_COPIES / 4 - 1))] = make_uint4(sp, sp, sp, sp);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(CB_READY);
     }
-    fence_proxy_async();
-    named_bar_sync(5, PP_CONS_WARPS * 32);
-    // the MMA-issuing threads of the CTA (one per consumer group + the unpack side's) sit on four
-    // different warp schedulers: group g issues from its warp g + 1, the unpack side from warp 12
-    const int issuer_quad = g + 1;
-    const uint32_t SO_g = tmem_base + (uint32_t)(PP_COL_SO + 32 * g);      // scores at +0, P.V accumulator at +16
-    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    constexpr uint32_t IDESC2 = umma_idesc(128, 16, false, false);
-    constexpr uint32_t IDESC3 = umma_idesc(128, 16, true, false);
-    const uint64_t qdesc = smem_desc_sw128(smem_u32(q_s), 16, 1024);
-    const uint64_t vdesc = smem_desc_sw128(smem_u32(v_s + g * PP_V_BYTES), 16384, 1024);
-    const uint64_t pdesc = smem_desc_sw128(smem_u32(p_s + g * PP_P_BYTES), 16, 1024);
-    unsigned char* v_g = v_s + g * PP_V_BYTES;
-    unsigned char* p_g = p_s + g * PP_P_BYTES;
-    float* alpha_g = alpha_s + 16 * g;
-    const uint4* phase_tab = reinterpret_cast<const uint4*>(sq.phase);
-    const unsigned char* vc_g = vc_s + g * PP_VC_BYTES;
-    int vc_issued = g < n_my ? 1 : 0;        // V code tiles requested for this group so far
-    const bool issuer = quad == issuer_quad && lane == 0;
-    // MMA1 of tile t: K_n[128 tok x 128] = A . W^T into key stage t % 2, issued third by third of the A
-    // slot as the unpack warps fill it, each third handed back as soon as its k-steps have run.
-    // Issued by a consumer group's issuing thread: tiles 0 and 1 at the start, tile t >= 2 by the
-    // thread that has just issued the scores product of tile t - 2 out of the same key stage (one
-    // thread's tensor-core instructions run in issue order, so the stage is not overwritten early).
-    // `mma1_next` keeps the issuing threads in tile order.  A k-step of 128 columns holds its
-    // issuing thread for about as long as the previous one runs (about 900 cycles per tile), which
-    // is why the issuing thread's warp takes no part in expanding the V codes: its three sibling
-    // warps do that for all 128 tokens meanwhile.
-    constexpr uint32_t IDESC1 = umma_idesc(128, 128, false, false);
-    const uint64_t wdesc = smem_desc_sw128(smem_u32(w_s), 16, 1024);
-    auto issue_mma1 = [&](int t) -> bool {
-      int spins = 0;
-      while (*mma1_next != t) {
-        if (++spins > (1 << 20) || *abort_s) { *abort_s = 1; return false; }
-        __nanosleep(32);
-      }
-      const uint32_t T_t = tmem_base + (uint32_t)(128 * (t & 1));
-#pragma unroll
-      for (int j = 0; j < NSUB; ++j) {
-        if (!mbar_wait(A_FULL(j), (uint32_t)(t & 1), abort_s)) return false;
-        if (t == 0) {                                             // only the very first MMA1 can be ahead of the weights
-          if (!mbar_wait(W_FULL(j), 0u, abort_s)) return false;
-          if (j == NSUB - 1 && W_ATOMS > NSUB && !mbar_wait(W_FULL(W_ATOMS - 1), 0u, abort_s)) return false;
-        }
-        tc_fence_after();
-        const int ks_hi = (j == NSUB - 1) ? KSTEPS : 4 * j + 4;
-#pragma unroll
-        for (int ks = 4 * j; ks < 4 * j + 5; ++ks) {
-          if (ks < ks_hi)
-            umma_ts_1t(T_t, tmem_base + PP_COL_A + 8 * ks, wdesc + (uint64_t)(((ks >> 2) * 16384 + (ks & 3) * 32) >> 4),
-                       IDESC1, ks > 0 ? 1u : 0u);
-        }
-        umma_commit_1t(A_EMPTY(j));
-      }
-      umma_commit_1t(KN_FULL(t % PP_STAGES));
-      if (t + 2 < n_my) { issue_coef(t + 2); c_cnt[t & 1] = c_cnt[t & 1] + 1; }   // the unpack warps are done with that buffer
-      *mma1_next = t + 1;
-      return true;
+    const float phq = __fmul_rn((float)sh.pos_q, p.inv_freq[tid & 63]);
+    float snq, csq;
+    sincosf(phq, &snq, &csq);
+    const __half c16 = __float2half_rn(csq), s16 = __float2half_rn(snq);
+    // cos / sin of the rows, laid out as the fragments want them (phase_table_kernel); step i of a tile takes pairs
+    // 16 (i / 2) .. + 15 of rows 16 (i % 2) .. + 15; loaded four steps ahead
+    const uint4* phase_tab = reinterpret_cast<const uint4*>(sq.phase) + lane;
+    const int last_blk = (sh.tok_end - sh.tok_begin - 1) >> 5;
+    auto phase_of = [&](int it) { return phase_tab + (size_t)min((tile_lo + it) * 4 + quad, last_blk) * 512; };
+    uint4 ph[8][2];
+    const uint4* prow = phase_of(min(grp, max(n_my - 1, 0)));
+    auto load_phase = [&](int i, const uint4* pr) {
+      ph[i][0] = pr[((2 * (i & 1)) * 4 + (i >> 1)) * 32];
+      ph[i][1] = pr[((2 * (i & 1) + 1) * 4 + (i >> 1)) * 32];
     };
-    // gather work of the three non-issuing warps: 512 units of (token row, 8 codes), 96 threads
-    const int gq = quad - (quad > issuer_quad ? 1 : 0);        // 0..2 among the gathering warps
-    const int gather_first = gq * 32 + lane;
-    const uint2* cbv4 = cbv + (lane & (PP_CB_COPIES - 1));   // this lane's copy of the codebook (fewer bank conflicts)
-
-    // 256 units of (token row, 16 codes) over the 96 threads of the three non-issuing warps;
-    // consecutive lanes take consecutive rows, so the eight 16-byte stores of a quarter-warp fall
-    // into eight different bank groups of the swizzled tile
-    auto gather_tile = [&]() {
-#pragma unroll 1
-      for (int u = gather_first; u < 256; u += 96) {
-        const int row = u & 127, hf = u >> 7;              // codes 16*hf .. 16*hf+15 of the row
-        const uint4 cq = *reinterpret_cast<const uint4*>(vc_g + row * VQ_GROUPS + 16 * hf);
-        const uint32_t cw[4] = {cq.x, cq.y, cq.z, cq.w};
-        unsigned char* dst = v_g + hf * 16384;
+    if (n_use > 0) {
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj) {
-          const uint32_t two = cw[jj >> 1] >> (16 * (jj & 1));
-          const uint2 e0 = cbv4[4 * (two & 0xff)], e1 = cbv4[4 * ((two >> 8) & 0xff)];
-          *reinterpret_cast<uint4*>(dst + sw128_off(row, jj)) = make_uint4(e0.x, e0.y, e1.x, e1.y);
-        }
-      }
-    };
-
-    bool bad = false;
-    if (issuer && g < 2 && g < n_my) bad |= !issue_mma1(g);
-    __syncwarp();
-    // the V codes of the group's first tile are cache data as well: expanded while waiting
-    if (g < n_my && quad != issuer_quad) {
-      bad |= !mbar_wait(V_FULL(g), 0u, abort_s);
-      gather_tile();
+      for (int i = 0; i < 4; ++i) load_phase(i, prow);
     }
-    // Up to here only tensors that no decode call ever writes were touched (weights, coefficients,
-    // V codes, codebooks): the set-up, the first two tiles' unpack and reconstruction products run
-    // while the launch before this one is still finishing.  The query, the new token, the stream
-    // rows, the scratch and the output may come from, or still be in use by, that launch: every
-    // role waits for it before it touches them.  (The phase table is complete before any CTA of this
-    // launch starts: the kernel that writes it never releases its dependents early.  So the first
-    // two groups also rotate their first tile before they wait.)
-    // The last consumer group -- whose first tile is the furthest away -- has two jobs here: its
-    // first two warps stage the query (the cos / sin of the query position do not depend on the
-    // launch before), and in the CTA that owns the newest streamed row its other two quantise the
-    // new token into it meanwhile (bit-identical to stream_quantize_kernel).  The row is read near
-    // the end of the kernel by the unpack warps, which wait on APPEND_DONE first.
-    const bool stages_q = g == PP_STAGES - 1 && quad < 2;
-    __half c16 = __float2half_rn(1.f), s16 = __float2half_rn(0.f);
-    if (stages_q) {
-      const float phase = __fmul_rn((float)sh.pos_q, p.inv_freq[tid - 256]);
-      float sn, cs;
-      sincosf(phase, &sn, &cs);
-      c16 = __float2half_rn(cs); s16 = __float2half_rn(sn);
-    }
-    if (g == PP_STAGES - 1) griddep_wait();
-    if (stages_q) {
-      // un-rotated query (fp16 arithmetic as the reference) -> Q operand rows 0..3 (rows 4..15 stay
-      // zero); element of pair i (c or d part) sits at the contraction position of the in-place K~
-      // layout: column 8*(i/8) + (i%8)/2 (+4 for the d part), two elements per column.  This thread
-      // takes pair i: dimensions i and i + 64.
-      const int i = tid - 256;
+    // Up to here only tensors that no decode call ever writes were touched (weights, coefficients, V codes,
+    // codebooks) and the phase table, complete before any CTA of this launch starts: the kernel that writes it never
+    // releases its dependents early.  All this, and the first tiles' unpack and reconstruction products, runs
+    // while the launch before this one is still finishing.  The query, the new token, the stream rows, the scratch
+    // and the output may come from, or still be in use by, that launch: every role waits before it touches them.
+    griddep_wait();
+    {
+      // un-rotated queries (fp16 arithmetic as the reference): thread = (pair i, one or two heads)
+      const int i = tid & 63;
       const __half* qg = reinterpret_cast<const __half*>(sq.q) + (size_t)kv * GQA * HD;
-      __half x_lo[GQA], x_hi[GQA];
 #pragma unroll
-      for (int h = 0; h < GQA; ++h) { x_lo[h] = qg[h * HD + i]; x_hi[h] = qg[h * HD + i + 64]; }
-#pragma unroll
-      for (int part2 = 0; part2 < 2; ++part2) {
-        const int d = i + 64 * part2;
-        const int kk = 2 * (8 * (i >> 3) + ((i & 7) >> 1) + (part2 ? 4 : 0)) + (i & 1);
-        unsigned char* qcol = q_s + (kk >> 6) * 2048 + (kk & 7) * 2;
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const __half x = part2 ? x_hi[h] : x_lo[h];
-          const __half rot = part2 ? x_lo[h] : __hneg(x_hi[h]);
-          const __half un = __hsub(__hmul(x, c16), __hmul(rot, s16));
-          *reinterpret_cast<__half*>(qcol + sw128_off(h, (kk >> 3) & 7)) = un;
-          qr_s[h * HD + d] = __half2float(x);
-        }
+      for (int h = tid >> 6; h < GQA; h += PP_CONS_WARPS / 2) {
+        const __half x_lo = qg[h * HD + i], x_hi = qg[h * HD + i + 64];
+        __half* f = reinterpret_cast<__half*>(smem_raw + PP_OFF_QF) + ((i >> 3) * 16 + 4 * h + ((i & 7) >> 1)) * 4 + (i & 1);
+        f[0] = __hsub(__hmul(x_lo, c16), __hmul(__hneg(x_hi), s16));
+        f[2] = __hsub(__hmul(x_hi, c16), __hmul(x_lo, s16));
+        qg_s[h * HD + i] = x_lo;
+        qg_s[h * HD + i + 64] = x_hi;
       }
-      fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(Q_READY);
-    } else if (append_here && g == PP_STAGES - 1) {
-      append_new_token(sq, sh, kv, cbs_s, quad == 3, lane);
+    }
+    ok = __all_sync(0xffffffffu, mbar_wait(CB_READY, 0u, abort_s) && mbar_wait(Q_READY, 0u, abort_s));
+    const uint2* qf_s = reinterpret_cast<const uint2*>(smem_raw + PP_OFF_QF) + (g8 >> 1) * 4 + t4;
+    const uint32_t v_u = smem_u32(smem_raw + PP_OFF_V);
+    const uint32_t cb_lane = cb_u + (uint32_t)(lane & (PP_CB_COPIES - 1)) * 8u;
+    const uint32_t lane_off = (uint32_t)(32 * quad) << 16;
+    const uint32_t sel0 = (g8 & 1) ? 0x1044u : 0x4410u, sel1 = (g8 & 1) ? 0x3244u : 0x4432u;
+    float run_m = neg_inf(), run_l = 0.f;             // of query head t4; log2 domain
+    float o[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
+
+#pragma unroll 1
+    for (int use = 0; use < n_use && ok; ++use) {
+      const int it = grp + use * PP_ST, s = grp;
+      const uint4* pnext = phase_of(min(it + PP_ST, n_my - 1));
+      ok = __all_sync(0xffffffffu, mbar_wait_soon(KN_FULL(s), (uint32_t)(use & 1), abort_s));
+      if (!ok) break;
+      tc_fence_after();
+      // ---- keys: rotate by the relative phase, straight into the A fragments of the scores product -----------
+      const uint32_t kn = tmem_base + (uint32_t)(128 * s) + lane_off;
+      float sc[2][2][4];                              // two sums of each, so that one product does not wait for the last
+#pragma unroll
+      for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sc[b >> 1][b & 1][j] = 0.f;
+      uint2 qf[2];
+      uint32_t kr[2][16];
+      tmem_ld_frag(kn, kr[0]);
+      tmem_ld_frag(kn + 64, kr[0] + 8);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint32_t* r = kr[i & 1];
+        tmem_wait_frags(r);
+        if (i < 7) {
+          const uint32_t at = kn + ((uint32_t)(16 * ((i + 1) & 1)) << 16) + 16 * ((i + 1) >> 1);
+          tmem_ld_frag(at, kr[(i + 1) & 1]);
+          tmem_ld_frag(at + 64, kr[(i + 1) & 1] + 8);
+        } else {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(KN_EMPTY(s));
+        }
+        load_phase((i + 4) & 7, i < 4 ? prow : pnext);
+        if ((i & 1) == 0) { qf[0] = qf_s[16 * i]; qf[1] = qf_s[16 * i + 16]; }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint32_t a[4];
+#pragma unroll
+          for (int rr = 0; rr < 2; ++rr) {            // rows g8, g8 + 8
+            const __half2 c2 = __floats2half2_rn(__uint_as_float(r[4 * k + 2 * rr]), __uint_as_float(r[4 * k + 2 * rr + 1]));
+            const __half2 d2 = __floats2half2_rn(__uint_as_float(r[8 + 4 * k + 2 * rr]), __uint_as_float(r[8 + 4 * k + 2 * rr + 1]));
+            const __half2 cs = as_half2(k ? ph[i][rr].z : ph[i][rr].x), sn = as_half2(k ? ph[i][rr].w : ph[i][rr].y);
+            a[rr] = as_u32(__hfma2(c2, cs, __hneg2(__hmul2(d2, sn))));       // c cos - d sin
+            a[2 + rr] = as_u32(__hfma2(d2, cs, __hmul2(c2, sn)));            // d cos + c sin
+          }
+          mma_16816(sc[i & 1][k], a[0], a[1], a[2], a[3], qf[k].x, qf[k].y);
+        }
+      }
+      prow = pnext;
+      // ---- V codes of the tile: row 8 m + 2 t4 (+ 1), codes 4 g8 .. + 3 ----------------------------------------
+      const int vb = it % PP_V_BUFS;
+      ok = __all_sync(0xffffffffu, mbar_wait_soon(V_FULL(vb), (uint32_t)((it / PP_V_BUFS) & 1), abort_s));
+      if (!ok) break;
+      uint32_t vc[4][2];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t at = v_u + (uint32_t)vb * 4096u + (uint32_t)((32 * quad + 8 * m + 2 * t4) * VQ_GROUPS + 4 * g8);
+        vc[m][0] = lds_u1(at);
+        vc[m][1] = lds_u1(at + VQ_GROUPS);
+      }
+      // ---- softmax: this lane has rows g8 + 8 m of query head t4 (columns 2 t4 and 2 t4 + 1 are the same head) ------
+      const int left = sh.tok_end - (tok_lo + it * 128 + 32 * quad + g8);
+      float pr[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) pr[m] = 8 * m < left ? (sc[m >> 1][0][2 * (m & 1)] + sc[m >> 1][1][2 * (m & 1)]) * (INV_SQRT_HD * LOG2E) : neg_inf();
+      const float top = fmaxf(fmaxf(pr[0], pr[1]), fmaxf(pr[2], pr[3]));
+      if (__any_sync(0xffffffffu, top > run_m + PP_LAZY_LOG2)) {
+        // The reference point of a (warp, head) only moves when the tile's maximum exceeds it by more than
+        // 2^PP_LAZY_LOG2 (weights then stay below that factor, far inside fp16 range).
+        float tm = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 4));
+        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 8));
+        tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, 16));
+        if (tm > run_m + PP_LAZY_LOG2) {
+          const float al = ex2(run_m - tm);           // (0 at the first valid token)
+          run_m = tm;
+          run_l *= al;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[i][j] *= al;
+        }
+      }
+      const float ref = run_m == neg_inf() ? 0.f : run_m;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        pr[m] = ex2(pr[m] - ref);
+        run_l += pr[m];
+      }
+      // ---- P.V: contraction over (token, parity of the channel), so that a codebook entry is a fragment as it is:
+      // O[pair of channels][(head, parity)] += V[pair][(token, parity')] . (P[token][head] if the parities agree) ---------
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const uint32_t x = transpose_8x8(pack_half2(pr[m], pr[m]));          // weights of rows 8 m + 2 t4, + 1 for head g8 / 2
+        const uint32_t b0 = __byte_perm(x, 0u, sel0), b1 = __byte_perm(x, 0u, sel1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint2 e0 = lds_u2((((i == 0 ? vc[m][0] << 7 : vc[m][0] >> (8 * i - 7))) & 0x7F80u) | cb_lane);
+          const uint2 e1 = lds_u2((((i == 0 ? vc[m][1] << 7 : vc[m][1] >> (8 * i - 7))) & 0x7F80u) | cb_lane);
+          mma_16816(o[i], e0.x, e0.y, e1.x, e1.y, b0, b1);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(V_EMPTY(vb));
+    }
+    // the warp's state: this lane has channels 16 g8 .. + 15 of query head t4, in units of the channels' scales
+    {
+      float* st = state_s + warp * PP_STATE;
+      float l = run_l + __shfl_xor_sync(0xffffffffu, run_l, 4);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      if (g8 == 0) { st[GQA * HD + t4] = run_m; st[GQA * HD + GQA + t4] = l; }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint2 cw = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.v_ch) + kv * HD + 16 * g8 + 4 * i);
+        const float2 ca = __half22float2(as_half2(cw.x)), cb = __half22float2(as_half2(cw.y));
+        *reinterpret_cast<float4*>(st + t4 * HD + 16 * g8 + 4 * i) = make_float4(o[i][0] * ca.x, o[i][1] * ca.y, o[i][2] * cb.x, o[i][3] * cb.y);
+      }
+    }
+  } else if (warp < PP_MMA_WARP) {
+    // =============================== unpack warps =========================================
+    const int m = quad * 32 + lane;
+    const uint32_t lane_A = tmem_base + PP_COL_A + ((uint32_t)(quad * 32) << 16);
+#pragma unroll
+    for (int s = 0; s < PP_ST; ++s) {
+      // constant part of the A operand: position R is 1.0 (it multiplies the mean slice of W)
+      const uint32_t ones[8] = {0x00003C00u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      tmem_st_x8(lane_A + s * A_COLS + R / 2, ones);
+    }
+#pragma unroll 1
+    for (int it = 0; it < n_my; ++it) {
+      const int cb = it % PP_C_BUFS, s = it % PP_ST;
+      ok = __all_sync(0xffffffffu, mbar_wait_soon(C_FULL(cb), (uint32_t)((it / PP_C_BUFS) & 1), abort_s));
+      if (!ok) break;                                     // uniform over the warp
+      const uint4* row = reinterpret_cast<const uint4*>(c_s + cb * pp_c_bytes(NW) + m * (R / 2));
+      uint4 x[NW];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) x[i] = row[i];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) {
+        uint32_t ov[16];
+        const uint32_t wv[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const uint32_t hi = wv[e] >> 8;
+          ov[4 * e + 0] = nib2half2_tc(wv[e]);            // ranks 8c+0, 8c+4 of word c = 4i+e
+          ov[4 * e + 1] = nib2half2_hi(wv[e]);            //       8c+1, 8c+5
+          ov[4 * e + 2] = nib2half2_tc(hi);               //       8c+2, 8c+6
+          ov[4 * e + 3] = nib2half2_hi(hi);               //       8c+3, 8c+7
+        }
+        // the slot is free once the MMA1 two tiles back has completed
+        if (i == 0 && it >= PP_ST) {
+          ok = __all_sync(0xffffffffu, mbar_wait_soon(KN_FULL(s), (uint32_t)((it / PP_ST - 1) & 1), abort_s));
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st_x16(lane_A + s * A_COLS + 16 * i, ov);
+      }
+      if (!ok) break;
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(A_FULL(s)); mbar_arrive(C_EMPTY(cb)); }
+    }
+    griddep_wait();
+  } else if (warp < PP_COEF_WARP) {
+    // =============================== issuing warp =========================================
+    // One thread each: MMA1 of every second tile, K_n[128 tok x 128] = A . W^T into the pipeline's key stage.  Two of them, because
+    // the tensor core would stand still during the waits of one (a hand-over takes a few hundred cycles).
+    if (lane == 0) {
+      constexpr uint32_t IDESC1 = umma_idesc(128, 128, false, false);
+      const uint64_t wdesc = smem_desc_sw128(smem_u32(w_s), 16, 1024);
+      const int s = warp - PP_MMA_WARP;
+      const uint32_t T_t = tmem_base + (uint32_t)(128 * s), A_t = tmem_base + PP_COL_A + (uint32_t)(s * A_COLS);
+#pragma unroll 1
+      for (int it = s; it < n_my && ok; it += PP_ST) {
+        ok = mbar_wait_soon(A_FULL(s), (uint32_t)((it / PP_ST) & 1), abort_s);
+        if (ok && it >= PP_ST) ok = mbar_wait_soon(KN_EMPTY(s), (uint32_t)((it / PP_ST - 1) & 1), abort_s);
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ++ks) {
+          if ((ks & 3) == 0) {
+            if (it == s) ok = ok && mbar_wait(W_FULL(ks >> 2), 0u, abort_s);    // only a thread's first MMA1 can be ahead of the weights
+            if (!ok) break;
+            if (ks == 0 || it == s) tc_fence_after();
+          }
+          umma_ts_1t(T_t, A_t + 8 * ks, wdesc + (uint64_t)(((ks >> 2) * 16384 + (ks & 3) * 32) >> 4), IDESC1, ks > 0 ? 1u : 0u);
+        }
+        if (ok) umma_commit_1t(KN_FULL(s));
+      }
+      if (!ok || *abort_s) {
+        // giving up: do not leave while the tensor core may still be at work in this CTA's memory
+        umma_commit_1t(MMA_DONE(s));
+        mbar_wait(MMA_DONE(s), 0u, abort_s);
+      }
+    }
+    __syncwarp();
+    griddep_wait();
+  } else {
+    // =============================== copying warps ========================================
+    // In the CTA that owns the newest streamed row they first quantise the new token into it (bit-identical to
+    // stream_quantize_kernel); the copies asked for so far last meanwhile.
+    if (append_here) {
+      griddep_wait();
+      ok = __all_sync(0xffffffffu, mbar_wait(CB_READY, 0u, abort_s));
+      if (ok) append_new_token(sq, sh, kv, cbs_s, warp == PP_VCODE_WARP, lane);
       __syncwarp();
       if (lane == 0) mbar_arrive(APPEND_DONE);
     }
-    int use = 0;
-    for (int it = g; it < n_my; it += PP_STAGES, ++use) {
-      const uint32_t par = (uint32_t)(use & 1);
-      const uint32_t T_s = tmem_base + (uint32_t)(128 * (it & 1));   // key stage of this tile
-      const uint32_t lane_T = T_s + lane_off;
-      const int t0 = sh.tok_begin + (tile_lo + it) * 128;
-      const int tok = min(t0 + m, sh.tok_end - 1);
-      const bool valid = (t0 + m) < sh.tok_end;
-      // cos/sin of the row: plane c of the token's block of 32 holds 8 pairs for each of its tokens,
-      // so a warp reads 512 contiguous bytes per plane; kept three chunks ahead of use
-      const int tl = tok - sh.tok_begin;
-      const uint4* prow = phase_tab + (size_t)(tl >> 5) * 512 + (tl & 31);
-      uint4 pc[8], ps[8];
-      pc[0] = prow[0 * 32]; ps[0] = prow[8 * 32];
-      pc[1] = prow[1 * 32]; ps[1] = prow[9 * 32];
-      pc[2] = prow[2 * 32]; ps[2] = prow[10 * 32];
-
-      bad |= !mbar_wait(KN_FULL(g), par, abort_s);
-      tc_fence_after();
-
-      // ---- rotate: 8 chunks of 8 pairs; K~ goes back in place --------------------------------
-      // chunk ch reads c columns [8ch, 8ch+8) and d columns [64+8ch, ...) and writes 4 columns of c'
-      // and 4 of d' (two pairs per column) over the 8 c columns it has just consumed
-#pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        uint32_t cr[8], dr[8];
-        tmem_ld_x8(lane_T + 8 * ch, cr);
-        tmem_ld_x8(lane_T + 64 + 8 * ch, dr);
-        if (ch + 3 < 8) { pc[ch + 3] = prow[(ch + 3) * 32]; ps[ch + 3] = prow[(8 + ch + 3) * 32]; }
-        const uint32_t cos2[4] = {pc[ch].x, pc[ch].y, pc[ch].z, pc[ch].w};
-        const uint32_t sin2[4] = {ps[ch].x, ps[ch].y, ps[ch].z, ps[ch].w};
-        tmem_wait_ld();
-        uint32_t oc[4], od[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const __half2 c2 = __floats2half2_rn(__uint_as_float(cr[2 * j]), __uint_as_float(cr[2 * j + 1]));
-          const __half2 d2 = __floats2half2_rn(__uint_as_float(dr[2 * j]), __uint_as_float(dr[2 * j + 1]));
-          const __half2 cs = as_half2(cos2[j]), sn = as_half2(sin2[j]);
-          oc[j] = as_u32(__hfma2(c2, cs, __hneg2(__hmul2(d2, sn))));   // c cos - d sin
-          od[j] = as_u32(__hfma2(d2, cs, __hmul2(c2, sn)));            // d cos + c sin
-        }
-        tmem_st_x4(lane_T + 8 * ch, oc);
-        tmem_st_x4(lane_T + 8 * ch + 4, od);
+    if (lane == 0 && warp == PP_COEF_WARP) {
+      for (int it = PP_C_BUFS; it < n_my && ok; ++it) {
+        ok = mbar_wait(C_EMPTY(it % PP_C_BUFS), (uint32_t)((it / PP_C_BUFS - 1) & 1), abort_s);
+        if (ok) { issue_coef(it); asked = it + 1; }
       }
-      tmem_wait_st();
-      tc_fence_before();
-      bad = named_bar_or(1 + g, 128, bad || *abort_s);
-      if (bad) break;                                   // uniform over the group
-      if (use == 0) griddep_wait();                     // (the last group has waited already)
-      if (issuer) {
-        if (use == 0) bad |= !mbar_wait(Q_READY, 0u, abort_s);
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_ts_1t(SO_g, T_s + 8 * ks, qdesc + (uint64_t)(((ks >> 2) * 2048 + (ks & 3) * 32) >> 4), IDESC2,
-                     ks > 0 ? 1u : 0u);
-        umma_commit_1t(S_FULL(g));
-        if (it + 2 < n_my) bad |= !issue_mma1(it + 2);  // the same key stage, behind the scores product
-      }
-      __syncwarp();
-      // (while the tensor core computes the scores)
-      // ---- gather the token's V row (32 codes) into the group's V tile ---------------------------
-      // the previous tile's P.V product must have finished reading the V tile and P
-      // (the first tile's were expanded before the loop)
-      if (use > 0) {
-        bad |= !mbar_wait(O_DONE(g), (uint32_t)((use - 1) & 1), abort_s);
-        bad |= !mbar_wait(V_FULL(g), par, abort_s);
-        if (quad != issuer_quad) gather_tile();
-      }
-
-      // ---- softmax over this warp's 32 tokens ---------------------------------------------------
-      // The reference point of a (warp, head) only moves when the tile's maximum exceeds it by more
-      // than 2^PP_LAZY_LOG2 (weights then stay below that factor, far inside fp16 range): the
-      // accumulator in tensor memory is rescaled only in those rare tiles.
-      bad |= !mbar_wait(S_FULL(g), par, abort_s);
-      tc_fence_after();
-      {
-        uint32_t sraw[4];
-        tmem_ld_x4(SO_g + lane_off, sraw);
-        tmem_wait_ld();
-#pragma unroll
-        for (int h = 0; h < GQA; ++h) {
-          const float s2 = valid ? __uint_as_float(sraw[h]) * (INV_SQRT_HD * LOG2E) : neg_inf();   // log2 domain
-          const float tm = warp_max(s2);
-          float al = 1.f;
-          if (tm > run_m[h] + PP_LAZY_LOG2) {            // also the first tile with a valid token (run_m = -inf)
-            al = (run_m[h] == neg_inf()) ? 0.f : exp2f(run_m[h] - tm);
-            run_m[h] = tm;
-          }
-          const float pr = valid ? exp2f(s2 - run_m[h]) : 0.f;
-          run_l[h] = run_l[h] * al + pr;
-          const int n = 4 * quad + h;
-          *reinterpret_cast<__half*>(p_g + (m >> 6) * 2048 + sw128_off(n, (m >> 3) & 7) + (m & 7) * 2) = __float2half_rn(pr);
-          if (lane == 0) alpha_g[n] = al;
-        }
-      }
-      fence_proxy_async();
-      tc_fence_before();
-      bad = named_bar_or(1 + g, 128, bad || *abort_s);
-      if (bad) break;                                   // uniform over the group
-      if (use > 0) {
-        // rescale channel m of the accumulator where a reference point moved (same decision in
-        // every thread of the group: all read the same 16 factors)
-        float al[16];
-#pragma unroll
-        for (int j4 = 0; j4 < 4; ++j4) {
-          const float4 a4 = *reinterpret_cast<const float4*>(alpha_g + 4 * j4);
-          al[4 * j4] = a4.x; al[4 * j4 + 1] = a4.y; al[4 * j4 + 2] = a4.z; al[4 * j4 + 3] = a4.w;
-        }
-        bool moved = false;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) moved |= al[j] != 1.f;
-        if (moved) {
-          uint32_t o[16];
-          tmem_ld_x16(SO_g + 16 + lane_off, o);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * al[j]);
-          tmem_st_x16(SO_g + 16 + lane_off, o);
-          tmem_wait_st();
-          tc_fence_before();
-          named_bar_sync(1 + g, 128);
-        }
-      }
-      if (issuer) {
-        if (it + PP_STAGES < n_my) { issue_vcodes(it + PP_STAGES); ++vc_issued; }   // every lane has read its codes
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_ss_1t(SO_g + 16, vdesc + (uint64_t)((ks * 2048) >> 4),
-                     pdesc + (uint64_t)(((ks >> 2) * 2048 + (ks & 3) * 32) >> 4), IDESC3, (ks > 0 || use > 0) ? 1u : 0u);
-        umma_commit_1t(O_DONE(g));
-      }
-      __syncwarp();
-    }
-    griddep_wait();                                     // a group without tiles, or one that gave up early
-    // the group's accumulated P.V: channel m, 16 (warp, head) columns
-    if (use > 0 && !(bad || *abort_s)) {
-      bad |= !mbar_wait(O_DONE(g), (uint32_t)((use - 1) & 1), abort_s);
-      tc_fence_after();
-      if (!bad) {
-        uint32_t o[16];
-        tmem_ld_x16(SO_g + 16 + lane_off, o);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(o[j]);
+    } else if (lane == 0) {
+      for (int it = PP_V_BUFS; it < n_my && ok; ++it) {
+        ok = mbar_wait(V_EMPTY(it % PP_V_BUFS), (uint32_t)((it / PP_V_BUFS - 1) & 1), abort_s);
+        if (ok) { issue_vcodes(it); asked = it + 1; }
       }
     }
-    // giving up: do not leave while a copy this thread asked for may still be landing
-    if ((bad || *abort_s) && issuer && vc_issued > 0)
-      mbar_wait(V_FULL(g), (uint32_t)((vc_issued - 1) & 1), abort_s);
-    // every consumer group parks its state in its own V tile (its last MMA3 has completed), so one CTA
-    // barrier separates the tile loops from the merge
-    float* acc_g = reinterpret_cast<float*>(v_g);      // [16][128], then the row sums (wide rows)
-#pragma unroll
-    for (int h = 0; h < GQA; ++h) {
-      const float l = warp_sum(run_l[h]);
-      if (lane == 0) { m_s[16 * g + 4 * quad + h] = run_m[h]; l_s[16 * g + 4 * quad + h] = l; }
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc_g[j * HD + m] = acc[j];
-    rows_ok = !bad;
-  } else {
-    // =============================== unpack warps =========================================
-    const int quad = warp - PP_UNPACK_WARP0, m = quad * 32 + lane;
-    const uint32_t lane_A = tmem_base + PP_COL_A + ((uint32_t)(quad * 32) << 16);
-    {
-      // constant part of the A operand: position R is 1.0 (it multiplies the mean slice of W)
-      const uint32_t ones[8] = {0x00003C00u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-      tmem_st_x8(lane_A + R / 2, ones);
-    }
-    bool bad = false;
-    for (int it = 0; it < n_my && !bad; ++it) {
-      bad = !mbar_wait(C_FULL(it & 1), (uint32_t)((it >> 1) & 1), abort_s);
-      const uint4* row = reinterpret_cast<const uint4*>(c_s + (it & 1) * pp_c_bytes(NW) + m * (R / 2));
-#pragma unroll
-      for (int j = 0; j < NSUB; ++j) {
-        // third j of the slot is free once the previous tile's MMA1 has run its k-steps over it
-        if (it > 0) bad |= !mbar_wait(A_EMPTY(j), (uint32_t)((it - 1) & 1), abort_s);
-        bad = __any_sync(0xffffffffu, bad || *abort_s);
-        if (bad) break;                                 // uniform over the warp
-        tc_fence_after();
-#pragma unroll
-        for (int i = 2 * j; i < 2 * j + 2 && i < NW; ++i) {
-          const uint4 xi = row[i];
-          const uint32_t wv[4] = {xi.x, xi.y, xi.z, xi.w};
-          uint32_t o[16];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t hi = wv[e] >> 8;
-            o[4 * e + 0] = nib2half2_tc(wv[e]);          // ranks 8c+0, 8c+4 of word c = 4i+e
-            o[4 * e + 1] = nib2half2_hi(wv[e]);          //       8c+1, 8c+5
-            o[4 * e + 2] = nib2half2_tc(hi);             //       8c+2, 8c+6
-            o[4 * e + 3] = nib2half2_hi(hi);             //       8c+3, 8c+7
-          }
-          tmem_st_x16(lane_A + 16 * i, o);
-        }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(A_FULL(j));          // this warp's rows of the third are in place
-      }
-    }
-    // the coefficient staging buffers are free by now and serve as the rows' merge scratch
-    bad = named_bar_or(4, 128, bad || *abort_s);
+    __syncwarp();
     griddep_wait();
-    rows_ok = !bad;
   }
 
-  // ---- rows: this warp's share of the fp16 and streamed rows (pair b belongs to CTA b % n_row_parts); the
-  // unpack warps merge theirs into one state, in the rotated space of the middle's accumulator.  (Some rows
-  // behind every tile instead of all behind the last: the unpack is on the tile loop's critical path, 12 to
-  // 30 % slower.) -------------------------------------------------------------------------------------------
-  if (warp >= PP_CONS_WARPS || wide_rows) {
-    const int row_w = (warp + 4) & 15;                    // unpack warps first
-    SoftmaxState st;
-    softmax_init(st);
-    if (rows_ok && p.n_row_parts > 0) {
-      rows_ok = mbar_wait(Q_READY, 0u, abort_s);
-      if (append_here) rows_ok = rows_ok && mbar_wait(APPEND_DONE, 0u, abort_s);
-      if (rows_ok)
-        process_rows(st, sq, sh, kv, part + p.n_row_parts * row_w, p.n_row_parts * (wide_rows ? 16 : 4), qr_s, cbs_s, lane);
-    }
-    if (row_w < 4) {
-      float* scratch = reinterpret_cast<float*>(c_s);
-      partial_store<4>(st, scratch, row_w, lane);
-      named_bar_sync(4, 128);
-      partial_merge<4, true>(scratch, rows_rec_s, row_w, lane);
-    } else {
-      float* sums = reinterpret_cast<float*>(v_s + ((row_w - 4) >> 2) * PP_V_BYTES + 8192) + (row_w & 3) * ROW_STATE;
-#pragma unroll
-      for (int h = 0; h < GQA; ++h) {
-        fwht128_lane4(st.acc[h], lane);
-        *reinterpret_cast<float4*>(sums + h * HD + 4 * lane) = make_float4(st.acc[h][0] * INV_SQRT_HD, st.acc[h][1] * INV_SQRT_HD,
-                                                                           st.acc[h][2] * INV_SQRT_HD, st.acc[h][3] * INV_SQRT_HD);
-        if (lane == 0) { sums[GQA * HD + h] = st.m[h]; sums[GQA * HD + GQA + h] = st.l[h]; }
+  // ---- rows: this warp's share of the blocks, taken to the rotated space of the middle's accumulator.  (Some rows behind every tile
+  // instead of all behind the last: the unpack is on the tile loop's critical path, slower.) --------------------------------------
+  if (wide_rows ? warp < PP_MMA_WARP : warp >= PP_UNPACK_WARP0 && warp < PP_MMA_WARP) {
+    const int row_w = warp >= PP_UNPACK_WARP0 ? warp - PP_UNPACK_WARP0 : warp + 4;        // unpack warps first
+    RowState st;
+    row_state_init(st);
+    if (ok && p.n_row_parts > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait(Q_READY, 0u, abort_s));
+      if (ok && blocks_s > 0) {
+        // the unpack warps take a query head each to the code space; the others wait for them
+        if (row_w < 4) {
+          stream_query(sq.signs, qg_s + row_w * HD, qs_s + row_w * 2 * HD, lane);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(QS_READY);
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait(QS_READY, 0u, abort_s));
+      }
+      if (ok && append_here) ok = __all_sync(0xffffffffu, mbar_wait(APPEND_DONE, 0u, abort_s));
+      if (ok) {
+        int b = part + p.n_row_parts * row_w;
+        const int step = p.n_row_parts * n_row_warps;
+        if (b < blocks_s) {
+#pragma unroll 1
+          for (; b < blocks_s; b += step) stream_block(st, sq, sh, kv, 16 * b, qs_s, cb_u + PP_CB_ALIGN + 4u * (uint32_t)(lane & (PP_SPLIT_COPIES - 1)), lane);
+          stream_sums_back(st, sq.signs, lane);
+        }
+#pragma unroll 1
+        for (; b < blocks; b += step) fp16_block(st, sq, sh, kv, 16 * (b - blocks_s), qg_s, lane);
       }
     }
+    row_state_store(st, state_s + warp * PP_STATE, warp < PP_CONS_WARPS, lane);
   }
 
-  // ---- epilogue: merge the 12 token-warps' states per head and emit the record -------------------
-  const float ch_scale = __half2float(reinterpret_cast<const __half*>(sq.v_ch)[kv * HD + (tid & 127)]);
-  __syncthreads();
-  {
-    // run_m is kept in the log2 domain (score * log2 e); the record carries the natural-log maximum
-    const int h = tid >> 7, m = tid & 127;              // 512 threads: one (head, channel) each
-    // the rows' state (natural-log reference, already in rotated space and final units)
-    const float rows_m = rows_rec_s[h * PART] * LOG2E, rows_l = rows_rec_s[h * PART + 1], rows_a = rows_rec_s[h * PART + 4 + m];
-    float M = rows_m;
-    auto row_state = [&](int e) { return reinterpret_cast<const float*>(v_s + (e >> 2) * PP_V_BYTES + 8192) + (e & 3) * ROW_STATE; };
-    if (wide_rows) {
-#pragma unroll 1
-      for (int e = 0; e < 12; ++e) M = fmaxf(M, row_state(e)[GQA * HD + h]);
-    }
-#pragma unroll
-    for (int e = 0; e < 12; ++e) M = fmaxf(M, m_s[16 * (e >> 2) + 4 * (e & 3) + h]);
-    float L = 0.f, a = 0.f;
-#pragma unroll
-    for (int e = 0; e < 12; ++e) {
-      const int idx = 16 * (e >> 2) + 4 * (e & 3) + h;
-      const float mv = m_s[idx];
-      const float wt = (mv == neg_inf()) ? 0.f : exp2f(mv - M);
-      L = fmaf(wt, l_s[idx], L);
-      a = fmaf(wt, reinterpret_cast<const float*>(v_s + (e >> 2) * PP_V_BYTES)[(4 * (e & 3) + h) * HD + m], a);
-    }
-    const float wr = (rows_m == neg_inf()) ? 0.f : exp2f(rows_m - M);
-    L = fmaf(wr, rows_l, L);
-    float ra = wr * rows_a;
-    if (wide_rows) {
-#pragma unroll 1
-      for (int e = 0; e < 12; ++e) {
-        const float* rs = row_state(e);
-        const float mv = rs[GQA * HD + h], wt = (mv == neg_inf()) ? 0.f : exp2f(mv - M);
-        L = fmaf(wt, rs[GQA * HD + GQA + h], L);
-        ra = fmaf(wt, rs[h * HD + m], ra);
-      }
-    }
-    float* rec = rec_base + h * PART;
-    if (m == 0) { rec[0] = M * LN2; rec[1] = L; rec[2] = 0.f; rec[3] = 0.f; }
-    rec[4 + m] = fmaf(a, ch_scale, ra);
-  }
-  if (tid == 0 && *abort_s) {
-    // gave up somewhere: do not leave while a bulk copy may still be landing in this CTA's memory
-    for (int a = 0; a < W_ATOMS && n_my > 0; ++a) mbar_wait(W_FULL(a), 0u, abort_s);
-    for (int b = 0; b < 2; ++b)
-      if (c_cnt[b] > 0) mbar_wait(C_FULL(b), (uint32_t)((c_cnt[b] - 1) & 1), abort_s);
-    if (p.status) atomicExch(p.status, 1);
-  }
-  // one barrier serves the hand-back of tensor memory and the release of this CTA's records
+  // ---- epilogue: merge the warps' states per head and emit the record -----------------------------------
   tc_fence_before();
   __syncthreads();
   if (warp == PP_UNPACK_WARP0) tmem_dealloc(tmem_base, PP_TMEM_COLS);
-  ticket_combine<PP_THREADS>(p, sq, kv, blockIdx.z, reinterpret_cast<float*>(v_s), tid, true);   // the V tiles are free
+  if (*abort_s) {
+    // gave up somewhere: do not leave while a bulk copy may still be landing in this CTA's memory
+    if (tid == 0 && p.status) atomicExch(p.status, 1);
+    if (tid == PP_COEF_WARP * 32) {
+      for (int a = 0; a < W_ATOMS && n_my > 0; ++a) mbar_wait(W_FULL(a), 0u, abort_s);
+      for (int c = max(0, asked - PP_C_BUFS); c < asked; ++c) mbar_wait(C_FULL(c % PP_C_BUFS), (uint32_t)((c / PP_C_BUFS) & 1), abort_s);
+    } else if (tid == PP_VCODE_WARP * 32) {
+      for (int c = max(0, asked - PP_V_BUFS); c < asked; ++c) mbar_wait(V_FULL(c % PP_V_BUFS), (uint32_t)((c / PP_V_BUFS) & 1), abort_s);
+    }
+  }
+  if (warp < PP_MMA_WARP) {
+    // Warp = (query head, one of three), lane = four channels; maxima are in the log2 domain, the record carries the natural
+    // logarithm's.  Each merges every third state, the head's first warp the three sums.
+    const int hq = warp & 3, sub = warp >> 2;
+    float M = neg_inf(), L = 0.f, a[4] = {0.f, 0.f, 0.f, 0.f};
+    auto add = [&](float m, float l, const float4& x) {
+      const float top = fmaxf(M, m), ref = top == neg_inf() ? 0.f : top, w0 = ex2(M - ref), w1 = ex2(m - ref);
+      M = top;
+      L = fmaf(w1, l, L * w0);
+      a[0] = fmaf(w1, x.x, a[0] * w0); a[1] = fmaf(w1, x.y, a[1] * w0); a[2] = fmaf(w1, x.z, a[2] * w0); a[3] = fmaf(w1, x.w, a[3] * w0);
+    };
+#pragma unroll
+    for (int e = sub; e < PP_ROW_WARPS; e += PP_SUB) {
+      const float* st = state_s + e * PP_STATE;
+      add(st[GQA * HD + hq], st[GQA * HD + GQA + hq], *reinterpret_cast<const float4*>(st + hq * HD + 4 * lane));
+    }
+    float* meet = reinterpret_cast<float*>(c_s) + hq * (PP_SUB * PP_MEET);        // (the coefficients have all been read)
+    if (sub > 0) {
+      *reinterpret_cast<float4*>(meet + sub * PP_MEET + 4 * lane) = make_float4(a[0], a[1], a[2], a[3]);
+      if (lane == 0) { meet[sub * PP_MEET + HD] = M; meet[sub * PP_MEET + HD + 1] = L; }
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(8 + hq), "n"(PP_SUB * 32) : "memory");
+    if (sub == 0) {
+#pragma unroll
+      for (int e = 1; e < PP_SUB; ++e) add(meet[e * PP_MEET + HD], meet[e * PP_MEET + HD + 1], *reinterpret_cast<const float4*>(meet + e * PP_MEET + 4 * lane));
+      float* rec = rec_base + hq * PART;
+      if (lane == 0) *reinterpret_cast<float4*>(rec) = make_float4(M * LN2, L, 0.f, 0.f);
+      *reinterpret_cast<float4*>(rec + 4 + 4 * lane) = make_float4(a[0], a[1], a[2], a[3]);
+    }
+    if (p.push.world == 0) {
+      head_combine<PP_SUB>(p, sq, kv, blockIdx.z, hq, sub, lane, meet);
+      return;
+    }
+  }
+  if (p.push.world > 0) ticket_combine<PP_THREADS, PP_SUB>(p, sq, kv, blockIdx.z, reinterpret_cast<float*>(state_s), tid);
 }
 
 // Prepared weights: per KV head, W = basis * coefficient scale as fp16 in the K-major, 128-byte

@@ -38,6 +38,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
+// The same for the hand-overs of a tight loop: the abort flag is only looked at once the first attempt has failed.
+__device__ __forceinline__ bool mbar_wait_soon(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try(bar, parity, TC_WAIT_HINT_NS)) return true;
+  return mbar_wait(bar, parity, abort_flag);
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }

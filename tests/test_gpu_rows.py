@@ -35,6 +35,35 @@ def test_decode_rows(n_comp, nkv, rows, streaming):
         assert (err <= 1.5e-3 + 5e-3 * want.abs()).all(), err.max()
 
 
+@pytest.mark.parametrize("n_comp,nkv,rows,streaming,scale", [
+    (300, 8, 15, True, 1.0), (300, 8, 16, True, 300.0), (300, 2, 17, True, 2e-3), (1, 1, 33, True, 300.0), (1500, 8, 1200, True, 300.0),
+    (300, 8, 28, False, 300.0), (300, 2, 29, False, 2e-3), (1, 1, 13, False, 1.0), (1500, 8, 1200, False, 300.0)])
+def test_row_blocks(n_comp, nkv, rows, streaming, scale):
+    """The ends of the blocks of sixteen rows, in one block, several blocks of a warp and all warps, with values far from one: the
+    weights are two fp16 parts and carry a streamed row's norm, which must cost neither small nor large values their digits.  Bound:
+    that of the other rows (fp16 rounding of values, weights and output), in units of the values."""
+    from shard_b200 import fused_attention_compressed
+    gc_np = random_gc(n_comp, nkv=nkv, seed=rows)
+    cache, layer = _cache(gc_np, nkv, streaming, capacity=rows + 4)
+    gc = layer._gpu_compressed
+    for name in ("sink_v", "win_v", "v_ch_f16"):           # everything that is summed, on the rows' scale
+        gc[name].mul_(scale if scale < 1 else 1.0)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda") for _ in range(2))
+    v *= scale * torch.exp2(torch.randint(-6, 1, (1, nkv, rows, 1), generator=g, device="cuda").float())
+    cache._fused_decode_update = True
+    layer.update(k.half(), v.half())
+    q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+    out = fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)
+    cache.check()
+    layer._needs_decompress = True
+    keys, values = layer.keys[0].double(), layer.values[0].double()
+    sc = torch.einsum("hqd,hnd->hqn", q[0].double(), keys.repeat_interleave(4, 0)) / 128 ** 0.5
+    want = torch.softmax(sc, -1) @ values.repeat_interleave(4, 0)
+    err = (out[0].double() - want).abs()
+    assert (err <= 1.5e-3 * scale + 5e-3 * want.abs()).all(), (err / scale).max()
+
+
 @pytest.mark.parametrize("n_comp,nkv", [(700, 8), (0, 2)])
 def test_decode_launch_writes_the_newest_fp16_row(n_comp, nkv):
     """`append = 2` of the C entry point: the launch copies new_k / new_v into the last row, then attends."""

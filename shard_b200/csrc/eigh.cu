@@ -13,14 +13,14 @@
 //                          division-free recurrence (one multiply-add of latency per row).
 //   3. tridiag_vectors_kernel  eigenvectors of the tridiagonal matrix by twisted factorisation, fp64,
 //                          thread = vector, one warp from either end.
-//   4. eig_back_kernel     the reflectors applied to the vectors, a warp per vector, two reflectors per
-//                          pass over its registers.
+//   4. eig_products_kernel, eig_back_kernel    the reflectors applied to the vectors, eight to eight vectors per pass.
 //   5. eig_check_kernel    neighbouring vectors must be orthogonal; a matrix with eigenvalues too close
 //                          for step 3 is reported to the caller.
 //
 // Bound: the latency chain of step 1 (p steps of exchange, two reductions and one pass over the matrix).
-// p = 1024, rank 192, up to seven matrices side by side: step 1 2.1 ms (4.5 ms before its column phases and
-// packed multiply-adds), steps 2 to 5 0.8 ms alone; torch.linalg.eigh takes 8 to 12 ms a matrix.
+// p = 1024, rank 192, one matrix / four side by side: step 1 2.1 ms (4.5 ms before its column phases and packed multiply-adds),
+// step 2 0.11 / 0.26 ms, step 3 0.08 ms (0.26 ms before its loads went ahead of its stores), step 4 0.19 / 0.27 ms (0.33 / 0.35),
+// step 5 0.02 ms; torch.linalg.eigh takes 8 to 12 ms a matrix.
 #include <atomic>
 #include <type_traits>
 
@@ -35,7 +35,7 @@ constexpr int EG_MAX_P = 1024;
 struct EighParams {
   const float* a;         // [L][p][p]
   int p, rank;
-  float* refl;            // [L][p][p] reflector k in row k (zeros up to k, one at k + 1)
+  float* refl;            // [L][p][p] reflector k in row k (zeros up to k, one at k + 1; the last row is zero)
   float* tau;             // [L][p]
   float* d;               // [L][p]
   float* e;               // [L][p]
@@ -43,6 +43,7 @@ struct EighParams {
   double* dplus;          // [L][blocks of 32 vectors][p][32]
   double* dminus;
   float* z;               // [L][blocks][p][32] vectors of the tridiagonal matrix
+  float* products;        // [L][p / 8][8][8] of the reflectors of a group
   float* basis;           // [L][p][rank]
   float* eigvals;         // [L][rank]
   int* flag;              // [L] 1: vectors not orthogonal, or a wait gave up
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(EG_THREADS, 1) tridiag_kernel(const __grid_con
         send_gamma(b ^ 1, 0.5f * tau * warp_sum(g));
       }
       if ((k & 15) == rank && rg == 0) {                        // the record of the step, off the critical path
-        float* o = p.refl + ((size_t)m * N + k) * N + c0 + 128 * J0;   // (retired columns are never read)
+        float* o = p.refl + ((size_t)m * N + k) * N + c0 + 128 * J0;   // (retired columns stay zero)
 #pragma unroll
         for (int j = 0; j < W; ++j) o[128 * j] = vn[j];
         if (tid == 0) {
@@ -534,132 +535,254 @@ __global__ void __launch_bounds__(64) tridiag_vectors_kernel(const __grid_consta
     double best = 1e300;
     int at = 0;
     const int lo = side ? n / 2 : 0, hi = side ? n : n / 2;
-#pragma unroll 8
-    for (int i = lo; i < hi; ++i) {
-      const double g = fabs(dp[(size_t)i * 32] + dm[(size_t)i * 32] - (td[i].x - lam));
-      if (g < best) { best = g; at = i; }
+    // (n / 2 is a multiple of 64: sixteen rows' loads in flight)
+#pragma unroll 1
+    for (int i = lo; i < hi; i += 16) {
+      double a[16], b[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) { a[j] = dp[(size_t)(i + j) * 32]; b[j] = dm[(size_t)(i + j) * 32]; }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const double g = fabs(a[j] + b[j] - (td[i + j].x - lam));
+        if (g < best) { best = g; at = i + j; }
+      }
     }
     gmin[side][lane] = best;
     gat[side][lane] = at;
   }
   __syncthreads();
   const int r = gmin[1][lane] < gmin[0][lane] ? gat[1][lane] : gat[0][lane];
+  // outwards from row r, sixteen rows at a time: the next sixteen quotients are on their way, and the reciprocals hang off the chain of
+  // products (read one by one they waited for the store of the row before: 200 cycles a row)
   float* z = p.z + base;
-  double v = 1.0;
-  if (side == 0) {
-    z[(size_t)r * 32] = 1.f;
-#pragma unroll 8
-    for (int i = n - 2; i >= 0; --i) {
-      const double f = -off_s[i] * eg_recip(dp[(size_t)i * 32]);
-      if (i < r) { v *= f; z[(size_t)i * 32] = (float)v; }
+  const double* quot = side ? dm : dp;
+  auto row_of = [&](int j) { return side ? j : n - 1 - j; };         // j = 1 .. n - 1 counts from this side's far end
+  if (side == 0) z[(size_t)r * 32] = 1.f;
+  double v = 1.0, q[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) q[j] = quot[(size_t)row_of(j) * 32];
+#pragma unroll 1
+  for (int j0 = 0; j0 < n; j0 += 16) {
+    double f[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int i = row_of(j0 + j);
+      f[j] = j0 + j ? -off_s[side ? i - 1 : i] * eg_recip(q[j]) : 0.0;
     }
-  } else {
-#pragma unroll 8
-    for (int i = 1; i < n; ++i) {
-      const double f = -off_s[i - 1] * eg_recip(dm[(size_t)i * 32]);
-      if (i > r) { v *= f; z[(size_t)i * 32] = (float)v; }
+    if (j0 + 16 < n) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) q[j] = quot[(size_t)row_of(j0 + 16 + j) * 32];
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int i = row_of(j0 + j);
+      if (side ? i > r : i < r) { v *= f[j]; z[(size_t)i * 32] = (float)v; }
     }
   }
 }
 
 // ---------------------------------------------------------------------------
-// back to the matrix's own coordinates: x = H_0 H_1 ... H_{n-3} z, a warp per vector
+// back to the matrix's own coordinates: x = H_0 H_1 ... H_{n-3} z, four vectors per CTA
 // ---------------------------------------------------------------------------
-// CB chunks of 128 rows; lane owns rows 128 j + 4 lane .. + 3.  (Two vectors per warp halve the reads of
-// the reflectors but leave too few warps to hide them: 430 against 260 us for four matrices.)  Two reflectors per pass: with
-// x' = x - t1 v1 (v1.x), v2.x' = v2.x - t1 (v1.x)(v2.v1), so the three sums go through one set of shuffles.
+// Eight reflectors per pass, k = 8 g + 7 - i for i = 0 .. 7: with y_i = v_i . x and the products G of the group's reflectors among
+// themselves, s_i = tau_i (y_i - sum over m < i of s_m G_im) and x -= sum of s_i v_i.  Element j of a thread is row 256 j + thread
+// of all four vectors; a reflector is read once for the four (a warp per vector read all of them for each: 768 warps x 2 MB,
+// 1.5 GB through L2, took 332 us for one 1024 x 1024 matrix and 352 us for four).  Pairs of vectors share packed multiply-adds.
+// 189 us for one matrix, 271 us for four (192 CTAs on 148 SMs).  Bound by a pass's chain: 32 sums over the lanes, two CTA
+// barriers, the eight-step substitution.  Eight vectors a CTA: 299 and 315 us; a thread of 128 with twice the rows: 386 us.
+constexpr int EB_V = 4, EB_G = 8;          // vectors of a CTA, reflectors of a group
+constexpr int EB_THREADS = 256;
+// products of a group's reflectors among themselves, G[m][group][i][l] = v_i . v_l for l < i; a warp per reflector
 template <int CB>
-__global__ void __launch_bounds__(128) eig_back_kernel(const __grid_constant__ EighParams p) {
+__global__ void __launch_bounds__(32 * EB_G) eig_products_kernel(const __grid_constant__ EighParams p) {
   constexpr int N = CB * 128;
-  const int m = blockIdx.y, lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (w >= p.rank) return;
-  const int n_blocks = (p.rank + 31) / 32;
-  const float* z = p.z + ((size_t)m * n_blocks + (w >> 5)) * N * 32 + (w & 31);
-  float x[CB][4];
-  float ss = 0.f;
+  const int g = blockIdx.x, m = blockIdx.y, i = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float* refl = p.refl + (size_t)m * N * N;
+  float v[4 * CB];
 #pragma unroll
-  for (int j = 0; j < CB; ++j)
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      x[j][t] = z[(size_t)(128 * j + 4 * lane + t) * 32];
-      ss = fmaf(x[j][t], x[j][t], ss);
-    }
-  const float inv = rsqrtf(warp_sum(ss));
-#pragma unroll
-  for (int j = 0; j < CB; ++j)
-#pragma unroll
-    for (int t = 0; t < 4; ++t) x[j][t] *= inv;
-  const float* refl = p.refl + (size_t)m * N * N + 4 * lane;
-  const float* tau = p.tau + (size_t)m * N;
-  float4 a[CB], b[CB];
-  auto load = [&](int k, float4 (&r)[CB]) {
-#pragma unroll
-    for (int j = 0; j < CB; ++j)
-      r[j] = (k >= 0 && 128 * (j + 1) > k + 1) ? *reinterpret_cast<const float4*>(refl + (size_t)k * N + 128 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  auto apply = [&](int k, const float4 (&a)[CB], const float4 (&b)[CB]) {
-    const float t1 = k >= 0 ? __ldg(tau + k) : 0.f, t2 = k >= 1 ? __ldg(tau + k - 1) : 0.f;
-    float s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      s1 = fmaf(a[j].x, x[j][0], fmaf(a[j].y, x[j][1], fmaf(a[j].z, x[j][2], fmaf(a[j].w, x[j][3], s1))));
-      s2 = fmaf(b[j].x, x[j][0], fmaf(b[j].y, x[j][1], fmaf(b[j].z, x[j][2], fmaf(b[j].w, x[j][3], s2))));
-      s3 = fmaf(b[j].x, a[j].x, fmaf(b[j].y, a[j].y, fmaf(b[j].z, a[j].z, fmaf(b[j].w, a[j].w, s3))));
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      s3 += __shfl_xor_sync(0xffffffffu, s3, o);
-    }
-    s1 *= t1;
-    s2 = t2 * fmaf(-s1, s3, s2);
-#pragma unroll
-    for (int j = 0; j < CB; ++j) {
-      x[j][0] = fmaf(-s2, b[j].x, fmaf(-s1, a[j].x, x[j][0]));
-      x[j][1] = fmaf(-s2, b[j].y, fmaf(-s1, a[j].y, x[j][1]));
-      x[j][2] = fmaf(-s2, b[j].z, fmaf(-s1, a[j].z, x[j][2]));
-      x[j][3] = fmaf(-s2, b[j].w, fmaf(-s1, a[j].w, x[j][3]));
-    }
-  };
-  // pairs (n - 2, n - 3), ... (reflector n - 2 is trivial: tau = 0); the next pair is on its way while one is applied
-  float4 a2[CB], b2[CB];
-  load(N - 2, a);
-  load(N - 3, b);
+  for (int j = 0; j < 4 * CB; ++j) v[j] = __ldg(refl + (size_t)(EB_G * g + EB_G - 1 - i) * N + 32 * j + lane);
 #pragma unroll 1
-  for (int k = N - 2; k >= 0; k -= 4) {
-    load(k - 2, a2);
-    load(k - 3, b2);
-    apply(k, a, b);
-    load(k - 4, a);
-    load(k - 5, b);
-    apply(k - 2, a2, b2);
+  for (int l = 0; l < i; ++l) {
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4 * CB; ++j) s = fmaf(v[j], __ldg(refl + (size_t)(EB_G * g + EB_G - 1 - l) * N + 32 * j + lane), s);
+    s = warp_sum(s);
+    if (lane == 0) p.products[(((size_t)m * (N / EB_G) + g) * EB_G + i) * EB_G + l] = s;
   }
-  float* out = p.basis + (size_t)m * N * p.rank + w;
+}
+template <int CB>
+__global__ void __launch_bounds__(EB_THREADS) eig_back_kernel(const __grid_constant__ EighParams p) {
+  constexpr int N = CB * 128, NG = N / EB_G, EL = (N + EB_THREADS - 1) / EB_THREADS, NW = EB_THREADS / 32, Q = EB_V / 2;
+  __shared__ float y_s[NW][EB_G * EB_V];   // sums of a warp's rows, [reflector][vector]
+  __shared__ __align__(16) float s_s[EB_G * EB_V];
+  __shared__ float g_s[2][EB_G * EB_G], tau_s[2][EB_G];
+  const int m = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31, w0 = blockIdx.x * EB_V;
+  const int n_blocks = (p.rank + 31) / 32;
+  const float* z = p.z + ((size_t)m * n_blocks + (w0 >> 5)) * N * 32 + (w0 & 31);
+  const float* refl = p.refl + (size_t)m * N * N;
+  const float* tau = p.tau + (size_t)m * N;
+  const float* products = p.products + (size_t)m * NG * EB_G * EB_G;
+  // 32 sums over the lanes: halve the values a lane carries; lane l ends up with value l
+  auto sums = [&](float (&a)[EB_G * EB_V], float* out) {
+    int off = 16;
 #pragma unroll
-  for (int j = 0; j < CB; ++j)
+    for (int h = EB_G * EB_V / 2; h >= 1; h >>= 1) {
+      const bool up = (lane & off) != 0;
 #pragma unroll
-    for (int t = 0; t < 4; ++t) out[(size_t)(128 * j + 4 * lane + t) * p.rank] = x[j][t];
+      for (int r = 0; r < h; ++r) {
+        const float keep = up ? a[r + h] : a[r], give = up ? a[r] : a[r + h];
+        a[r] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+      }
+      off >>= 1;
+    }
+    out[lane] = a[0];
+  };
+  auto total = [&](int i) {                // of value i, over the warps
+    float y = y_s[0][i];
+#pragma unroll
+    for (int w = 1; w < NW; ++w) y += y_s[w][i];
+    return y;
+  };
+  auto load_group = [&](int g, float (&v)[EB_G][EL]) {
+    const float* rows = refl + (size_t)(EB_G * g) * N + t;
+#pragma unroll
+    for (int i = 0; i < EB_G; ++i)
+#pragma unroll
+      for (int j = 0; j < EL; ++j)         // (an odd number of blocks: the upper half of the last 256 rows does not exist)
+        v[i][j] = (CB % 2 == 0 || j < EL - 1 || t < 128) ? __ldg(rows + (EB_G - 1 - i) * N + EB_THREADS * j) : 0.f;
+  };
+  unsigned long long x[EL][Q];             // pairs of vectors
+#pragma unroll
+  for (int j = 0; j < EL; ++j) {
+    float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (2 * j + (t >> 7) < CB) f = *reinterpret_cast<const float4*>(z + (size_t)(EB_THREADS * j + t) * 32);
+    x[j][0] = f2_pack(f.x, f.y); x[j][1] = f2_pack(f.z, f.w);
+  }
+  {                                        // to length one
+    float a[EB_G * EB_V];
+#pragma unroll
+    for (int q = 0; q < EB_G * EB_V; ++q) a[q] = 0.f;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      unsigned long long s = 0ull;
+#pragma unroll
+      for (int j = 0; j < EL; ++j) s = f2_fma(x[j][q], x[j][q], s);
+      const float2 f = f2_unpack(s);
+      a[2 * q] = f.x;
+      a[2 * q + 1] = f.y;
+    }
+    sums(a, y_s[warp]);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const unsigned long long inv = f2_pack(rsqrtf(total(2 * q)), rsqrtf(total(2 * q + 1)));
+#pragma unroll
+      for (int j = 0; j < EL; ++j) x[j][q] = f2_fma(x[j][q], inv, 0ull);
+    }
+    __syncthreads();
+  }
+  // the next group's reflectors are on their way while one is applied
+  float v[EB_G][EL];
+  load_group(NG - 1, v);
+#pragma unroll 1
+  for (int g = NG - 1; g >= 0; --g) {
+    const int j0 = g >> 5;                 // first 256 rows with a non-zero element
+    if (t < EB_G * EB_G) g_s[g & 1][t] = products[(size_t)g * EB_G * EB_G + t];
+    else if (t < EB_G * EB_G + EB_G) tau_s[g & 1][t - EB_G * EB_G] = tau[EB_G * g + EB_G - 1 - (t - EB_G * EB_G)];
+    float next[EB_G][EL];
+    load_group(max(g - 1, 0), next);
+    {
+      unsigned long long acc[EB_G][Q];
+#pragma unroll
+      for (int i = 0; i < EB_G * Q; ++i) acc[i / Q][i % Q] = 0ull;
+#pragma unroll
+      for (int j = 0; j < EL; ++j)
+        if (j >= j0) {
+#pragma unroll
+          for (int i = 0; i < EB_G; ++i) {
+            const unsigned long long vv = f2_pack(v[i][j], v[i][j]);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) acc[i][q] = f2_fma(vv, x[j][q], acc[i][q]);
+          }
+        }
+      float a[EB_G * EB_V];
+#pragma unroll
+      for (int i = 0; i < EB_G * Q; ++i) {
+        const float2 f = f2_unpack(acc[i / Q][i % Q]);
+        a[2 * i] = f.x;
+        a[2 * i + 1] = f.y;
+      }
+      sums(a, y_s[warp]);
+    }
+    __syncthreads();
+    if (t < EB_V) {                        // vector t
+      float y[EB_G];
+#pragma unroll
+      for (int i = 0; i < EB_G; ++i) y[i] = total(EB_V * i + t);
+#pragma unroll
+      for (int i = 0; i < EB_G; ++i) {
+        const float s = tau_s[g & 1][i] * y[i];
+        s_s[EB_V * i + t] = -s;
+#pragma unroll
+        for (int l = i + 1; l < EB_G; ++l) y[l] = fmaf(-s, g_s[g & 1][EB_G * l + i], y[l]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < EB_G; ++i) {
+      const ulonglong2 s2 = *reinterpret_cast<const ulonglong2*>(&s_s[EB_V * i]);
+      const unsigned long long s[Q] = {s2.x, s2.y};
+#pragma unroll
+      for (int j = 0; j < EL; ++j)
+        if (j >= j0) {
+          const unsigned long long vv = f2_pack(v[i][j], v[i][j]);
+#pragma unroll
+          for (int q = 0; q < Q; ++q) x[j][q] = f2_fma(vv, s[q], x[j][q]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < EB_G * EL; ++i) v[i / EL][i % EL] = next[i / EL][i % EL];
+  }
+  float* out = p.basis + (size_t)m * N * p.rank;
+#pragma unroll
+  for (int j = 0; j < EL; ++j)
+    if (2 * j + (t >> 7) < CB) {
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const float2 f = f2_unpack(x[j][q]);
+        float* at = out + (size_t)(EB_THREADS * j + t) * p.rank + w0 + 2 * q;
+        if (w0 + 2 * q < p.rank) at[0] = f.x;
+        if (w0 + 2 * q + 1 < p.rank) at[1] = f.y;
+      }
+    }
 }
 
 // Vectors of close eigenvalues that step 3 could not tell apart: the next two neighbours of every vector
 // must be orthogonal to it, and its length one.
-__global__ void __launch_bounds__(256) eig_check_kernel(const __grid_constant__ EighParams p) {
-  const int m = blockIdx.y, w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (w >= p.rank) return;
+// CTA = 32 vectors, lane = vector, warp = every 32nd row.
+constexpr int EC_WARPS = 32;
+__global__ void __launch_bounds__(32 * EC_WARPS) eig_check_kernel(const __grid_constant__ EighParams p) {
+  __shared__ float sum[EC_WARPS][3][32];
+  const int m = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w = blockIdx.x * 32 + lane;
   const float* v = p.basis + (size_t)m * p.p * p.rank;
+  const int w0 = min(w, p.rank - 1), w1 = min(w + 1, p.rank - 1), w2 = min(w + 2, p.rank - 1);
   float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  for (int i = lane; i < p.p; i += 32) {
+#pragma unroll 8
+  for (int i = warp; i < p.p; i += EC_WARPS) {
     const float* row = v + (size_t)i * p.rank;
-    const float a = row[w];
+    const float a = row[w0];
     s0 = fmaf(a, a, s0);
-    s1 = fmaf(a, w + 1 < p.rank ? row[w + 1] : 0.f, s1);
-    s2 = fmaf(a, w + 2 < p.rank ? row[w + 2] : 0.f, s2);
+    s1 = fmaf(a, row[w1], s1);
+    s2 = fmaf(a, row[w2], s2);
   }
-  s0 = warp_sum(s0);
-  s1 = warp_sum(s1);
-  s2 = warp_sum(s2);
-  if (lane == 0 && !(fabsf(s0 - 1.f) < 1e-3f && fabsf(s1) < 1e-3f && fabsf(s2) < 1e-3f)) p.flag[m] = 1;   // (NaN: flagged)
+  sum[warp][0][lane] = s0; sum[warp][1][lane] = s1; sum[warp][2][lane] = s2;
+  __syncthreads();
+  if (warp > 0 || w >= p.rank) return;
+#pragma unroll
+  for (int i = 1; i < EC_WARPS; ++i) { s0 += sum[i][0][lane]; s1 += sum[i][1][lane]; s2 += sum[i][2][lane]; }
+  if (w + 1 >= p.rank) s1 = 0.f;
+  if (w + 2 >= p.rank) s2 = 0.f;
+  if (!(fabsf(s0 - 1.f) < 1e-3f && fabsf(s1) < 1e-3f && fabsf(s2) < 1e-3f)) p.flag[m] = 1;   // (NaN: flagged)
 }
 
 template <int CB>
@@ -691,13 +814,14 @@ static int launch_eigh(const EighParams& p, int count, cudaStream_t st) {
   if (e != cudaSuccess) return (int)e;
   tridiag_values_kernel<<<dim3(p.rank, count), EG_PTS / 2, 0, st>>>(p);
   tridiag_vectors_kernel<<<dim3((p.rank + 31) / 32, count), 64, 0, st>>>(p);
-  eig_back_kernel<CB><<<dim3((p.rank + 3) / 4, count), 128, 0, st>>>(p);
-  eig_check_kernel<<<dim3((p.rank + 7) / 8, count), 256, 0, st>>>(p);
+  eig_products_kernel<CB><<<dim3(CB * 128 / EB_G, count), 32 * EB_G, 0, st>>>(p);
+  eig_back_kernel<CB><<<dim3((p.rank + EB_V - 1) / EB_V, count), EB_THREADS, 0, st>>>(p);
+  eig_check_kernel<<<dim3((p.rank + 31) / 32, count), 32 * EC_WARPS, 0, st>>>(p);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : (int)e;
 }
 
-struct EighLayout { size_t refl, tau, d, e, lam, dplus, dminus, z, bytes; };
+struct EighLayout { size_t refl, tau, d, e, lam, dplus, dminus, z, products, bytes; };
 static EighLayout eg_layout(size_t L, size_t p, size_t rank) {
   EighLayout l;
   auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -710,6 +834,7 @@ static EighLayout eg_layout(size_t L, size_t p, size_t rank) {
   l.dplus = l.lam + up(L * rank * 8);
   l.dminus = l.dplus + up(L * nb * p * 8);
   l.z = l.dminus + up(L * nb * p * 8);
+  l.products = l.dplus;                    // (the factorisations have been used by then)
   l.bytes = l.z + up(L * nb * p * 4);
   return l;
 }
@@ -744,11 +869,14 @@ extern "C" int shard_b200_eigh(const float* a, int32_t count, int32_t p, int32_t
   q.dplus = (double*)(ws + l.dplus);
   q.dminus = (double*)(ws + l.dminus);
   q.z = (float*)(ws + l.z);
+  q.products = (float*)(ws + l.products);
   q.basis = basis_out;
   q.eigvals = eigvals_out;
   q.flag = flag_out;
   cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = cudaMemsetAsync(flag_out, 0, (size_t)count * 4, st);
+  // (a step leaves the blocks of columns that have retired alone, and the back-transformation reads whole rows)
+  if (e == cudaSuccess) e = cudaMemsetAsync(q.refl, 0, (size_t)count * p * p * 4, st);
   if (e != cudaSuccess) return (int)e;
   switch (p / 128) {
     case 1: return launch_eigh<1>(q, count, st);

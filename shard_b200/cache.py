@@ -617,8 +617,6 @@ class Cache(HFCache):
         on a few SMs: it runs on a second stream beside the group's value path (k-means) and the next
         group's covariances; the host waits only for the eigenvalues, which decide the bit widths."""
         n_layers = self._num_layers
-        # (the state the global generator is left in: the reference seeds it for every layer's randomised SVD)
-        torch.manual_seed(42 + n_layers - 1)
         main = torch.cuda.current_stream()
         side = _second_stream(main.device)
         n_groups = -(-n_layers // EIGH_GROUP)
@@ -627,10 +625,6 @@ class Cache(HFCache):
         n, p = end - start, self._per_layer_dim
         rank = min(self._max_rank_k, p, n - 1)
         side.wait_stream(main)
-        with torch.cuda.stream(side):
-            # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
-            init_rows = initial_rows(n * p // self._v_vq_group_size, self._v_vq_codebook_size, main.device)
-            drawn = side.record_event()
         dev = main.device
         inv_freq = self._inv_freq(dev)
         cov_ws = enc_ws = None
@@ -659,13 +653,21 @@ class Cache(HFCache):
                     cov_ws = ops.k_covariance(keys(li), start, inv_freq, f, m, m16, gr, cov_ws)
             return rows, gram, main.record_event()
 
+        # The covariances first, with the eigensolver right behind them: they are the long chain.
         ready = covariances(0)
-        main.wait_event(drawn)
+        with torch.cuda.stream(side):
+            # every layer's k-means starts from the same rows (same seed, same number of sub-vectors)
+            init_rows = initial_rows(n * p // self._v_vq_group_size, self._v_vq_codebook_size, main.device)
+            drawn = side.record_event()
         for g in range(n_groups):
             rows, gram, done = ready
             side.wait_event(done)
             with torch.cuda.stream(side):
                 solved = leading_eigenpairs(gram, rank, None if cov_ws is None else ops.covariance_status(cov_ws))
+            if g == 0:
+                main.wait_event(drawn)
+                # (the state the global generator is left in: the reference seeds it for every layer's randomised SVD)
+                torch.manual_seed(42 + n_layers - 1)
             vparts = self._compress_v_layers([self.layers[li]._values[0, :, start:end, :]
                                               for li in range(bounds[g], bounds[g + 1])], init_rows=init_rows)
             ends = [self._ends(li, end) for li in range(bounds[g], bounds[g + 1])]

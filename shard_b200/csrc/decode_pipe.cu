@@ -5,9 +5,9 @@
 // One CTA per SM (16 warps) owns one KV head and a run of 128-token tiles of the middle segment.  Two pipelines take the
 // tiles in turn; each has an A slot and a key stage in tensor memory, an issuing thread and a group of four consumer warps.
 //
-//   copying threads (2) bulk copies: the weights W once, the packed int4 coefficient rows of a tile, its V codes.  No load
-//                       instruction touches the cache data.  In the CTA that owns the newest streamed row their
-//                       two warps first quantise the new token into it
+//   copying warps (2)   one thread each: bulk copies of the weights W once, the packed int4 coefficient rows of a tile, its V
+//                       codes.  No load instruction touches the cache data.  When the launch before has finished, the two warps
+//                       stage the query and, in the CTA that owns the newest streamed row, quantise the new token into it
 //   unpack warps (4)    coefficient rows -> fp16 A operand in tensor memory; then this CTA's share of the fp16 sink / window /
 //                       decode rows and the streamed rows, sixteen at a time
 //   issuing threads (2) MMA1  K_n[128 tok x 128] = A . W^T   (A from tensor memory, W in shared memory; the last k-step adds the
@@ -27,12 +27,13 @@
 // instead: a stream of tcgen05.mma keeps mma.sync waiting, so the consumers' products run between the reconstruction
 // products of two tiles.  That, with the latency of a consumer's chain (tensor memory, rotation, scores, softmax, look-ups, P.V: about
 // 3 K cycles), bounds a tile: 2.7 K cycles.  Against the kernel with all products on tcgen05, shared-memory V tiles and three groups
-// (us a pass): 8K x 12 layers 197 -> 161, 32K x 12 383 -> 345, 131K x 4 408 -> 360, 64 sequences of 8K x 2 923 -> 742.
+// (us a pass): 8K x 12 layers 198 -> 162, 32K x 12 383 -> 324, 131K x 4 408 -> 354, 64 sequences of 8K x 2 923 -> 738.
 // Measured and not kept: eight warps to a tile (80 registers: 8K 197, 131K 377), one paced issuing thread, the stage
 // handed back before the scores product, polling instead of suspended waits (131K 396).
 //
-// Launched with programmatic stream serialization: the set-up, the first tiles' unpack and reconstruction products use only
-// tensors that no decode call writes and run before griddepcontrol.wait.
+// Launched with programmatic stream serialization: the set-up, the first tiles' unpack and reconstruction products and the rotation of
+// each group's first keys (which wait for the query in registers: 32K x 12 345 -> 324 us, 131K x 4 360 -> 354) use only tensors that no
+// decode call writes and run before griddepcontrol.wait.
 //
 // Tensor memory: two key stages of 128 columns, two A slots of R/2 + 8 columns from column 256 on.
 // Every hand-over is an mbarrier whose waiters see each of its phases; every wait is bounded and
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   } else if (tid == PP_MMA_WARP * 32) {
     for (int s = 0; s < PP_ST; ++s) { mbar_init(KN_FULL(s), 1); mbar_init(KN_EMPTY(s), 4); mbar_init(A_FULL(s), 4); mbar_init(MMA_DONE(s), 1); }
     mbar_init(CB_READY, PP_CONS_WARPS);
-    mbar_init(Q_READY, PP_CONS_WARPS);
+    mbar_init(Q_READY, 2);
     mbar_init(APPEND_DONE, 2);
     mbar_init(QS_READY, 4);
     *abort_s = 0;
@@ -545,10 +546,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       __syncwarp();
       if (lane == 0) mbar_arrive(CB_READY);
     }
-    const float phq = __fmul_rn((float)sh.pos_q, p.inv_freq[tid & 63]);
-    float snq, csq;
-    sincosf(phq, &snq, &csq);
-    const __half c16 = __float2half_rn(csq), s16 = __float2half_rn(snq);
     // cos / sin of the rows, laid out as the fragments want them (phase_table_kernel); step i of a tile takes pairs
     // 16 (i / 2) .. + 15 of rows 16 (i % 2) .. + 15; loaded four steps ahead
     const uint4* phase_tab = reinterpret_cast<const uint4*>(sq.phase) + lane;
@@ -560,37 +557,56 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       ph[i][0] = pr[((2 * (i & 1)) * 4 + (i >> 1)) * 32];
       ph[i][1] = pr[((2 * (i & 1) + 1) * 4 + (i >> 1)) * 32];
     };
+    const uint32_t kn = tmem_base + (uint32_t)(128 * grp) + ((uint32_t)(32 * quad) << 16);       // the warp's rows of its key stage
+    auto load_keys = [&](int i, uint32_t* r) {        // columns of step i: 16 of the first half of the channels, the same 16 of the second
+      const uint32_t at = kn + ((uint32_t)(16 * (i & 1)) << 16) + 16 * (i >> 1);
+      tmem_ld_frag(at, r);
+      tmem_ld_frag(at + 64, r + 8);
+    };
+    // keys of step i, half k, rotated by the relative phase: an A fragment of the scores product
+    auto rotate = [&](const uint32_t* r, int i, int k, uint32_t (&a)[4]) {
+#pragma unroll
+      for (int rr = 0; rr < 2; ++rr) {                // rows g8, g8 + 8
+        const __half2 c2 = __floats2half2_rn(__uint_as_float(r[4 * k + 2 * rr]), __uint_as_float(r[4 * k + 2 * rr + 1]));
+        const __half2 d2 = __floats2half2_rn(__uint_as_float(r[8 + 4 * k + 2 * rr]), __uint_as_float(r[8 + 4 * k + 2 * rr + 1]));
+        const __half2 cs = as_half2(k ? ph[i][rr].z : ph[i][rr].x), sn = as_half2(k ? ph[i][rr].w : ph[i][rr].y);
+        a[rr] = as_u32(__hfma2(c2, cs, __hneg2(__hmul2(d2, sn))));           // c cos - d sin
+        a[2 + rr] = as_u32(__hfma2(d2, cs, __hmul2(c2, sn)));                // d cos + c sin
+      }
+    };
+    // the group's first tile: its keys are rotated here and wait in registers for the query
+    uint32_t first[8][2][4];
     if (n_use > 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) load_phase(i, prow);
+      const uint4* pnext = phase_of(min(grp + PP_ST, n_my - 1));
+      ok = __all_sync(0xffffffffu, mbar_wait_soon(KN_FULL(grp), 0u, abort_s));
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint32_t r[16];
+        load_keys(i, r);
+        tmem_wait_frags(r);
+        rotate(r, i, 0, first[i][0]);
+        rotate(r, i, 1, first[i][1]);
+        load_phase((i + 4) & 7, i < 4 ? prow : pnext);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(KN_EMPTY(grp));
+      prow = pnext;
     }
     // Up to here only tensors that no decode call ever writes were touched (weights, coefficients, V codes,
     // codebooks) and the phase table, complete before any CTA of this launch starts: the kernel that writes it never
-    // releases its dependents early.  All this, and the first tiles' unpack and reconstruction products, runs
+    // releases its dependents early.  All this, the first tiles' unpack and reconstruction products among it, runs
     // while the launch before this one is still finishing.  The query, the new token, the stream rows, the scratch
     // and the output may come from, or still be in use by, that launch: every role waits before it touches them.
+    // (The copying warps stage the query: these may still be at their first tile when the launch before has finished.)
     griddep_wait();
-    {
-      // un-rotated queries (fp16 arithmetic as the reference): thread = (pair i, one or two heads)
-      const int i = tid & 63;
-      const __half* qg = reinterpret_cast<const __half*>(sq.q) + (size_t)kv * GQA * HD;
-#pragma unroll
-      for (int h = tid >> 6; h < GQA; h += PP_CONS_WARPS / 2) {
-        const __half x_lo = qg[h * HD + i], x_hi = qg[h * HD + i + 64];
-        __half* f = reinterpret_cast<__half*>(smem_raw + PP_OFF_QF) + ((i >> 3) * 16 + 4 * h + ((i & 7) >> 1)) * 4 + (i & 1);
-        f[0] = __hsub(__hmul(x_lo, c16), __hmul(__hneg(x_hi), s16));
-        f[2] = __hsub(__hmul(x_hi, c16), __hmul(x_lo, s16));
-        qg_s[h * HD + i] = x_lo;
-        qg_s[h * HD + i + 64] = x_hi;
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(Q_READY);
-    }
-    ok = __all_sync(0xffffffffu, mbar_wait(CB_READY, 0u, abort_s) && mbar_wait(Q_READY, 0u, abort_s));
+    ok = __all_sync(0xffffffffu, ok && mbar_wait(CB_READY, 0u, abort_s) && mbar_wait(Q_READY, 0u, abort_s));
     const uint2* qf_s = reinterpret_cast<const uint2*>(smem_raw + PP_OFF_QF) + (g8 >> 1) * 4 + t4;
     const uint32_t v_u = smem_u32(smem_raw + PP_OFF_V);
     const uint32_t cb_lane = cb_u + (uint32_t)(lane & (PP_CB_COPIES - 1)) * 8u;
-    const uint32_t lane_off = (uint32_t)(32 * quad) << 16;
     const uint32_t sel0 = (g8 & 1) ? 0x1044u : 0x4410u, sel1 = (g8 & 1) ? 0x3244u : 0x4432u;
     float run_m = neg_inf(), run_l = 0.f;             // of query head t4; log2 domain
     float o[4][4];
@@ -599,54 +615,26 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
 #pragma unroll
       for (int j = 0; j < 4; ++j) o[i][j] = 0.f;
 
-#pragma unroll 1
-    for (int use = 0; use < n_use && ok; ++use) {
-      const int it = grp + use * PP_ST, s = grp;
-      const uint4* pnext = phase_of(min(it + PP_ST, n_my - 1));
-      ok = __all_sync(0xffffffffu, mbar_wait_soon(KN_FULL(s), (uint32_t)(use & 1), abort_s));
-      if (!ok) break;
-      tc_fence_after();
-      // ---- keys: rotate by the relative phase, straight into the A fragments of the scores product -----------
-      const uint32_t kn = tmem_base + (uint32_t)(128 * s) + lane_off;
-      float sc[2][2][4];                              // two sums of each, so that one product does not wait for the last
+    float sc[2][2][4];                                // scores: two sums of each, so that one product does not wait for the last
+    auto clear_scores = [&]() {
 #pragma unroll
       for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int j = 0; j < 4; ++j) sc[b >> 1][b & 1][j] = 0.f;
-      uint2 qf[2];
-      uint32_t kr[2][16];
-      tmem_ld_frag(kn, kr[0]);
-      tmem_ld_frag(kn + 64, kr[0] + 8);
+    };
+    clear_scores();
+    if (n_use > 0 && ok) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        uint32_t* r = kr[i & 1];
-        tmem_wait_frags(r);
-        if (i < 7) {
-          const uint32_t at = kn + ((uint32_t)(16 * ((i + 1) & 1)) << 16) + 16 * ((i + 1) >> 1);
-          tmem_ld_frag(at, kr[(i + 1) & 1]);
-          tmem_ld_frag(at + 64, kr[(i + 1) & 1] + 8);
-        } else {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(KN_EMPTY(s));
-        }
-        load_phase((i + 4) & 7, i < 4 ? prow : pnext);
-        if ((i & 1) == 0) { qf[0] = qf_s[16 * i]; qf[1] = qf_s[16 * i + 16]; }
+      for (int i = 0; i < 8; ++i)
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-          uint32_t a[4];
-#pragma unroll
-          for (int rr = 0; rr < 2; ++rr) {            // rows g8, g8 + 8
-            const __half2 c2 = __floats2half2_rn(__uint_as_float(r[4 * k + 2 * rr]), __uint_as_float(r[4 * k + 2 * rr + 1]));
-            const __half2 d2 = __floats2half2_rn(__uint_as_float(r[8 + 4 * k + 2 * rr]), __uint_as_float(r[8 + 4 * k + 2 * rr + 1]));
-            const __half2 cs = as_half2(k ? ph[i][rr].z : ph[i][rr].x), sn = as_half2(k ? ph[i][rr].w : ph[i][rr].y);
-            a[rr] = as_u32(__hfma2(c2, cs, __hneg2(__hmul2(d2, sn))));       // c cos - d sin
-            a[2 + rr] = as_u32(__hfma2(d2, cs, __hmul2(c2, sn)));            // d cos + c sin
-          }
-          mma_16816(sc[i & 1][k], a[0], a[1], a[2], a[3], qf[k].x, qf[k].y);
+          const uint2 qf = qf_s[16 * (2 * (i >> 1) + k)];
+          mma_16816(sc[i & 1][k], first[i][k][0], first[i][k][1], first[i][k][2], first[i][k][3], qf.x, qf.y);
         }
-      }
-      prow = pnext;
+    }
+#pragma unroll 1
+    for (int use = 0; use < n_use && ok; ) {
+      const int it = grp + use * PP_ST;
       // ---- V codes of the tile: row 8 m + 2 t4 (+ 1), codes 4 g8 .. + 3 ----------------------------------------
       const int vb = it % PP_V_BUFS;
       ok = __all_sync(0xffffffffu, mbar_wait_soon(V_FULL(vb), (uint32_t)((it / PP_V_BUFS) & 1), abort_s));
@@ -701,6 +689,37 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(V_EMPTY(vb));
+      if (++use == n_use) break;
+      // ---- keys of the next tile: rotated straight into the A fragments of its scores product -------------------
+      const uint4* pnext = phase_of(min(it + 2 * PP_ST, n_my - 1));
+      ok = __all_sync(0xffffffffu, mbar_wait_soon(KN_FULL(grp), (uint32_t)(use & 1), abort_s));
+      if (!ok) break;
+      tc_fence_after();
+      clear_scores();
+      uint2 qf[2];
+      uint32_t kr[2][16];
+      load_keys(0, kr[0]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        uint32_t* r = kr[i & 1];
+        tmem_wait_frags(r);
+        if (i < 7) {
+          load_keys(i + 1, kr[(i + 1) & 1]);
+        } else {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(KN_EMPTY(grp));
+        }
+        load_phase((i + 4) & 7, i < 4 ? prow : pnext);
+        if ((i & 1) == 0) { qf[0] = qf_s[16 * i]; qf[1] = qf_s[16 * i + 16]; }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          uint32_t a[4];
+          rotate(r, i, k, a);
+          mma_16816(sc[i & 1][k], a[0], a[1], a[2], a[3], qf[k].x, qf[k].y);
+        }
+      }
+      prow = pnext;
     }
     // the warp's state: this lane has channels 16 g8 .. + 15 of query head t4, in units of the channels' scales
     {
@@ -796,10 +815,31 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     griddep_wait();
   } else {
     // =============================== copying warps ========================================
-    // In the CTA that owns the newest streamed row they first quantise the new token into it (bit-identical to
+    // First the query, and in the CTA that owns the newest streamed row the new token, quantised into it (bit-identical to
     // stream_quantize_kernel); the copies asked for so far last meanwhile.
-    if (append_here) {
+    {
+      // un-rotated queries (fp16 arithmetic as the reference): thread = pair i of all heads
+      const int i = (warp - PP_COEF_WARP) * 32 + lane;
+      float sn, cs;
+      sincosf(__fmul_rn((float)sh.pos_q, p.inv_freq[i]), &sn, &cs);
+      const __half c16 = __float2half_rn(cs), s16 = __float2half_rn(sn);
+      const __half* qg = reinterpret_cast<const __half*>(sq.q) + (size_t)kv * GQA * HD;
+      __half x_lo[GQA], x_hi[GQA];
       griddep_wait();
+#pragma unroll
+      for (int h = 0; h < GQA; ++h) { x_lo[h] = qg[h * HD + i]; x_hi[h] = qg[h * HD + i + 64]; }
+#pragma unroll
+      for (int h = 0; h < GQA; ++h) {
+        __half* f = reinterpret_cast<__half*>(smem_raw + PP_OFF_QF) + ((i >> 3) * 16 + 4 * h + ((i & 7) >> 1)) * 4 + (i & 1);
+        f[0] = __hsub(__hmul(x_lo[h], c16), __hmul(__hneg(x_hi[h]), s16));
+        f[2] = __hsub(__hmul(x_hi[h], c16), __hmul(x_lo[h], s16));
+        qg_s[h * HD + i] = x_lo[h];
+        qg_s[h * HD + i + 64] = x_hi[h];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(Q_READY);
+    }
+    if (append_here) {
       ok = __all_sync(0xffffffffu, mbar_wait(CB_READY, 0u, abort_s));
       if (ok) append_new_token(sq, sh, kv, cbs_s, warp == PP_VCODE_WARP, lane);
       __syncwarp();
@@ -817,7 +857,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       }
     }
     __syncwarp();
-    griddep_wait();
   }
 
   // ---- rows: this warp's share of the blocks, taken to the rotated space of the middle's accumulator.  (Some rows behind every tile

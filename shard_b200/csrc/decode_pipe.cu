@@ -156,6 +156,17 @@ __device__ __forceinline__ uint32_t split_half2(float x) {
   const __half hi = __float2half_rn(x), lo = __float2half_rn(x - __half2float(hi));
   return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
+// 16 bytes, L2-coherent, in pieces of PIECE bytes where the address is no multiple of 16
+template <int PIECE>
+__device__ __forceinline__ uint4 row_load16(const void* at, bool aligned) {
+  if (aligned) return __ldcg(reinterpret_cast<const uint4*>(at));
+  if (PIECE == 8) {
+    const uint2 a = __ldcg(reinterpret_cast<const uint2*>(at)), b = __ldcg(reinterpret_cast<const uint2*>(at) + 1);
+    return make_uint4(a.x, a.y, b.x, b.y);
+  }
+  const unsigned int* w = reinterpret_cast<const unsigned int*>(at);
+  return make_uint4(__ldcg(w), __ldcg(w + 1), __ldcg(w + 2), __ldcg(w + 3));
+}
 // one query head as given -> the code space, fp16 parts out[0..127] and out[128..255]; one warp
 __device__ __forceinline__ void stream_query(const float* __restrict__ signs, const __half* q, __half* out, int lane) {
   const uint2 raw = *reinterpret_cast<const uint2*>(q + 4 * lane);
@@ -202,21 +213,22 @@ __device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2]
 __device__ __forceinline__ void fp16_block(RowState& st, const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u0, const __half* qg_s, int lane) {
   const int g8 = lane >> 2, t4 = lane & 3, last = sh.n_sink + sh.n_win + sh.n_dec - 1;
   // keys: channels 32 j + 8 t4 .. + 7 of rows g8 and g8 + 8; values: channels 16 g8 .. + 15 of rows 2 t4, 2 t4 + 1, and 8 further
-  // (8-byte loads: the rows may start between 16-byte boundaries; L2-coherent: the newest row may be this CTA's.  A row behind the
-  // last repeats it and gets no weight.)
-  uint2 k[2][8], v[4][4];
+  // (the rows may start between 16-byte boundaries; L2-coherent: the newest row may be this CTA's.  A row behind the last repeats it
+  // and gets no weight.)
+  uint4 k[2][4], v[4][2];
   const __half *kp, *vp;
+  const bool aligned = (((uintptr_t)sq.sink_k | (uintptr_t)sq.sink_v | (uintptr_t)sq.win_k | (uintptr_t)sq.win_v | (uintptr_t)sq.dec_k | (uintptr_t)sq.dec_v) & 15) == 0;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     fp16_row(sq, sh, kv, min(u0 + g8 + 8 * r, last), kp, vp);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) k[r][j] = __ldcg(reinterpret_cast<const uint2*>(kp + 32 * (j >> 1) + 8 * t4 + 4 * (j & 1)));
+    for (int j = 0; j < 4; ++j) k[r][j] = row_load16<8>(kp + 32 * j + 8 * t4, aligned);
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     fp16_row(sq, sh, kv, min(u0 + 8 * (r >> 1) + 2 * t4 + (r & 1), last), kp, vp);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[r][i] = __ldcg(reinterpret_cast<const uint2*>(vp + 16 * g8 + 4 * i));
+    for (int i = 0; i < 2; ++i) v[r][i] = row_load16<8>(vp + 16 * g8 + 8 * i, aligned);
   }
   float s[2][4];
 #pragma unroll
@@ -224,8 +236,8 @@ __device__ __forceinline__ void fp16_block(RowState& st, const ShardSeq& sq, con
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const uint4 q = *reinterpret_cast<const uint4*>(qg_s + (g8 >> 1) * HD + 32 * j + 8 * t4);
-    mma_16816(s[0], k[0][2 * j].x, k[1][2 * j].x, k[0][2 * j].y, k[1][2 * j].y, q.x, q.y);
-    mma_16816(s[1], k[0][2 * j + 1].x, k[1][2 * j + 1].x, k[0][2 * j + 1].y, k[1][2 * j + 1].y, q.z, q.w);
+    mma_16816(s[0], k[0][j].x, k[1][j].x, k[0][j].y, k[1][j].y, q.x, q.y);
+    mma_16816(s[1], k[0][j].z, k[1][j].z, k[0][j].w, k[1][j].w, q.z, q.w);
   }
   float sc[2];
   const float lv[2] = {0.f, 0.f};
@@ -238,8 +250,11 @@ __device__ __forceinline__ void fp16_block(RowState& st, const ShardSeq& sq, con
 #pragma unroll
     for (int part = 0; part < 2; ++part)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        mma_16816(st.o[i], v[2 * m][i].x, v[2 * m][i].y, v[2 * m + 1][i].x, v[2 * m + 1][i].y, w[part][m][0], w[part][m][1]);
+      for (int i = 0; i < 4; ++i) {
+        const uint4 a = v[2 * m][i >> 1], b = v[2 * m + 1][i >> 1];
+        if (i & 1) mma_16816(st.o[i], a.z, a.w, b.z, b.w, w[part][m][0], w[part][m][1]);
+        else mma_16816(st.o[i], a.x, a.y, b.x, b.y, w[part][m][0], w[part][m][1]);
+      }
 }
 // four codes -> the two fp16 parts of their codebook entries, part p of entries (0, 1) in x[p][0] and of (2, 3) in x[p][1]
 __device__ __forceinline__ void split_values(uint32_t codes, uint32_t split, uint32_t (&x)[2][2]) {
@@ -256,42 +271,48 @@ __device__ __forceinline__ void split_values(uint32_t codes, uint32_t split, uin
 __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u0, const __half* qs_s,
                                              uint32_t split, int lane) {
   const int g8 = lane >> 2, t4 = lane & 3, last = sh.n_stream - 1;
-  uint32_t k[2][8], v[4][4];
-  float kn[2], lv[2];
+  // keys: channels 32 t4 .. + 31 of rows g8 and g8 + 8; values: channels 16 g8 .. + 15 of rows 2 t4, 2 t4 + 1, and 8 further.  All loads
+  // before the first use of one, and 16 bytes wide: with the norms converted where they were read, the block began with three round
+  // trips to L2 instead of one, and 32 loads of 4 bytes, eight rows each, kept the L1 busy: 2.8 K of a block's 8 K cycles.
+  uint4 k[2][2], v[4];
+  unsigned short kn[2], vn[2];
+  const bool aligned = (((uintptr_t)sq.st_k_idx | (uintptr_t)sq.st_v_idx) & 15) == 0;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
     const size_t row = (size_t)min(u0 + g8 + 8 * r, last) * sh.nkv + kv;
+    kn[r] = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row);
+    vn[r] = __ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) k[r][j] = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_k_idx + row * HD + 32 * (j >> 1) + 8 * t4 + 4 * (j & 1)));
-    kn[r] = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_k_norm) + row)));
-    lv[r] = __log2f(__half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(sq.st_v_norm) + row))));
+    for (int j = 0; j < 2; ++j) k[r][j] = row_load16<4>(sq.st_k_idx + row * HD + 32 * t4 + 16 * j, aligned);
   }
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const size_t row = (size_t)min(u0 + 8 * (r >> 1) + 2 * t4 + (r & 1), last) * sh.nkv + kv;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[r][i] = __ldcg(reinterpret_cast<const unsigned int*>(sq.st_v_idx + row * HD + 16 * g8 + 4 * i));
+    v[r] = row_load16<4>(sq.st_v_idx + row * HD + 16 * g8, aligned);
   }
+  auto word = [](const uint4& x, int i) { return i == 0 ? x.x : i == 1 ? x.y : i == 2 ? x.z : x.w; };
   // columns 2 h and 2 h + 1 are the two parts of query head h: their sum is the score
   float s[2][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] = 0.f;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const uint4 q = *reinterpret_cast<const uint4*>(qs_s + g8 * HD + 32 * j + 8 * t4);
+    const uint4 q = *reinterpret_cast<const uint4*>(qs_s + g8 * HD + 32 * t4 + 8 * j);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t x0[2][2], x1[2][2];
-      split_values(k[0][2 * j + h], split, x0);
-      split_values(k[1][2 * j + h], split, x1);
+      split_values(word(k[0][j >> 1], 2 * (j & 1) + h), split, x0);
+      split_values(word(k[1][j >> 1], 2 * (j & 1) + h), split, x1);
 #pragma unroll
       for (int part = 0; part < 2; ++part) mma_16816(s[part], x0[part][0], x1[part][0], x0[part][1], x1[part][1], h ? q.z : q.x, h ? q.w : q.y);
     }
   }
-  float sc[2];
+  float sc[2], lv[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) lv[r] = __log2f(__half2float(__ushort_as_half(vn[r])));
 #pragma unroll
   for (int r = 0; r < 2; ++r)
-    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * kn[r] * (INV_SQRT_HD * LOG2E) : neg_inf();
+    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * __half2float(__ushort_as_half(kn[r])) * (INV_SQRT_HD * LOG2E) : neg_inf();
   uint32_t w[2][2][2];
   block_weights(st, sc, lv, w, lane);
 #pragma unroll
@@ -299,8 +320,8 @@ __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, c
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       uint32_t x0[2][2], x1[2][2];
-      split_values(v[2 * m][i], split, x0);
-      split_values(v[2 * m + 1][i], split, x1);
+      split_values(word(v[2 * m], i), split, x0);
+      split_values(word(v[2 * m + 1], i), split, x1);
 #pragma unroll
       for (int part = 0; part < 4; ++part)
         mma_16816(st.o[i], x0[part >> 1][0], x0[part >> 1][1], x1[part >> 1][0], x1[part >> 1][1], w[part & 1][m][0], w[part & 1][m][1]);
@@ -331,12 +352,12 @@ __device__ __forceinline__ void row_sums_fwht(RowState& st, int lane) {
 }
 // the streamed sums out of the code space
 __device__ __forceinline__ void stream_sums_back(RowState& st, const float* __restrict__ signs, int lane) {
+  float4 sg[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sg[i] = __ldg(reinterpret_cast<const float4*>(signs + 16 * (lane >> 2) + 4 * i));
   row_sums_fwht(st, lane);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float4 sg = *reinterpret_cast<const float4*>(signs + 16 * (lane >> 2) + 4 * i);
-    st.o[i][0] *= sg.x; st.o[i][1] *= sg.y; st.o[i][2] *= sg.z; st.o[i][3] *= sg.w;
-  }
+  for (int i = 0; i < 4; ++i) { st.o[i][0] *= sg[i].x; st.o[i][1] *= sg[i].y; st.o[i][2] *= sg[i].z; st.o[i][3] *= sg[i].w; }
 }
 // into the rotated space, and out to the epilogue as a warp's state (acc[4][128], max[4], sum-exp[4]); `merge`: joined with the state
 // that the warp has there from its tiles

@@ -64,6 +64,39 @@ def test_row_blocks(n_comp, nkv, rows, streaming, scale):
     assert (err <= 1.5e-3 * scale + 5e-3 * want.abs()).all(), (err / scale).max()
 
 
+@pytest.mark.parametrize("streaming", [True, False])
+def test_rows_between_16_byte_boundaries(streaming):
+    """Rows that start 8 bytes (fp16) or 4 bytes (codes) behind a 16-byte boundary are read in pieces: the same result to the bit."""
+    from shard_b200 import fused_attention_compressed
+
+    def shifted(x, by):
+        room = torch.zeros(x.numel() + 64, dtype=x.dtype, device=x.device)
+        y = room[by:by + x.numel()].view(x.shape)
+        y.copy_(x)
+        return y
+
+    outs = []
+    g = torch.Generator(device="cuda").manual_seed(3)
+    k, v, q = (torch.randn(1, h, n, 128, generator=g, device="cuda").half() for h, n in ((2, 45), (2, 45), (8, 1)))
+    for shift in (False, True):
+        cache, layer = _cache(random_gc(300, nkv=2, seed=9), 2, streaming, capacity=64)
+        gc = layer._gpu_compressed
+        cache._fused_decode_update = True
+        layer.update(k, v)
+        if shift:
+            for name in ("sink_k", "sink_v", "win_k", "win_v"):
+                gc[name] = shifted(gc[name], 4)
+            for name in ("k_idx_buf", "v_idx_buf") if streaming else ():
+                gc[name] = shifted(gc[name], 4)
+            gc.pop("_launch", None)
+            gc.pop("_native", None)
+        outs.append(fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq))
+        cache.check()
+        if shift:
+            assert gc["sink_k"].data_ptr() % 16 == 8 and (not streaming or gc["k_idx_buf"].data_ptr() % 16 == 4)
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("n_comp,nkv", [(700, 8), (0, 2)])
 def test_decode_launch_writes_the_newest_fp16_row(n_comp, nkv):
     """`append = 2` of the C entry point: the launch copies new_k / new_v into the last row, then attends."""

@@ -43,8 +43,13 @@ struct DecodeParams {
   PeerPush push;        // sequence-split: deliver the combined record to every rank's exchange buffer
 };
 
-// release and acquire at device scope (lighter than the sequentially consistent __threadfence)
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// add that releases what this thread's warp has written and acquires what the others had written before theirs (lighter than
+// sequentially consistent fences around a plain one)
+__device__ __forceinline__ unsigned int atomic_add_acq_rel(unsigned int* at, unsigned int v) {
+  unsigned int old;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(at), "r"(v) : "memory");
+  return old;
+}
 
 struct SoftmaxState {
   float m[GQA];
@@ -417,15 +422,12 @@ __device__ __forceinline__ void head_combine(const DecodeParams& p, const ShardS
     __syncwarp();
     if (lane == 0) {
       unsigned int* ctr = reinterpret_cast<unsigned int*>(p.tickets) + b * p.sh.nkv + kv;
-      fence_acq_rel_gpu();
-      last = ((atomicAdd(ctr, 1u << (8 * hq)) >> (8 * hq)) & 255u) == (unsigned int)(p.n_ctas - 1);
-      if (last) {
-        fence_acq_rel_gpu();
-        atomicSub(ctr, (unsigned int)p.n_ctas << (8 * hq));   // (nobody looks at it before the next launch)
-      }
+      last = ((atomic_add_acq_rel(ctr, 1u << (8 * hq)) >> (8 * hq)) & 255u) == (unsigned int)(p.n_ctas - 1);
+      if (last) atomicSub(ctr, (unsigned int)p.n_ctas << (8 * hq));   // (nobody looks at it before the next launch)
       last_of[hq] = last;
     }
     last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();                                        // (the records that lane 0 has acquired are read by all)
   }
   if (p.n_parts > HEAD_PARTS) {                          // (the head's other warps are needed)
     asm volatile("bar.sync %0, %1;" ::"r"(8 + hq), "r"(NSUB * 32) : "memory");

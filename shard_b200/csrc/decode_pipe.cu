@@ -73,6 +73,7 @@ __host__ __device__ constexpr int pp_c_bytes(int nw) { return nw < 2 ? 2560 : 12
 // Shared memory, by address within the CTA's window.  The codebook sits on a multiple of 32 KB, so that a
 // look-up's address is (code's bits | this lane's base): one shift and one three-input logic operation.
 constexpr int PP_OFF_MISC = 0;                                        // barriers, flags
+constexpr int PP_OFF_CH = 640;                                        // the head's channel scales, fp16 [128]
 constexpr int PP_OFF_QG = 1024;                                       // queries as given, fp16 [4][128]
 constexpr int PP_OFF_QS = PP_OFF_QG + GQA * HD * 2;                   // queries in the stream's code space, two fp16 parts [4][2][128]
 constexpr int PP_OFF_QF = PP_OFF_QS + GQA * HD * 4;                   // un-rotated queries as matrix fragments [8 k-steps][4 q x 4][2 x half2]
@@ -167,11 +168,10 @@ __device__ __forceinline__ uint4 row_load16(const void* at, bool aligned) {
   const unsigned int* w = reinterpret_cast<const unsigned int*>(at);
   return make_uint4(__ldcg(w), __ldcg(w + 1), __ldcg(w + 2), __ldcg(w + 3));
 }
-// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255]; one warp
-__device__ __forceinline__ void stream_query(const float* __restrict__ signs, const __half* q, __half* out, int lane) {
+// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255]; one warp, `sg` its lanes' four signs
+__device__ __forceinline__ void stream_query(const float4 sg, const __half* q, __half* out, int lane) {
   const uint2 raw = *reinterpret_cast<const uint2*>(q + 4 * lane);
   const float2 a = __half22float2(as_half2(raw.x)), c = __half22float2(as_half2(raw.y));
-  const float4 sg = *reinterpret_cast<const float4*>(signs + 4 * lane);
   float x[4] = {a.x * sg.x, a.y * sg.y, c.x * sg.z, c.y * sg.w};
   fwht128_lane4(x, lane);
   uint32_t sp[4];
@@ -564,6 +564,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
 #pragma unroll
         for (int j = 0; j < PP_SPLIT_COPIES / 4; ++j) split_s[PP_SPLIT_COPIES / 4 * tid + ((j + (lane >> 1)) & (PP_SPLIT_COPIES / 4 - 1))] = make_uint4(sp, sp, sp, sp);
       }
+      if (tid < 32) *reinterpret_cast<uint2*>(smem_raw + PP_OFF_CH + 8 * lane) = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.v_ch) + kv * HD + 4 * lane);
       __syncwarp();
       if (lane == 0) mbar_arrive(CB_READY);
     }
@@ -751,7 +752,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       if (g8 == 0) { st[GQA * HD + t4] = run_m; st[GQA * HD + GQA + t4] = l; }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint2 cw = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.v_ch) + kv * HD + 16 * g8 + 4 * i);
+        const uint2 cw = *reinterpret_cast<const uint2*>(smem_raw + PP_OFF_CH + 2 * (16 * g8 + 4 * i));
         const float2 ca = __half22float2(as_half2(cw.x)), cb = __half22float2(as_half2(cw.y));
         *reinterpret_cast<float4*>(st + t4 * HD + 16 * g8 + 4 * i) = make_float4(o[i][0] * ca.x, o[i][1] * ca.y, o[i][2] * cb.x, o[i][3] * cb.y);
       }
@@ -887,11 +888,13 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
     RowState st;
     row_state_init(st);
     if (ok && p.n_row_parts > 0) {
+      float4 sg = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (blocks_s > 0 && row_w < 4) sg = *reinterpret_cast<const float4*>(sq.signs + 4 * lane);
       ok = __all_sync(0xffffffffu, mbar_wait(Q_READY, 0u, abort_s));
       if (ok && blocks_s > 0) {
         // the unpack warps take a query head each to the code space; the others wait for them
         if (row_w < 4) {
-          stream_query(sq.signs, qg_s + row_w * HD, qs_s + row_w * 2 * HD, lane);
+          stream_query(sg, qg_s + row_w * HD, qs_s + row_w * 2 * HD, lane);
           __syncwarp();
           if (lane == 0) mbar_arrive(QS_READY);
         }

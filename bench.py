@@ -99,15 +99,29 @@ class ClockSampler:
         self.gpu = gpu_index
         self.proc = None
         self.path = None
+        self.skip = 0
+
+    def lines(self):
+        with open(self.path) as f:
+            return f.read().split("\n")[:-1]              # (the last piece is empty or a line that is being written)
+
+    def mark(self):
+        """The timed region begins: samples from before do not count unless there are no others."""
+        if self.proc is not None:
+            self.skip = len(self.lines())
 
     def start(self):
+        """Returns when the first sample is there (the tool takes longer to start than a short region lasts)."""
         try:
             fd, self.path = tempfile.mkstemp(suffix=".csv")
             os.close(fd)
             self.proc = subprocess.Popen(
                 ["nvidia-smi", "-i", str(self.gpu), f"--query-gpu={self.FIELDS}",
-                 "--format=csv,noheader,nounits", "-lms", "20"],
+                 "--format=csv,noheader,nounits", "-lms", "5"],
                 stdout=open(self.path, "w"), stderr=subprocess.DEVNULL)
+            end = time.perf_counter() + 3.0
+            while time.perf_counter() < end and self.proc.poll() is None and not self.lines():
+                time.sleep(0.01)
         except Exception:
             self.proc = None
 
@@ -122,7 +136,8 @@ class ClockSampler:
             self.proc.kill()
         sm, mx, reasons = [], [], set()
         try:
-            for line in open(self.path):
+            lines = self.lines()
+            for line in lines[self.skip:] or lines[-1:]:
                 parts = [p.strip() for p in line.split(",")]
                 if len(parts) < 7:
                     continue
@@ -422,11 +437,13 @@ def time_batched(D, caches, T, L, K, W, sampler=None):
         bd.new_v.copy_(v_pool[j])
         bd.step(T + j)
 
+    if sampler is not None:
+        sampler.start()
     for j in range(W):
         one_step(j)
     D.barrier()
     if sampler is not None:
-        sampler.start()
+        sampler.mark()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     D.barrier()
     ev0.record()

@@ -20,12 +20,12 @@ from .streaming import get_codebook
 GQA = 4
 # From this many new tokens on, one read-back of the layer serves all of them; below, a decode launch per
 # query token is taken.  Three tokens, us a layer (read-back and attention / three decode launches, several layers
-# sharing their phase tables): 8 KV heads 32 / 84 at 2K tokens of context, 42 / 84 at 8K, 112 / 120 at 32K,
-# 198 / 194 at 64K, 337 / 332 at 128K; 4 heads 72 / 89, 127 / 127, 211 / 201 from 32K on; 2 heads 57 / 83, 91 / 100,
-# 151 / 139.  Four tokens: the read-back at every context (8 heads 335 / 440 at 128K).
+# sharing their phase tables, host work included): 8 KV heads 74 / 113 at 16K tokens of context, 108 / 114 at 24K, 121 / 116 at 32K,
+# 165 / 146 at 48K, 349 / 293 at 128K; 4 heads 110 / 114 at 48K, 136 / 123 at 64K; 2 heads 100 / 114 at 64K, 160 / 140 at 128K.
+# Four tokens: the read-back at every context (8 heads 119 / 153 at 32K, 348 / 389 at 128K).
 MIN_MULTIQUERY_TOKENS = 3
-# Three tokens take their own launches where the layer's middle is longer than this.
-THREE_TOKENS_MAX_MIDDLE = 49152
+# Three tokens take their own launches where the layer's middle has more than this many (token, KV head) pairs.
+THREE_TOKENS_MAX_PAIRS = 200000
 # a forward over more new tokens than this after compression takes the dequantised path
 MAX_FUSED_QUERY_TOKENS = 256
 
@@ -312,7 +312,7 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
         raise _lib.ShardError("append the new tokens (update) before attending with them")
     res = torch.empty(s_q, n_q, hd, dtype=torch.float16, device=q_rope.device)
     nkv = cache._n_kv_heads
-    if (s_q >= MIN_MULTIQUERY_TOKENS and (s_q > 3 or gc["n_compress"] <= THREE_TOKENS_MAX_MIDDLE) and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
+    if (s_q >= MIN_MULTIQUERY_TOKENS and (s_q > 3 or gc["n_compress"] * nkv <= THREE_TOKENS_MAX_PAIRS) and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
             and not (gc.get("stream_n", 0) and "decode_k" in gc)):
         # all query tokens over one read-back of the layer
         dev = q_rope.device

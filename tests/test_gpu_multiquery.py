@@ -57,6 +57,11 @@ def test_three_tokens_either_side_of_the_rule(n_comp):
     test_multiquery(n_comp, 192, 1, 3, 3, True)
 
 
+@pytest.mark.parametrize("n_comp", [50000, 50001])
+def test_three_tokens_either_side_of_the_rule_with_four_heads(n_comp):
+    test_multiquery(n_comp, 192, 4, 3, 3, True)
+
+
 @pytest.mark.parametrize("nkv,rows,s", [(4, 1400, 20), (8, 300, 3), (1, 77, 33)])
 def test_rows_outside_the_middle_are_weighed_in_full(nkv, rows, s):
     """Where the decoded tokens carry the attention the output is float64's, rounded to fp16: their weights

@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       if (lane == 0) mbar_arrive(CB_READY);
     }
     // cos / sin of the rows, laid out as the fragments want them (phase_table_kernel); step i of a tile takes pairs
-    // 16 (i / 2) .. + 15 of rows 16 (i % 2) .. + 15; loaded four steps ahead
+    // 16 (i / 2) .. + 15 of rows 16 (i % 2) .. + 15; loaded four steps ahead (131K x 4 layers: 355 us; two ahead 393, three 378, six 375)
     const uint4* phase_tab = reinterpret_cast<const uint4*>(sq.phase) + lane;
     const int last_blk = (sh.tok_end - sh.tok_begin - 1) >> 5;
     auto phase_of = [&](int it) { return phase_tab + (size_t)min((tile_lo + it) * 4 + quad, last_blk) * 512; };

@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   auto C_EMPTY = [&](int b) { return bar0 + 8u * (uint32_t)(16 + b); };    // the unpack warps have read it
   auto V_FULL = [&](int b) { return bar0 + 8u * (uint32_t)(20 + b); };     // V code tile has landed
   auto V_EMPTY = [&](int b) { return bar0 + 8u * (uint32_t)(28 + b); };    // its group has read it
-  const uint32_t CB_READY = bar0 + 8u * 36u;                               // the codebooks are in shared memory
+  const uint32_t CB_READY = bar0 + 8u * 36u;                               // the codebooks are in shared memory (whoever looks codes up waits for it)
   const uint32_t Q_READY = bar0 + 8u * 37u;                                // the query fragments and the queries as given are staged
   const uint32_t QS_READY = bar0 + 8u * 39u;                               // the queries in code space are there
   const uint32_t APPEND_DONE = bar0 + 8u * 38u;                            // the newest streamed row has been written
@@ -898,7 +898,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
           __syncwarp();
           if (lane == 0) mbar_arrive(QS_READY);
         }
-        ok = __all_sync(0xffffffffu, mbar_wait(QS_READY, 0u, abort_s));
+        // (the split codebook too: the consumer warps write it behind the CTA's only barrier, and in a CTA of a few tiles, or none,
+        // nothing else here comes after that)
+        ok = __all_sync(0xffffffffu, mbar_wait(QS_READY, 0u, abort_s) && mbar_wait(CB_READY, 0u, abort_s));
       }
       if (ok && append_here) ok = __all_sync(0xffffffffu, mbar_wait(APPEND_DONE, 0u, abort_s));
       if (ok) {

@@ -64,6 +64,39 @@ def test_row_blocks(n_comp, nkv, rows, streaming, scale):
     assert (err <= 1.5e-3 * scale + 5e-3 * want.abs()).all(), (err / scale).max()
 
 
+@pytest.mark.parametrize("n_comp,rows", [(1, 901), (130, 75), (2304, 300), (4608, 40), (9000, 700), (11520, 2000)])   # 0 to 5 tiles a CTA
+def test_codes_are_looked_up_in_this_launch_s_codebook(n_comp, rows):
+    """Plain launches out of a cold L2, each behind one that left another codebook's tables in the same shared memory: a look-up that
+    does not wait for the tables finds entries of the wrong sign."""
+    from shard_b200 import ops
+    from shard_b200.attention import decode_layer
+    from shard_b200.streaming import get_codebook
+    nkv = 8
+    cache, layer = _cache(random_gc(n_comp, nkv=nkv, seed=rows), nkv, True, capacity=rows)
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda").half() for _ in range(2))
+    cache._fused_decode_update = True
+    layer.update(k, v)
+    q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+    first = decode_layer(q, layer, layer.get_seq_length() - 1).clone()
+    layer._needs_decompress = True
+    keys, values = layer.keys[0].double(), layer.values[0].double()
+    sc = torch.einsum("hqd,hnd->hqn", q[0].double(), keys.repeat_interleave(4, 0)) / 128 ** 0.5
+    want = (torch.softmax(sc, -1) @ values.repeat_interleave(4, 0))[:, 0]
+    assert ((first - want).abs() <= 1.5e-3 + 5e-3 * want.abs()).all()
+    ls, out, other = layer._gpu_compressed["_launch"], torch.empty_like(first), torch.empty_like(first)
+    right = get_codebook(128, 8, torch.device("cuda", 0))
+    wrong, flush = -right, torch.empty(1 << 26, device="cuda")
+    ls.shape.no_overlap = 1
+    for _ in range(10):
+        for codebook, dst in ((wrong, other), (right, out)):
+            flush.zero_()
+            ls.seq.out = dst.data_ptr()
+            ops.decode_attn(ls.seq, 1, ls.shape, ls.inv_ptr, codebook, cache._decode_ws)
+        assert torch.equal(out, first) and not torch.equal(other, first)
+    cache.check()
+
+
 @pytest.mark.parametrize("streaming", [True, False])
 def test_rows_between_16_byte_boundaries(streaming):
     """Rows that start 8 bytes (fp16) or 4 bytes (codes) behind a 16-byte boundary are read in pieces: the same result to the bit."""

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   auto V_FULL = [&](int b) { return bar0 + 8u * (uint32_t)(20 + b); };     // V code tile has landed
   auto V_EMPTY = [&](int b) { return bar0 + 8u * (uint32_t)(28 + b); };    // its group has read it
   const uint32_t CB_READY = bar0 + 8u * 36u;                               // the codebooks are in shared memory (whoever looks codes up waits for it)
-  const uint32_t Q_READY = bar0 + 8u * 37u;                                // the query fragments and the queries as given are staged
+  const uint32_t Q_READY = bar0 + 8u * 37u;                                // the query fragments, the queries as given and the channel scales are staged
   const uint32_t QS_READY = bar0 + 8u * 39u;                               // the queries in code space are there
   const uint32_t APPEND_DONE = bar0 + 8u * 38u;                            // the newest streamed row has been written
 
@@ -564,7 +564,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
 #pragma unroll
         for (int j = 0; j < PP_SPLIT_COPIES / 4; ++j) split_s[PP_SPLIT_COPIES / 4 * tid + ((j + (lane >> 1)) & (PP_SPLIT_COPIES / 4 - 1))] = make_uint4(sp, sp, sp, sp);
       }
-      if (tid < 32) *reinterpret_cast<uint2*>(smem_raw + PP_OFF_CH + 8 * lane) = *reinterpret_cast<const uint2*>(reinterpret_cast<const __half*>(sq.v_ch) + kv * HD + 4 * lane);
       __syncwarp();
       if (lane == 0) mbar_arrive(CB_READY);
     }
@@ -850,6 +849,8 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       griddep_wait();
 #pragma unroll
       for (int h = 0; h < GQA; ++h) { x_lo[h] = qg[h * HD + i]; x_hi[h] = qg[h * HD + i + 64]; }
+      // (the channel scales with the query: the kernel in front may be the one that writes them, and they cost no trip of their own here)
+      const uint32_t scales = reinterpret_cast<const uint32_t*>(reinterpret_cast<const __half*>(sq.v_ch) + kv * HD)[i];
 #pragma unroll
       for (int h = 0; h < GQA; ++h) {
         __half* f = reinterpret_cast<__half*>(smem_raw + PP_OFF_QF) + ((i >> 3) * 16 + 4 * h + ((i & 7) >> 1)) * 4 + (i & 1);
@@ -858,6 +859,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
         qg_s[h * HD + i] = x_lo[h];
         qg_s[h * HD + i + 64] = x_hi[h];
       }
+      *reinterpret_cast<uint32_t*>(smem_raw + PP_OFF_CH + 4 * i) = scales;
       __syncwarp();
       if (lane == 0) mbar_arrive(Q_READY);
     }

@@ -97,6 +97,39 @@ def test_codes_are_looked_up_in_this_launch_s_codebook(n_comp, rows):
     cache.check()
 
 
+@pytest.mark.parametrize("n_comp", [300, 9000])
+def test_channel_scales_from_the_launch_in_front(n_comp):
+    """The channel scales may be written by a launch that lets its successors start early (here a decode launch's output): they are not
+    among the tensors that are read ahead of it."""
+    from shard_b200 import ops
+    from shard_b200.attention import decode_layer
+    nkv = 8
+    layers = [_cache(random_gc(n, nkv=nkv, seed=n), nkv, False) for n in (20000, n_comp)]
+    g = torch.Generator(device="cuda").manual_seed(n_comp)
+    q = [torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half() for _ in range(5)]
+    scales = torch.empty(4 * nkv, 128, dtype=torch.float16, device="cuda")
+    (front_cache, front), (cache, layer) = layers
+    decode_layer(q[0], front, 30000, out=scales)
+    decode_layer(q[0], layer, 30000)
+    ls = layer._gpu_compressed["_launch"]
+    ls.seq.v_ch, ls.seq.q, ls.shape.no_overlap = scales.data_ptr(), q[0].data_ptr(), 0
+
+    def launch():
+        out = torch.empty(4 * nkv, 128, dtype=torch.float16, device="cuda")
+        ls.seq.out = out.data_ptr()
+        ops.decode_attn(ls.seq, 1, ls.shape, ls.inv_ptr, None, cache._decode_ws)
+        return out
+
+    for x in q:
+        scales.fill_(7.0)
+        decode_layer(x, front, 30000, out=scales)
+        got = launch()
+        torch.cuda.synchronize()
+        assert torch.equal(got, launch())
+    cache.check()
+    front_cache.check()
+
+
 @pytest.mark.parametrize("streaming", [True, False])
 def test_rows_between_16_byte_boundaries(streaming):
     """Rows that start 8 bytes (fp16) or 4 bytes (codes) behind a 16-byte boundary are read in pieces: the same result to the bit."""

@@ -369,6 +369,7 @@ __device__ __forceinline__ void row_state_store(RowState& st, float* out, bool m
   for (int off = 4; off < 32; off <<= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
   float m = st.m, f0 = 0.f;
   if (merge) {
+    __syncwarp();                                     // (the maxima and sums are other lanes' stores)
     const float m_mid = out[GQA * HD + t4], l_mid = out[GQA * HD + GQA + t4];
     m = fmaxf(m, m_mid);
     const float ref = m == neg_inf() ? 0.f : m;

@@ -37,6 +37,7 @@ def test_decode_rows(n_comp, nkv, rows, streaming):
 
 @pytest.mark.parametrize("n_comp,nkv,rows,streaming,scale", [
     (300, 8, 15, True, 1.0), (300, 8, 16, True, 300.0), (300, 2, 17, True, 2e-3), (1, 1, 33, True, 300.0), (1500, 8, 1200, True, 300.0),
+    (2304, 8, 4000, True, 1.0),    # all warps on the rows, behind a tile or two of their own
     (300, 8, 28, False, 300.0), (300, 2, 29, False, 2e-3), (1, 1, 13, False, 1.0), (1500, 8, 1200, False, 300.0)])
 def test_row_blocks(n_comp, nkv, rows, streaming, scale):
     """The ends of the blocks of sixteen rows, in one block, several blocks of a warp and all warps, with values far from one: the

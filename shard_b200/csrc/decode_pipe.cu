@@ -73,6 +73,7 @@ __host__ __device__ constexpr int pp_c_bytes(int nw) { return nw < 2 ? 2560 : 12
 // Shared memory, by address within the CTA's window.  The codebook sits on a multiple of 32 KB, so that a
 // look-up's address is (code's bits | this lane's base): one shift and one three-input logic operation.
 constexpr int PP_OFF_MISC = 0;                                        // barriers, flags
+constexpr int PP_OFF_QUP = 384;                                       // the powers of two by which the queries in code space are scaled, inverse, fp32 [4]
 constexpr int PP_OFF_CH = 640;                                        // the head's channel scales, fp16 [128]
 constexpr int PP_OFF_QG = 1024;                                       // queries as given, fp16 [4][128]
 constexpr int PP_OFF_QS = PP_OFF_QG + GQA * HD * 2;                   // queries in the stream's code space, two fp16 parts [4][2][128]
@@ -168,17 +169,25 @@ __device__ __forceinline__ uint4 row_load16(const void* at, bool aligned) {
   const unsigned int* w = reinterpret_cast<const unsigned int*>(at);
   return make_uint4(__ldcg(w), __ldcg(w + 1), __ldcg(w + 2), __ldcg(w + 3));
 }
-// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255]; one warp, `sg` its lanes' four signs
-__device__ __forceinline__ void stream_query(const float4 sg, const __half* q, __half* out, int lane) {
+// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255] of the query times a power of two that takes its
+// largest coordinate to 2^14 .. 2^15 (a sum of 128 channels may be beyond fp16's range, or at its lower end); returns the power's inverse.
+// One warp, `sg` its lanes' four signs
+__device__ __forceinline__ float stream_query(const float4 sg, const __half* q, __half* out, int lane) {
   const uint2 raw = *reinterpret_cast<const uint2*>(q + 4 * lane);
   const float2 a = __half22float2(as_half2(raw.x)), c = __half22float2(as_half2(raw.y));
   float x[4] = {a.x * sg.x, a.y * sg.y, c.x * sg.z, c.y * sg.w};
   fwht128_lane4(x, lane);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) x[j] *= INV_SQRT_HD;
+  // (biased exponent; an all-zero query counts as 2^-63, infinities stay what they are)
+  const int e = max((int)(__float_as_uint(warp_max(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))))) >> 23), 64);
+  const float up = __uint_as_float((uint32_t)(127 + 14 + 127 - e) << 23);
   uint32_t sp[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) sp[j] = split_half2(x[j] * INV_SQRT_HD);
+  for (int j = 0; j < 4; ++j) sp[j] = split_half2(x[j] * up);
   *reinterpret_cast<uint2*>(out + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x5410), __byte_perm(sp[2], sp[3], 0x5410));
   *reinterpret_cast<uint2*>(out + HD + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x7632), __byte_perm(sp[2], sp[3], 0x7632));
+  return __uint_as_float((uint32_t)(e - 14) << 23);
 }
 // weights of a block's rows: this lane has the scores sc[r] of rows lane / 4 + 8 r (log2 domain, -inf: no such row) and the
 // logarithms lv[r] of their values' norms; gives the value weights as B fragments, w[part][m][slot] for rows 8 m + 2 (lane % 4) + slot
@@ -267,9 +276,10 @@ __device__ __forceinline__ void split_values(uint32_t codes, uint32_t split, uin
     x[1][j] = __byte_perm(e[2 * j], e[2 * j + 1], 0x7632);
   }
 }
-// streamed rows u0 .. u0 + 15; `split`: address of this lane's copy of the split codebook
+// streamed rows u0 .. u0 + 15; `unit`: what a score of query head lane % 4 counts, in the log2 domain; `split`: address of this lane's copy of
+// the split codebook
 __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, const ShardDecodeShape& sh, int kv, int u0, const __half* qs_s,
-                                             uint32_t split, int lane) {
+                                             float unit, uint32_t split, int lane) {
   const int g8 = lane >> 2, t4 = lane & 3, last = sh.n_stream - 1;
   // keys: channels 32 t4 .. + 31 of rows g8 and g8 + 8; values: channels 16 g8 .. + 15 of rows 2 t4, 2 t4 + 1, and 8 further.  All loads
   // before the first use of one, and 16 bytes wide: with the norms converted where they were read, the block began with three round
@@ -312,7 +322,7 @@ __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, c
   for (int r = 0; r < 2; ++r) lv[r] = __log2f(__half2float(__ushort_as_half(vn[r])));
 #pragma unroll
   for (int r = 0; r < 2; ++r)
-    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * __half2float(__ushort_as_half(kn[r])) * (INV_SQRT_HD * LOG2E) : neg_inf();
+    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * (__half2float(__ushort_as_half(kn[r])) * unit) : neg_inf();
   uint32_t w[2][2][2];
   block_weights(st, sc, lv, w, lane);
 #pragma unroll
@@ -897,7 +907,8 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
       if (ok && blocks_s > 0) {
         // the unpack warps take a query head each to the code space; the others wait for them
         if (row_w < 4) {
-          stream_query(sg, qg_s + row_w * HD, qs_s + row_w * 2 * HD, lane);
+          const float inv = stream_query(sg, qg_s + row_w * HD, qs_s + row_w * 2 * HD, lane);
+          if (lane == 0) reinterpret_cast<float*>(smem_raw + PP_OFF_QUP)[row_w] = inv;
           __syncwarp();
           if (lane == 0) mbar_arrive(QS_READY);
         }
@@ -910,8 +921,9 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
         int b = part + p.n_row_parts * row_w;
         const int step = p.n_row_parts * n_row_warps;
         if (b < blocks_s) {
+          const float unit = reinterpret_cast<const float*>(smem_raw + PP_OFF_QUP)[lane & 3] * (INV_SQRT_HD * LOG2E);
 #pragma unroll 1
-          for (; b < blocks_s; b += step) stream_block(st, sq, sh, kv, 16 * b, qs_s, cb_u + PP_CB_ALIGN + 4u * (uint32_t)(lane & (PP_SPLIT_COPIES - 1)), lane);
+          for (; b < blocks_s; b += step) stream_block(st, sq, sh, kv, 16 * b, qs_s, unit, cb_u + PP_CB_ALIGN + 4u * (uint32_t)(lane & (PP_SPLIT_COPIES - 1)), lane);
           stream_sums_back(st, sq.signs, lane);
         }
 #pragma unroll 1

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from gpu_helpers import random_gc
-from test_gpu_readback import _cache
+from test_gpu_readback import _cache, middle_float64
 
 pytestmark = pytest.mark.gpu
 
@@ -63,6 +63,70 @@ def test_row_blocks(n_comp, nkv, rows, streaming, scale):
     want = torch.softmax(sc, -1) @ values.repeat_interleave(4, 0)
     err = (out[0].double() - want).abs()
     assert (err <= 1.5e-3 * scale + 5e-3 * want.abs()).all(), (err / scale).max()
+
+
+def rows_float64(layer, nkv):
+    """Keys and values (nkv, rows, 128) of everything outside the middle, float64, streamed rows from their codes."""
+    from shard_b200.streaming import get_codebook
+    gc = layer._gpu_compressed
+    keys, values = ([gc[s + x][0].double() for s in ("sink_", "win_")] for x in "kv")
+    if "decode_k" in gc:
+        keys.append(gc["decode_k"][0].double())
+        values.append(gc["decode_v"][0].double())
+    m = gc.get("stream_n", 0)
+    if m:
+        had = torch.ones(1, 1, dtype=torch.float64, device="cuda")
+        for _ in range(7):
+            had = torch.cat([torch.cat([had, had], 1), torch.cat([had, -had], 1)], 0)
+        codebook = get_codebook(128, 8, torch.device("cuda", 0)).double()
+        for x, out in (("k", keys), ("v", values)):
+            e = codebook[gc[x + "_idx_buf"][:m].long()].view(m, nkv, 128) @ had / 128 ** 0.5
+            out.append((e * gc["signs"].double() * gc[x + "_norm_buf"][:m].view(m, nkv, 1).double()).transpose(0, 1))
+    return torch.cat(keys, 1), torch.cat(values, 1)
+
+
+def attend_float64(q, keys, values):
+    sc = torch.einsum("hgd,hnd->hgn", q.double().view(keys.shape[0], 4, 128), keys) / 128 ** 0.5
+    return (torch.softmax(sc, -1) @ values).view(-1, 128)
+
+
+def rows_layer(nkv, streaming, k, v, seed):
+    """A layer whose middle is one token without a value, and its keys and values in float64 (the token's key in fp16 terms: its weight
+    is that of one row, in the sum of the weights alone)."""
+    gc_np = random_gc(1, nkv=nkv, seed=seed)
+    cache, layer = _cache(gc_np, nkv, streaming, capacity=k.shape[2] + 4)
+    layer._gpu_compressed["v_ch_f16"].zero_()
+    cache._fused_decode_update = True
+    layer.update(k, v)
+    middle = torch.from_numpy(middle_float64(gc_np, nkv)[0]).cuda()
+    keys, values = rows_float64(layer, nkv)
+    return cache, layer, torch.cat([middle, keys], 1), torch.cat([0 * middle, values], 1)
+
+
+def partial_attention(cache, layer, q):
+    """The launch's fp32 sums, divided: what it has before it rounds to fp16."""
+    from shard_b200.attention import decode_layer
+    rec = decode_layer(q, layer, layer.get_seq_length() - 1, partial_out=True)
+    cache.check()
+    return rec[:, 4:].double() / rec[:, 1:2].double()
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+def test_queries_beyond_the_range_of_fp16_in_code_space(streaming):
+    """A query whose coordinate in the stream's code space is 67 882 (128 channels of 6000 with the transform's signs), one of 1e-3 and an
+    all-zero one beside it: every coordinate is finite, and so is the attention."""
+    nkv, rows = 2, 40
+    g = torch.Generator(device="cuda").manual_seed(1)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda").half() * s for s in (0.01, 1.0))
+    from shard_b200.streaming import stream_signs
+    signs = stream_signs(0, 128, torch.device("cuda")).half()
+    k[:, :, 7] = 0.5 * signs
+    cache, layer, keys, values = rows_layer(nkv, streaming, k, v, 1)
+    q = torch.stack([6000 * signs, 1e-3 * signs, 0 * signs, signs] * nkv).view(1, 4 * nkv, 1, 128)
+    got = partial_attention(cache, layer, q)
+    want = attend_float64(q, keys, values)
+    # bound: the weights' (two roundings to 2**-22, scores of up to 30 in fp32) and the fp32 sums'; the token's key is an fp16 product
+    assert ((got - want).norm(dim=1) <= 2e-5 * want.norm(dim=1)).all(), ((got - want).norm(dim=1) / want.norm(dim=1)).max()
 
 
 @pytest.mark.parametrize("n_comp,rows", [(1, 901), (130, 75), (2304, 300), (4608, 40), (9000, 700), (11520, 2000)])   # 0 to 5 tiles a CTA

@@ -146,6 +146,22 @@ def test_one_launch_step_with_a_world_of_one_and_its_wait_running_out():
     assert np.array_equal(decode_layer(q, layer, 2100).cpu().numpy(), plain)   # the context is fine
 
 
+def test_one_launch_step_divides_as_the_plain_launch():
+    """The launch that merges what the ranks delivered and the plain one round the same quotient, whatever the sums are."""
+    from gpu_helpers import FakeCache, FakeLayer, gc_to_device, random_gc, random_query
+    from shard_b200.attention import decode_layer
+    layer = FakeLayer(gc_to_device(random_gc(2000, seed=81)), FakeCache(torch.from_numpy(O.default_inv_freq())))
+    bufs, ptrs = _exchange_buffers(1)
+    rk = _LocalRank(ptrs, 0, 1)
+    for seed in range(40):
+        q = torch.from_numpy(random_query(seed=seed)).to(DEV).view(1, 32, 1, 128)
+        plain = decode_layer(q, layer, 2100)
+        rk.fused_out = torch.empty(32, 128, dtype=torch.float16, device=DEV)
+        decode_layer(q, layer, 2100, partial_out=True, push=rk)
+        assert torch.equal(rk.fused_out, plain.view(32, 128)), seed
+    assert int(rk.status.item()) == 0
+
+
 @pytest.mark.parametrize("kernel", ["exchange_merge", "wait_merge"])
 def test_bounded_wait_runs_out_and_reports(kernel):
     """World of two, only rank 0 is ever launched: rank 1's flag stays unset, the wait gives up

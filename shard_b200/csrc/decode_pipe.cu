@@ -60,6 +60,7 @@ constexpr int PP_TMEM_COLS = 512;
 constexpr int PP_COL_A = 128 * PP_ST;               // the A operand slots: R/2 coefficient columns + 8 constant columns 1, 0, ... each
 __host__ __device__ constexpr int pp_a_cols(int nw) { return 16 * nw + 8; }
 constexpr int PP_STATE = GQA * HD + 2 * GQA;        // a warp's state, floats: acc[4][128], max[4], sum-exp[4]
+constexpr float PP_W_LOG2 = 14.f;                   // weights of rows' values, at most 1, times 2^14 in fp16
 constexpr float PP_LAZY_LOG2 = 8.f;                 // a softmax reference point moves only when exceeded by more than 2^8
 constexpr int PP_C_BUFS = 4;                        // coefficient tiles in shared memory
 constexpr int PP_V_BUFS = 6;                        // V code tiles (4 KB) in shared memory
@@ -133,29 +134,35 @@ __device__ __forceinline__ uint32_t lds_u1(uint32_t addr) {
 // ---- rows outside the middle, sixteen at a time on the tensor core -----------------------------------------------------------
 // A block of rows has the form of the middle's products: keys are A fragments (a row's 128 channels in any order, as long as the
 // query's are in the same), the scores come out with row lane / 4 (+ 8) and query head lane % 4 in a lane, and the values
-// are contracted over (row, parity of the channel).  Everything that was 32-bit arithmetic when a warp took two rows at a time
-// keeps 22 bits: the weights, the codebook and the queries in code space are two fp16 parts each, both products of
-// every pair; queries and keys of fp16 rows are exact, and all sums are fp32.  The weights of the values, p times the norm of a streamed row, have a
-// running reference of their own, so that they are at most 1 whatever the norms are.
-// Bound: latency of one block (loads, a chain of products, a softmax over 16 rows) -- about 130 instructions for 16 fp16 rows and
-// 600 for streamed ones, whose codes are looked up one by one; two rows at a time, with a reduction over the lanes for each, took
+// are contracted over (row, parity of the channel).  What was 32-bit arithmetic when a warp took two rows at a time (and is in a launch
+// without a middle) keeps 22 bits: the weights, the codebook and the queries in code space are two fp16 parts each, the second scaled by 2^11 with
+// sums of its own, all products of every pair; queries and keys of fp16 rows are exact, and all sums are fp32.  (A second part that is
+// not scaled falls into fp16's subnormals: a weight of 2^-16 kept 9 bits.)  The weights of the values, p times the norm of a streamed row, are
+// split as w . 2^14 for w <= 1, a power of two from the running reference's: 22 bits from 1 down to 2^-28, and an error of 2^-50 below.
+// Relative error of the sums against float64, fp16 rows / streamed ones: with even weights over 333 rows 6.8e-7 / 7.1e-7 (in 32-bit
+// arithmetic 7.0e-7 / 6.4e-7), where rows of weight 2^-20 carry the result 9.4e-7 / 9.4e-7 (8.5e-7 / 8.2e-7; 1.7e-3 and 6.3e-6 with unscaled
+// second parts and the products chained).  It costs 0.1 us a launch with streamed rows (8K x 12 layers 160.5 -> 161.4 us, 8 layers with 3001 streamed
+// rows 133.5 -> 133.6).
+// Bound: latency of one block (loads, a chain of products, a softmax over 16 rows) -- some 200 instructions for 16 fp16 rows and
+// 700 for streamed ones, whose codes are looked up one by one; two rows at a time, with a reduction over the lanes for each, took
 // 1 K cycles a pair.
 //
 // A streamed row is never rotated back: its key is norm / sqrt(128) . signs o H(codebook[code]), so the QUERY is taken to the
 // code space (H(signs o q) / sqrt(128)) and the score is norm . (query . codebook[code]); streamed values are summed in code space
 // and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of accumulators serves both kinds.
 struct RowState {
-  float m, l, u;      // of query head lane % 4, log2 domain: reference and sum of the weights, reference of the value weights
+  float m, l, j;      // of query head lane % 4: reference (log2 domain) and sum of the weights; o is in units of 2^(m + j - PP_W_LOG2), j whole
   float o[4][4];      // channels 16 (lane / 4) + 4 i + j of that head
 };
 __device__ __forceinline__ void row_state_init(RowState& st) {
-  st.m = neg_inf(); st.l = 0.f; st.u = neg_inf();
+  st.m = neg_inf(); st.l = 0.f; st.j = 0.f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] = 0.f;
 }
-// x as the sum of two fp16 values, the larger in the lower half
+// x = a + b / 2^11 with two fp16 values, a in the lower half: 22 bits of x where |x| >= 2^-14, an error of 2^-36 below
+constexpr float PP_LO_UP = 2048.f, PP_LO_DOWN = 1.f / PP_LO_UP;
 __device__ __forceinline__ uint32_t split_half2(float x) {
-  const __half hi = __float2half_rn(x), lo = __float2half_rn(x - __half2float(hi));
+  const __half hi = __float2half_rn(x), lo = __float2half_rn((x - __half2float(hi)) * PP_LO_UP);
   return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
 // 16 bytes, L2-coherent, in pieces of PIECE bytes where the address is no multiple of 16
@@ -169,47 +176,48 @@ __device__ __forceinline__ uint4 row_load16(const void* at, bool aligned) {
   const unsigned int* w = reinterpret_cast<const unsigned int*>(at);
   return make_uint4(__ldcg(w), __ldcg(w + 1), __ldcg(w + 2), __ldcg(w + 3));
 }
-// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255] of the query times a power of two that takes its
-// largest coordinate to 2^14 .. 2^15 (a sum of 128 channels may be beyond fp16's range, or at its lower end); returns the power's inverse.
-// One warp, `sg` its lanes' four signs
+// one query head as given -> the code space, fp16 parts out[0..127] and out[128..255] of the query times a power of two that takes
+// it into fp16's range (a coordinate is at most 128 / sqrt(128) < 2^3.6 of the largest channel, which the scaling takes to 2^10 .. 2^11);
+// returns the power's inverse.  One warp, `sg` its lanes' four signs
 __device__ __forceinline__ float stream_query(const float4 sg, const __half* q, __half* out, int lane) {
   const uint2 raw = *reinterpret_cast<const uint2*>(q + 4 * lane);
+  const uint32_t mags = __vmaxu2(raw.x & 0x7FFF7FFFu, raw.y & 0x7FFF7FFFu);
+  const uint32_t e = __reduce_max_sync(0xffffffffu, max(mags & 0xFFFFu, mags >> 16)) >> 10;   // biased by 15; 0: below 2^-14
   const float2 a = __half22float2(as_half2(raw.x)), c = __half22float2(as_half2(raw.y));
   float x[4] = {a.x * sg.x, a.y * sg.y, c.x * sg.z, c.y * sg.w};
   fwht128_lane4(x, lane);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) x[j] *= INV_SQRT_HD;
-  // (biased exponent; an all-zero query counts as 2^-63, infinities stay what they are)
-  const int e = max((int)(__float_as_uint(warp_max(fmaxf(fmaxf(fabsf(x[0]), fabsf(x[1])), fmaxf(fabsf(x[2]), fabsf(x[3]))))) >> 23), 64);
-  const float up = __uint_as_float((uint32_t)(127 + 14 + 127 - e) << 23);
+  const float up = __uint_as_float((127u + 25u - e) << 23);
   uint32_t sp[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) sp[j] = split_half2(x[j] * up);
+  for (int j = 0; j < 4; ++j) sp[j] = split_half2(x[j] * INV_SQRT_HD * up);
   *reinterpret_cast<uint2*>(out + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x5410), __byte_perm(sp[2], sp[3], 0x5410));
   *reinterpret_cast<uint2*>(out + HD + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x7632), __byte_perm(sp[2], sp[3], 0x7632));
-  return __uint_as_float((uint32_t)(e - 14) << 23);
+  return __uint_as_float((127u - 25u + e) << 23);
 }
-// weights of a block's rows: this lane has the scores sc[r] of rows lane / 4 + 8 r (log2 domain, -inf: no such row) and the
-// logarithms lv[r] of their values' norms; gives the value weights as B fragments, w[part][m][slot] for rows 8 m + 2 (lane % 4) + slot
-__device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2], const float (&lv)[2], uint32_t (&w)[2][2][2], int lane) {
-  const float u0 = sc[0] + lv[0], u1 = sc[1] + lv[1];
-  float tm = fmaxf(sc[0], sc[1]), tu = fmaxf(u0, u1);
+// 2^n, exact; n whole and within +-126
+__device__ __forceinline__ float pow2_whole(float n) { return __int_as_float(((int)n + 127) << 23); }
+// weights of a block's rows: this lane has the scores sc[r] of rows lane / 4 + 8 r (log2 domain, -inf: no such row) and the norms vn[r] of
+// their values; gives the value weights as B fragments, w[part][m][slot] for rows 8 m + 2 (lane % 4) + slot
+__device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2], const float (&vn)[2], uint32_t (&w)[2][2][2], int lane) {
+  // (the logarithms choose the reference and nothing else: the weight is p times the norm)
+  float tm = fmaxf(sc[0], sc[1]), tu = fmaxf(sc[0] + __log2f(vn[0]), sc[1] + __log2f(vn[1]));
 #pragma unroll
   for (int off = 4; off < 32; off <<= 1) {
     tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, off));
     tu = fmaxf(tu, __shfl_xor_sync(0xffffffffu, tu, off));
   }
-  const float m = fmaxf(st.m, tm), u = fmaxf(st.u, tu);
-  const float m0 = m == neg_inf() ? 0.f : m, uu = u == neg_inf() ? 0.f : u;
-  st.l = fmaf(st.l, ex2(st.m - m0), ex2(sc[0] - m0) + ex2(sc[1] - m0));
-  const float al = ex2(st.u - uu);
-  st.m = m; st.u = u;
+  const float m = fmaxf(st.m, tm), m0 = m == neg_inf() ? 0.f : m, u = fmaxf(st.m + st.j, tu);
+  const float j = u == neg_inf() ? st.j : fminf(fmaxf(ceilf(u - m0), -100.f), 100.f);
+  const float pr[2] = {ex2(sc[0] - m0), ex2(sc[1] - m0)}, al = ex2(st.m - m0);
+  st.l = fmaf(st.l, al, pr[0] + pr[1]);
+  const float al_o = al * pow2_whole(fminf(fmaxf(st.j - j, -126.f), 126.f)), up = pow2_whole(PP_W_LOG2 - j);
+  st.m = m; st.j = j;
 #pragma unroll
-  for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] *= al;
+  for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] *= al_o;
   const uint32_t odd = (lane >> 2) & 1, sel0 = odd ? 0x1044u : 0x4410u, sel1 = odd ? 0x3244u : 0x4432u;
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
-    const uint32_t sp = split_half2(ex2((r ? u1 : u0) - uu));
+    const uint32_t sp = split_half2(pr[r] * vn[r] * up);
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
       const uint32_t x = transpose_8x8(__byte_perm(sp, 0u, part ? 0x3232 : 0x1010));
@@ -239,31 +247,36 @@ __device__ __forceinline__ void fp16_block(RowState& st, const ShardSeq& sq, con
 #pragma unroll
     for (int i = 0; i < 2; ++i) v[r][i] = row_load16<8>(vp + 16 * g8 + 8 * i, aligned);
   }
-  float s[2][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] = 0.f;
+  float dot[2][4];                                    // (summed pairwise, rounded to nearest: a chain of products truncates)
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const uint4 q = *reinterpret_cast<const uint4*>(qg_s + (g8 >> 1) * HD + 32 * j + 8 * t4);
+    float s[2][4] = {};
     mma_16816(s[0], k[0][j].x, k[1][j].x, k[0][j].y, k[1][j].y, q.x, q.y);
     mma_16816(s[1], k[0][j].z, k[1][j].z, k[0][j].w, k[1][j].w, q.z, q.w);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) dot[r][j] = s[0][2 * r] + s[1][2 * r];
   }
   float sc[2];
-  const float lv[2] = {0.f, 0.f};
+  const float vn[2] = {1.f, 1.f};
 #pragma unroll
-  for (int r = 0; r < 2; ++r) sc[r] = u0 + g8 + 8 * r <= last ? (s[0][2 * r] + s[1][2 * r]) * (INV_SQRT_HD * LOG2E) : neg_inf();
+  for (int r = 0; r < 2; ++r) sc[r] = u0 + g8 + 8 * r <= last ? ((dot[r][0] + dot[r][1]) + (dot[r][2] + dot[r][3])) * (INV_SQRT_HD * LOG2E) : neg_inf();
   uint32_t w[2][2][2];
-  block_weights(st, sc, lv, w, lane);
+  block_weights(st, sc, vn, w, lane);
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int i = 0; i < 4; ++i) {
+    float o[2][4] = {};
 #pragma unroll
     for (int part = 0; part < 2; ++part)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int m = 0; m < 2; ++m) {
         const uint4 a = v[2 * m][i >> 1], b = v[2 * m + 1][i >> 1];
-        if (i & 1) mma_16816(st.o[i], a.z, a.w, b.z, b.w, w[part][m][0], w[part][m][1]);
-        else mma_16816(st.o[i], a.x, a.y, b.x, b.y, w[part][m][0], w[part][m][1]);
+        if (i & 1) mma_16816(o[part], a.z, a.w, b.z, b.w, w[part][m][0], w[part][m][1]);
+        else mma_16816(o[part], a.x, a.y, b.x, b.y, w[part][m][0], w[part][m][1]);
       }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) st.o[i][c] += fmaf(o[1][c], PP_LO_DOWN, o[0][c]);
+  }
 }
 // four codes -> the two fp16 parts of their codebook entries, part p of entries (0, 1) in x[p][0] and of (2, 3) in x[p][1]
 __device__ __forceinline__ void split_values(uint32_t codes, uint32_t split, uint32_t (&x)[2][2]) {
@@ -301,41 +314,49 @@ __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, c
     v[r] = row_load16<4>(sq.st_v_idx + row * HD + 16 * g8, aligned);
   }
   auto word = [](const uint4& x, int i) { return i == 0 ? x.x : i == 1 ? x.y : i == 2 ? x.z : x.w; };
-  // columns 2 h and 2 h + 1 are the two parts of query head h: their sum is the score
-  float s[2][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s[i >> 2][i & 3] = 0.f;
+  // columns 2 h and 2 h + 1 are the two parts of query head h
+  float lo[4] = {}, dot[2][4], cross[2] = {0.f, 0.f};
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const uint4 q = *reinterpret_cast<const uint4*>(qs_s + g8 * HD + 32 * t4 + 8 * j);
+    float hi[2][4] = {};
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t x0[2][2], x1[2][2];
       split_values(word(k[0][j >> 1], 2 * (j & 1) + h), split, x0);
       split_values(word(k[1][j >> 1], 2 * (j & 1) + h), split, x1);
-#pragma unroll
-      for (int part = 0; part < 2; ++part) mma_16816(s[part], x0[part][0], x1[part][0], x0[part][1], x1[part][1], h ? q.z : q.x, h ? q.w : q.y);
+      mma_16816(hi[h], x0[0][0], x1[0][0], x0[0][1], x1[0][1], h ? q.z : q.x, h ? q.w : q.y);
+      mma_16816(lo, x0[1][0], x1[1][0], x0[1][1], x1[1][1], h ? q.z : q.x, h ? q.w : q.y);
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) { dot[r][j] = hi[0][2 * r] + hi[1][2 * r]; cross[r] += hi[0][2 * r + 1] + hi[1][2 * r + 1]; }
   }
-  float sc[2], lv[2];
+  float sc[2], nv[2];
 #pragma unroll
-  for (int r = 0; r < 2; ++r) lv[r] = __log2f(__half2float(__ushort_as_half(vn[r])));
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-    sc[r] = u0 + g8 + 8 * r <= last ? ((s[1][2 * r] + s[1][2 * r + 1]) + (s[0][2 * r] + s[0][2 * r + 1])) * (__half2float(__ushort_as_half(kn[r])) * unit) : neg_inf();
+  for (int r = 0; r < 2; ++r) {
+    nv[r] = __half2float(__ushort_as_half(vn[r]));
+    const float x = fmaf(fmaf(lo[2 * r + 1], PP_LO_DOWN, lo[2 * r] + cross[r]), PP_LO_DOWN, (dot[r][0] + dot[r][1]) + (dot[r][2] + dot[r][3]));
+    sc[r] = u0 + g8 + 8 * r <= last ? x * (__half2float(__ushort_as_half(kn[r])) * unit) : neg_inf();
+  }
   uint32_t w[2][2][2];
-  block_weights(st, sc, lv, w, lane);
+  block_weights(st, sc, nv, w, lane);
 #pragma unroll
-  for (int m = 0; m < 2; ++m)
+  for (int i = 0; i < 4; ++i) {
+    uint32_t x[2][2][2][2];                           // [m][row][part][pair of codes]
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t x0[2][2], x1[2][2];
-      split_values(word(v[2 * m], i), split, x0);
-      split_values(word(v[2 * m + 1], i), split, x1);
+    for (int r = 0; r < 4; ++r) split_values(word(v[r], i), split, x[r >> 1][r & 1]);
+    float lo[4] = {}, cross[2][4] = {}, hi[4] = {};
+    auto products = [&](float(&o)[4], int vp, int wp) {
 #pragma unroll
-      for (int part = 0; part < 4; ++part)
-        mma_16816(st.o[i], x0[part >> 1][0], x0[part >> 1][1], x1[part >> 1][0], x1[part >> 1][1], w[part & 1][m][0], w[part & 1][m][1]);
-    }
+      for (int m = 0; m < 2; ++m) mma_16816(o, x[m][0][vp][0], x[m][0][vp][1], x[m][1][vp][0], x[m][1][vp][1], w[wp][m][0], w[wp][m][1]);
+    };
+    products(lo, 1, 1);
+    products(cross[0], 0, 1);
+    products(cross[1], 1, 0);
+    products(hi, 0, 0);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) st.o[i][c] += fmaf(fmaf(lo[c], PP_LO_DOWN, cross[0][c] + cross[1][c]), PP_LO_DOWN, hi[c]);
+  }
 }
 // normalised 128-point Hadamard transform of every query head's sums (channel 16 (lane / 4) + 4 i + j in o[i][j])
 __device__ __forceinline__ void row_sums_fwht(RowState& st, int lane) {
@@ -386,7 +407,7 @@ __device__ __forceinline__ void row_state_store(RowState& st, float* out, bool m
     f0 = ex2(m_mid - ref);
     l = fmaf(l, ex2(st.m - ref), l_mid * f0);
   }
-  const float f = st.u == neg_inf() ? 0.f : ex2(st.u - m);
+  const float f = st.m == neg_inf() ? 0.f : ex2(st.m - m) * pow2_whole(st.j - PP_W_LOG2);
   __syncwarp();
   if (g8 == 0) { out[GQA * HD + t4] = m; out[GQA * HD + GQA + t4] = l; }
 #pragma unroll

@@ -40,9 +40,9 @@ def test_decode_rows(n_comp, nkv, rows, streaming):
     (2304, 8, 4000, True, 1.0),    # all warps on the rows, behind a tile or two of their own
     (300, 8, 28, False, 300.0), (300, 2, 29, False, 2e-3), (1, 1, 13, False, 1.0), (1500, 8, 1200, False, 300.0)])
 def test_row_blocks(n_comp, nkv, rows, streaming, scale):
-    """The ends of the blocks of sixteen rows, in one block, several blocks of a warp and all warps, with values far from one: the
-    weights are two fp16 parts and carry a streamed row's norm, which must cost neither small nor large values their digits.  Bound:
-    that of the other rows (fp16 rounding of values, weights and output), in units of the values."""
+    """The ends of the blocks of sixteen rows, in one block, several blocks of a warp and all warps, with values far from one (a streamed row's
+    norm goes into its weight).  Bound: that of the other rows (fp16 rounding of values, weights and output), in units of the values;
+    what the weights keep is measured by the tests of the launch's fp32 sums above."""
     from shard_b200 import fused_attention_compressed
     gc_np = random_gc(n_comp, nkv=nkv, seed=rows)
     cache, layer = _cache(gc_np, nkv, streaming, capacity=rows + 4)
@@ -127,6 +127,47 @@ def test_queries_beyond_the_range_of_fp16_in_code_space(streaming):
     want = attend_float64(q, keys, values)
     # bound: the weights' (two roundings to 2**-22, scores of up to 30 in fp32) and the fp32 sums'; the token's key is an fp16 product
     assert ((got - want).norm(dim=1) <= 2e-5 * want.norm(dim=1)).all(), ((got - want).norm(dim=1) / want.norm(dim=1)).max()
+
+
+# What 32-bit arithmetic leaves: a score of up to 24 in the log2 domain with three roundings at its full size (3 . 24 . 2**-24 . ln 2 = 3e-6 of
+# a weight), ex2 and the fp32 sums; the middle's token, whose key is an fp16 product, has 1e-3 of its weight in 85 (8, 16) to 4069 rows'.
+# A part dropped anywhere leaves 11 bits, 2e-4; second parts in fp16's subnormals 2e-5 and more where small weights carry the result.
+ROWS_REL = 4e-6
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("nkv,rows", [(8, 16), (2, 333), (8, 1200), (1, 4000)])
+def test_rows_are_weighed_in_full(nkv, rows, streaming):
+    """Even attention over the rows: the launch's fp32 sums are float64's to the precision of 32-bit arithmetic."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda").half() for _ in range(2))
+    cache, layer, keys, values = rows_layer(nkv, streaming, k, v, rows)
+    q = torch.randn(1, 4 * nkv, 1, 128, generator=g, device="cuda").half()
+    got, want = partial_attention(cache, layer, q), attend_float64(q, keys, values)
+    err = (got - want).norm() / want.norm()
+    assert err <= ROWS_REL, err
+
+
+@pytest.mark.parametrize("streaming", [True, False])
+@pytest.mark.parametrize("nkv,rows,power", [(8, 40, 12), (2, 333, 20), (8, 1200, 16), (1, 4000, 24)])
+def test_rows_of_small_weight_and_large_values(nkv, rows, power, streaming):
+    """One row has nearly all of the attention and a value of nearly nothing; the result is made of the others, whose weights are about
+    2**-power of its."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    base = torch.randn(nkv, 1, 128, generator=g, device="cuda")
+    base *= 128 ** 0.5 / base.norm(dim=-1, keepdim=True)
+    q = (base + 0.05 * torch.randn(nkv, 4, 128, generator=g, device="cuda")).half().view(1, 4 * nkv, 1, 128)
+    k, v = (torch.randn(1, nkv, rows, 128, generator=g, device="cuda") for _ in range(2))
+    v *= 2.0 ** min(power - 8, 8)
+    k[:, :, rows // 3] = base[:, 0] * (power * 0.6931 / 128 ** 0.5)
+    v[:, :, rows // 3] = 2.0 ** -12
+    cache, layer, keys, values = rows_layer(nkv, streaming, k.half(), v.half(), rows)
+    got, want = partial_attention(cache, layer, q), attend_float64(q, keys, values)
+    small = values.clone()
+    small[:, 69 + rows // 3] = 0
+    assert attend_float64(q, keys, small).norm() > 0.9 * want.norm()
+    err = (got - want).norm() / want.norm()
+    assert err <= ROWS_REL, err
 
 
 @pytest.mark.parametrize("n_comp,rows", [(1, 901), (130, 75), (2304, 300), (4608, 40), (9000, 700), (11520, 2000)])   # 0 to 5 tiles a CTA

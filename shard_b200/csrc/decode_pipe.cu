@@ -89,6 +89,13 @@ static_assert(PP_HEAD_BYTES <= PP_CB_ALIGN - 2048, "the head of the layout ends 
 __host__ __device__ constexpr int pp_smem_bytes(int nw) {             // from the end of the 1 KB the system keeps
   return 2 * PP_CB_ALIGN + PP_SPLIT_BYTES - 1024 + pp_w_bytes(nw) + PP_C_BUFS * pp_c_bytes(nw) + PP_ROW_WARPS * PP_STATE * 4;
 }
+// The dynamic part starts behind what the system keeps and the kernel's static variables, on a multiple of 1 KB; the codebook is on the first
+// multiple of 32 KB only if the head of the layout ends before it.  The host asks for both sizes before the first launch on a device.
+constexpr bool pp_layout_fits(size_t system_bytes, size_t static_bytes) {
+  return ((system_bytes + static_bytes + 1023) & ~(size_t)1023) + PP_HEAD_BYTES <= PP_CB_ALIGN;
+}
+static_assert(pp_layout_fits(1024, 1024) && pp_layout_fits(1024, 0) && !pp_layout_fits(1024, 1025) && !pp_layout_fits(2048, 1024) && !pp_layout_fits(4096, 0),
+              "what is there today fits, a static variable beyond the first KB or a larger share of the system's does not");
 
 // single-thread forms (the caller is one elected thread)
 __device__ __forceinline__ void umma_ts_1t(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t raw_u = smem_u32(smem_raw);
   const uint32_t cb_u = (raw_u + PP_HEAD_BYTES + PP_CB_ALIGN - 1) & ~(uint32_t)(PP_CB_ALIGN - 1);
-  if (cb_u != PP_CB_ALIGN) {                                       // (the layout is sized for a window that starts this low)
+  if (cb_u != PP_CB_ALIGN) {                                       // (the host has refused such a launch already: pp_layout_fits)
     if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
     return;
   }
@@ -1055,7 +1062,13 @@ static int launch_pipe_one(const DecodeParams& p, dim3 grid, cudaStream_t st) {
   if (de != cudaSuccess) return (int)de;
   if (dev < 0 || dev >= MAX_DEVICES) return SHARD_E_ARG;
   if (!configured[dev].load(std::memory_order_acquire)) {
-    cudaError_t e = cudaFuncSetAttribute(decode_partial_pipe_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    cudaFuncAttributes attrs;
+    int reserved = 0;
+    cudaError_t e = cudaFuncGetAttributes(&attrs, decode_partial_pipe_kernel<NW>);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+    if (e != cudaSuccess) return (int)e;
+    if (!pp_layout_fits((size_t)reserved, attrs.sharedSizeBytes)) return (int)cudaErrorInvalidConfiguration;
+    e = cudaFuncSetAttribute(decode_partial_pipe_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
     configured[dev].store(true, std::memory_order_release);
   }

@@ -137,7 +137,8 @@ class ClockSampler:
         sm, mx, reasons = [], [], set()
         try:
             lines = self.lines()
-            for line in lines[self.skip:] or lines[-1:]:
+            during = lines[self.skip:]
+            for line in during or lines[-1:]:
                 parts = [p.strip() for p in line.split(",")]
                 if len(parts) < 7:
                     continue
@@ -155,7 +156,9 @@ class ClockSampler:
             pass
         if sm:
             out.update(sm_mhz=statistics.median(sm), sm_max_mhz=max(mx), reasons=sorted(reasons),
-                       samples=len(sm))
+                       samples=len(sm) if during else 0)
+            if not during:
+                out["note"] = "no sample fell into the timed region: the last one from before it"
         return out
 
 

@@ -78,3 +78,22 @@ def test_stream_signs_are_the_callers():
     a, b = stream_signs(3, 128, "cpu"), stream_signs(3, 128, "cpu")
     a.zero_()
     assert bool((b.abs() == 1).all()) and torch.equal(b, stream_signs(3, 128, "cpu"))
+
+
+@pytest.mark.parametrize("before,during", [(3, 0), (3, 2), (0, 4)])
+def test_the_clock_record_says_what_it_was_sampled_in(tmp_path, before, during):
+    """Samples of the timed region count; where there are none the last one from before it stands in, and the record says so."""
+    import bench
+    sampler = bench.ClockSampler(0)
+    sampler.path = str(tmp_path / "clocks.csv")
+    sampler.proc = subprocess.Popen([sys.executable, "-c", ""])
+    idle, busy = "120, 1965, 200.0, Not Active, Not Active, Not Active, Not Active\n", "1965, 1965, 700.0, Not Active, Not Active, Not Active, Active\n"
+    with open(sampler.path, "w") as f:
+        f.write(idle * before)
+    sampler.mark()
+    with open(sampler.path, "a") as f:
+        f.write(busy * during)
+    got = sampler.stop()
+    assert got["samples"] == during and got["sm_mhz"] == (1965 if during else 120)
+    assert ("note" in got) == (during == 0)
+    assert got["reasons"] == (["sw_power_cap"] if during else [])

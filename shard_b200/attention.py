@@ -19,13 +19,16 @@ from .streaming import get_codebook
 
 GQA = 4
 # From this many new tokens on, one read-back of the layer serves all of them; below, a decode launch per
-# query token is taken.  Three tokens, us a layer (read-back and attention / three decode launches, several layers
-# sharing their phase tables, host work included): 8 KV heads 74 / 113 at 16K tokens of context, 108 / 114 at 24K, 121 / 116 at 32K,
-# 165 / 146 at 48K, 349 / 293 at 128K; 4 heads 110 / 114 at 48K, 136 / 123 at 64K; 2 heads 100 / 114 at 64K, 160 / 140 at 128K.
+# query token is taken.  Three tokens, us a layer of a forward through `update` and `fused_attention_compressed` (four layers of one cache,
+# 100 streamed tokens; read-back / decode launches): 8 KV heads 75 / 120 at 16K tokens of context, 108 / 119 at 24K, 121 / 120 at 32K, 165 / 147 at 48K,
+# 351 / 296 at 128K; 4 heads 81 / 121 at 32K, 110 / 121 at 48K, 136 / 124 at 64K; 2 heads 102 / 121 at 64K, 136 / 125 at 96K,
+# 161 / 142 at 128K; 1 head 92 / 122 at 64K, 118 / 122 at 96K, 135 / 124 at 128K, 186 / 150 at 192K.
 # Four tokens: the read-back at every context (8 heads 119 / 153 at 32K, 348 / 389 at 128K).
 MIN_MULTIQUERY_TOKENS = 3
-# Three tokens take their own launches where the layer's middle has more than this many (token, KV head) pairs.
+# Three tokens take their own launches where the layer's middle has more than this many (token, KV head) pairs (8 and 4 heads cross at
+# about 240 000, 2 at 180 000), or, with few heads, more than this many tokens (1 head: 105 000).
 THREE_TOKENS_MAX_PAIRS = 200000
+THREE_TOKENS_MAX_MIDDLE = 90000
 # a forward over more new tokens than this after compression takes the dequantised path
 MAX_FUSED_QUERY_TOKENS = 256
 
@@ -312,7 +315,7 @@ def fused_attention_compressed(q_rope, layer, pos_q, inv_freq=None, attn_mask=No
         raise _lib.ShardError("append the new tokens (update) before attending with them")
     res = torch.empty(s_q, n_q, hd, dtype=torch.float16, device=q_rope.device)
     nkv = cache._n_kv_heads
-    if (s_q >= MIN_MULTIQUERY_TOKENS and (s_q > 3 or gc["n_compress"] * nkv <= THREE_TOKENS_MAX_PAIRS) and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
+    if (s_q >= MIN_MULTIQUERY_TOKENS and (s_q > 3 or gc["n_compress"] <= min(THREE_TOKENS_MAX_MIDDLE, THREE_TOKENS_MAX_PAIRS // nkv)) and q_rope.dtype == torch.float16 and n_q == GQA * nkv and hd == 128
             and not (gc.get("stream_n", 0) and "decode_k" in gc)):
         # all query tokens over one read-back of the layer
         dev = q_rope.device

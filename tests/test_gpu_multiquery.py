@@ -52,14 +52,16 @@ def test_queries_of_two_sequences_are_refused(s):
         fused_attention_compressed(q, layer, layer.get_seq_length() - 1, cache._rope_inv_freq)
 
 
-@pytest.mark.parametrize("n_comp", [49152, 49153])
-def test_three_tokens_either_side_of_the_rule(n_comp):
-    test_multiquery(n_comp, 192, 1, 3, 3, True)
-
-
-@pytest.mark.parametrize("n_comp", [50000, 50001])
-def test_three_tokens_either_side_of_the_rule_with_four_heads(n_comp):
-    test_multiquery(n_comp, 192, 4, 3, 3, True)
+@pytest.mark.parametrize("nkv,last", [(8, 25000), (4, 50000), (2, 90000), (1, 90000)])
+@pytest.mark.parametrize("over", [0, 1])
+def test_three_tokens_either_side_of_the_rule(nkv, last, over, monkeypatch):
+    """The longest middle that is read back once, and one token more, which takes decode launches."""
+    from shard_b200 import attention
+    assert last == min(attention.THREE_TOKENS_MAX_MIDDLE, attention.THREE_TOKENS_MAX_PAIRS // nkv)
+    real, calls = attention.ops.multiquery_attn, []
+    monkeypatch.setattr(attention.ops, "multiquery_attn", lambda *a: (calls.append(1), real(*a))[1])
+    test_multiquery(last + over, 192, nkv, 3, 3, True)
+    assert len(calls) == (0 if over else 2)            # (the test attends twice)
 
 
 @pytest.mark.parametrize("nkv,rows,s", [(4, 1400, 20), (8, 300, 3), (1, 77, 33)])

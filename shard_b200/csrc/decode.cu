@@ -51,12 +51,15 @@ static DecodePlan make_plan(const ShardDecodeShape& sh, int batch) {
   const int groups = sh.nkv * batch;
   if (n_tiles > 0) {
     // One CTA per SM.  Fewer (sequence, KV head) pairs than SMs: one wave, the tiles of every pair spread
-    // evenly over its CTAs.  More: CTAs come in waves, and a CTA costs its tiles (3 K cycles each) plus
-    // what it does outside the tile loop (about 16 K cycles: set-up, first tile's latency, epilogue),
-    // CTA_TILES tiles' worth; the number of chunks whose waves cost least.
+    // evenly over its CTAs.  More: CTAs come in waves, and a CTA costs its tiles (2.45 K cycles each) plus what it does outside the
+    // tile loop (set-up, first tile's latency, rows, epilogue; less where the next wave's CTAs overlap it), CTA_TILES tiles' worth; the number
+    // of chunks whose waves cost least.  Measured with 1 to 9 chunks for 23 batches of 19 to 64 sequences of 500 to 16K tokens, 8 and 4
+    // heads: mean time over that of the best number of chunks 1.012 / 1.003 / 1.001 / 1.000 / 1.002 / 1.008 / 1.011 with
+    // 3 / 4 / 5 / 6 and 7 / 8 and 9 / 10 / 12 tiles' worth (64 x 8192 tokens 386 us with one chunk, 374 with two, 395 with three; 60 x 12223
+    // tokens 541 / 506 / 519; 20 x 16384 tokens 349 / 276 / 257 and 249 with four).
     int chunks = CTA_SLOTS / groups;
     if (chunks < 1) {
-      constexpr int CTA_TILES = 5;
+      constexpr int CTA_TILES = 6;
       long long best = 0;
       for (int c = 1; c <= n_tiles && c <= 16; ++c) {
         const long long waves = ((long long)groups * c + CTA_SLOTS - 1) / CTA_SLOTS;
@@ -73,8 +76,8 @@ static DecodePlan make_plan(const ShardDecodeShape& sh, int batch) {
     pl.tiles_per_chunk = n_tiles / chunks;
     pl.tiles_rem = n_tiles % chunks;
   }
-  // the fp16 / streamed rows ride along in the chunk CTAs (dealt out row by row, handled while a
-  // CTA waits for its first tile); only a launch without a middle gets CTAs just for them
+  // the fp16 / streamed rows ride along in the chunk CTAs (dealt out in blocks of sixteen, behind a CTA's
+  // tiles); only a launch without a middle gets CTAs just for them
   const int n_rows = sh.n_sink + sh.n_win + sh.n_dec + sh.n_stream;
   if (n_rows > 0) {
     pl.n_row_parts = pl.n_chunks;

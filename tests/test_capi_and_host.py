@@ -246,3 +246,18 @@ def test_hf_glue_short_prompt_on_cpu():
     assert not cache._compressed and cache.get_seq_length() == 25
     assert cache.memory_bytes() == 2 * 2 * 25 * 128 * 4      # raw fp32 K and V of 2 layers
     assert torch.allclose(cache._rope_inv_freq, 1.0 / (500000.0 ** (torch.arange(0, 128, 2).float() / 128)))
+
+
+@pytest.mark.parametrize("seqs,tokens,nkv,chunks", [
+    (64, 8192, 8, 2), (64, 2048, 8, 1), (20, 16384, 8, 4), (19, 8192, 8, 4), (50, 5000, 4, 2), (60, 12223, 8, 2), (32, 13934, 8, 1),
+    (24, 3000, 8, 2)])
+def test_chunks_of_a_batch_are_the_fastest_measured(seqs, tokens, nkv, chunks):
+    """The decode plan of batches whose times with 1 to 9 chunks were measured on 148 SMs takes the fastest (the workspace has one
+    record per chunk and query head)."""
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("measured on 148 SMs")
+    from shard_b200 import _lib, ops
+    shape = ops.make_shape(4 * nkv, nkv, 192, tokens - 68, 0, tokens - 68, 4, 64, 100, tokens + 100)
+    got = ops.decode_workspace_bytes(shape, seqs)
+    header = 16 + (4 * seqs * nkv + 15) // 16 * 16
+    assert got == header + seqs * chunks * 4 * nkv * _lib.PART_STRIDE * 4

@@ -7,6 +7,8 @@
 //   nvcc -O3 -std=c++17 -gencode arch=compute_100a,code=sm_100a -o tcgen05_mma_rate tcgen05_mma_rate.cu
 //   ./tcgen05_mma_rate
 //
+// At the end the same beside mma.sync, the other kind of tensor instruction the kernel uses.
+//
 // Every wait is bounded (about 40 ms); a case that times out prints "timeout" and the program
 // goes on.
 #include <cstdint>
@@ -182,6 +184,83 @@ __global__ void __launch_bounds__(512) bench(int reps, long long* out) {
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512) : "memory");
 }
 
+// tcgen05.mma and mma.sync on the same SM: a stream of 128 x 128 x 16 products by one thread (STREAM, or POLL: with a look at a shared word
+// between two of them, as a thread that polls for its next tile would) and one warp per scheduler with eight independent chains of m16n8k16
+// (SYNC).  The stream runs until the other warps are done, at most 4000 products.
+// out[0], out[1]: cycles and number of the stream's instructions, out[2], out[3]: cycles and number of a scheduler's mma.sync; out[0] = -1: timeout
+enum Mixed { STREAM = 1, SYNC = 2, POLL = 4 };
+template <int what>
+__global__ void __launch_bounds__(256) mixed(int iters, long long* out) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  __shared__ uint32_t slot;
+  __shared__ uint64_t bar;
+  __shared__ int done;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int i = tid; i < 64 * 1024 / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(smem)[i] = 0x3c003c00u;
+  if (tid == 0) { mbar_init(smem_u32(&bar), 1); done = 0; }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tb = slot;
+  if (warp == 0 && (what & STREAM)) {
+    const uint64_t bd = desc_sw128(smem_u32(smem), 16, 1024);
+    if (lane == 0) {
+      const long long t0 = clock64();
+      int n = 0;
+      for (; n < ((what & SYNC) ? 4000 : iters); ++n) {
+        umma_ts(tb, tb + 256 + 8 * (n & 7), bd + 2 * (n & 3), mk_idesc(128, 128), 1u);
+        // (a stream beside the other warps looks once in 16 whether they are done)
+        if (((what & POLL) || ((what & SYNC) && (n & 15) == 15)) && *reinterpret_cast<volatile int*>(&done) == 4) break;
+      }
+      if (blockIdx.x == 0) { out[0] = clock64() - t0; out[1] = n; }
+      umma_commit(smem_u32(&bar));
+    }
+    __syncwarp();
+    if (!mbar_wait(smem_u32(&bar), 0) && lane == 0 && blockIdx.x == 0) out[0] = -1;
+  } else if (warp >= 4 && (what & SYNC)) {
+    float d[8][4] = {};
+    const uint32_t a = 0x3c003c00u;
+    const long long t0 = clock64();
+    for (int i = 0; i < iters; ++i)
+#pragma unroll
+      for (int c = 0; c < 8; ++c)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%4,%4,%4}, {%4,%5}, {%0,%1,%2,%3};"
+                     : "+f"(d[c][0]), "+f"(d[c][1]), "+f"(d[c][2]), "+f"(d[c][3]) : "r"(a), "r"(lane));
+    const long long t1 = clock64();
+    float sum = 0.f;
+    for (int c = 0; c < 8; ++c) sum += d[c][0] + d[c][3];
+    if (lane == 0 && warp == 4 && blockIdx.x == 0) { out[2] = t1 - t0; out[3] = 8ll * iters; }
+    if (sum == 1.2345f) out[5] = 1;
+    __syncwarp();
+    if (lane == 0) atomicAdd(&done, 1);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tb), "r"(512) : "memory");
+}
+template <int what>
+int run_mixed(const char* name, int iters, long long* d) {
+  cudaFuncSetAttribute(mixed<what>, cudaFuncAttributeMaxDynamicSharedMemorySize, 66 * 1024);
+  cudaMemset(d, 0, 64);
+  mixed<what><<<148, 256, 66 * 1024>>>(iters, d);
+  const cudaError_t e = cudaDeviceSynchronize();
+  long long h[4] = {0, 0, 0, 0};
+  cudaMemcpy(h, d, 32, cudaMemcpyDeviceToHost);
+  if (e != cudaSuccess || h[0] < 0) {
+    printf("%-56s: %s\n", name, e != cudaSuccess ? cudaGetErrorString(e) : "timeout");
+    return 1;
+  }
+  printf("%-56s: %6.1f cycles/mma of the issuing thread, %6.1f cycles/mma.sync of a scheduler\n", name, h[1] ? h[0] / (double)h[1] : 0.0,
+         h[3] ? h[2] / (double)h[3] : 0.0);
+  return 0;
+}
+
 template <int C>
 void launch_one(int reps, long long* d) {
   cudaFuncSetAttribute(bench<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 130 * 1024);
@@ -244,6 +323,11 @@ int main() {
       printf("%-56s: %6.1f cycles/mma until complete, %6.1f cycles/mma of the issuing thread\n", names[c],
              h[0] / (double)reps / per_rep, h[1] / (double)reps / per_rep);
   }
+  // (the SM's shared memory leaves room for one CTA of the others, two of these: 148 CTAs spread over 148 SMs all the same)
+  if (!bad) bad |= run_mixed<SYNC>("mma.sync m16n8k16, a warp per scheduler", 100, d);
+  if (!bad) bad |= run_mixed<STREAM | SYNC>("the same beside a stream of m128 n128 TS", 100, d);
+  if (!bad) bad |= run_mixed<STREAM>("m128 n128 TS, long stream", 400, d);
+  if (!bad) bad |= run_mixed<STREAM | POLL>("m128 n128 TS, a shared word polled in between", 400, d);
   cudaFree(d);
   return bad;
 }

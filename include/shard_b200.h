@@ -99,9 +99,9 @@ typedef struct ShardDecodeShape {
  * t in [0, n_tok), i in [0, 64): the table of src/shard/attention.py:76-79.
  * It depends only on positions, so one table serves every layer of a step.
  * out (16-byte aligned, shard_b200_phase_table_bytes(n_tok) bytes) is opaque to the caller:
- * tokens are grouped in blocks of 32, and a block stores 16 planes of 32 x 16 bytes -- plane c < 8
- * the cosines of pairs 8c..8c+7 for each of its tokens, plane 8 + c the sines -- so that a warp
- * owning 32 consecutive tokens reads each plane as one contiguous 512-byte run.
+ * tokens are grouped in blocks of 32, and a block's 8 KB interleave cosines and sines in the order in
+ * which the 32 lanes of the warp that attends to it take them as matrix fragments, 16 bytes a lane.
+ * The last block is written whole.
  */
 size_t shard_b200_phase_table_bytes(int32_t n_tok);
 int shard_b200_phase_table(int32_t compress_start, int32_t pos_q, int32_t n_tok,
@@ -165,7 +165,7 @@ size_t shard_b200_decode_workspace_bytes(const ShardDecodeShape* shape_host, int
  * (shard_b200_decode_prepare, the kernels that produce the codes, a copy into the table): for
  * the first decode call behind such work set shape.no_overlap = 1, which launches the plain way
  * (or set SHARD_B200_PDL=0 in the environment to do so always).  Everything else -- query, new
- * token, stream rows, workspace, output -- is read and written only after the
+ * token, channel scales, stream rows, workspace, output -- is read and written only after the
  * preceding work has completed.
  */
 int shard_b200_decode_attn(const ShardSeq* seqs, int32_t batch, const ShardDecodeShape* shape_host,

@@ -9,7 +9,9 @@
 //   phase_table_kernel          cos/sin(fp32(pos_t - pos_q) * inv_freq) in fp16, shared by all layers
 //   decode_partial_pipe_kernel  (decode_pipe.cu) one launch per layer-step: optional stream append,
 //                               split-KV pass over the middle / fp16 rows / streamed rows, and the
-//                               combine, done by the last CTA of each KV head to arrive
+//                               combine, done per query head by the last warp to arrive with its record (per KV
+//                               head by the last CTA where the result goes to the exchange buffers, or there is
+//                               no middle)
 //   decode_combine_kernel       the same combine as a kernel of its own, for merging the partial
 //                               records of several launches or several GPUs (shard_b200_lse_merge)
 #include <cstdlib>

@@ -1,6 +1,5 @@
-// Pieces shared by the decode kernels: launch plan, per-CTA query staging, the
-// warp-per-token path for fp16 / streamed rows, and the CTA-level merge that emits one
-// (max, sum-exp, acc[128]) record per query head.
+// Pieces shared by the decode kernels: launch parameters, per-CTA query staging, the rows of launches
+// without a middle segment, and the merges into one (max, sum-exp, acc[128]) record per query head.
 #pragma once
 
 #include "common.cuh"
@@ -38,7 +37,7 @@ struct DecodeParams {
   int tiles_rem;        // the first tiles_rem chunks walk one tile more
   int n_row_parts;      // CTAs (per KV head) that share the fp16 / streamed rows: the chunk CTAs
                         // themselves when there is a middle, else CTAs of their own; 0: no rows
-  int n_parts;          // records per (sequence, query head): n_chunks rotated-space + n_row_parts standard
+  int n_parts;          // records per (sequence, query head): n_chunks in rotated space, or without a middle n_row_parts in standard space
   int n_ctas;           // CTAs per (sequence, KV head) = gridDim.x
   PeerPush push;        // sequence-split: deliver the combined record to every rank's exchange buffer
 };

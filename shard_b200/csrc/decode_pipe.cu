@@ -26,7 +26,7 @@
 // 0.94 of a tile's 1.8 K cycles on the tensor core; as mma.sync they take 32 instructions of 8 cycles a warp.  What they cost
 // instead: a stream of tcgen05.mma keeps mma.sync waiting, so the consumers' products run between the reconstruction
 // products of two tiles.  That, with the latency of a consumer's chain (tensor memory, rotation, scores, softmax, look-ups, P.V: about
-// 3 K cycles), bounds a tile: 2.7 K cycles.  Against the kernel with all products on tcgen05, shared-memory V tiles and three groups
+// 3 K cycles), bounds a tile: 2.4 to 2.7 K cycles.  Against the kernel with all products on tcgen05, shared-memory V tiles and three groups
 // (us a pass): 8K x 12 layers 198 -> 162, 32K x 12 383 -> 324, 131K x 4 408 -> 354, 64 sequences of 8K x 2 923 -> 738.
 // Measured and not kept: eight warps to a tile (80 registers: 8K 197, 131K 377), one paced issuing thread, the stage
 // handed back before the scores product, polling instead of suspended waits (131K 396).

@@ -13,7 +13,7 @@
 //                          division-free recurrence (one multiply-add of latency per row).
 //   3. tridiag_vectors_kernel  eigenvectors of the tridiagonal matrix by twisted factorisation, fp64,
 //                          thread = vector, one warp from either end.
-//   4. eig_products_kernel, eig_back_kernel    the reflectors applied to the vectors, eight to eight vectors per pass.
+//   4. eig_products_kernel, eig_back_kernel    the reflectors applied to the vectors, eight per pass to the four vectors of a CTA.
 //   5. eig_check_kernel    neighbouring vectors must be orthogonal; a matrix with eigenvalues too close
 //                          for step 3 is reported to the caller.
 //

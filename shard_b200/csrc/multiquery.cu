@@ -12,8 +12,8 @@
 //     warp 4      bulk copies of the tile images (two stages each) and all MMAs: S = Q K^T for the next
 //                 tile while the softmax works on this one, then O += P V with P's parts from tensor memory
 //
-// Weights of 11 bits would leave the output further from float64 than the decode launch's, which attends to
-// the rows outside the middle in fp32 and has exact fp16 values in the middle: up to 25 % where decoded tokens carry
+// Weights of 11 bits would leave the output further from float64 than the decode launch's, which weighs
+// the rows outside the middle with 22 bits and has exact fp16 values in the middle: up to 25 % where decoded tokens carry
 // the attention (2-norm 2.9e-4 against 2.3e-4; 2.2e-4 with both parts), 5 % with two KV heads.
 //
 // Shares are merged by multiquery_merge_kernel (their partial rows are fp32; a single share writes the

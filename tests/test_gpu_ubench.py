@@ -2,7 +2,8 @@
 that the figures the decode kernel's design rests on still hold on the GPU at hand: a 128-column
 k-step takes about 67 cycles and holds its issuing thread for nearly as long; a 16-column k-step is
 barely cheaper (about 59 cycles), whatever the accumulator or M; one decode tile's 29 instructions
-keep the tensor path busy for about 1.5 K cycles."""
+keep the tensor path busy for about 1.5 K cycles; mma.sync, a tenth of that alone, gets in once per
+tcgen05.mma of a stream; and a thread that does anything between two products waits for the first."""
 import os
 import re
 import shutil
@@ -46,3 +47,9 @@ def test_tcgen05_mma_cycle_table(tmp_path):
     heavy = rows["one decode tile (MN-major) + 15 warps of heavy shared-memory traffic"]
     assert 1200 <= tile_mn[0] <= 3000
     assert heavy[0] >= 0.95 * tile_mn[0]
+    # the two kinds of tensor instruction beside each other, and an issuing thread that polls
+    alone = rows["mma.sync m16n8k16, a warp per scheduler"][1]
+    beside = rows["the same beside a stream of m128 n128 TS"]
+    stream = rows["m128 n128 TS, long stream"][0]
+    assert 7 <= alone <= 14 and beside[1] >= 4 * alone and beside[0] >= stream
+    assert rows["m128 n128 TS, a shared word polled in between"][0] >= 2 * stream

@@ -408,7 +408,7 @@ __device__ __forceinline__ void head_output(const DecodeParams& p, const ShardSe
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       const float q = o4[c] * inv, r = fmaf(-q, L, o4[c]);
-      x[c] = r < 0.f || r > 0.f ? fmaf(r, inv, q) : q;
+      x[c] = fabsf(r) > 0.f ? fmaf(r, inv, q) : q;
     }
     const __half2 lo = __floats2half2_rn(x[0], x[1]), hi = __floats2half2_rn(x[2], x[3]);
     uint2 pk;

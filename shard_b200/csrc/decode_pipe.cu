@@ -60,7 +60,7 @@ constexpr int PP_TMEM_COLS = 512;
 constexpr int PP_COL_A = 128 * PP_ST;               // the A operand slots: R/2 coefficient columns + 8 constant columns 1, 0, ... each
 __host__ __device__ constexpr int pp_a_cols(int nw) { return 16 * nw + 8; }
 constexpr int PP_STATE = GQA * HD + 2 * GQA;        // a warp's state, floats: acc[4][128], max[4], sum-exp[4]
-constexpr float PP_W_LOG2 = 14.f;                   // weights of rows' values, at most 1, times 2^14 in fp16
+constexpr int PP_W_LOG2 = 14;                       // weights of rows' values, at most 2^0.5, times 2^14 in fp16
 constexpr float PP_LAZY_LOG2 = 8.f;                 // a softmax reference point moves only when exceeded by more than 2^8
 constexpr int PP_C_BUFS = 4;                        // coefficient tiles in shared memory
 constexpr int PP_V_BUFS = 6;                        // V code tiles (4 KB) in shared memory
@@ -143,13 +143,15 @@ __device__ __forceinline__ uint32_t lds_u1(uint32_t addr) {
 // query's are in the same), the scores come out with row lane / 4 (+ 8) and query head lane % 4 in a lane, and the values
 // are contracted over (row, parity of the channel).  What was 32-bit arithmetic when a warp took two rows at a time (and is in a launch
 // without a middle) keeps 22 bits: the weights, the codebook and the queries in code space are two fp16 parts each, the second scaled by 2^11 with
-// sums of its own, all products of every pair; queries and keys of fp16 rows are exact, and all sums are fp32.  (A second part that is
-// not scaled falls into fp16's subnormals: a weight of 2^-16 kept 9 bits.)  The weights of the values, p times the norm of a streamed row, are
-// split as w . 2^14 for w <= 1, a power of two from the running reference's: 22 bits from 1 down to 2^-28, and an error of 2^-50 below.
+// sums of its own; queries and keys of fp16 rows are exact, and all sums are fp32, rounded to nearest between products.  (A second part
+// that is not scaled falls into fp16's subnormals: a weight of 2^-16 kept 9 bits.  A product accumulates with truncation, which a chain of
+// them over all channels or blocks adds up.  Values take three of the four products of two parts: the fourth is 2^-22 of the first.)
+// The weights of the values, p times the norm of a streamed row, are split as w . 2^14 for w <= 2^0.5, w = p norm over a power
+// of two that follows the largest: 22 bits from 1 down to 2^-28, and an error of 2^-50 below.
 // Relative error of the sums against float64, fp16 rows / streamed ones: with even weights over 333 rows 6.8e-7 / 7.1e-7 (in 32-bit
 // arithmetic 7.0e-7 / 6.4e-7), where rows of weight 2^-20 carry the result 9.4e-7 / 9.4e-7 (8.5e-7 / 8.2e-7; 1.7e-3 and 6.3e-6 with unscaled
-// second parts and the products chained).  It costs 0.1 us a launch with streamed rows (8K x 12 layers 160.5 -> 161.4 us, 8 layers with 3001 streamed
-// rows 133.5 -> 133.6).
+// second parts and the products chained).  Against that cheaper form: 8K x 12 layers 160.8 -> 161.7 us, 8 layers with 3001 streamed rows
+// 133.7 -> 133.5, one layer of 2K tokens 15.9 -> 16.3 (with what the rounded quotient of the output costs).
 // Bound: latency of one block (loads, a chain of products, a softmax over 16 rows) -- some 200 instructions for 16 fp16 rows and
 // 700 for streamed ones, whose codes are looked up one by one; two rows at a time, with a reduction over the lanes for each, took
 // 1 K cycles a pair.
@@ -158,11 +160,12 @@ __device__ __forceinline__ uint32_t lds_u1(uint32_t addr) {
 // code space (H(signs o q) / sqrt(128)) and the score is norm . (query . codebook[code]); streamed values are summed in code space
 // and the SUM is rotated back, once per warp.  Streamed rows come first, so that one set of accumulators serves both kinds.
 struct RowState {
-  float m, l, j;      // of query head lane % 4: reference (log2 domain) and sum of the weights; o is in units of 2^(m + j - PP_W_LOG2), j whole
+  float m, l;         // of query head lane % 4: reference (log2 domain) and sum of the weights
+  int j;              // o is in units of 2^(m + j - PP_W_LOG2)
   float o[4][4];      // channels 16 (lane / 4) + 4 i + j of that head
 };
 __device__ __forceinline__ void row_state_init(RowState& st) {
-  st.m = neg_inf(); st.l = 0.f; st.j = 0.f;
+  st.m = neg_inf(); st.l = 0.f; st.j = 0;
 #pragma unroll
   for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] = 0.f;
 }
@@ -201,8 +204,8 @@ __device__ __forceinline__ float stream_query(const float4 sg, const __half* q, 
   *reinterpret_cast<uint2*>(out + HD + 4 * lane) = make_uint2(__byte_perm(sp[0], sp[1], 0x7632), __byte_perm(sp[2], sp[3], 0x7632));
   return __uint_as_float((127u - 25u + e) << 23);
 }
-// 2^n, exact; n whole and within +-126
-__device__ __forceinline__ float pow2_whole(float n) { return __int_as_float(((int)n + 127) << 23); }
+// 2^n, n within -126 .. 127
+__device__ __forceinline__ float pow2_whole(int n) { return __int_as_float((n + 127) << 23); }
 // weights of a block's rows: this lane has the scores sc[r] of rows lane / 4 + 8 r (log2 domain, -inf: no such row) and the norms vn[r] of
 // their values; gives the value weights as B fragments, w[part][m][slot] for rows 8 m + 2 (lane % 4) + slot
 __device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2], const float (&vn)[2], uint32_t (&w)[2][2][2], int lane) {
@@ -213,11 +216,12 @@ __device__ __forceinline__ void block_weights(RowState& st, const float (&sc)[2]
     tm = fmaxf(tm, __shfl_xor_sync(0xffffffffu, tm, off));
     tu = fmaxf(tu, __shfl_xor_sync(0xffffffffu, tu, off));
   }
-  const float m = fmaxf(st.m, tm), m0 = m == neg_inf() ? 0.f : m, u = fmaxf(st.m + st.j, tu);
-  const float j = u == neg_inf() ? st.j : fminf(fmaxf(ceilf(u - m0), -100.f), 100.f);
+  const float m = fmaxf(st.m, tm), m0 = m == neg_inf() ? 0.f : m, u = fmaxf(st.m + (float)st.j, tu);
+  // (adding 1.5 . 2^23 rounds to a whole number in the low bits: the weights are at most 2^0.5)
+  const int j = u == neg_inf() ? st.j : __float_as_int(fminf(fmaxf(u - m0, -100.f), 100.f) + 12582912.f) - 0x4B400000;
   const float pr[2] = {ex2(sc[0] - m0), ex2(sc[1] - m0)}, al = ex2(st.m - m0);
   st.l = fmaf(st.l, al, pr[0] + pr[1]);
-  const float al_o = al * pow2_whole(fminf(fmaxf(st.j - j, -126.f), 126.f)), up = pow2_whole(PP_W_LOG2 - j);
+  const float al_o = al * pow2_whole(min(max(st.j - j, -126), 126)), up = pow2_whole(PP_W_LOG2 - j);
   st.m = m; st.j = j;
 #pragma unroll
   for (int i = 0; i < 16; ++i) st.o[i >> 2][i & 3] *= al_o;
@@ -352,17 +356,16 @@ __device__ __forceinline__ void stream_block(RowState& st, const ShardSeq& sq, c
     uint32_t x[2][2][2][2];                           // [m][row][part][pair of codes]
 #pragma unroll
     for (int r = 0; r < 4; ++r) split_values(word(v[r], i), split, x[r >> 1][r & 1]);
-    float lo[4] = {}, cross[2][4] = {}, hi[4] = {};
+    float cross[4] = {}, hi[4] = {};
     auto products = [&](float(&o)[4], int vp, int wp) {
 #pragma unroll
       for (int m = 0; m < 2; ++m) mma_16816(o, x[m][0][vp][0], x[m][0][vp][1], x[m][1][vp][0], x[m][1][vp][1], w[wp][m][0], w[wp][m][1]);
     };
-    products(lo, 1, 1);
-    products(cross[0], 0, 1);
-    products(cross[1], 1, 0);
+    products(cross, 0, 1);
+    products(cross, 1, 0);
     products(hi, 0, 0);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) st.o[i][c] += fmaf(fmaf(lo[c], PP_LO_DOWN, cross[0][c] + cross[1][c]), PP_LO_DOWN, hi[c]);
+    for (int c = 0; c < 4; ++c) st.o[i][c] += fmaf(cross[c], PP_LO_DOWN, hi[c]);
   }
 }
 // normalised 128-point Hadamard transform of every query head's sums (channel 16 (lane / 4) + 4 i + j in o[i][j])

@@ -868,11 +868,6 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
         }
         if (ok) umma_commit_1t(KN_FULL(s));
       }
-      if (!ok || *abort_s) {
-        // giving up: do not leave while the tensor core may still be at work in this CTA's memory
-        umma_commit_1t(MMA_DONE(s));
-        mbar_wait(MMA_DONE(s), 0u, abort_s);
-      }
     }
     __syncwarp();
     griddep_wait();
@@ -967,17 +962,22 @@ __global__ void __launch_bounds__(PP_THREADS, 1) decode_partial_pipe_kernel(cons
   // ---- epilogue: merge the warps' states per head and emit the record -----------------------------------
   tc_fence_before();
   __syncthreads();
-  if (warp == PP_UNPACK_WARP0) tmem_dealloc(tmem_base, PP_TMEM_COLS);
-  if (*abort_s) {
-    // gave up somewhere: do not leave while a bulk copy may still be landing in this CTA's memory
+  if (__builtin_expect(*abort_s, 0)) {
+    // gave up somewhere, whichever role it was (nobody changes the flag any more): nobody leaves, and tensor memory is not freed, while the
+    // tensor core may still be at work in it or a bulk copy may still be landing in this CTA's memory
     if (tid == 0 && p.status) atomicExch(p.status, 1);
-    if (tid == PP_COEF_WARP * 32) {
+    if (warp >= PP_MMA_WARP && warp < PP_COEF_WARP && lane == 0) {
+      umma_commit_1t(MMA_DONE(warp - PP_MMA_WARP));
+      mbar_wait(MMA_DONE(warp - PP_MMA_WARP), 0u, abort_s);
+    } else if (tid == PP_COEF_WARP * 32) {
       for (int a = 0; a < W_ATOMS && n_my > 0; ++a) mbar_wait(W_FULL(a), 0u, abort_s);
       for (int c = max(0, asked - PP_C_BUFS); c < asked; ++c) mbar_wait(C_FULL(c % PP_C_BUFS), (uint32_t)((c / PP_C_BUFS) & 1), abort_s);
     } else if (tid == PP_VCODE_WARP * 32) {
       for (int c = max(0, asked - PP_V_BUFS); c < asked; ++c) mbar_wait(V_FULL(c % PP_V_BUFS), (uint32_t)((c / PP_V_BUFS) & 1), abort_s);
     }
+    __syncthreads();
   }
+  if (warp == PP_UNPACK_WARP0) tmem_dealloc(tmem_base, PP_TMEM_COLS);
   if (warp < PP_MMA_WARP) {
     // Warp = (query head, one of three), lane = four channels; maxima are in the log2 domain, the record carries the natural
     // logarithm's.  Each merges every third state, the head's first warp the three sums.
